@@ -91,17 +91,11 @@ static int check_mul(const TriMulDesc* d) {
   return 0;
 }
 
-// What the tensor-core attention kernels need beyond the descriptor: every tensor they reach through a tensor map
-// starts on a 16-byte boundary, and a bias that is present is not a broadcast view over heads or queries (its batch
-// stride may be zero).  Anything else runs on the CUDA-core kernels, which take any pointer and stride.
-static bool attn_operands_fit_tma(const TriAttnDesc* d, const void* bias, std::initializer_list<const void*> ptrs) {
+// What the tensor-core attention kernels need beyond the descriptor: q, k, v and dO, which they reach through tensor
+// maps, start on a 16-byte boundary.  Anything else runs on the CUDA-core kernels, which take any pointer and stride.
+static bool attn_operands_fit_tma(std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)
     if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
-  if (bias != nullptr) {
-    if ((reinterpret_cast<uintptr_t>(bias) & 15) != 0) return false;
-    if (d->bias_st[1] == 0 && d->H > 1) return false;
-    if (d->bias_st[2] == 0 && d->n_res > 1) return false;
-  }
   return true;
 }
 
@@ -162,7 +156,7 @@ int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void*
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_bytes, tri_stream_t stream) {
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse) return fail(TRI_ERR_ARG, "q, k, v, o and lse must not be null");
-  if (tc::attn_fwd_supported(d) && attn_operands_fit_tma(d, bias, {q, k, v})) {
+  if (tc::attn_fwd_supported(d) && attn_operands_fit_tma({q, k, v})) {
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -176,7 +170,7 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse || !d_o || !dq || !dk || !dv || !ws)
     return fail(TRI_ERR_ARG, "q, k, v, o, lse, d_o, dq, dk, dv and ws must not be null");
-  if (tc::attn_bwd_supported(d) && attn_operands_fit_tma(d, bias, {q, k, v, d_o})) {
+  if (tc::attn_bwd_supported(d) && attn_operands_fit_tma({q, k, v, d_o})) {
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);

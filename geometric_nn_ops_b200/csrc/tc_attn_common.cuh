@@ -1,0 +1,62 @@
+// Small device helpers shared by the tensor-core attention kernels.
+#pragma once
+
+#include "tc_common.cuh"
+
+namespace tri {
+namespace tc {
+namespace {
+
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kMaskSentinel = 1e9f;
+constexpr float kMaskLog2 = 1442695040.0f;   // the sentinel in units of log 2
+
+// byte offset of 16-byte chunk `g` (0..15, 8 elements each) of row r inside a [128 x 128] two-block SW128 tile
+__device__ __forceinline__ int sw128_chunk(int r, int g) {
+  return (g >> 3) * 16384 + r * 128 + (((g & 7) ^ (r & 7)) << 4);
+}
+
+template <typename T> struct ElemIsBf16 { static constexpr bool value = false; };
+template <> struct ElemIsBf16<__nv_bfloat16> { static constexpr bool value = true; };
+
+// two fp32 -> one packed pair of 16-bit values with a single conversion instruction
+template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+  __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+// one packed pair of 16-bit values -> two fp32
+template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t w);
+template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+// three-input maximum (one instruction on sm_100)
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float2 pair(uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); }
+__device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
+
+template <typename T>
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  union { uint4 u; T h[8]; } pk;
+  pk.u = v;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = to_f32(pk.h[i]);
+}
+
+// byte offset of 16-byte chunk g (0..7) of row r inside a one-block SW128 tile (rows of 64 16-bit elements)
+__device__ __forceinline__ int sw128_chunk1(int r, int g) { return r * 128 + ((g ^ (r & 7)) << 4); }
+
+}  // namespace
+}  // namespace tc
+}  // namespace tri

@@ -1,0 +1,451 @@
+// Forward triangle attention, 16-bit types, head dim up to 32: three rows of the pair tensor share a pair-bias tile.
+//
+// The pair bias depends on (head, query, key) only, so rows s .. s+2 of one head and 128-query block read the same
+// bias tiles.  A CTA takes such a triple: three groups of four softmax warps, one row each, walk the key axis in steps
+// of 64 keys; the bias tile of a step comes to shared memory once for the three of them.  Otherwise a group is on its
+// own: its Q, K, V tiles, its 160 TMEM columns and the lane that issues its copies and products.
+//
+// Per step and thread (one query row, 64 keys), sixteen logits at a time, in units of log 2:
+//   x = bias log2e + (S scale log2e + mask term) -> P = 2^(x - m), 16 bit -> O += P V.
+// One sweep without a maximum: P is formed against the reference m of the row (the largest of its first four logits to
+// start with).  P, its sum and O are floating point, so a reference that lags the maximum by a factor of up to kTooBig
+// loses nothing; the sum of a step shows whether a row has outgrown it, and then O and the sum are rescaled and the step
+// is done again.  S stays in TMEM until the check: P is stored over it afterwards.
+//
+// S is double buffered and P(c) takes the columns of S(c).  After P(c) the issuing lane sends P V(c) and S(c + 2),
+// which run in that order, so S(c + 1) is there before a thread asks for it and one arrival per step (p_ready) is all
+// that the softmax warps owe.  With S single buffered each step waited about 600 clocks for the next product, and the
+// waiting warps' polling took half of all issue slots.
+//
+// What bounds it: the exponentials (16 per clock and SM: 8 clocks of a sub-partition per 32), then the waits a row's four
+// warps, which run on four sub-partitions, have for one another.  N = 768, 4 heads, bf16: 0.73 ms, 58 % of the exponential
+// pipe, against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
+// also read 2 bytes of bias per logit from L2; here 0.67).
+#include <algorithm>
+
+#include "tc_attn_common.cuh"
+#include "tc_attn_rows.cuh"
+
+namespace tri {
+namespace tc {
+
+namespace {
+
+constexpr int kGroups = 3;                  // rows per CTA
+constexpr int kBiasStages = 4;
+constexpr int kThreads = (4 * kGroups + kGroups + 1) * 32;   // softmax warps, issuing warps, one warp for the bias tiles
+constexpr float kLn2 = 0.6931471805599453f;
+
+struct RowsArgs {
+  int B, S, N, H, D;
+  float scale2;              // scale * log2e
+  void* o;
+  int64_t o_st[4];
+  float* stats;              // [2][B][S][H][N]: row maximum, log row sum
+  const float* mask_terms;
+  int npad;
+  int bias_b_mul;
+  int rows_per_item;         // groups in use (fewer where a quad per CTA would leave SMs idle)
+  uint32_t idesc_s, idesc_pv;
+  int* err;
+};
+
+struct RowsSmem {
+  static constexpr int TQ = 128 * 64, TK = 64 * 64, TB = 128 * 128;   // bytes: Q tile, K or V tile, bias tile
+  static constexpr int OFF_BIAS = 0;
+  static constexpr int OFF_Q = OFF_BIAS + kBiasStages * TB;     // [group][3]
+  static constexpr int OFF_K = OFF_Q + kGroups * 3 * TQ;        // [group][3]
+  static constexpr int OFF_V = OFF_K + kGroups * 3 * TK;        // [group][3]
+  static constexpr int OFF_M = OFF_V + kGroups * 3 * TK;        // [bias stage][group] x 64 mask terms
+  static constexpr int OFF_BAR = OFF_M + kBiasStages * kGroups * 256;
+  static constexpr int SMEM = OFF_BAR + 1024 + 1024;
+};
+
+// barriers of one group
+struct GroupBars {
+  uint64_t first[2];  // Q, K of the first two S products
+  uint64_t in[3];     // [c % 3]: what the issuing lane needs at step c
+  uint64_t mma[2];    // [c & 1]: S(c) is in TMEM and P V(c - 2) is done
+  uint64_t p_ready[2];   // [c & 1]: the four warps have read S(c) and its mask terms and stored P(c); they may do so for
+                         // step c + 1 before the issuing lane has seen step c, hence two
+};
+
+// tcgen05.wait::ld that the registers of the load pass through, so that no use of them can move above it
+__device__ __forceinline__ void ld_wait16(uint32_t (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                 "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
+
+template <typename T, bool HB>
+__global__ void __launch_bounds__(kThreads, 1)
+attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias, const RowsArgs a) {
+  using M = RowsSmem;
+  constexpr float kTooBig = ElemIsBf16<T>::value ? 1.152921504606847e18f : 32768.0f;   // 2^60; fp16 tops out at 2^16
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  GroupBars* bars = reinterpret_cast<GroupBars*>(smem + M::OFF_BAR);
+  uint64_t* b_full = reinterpret_cast<uint64_t*>(bars + kGroups);   // [kBiasStages]
+  uint64_t* b_free = b_full + kBiasStages;                          // [kBiasStages]: 16 warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_free + kBiasStages);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qblocks = (a.N + 127) / 128, nk = (a.N + 63) / 64;
+  const int R = a.rows_per_item, squads = (a.S + R - 1) / R;
+  const long long items = (long long)qblocks * a.H * squads * a.B;
+  const int my_items = blockIdx.x < items ? (int)((items - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+  struct Item { int q0, h, s0, b; };
+  auto item_of = [&](int n) {
+    unsigned z = blockIdx.x + (unsigned)n * gridDim.x;
+    Item it;
+    it.q0 = (int)(z % (unsigned)qblocks) * 128; z /= (unsigned)qblocks;
+    it.h = (int)(z % (unsigned)a.H); z /= (unsigned)a.H;
+    it.s0 = (int)(z % (unsigned)squads) * R;
+    it.b = (int)(z / (unsigned)squads);
+    return it;
+  };
+
+  if (tid == 0) {
+    for (int g = 0; g < kGroups; ++g) {
+      mbar_init(&bars[g].first[0], 1); mbar_init(&bars[g].first[1], 1);
+      for (int i = 0; i < 3; ++i) mbar_init(&bars[g].in[i], 1);
+      mbar_init(&bars[g].mma[0], 1); mbar_init(&bars[g].mma[1], 1); mbar_init(&bars[g].p_ready[0], 4); mbar_init(&bars[g].p_ready[1], 4);
+    }
+    for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_free[i], 4 * R); }
+    mbar_fence_init();
+  }
+  if (warp == 0) tmem_alloc(tmem_slot, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  constexpr uint32_t COLS = 160, COL_O = 128;   // a group's columns: S / P of even and odd steps at 0 and 64, O
+  bool ok = true;
+
+  if (warp == 5 * kGroups) {
+    // ------------------------------------ bias tiles and mask terms --------------------------------
+    if (lane == 0) {
+      int stg = 0;
+      uint32_t ph = 0;
+      for (int n = 0; n < my_items && ok; ++n) {
+        const Item it = item_of(n);
+        for (int j = 0; j < nk; ++j) {
+          ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51);
+          if (!ok) break;
+          const int rows = min(R, a.S - it.s0);
+          mbar_expect_tx(&b_full[stg], (HB ? M::TB : 0) + rows * 256);
+          for (int g = 0; g < rows; ++g)
+            bulk_load(smem + M::OFF_M + (stg * kGroups + g) * 256, a.mask_terms + ((long long)it.b * a.S + it.s0 + g) * a.npad + j * 64, 256, &b_full[stg]);
+          if (HB) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB, &tmBias, &b_full[stg], j * 64, it.q0, it.h, it.b * a.bias_b_mul);
+          if (++stg == kBiasStages) { stg = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp >= 4 * kGroups) {
+    // ------------------------------------ copies and products of group g --------------------------
+    // The whole warp runs this code and one lane issues: every index is warp-uniform and stays in uniform registers.
+    const int g = warp - 4 * kGroups;
+    if (g < R) {
+      GroupBars& gb = bars[g];
+      uint8_t* sQ = smem + M::OFF_Q + g * 3 * M::TQ;
+      uint8_t* sK = smem + M::OFF_K + g * 3 * M::TK;
+      uint8_t* sV = smem + M::OFF_V + g * 3 * M::TK;
+      const uint32_t t0 = tmem_base + g * COLS;
+      const bool leader = elect_one();
+      constexpr uint32_t HI = desc_hi(8 * 64, 4);   // 64-byte rows, SWIZZLE_64B
+      const uint32_t q_lo = desc_lo(smem_u32(sQ), 16), k_lo = desc_lo(smem_u32(sK), 16), v_lo = desc_lo(smem_u32(sV), 64 * 64);
+      int total = 0;                        // steps of this group: rows beyond S are left out
+      for (int n = 0; n < my_items; ++n) total += item_of(n).s0 + g < a.S ? nk : 0;
+      // a position in the group's stream: item, key step, ring stage, Q buffer
+      struct Cursor { Item it; int n, j, left, stg, q; };
+      auto start = [&](Cursor& u) {         // the item at (or after) n that this group has a row in
+        while (u.it.s0 + g >= a.S) u.it = item_of(++u.n);
+      };
+      auto next = [&](Cursor& u) {
+        --u.left;
+        if (++u.stg == 3) u.stg = 0;
+        if (++u.j == nk) {
+          u.j = 0;
+          if (++u.q == 3) u.q = 0;
+          if (u.left > 0) { u.it = item_of(++u.n); start(u); }
+        }
+      };
+      Cursor kc{item_of(0), 0, 0, total, 0, 0};
+      if (total > 0) start(kc);
+      Cursor vc = kc;
+      // What step c needs besides P(c) -- V(c), and K(c + 2) with its Q for S(c + 2) -- arrives on one barrier, in[c % 3].
+      auto load = [&](uint64_t* bar, bool k, bool v) {
+        if (leader) {
+          mbar_expect_tx(bar, (k ? M::TK + (kc.j == 0 ? M::TQ : 0) : 0) + (v ? M::TK : 0));
+          if (k && kc.j == 0) tma_load_5d(sQ + kc.q * M::TQ, &tmQ, bar, 0, kc.it.h, kc.it.q0, kc.it.s0 + g, kc.it.b);
+          if (k) tma_load_5d(sK + kc.stg * M::TK, &tmK, bar, 0, kc.it.h, kc.j * 64, kc.it.s0 + g, kc.it.b);
+          if (v) tma_load_5d(sV + vc.stg * M::TK, &tmV, bar, 0, vc.it.h, vc.j * 64, vc.it.s0 + g, vc.it.b);
+        }
+        if (k) next(kc);
+        if (v) next(vc);
+      };
+      int sj = 0, sq = 0, sk = 0;           // key step, Q buffer and K stage of the next S product
+      auto issue_s = [&](uint32_t t) {
+        const uint32_t s_q = q_lo + sq * (M::TQ >> 4), s_k = k_lo + sk * (M::TK >> 4);
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            umma<KIND_F16>(t, desc_join(s_q + ks * 2, HI), desc_join(s_k + ks * 2, HI), a.idesc_s, ks > 0);
+        }
+        if (++sj == nk) { sj = 0; if (++sq == 3) sq = 0; }
+        if (++sk == 3) sk = 0;
+      };
+      for (int c = 0; c < 2 && c < total; ++c) load(&gb.first[c], true, false);
+      if (total > 0) load(&gb.in[0], total > 2, true);
+      for (int c = 0; c < 2 && c < total; ++c) {
+        ok = mbar_wait(&gb.first[c], 0, a.err, 52) && ok;
+        tc_fence_after_sync();
+        issue_s(t0 + c * 64);
+        if (leader) umma_commit(&gb.mma[c]);
+      }
+      int j = 0, stg = 0;                   // key step and ring stage (V and barrier) of step c
+      uint32_t ph = 0;
+      for (int c = 0; c < total && ok; ++c) {
+        const bool more = c + 2 < total;
+        const uint32_t v_at = v_lo + stg * (M::TK >> 4), tp = t0 + (c & 1) * 64, first = j > 0 ? 1u : 0u;
+        ok = mbar_wait_relaxed(&gb.in[stg], ph, a.err, 53) && ok;
+        // every warp has stored P(c): it had waited for S(c), which followed P V(c - 2): the K stage of c and the V stage
+        // of c - 2 are free
+        ok = mbar_wait_relaxed(&gb.p_ready[c & 1], (c >> 1) & 1, a.err, 55) && ok;
+        tc_fence_after_sync();
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_ts_f16(t0 + COL_O, tp + kk * 8, desc_join(v_at + kk * 64, HI), a.idesc_pv, kk > 0 ? 1u : first);
+        }
+        if (more) issue_s(tp);               // into the columns P V(c) reads: products of one thread run in order
+        if (leader) umma_commit(&gb.mma[c & 1]);
+        if (++stg == 3) { stg = 0; ph ^= 1; }
+        if (c + 1 < total) load(&gb.in[stg], c + 3 < total, true);   // V(c + 1), K(c + 3)
+        if (++j == nk) j = 0;
+      }
+    }
+  } else {
+    // ------------------------------------ softmax of group g --------------------------------------
+    const int g = warp >> 2, r = tid & 127;
+    GroupBars& gb = bars[g];
+    const uint32_t t_row = tmem_base + g * COLS + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t mask_s = smem_u32(smem + M::OFF_M) + g * 256, bias_row = smem_u32(smem + M::OFF_BIAS) + r * 128 + ((r & 7) << 4);
+    const float2 sc2 = splat(a.scale2), l2e2 = splat(kLog2e);
+    int c = 0, bstg = 0;
+    uint32_t bph = 0;
+    bool early_s = false, early_b = false;
+    // the row that is finished but for its last P V: statistics, where its results go
+    bool pend = false;
+    float pm = 0.f, pl = 0.f, pseen = 0.f;
+    int po = -1, pstat = 0;   // O row in units of 8 elements, -1 where the query is beyond N; row of the statistics
+    // O and the statistics of the row, once P V of its last step `cl` is done; no later P V can have been issued yet
+    auto finish = [&](int cl) {
+      if (!mbar_wait(&gb.mma[cl & 1], ((cl >> 1) + 1) & 1, a.err, 59)) ok = false;
+      tc_fence_after_sync();
+      uint32_t o[2][16];
+      tmem_ld_32x16(t_row + COL_O, o[0]);
+      tmem_ld_32x16(t_row + COL_O + 16, o[1]);
+      ld_wait16(o[0]);
+      ld_wait16(o[1]);
+      if (po >= 0 && ok) {
+        const float inv = 1.0f / pl;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (h * 8 < a.D) {
+            uint4 pk;
+            auto f = [&](int i) { return __uint_as_float(o[h >> 1][(h & 1) * 8 + i]) * inv; };
+            pk.x = pack2<T>(f(0), f(1)); pk.y = pack2<T>(f(2), f(3)); pk.z = pack2<T>(f(4), f(5)); pk.w = pack2<T>(f(6), f(7));
+            (reinterpret_cast<uint4*>(a.o) + po)[h] = pk;
+          }
+        }
+        // Natural units.  The largest of the steps' sums over 64 keys is 1 to 64 times the largest P, so that m plus
+        // log2(sum / 64) lies at most 6 below the row's maximum; m itself is one of the logits.  A fully masked row keeps
+        // the sentinel's exact value, which the backward forms again.
+        const bool masked = pm < -1e8f;
+        const float lift = masked ? 0.f : fmaxf(__log2f(pseen) - 6.0f, 0.f);
+        a.stats[pstat] = masked ? fmaf(pm + kMaskLog2, kLn2, -kMaskSentinel) : (pm + lift) * kLn2;
+        a.stats[(long long)a.B * a.S * a.H * a.N + pstat] = logf(pl) - lift * kLn2;
+      }
+    };
+    for (int n = 0; g < R && n < my_items && ok; ++n) {
+      const Item it = item_of(n);
+      if (it.s0 + g >= a.S) {   // no row for this group: let the bias tiles pass
+        for (int j = 0; j < nk && ok; ++j) {
+          ok = mbar_wait_relaxed(&b_full[bstg], bph, a.err, 57);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&b_free[bstg]);
+          if (++bstg == kBiasStages) { bstg = 0; bph ^= 1; }
+        }
+        early_b = false;
+        continue;
+      }
+      float m = -INFINITY, l = 0.f;   // reference, sum of P
+      float seen = 0.f;               // largest sum of a step against this reference
+      for (int j = 0; j < nk; ++j, ++c) {
+        if (!early_s && !mbar_wait(&gb.mma[c & 1], (c >> 1) & 1, a.err, 58)) ok = false;
+        if (!early_b && !mbar_wait(&b_full[bstg], bph, a.err, 57)) ok = false;
+        tc_fence_after_sync();
+        const uint32_t mrow = mask_s + bstg * (kGroups * 256), brow = bias_row + bstg * M::TB, t_s = t_row + (c & 1) * 64;
+        auto logits = [&](const uint32_t (&cur)[16], int q, float2 (&x)[8]) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float4 mA = lds128f(mrow + (q * 4 + u * 2) * 16), mB = lds128f(mrow + (q * 4 + u * 2 + 1) * 16);
+            const float2 mk[4] = {make_float2(mA.x, mA.y), make_float2(mA.z, mA.w), make_float2(mB.x, mB.y), make_float2(mB.z, mB.w)};
+            uint4 raw = make_uint4(0, 0, 0, 0);
+            if constexpr (HB) raw = lds128(brow ^ ((q * 2 + u) << 4));   // (128-byte rows, 16-byte chunks swizzled by the row)
+            const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
+              if constexpr (HB) v = __ffma2_rn(unpack2<T>(bw[i]), l2e2, v);
+              x[u * 4 + i] = v;
+            }
+          }
+        };
+        auto exps = [&](const float2 (&x)[8], float2 nm, uint32_t* w, float2& sum) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float2 e = __fadd2_rn(x[i], nm);
+            const float2 p = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+            sum = __fadd2_rn(sum, p);
+            w[i] = pack2<T>(p.x, p.y);
+          }
+        };
+        // P = 2^(x - m) of this thread's 64 keys and their sum
+        float2 ps = make_float2(0.f, 0.f);
+        uint32_t pw[32], ra[16], rb[16];
+        auto chunk = [&](uint32_t (&cur)[16], uint32_t (&nxt)[16], int q) {   // sixteen keys; the next sixteen on their way
+          ld_wait16(cur);
+          if (q < 3) tmem_ld_32x16(t_s + (q + 1) * 16, nxt);
+          float2 x[8];
+          logits(cur, q, x);
+          if (q == 0) m = j > 0 ? m : fmaxf(fmaxf(x[0].x, x[0].y), fmaxf(x[1].x, x[1].y));   // (key 0 is in range: finite)
+          exps(x, splat(-m), pw + q * 8, ps);
+        };
+        tmem_ld_32x16(t_s, ra);
+        chunk(ra, rb, 0);
+        chunk(rb, ra, 1);
+        chunk(ra, rb, 2);
+        chunk(rb, ra, 3);
+        // whether the next step's S and bias tile are there: asked now, needed at the top
+        early_s = mbar_test(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1);
+        early_b = mbar_test(&b_full[bstg + 1 == kBiasStages ? 0 : bstg + 1], bstg + 1 == kBiasStages ? bph ^ 1 : bph);
+        float sum = ps.x + ps.y;
+        if (!__any_sync(0xffffffffu, !(sum < kTooBig))) {
+          tmem_st_32x32(t_s, pw);   // over the S values this warp has read: 64 keys as 32 packed columns
+        } else {
+          // Some row of the warp outgrew its reference: take the maximum of the step, scale by 2^(m - m_new) the sum and O
+          // (once P V of the step before is done), and form P again.  (Sixteen keys' P end before the next sixteen's S.)
+          float top = m;
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            float2 x[8];
+            tmem_ld_32x16(t_s + q * 16, ra);
+            ld_wait16(ra);
+            logits(ra, q, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) top = fmax3(top, x[i].x, x[i].y);
+          }
+          const float alpha = ex2_approx(m - top);
+          m = top;
+          l *= alpha;
+          if (j > 0) {
+            ok = mbar_wait(&gb.mma[(c - 1) & 1], (((c - 1) >> 1) + 1) & 1, a.err, 59) && ok;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              tmem_ld_32x16(t_row + COL_O + h * 16, ra);
+              ld_wait16(ra);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) * alpha);
+              tmem_st_32x16(t_row + COL_O + h * 16, ra);
+            }
+          }
+          ps = make_float2(0.f, 0.f);
+          seen = 0.f;
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            float2 x[8];
+            uint32_t w[8];
+            tmem_ld_32x16(t_s + q * 16, ra);
+            ld_wait16(ra);
+            logits(ra, q, x);
+            exps(x, splat(-m), w, ps);
+            tmem_st_32x8(t_s + q * 8, w);
+          }
+          sum = ps.x + ps.y;
+        }
+        l += sum;
+        seen = fmaxf(seen, sum);
+        if (j == 0 && pend) finish(c - 1);   // the row before this one
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&gb.p_ready[c & 1]);
+          mbar_arrive(&b_free[bstg]);
+        }
+        if (++bstg == kBiasStages) { bstg = 0; bph ^= 1; }
+        if (!ok) break;
+      }
+      pend = true; pm = m; pl = l; pseen = seen;
+      const int qi = it.q0 + r, s = it.s0 + g;
+      po = qi < a.N ? (int)((it.b * a.o_st[0] + s * a.o_st[1] + qi * a.o_st[2] + it.h * a.o_st[3]) >> 3) : -1;
+      pstat = ((it.b * a.S + s) * a.H + it.h) * a.N + qi;
+    }
+    if (pend && ok) finish(c - 1);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+}  // namespace
+
+bool attn_fwd_rows_fits(const TriAttnDesc* d) {
+  const int64_t last = (d->B - 1) * d->o_st[0] + (d->n_seq - 1) * d->o_st[1] + (d->n_res - 1) * d->o_st[2] + (d->H - 1) * d->o_st[3];
+  return (int64_t)d->B * d->n_seq * d->H * d->n_res < (int64_t)1 << 31 && last / 8 < ((int64_t)1 << 31) - 8;
+}
+
+int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void* v, const CUtensorMap* tbias,
+                  bool bias_batched, void* o, float* stats, const float* mask_terms, int* err, cudaStream_t st) {
+  CUtensorMap tq, tk, tv;
+  TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, 32));
+  TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, 32));
+  TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, 32));
+  RowsArgs a;
+  a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D;
+  a.scale2 = d->scale * kLog2e;
+  a.o = o;
+  for (int i = 0; i < 4; ++i) a.o_st[i] = d->o_st[i];
+  a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
+  a.bias_b_mul = bias_batched ? 1 : 0;
+  a.err = err;
+  const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
+  a.idesc_s = make_idesc(kind, 128, 64, false, false);
+  a.idesc_pv = make_idesc(kind, 128, 32, false, true);
+  const long long combos = (long long)((d->n_res + 127) / 128) * d->H * d->B;
+  int rows = kGroups;
+  while (rows > 1 && combos * cdiv(d->n_seq, rows) < sm_count()) --rows;   // fewer rows per CTA before an SM stays idle
+  a.rows_per_item = rows;
+  const long long items = combos * cdiv(d->n_seq, rows);
+  const double pairs = (double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res;
+  KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
+  auto launch = [&](auto kern, const CUtensorMap& tb) {
+    TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem::SMEM));
+    kern<<<(unsigned)std::min<long long>(items, sm_count()), kThreads, RowsSmem::SMEM, st>>>(tq, tk, tv, tb, a);
+    TRI_LAUNCH_OK();
+    return 0;
+  };
+  if (d->dtype == TRI_BF16)
+    return tbias ? launch(attn_fwd_rows_kernel<__nv_bfloat16, true>, *tbias) : launch(attn_fwd_rows_kernel<__nv_bfloat16, false>, tq);
+  return tbias ? launch(attn_fwd_rows_kernel<__half, true>, *tbias) : launch(attn_fwd_rows_kernel<__half, false>, tq);
+}
+
+}  // namespace tc
+}  // namespace tri

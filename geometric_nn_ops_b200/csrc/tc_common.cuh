@@ -1,7 +1,7 @@
 // Blackwell (sm_100a) building blocks: mbarrier, TMA (cp.async.bulk.tensor), TMEM allocation,
 // tcgen05.mma / commit / ld, and the shared-memory and instruction descriptors they take.
 //
-// Every wait here is BOUNDED: after kSpinLimit polls the waiter records a code in a device error
+// Every wait here is BOUNDED: after a limit (kWaitLimitCycles) the waiter records a code in a device error
 // word and returns, so a protocol bug shows up as TRI_ERR_DEVICE instead of a hung GPU.
 #pragma once
 
@@ -15,10 +15,11 @@ namespace tc {
 // ---------------------------------------------------------------------------------------------
 // device error word (one per launch, zeroed by the host before the launch)
 // ---------------------------------------------------------------------------------------------
-// A try_wait suspends the thread in hardware until the phase completes or kWaitHintNs elapse, so a waiting
-// warp issues almost no instructions (a bare polling loop took a third of all issue slots in the attention
-// kernels).  Every wait gives up after kWaitLimitCycles SM clocks (about two seconds).
-constexpr uint32_t kWaitHintNs = 1000000;
+// A try_wait suspends the thread in hardware for a moment and is repeated in a loop of three instructions: with the loop
+// in C (a counter, the error word, a hint of a long suspension that put the warp to sleep past the arrival) the waiting
+// warps issued as many instructions as the arithmetic of the attention kernels.  After kPolls failures the waiter looks
+// at the error word and the clock; every wait gives up after kWaitLimitCycles SM clocks (about two seconds).
+constexpr uint32_t kPolls = 512;
 constexpr long long kWaitLimitCycles = 4000000000LL;
 
 __device__ __forceinline__ void report_timeout(int* err, int code) {
@@ -42,30 +43,86 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+// up to `polls` attempts; true once the phase has completed
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t polls) {
   uint32_t ok;
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
+      "TRY:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra DONE;\n\t"
+      "sub.u32 n, n, 1;\n\t"
+      "setp.ne.u32 q, n, 0;\n\t"
+      "@q bra TRY;\n"
+      "DONE:\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(polls)
       : "memory");
   return ok != 0;
 }
-// Returns false (and records `code`) if the phase did not complete within the poll limit.
+// has the phase completed?  Never suspends: asked ahead of need, its latency hides under other work.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Returns false (and records `code`) if the phase did not complete within the limit.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait(bar, parity, kPolls)) return true;
   const long long t0 = clock64();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 0xf) == 0) {
-      if (err != nullptr && *(volatile int*)err != 0) return false;  // someone else gave up
-      if (clock64() - t0 > kWaitLimitCycles) break;
+  while (!mbar_try_wait(bar, parity, kPolls)) {
+    if (err != nullptr && *(volatile int*)err != 0) return false;  // someone else gave up
+    if (clock64() - t0 > kWaitLimitCycles) {
+      report_timeout(err, code);
+      return false;
     }
+  }
+  return true;
+}
+
+// The same wait for threads that issue copies and products well ahead of their use: it sleeps between attempts and leaves
+// the issue slots to the warps that compute.
+__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, int* err, int code) {
+  if (mbar_test(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    for (uint32_t i = 0; i < 1024; ++i) {
+      __nanosleep(100);
+      if (mbar_test(bar, parity)) return true;
+    }
+    if (err != nullptr && *(volatile int*)err != 0) return false;
+    if (clock64() - t0 > kWaitLimitCycles) break;
   }
   report_timeout(err, code);
   return false;
+}
+
+// Shared-memory accesses by 32-bit address.  The tiles start at an address rounded up at run time, which hides from
+// the compiler that they are in shared memory: through a plain pointer these became generic loads and stores.
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 lds128f(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float lds32f(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
 // generic-proxy writes to smem -> visible to the async proxy (TMA store, tcgen05.mma operands)
@@ -173,6 +230,28 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
       "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
       "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+      "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+      "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
