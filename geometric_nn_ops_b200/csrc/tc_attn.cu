@@ -95,7 +95,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const AttnArgs a) {
   using G = Geo<HD>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sQ = smem + G::OFF_Q;
   uint8_t* sK = smem + G::OFF_K;
   uint8_t* sV = smem + G::OFF_V;
@@ -486,7 +486,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                      const __grid_constant__ CUtensorMap tmBias, const AttnBwdArgs a) {
   using G = GeoC<HD>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem + G::OFF_K;
   uint8_t* sV = smem + G::OFF_V;
   uint8_t* sQ = smem + G::OFF_Q;
@@ -818,7 +818,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmBias, const AttnBwdArgs a) {
   using G = GeoQ<HD>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sQ = smem + G::OFF_Q;
   uint8_t* sDO = smem + G::OFF_DO;
   uint8_t* sK = smem + G::OFF_K;
@@ -1056,7 +1056,7 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                       const __grid_constant__ CUtensorMap tmBias, const AttnBwdArgs a) {
   using G = GeoB<HD>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sBias = smem + G::OFF_BIAS;
   uint64_t* bar_once = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);   // bias tile
   uint64_t* bar_in = bar_once + 1;     // [NS]

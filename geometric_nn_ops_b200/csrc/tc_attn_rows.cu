@@ -84,7 +84,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   using M = RowsSmem;
   constexpr float kTooBig = ElemIsBf16<T>::value ? 1.152921504606847e18f : 32768.0f;   // 2^60; fp16 tops out at 2^16
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   GroupBars* bars = reinterpret_cast<GroupBars*>(smem + M::OFF_BAR);
   uint64_t* b_full = reinterpret_cast<uint64_t*>(bars + kGroups);   // [kBiasStages]
   uint64_t* b_free = b_full + kBiasStages;                          // [kBiasStages]: 16 warps

@@ -38,10 +38,10 @@ enum Epilogue {
 
 constexpr int kBM = 128;
 constexpr int kStageA = kBM * 128;  // bytes
-// warp 0 producer, warp 1 MMA, then the epilogue warps: 16 for the gate-in, gate-out and gate-out backward
-// epilogues, whose per-element arithmetic (sigmoid, products) is latency-bound with fewer warps per scheduler; 8 for
-// the plain store and for gate-in backward (which spends its registers on a tile-ahead prefetch instead)
-constexpr int gemm_epi_warps(int epi) { return (epi == 0 || epi == 4) ? 8 : 16; }
+// warp 0 producer, warp 1 MMA, then the epilogue warps: 16 for the gate epilogues, whose per-element arithmetic (sigmoid,
+// products) is latency-bound with fewer warps per scheduler, 8 for the plain store.  (Gate-in backward on 8 warps with the
+// gradients fetched a tile ahead into registers: 0.381 ms per launch at 768 x 768 pixels against 0.365.)
+constexpr int gemm_epi_warps(int epi) { return epi == 0 ? 8 : 16; }
 constexpr int gemm_threads(int epi) { return 64 + 32 * gemm_epi_warps(epi); }
 
 struct GemmArgs {
@@ -77,15 +77,16 @@ template <> struct ElemTraits<__half> { static constexpr int kind = KIND_F16; };
 template <> struct ElemTraits<float> { static constexpr int kind = KIND_TF32; };
 
 __device__ __forceinline__ float fast_sigmoid(float x) {
-  return __fdividef(1.0f, 1.0f + ex2_approx(-1.4426950408889634f * x));
+  return rcp_approx(1.0f + ex2_approx(-1.4426950408889634f * x));
 }
 
-// sigmoid of two values with packed fp32x2 arithmetic around the two MUFU pairs (the gate epilogues are bound by
-// instruction issue, and a packed instruction does the work of two)
-__device__ __forceinline__ float2 sigmoid2(float2 x) {
-  const float2 t = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+// sigmoid(x + b) of two values, x from the accumulator and nb2 = -b log2e: packed fp32x2 arithmetic around the two MUFU
+// pairs.  (A quotient by __fdividef costs several instructions of range handling, which the denominator 1 + 2^y, at
+// least one, does not need.)
+__device__ __forceinline__ float2 sigmoid2(float2 x, float2 nb2 = make_float2(0.f, 0.f)) {
+  const float2 t = __ffma2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f), nb2);
   const float2 den = __fadd2_rn(make_float2(ex2_approx(t.x), ex2_approx(t.y)), make_float2(1.0f, 1.0f));
-  return make_float2(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
+  return make_float2(rcp_approx(den.x), rcp_approx(den.y));
 }
 
 // 8 consecutive elements <-> registers, with 16-byte (16-bit types) or 2 x 16-byte (fp32) accesses
@@ -105,10 +106,7 @@ template <typename T> __device__ __forceinline__ void store8(T* p, const float* 
     reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
     reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
   } else {
-    union { uint4 u; T h[8]; } pk;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) pk.h[i] = from_f32<T>(v[i]);
-    *reinterpret_cast<uint4*>(p) = pk.u;
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack2<T>(v[0], v[1]), pack2<T>(v[2], v[3]), pack2<T>(v[4], v[5]), pack2<T>(v[6], v[7]));
   }
 }
 
@@ -133,6 +131,18 @@ template <typename T> __device__ __forceinline__ void cvtraw8(const Raw8<T>& r, 
   }
 }
 
+// the same as four packed pairs
+template <typename T> __device__ __forceinline__ void cvtraw8p(const Raw8<T>& r, float2 (&v)[4]) {
+  const uint4 a = r.w[0];
+  if constexpr (sizeof(T) == 4) {
+    const uint4 b = r.w[1];
+    v[0] = make_float2(__uint_as_float(a.x), __uint_as_float(a.y)); v[1] = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
+    v[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); v[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
+  } else {
+    v[0] = unpack2<T>(a.x); v[1] = unpack2<T>(a.y); v[2] = unpack2<T>(a.z); v[3] = unpack2<T>(a.w);
+  }
+}
+
 // 32-byte accesses (16 values of a 16-bit type) for the channel-major tensors of the transposed gate GEMMs: a lane
 // then reads or writes whole 32-byte sectors of its channel row instead of two half sectors in two requests.
 template <typename T> __device__ __forceinline__ void ldraw16(const T* p, Raw8<T>& lo, Raw8<T>& hi) {
@@ -142,13 +152,34 @@ template <typename T> __device__ __forceinline__ void ldraw16(const T* p, Raw8<T
                  "=r"(hi.w[0].z), "=r"(hi.w[0].w)
                : "l"(p));
 }
+// the i-th pair of eight values, and stores of eight and sixteen
+template <typename T> __device__ __forceinline__ void putraw8(Raw8<T>& r, int i, float2 v) {
+  if constexpr (sizeof(T) == 4) {
+    uint4& w = r.w[i >> 1];
+    if (i & 1) { w.z = __float_as_uint(v.x); w.w = __float_as_uint(v.y); }
+    else { w.x = __float_as_uint(v.x); w.y = __float_as_uint(v.y); }
+  } else {
+    const uint32_t k = pack2<T>(v.x, v.y);
+    if (i == 0) r.w[0].x = k; else if (i == 1) r.w[0].y = k; else if (i == 2) r.w[0].z = k; else r.w[0].w = k;
+  }
+}
+template <typename T> __device__ __forceinline__ void straw8(T* p, const Raw8<T>& r) {
+  reinterpret_cast<uint4*>(p)[0] = r.w[0];
+  if constexpr (sizeof(T) == 4) reinterpret_cast<uint4*>(p)[1] = r.w[1];
+}
+template <typename T> __device__ __forceinline__ void straw16(T* p, const Raw8<T>& lo, const Raw8<T>& hi) {
+  static_assert(sizeof(T) == 2, "16-bit types");
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.w[0].x), "r"(lo.w[0].y), "r"(lo.w[0].z),
+               "r"(lo.w[0].w), "r"(hi.w[0].x), "r"(hi.w[0].y), "r"(hi.w[0].z), "r"(hi.w[0].w)
+               : "memory");
+}
 template <typename T> __device__ __forceinline__ void store16(T* p, const float* v) {
   static_assert(sizeof(T) == 2, "16-bit types");
-  union { uint4 u[2]; T h[16]; } pk;
+  uint32_t w[8];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) pk.h[i] = from_f32<T>(v[i]);
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(pk.u[0].x), "r"(pk.u[0].y), "r"(pk.u[0].z),
-               "r"(pk.u[0].w), "r"(pk.u[1].x), "r"(pk.u[1].y), "r"(pk.u[1].z), "r"(pk.u[1].w)
+  for (int i = 0; i < 8; ++i) w[i] = pack2<T>(v[2 * i], v[2 * i + 1]);
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
 }
 
@@ -225,7 +256,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   constexpr int KIND = ElemTraits<TIN>::kind == KIND_TF32 ? KIND_TF32 : KIND_F16;
 
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * kStageA;
   uint64_t* full = reinterpret_cast<uint64_t*>(sB + STAGES * STAGE_B);
@@ -342,26 +373,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     const int row = quarter * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    // The backward gate epilogues read a gradient tile from global memory.  Gate-in backward fetches it a whole tile
-    // ahead (the loads of tile t+1 are issued before tile t's arithmetic): its warps are too few to hide a load
-    // issued just before its use.
+    // The backward gate epilogues read a gradient tile from global memory, just before they wait for the product.
     constexpr bool kGradTile = EPI == EPI_GATE_IN_BWD || EPI == EPI_GATE_OUT_BWD;
     auto fetch_grad = [&](int t, Raw8<TIN> (&dst)[CPG][4]) {
       int tm, tn, bz;
       decode(t, tm, tn, bz);
       if constexpr (EPI == EPI_GATE_IN_BWD) {
         const TIN* dplane = reinterpret_cast<const TIN*>(tm == 0 ? g.aux2 : g.aux3);
-        const long long t0 = (long long)tn * 128, tb0 = t0 / g.plane, tp0 = t0 - tb0 * g.plane;   // one division per tile
+        const uint32_t t0 = (uint32_t)tn * 128, plane = (uint32_t)g.plane, tb0 = t0 / plane, tp0 = t0 - tb0 * plane;
+        const TIN* base = dplane + ((long long)tb0 * 128 + row) * g.plane + tp0;
         const bool wide = sizeof(TIN) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0;   // 16-pixel groups: aligned, never split
 #pragma unroll
         for (int jj = 0; jj < CPG; ++jj)
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int off = (grp * CPG + jj) * 32 + u * 8;
-            if (t0 + off < g.N) {
-              long long bb = tb0, pix = tp0 + off;
-              while (pix >= g.plane) { pix -= g.plane; ++bb; }
-              const TIN* src = dplane + (bb * 128 + row) * g.plane + pix;
+            if (t0 + off < (uint32_t)g.N) {
+              const TIN* src = base + off;
+              for (uint32_t pix = tp0 + off; pix >= plane; pix -= plane) src += 127 * g.plane;   // the next batch entry's plane of this channel
               if constexpr (sizeof(TIN) == 2) {
                 if (wide) { if ((u & 1) == 0) ldraw16<TIN>(src, dst[jj][u], dst[jj][u + 1]); }
                 else dst[jj][u] = ldraw8<TIN>(src);
@@ -388,26 +417,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         }
       }
     };
-    // (gate-in backward: 8 epilogue warps with registers to spare; gate-out backward, on 16 warps and already at 70 %
-    // of HBM bandwidth, fetches its tile just before waiting for the product)
-    constexpr bool kAhead = EPI == EPI_GATE_IN_BWD && sizeof(TIN) == 2;   // (fp32 tiles would not fit the registers twice)
-    Raw8<TIN> dnext[kAhead ? CPG : 1][4];
-    if constexpr (kAhead) {
-      if ((int)blockIdx.x < total) fetch_grad(blockIdx.x, dnext);
-    }
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
       int tm, tn, bz;
       decode(tile, tm, tn, bz);
       Raw8<TIN> dpre[CPG][4];
-      if constexpr (kAhead) {
-#pragma unroll
-        for (int jj = 0; jj < CPG; ++jj)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) dpre[jj][u] = dnext[jj][u];
-        if (tile + (int)gridDim.x < total) fetch_grad(tile + gridDim.x, dnext);
-      } else if constexpr (kGradTile) {
-        fetch_grad(tile, dpre);
-      }
+      if constexpr (kGradTile) fetch_grad(tile, dpre);
       if (!mbar_wait(&tfull[acc], acc_phase, g.err, 4)) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
@@ -430,74 +444,72 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         }
       } else if constexpr (EPI == EPI_GATE_IN || EPI == EPI_GATE_IN_BWD) {
         // row = channel of half tm; columns: P for pixels n0..n0+127, then G for the same pixels
-        const long long n0 = (long long)tn * 128;
-        const long long nb0 = n0 / g.plane, np0 = n0 - nb0 * g.plane;   // one division per tile
+        const uint32_t n0 = (uint32_t)tn * 128, plane = (uint32_t)g.plane, np0 = n0 % plane;
         const bool wide16 = sizeof(TOUT) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0 && (g.ld_out & 15) == 0;
         const TIN* mask = reinterpret_cast<const TIN*>(g.aux);
         float bp = 0.f, bg = 0.f;
         if (g.bias0 != nullptr) { bp = g.bias0[tm * 256 + row]; bg = g.bias0[tm * 256 + 128 + row]; }
+        const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+        // gate-in: this channel's plane at the tile's first pixel; backward: the dP row (dG lies 128 rows on)
+        TOUT* dst0;
+        if constexpr (EPI == EPI_GATE_IN) dst0 = gate_in_dst<TOUT>(g, tm, n0 / plane, row, np0);
+        else dst0 = reinterpret_cast<TOUT*>(g.out0) + (long long)(tm * 256 + row) * g.ld_out + n0;
 #pragma unroll
         for (int jj = 0; jj < CPG; ++jj) {
           const int j = grp * CPG + jj;
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {   // 16 pixels at a time keeps the registers of 576 threads within budget
+            const uint32_t off = j * 32 + hf * 16;
             float p[16], gt[16];
-            ld16x2_f(t_row + j * 32 + hf * 16, t_row + 128 + j * 32 + hf * 16, p, gt);
-            float o0[16], o1[16];   // GATE_IN: gated value; GATE_IN_BWD: dP and dG
-            long long bb16 = 0, pix16 = 0;
+            ld16x2_f(t_row + off, t_row + 128 + off, p, gt);
+            Raw8<TOUT> o0[2], o1[2];   // GATE_IN: gated value; GATE_IN_BWD: dP and dG
 #pragma unroll
             for (int uu = 0; uu < 2; ++uu) {
-              const int u = hf * 2 + uu;
-              const long long m8 = n0 + j * 32 + u * 8;   // 8 pixels: same batch entry, all valid or none
-              if (m8 >= g.N) continue;
-              long long bb = nb0, pix = np0 + j * 32 + u * 8;
-              while (pix >= g.plane) { pix -= g.plane; ++bb; }
-              if (uu == 0) { bb16 = bb; pix16 = pix; }
-              float mk[8];
-              if (mask != nullptr) load8<TIN>(mask + m8, mk);
-              const float2 bp2 = make_float2(bp, bp), bg2 = make_float2(bg, bg);
-              if constexpr (EPI == EPI_GATE_IN) {
+              const uint32_t m8 = n0 + off + uu * 8;   // 8 pixels: same batch entry, all valid or none
+              if (m8 >= (uint32_t)g.N) continue;
+              float2 mk[4];
+              if (mask != nullptr) cvtraw8p<TIN>(ldraw8<TIN>(mask + m8), mk);
+              float2 d[4];
+              if constexpr (EPI == EPI_GATE_IN_BWD) cvtraw8p<TIN>(dpre[jj][hf * 2 + uu], d);
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                  const float2 pv = __fadd2_rn(make_float2(p[uu * 8 + i], p[uu * 8 + i + 1]), bp2);
-                  const float2 sg = sigmoid2(__fadd2_rn(make_float2(gt[uu * 8 + i], gt[uu * 8 + i + 1]), bg2));
+              for (int i = 0; i < 4; ++i) {
+                const int e = uu * 8 + 2 * i;
+                const float2 pv = __fadd2_rn(make_float2(p[e], p[e + 1]), bp2);
+                const float2 sg = sigmoid2(make_float2(gt[e], gt[e + 1]), nbg2);
+                if constexpr (EPI == EPI_GATE_IN) {
                   float2 r = __fmul2_rn(pv, sg);
-                  if (mask != nullptr) r = __fmul2_rn(r, make_float2(mk[i], mk[i + 1]));
-                  o0[uu * 8 + i] = r.x;
-                  o0[uu * 8 + i + 1] = r.y;
-                }
-                if (!wide16) store8<TOUT>(gate_in_dst<TOUT>(g, tm, bb, row, pix), &o0[uu * 8]);
-              } else {
-                float d[8];
-                cvtraw8<TIN>(dpre[jj][u], d);
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                  float2 dd = make_float2(d[i], d[i + 1]);
-                  if (mask != nullptr) dd = __fmul2_rn(dd, make_float2(mk[i], mk[i + 1]));
-                  const float2 sg = sigmoid2(__fadd2_rn(make_float2(gt[uu * 8 + i], gt[uu * 8 + i + 1]), bg2));
-                  const float2 pv = __fadd2_rn(make_float2(p[uu * 8 + i], p[uu * 8 + i + 1]), bp2);
+                  if (mask != nullptr) r = __fmul2_rn(r, mk[i]);
+                  putraw8(o0[uu], i, r);
+                } else {
+                  float2 dd = d[i];
+                  if (mask != nullptr) dd = __fmul2_rn(dd, mk[i]);
                   const float2 dp = __fmul2_rn(dd, sg);                                           // d * sig
                   const float2 oms = __ffma2_rn(sg, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
                   const float2 dg = __fmul2_rn(__fmul2_rn(dp, pv), oms);                          // d * P * sig * (1 - sig)
-                  o0[uu * 8 + i] = dp.x; o0[uu * 8 + i + 1] = dp.y;
-                  o1[uu * 8 + i] = dg.x; o1[uu * 8 + i + 1] = dg.y;
+                  putraw8(o0[uu], i, dp);
+                  putraw8(o1[uu], i, dg);
                 }
-                if (!wide16) {
-                  TOUT* o = reinterpret_cast<TOUT*>(g.out0);
-                  store8<TOUT>(o + (long long)(tm * 256 + row) * g.ld_out + m8, &o0[uu * 8]);
-                  store8<TOUT>(o + (long long)(tm * 256 + 128 + row) * g.ld_out + m8, &o1[uu * 8]);
+              }
+              if (!wide16) {
+                TOUT* dst = dst0 + off + uu * 8;
+                if constexpr (EPI == EPI_GATE_IN) {
+                  if (np0 + off + uu * 8 >= plane) dst = gate_in_dst<TOUT>(g, tm, m8 / plane, row, m8 % plane);
+                  straw8<TOUT>(dst, o0[uu]);
+                } else {
+                  straw8<TOUT>(dst, o0[uu]);
+                  straw8<TOUT>(dst + 128 * g.ld_out, o1[uu]);
                 }
               }
             }
             if constexpr (sizeof(TOUT) == 2) {
-              const long long m16 = n0 + j * 32 + hf * 16;
-              if (wide16 && m16 < g.N) {   // one 32-byte store per output row
+              if (wide16 && n0 + off < (uint32_t)g.N) {   // one 32-byte store per output row
+                TOUT* dst = dst0 + off;
                 if constexpr (EPI == EPI_GATE_IN) {
-                  store16<TOUT>(gate_in_dst<TOUT>(g, tm, bb16, row, pix16), o0);
+                  if (np0 + off >= plane) dst = gate_in_dst<TOUT>(g, tm, (n0 + off) / plane, row, (n0 + off) % plane);
+                  straw16<TOUT>(dst, o0[0], o0[1]);
                 } else {
-                  TOUT* o = reinterpret_cast<TOUT*>(g.out0);
-                  store16<TOUT>(o + (long long)(tm * 256 + row) * g.ld_out + m16, o0);
-                  store16<TOUT>(o + (long long)(tm * 256 + 128 + row) * g.ld_out + m16, o1);
+                  straw16<TOUT>(dst, o0[0], o0[1]);
+                  straw16<TOUT>(dst + 128 * g.ld_out, o1[0], o1[1]);
                 }
               }
             }
@@ -519,20 +531,26 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               float r0[16], r1[16];
 #pragma unroll
               for (int uu = 0; uu < 2; ++uu) {
-                const int u = hf * 2 + uu;
-                float d[8];
-                if constexpr (EPI == EPI_GATE_OUT_BWD) cvtraw8<TIN>(dpre[jj][u], d);
+                float2 d[4];
+                if constexpr (EPI == EPI_GATE_OUT_BWD) cvtraw8p<TIN>(dpre[jj][hf * 2 + uu], d);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const int c = j * 32 + u * 8 + i;
-                  float yv = y[uu * 8 + i], gv = gt[uu * 8 + i];
-                  if (g.bias0 != nullptr) { yv += g.bias0[c]; gv += g.bias0[128 + c]; }
-                  const float sg = fast_sigmoid(gv);
+                for (int i = 0; i < 4; ++i) {
+                  const int e = uu * 8 + 2 * i, c = j * 32 + hf * 16 + e;
+                  float2 yv = make_float2(y[e], y[e + 1]), gv = make_float2(gt[e], gt[e + 1]);
+                  if (g.bias0 != nullptr) {
+                    yv = __fadd2_rn(yv, *reinterpret_cast<const float2*>(g.bias0 + c));
+                    gv = __fadd2_rn(gv, *reinterpret_cast<const float2*>(g.bias0 + 128 + c));
+                  }
+                  const float2 sg = sigmoid2(gv);
                   if constexpr (EPI == EPI_GATE_OUT) {
-                    r0[uu * 8 + i] = yv * sg;
+                    const float2 r = __fmul2_rn(yv, sg);
+                    r0[e] = r.x; r0[e + 1] = r.y;
                   } else {
-                    r0[uu * 8 + i] = d[i] * sg;
-                    r1[uu * 8 + i] = d[i] * yv * sg * (1.0f - sg);
+                    const float2 dy = __fmul2_rn(d[i], sg);
+                    const float2 oms = __ffma2_rn(sg, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
+                    const float2 dg = __fmul2_rn(__fmul2_rn(dy, yv), oms);
+                    r0[e] = dy.x; r0[e + 1] = dy.y;
+                    r1[e] = dg.x; r1[e + 1] = dg.y;
                   }
                 }
               }

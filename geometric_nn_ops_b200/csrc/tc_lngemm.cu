@@ -13,10 +13,11 @@
 //   warps 6-21   gate epilogue, thread = channel holding consecutive pixels (the order of the channel-major a / b)
 //
 // Against the two-kernel form (LayerNorm kernel, then the gate GEMM reading z once per half) x is read once, z is
-// written from shared memory and never read back here, and the weights stay in shared memory.  The gate epilogue is
-// bound by instruction issue, and the LayerNorm role's instructions compete with it for the same schedulers, so the
-// kernel is slower than the gate GEMM alone (0.21 against 0.165 ms per launch at 768 x 768 pixels) but faster than
-// the pair (0.24).
+// written from shared memory and never read back here, and the weights stay in shared memory.  a and b leave through
+// shared memory too, by TMA in whole 128-byte lines; the epilogue threads' own stores carried 32 bytes per request, a
+// channel's rows lying a plane apart.  Per launch at 768 x 768 pixels: 0.24 ms for the pair of kernels, 0.197 for this one
+// at first, 0.164 with a reciprocal instead of a quotient in the sigmoid, pairwise conversions and the mask read once per
+// tile, and 0.148 with the staged stores; floor by bytes 0.092.
 // Every mbarrier wait is bounded; a timeout lands in *err and all roles drain.
 #include "tc_lngemm.cuh"
 
@@ -32,6 +33,7 @@ constexpr int kSub = 16384;                 // one [128 rows x 128 bytes] swizzl
 constexpr uint32_t kWBytes = 8 * kSub;      // (Pa, Ga, Pb, Gb) x (k 0..63, k 64..127)
 constexpr uint32_t kXBytes = 2 * kSub;      // one pixel tile: two 64-channel halves
 constexpr int kXBufs = 2;                 // (a third buffer, which still fits, changed nothing)
+constexpr int kMaskRing = 4;              // tile i + 4 lands only after the products of tile i + 2, hence after the epilogue of tile i
 
 struct Args {
   long long M, plane;
@@ -45,34 +47,32 @@ struct Args {
   void* b_cm;
   float* mean;
   float* rstd;
+  int staged;           // a / b leave through shared memory by TMA (planes of whole 64-pixel chunks)
   int* err;
 };
 
-template <typename T> __device__ __forceinline__ void unpack8(const uint4& w, float (&v)[8]) {
-  union { uint4 u; T h[8]; } pk;
-  pk.u = w;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = to_f32(pk.h[i]);
+template <typename T> __device__ __forceinline__ void unpack8p(const uint4& w, float2 (&v)[4]) {
+  v[0] = unpack2<T>(w.x); v[1] = unpack2<T>(w.y); v[2] = unpack2<T>(w.z); v[3] = unpack2<T>(w.w);
 }
-template <typename T> __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
-  union { uint4 u; T h[8]; } pk;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) pk.h[i] = from_f32<T>(v[i]);
-  return pk.u;
+template <typename T> __device__ __forceinline__ uint4 pack8p(const float2 (&v)[4]) {
+  return make_uint4(pack2<T>(v[0].x, v[0].y), pack2<T>(v[1].x, v[1].y), pack2<T>(v[2].x, v[2].y), pack2<T>(v[3].x, v[3].y));
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                  const __grid_constant__ CUtensorMap tmZ, const Args g) {
+                  const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmA,
+                  const __grid_constant__ CUtensorMap tmB, const Args g) {
   constexpr int KIND = ElemTraits<T>::kind;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
   uint8_t* sX = smem + kWBytes;
-  float* s_gamma = reinterpret_cast<float*>(sX + kXBufs * kXBytes);
-  float* s_beta = s_gamma + 128;
-  uint64_t* wfull = reinterpret_cast<uint64_t*>(s_beta + 128);
+  uint8_t* sO = sX + kXBufs * kXBytes;     // two chunks of [128 channels x 64 pixels] of a or b
+  T* s_gamma = reinterpret_cast<T*>(sO + kXBytes);
+  T* s_beta = s_gamma + 128;
+  T* s_mask = s_beta + 128;               // [kMaskRing][128] pixel mask of a tile
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(s_mask + kMaskRing * 128);
   uint64_t* xfull = wfull + 1;            // [kXBufs] tile landed (TMA bytes)
   uint64_t* xnorm = xfull + kXBufs;       // [kXBufs] tile normalised (one arrival per LayerNorm warp)
   uint64_t* xempty = xnorm + kXBufs;      // [kXBufs] tile consumed: the products (commit) and the z store (its reads) are done
@@ -91,8 +91,8 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tma_prefetch_desc(&tmZ);
   }
   if (threadIdx.x < 128) {
-    s_gamma[threadIdx.x] = g.gamma ? to_f32(reinterpret_cast<const T*>(g.gamma)[threadIdx.x]) : 1.f;
-    s_beta[threadIdx.x] = g.beta ? to_f32(reinterpret_cast<const T*>(g.beta)[threadIdx.x]) : 0.f;
+    s_gamma[threadIdx.x] = g.gamma ? reinterpret_cast<const T*>(g.gamma)[threadIdx.x] : from_f32<T>(1.f);
+    s_beta[threadIdx.x] = g.beta ? reinterpret_cast<const T*>(g.beta)[threadIdx.x] : from_f32<T>(0.f);
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
@@ -151,6 +151,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // ------------------------------------------------------------------ LayerNorm: thread = pixel row of the tile
     const int r0 = threadIdx.x - 64;
     const uint32_t sw = (uint32_t)(r0 & 7) << 4;
+    const T* mask = reinterpret_cast<const T*>(g.mask);
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const int b = i % kXBufs;
@@ -162,18 +163,13 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       // of the 128 samples, so (mean - K)^2 <= 128 var and the subtraction below loses at most seven bits of fp32.
       // Packed fp32x2 arithmetic and two accumulators each: the pass is a chain of dependent additions.
       float2 s0 = make_float2(0.f, 0.f), s1 = s0, q0 = s0, q1 = s0;
-      float2 nk;
-      {
-        float v[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(rowp + sw), v);
-        nk = make_float2(-v[0], -v[0]);
-      }
+      const float k0 = unpack2<T>(*reinterpret_cast<const uint32_t*>(rowp + sw)).x;
+      const float2 nk = make_float2(-k0, -k0);
 #pragma unroll 4
       for (int c = 0; c < 16; ++c) {
-        float v[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(rowp + (c >> 3) * kSub + (((c & 7) << 4) ^ sw)), v);
-        const float2 d0 = __fadd2_rn(make_float2(v[0], v[1]), nk), d1 = __fadd2_rn(make_float2(v[2], v[3]), nk);
-        const float2 d2 = __fadd2_rn(make_float2(v[4], v[5]), nk), d3 = __fadd2_rn(make_float2(v[6], v[7]), nk);
+        float2 v[4];
+        unpack8p<T>(*reinterpret_cast<const uint4*>(rowp + (c >> 3) * kSub + (((c & 7) << 4) ^ sw)), v);
+        const float2 d0 = __fadd2_rn(v[0], nk), d1 = __fadd2_rn(v[1], nk), d2 = __fadd2_rn(v[2], nk), d3 = __fadd2_rn(v[3], nk);
         s0 = __fadd2_rn(s0, d0); q0 = __ffma2_rn(d0, d0, q0);
         s1 = __fadd2_rn(s1, d1); q1 = __ffma2_rn(d1, d1, q1);
         s0 = __fadd2_rn(s0, d2); q0 = __ffma2_rn(d2, d2, q0);
@@ -188,19 +184,20 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 #pragma unroll 4
       for (int c = 0; c < 16; ++c) {
         uint4* p = reinterpret_cast<uint4*>(rowp + (c >> 3) * kSub + (((c & 7) << 4) ^ sw));
-        float v[8];
-        unpack8<T>(*p, v);
-        const float4 g0 = *reinterpret_cast<const float4*>(s_gamma + c * 8), g1 = *reinterpret_cast<const float4*>(s_gamma + c * 8 + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(s_beta + c * 8), b1 = *reinterpret_cast<const float4*>(s_beta + c * 8 + 4);
-        const float2 o0 = __ffma2_rn(__fadd2_rn(make_float2(v[0], v[1]), nmu), __fmul2_rn(rs2, make_float2(g0.x, g0.y)), make_float2(b0.x, b0.y));
-        const float2 o1 = __ffma2_rn(__fadd2_rn(make_float2(v[2], v[3]), nmu), __fmul2_rn(rs2, make_float2(g0.z, g0.w)), make_float2(b0.z, b0.w));
-        const float2 o2 = __ffma2_rn(__fadd2_rn(make_float2(v[4], v[5]), nmu), __fmul2_rn(rs2, make_float2(g1.x, g1.y)), make_float2(b1.x, b1.y));
-        const float2 o3 = __ffma2_rn(__fadd2_rn(make_float2(v[6], v[7]), nmu), __fmul2_rn(rs2, make_float2(g1.z, g1.w)), make_float2(b1.z, b1.w));
-        const float o[8] = {o0.x, o0.y, o1.x, o1.y, o2.x, o2.y, o3.x, o3.y};
-        *p = pack8<T>(o);
+        float2 v[4];
+        unpack8p<T>(*p, v);
+        float2 gm[4], bt[4], o[4];
+        unpack8p<T>(*reinterpret_cast<const uint4*>(s_gamma + c * 8), gm);
+        unpack8p<T>(*reinterpret_cast<const uint4*>(s_beta + c * 8), bt);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = __ffma2_rn(__fadd2_rn(v[e], nmu), __fmul2_rn(rs2, gm[e]), bt[e]);
+        *p = pack8p<T>(o);
       }
       const long long m = (long long)tile * 128 + r;
-      if (m < g.M) { g.mean[m] = mu; g.rstd[m] = rs; }
+      if (m < g.M) {
+        g.mean[m] = mu; g.rstd[m] = rs;
+        if (mask != nullptr) s_mask[(i % kMaskRing) * 128 + r] = mask[m];
+      }
       fence_proxy_async_smem();   // the tile is read next by tcgen05.mma and by the TMA store
       __syncwarp();
       if (lane == 0) mbar_arrive(&xnorm[b]);
@@ -221,55 +218,70 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
     const int quarter = warp & 3, j = (warp - 6) >> 2;   // TMEM lane quarter; 32-pixel chunk of the tile
     const int row = quarter * 32 + lane;
-    const bool wide16 = (g.plane & 15) == 0 && (g.M & 15) == 0;
-    const T* mask = reinterpret_cast<const T*>(g.mask);
+    const bool masked = g.mask != nullptr, staged = g.staged != 0;
+    const uint32_t plane = (uint32_t)g.plane, M = (uint32_t)g.M;
+    // staging: the 64-pixel chunk of warps j, j ^ 1 and its issuing thread
+    uint8_t* orow = sO + (j >> 1) * kSub + row * 128;
+    const bool issuer = (j & 1) == 0 && quarter == 0 && lane == 0;
     int i = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
-      const long long n0 = (long long)tile * 128;
-      const long long nb0 = n0 / g.plane, np0 = n0 - nb0 * g.plane;   // one division per tile
+    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
+      const uint32_t n0 = (uint32_t)tile * 128, nb0 = n0 / plane, np0 = n0 - nb0 * plane;   // one division per tile
+      const uint4* mrow = reinterpret_cast<const uint4*>(s_mask + (i % kMaskRing) * 128 + j * 32);
       for (int half = 0; half < 2; ++half) {
-        const bool done = mbar_wait(&tfull[half], i & 1, g.err, 16);
-        if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
+        ok = mbar_wait(&tfull[half], i & 1, g.err, 16) && ok;
         tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 256;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 256 + j * 32;
         float bp = 0.f, bg = 0.f;
         if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
-        const float2 bp2 = make_float2(bp, bp), bg2 = make_float2(bg, bg);
-        T* dplane = reinterpret_cast<T*>(half == 0 ? g.a_cm : g.b_cm);
+        const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+        Raw8<T> o[4];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-          float p[16], gt[16], o[16];
-          ld16x2_f(t_row + j * 32 + hf * 16, t_row + 128 + j * 32 + hf * 16, p, gt);
-          long long bb16 = 0, pix16 = 0;
+          float p[16], gt[16];
+          ld16x2_f(t_row + hf * 16, t_row + 128 + hf * 16, p, gt);
+          if (hf == 1) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[half]);
+          }
 #pragma unroll
           for (int uu = 0; uu < 2; ++uu) {
-            const int off = j * 32 + hf * 16 + uu * 8;
-            const long long m8 = n0 + off;   // 8 pixels: same batch entry, all valid or none
-            if (m8 >= g.M) continue;
-            long long bb = nb0, pix = np0 + off;
-            while (pix >= g.plane) { pix -= g.plane; ++bb; }
-            if (uu == 0) { bb16 = bb; pix16 = pix; }
-            float mk[8];
-            if (mask != nullptr) load8<T>(mask + m8, mk);
+            float2 mk[4];
+            if (masked) unpack8p<T>(mrow[hf * 2 + uu], mk);
 #pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-              const float2 pv = __fadd2_rn(make_float2(p[uu * 8 + e], p[uu * 8 + e + 1]), bp2);
-              const float2 sg = sigmoid2(__fadd2_rn(make_float2(gt[uu * 8 + e], gt[uu * 8 + e + 1]), bg2));
-              float2 rr = __fmul2_rn(pv, sg);
-              if (mask != nullptr) rr = __fmul2_rn(rr, make_float2(mk[e], mk[e + 1]));
-              o[uu * 8 + e] = rr.x;
-              o[uu * 8 + e + 1] = rr.y;
+            for (int k = 0; k < 4; ++k) {
+              const int e = uu * 8 + 2 * k;
+              float2 r = __fmul2_rn(__fadd2_rn(make_float2(p[e], p[e + 1]), bp2), sigmoid2(make_float2(gt[e], gt[e + 1]), nbg2));
+              if (masked) r = __fmul2_rn(r, mk[k]);
+              putraw8(o[hf * 2 + uu], k, r);
             }
-            if (!wide16) store8<T>(dplane + (bb * 128 + row) * g.plane + pix, &o[uu * 8]);
           }
-          if (wide16 && n0 + j * 32 + hf * 16 < g.M) store16<T>(dplane + (bb16 * 128 + row) * g.plane + pix16, o);
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[half]);
+        if (staged) {
+          if (issuer) bulk_wait_group_read0();   // the previous half's store has left the chunk
+          named_barrier(1 + (j >> 1), 256);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(orow + ((((j & 1) * 4 + u) ^ (row & 7)) << 4)) = o[u].w[0];
+          fence_proxy_async_smem();
+          named_barrier(3 + (j >> 1), 256);
+          const uint32_t px = n0 + (j >> 1) * 64;
+          if (issuer && px < M && ok) {          // a chunk of 64 pixels never straddles two batch entries here
+            tma_store_3d(half == 0 ? &tmA : &tmB, sO + (j >> 1) * kSub, px % plane, 0, px / plane);
+            bulk_commit_group();
+          }
+        } else if (ok) {
+          T* base = reinterpret_cast<T*>(half == 0 ? g.a_cm : g.b_cm) + ((long long)nb0 * 128 + row) * g.plane + np0 + j * 32;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {          // 8 pixels: same batch entry, all valid or none
+            T* d8 = base + u * 8;
+            for (uint32_t pix = np0 + j * 32 + u * 8; pix >= plane; pix -= plane) d8 += 127 * g.plane;   // the next batch entry's plane of this channel
+            if (n0 + j * 32 + u * 8 < M) straw8<T>(d8, o[u]);
+          }
+        }
       }
     }
+    if (issuer) bulk_wait_group0();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -282,7 +294,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 template <typename T>
 int launch(cudaStream_t st, const LnGateIn& p) {
   const uint64_t M = (uint64_t)p.M;
-  CUtensorMap tmX, tmW, tmZ;
+  CUtensorMap tmX, tmW, tmZ, tmA, tmB;
   const uint64_t xd[3] = {128, M, 1}, xs[2] = {128, 128 * M};
   const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
   const uint32_t box[3] = {64, 128, 1};
@@ -291,16 +303,23 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   TRI_TRY(make_tmap_3d(&tmW, p.wcat, 2, f16, wd, wsd, box, false));
   TRI_TRY(make_tmap_3d(&tmZ, p.z, 2, f16, xd, xs, box, false));
   Args a;
+  a.staged = p.plane % 64 == 0;
+  tmA = tmB = tmX;
+  if (a.staged) {
+    const uint64_t P = (uint64_t)p.plane, ad[3] = {P, 128, M / P}, as[2] = {P, 128 * P};
+    TRI_TRY(make_tmap_3d(&tmA, p.a_cm, 2, f16, ad, as, box, false));
+    TRI_TRY(make_tmap_3d(&tmB, p.b_cm, 2, f16, ad, as, box, false));
+  }
   a.M = p.M; a.plane = p.plane; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps;
   a.gamma = p.gamma; a.beta = p.beta; a.bias = p.bias_cat; a.mask = p.mask;
   a.a_cm = p.a_cm; a.b_cm = p.b_cm; a.mean = p.mean; a.rstd = p.rstd; a.err = p.err;
-  constexpr size_t smem = 1024 + kWBytes + kXBufs * kXBytes + 2 * 128 * sizeof(float) + (1 + 3 * kXBufs + 4) * 8 + 16;
+  constexpr size_t smem = 1024 + kWBytes + kXBufs * kXBytes + kXBytes + (2 + kMaskRing) * 128 * sizeof(T) + (1 + 3 * kXBufs + 4) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_in_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(a.tiles, sm_count());
   KernelTimer kt("tc_ln_gate_in", st, 2.0 * p.M * 128 * 512, 4.0 * p.M * 128 * 2);
-  kern<<<grid, kThreads, smem, st>>>(tmX, tmW, tmZ, a);
+  kern<<<grid, kThreads, smem, st>>>(tmX, tmW, tmZ, tmA, tmB, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -340,7 +359,7 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
                    const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmWg, const OutArgs g) {
   constexpr int KIND = ElemTraits<T>::kind;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
   uint8_t* sT = smem + kOWBytes;
   float* s_pm = reinterpret_cast<float*>(sT + kOBufs * kOTile);   // [8][128] partial means
@@ -452,22 +471,22 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       // partial statistics of 8 pixels over 16 channels, shifted by the first channel's values
       float2 nk[4], s[4], q[4];
       {
-        float v[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(part + (gg << 4)), v);
+        float2 v[4];
+        unpack8p<T>(*reinterpret_cast<const uint4*>(part + (gg << 4)), v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          nk[e] = make_float2(-v[2 * e], -v[2 * e + 1]);
+          nk[e] = make_float2(-v[e].x, -v[e].y);
           s[e] = make_float2(0.f, 0.f);
           q[e] = s[e];
         }
       }
 #pragma unroll 4
       for (int r = 0; r < 16; ++r) {
-        float v[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(part + r * 128 + ((gg ^ (r & 7)) << 4)), v);
+        float2 v[4];
+        unpack8p<T>(*reinterpret_cast<const uint4*>(part + r * 128 + ((gg ^ (r & 7)) << 4)), v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 d = __fadd2_rn(make_float2(v[2 * e], v[2 * e + 1]), nk[e]);
+          const float2 d = __fadd2_rn(v[e], nk[e]);
           s[e] = __fadd2_rn(s[e], d);
           q[e] = __ffma2_rn(d, d, q[e]);
         }
@@ -518,17 +537,13 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
 #pragma unroll 4
         for (int r = 0; r < 16; ++r) {
           uint4* p = reinterpret_cast<uint4*>(part + r * 128 + ((gg ^ (r & 7)) << 4));
-          float v[8], o[8];
-          unpack8<T>(*p, v);
+          float2 v[4], o[4];
+          unpack8p<T>(*p, v);
           const float gm = s_gamma[kp * 16 + r], bt = s_beta[kp * 16 + r];
           const float2 gm2 = make_float2(gm, gm), bt2 = make_float2(bt, bt);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 y = __ffma2_rn(__fadd2_rn(make_float2(v[2 * e], v[2 * e + 1]), nm[e]), __fmul2_rn(rr[e], gm2), bt2);
-            o[2 * e] = y.x;
-            o[2 * e + 1] = y.y;
-          }
-          const uint4 w = pack8<T>(o);
+          for (int e = 0; e < 4; ++e) o[e] = __ffma2_rn(__fadd2_rn(v[e], nm[e]), __fmul2_rn(rr[e], gm2), bt2);
+          const uint4 w = pack8p<T>(o);
           *p = w;
           if (udst != nullptr) *reinterpret_cast<uint4*>(udst + (long long)r * g.M) = w;
         }
@@ -557,11 +572,15 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
         if (m < g.M) {
           float o[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
+          for (int e = 0; e < 16; e += 2) {
             const int c = j * 32 + hf * 16 + e;
-            float yv = y[e], gv = gt[e];
-            if (g.bias != nullptr) { yv += g.bias[c]; gv += g.bias[128 + c]; }
-            o[e] = yv * fast_sigmoid(gv);
+            float2 yv = make_float2(y[e], y[e + 1]), gv = make_float2(gt[e], gt[e + 1]);
+            if (g.bias != nullptr) {
+              yv = __fadd2_rn(yv, *reinterpret_cast<const float2*>(g.bias + c));
+              gv = __fadd2_rn(gv, *reinterpret_cast<const float2*>(g.bias + 128 + c));
+            }
+            const float2 r = __fmul2_rn(yv, sigmoid2(gv));
+            o[e] = r.x; o[e + 1] = r.y;
           }
           store16<T>(orow + j * 32 + hf * 16, o);
         }
@@ -607,7 +626,237 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   return 0;
 }
 
+// =================================================================================================================
+// gate_in_bwd: dP = d sig(G) mask, dG = d P sig (1 - sig) mask for d = da, db, with P and G recomputed from z
+// =================================================================================================================
+// 576 threads: warp 0 TMA, warp 1 tcgen05.mma, warps 2-17 the gate epilogue (thread = channel of the half, 16 of the
+// tile's 64 pixels).  As in ln_gate_in the weights stay in shared memory and a z tile feeds the products of both halves,
+// so z is read once.  The gradient tile of a half ([128 channels x 64 pixels]) comes by TMA; the epilogue copies it to
+// registers at once, so that its buffer takes the next tile's during the arithmetic.  dP and dG leave through a staging
+// tile each and a TMA store: whole 128-byte lines.  Written by the threads, a request carried 32 bytes (a channel's rows
+// lie a plane apart), 4096 of them per 128 pixels, and the load / store pipe held the kernel at 0.29 ms for 768 x 768
+// pixels; with the gradients read that way too (the batched GEMM's form) it took 0.365.  Now 0.22, floor by bytes 0.16.
+constexpr int kBwdThreads = 576;
+constexpr int kBwdMaskRing = 4;           // as kMaskRing
+constexpr int kBSub = 8192;               // [64 rows x 128 bytes]
+constexpr uint32_t kBTile = 16384;        // z tile: two 64-channel halves; gradient or output tile of a half
+
+struct BwdArgs {
+  long long M;
+  int tiles;
+  const float* bias;
+  const void* mask;
+  uint32_t zero;        // 0
+  int* err;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmW,
+                   const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmO, const BwdArgs g) {
+  constexpr int KIND = ElemTraits<T>::kind;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  uint8_t* sW = smem;
+  uint8_t* sZ = smem + kWBytes;            // [2] z tiles
+  uint8_t* sG = sZ + 2 * kBTile;           // [half] gradient tile
+  uint8_t* sO = sG + 2 * kBTile;           // dP, dG of a half
+  uint8_t* sM = sO + 2 * kBTile;           // [kBwdMaskRing] x 64 mask values
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(sM + kBwdMaskRing * 128);
+  uint64_t* zfull = wfull + 1;             // [2]
+  uint64_t* zempty = zfull + 2;            // [2] both halves' products of the tile are done
+  uint64_t* gfull = zempty + 2;            // [half] gradient tile (half a: with the tile's mask)
+  uint64_t* gempty = gfull + 2;            // [half] ... copied to registers by all 16 epilogue warps
+  uint64_t* tfull = gempty + 2;            // [tile & 1][half] accumulator complete
+  uint64_t* tempty = tfull + 4;            // ... read by all 16 epilogue warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 4);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(wfull, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(&zfull[b], 1); mbar_init(&zempty[b], 1); mbar_init(&gfull[b], 1); mbar_init(&gempty[b], 16); }
+    for (int b = 0; b < 4; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 16); }
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      mbar_expect_tx(wfull, kWBytes);
+      for (int blk = 0; blk < 4; ++blk)
+        for (int kb = 0; kb < 2; ++kb) tma_load_3d(sW + (blk * 2 + kb) * kSub, &tmW, wfull, kb * 64, blk * 128, 0);
+      bool ok = true;
+      auto load_z = [&](int i, int tile) {
+        const int b = i & 1;
+        if (!mbar_wait(&zempty[b], ((i >> 1) & 1) ^ 1, g.err, 60)) { ok = false; return; }
+        mbar_expect_tx(&zfull[b], kBTile);
+        for (int kb = 0; kb < 2; ++kb) tma_load_3d(sZ + b * kBTile + kb * kBSub, &tmZ, &zfull[b], kb * 64, tile * 64, 0);
+      };
+      if ((int)blockIdx.x < g.tiles) load_z(0, blockIdx.x);
+      int i = 0;
+      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
+        if (tile + (int)gridDim.x < g.tiles) load_z(i + 1, tile + gridDim.x);   // one tile ahead
+        for (int half = 0; half < 2 && ok; ++half) {
+          if (!mbar_wait(&gempty[half], (i & 1) ^ 1, g.err, 61)) { ok = false; break; }
+          const bool with_mask = half == 0 && g.mask != nullptr;
+          mbar_expect_tx(&gfull[half], kBTile + (with_mask ? 128 : 0));
+          tma_load_3d(sG + half * kBTile, half == 0 ? &tmA : &tmB, &gfull[half], tile * 64, 0, 0);
+          if (with_mask) bulk_load(sM + (i % kBwdMaskRing) * 128, static_cast<const uint8_t*>(g.mask) + (long long)tile * 128, 128, &gfull[0]);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc(KIND, 128, 64, false, false);
+      const uint32_t w_base = smem_u32(sW), z_base = smem_u32(sZ);
+      bool ok = mbar_wait(wfull, 0, g.err, 62);
+      int i = 0;
+      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
+        const int b = i & 1;
+        if (!mbar_wait(&zfull[b], (i >> 1) & 1, g.err, 63)) break;
+        for (int half = 0; half < 2 && ok; ++half) {
+          const int acc = b * 2 + half;
+          if (!mbar_wait(&tempty[acc], ((i >> 1) & 1) ^ 1, g.err, 64)) { ok = false; break; }
+          tc_fence_after_sync();
+#pragma unroll
+          for (int pg = 0; pg < 2; ++pg) {   // P block, G block of this half
+            const uint32_t d_addr = tmem_base + acc * 128 + pg * 64;
+#pragma unroll
+            for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) {
+                const uint64_t ad = make_smem_desc(w_base + ((half * 2 + pg) * 2 + kb) * kSub + ks * 32, 16, 1024);
+                const uint64_t bd = make_smem_desc(z_base + b * kBTile + kb * kBSub + ks * 32, 16, 1024);
+                umma<KIND>(d_addr, ad, bd, idesc, (kb == 0 && ks == 0) ? 0u : 1u);
+              }
+          }
+          umma_commit(&tfull[acc]);
+        }
+        if (ok) umma_commit(&zempty[b]);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
+    const int quarter = warp & 3, j = (warp - 2) >> 2;   // TMEM lane quarter; 16-pixel part of the tile
+    const int row = quarter * 32 + lane;
+    const uint32_t at = row * 128, c0 = ((j * 2) ^ (row & 7)) << 4, c1 = ((j * 2 + 1) ^ (row & 7)) << 4;   // this thread's two pieces of a tile row
+    const bool masked = g.mask != nullptr;
+    int i = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
+      const uint4* mrow = reinterpret_cast<const uint4*>(sM + (i % kBwdMaskRing) * 128 + j * 32);
+      for (int half = 0; half < 2; ++half) {
+        const int acc = (i & 1) * 2 + half;
+        const uint8_t* gt_row = sG + half * kBTile + at;
+        ok = mbar_wait(&gfull[half], i & 1, g.err, 65) && ok;
+        const uint4 d[2] = {*reinterpret_cast<const uint4*>(gt_row + c0), *reinterpret_cast<const uint4*>(gt_row + c1)};
+        // The arrival must not pass the loads, which queue behind other accesses of this warp: its address takes in what
+        // they returned (and-ed with an argument that is zero), so the warp cannot issue it before they are complete.
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&gempty[half] + ((d[0].w | d[1].w) & g.zero));
+        ok = mbar_wait(&tfull[acc], (i >> 1) & 1, g.err, 66) && ok;
+        tc_fence_after_sync();
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * 16;
+        float bp = 0.f, bg = 0.f;
+        if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
+        const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+        float p[16], gt[16];
+        ld16x2_f(t_row, t_row + 64, p, gt);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[acc]);
+        Raw8<T> o0[2], o1[2];
+#pragma unroll
+        for (int uu = 0; uu < 2; ++uu) {
+          float2 dv[4], mk[4];
+          unpack8p<T>(d[uu], dv);
+          if (masked) {
+            unpack8p<T>(mrow[uu], mk);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dv[k] = __fmul2_rn(dv[k], mk[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int e = uu * 8 + 2 * k;
+            const float2 sg = sigmoid2(make_float2(gt[e], gt[e + 1]), nbg2);
+            const float2 dp = __fmul2_rn(dv[k], sg);
+            const float2 oms = __ffma2_rn(sg, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
+            putraw8(o0[uu], k, dp);
+            putraw8(o1[uu], k, __fmul2_rn(__fmul2_rn(dp, __fadd2_rn(make_float2(p[e], p[e + 1]), bp2)), oms));
+          }
+        }
+        if (threadIdx.x == 64) bulk_wait_group_read0();   // the previous half's stores have left the staging tiles
+        named_barrier(1, 512);
+        *reinterpret_cast<uint4*>(sO + at + c0) = o0[0].w[0];
+        *reinterpret_cast<uint4*>(sO + at + c1) = o0[1].w[0];
+        *reinterpret_cast<uint4*>(sO + kBTile + at + c0) = o1[0].w[0];
+        *reinterpret_cast<uint4*>(sO + kBTile + at + c1) = o1[1].w[0];
+        fence_proxy_async_smem();
+        named_barrier(2, 512);
+        if (threadIdx.x == 64 && ok) {
+          tma_store_3d(&tmO, sO, tile * 64, half * 256, 0);
+          tma_store_3d(&tmO, sO + kBTile, tile * 64, half * 256 + 128, 0);
+          bulk_commit_group();
+        }
+      }
+    }
+    if (threadIdx.x == 64) bulk_wait_group0();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <typename T>
+int launch_bwd(cudaStream_t st, const GateInBwd& p) {
+  const uint64_t M = (uint64_t)p.M;
+  CUtensorMap tmZ, tmW, tmA, tmB, tmO;
+  const bool f16 = p.dtype == TRI_F16;
+  const uint64_t zd[3] = {128, M, 1}, zs[2] = {128, 128 * M};
+  const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
+  const uint64_t gd[3] = {M, 128, 1}, od[3] = {M, 512, 1}, gs[2] = {M, 512 * M};
+  const uint32_t zbox[3] = {64, 64, 1}, box[3] = {64, 128, 1};
+  TRI_TRY(make_tmap_3d(&tmZ, p.z, 2, f16, zd, zs, zbox, false));
+  TRI_TRY(make_tmap_3d(&tmW, p.wcat, 2, f16, wd, wsd, box, false));
+  TRI_TRY(make_tmap_3d(&tmA, p.da_cm, 2, f16, gd, gs, box, false));
+  TRI_TRY(make_tmap_3d(&tmB, p.db_cm, 2, f16, gd, gs, box, false));
+  TRI_TRY(make_tmap_3d(&tmO, p.dpg, 2, f16, od, gs, box, false));
+  BwdArgs a;
+  a.M = p.M; a.tiles = (int)(p.M / 64); a.bias = p.bias_cat; a.mask = p.mask; a.zero = 0; a.err = p.err;
+  constexpr size_t smem = 1024 + kWBytes + 6 * kBTile + kBwdMaskRing * 128 + 17 * 8 + 16;
+  static_assert(smem <= 232448, "shared memory of one CTA");
+  auto kern = gate_in_bwd_kernel<T>;
+  TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = std::min(a.tiles, sm_count());
+  KernelTimer kt("tc_gate_in_bwd", st, 0.0, 7.0 * p.M * 128 * 2);
+  kern<<<grid, kBwdThreads, smem, st>>>(tmZ, tmW, tmA, tmB, tmO, a);
+  TRI_LAUNCH_OK();
+  return 0;
+}
+
 }  // namespace
+
+// one batch entry (its channel planes are M pixels apart), whole tiles (any square of a multiple of eight)
+bool gate_in_bwd_supported(int dtype, long long M, long long plane) {
+  return (dtype == TRI_BF16 || dtype == TRI_F16) && M > 0 && M == plane && M % 64 == 0 && M < (1LL << 31) - 128;
+}
+
+int gate_in_bwd(cudaStream_t st, const GateInBwd& p) {
+  if (!gate_in_bwd_supported(p.dtype, p.M, p.M)) return fail(TRI_ERR_ARG, "gate_in_bwd: unsupported shape or dtype");
+  return p.dtype == TRI_BF16 ? launch_bwd<__nv_bfloat16>(st, p) : launch_bwd<__half>(st, p);
+}
 
 bool ln_gate_in_supported(int dtype, long long M, long long plane) {
   return (dtype == TRI_BF16 || dtype == TRI_F16) && M > 0 && plane > 0 && plane % 8 == 0 && M % plane == 0 &&

@@ -6,6 +6,7 @@
 //   ln_gate_out  t (channel-major) -> u = LayerNorm over channels, normalised in shared memory in the layout the
 //                contraction left it in (the MMA reads it as an MN-major operand, so nothing is transposed), then
 //                out = (u Wo^T + bo) * sigmoid(z Wgo^T + bgo); u is kept channel-major for the backward pass.
+//   gate_in_bwd  z, da, db -> dP, dG of both halves (no LayerNorm: the same kernel shape with resident weights).
 #pragma once
 
 #include "tc_common.cuh"
@@ -55,6 +56,22 @@ struct LnGateOut {
 // One batch entry, 64-pixel groups aligned: M a multiple of 64.
 bool ln_gate_out_supported(int dtype, long long M, long long plane);
 int ln_gate_out(cudaStream_t st, const LnGateOut& p);
+
+// Input gate backward: dP, dG of both halves from the recomputed projections of z and the gradients of a and b.
+struct GateInBwd {
+  int dtype;                 // TRI_BF16 / TRI_F16
+  long long M;               // pixels (one batch entry)
+  const void* z;             // [M, 128]
+  const void* wcat;          // [512, 128]: rows [Wp_a; Wg_a; Wp_b; Wg_b]
+  const float* bias_cat;     // [512] or null
+  const void* mask;          // [M] or null
+  const void* da_cm;         // [128, M]
+  const void* db_cm;
+  void* dpg;                 // [512, M]: rows [dP_a; dG_a; dP_b; dG_b]
+  int* err;
+};
+bool gate_in_bwd_supported(int dtype, long long M, long long plane);
+int gate_in_bwd(cudaStream_t st, const GateInBwd& p);
 
 }  // namespace tc
 }  // namespace tri

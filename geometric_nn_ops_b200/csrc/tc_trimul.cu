@@ -68,8 +68,9 @@ template <typename T> __device__ __forceinline__ void store4(T* p, const float (
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void prep_weights_kernel(const T* wp, const T* wg, const T* bp, const T* bg, const T* bo, const T* bgo,
-                                    T* wcat, float* bias_cat, float* bias_out) {
+                                    T* wcat, float* bias_cat, float* bias_out, int* err) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx == 0) *err = 0;   // the error word of the launches that follow
   if (idx < 4 * CW * CW) {
     const int r = idx / CW, k = idx % CW, blk = r / CW, c = r % CW;
     const T* src = (blk & 1) ? wg : wp;
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float* partial, int n
   if (lane4 == 0 && j < n) out[j] = (sub[0][o] + sub[1][o]) + (sub[2][o] + sub[3][o]);
 }
 
-// Up to six such reductions in one launch (blockIdx.y selects the job): the backward has groups of small reductions
+// Up to six such reductions in one launch: the backward has groups of small reductions
 // (weight gradients, LayerNorm weight and bias) whose launches cost more than their work.  A job with `rowlen` set
 // sums partials of a [512, rowlen] tensor in Wcat row order and scatters its rows to the p_in (out) and g_in (out2)
 // gradients; either may be null.
@@ -552,39 +553,54 @@ struct ReduceJobs {
   const float* partial[kReduceJobs];
   float* out[kReduceJobs];
   float* out2[kReduceJobs];
-  int nparts[kReduceJobs], n[kReduceJobs], rowlen[kReduceJobs];
+  int nparts[kReduceJobs], n[kReduceJobs], rowlen[kReduceJobs], first[kReduceJobs];   // first: the job's first block
 };
-// 32 outputs per block (one warp reads 128 contiguous bytes of a partial), 8 warps each summing every eighth
-// partial with eight independent accumulators so that loads overlap (the first version walked 37 partials with one
-// dependent load each: 16 us per launch of pure latency); the warps' sums are added in a fixed order, so the
-// result does not depend on scheduling.
-__global__ void __launch_bounds__(256) reduce_multi_kernel(const ReduceJobs jobs) {
-  __shared__ float sub[8][32];
-  const int job = blockIdx.y, n = jobs.n[job], nparts = jobs.nparts[job];
-  if (blockIdx.x * 32 >= n) return;
-  const float* partial = jobs.partial[job];
+// 128 outputs per block (a warp reads 512 contiguous bytes of a partial), 16 warps each summing every 16th partial with
+// eight loads in flight; the warps' sums are added in a fixed order, so the result does not depend on scheduling.  Blocks
+// are numbered through the jobs (`first`): a grid sized for the largest job for each of them launched three times as many
+// blocks, most of them empty.  What bounds it is the longest chain of dependent load rounds, that of the LayerNorm sums'
+// 592 partials.  Two launches per step at any N: 40 us at first, 26 now.
+constexpr int kReduceThreads = 512;
+__global__ void __launch_bounds__(kReduceThreads) reduce_multi_kernel(const ReduceJobs jobs) {
+  constexpr int W = kReduceThreads / 32;
+  __shared__ float4 sub[W][32];
+  int job = 0;
+  while (job + 1 < kReduceJobs && (int)blockIdx.x >= jobs.first[job + 1]) ++job;
+  const int n = jobs.n[job], nparts = jobs.nparts[job];
   const int o = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int j = blockIdx.x * 32 + o;
-  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (j < n) {
-    int p = w;
-    for (; p + 56 < nparts; p += 64) {   // eight independent loads in flight
+  const int j = ((blockIdx.x - jobs.first[job]) * 32 + o) * 4;   // n is a multiple of 128
+  const float* partial = jobs.partial[job] + j;
+  float4 a[4];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) a[u] += partial[(long long)(p + 8 * u) * n + j];
-    }
-    for (; p < nparts; p += 8) a[0] += partial[(long long)p * n + j];
+  for (int u = 0; u < 4; ++u) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+  for (int p = w; p < nparts; p += 4 * W) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + W * u < nparts) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(partial + (long long)(p + W * u) * n));
+        a[u].x += v.x; a[u].y += v.y; a[u].z += v.z; a[u].w += v.w;
+      }
   }
-  sub[w][o] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+  auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
+  sub[w][o] = add(add(a[0], a[1]), add(a[2], a[3]));
   __syncthreads();
-  if (w != 0 || j >= n) return;
-  const float sum = ((sub[0][o] + sub[1][o]) + (sub[2][o] + sub[3][o])) + ((sub[4][o] + sub[5][o]) + (sub[6][o] + sub[7][o]));
+  if (w != 0) return;
+  float4 sum = sub[0][o];
+#pragma unroll
+  for (int u = 1; u < W; ++u) sum = add(sum, sub[u][o]);
   const int rowlen = jobs.rowlen[job];
-  if (rowlen == 0) {
-    jobs.out[job][j] = sum;
-  } else {
+  float* dst = jobs.out[job] + j;
+  if (rowlen != 0) {
     const int r = j / rowlen, k = j % rowlen, blk = r / CW, c = r % CW;
-    float* dst = (blk & 1) ? jobs.out2[job] : jobs.out[job];
-    if (dst != nullptr) dst[((blk >> 1) * CW + c) * rowlen + k] = sum;
+    float* half = (blk & 1) ? jobs.out2[job] : jobs.out[job];
+    if (half == nullptr) return;
+    dst = half + ((blk >> 1) * CW + c) * rowlen + k;
+  }
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    *reinterpret_cast<float4*>(dst) = sum;
+  } else {
+    dst[0] = sum.x; dst[1] = sum.y; dst[2] = sum.z; dst[3] = sum.w;
   }
 }
 
@@ -673,12 +689,14 @@ int contraction(cudaStream_t st, int dtype, int planes, int n, const void* a, bo
 
 template <typename T>
 int run_prep(cudaStream_t st, const TriMulWeights* w, const Prep& pr, bool weights_ready = false) {
-  TRI_CUDA_OK(cudaMemsetAsync(pr.err, 0, 256, st));
-  if (weights_ready) return 0;   // the caller kept the prepared weights of an earlier phase of the same call
+  if (weights_ready) {   // the caller kept the prepared weights of an earlier phase of the same call
+    TRI_CUDA_OK(cudaMemsetAsync(pr.err, 0, 256, st));
+    return 0;
+  }
   KernelTimer kt("tc_prep_weights", st, 0.0, 0.0);
   prep_weights_kernel<T><<<cdiv(4 * CW * CW, 256), 256, 0, st>>>(
       (const T*)w->p_in_w, (const T*)w->g_in_w, (const T*)w->p_in_b, (const T*)w->g_in_b, (const T*)w->p_out_b,
-      (const T*)w->g_out_b, (T*)pr.wcat, pr.bias_cat, pr.bias_out);
+      (const T*)w->g_out_b, (T*)pr.wcat, pr.bias_cat, pr.bias_out, pr.err);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -766,9 +784,12 @@ int split_k_grad(cudaStream_t st, const Geom& gm, const void* lhs, int lhs_w, co
   const long long M = gm.M;
   const int bke = gm.dtype == TRI_F32 ? 32 : 64;
   // One split per SM for the single-GPU op.  A row shard gets proportionally fewer (at least 2048 pixels per split,
-  // never under 37 splits), so that the partials written here and summed by the reduction shrink with the shard
+  // never under 37 splits; of 128 rows), so that the partials written here and summed by the reduction shrink with the shard
   // instead of staying sized for 148 SMs; the SMs this leaves idle run the other streams' kernels of the sharded step.
   int splits = gm.sharded ? (int)std::min<long long>(kSplitK, std::max<long long>(37, M / 2048)) : kSplitK;
+  // ... and one output tile per SM: a gradient of 512 rows has four tiles per split, and 148 splits of it only made four
+  // times the partials for the reduction (39 MB; the two reduction launches of a step took 40 us at any N, 34 after this alone).
+  splits = std::max(1, splits * CW / lhs_w);
   splits = (int)std::min<long long>(splits, (M + bke - 1) / bke);
   long long kper = ((M + splits - 1) / splits + bke - 1) / bke * bke;
   splits = (int)((M + kper - 1) / kper);
@@ -792,19 +813,21 @@ int split_k_grad(cudaStream_t st, const Geom& gm, const void* lhs, int lhs_w, co
 struct ReduceJob { const float* partial; int nparts, n; float* out; float* out2 = nullptr; int rowlen = 0; };
 int reduce_many(cudaStream_t st, std::initializer_list<ReduceJob> list) {
   ReduceJobs jobs = {};
-  int count = 0, nmax = 0;
+  int count = 0, blocks = 0;
   double bytes = 0.0;
   for (const ReduceJob& j : list) {
     if ((j.out == nullptr && j.out2 == nullptr) || j.nparts == 0) continue;
     jobs.partial[count] = j.partial; jobs.out[count] = j.out; jobs.out2[count] = j.out2;
     jobs.nparts[count] = j.nparts; jobs.n[count] = j.n; jobs.rowlen[count] = j.rowlen;
-    nmax = std::max(nmax, j.n);
+    jobs.first[count] = blocks;
+    blocks += j.n / 128;
     bytes += 4.0 * (j.nparts + 1) * j.n;
     ++count;
   }
   if (count == 0) return 0;
+  for (int i = count; i < kReduceJobs; ++i) jobs.first[i] = 1 << 30;
   KernelTimer kt("tc_reduce", st, 0.0, bytes);
-  reduce_multi_kernel<<<dim3(cdiv(nmax, 32), count), 256, 0, st>>>(jobs);
+  reduce_multi_kernel<<<blocks, kReduceThreads, 0, st>>>(jobs);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -913,7 +936,12 @@ int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void
                       void* dpg, void* dz, void* dx, float* partial) {
   const long long M = gm.M;
   int nparts = 0;
-  {
+  if (gate_in_bwd_supported(gm.dtype, M, gm.plane) && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) {
+    GateInBwd f;
+    f.dtype = gm.dtype; f.M = M; f.z = z; f.wcat = pr.wcat; f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr;
+    f.mask = mask; f.da_cm = da_cm; f.db_cm = db_cm; f.dpg = dpg; f.err = pr.err;
+    TRI_TRY(gate_in_bwd(st, f));
+  } else {
     GemmPlan p;   // input gate backward fused into the recomputed projection GEMM
     gate_in_operands(&p, gm, pr, z);
     p.out0 = dpg; p.ld_out = M; p.bias0 = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr;
