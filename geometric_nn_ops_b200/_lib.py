@@ -126,6 +126,24 @@ EXPORTS = {
 }
 
 _lib = None
+_host = None
+
+
+def host():
+    """The native host extension (csrc/torch_host.cpp), bound to the library that :func:`load` loaded."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as ext
+        except ImportError as exc:
+            raise RuntimeError(
+                "the host extension is not built for this interpreter: run `python -m geometric_nn_ops_b200.build` "
+                f"(there is no fallback implementation): {exc}"
+            ) from exc
+        ext.bind(LIB_PATH)
+        _host = ext
+    return _host
 
 
 def load():

@@ -1,0 +1,381 @@
+// The host side of the two ops: argument canonicalisation, allocation from torch's caching allocator, the C-ABI calls
+// and autograd, as one Python extension.
+//
+// The same steps in Python -- descriptor structs over ctypes, a Python autograd Function, a dozen small tensor calls --
+// took about 65 us per call, which is what a call on a small pair tensor costs in all (its kernels take 10).  Here a call
+// without gradients goes straight to the library, and the backward runs on autograd's thread without the interpreter.
+//
+// Semantics follow the reference's public wrappers (geometric_nn_ops_torch/triangle/_triattn.py:23-106, _trimul.py:39-88).
+// The library is reached through function pointers taken from the one that the ctypes binding loaded.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <algorithm>
+#include <array>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <optional>
+#include <vector>
+
+#include "../../include/tri_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+struct Api {
+  decltype(&tri_last_error) last_error;
+  decltype(&tri_last_path) last_path;
+  decltype(&tri_ws_status) ws_status;
+  decltype(&tri_attn_ws_bytes) attn_ws_bytes;
+  decltype(&tri_attn_fwd) attn_fwd;
+  decltype(&tri_attn_bwd) attn_bwd;
+  decltype(&tri_mul_saved_bytes) mul_saved_bytes;
+  decltype(&tri_mul_ws_bytes) mul_ws_bytes;
+  decltype(&tri_mul_fwd) mul_fwd;
+  decltype(&tri_mul_bwd) mul_bwd;
+} api;
+
+void bind(const std::string& path) {
+  void* lib = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(lib != nullptr, "cannot load ", path, ": ", dlerror());
+  auto get = [&](auto& fn, const char* name) {
+    fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(lib, name));
+    TORCH_CHECK(fn != nullptr, path, " has no ", name);
+  };
+  get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
+  get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
+  get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
+  get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
+}
+
+void ok(int code, const char* what) {
+  TORCH_CHECK(code == 0, what, " failed with code ", code, ": ", api.last_error());
+}
+// with TRI_B200_CHECK=1, read back the tensor-core kernels' status word (synchronises the stream)
+void check_device(const Tensor& ws, cudaStream_t st) {
+  const char* e = std::getenv("TRI_B200_CHECK");
+  if (e != nullptr && std::strcmp(e, "1") == 0 && std::strcmp(api.last_path(), "tcgen05") == 0)
+    ok(api.ws_status(ws.data_ptr(), reinterpret_cast<tri_stream_t>(st)), "device status");
+}
+
+int dtype_code(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return TRI_F32;
+    case at::kBFloat16: return TRI_BF16;
+    case at::kHalf: return TRI_F16;
+    default: TORCH_CHECK_TYPE(false, "unsupported dtype torch.", at::toString(t.scalar_type()));
+  }
+}
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+Tensor bytes(size_t n, const Tensor& like) {
+  return at::empty({(int64_t)std::max<size_t>(n, 1)}, like.options().dtype(at::kByte));
+}
+tri_stream_t stream_of(const Tensor& t) {
+  return reinterpret_cast<tri_stream_t>(c10::cuda::getCurrentCUDAStream(t.get_device()).stream());
+}
+
+// --------------------------------------------------------------------------------------------------- attention
+
+// a tensor whose last axis has stride 1 (copied only if it does not)
+Tensor inner_contiguous(const Tensor& t) { return t.stride(-1) == 1 || t.size(-1) == 1 ? t : t.contiguous(); }
+
+// an output with t's layout where t is a permutation of a dense block, else contiguous
+Tensor like(const Tensor& t) {
+  if (t.is_contiguous()) return at::empty(t.sizes(), t.options());
+  bool dense = t.stride(-1) == 1;
+  if (dense) {
+    std::vector<std::pair<int64_t, int64_t>> ax;   // (stride, size)
+    for (int64_t i = 0; i < t.dim(); ++i)
+      if (t.size(i) != 1) ax.emplace_back(t.stride(i), t.size(i));
+    std::sort(ax.begin(), ax.end());
+    int64_t expect = 1;
+    for (auto& a : ax) {
+      if (a.first != expect) { dense = false; break; }
+      expect *= a.second;
+    }
+  }
+  return dense ? at::empty_strided(t.sizes(), t.strides(), t.options()) : at::empty(t.sizes(), t.options());
+}
+
+void st4(int64_t (&dst)[4], const Tensor& t) {
+  for (int i = 0; i < 4; ++i) dst[i] = t.stride(i);
+}
+
+TriAttnDesc attn_desc(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& bias, const Tensor& mask,
+                      double scale, int64_t precision) {
+  TriAttnDesc d{};
+  d.B = q.size(0); d.n_seq = q.size(1); d.n_res = q.size(2); d.H = q.size(3); d.D = q.size(4);
+  d.dtype = dtype_code(q); d.precision = (int)precision; d.scale = (float)scale;
+  st4(d.q_st, q); st4(d.k_st, k); st4(d.v_st, v); st4(d.o_st, o);
+  if (bias.defined()) { d.bias_st[0] = bias.stride(0); d.bias_st[1] = bias.stride(2); d.bias_st[2] = bias.stride(3); }
+  if (mask.defined()) { d.mask_st[0] = mask.stride(0); d.mask_st[1] = mask.stride(1); }
+  return d;
+}
+
+struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, S, N]
+
+// q, k, v [B, S, N, H, D], bias [B, 1, H, N, N], mask [B, S, 1, 1, N]
+AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias_, const Tensor& mask_, double scale,
+                      int64_t precision) {
+  AttnCall c;
+  c.q = inner_contiguous(q_); c.k = inner_contiguous(k_); c.v = inner_contiguous(v_);
+  if (bias_.defined()) c.bias = inner_contiguous(bias_);
+  const int64_t B = c.q.size(0), S = c.q.size(1), N = c.q.size(2), H = c.q.size(3);
+  if (mask_.defined()) c.mask = mask_.reshape({B, S, N}).contiguous();
+  c.o = like(c.q);
+  c.stats = at::empty({2, B, S, H, N}, c.q.options().dtype(at::kFloat));
+  const TriAttnDesc d = attn_desc(c.q, c.k, c.v, c.o, c.bias, c.mask, scale, precision);
+  const c10::cuda::CUDAGuard guard(c.q.device());
+  const size_t n = api.attn_ws_bytes(&d, 0);
+  const Tensor ws = bytes(n, c.q);
+  const tri_stream_t st = stream_of(c.q);
+  ok(api.attn_fwd(&d, ptr(c.q), ptr(c.k), ptr(c.v), ptr(c.bias), static_cast<const uint8_t*>(ptr(c.mask)), ptr(c.o),
+                  static_cast<float*>(ptr(c.stats)), ptr(ws), n, st), "tri_attn_fwd");
+  check_device(ws, reinterpret_cast<cudaStream_t>(st));
+  return c;
+}
+
+// (an autograd Function takes an absent tensor as an empty optional; needs_input_grad counts the tensors that are there)
+OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
+Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+
+struct AttnFn : torch::autograd::Function<AttnFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& bias,
+                               const OptTensor& mask, double scale, int64_t precision) {
+    const AttnCall c = attn_forward(q, k, v, or_undefined(bias), or_undefined(mask), scale, precision);
+    ctx->save_for_backward({c.q, c.k, c.v, c.bias, c.mask, c.o, c.stats});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["precision"] = precision;
+    ctx->mark_non_differentiable({c.stats});
+    return {c.o, c.stats};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &q = s[0], &k = s[1], &v = s[2], &bias = s[3], &mask = s[4], &o = s[5], &stats = s[6];
+    const Tensor d_o = inner_contiguous(grads[0]);
+    const int64_t B = q.size(0), N = q.size(2), H = q.size(3);
+    Tensor dq = like(q), dk = like(k), dv = like(v), dbias;
+    if (bias.defined() && ctx->needs_input_grad(3)) dbias = at::empty({B, H, N, N}, q.options().dtype(at::kFloat));
+    TriAttnDesc d = attn_desc(q, k, v, o, bias, mask, ctx->saved_data["scale"].toDouble(), ctx->saved_data["precision"].toInt());
+    st4(d.do_st, d_o); st4(d.dq_st, dq); st4(d.dk_st, dk); st4(d.dv_st, dv);
+    const c10::cuda::CUDAGuard guard(q.device());
+    const size_t n = api.attn_ws_bytes(&d, 1);
+    const Tensor ws = bytes(n, q);
+    const tri_stream_t st = stream_of(q);
+    ok(api.attn_bwd(&d, ptr(q), ptr(k), ptr(v), ptr(bias), static_cast<const uint8_t*>(ptr(mask)), ptr(o),
+                    static_cast<const float*>(ptr(stats)), ptr(d_o), ptr(dq), ptr(dk), ptr(dv), static_cast<float*>(ptr(dbias)),
+                    ptr(ws), n, st), "tri_attn_bwd");
+    check_device(ws, reinterpret_cast<cudaStream_t>(st));
+    if (dbias.defined()) dbias = dbias.to(bias.scalar_type()).view({B, 1, H, N, N});
+    return {dq, dk, dv, dbias, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// leading axes folded (or added) to rank 5
+Tensor rank5(const Tensor& t) {
+  if (t.dim() == 5) return t;
+  std::vector<int64_t> s(t.sizes().begin(), t.sizes().end());
+  if (t.dim() < 5) {
+    s.insert(s.begin(), 5 - t.dim(), 1);
+    return t.reshape(s);
+  }
+  return t.reshape({-1, s[s.size() - 4], s[s.size() - 3], s[s.size() - 2], s[s.size() - 1]});
+}
+
+py::object attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& bias_, const OptTensor& mask_,
+                     std::optional<double> scale_, int64_t precision, bool return_aux) {
+  TORCH_CHECK(q_.is_cuda(), "triangle_attention needs CUDA tensors: there is no CPU implementation");
+  dtype_code(q_);
+  const bool canonical = q_.dim() == 5;
+  const Tensor q = rank5(q_);
+  Tensor k = rank5(k_), v = rank5(v_), bias, mask;
+  if (k.scalar_type() != q.scalar_type()) k = k.to(q.scalar_type());
+  if (v.scalar_type() != q.scalar_type()) v = v.to(q.scalar_type());
+  const int64_t B = q.size(0), S = q.size(1), N = q.size(2), H = q.size(3);
+  if (bias_.has_value()) {
+    bias = *bias_;
+    if (bias.dim() == 4) bias = bias.unsqueeze(-4);
+    else if (bias.dim() > 5) bias = rank5(bias);
+    bias = bias.expand({B, 1, H, N, N});
+    if (bias.scalar_type() != q.scalar_type()) bias = bias.to(q.scalar_type());
+  }
+  if (mask_.has_value()) {
+    mask = *mask_;
+    if (mask.dim() > 5) mask = rank5(mask);
+    mask = mask.expand({B, S, 1, 1, N});
+  }
+  const double scale = scale_.has_value() ? *scale_ : 1.0 / std::sqrt((double)q.size(4));
+  Tensor o, stats;
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()))) {
+    const variable_list r = AttnFn::apply(q, k, v, opt(bias), opt(mask), scale, precision);
+    o = r[0]; stats = r[1];
+  } else {
+    const AttnCall c = attn_forward(q, k, v, bias, mask, scale, precision);
+    o = c.o; stats = c.stats;
+  }
+  if (!canonical) o = o.reshape(q_.sizes());
+  if (!return_aux) return py::cast(o);
+  const Tensor m = stats.select(0, 0);
+  return py::make_tuple(o, (m + stats.select(0, 1)).unsqueeze(-1), m.unsqueeze(-1));
+}
+
+// ------------------------------------------------------------------------------------- multiplicative update
+
+constexpr int kWeights = 12;   // in the order of TriMulWeights
+using Weights = std::array<Tensor, kWeights>;
+static_assert(sizeof(TriMulWeights) == kWeights * sizeof(void*) && sizeof(TriMulWeightGrads) == kWeights * sizeof(void*));
+const char* const kNames[kWeights] = {"norm_in_weight", "norm_in_bias", "p_in_weight", "p_in_bias", "g_in_weight", "g_in_bias",
+                                      "norm_out_weight", "norm_out_bias", "p_out_weight", "p_out_bias", "g_out_weight", "g_out_bias"};
+
+// contiguous and 16-byte aligned (TMA and the vector loads need it); copied only if it must be
+Tensor aligned(const Tensor& t_) {
+  const Tensor t = t_.contiguous();
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+
+TriMulWeights weight_ptrs(const Weights& w) {
+  TriMulWeights p;
+  const void* a[kWeights];
+  for (int i = 0; i < kWeights; ++i) a[i] = ptr(w[i]);
+  std::memcpy(&p, a, sizeof p);
+  return p;
+}
+
+struct MulCall { TriMulDesc d; Tensor x, mask, saved, out; Weights w; };
+
+MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights, bool outgoing, double eps, int64_t precision, bool keep) {
+  TORCH_CHECK(x.is_cuda(), "triangle_multiplicative_update needs CUDA tensors: there is no CPU implementation");
+  MulCall c{};
+  c.d.dtype = dtype_code(x);
+  for (int i : {2, 4, 8, 10}) TORCH_CHECK_VALUE(weights[i].defined(), kNames[i], " is required");
+  TORCH_CHECK_VALUE(x.dim() >= 3 && x.size(-2) == x.size(-3), "x must be [*, N, N, C], got ", x.sizes());
+  const int64_t N = x.size(-2), C = x.size(-1);
+  c.x = aligned(x.dim() == 4 ? x : x.reshape({-1, N, N, C}));
+  const int64_t B = c.x.size(0);
+  if (mask.defined()) c.mask = aligned(mask.to(x.scalar_type()).expand(x.sizes().slice(0, x.dim() - 1)).reshape({B, N, N}));
+  for (int i = 0; i < kWeights; ++i)
+    if (weights[i].defined()) c.w[i] = aligned(weights[i].scalar_type() == x.scalar_type() ? weights[i].detach() : weights[i].detach().to(x.scalar_type()));
+  const int64_t Ch = c.w[2].size(0) / 2;
+  const int64_t rows[kWeights] = {C, C, 2 * Ch, 2 * Ch, 2 * Ch, 2 * Ch, Ch, Ch, C, C, C, C};
+  const int64_t cols[kWeights] = {0, 0, C, 0, C, 0, 0, 0, Ch, 0, C, 0};
+  for (int i = 0; i < kWeights; ++i) {
+    if (!c.w[i].defined()) continue;
+    const auto s = c.w[i].sizes();
+    const bool fits = cols[i] ? s.size() == 2 && s[0] == rows[i] && s[1] == cols[i] : s.size() == 1 && s[0] == rows[i];
+    TORCH_CHECK_VALUE(fits, kNames[i], " has shape ", s, ", expected [", rows[i], cols[i] ? ", " + std::to_string(cols[i]) : std::string(), "]");
+  }
+  c.d.B = B; c.d.N = N; c.d.C = C; c.d.Ch = Ch; c.d.precision = (int)precision;
+  c.d.direction = outgoing ? TRI_OUTGOING : TRI_INCOMING; c.d.eps = (float)eps;
+  const c10::cuda::CUDAGuard guard(x.device());
+  if (keep) c.saved = bytes(api.mul_saved_bytes(&c.d), x);
+  const size_t n = api.mul_ws_bytes(&c.d, 0);
+  const Tensor ws = bytes(n, x);
+  c.out = at::empty(c.x.sizes(), c.x.options());
+  const TriMulWeights w = weight_ptrs(c.w);
+  const tri_stream_t st = stream_of(x);
+  ok(api.mul_fwd(&c.d, ptr(c.x), ptr(c.mask), &w, ptr(c.out), ptr(c.saved), ptr(ws), n, st), "tri_mul_fwd");
+  check_device(ws, reinterpret_cast<cudaStream_t>(st));
+  return c;
+}
+
+struct MulFn : torch::autograd::Function<MulFn> {
+  using O = const OptTensor&;
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, O mask, O w0, O w1, O w2, O w3, O w4, O w5, O w6, O w7, O w8, O w9, O w10,
+                        O w11, bool outgoing, double eps, int64_t precision) {
+    Weights in;
+    int n = 0;
+    for (O w : {std::cref(w0), std::cref(w1), std::cref(w2), std::cref(w3), std::cref(w4), std::cref(w5), std::cref(w6), std::cref(w7),
+                std::cref(w8), std::cref(w9), std::cref(w10), std::cref(w11)})
+      in[n++] = or_undefined(w);
+    const MulCall c = mul_forward(x, or_undefined(mask), in, outgoing, eps, precision, /*keep=*/true);
+    variable_list keep = {c.x, c.mask, c.saved};
+    std::vector<int64_t> dtypes(kWeights, -1);
+    for (int i = 0; i < kWeights; ++i) {
+      keep.push_back(c.w[i]);
+      if (in[i].defined()) dtypes[i] = (int64_t)in[i].scalar_type();
+    }
+    ctx->save_for_backward(keep);
+    ctx->saved_data["desc"] = std::string(reinterpret_cast<const char*>(&c.d), sizeof c.d);
+    ctx->saved_data["dtypes"] = dtypes;
+    ctx->saved_data["shape"] = x.sizes().vec();
+    return c.out.reshape(x.sizes());
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &mask = s[1], &saved = s[2];
+    TriMulDesc d;
+    std::memcpy(&d, ctx->saved_data["desc"].toStringRef().data(), sizeof d);
+    const auto dtypes = ctx->saved_data["dtypes"].toIntVector();
+    Weights w;
+    for (int i = 0; i < kWeights; ++i) w[i] = s[3 + i];
+    // the weight gradients, fp32 as the library writes them, side by side: one conversion to the weights' dtype for all
+    std::array<int64_t, kWeights> at_{};
+    int64_t total = 0, one = -1;
+    bool same = true;
+    size_t input = mask.defined() ? 2 : 1;   // x, the mask, then the weights that are there
+    for (int i = 0; i < kWeights; ++i) {
+      at_[i] = -1;
+      if (!w[i].defined() || !ctx->needs_input_grad(input++)) continue;
+      at_[i] = total;
+      total += (w[i].numel() + 15) / 16 * 16;
+      if (one >= 0 && one != dtypes[i]) same = false;
+      one = dtypes[i];
+    }
+    Tensor flat = at::empty({total}, x.options().dtype(at::kFloat));
+    void* g_ptr[kWeights];
+    for (int i = 0; i < kWeights; ++i) g_ptr[i] = at_[i] < 0 ? nullptr : flat.data_ptr<float>() + at_[i];
+    TriMulWeightGrads g;
+    std::memcpy(&g, g_ptr, sizeof g);
+    const Tensor d_out = aligned(grads[0].reshape(x.sizes()).to(x.scalar_type()));
+    Tensor dx = at::empty(x.sizes(), x.options());
+    const c10::cuda::CUDAGuard guard(x.device());
+    const size_t n = api.mul_ws_bytes(&d, 1);
+    const Tensor ws = bytes(n, x);
+    const TriMulWeights wp = weight_ptrs(w);
+    const tri_stream_t st = stream_of(x);
+    ok(api.mul_bwd(&d, ptr(x), ptr(mask), &wp, ptr(saved), ptr(d_out), ptr(dx), &g, ptr(ws), n, st), "tri_mul_bwd");
+    check_device(ws, reinterpret_cast<cudaStream_t>(st));
+    variable_list out(2 + kWeights + 3);
+    if (ctx->needs_input_grad(0)) out[0] = dx.reshape(ctx->saved_data["shape"].toIntVector());
+    if (same && one >= 0) flat = flat.to((at::ScalarType)one);
+    for (int i = 0; i < kWeights; ++i) {
+      if (at_[i] < 0) continue;
+      Tensor t = flat.narrow(0, at_[i], w[i].numel()).view(w[i].sizes());
+      out[2 + i] = same ? t : t.to((at::ScalarType)dtypes[i]);
+    }
+    return out;
+  }
+};
+
+Tensor multiplicative_update(const Tensor& x, const OptTensor& mask_, bool outgoing, double eps, int64_t precision,
+                             const std::vector<OptTensor>& weights) {
+  TORCH_CHECK(weights.size() == kWeights, "expected ", kWeights, " weights");
+  Weights w;
+  bool grad = x.requires_grad();
+  for (int i = 0; i < kWeights; ++i) {
+    if (!weights[i].has_value()) continue;
+    w[i] = *weights[i];
+    grad = grad || w[i].requires_grad();
+  }
+  const Tensor mask = mask_.has_value() ? *mask_ : Tensor();
+  if (at::GradMode::is_enabled() && grad)
+    return MulFn::apply(x, mask_, weights[0], weights[1], weights[2], weights[3], weights[4], weights[5], weights[6], weights[7], weights[8],
+                        weights[9], weights[10], weights[11], outgoing, eps, precision);
+  return mul_forward(x, mask, w, outgoing, eps, precision, /*keep=*/false).out.reshape(x.sizes());
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("bind", &bind);
+  m.def("attention", &attention);
+  m.def("multiplicative_update", &multiplicative_update);
+}
