@@ -12,6 +12,7 @@
 #include "attn_simt.cuh"
 #include "common.cuh"
 #include "tc_gemm.cuh"
+#include "tc_lnproject.cuh"
 #include "tc_paths.cuh"
 #include "trimul_simt.cuh"
 
@@ -207,6 +208,17 @@ int tri_attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w, 
   if (!z || !w_qkv || !w_bias || !qkv || !bias || !ws) return fail(TRI_ERR_ARG, "z, w_qkv, w_bias, qkv, bias and ws must not be null");
   set_path("tcgen05");
   return tc::attn_project(d, z, ln_w, ln_b, w_qkv, w_bias, qkv, bias, ws, ws_bytes, (cudaStream_t)stream);
+}
+
+int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z, const void* ln_w, const void* ln_b,
+                          const void* w_bias, void* bias, void* ws, tri_stream_t stream) {
+  if (d == nullptr) return fail(TRI_ERR_ARG, "descriptor is null");
+  if (!z || !w_bias || !bias || !ws) return fail(TRI_ERR_ARG, "z, w_bias, bias and ws must not be null");
+  if (d->C != 128 || !tc::ln_project_supported(d->dtype, d->M, 0, d->H))
+    return fail(TRI_ERR_UNSUPPORTED, "the pair-bias projection needs C = 128, 1 <= H <= 16 and bf16 / fp16");
+  if (plane < 1 || d->M % plane != 0) return fail(TRI_ERR_ARG, "plane %lld does not divide M = %lld", (long long)plane, (long long)d->M);
+  set_path("tcgen05");
+  return tc::attn_project_bias(d, plane, z, ln_w, ln_b, w_bias, bias, ws, (cudaStream_t)stream);
 }
 
 size_t tri_mul_saved_bytes(const TriMulDesc* d) {

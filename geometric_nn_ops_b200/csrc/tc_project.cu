@@ -12,6 +12,7 @@
 // geometric_nn_ops_torch/triangle/_triattn.py:36-44); eager torch does the same work in a LayerNorm, four linears and
 // a permute, about 10 pair-sized tensors of HBM traffic against 6 here.
 #include "tc_gemm.cuh"
+#include "tc_lnproject.cuh"
 #include "tc_paths.cuh"
 
 namespace tri {
@@ -153,6 +154,17 @@ int project_t(const TriAttnProjDesc* d, const void* z, const void* ln_w, const v
   return launch_gemm(st, d->dtype, EPI_STORE, 128, false, p, err);
 }
 
+// 16-bit projections of up to 384 columns: the one-kernel form (zn stays on the SM).  Wider ones do not leave room for
+// resident weights beside the tiles, and fp32 (TF32) operands are twice as wide.
+bool in_one_kernel(const TriAttnProjDesc* d) { return ln_project_supported(d->dtype, d->M, 3 * d->H * d->D, d->H); }
+
+LnProject one_kernel(const TriAttnProjDesc* d, const void* z, const void* ln_w, const void* ln_b, const void* w_bias, void* bias, void* ws) {
+  LnProject p{};
+  p.dtype = d->dtype; p.M = p.plane = d->M; p.heads = d->H; p.eps = d->eps;
+  p.z = z; p.gamma = ln_w; p.beta = ln_b; p.w_bias = w_bias; p.bias = bias; p.err = static_cast<int*>(ws);
+  return p;
+}
+
 }  // namespace
 
 bool attn_project_supported(const TriAttnProjDesc* d) {
@@ -162,18 +174,33 @@ bool attn_project_supported(const TriAttnProjDesc* d) {
 }
 
 size_t attn_project_ws_bytes(const TriAttnProjDesc* d) {
+  if (in_one_kernel(d)) return 256;
   return 256 + align_up((size_t)d->M * CW * (d->dtype == TRI_F32 ? 4 : 2));
 }
 
 int attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w, const void* ln_b, const void* w_qkv,
                  const void* w_bias, void* qkv, void* bias, void* ws, size_t ws_size, cudaStream_t st) {
   if (ws_size < attn_project_ws_bytes(d)) return fail(TRI_ERR_WORKSPACE, "projection workspace too small");
+  if (in_one_kernel(d)) {
+    LnProject p = one_kernel(d, z, ln_w, ln_b, w_bias, bias, ws);
+    p.n_out = 3 * d->H * d->D; p.w_qkv = w_qkv; p.qkv = qkv;
+    TRI_CUDA_OK(cudaMemsetAsync(ws, 0, 256, st));
+    return ln_project(st, p);
+  }
   switch (d->dtype) {
     case TRI_F32: return project_t<float>(d, z, ln_w, ln_b, w_qkv, w_bias, qkv, bias, ws, st);
     case TRI_BF16: return project_t<__nv_bfloat16>(d, z, ln_w, ln_b, w_qkv, w_bias, qkv, bias, ws, st);
     case TRI_F16: return project_t<__half>(d, z, ln_w, ln_b, w_qkv, w_bias, qkv, bias, ws, st);
   }
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
+}
+
+int attn_project_bias(const TriAttnProjDesc* d, long long plane, const void* z, const void* ln_w, const void* ln_b, const void* w_bias,
+                      void* bias, void* ws, cudaStream_t st) {
+  LnProject p = one_kernel(d, z, ln_w, ln_b, w_bias, bias, ws);
+  p.plane = plane;
+  TRI_CUDA_OK(cudaMemsetAsync(ws, 0, 256, st));
+  return ln_project(st, p);
 }
 
 }  // namespace tc

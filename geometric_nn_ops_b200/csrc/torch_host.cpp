@@ -7,6 +7,7 @@
 //
 // Semantics follow the reference's public wrappers (geometric_nn_ops_torch/triangle/_triattn.py:23-106, _trimul.py:39-88).
 // The library is reached through function pointers taken from the one that the ctypes binding loaded.
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -37,6 +38,7 @@ struct Api {
   decltype(&tri_attn_ws_bytes) attn_ws_bytes;
   decltype(&tri_attn_fwd) attn_fwd;
   decltype(&tri_attn_bwd) attn_bwd;
+  decltype(&tri_attn_project_bias) attn_project_bias;
   decltype(&tri_mul_saved_bytes) mul_saved_bytes;
   decltype(&tri_mul_ws_bytes) mul_ws_bytes;
   decltype(&tri_mul_fwd) mul_fwd;
@@ -52,6 +54,7 @@ void bind(const std::string& path) {
   };
   get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
   get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
+  get(api.attn_project_bias, "tri_attn_project_bias");
   get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
   get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
 }
@@ -372,10 +375,34 @@ Tensor multiplicative_update(const Tensor& x, const OptTensor& mask_, bool outgo
   return mul_forward(x, mask, w, outgoing, eps, precision, /*keep=*/false).out.reshape(x.sizes());
 }
 
+// ---------------------------------------------------------------------------------------------------- pair bias
+
+// z [B, U, V, 128] -> LayerNorm (weight only) -> projection to H <= 16 heads -> [B, H, U, V], without gradients; None where
+// the kernel does not take the call (mixed or other types, other channel counts, gradients or autocast in force)
+py::object pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
+  const auto dt = z.scalar_type();
+  const bool fits = z.is_cuda() && z.dim() == 4 && (dt == at::kBFloat16 || dt == at::kHalf) && z.size(3) == 128 && w.dim() == 2 &&
+                    w.size(1) == 128 && w.size(0) >= 1 && w.size(0) <= 16 && w.scalar_type() == dt && w.device() == z.device() &&
+                    (!ln_w.has_value() || (ln_w->scalar_type() == dt && ln_w->dim() == 1 && ln_w->size(0) == 128 && ln_w->device() == z.device()));
+  const bool grad = at::GradMode::is_enabled() && (z.requires_grad() || w.requires_grad() || (ln_w.has_value() && ln_w->requires_grad()));
+  const int64_t plane = z.dim() == 4 ? z.size(1) * z.size(2) : 0, M = fits ? z.size(0) * plane : 0;
+  if (!fits || grad || M < 1 || M >= (1LL << 31) - 128 || at::autocast::is_autocast_enabled(at::kCUDA)) return py::none();
+  TriAttnProjDesc d{};
+  d.M = M; d.C = 128; d.H = (int32_t)w.size(0); d.dtype = dtype_code(z); d.eps = (float)eps;
+  const c10::cuda::CUDAGuard guard(z.device());
+  const Tensor zc = aligned(z), wc = aligned(w), lw = ln_w.has_value() ? ln_w->contiguous() : Tensor(), ws = bytes(256, z);
+  const Tensor out = at::empty({z.size(0), w.size(0), z.size(1), z.size(2)}, z.options());
+  const tri_stream_t st = stream_of(z);
+  ok(api.attn_project_bias(&d, plane, ptr(zc), ptr(lw), nullptr, ptr(wc), ptr(out), ptr(ws), st), "tri_attn_project_bias");
+  check_device(ws, reinterpret_cast<cudaStream_t>(st));
+  return py::cast(out);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bind", &bind);
   m.def("attention", &attention);
   m.def("multiplicative_update", &multiplicative_update);
+  m.def("pair_bias", &pair_bias);
 }

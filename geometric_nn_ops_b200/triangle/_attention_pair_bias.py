@@ -18,12 +18,17 @@ torch operations in both cases.
 import torch
 import torch.nn.functional as F
 
+from .. import _lib
 from ._masking import mask_val
 from ._triattn import _DTYPES, triangle_attention_b200
 
 
 def _pair_bias(z, ln_z_weight, proj_z_weight, eps):
     """``(B, U, V, Zc)`` -> LayerNorm (weight only) -> ``Zc -> H`` projection -> ``(B, H, U, V)`` contiguous."""
+    if z.is_cuda:   # one kernel where no gradient is recorded and it has the shape (16-bit types, 128 channels, H <= 16)
+        pz = _lib.host().pair_bias(z, ln_z_weight, proj_z_weight, eps)
+        if pz is not None:
+            return pz
     zn = F.layer_norm(z, z.shape[-1:], ln_z_weight, None, eps)
     return F.linear(zn, proj_z_weight).permute(0, 3, 1, 2).contiguous()
 

@@ -138,6 +138,11 @@ int tri_attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w /
                      const void* w_qkv, const void* w_bias, void* qkv, void* bias, void* ws, size_t ws_bytes,
                      tri_stream_t stream);
 
+/* The same LayerNorm and the pair bias alone, for up to 16 heads (bf16 / fp16; d->D is not read).  `plane`: pixels of
+ * one batch entry (it divides M); bias: [M / plane, H, plane].  ws: 256 bytes of device memory (the status word). */
+int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z, const void* ln_w /*nullable*/,
+                          const void* ln_b /*nullable*/, const void* w_bias, void* bias, void* ws, tri_stream_t stream);
+
 /* ------------------------------------------------------------------------ */
 /* Triangle multiplicative update                                           */
 /* ------------------------------------------------------------------------ */
