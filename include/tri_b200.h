@@ -45,7 +45,8 @@ enum {
 int tri_abi_version(void);
 const char* tri_last_error(void);
 /* Name of the kernel family the most recent forward/backward (on any thread) ran on:
- * "simt" (CUDA-core fp32 path) or "tcgen05" (tensor-core path). */
+ * "tcgen05" (fifth-generation tensor cores) or "simt" (CUDA cores, and warp-level matrix instructions for TF32 products of
+ * fp32 attention). */
 const char* tri_last_path(void);
 /* Number of kernel launches issued by this library (all threads) since the
  * last call to tri_reset_launch_count(). */
