@@ -17,6 +17,8 @@
 namespace tri {
 namespace simt {
 
+__device__ __forceinline__ int cdiv_dev(int a, int b) { return (a + b - 1) / b; }
+
 // ============================================================================
 // generic strided GEMM   C[m,n] (+)= sum_k A(m,k) * B(n,k)  (+ bias[n])
 // ============================================================================
@@ -32,73 +34,107 @@ struct GemmP {
   int accumulate;
 };
 
-template <bool TF32>
-__global__ void __launch_bounds__(256) gemm_kernel(GemmP p) {
-  __shared__ float As[16][65];
-  __shared__ float Bs[16][65];
-  const int tid = threadIdx.y * 16 + threadIdx.x;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+// A tile of 16 T x 16 T outputs, T x T per thread (two runs of T / 2 or one of T, so that operands are read four at a time), K in steps
+// of 16 through double-buffered shared memory; the next step's operands are fetched into registers while this one runs.
+// T = 8 reads 4 x 16 bytes per 64 FMAs, T = 4 reads 2 per 16; a 4 x 4 tile of scalar reads, eight per 16, was bound by
+// them.
+template <int T, bool TF32>
+__global__ void __launch_bounds__(256, 2) gemm_kernel(GemmP p) {
+  constexpr int W = 16 * T, E = T;            // tile width; elements of one operand per thread and step
+  __shared__ __align__(16) float As[2][16][W + 4];
+  __shared__ __align__(16) float Bs[2][16][W + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * W, n0 = blockIdx.x * W;
   int kper = (p.K + p.ksplit - 1) / p.ksplit;
   kper = (kper + 15) / 16 * 16;
   const int kbeg = blockIdx.z * kper;
   const int kend = min(p.K, kbeg + kper);
-  float acc[4][4] = {};
-  for (int k0 = kbeg; k0 < kend; k0 += 16) {
+  float ra[E], rb[E];
+  // an element's row and k: sixteen k of E rows where k is contiguous, else W rows and every (256 / W)-th k
+  const bool ak = p.a_k == 1, bk = p.b_k == 1;
+  const int a_row = ak ? tid >> 4 : tid % W, a_kk = ak ? tid & 15 : tid / W, b_row = bk ? tid >> 4 : tid % W, b_kk = bk ? tid & 15 : tid / W;
+  const int a_dr = ak ? 16 : 0, a_dk = ak ? 0 : 256 / W, b_dr = bk ? 16 : 0, b_dk = bk ? 0 : 256 / W;
+  const float* pa = p.A + (long long)(m0 + a_row) * p.a_m + (long long)(kbeg + a_kk) * p.a_k;
+  const float* pb = p.B + (long long)(n0 + b_row) * p.b_n + (long long)(kbeg + b_kk) * p.b_k;
+  const long long a_e = a_dr * p.a_m + a_dk * p.a_k, b_e = b_dr * p.b_n + b_dk * p.b_k;
+  const bool whole = m0 + W <= p.M && n0 + W <= p.N;
+  auto fetch = [&](int k0) {
+    const float *qa = pa, *qb = pb;
+    if (whole && k0 + 16 <= kend) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      int idx = tid + 256 * e;
-      int mm, kk;
-      if (p.a_k == 1) { kk = idx & 15; mm = idx >> 4; } else { mm = idx & 63; kk = idx >> 6; }
-      float v = 0.f;
-      if (m0 + mm < p.M && k0 + kk < kend) v = p.A[(long long)(m0 + mm) * p.a_m + (long long)(k0 + kk) * p.a_k];
-      As[kk][mm] = TF32 ? round_tf32(v) : v;
-      int nn;
-      if (p.b_k == 1) { kk = idx & 15; nn = idx >> 4; } else { nn = idx & 63; kk = idx >> 6; }
-      v = 0.f;
-      if (n0 + nn < p.N && k0 + kk < kend) v = p.B[(long long)(n0 + nn) * p.b_n + (long long)(k0 + kk) * p.b_k];
-      Bs[kk][nn] = TF32 ? round_tf32(v) : v;
+      for (int e = 0; e < E; ++e, qa += a_e, qb += b_e) { ra[e] = *qa; rb[e] = *qb; }
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e, qa += a_e, qb += b_e) {
+        ra[e] = m0 + a_row + e * a_dr < p.M && k0 + a_kk + e * a_dk < kend ? *qa : 0.f;
+        rb[e] = n0 + b_row + e * b_dr < p.N && k0 + b_kk + e * b_dk < kend ? *qb : 0.f;
+      }
     }
-    __syncthreads();
+    pa += 16 * p.a_k;
+    pb += 16 * p.b_k;
+  };
+  auto put = [&](int buf) {
 #pragma unroll
+    for (int e = 0; e < E; ++e) {
+      As[buf][a_kk + e * a_dk][a_row + e * a_dr] = TF32 ? round_tf32(ra[e]) : ra[e];
+      Bs[buf][b_kk + e * b_dk][b_row + e * b_dr] = TF32 ? round_tf32(rb[e]) : rb[e];
+    }
+  };
+  float2 acc[T / 2][T] = {};   // rows 2 r, 2 r + 1 packed
+  if (kbeg < kend) { fetch(kbeg); put(0); }
+  for (int k0 = kbeg, buf = 0; k0 < kend; k0 += 16, buf ^= 1) {
+    __syncthreads();
+    const bool more = k0 + 16 < kend;
+    if (more) fetch(k0 + 16);
+#pragma unroll 4
     for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
+      float a[T], b[T];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[kk][ty + 16 * r];
+      for (int h = 0; h < T / 4; ++h) {
+        const float4 x = *reinterpret_cast<const float4*>(&As[buf][kk][h * 64 + ty * 4]);
+        const float4 y = *reinterpret_cast<const float4*>(&Bs[buf][kk][h * 64 + tx * 4]);
+        a[h * 4] = x.x; a[h * 4 + 1] = x.y; a[h * 4 + 2] = x.z; a[h * 4 + 3] = x.w;
+        b[h * 4] = y.x; b[h * 4 + 1] = y.y; b[h * 4 + 2] = y.z; b[h * 4 + 3] = y.w;
+      }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx + 16 * c];
+      for (int c = 0; c < T; ++c)
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
+        for (int r = 0; r < T / 2; ++r) acc[r][c] = __ffma2_rn(make_float2(a[2 * r], a[2 * r + 1]), make_float2(b[c], b[c]), acc[r][c]);
     }
-    __syncthreads();
+    if (more) put(buf ^ 1);
   }
   float* C = p.C + (long long)blockIdx.z * p.c_split;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    int m = m0 + ty + 16 * r;
+  for (int r = 0; r < T; ++r) {
+    const int m = m0 + (r >> 2) * 64 + ty * 4 + (r & 3);
     if (m >= p.M) continue;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      int n = n0 + tx + 16 * c;
+    for (int c = 0; c < T; ++c) {
+      const int n = n0 + (c >> 2) * 64 + tx * 4 + (c & 3);
       if (n >= p.N) continue;
-      float v = acc[r][c];
+      float v = r & 1 ? acc[r >> 1][c].y : acc[r >> 1][c].x;
       if (p.bias != nullptr && blockIdx.z == 0) v += p.bias[n];
-      long long o = (long long)m * p.c_m + (long long)n * p.c_n;
+      const long long o = (long long)m * p.c_m + (long long)n * p.c_n;
       if (p.accumulate) v += C[o];
       C[o] = v;
     }
   }
 }
 
+// 128 x 128 tiles where there is one for every SM, else 64 x 64
 static int gemm(cudaStream_t st, bool tf32, GemmP p) {
   if (p.M <= 0 || p.N <= 0) return 0;
-  dim3 grid(cdiv(p.N, 64), cdiv(p.M, 64), p.ksplit);
-  dim3 block(16, 16);
   KernelTimer kt("simt_gemm", st, 2.0 * p.M * p.N * p.K, 4.0 * ((double)p.M * p.K + (double)p.N * p.K + (double)p.M * p.N));
-  if (tf32) gemm_kernel<true><<<grid, block, 0, st>>>(p);
-  else gemm_kernel<false><<<grid, block, 0, st>>>(p);
+  const bool wide = (long long)cdiv(p.N, 128) * cdiv(p.M, 128) * p.ksplit >= 148 && p.M > 64 && p.N > 64;
+  const int w = wide ? 128 : 64;
+  const dim3 grid(cdiv(p.N, w), cdiv(p.M, w), p.ksplit);
+  if (wide) {
+    if (tf32) gemm_kernel<8, true><<<grid, 256, 0, st>>>(p);
+    else gemm_kernel<8, false><<<grid, 256, 0, st>>>(p);
+  } else {
+    if (tf32) gemm_kernel<4, true><<<grid, 256, 0, st>>>(p);
+    else gemm_kernel<4, false><<<grid, 256, 0, st>>>(p);
+  }
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -134,68 +170,117 @@ static int weight_grad(cudaStream_t st, bool tf32, const float* D, int ldd, int 
 
 // ============================================================================
 // per-channel contraction  O[p,q,c] = sum_r X(p,r,c) * Y(q,r,c)
-// One thread per channel (coalesced along c), 8x8 output pixels per thread.
 // ============================================================================
 struct ContractP {
   const float* X;
   const float* Y;
   float* O;
-  int N, Ch, cblocks;
+  int N, Ch;
   long long xs_p, xs_r, ys_q, ys_r, os_p, os_q;  // pixel strides inside one N x N plane
   int ldx, ldy, ldo;                             // channels per pixel in each buffer
   int xoff, yoff, ooff;                          // first channel inside the buffer
+  int vec;                                       // channels can be copied four at a time
 };
 
-template <bool TF32>
-__global__ void __launch_bounds__(128) contract_kernel(ContractP p) {
-  const int cb = blockIdx.z % p.cblocks;
-  const int b = blockIdx.z / p.cblocks;
-  const int c = cb * blockDim.x + threadIdx.x;
-  const bool c_ok = c < p.Ch;
-  const int p0 = blockIdx.x * 8;
-  const int q0 = (blockIdx.y * blockDim.y + threadIdx.y) * 8;
+// A CTA has PT x QT output pixels of 32 channels (lane = channel) and steps through the r axis R pixels at a time, double-
+// buffered by cp.async; each of its eight warps has TP x TQ of the pixels in registers.  TP + TQ shared loads feed TP * TQ
+// FMAs: at 16 x 8 the FMAs bound it (32 TFLOP/s at 384 residues).  One thread per channel reading 8 x 8 pixels from global
+// memory took a byte of L2 traffic per FMA and was bound by that (6.6 TFLOP/s; 66 us at 64 residues against 8).
+template <int TP, int TQ>
+struct ContractTile {
+  static constexpr int kWarpsP = TP == 16 ? 2 : 4, kWarpsQ = 8 / kWarpsP, PT = TP * kWarpsP, QT = TQ * kWarpsQ;
+  static constexpr int R = TP == 4 ? 16 : 8, kStage = R * (PT + QT) * 32, kSmem = 2 * kStage * 4;
+};
+
+template <int TP, int TQ, bool TF32>
+__global__ void __launch_bounds__(256) contract_kernel(ContractP p) {
+  using L = ContractTile<TP, TQ>;
+  constexpr int PT = L::PT, QT = L::QT, R = L::R;
+  extern __shared__ __align__(16) float sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cblocks = cdiv_dev(p.Ch, 32), cb = blockIdx.z % cblocks, b = blockIdx.z / cblocks, c0 = cb * 32;
+  const int p0 = blockIdx.x * PT, q0 = blockIdx.y * QT;
   const long long plane = (long long)b * p.N * p.N;
-  float acc[8][8] = {};
-  const float* X = p.X + p.xoff + (c_ok ? c : 0);
-  const float* Y = p.Y + p.yoff + (c_ok ? c : 0);
-  for (int r = 0; r < p.N; ++r) {
-    float xv[8], yv[8];
+  // this thread's copies: four channels of one row of X and one of Y, every 32 / PT (32 / QT) th r
+  const int c4 = c0 + (threadIdx.x & 7) * 4, slot = threadIdx.x >> 3, left = p.Ch - c4;
+  const int xr = slot / PT, xrow = slot % PT, yr = slot / QT, yrow = slot % QT;
+  const float* X = p.X + p.xoff + (plane + min(p0 + xrow, p.N - 1) * p.xs_p + xr * p.xs_r) * p.ldx + c4;
+  const float* Y = p.Y + p.yoff + (plane + min(q0 + yrow, p.N - 1) * p.ys_q + yr * p.ys_r) * p.ldy + c4;
+  const long long x_step = p.xs_r * p.ldx * (32 / PT), y_step = p.ys_r * p.ldy * (32 / QT);
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+  const uint32_t xd = base + ((xr * PT + xrow) * 32 + (threadIdx.x & 7) * 4) * 4, yd = base + (R * PT * 32 + (yr * QT + yrow) * 32 + (threadIdx.x & 7) * 4) * 4;
+  auto copy = [&](uint32_t dst, const float* src, bool live, const float* safe) {
+    if (p.vec) {
+      const bool on = live && left > 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(on ? src : safe), "r"(on ? 16 : 0) : "memory");
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int pp = p0 + i;
-      xv[i] = (c_ok && pp < p.N) ? X[(plane + pp * p.xs_p + r * p.xs_r) * p.ldx] : 0.f;
-      int qq = q0 + i;
-      yv[i] = (c_ok && qq < p.N) ? Y[(plane + qq * p.ys_q + r * p.ys_r) * p.ldy] : 0.f;
-      if (TF32) { xv[i] = round_tf32(xv[i]); yv[i] = round_tf32(yv[i]); }
+      for (int e = 0; e < 4; ++e) {
+        const bool on = live && e < left;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * e), "l"(on ? src + e : safe), "r"(on ? 4 : 0) : "memory");
+      }
     }
+  };
+  auto issue = [&](int r0, int buf) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int e = 0; e < R * PT / 32; ++e, X += x_step) copy(xd + buf * L::kStage * 4 + e * 32 * 128, X, r0 + xr + e * (32 / PT) < p.N, p.X);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(xv[i], yv[j], acc[i][j]);
+    for (int e = 0; e < R * QT / 32; ++e, Y += y_step) copy(yd + buf * L::kStage * 4 + e * 32 * 128, Y, r0 + yr + e * (32 / QT) < p.N, p.Y);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int wp = warp / L::kWarpsQ * TP, wq = warp % L::kWarpsQ * TQ;
+  float2 acc[TP / 2][TQ] = {};   // pixels 2 i, 2 i + 1 packed
+  issue(0, 0);
+  for (int r0 = 0, buf = 0; r0 < p.N; r0 += R, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (r0 + R < p.N) issue(r0 + R, buf ^ 1);
+    const float* xs = sm + buf * L::kStage + wp * 32 + lane;
+    const float* ys = sm + buf * L::kStage + R * PT * 32 + wq * 32 + lane;
+#pragma unroll 2
+    for (int r = 0; r < R; ++r) {
+      float xv[TP], yv[TQ];
+#pragma unroll
+      for (int j = 0; j < TQ; ++j) yv[j] = TF32 ? round_tf32(ys[(r * QT + j) * 32]) : ys[(r * QT + j) * 32];
+#pragma unroll
+      for (int i = 0; i < TP; ++i) xv[i] = TF32 ? round_tf32(xs[(r * PT + i) * 32]) : xs[(r * PT + i) * 32];
+#pragma unroll
+      for (int j = 0; j < TQ; ++j)
+#pragma unroll
+        for (int i = 0; i < TP / 2; ++i) acc[i][j] = __ffma2_rn(make_float2(xv[2 * i], xv[2 * i + 1]), make_float2(yv[j], yv[j]), acc[i][j]);
+    }
   }
-  if (!c_ok) return;
+  if (c0 + lane >= p.Ch) return;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (p0 + i >= p.N) continue;
+  for (int i = 0; i < TP; ++i) {
+    if (p0 + wp + i >= p.N) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (q0 + j >= p.N) continue;
-      p.O[(plane + (p0 + i) * p.os_p + (q0 + j) * p.os_q) * p.ldo + p.ooff + c] = acc[i][j];
+    for (int j = 0; j < TQ; ++j) {
+      if (q0 + wq + j >= p.N) continue;
+      p.O[(plane + (p0 + wp + i) * p.os_p + (q0 + wq + j) * p.os_q) * p.ldo + p.ooff + c0 + lane] = i & 1 ? acc[i >> 1][j].y : acc[i >> 1][j].x;
     }
   }
 }
 
-static int contract(cudaStream_t st, bool tf32, int B, ContractP p) {
-  int bx = p.Ch >= 128 ? 128 : (p.Ch + 31) / 32 * 32;
-  int by = 128 / bx;
-  p.cblocks = cdiv(p.Ch, bx);
-  dim3 block(bx, by);
-  dim3 grid(cdiv(p.N, 8), cdiv(p.N, 8 * by), B * p.cblocks);
+template <int TP, int TQ>
+static int contract_start(cudaStream_t st, bool tf32, int B, const ContractP& p) {
+  using L = ContractTile<TP, TQ>;
+  const auto kern = tf32 ? contract_kernel<TP, TQ, true> : contract_kernel<TP, TQ, false>;
+  TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem));
+  const dim3 grid(cdiv(p.N, L::PT), cdiv(p.N, L::QT), B * cdiv(p.Ch, 32));
   KernelTimer kt("simt_contract", st, 2.0 * B * p.N * (double)p.N * p.N * p.Ch, 12.0 * B * (double)p.N * p.N * p.Ch);
-  if (tf32) contract_kernel<true><<<grid, block, 0, st>>>(p);
-  else contract_kernel<false><<<grid, block, 0, st>>>(p);
+  kern<<<grid, 256, L::kSmem, st>>>(p);
   TRI_LAUNCH_OK();
   return 0;
+}
+
+// The largest tile that still makes a CTA for every SM.
+static int contract(cudaStream_t st, bool tf32, int B, ContractP p) {
+  p.vec = p.ldx % 4 == 0 && p.ldy % 4 == 0 && p.xoff % 4 == 0 && p.yoff % 4 == 0 && p.Ch % 4 == 0;
+  const long long planes = (long long)B * cdiv(p.Ch, 32);
+  if (planes * cdiv(p.N, 32) * cdiv(p.N, 32) >= 148) return contract_start<16, 8>(st, tf32, B, p);
+  if (planes * cdiv(p.N, 32) * cdiv(p.N, 16) >= 120) return contract_start<8, 8>(st, tf32, B, p);
+  return contract_start<4, 4>(st, tf32, B, p);
 }
 
 // ============================================================================
@@ -473,6 +558,261 @@ static GemmP linear_t_p(const float* D, int ldd, const float* W, float* out, lon
   return p;
 }
 
+// ============================================================================
+// forward in three kernels: LayerNorm + input projections + gate, contraction, LayerNorms + output projections + gate
+// ============================================================================
+// A CTA of 256 threads has 64 output channels of two products, whose weights stay in shared memory, and walks over tiles of
+// 64 pixels, which it normalises in shared memory: z, the projections and the LayerNormed contraction are written only where
+// the backward needs them.  Both operands lie k-major, so that a thread's 8 pixels x 4 + 4 channels take four 16-byte
+// shared loads per 64 FMAs (output stage, whose products have their own left operands: three per 32); the two halves of the
+// CTA have half of each contraction and exchange half of their sums.  Two CTAs share an SM; one's loads and LayerNorm run
+// under the other's products.  The FMAs are packed in pairs: 1.2 clocks per 32 of them against 1.4 for single ones.
+//   One stage per kernel -- 9 conversions, 2 LayerNorms, 4 GEMMs of 16 us and two gates -- took 116 us of the 183 us of a
+// 64 x 64 x 128 fp32 call; these take 22 and 19 us of 52 (and 0.60 and 0.38 ms at 384 x 384, against 2.1 ms).
+struct FusedP {
+  const void *x, *mask, *norm_in_w, *norm_in_b, *p_w, *p_b, *g_w, *g_b, *norm_out_w, *norm_out_b;
+  const float* t;                                   // output stage: the contraction
+  float *z, *mean, *rstd, *P, *G, *ab;              // input stage; z, mean, rstd, P, G null unless saved
+  void* out;                                        // output stage (y, go: its two products, null unless saved)
+  long long M;
+  int C, Ch, n_out;                                 // n_out: 2 Ch, or C
+  float eps;
+};
+
+template <typename T> constexpr bool kCanTf32 = sizeof(T) == 4;
+constexpr int kFusedMax = 256;                      // channels of a row: two float4 per lane
+
+
+template <typename T>
+__device__ __forceinline__ float4 load_four(const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    union { uint2 u; T h[4]; } v;
+    v.u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(to_f32(v.h[0]), to_f32(v.h[1]), to_f32(v.h[2]), to_f32(v.h[3]));
+  }
+}
+template <bool TF32>
+__device__ __forceinline__ float4 round_four(float4 v) {
+  if constexpr (TF32) return make_float4(round_tf32(v.x), round_tf32(v.y), round_tf32(v.z), round_tf32(v.w));
+  return v;
+}
+
+// Four rows' values at four consecutive k, transposed into a tile [K][64]: the 16-byte chunk of four rows is XORed with k / 4,
+// which keeps the lanes of a warp (consecutive k / 4) apart.
+__device__ __forceinline__ void put_transposed(float* tile, int k, int row0, const float4& v0, const float4& v1, const float4& v2, const float4& v3) {
+  float* to = tile + k * 64 + (((row0 >> 2) ^ (k >> 2 & 7)) << 2);
+  *reinterpret_cast<float4*>(to) = make_float4(v0.x, v1.x, v2.x, v3.x);
+  *reinterpret_cast<float4*>(to + 64) = make_float4(v0.y, v1.y, v2.y, v3.y);
+  *reinterpret_cast<float4*>(to + 128) = make_float4(v0.z, v1.z, v2.z, v3.z);
+  *reinterpret_cast<float4*>(to + 192) = make_float4(v0.w, v1.w, v2.w, v3.w);
+}
+
+// 64 rows of W [n_out, K] from row n0 into shared memory as [K][64], zero beyond n_out
+template <typename T, bool TF32>
+__device__ __forceinline__ void stage_weights(float* dst, const T* W, int n0, int n_out, int K) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r0 = warp * 8 + i * 4;
+    for (int k = lane * 4; k < K; k += 128) {
+      float4 v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        v[r] = round_four<TF32>(n0 + r0 + r < n_out ? load_four(W + (long long)(n0 + r0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f));
+      put_transposed(dst, k, r0, v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+// 64 rows of X [M, K] from row m0, LayerNormed, into shared memory as [K][64]; a warp has eight rows, four at a time
+template <typename TX, typename T, bool TF32>
+__device__ __forceinline__ void stage_normalised(float* dst, const TX* X, const T* gamma, const T* beta, float eps, long long m0, long long M,
+                                                 int K, float* z, float* mean, float* rstd) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i) {
+    const int r0 = warp * 8 + i * 4;
+    float4 v[4][2];
+    float s[4], mu[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      s[r] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int k = (lane + 32 * j) * 4;
+        v[r][j] = k < K && m0 + r0 + r < M ? load_four(X + (m0 + r0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        s[r] += (v[r][j].x + v[r][j].y) + (v[r][j].z + v[r][j].w);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      mu[r] = warp_sum(s[r]) / K;
+      s[r] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if ((lane + 32 * j) * 4 < K) {
+          float4& x = v[r][j];
+          x = make_float4(x.x - mu[r], x.y - mu[r], x.z - mu[r], x.w - mu[r]);
+          s[r] += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      s[r] = 1.0f / sqrtf(warp_sum(s[r]) / K + eps);
+      if (mean != nullptr && m0 + r0 + r < M && lane == 0) { mean[m0 + r0 + r] = mu[r]; rstd[m0 + r0 + r] = s[r]; }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int k = (lane + 32 * j) * 4;
+      if (k >= K) continue;
+      const float4 g = gamma ? load_four(gamma + k) : make_float4(1.f, 1.f, 1.f, 1.f), o = beta ? load_four(beta + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float4& x = v[r][j];
+        x = make_float4(x.x * s[r] * g.x + o.x, x.y * s[r] * g.y + o.y, x.z * s[r] * g.z + o.z, x.w * s[r] * g.w + o.w);
+        if (z != nullptr && m0 + r0 + r < M) *reinterpret_cast<float4*>(z + (m0 + r0 + r) * K + k) = x;
+        x = round_four<TF32>(x);
+      }
+      put_transposed(dst, k, r0, v[0][j], v[1][j], v[2][j], v[3][j]);
+    }
+  }
+}
+
+// acc[w][i][j] += A^T B[w] over k_begin .. k_end, for pixels 2 i, 2 i + 1 of the eight in chunks ch, ch + 1 of A's rows and
+// channel j of chunk cn of each of W weight blocks
+template <int W>
+__device__ __forceinline__ void dot_tile(float2 (&acc)[W][4][4], const float* A, const float* B, int K, int k_begin, int k_end, int ch, int cn) {
+#pragma unroll 1
+  for (int k4 = k_begin; k4 < k_end; k4 += 4) {
+    const int sw = k4 >> 2 & 7;
+    const float* a0 = A + k4 * 64 + ((ch ^ sw) << 2);
+    const float* a1 = A + k4 * 64 + (((ch + 1) ^ sw) << 2);
+    const float* b0 = B + k4 * 64 + ((cn ^ sw) << 2);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 x = *reinterpret_cast<const float4*>(a0 + e * 64), y = *reinterpret_cast<const float4*>(a1 + e * 64);
+      const float2 a[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), make_float2(y.z, y.w)};
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const float4 b = *reinterpret_cast<const float4*>(b0 + (w * K + e) * 64);
+        const float2 bb[4] = {make_float2(b.x, b.x), make_float2(b.y, b.y), make_float2(b.z, b.z), make_float2(b.w, b.w)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[w][i][j] = __ffma2_rn(a[i], bb[j], acc[w][i][j]);
+      }
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void store_four(T* p, float4 v) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    union { uint2 u; T h[4]; } o;
+    o.h[0] = from_f32<T>(v.x); o.h[1] = from_f32<T>(v.y); o.h[2] = from_f32<T>(v.z); o.h[3] = from_f32<T>(v.w);
+    *reinterpret_cast<uint2*>(p) = o.u;
+  }
+}
+
+// where the second half of a contraction over K starts
+__device__ __forceinline__ int split(int K) { return (K / 4 + 1) / 2 * 4; }
+
+// OUT: the output stage (first product on the LayerNormed contraction), else the input stage (both on z)
+template <typename T, bool OUT, bool TF32>
+__global__ void __launch_bounds__(256, 2) fused_kernel(const FusedP p) {
+  extern __shared__ __align__(16) float sm[];
+  const int C = p.C, K0 = OUT ? p.Ch : p.C, n0 = blockIdx.x * 64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = warp >> 2, t = threadIdx.x & 127;
+  const int ty = (warp >> 1 & 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);   // pixels 8 ty .., channels 4 tx ..
+  const bool first = blockIdx.x == 0;
+  const T *gin = static_cast<const T*>(p.norm_in_w), *bin = static_cast<const T*>(p.norm_in_b);
+  float *sW = sm, *sG = sW + 64 * K0, *sA = sG + 64 * C;
+  stage_weights<T, TF32>(sW, static_cast<const T*>(p.p_w), n0, p.n_out, K0);
+  stage_weights<T, TF32>(sG, static_cast<const T*>(p.g_w), n0, p.n_out, C);
+  const int n = n0 + 4 * tx;
+  float4 pb = make_float4(0.f, 0.f, 0.f, 0.f), gb = pb;
+  if (n < p.n_out && p.p_b) pb = load_four(static_cast<const T*>(p.p_b) + n);
+  if (n < p.n_out && p.g_b) gb = load_four(static_cast<const T*>(p.g_b) + n);
+  for (long long m0 = blockIdx.y * 64LL; m0 < p.M; m0 += gridDim.y * 64LL) {
+    float2 acc[2][4][4] = {};
+    __syncthreads();
+    if constexpr (OUT) {
+      stage_normalised<float, T, TF32>(sA, p.t, static_cast<const T*>(p.norm_out_w), static_cast<const T*>(p.norm_out_b), p.eps, m0, p.M, K0,
+                                       nullptr, first ? p.mean : nullptr, p.rstd);
+      __syncthreads();
+      dot_tile<1>(reinterpret_cast<float2(&)[1][4][4]>(acc[0]), sA, sW, K0, half ? split(K0) : 0, half ? K0 : split(K0), 2 * ty, tx);
+      __syncthreads();
+      stage_normalised<T, T, TF32>(sA, static_cast<const T*>(p.x), gin, bin, p.eps, m0, p.M, C, nullptr, nullptr, nullptr);
+      __syncthreads();
+      dot_tile<1>(reinterpret_cast<float2(&)[1][4][4]>(acc[1]), sA, sG, C, half ? split(C) : 0, half ? C : split(C), 2 * ty, tx);
+    } else {
+      stage_normalised<T, T, TF32>(sA, static_cast<const T*>(p.x), gin, bin, p.eps, m0, p.M, C, first ? p.z : nullptr, first ? p.mean : nullptr,
+                                   p.rstd);
+      __syncthreads();
+      dot_tile<2>(acc, sA, sW, C, half ? split(C) : 0, half ? C : split(C), 2 * ty, tx);
+    }
+    // each half keeps four of the eight pixels: it hands the other four's sums over through the row tile
+    __syncthreads();
+    float2* swap = reinterpret_cast<float2*>(sA);
+#pragma unroll
+    for (int x = 0; x < 16; ++x) swap[(half * 16 + x) * 128 + t] = half ? acc[x >> 3][x >> 2 & 1][x & 3] : acc[x >> 3][2 + (x >> 2 & 1)][x & 3];
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < 16; ++x) {
+      const float2 o = swap[((half ^ 1) * 16 + x) * 128 + t];
+      float2& mine = acc[x >> 3][x >> 2 & 1][x & 3];
+      const float2 own = half ? acc[x >> 3][2 + (x >> 2 & 1)][x & 3] : mine;
+      mine = half ? __fadd2_rn(o, own) : __fadd2_rn(own, o);
+    }
+    if (n >= p.n_out) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const long long m = m0 + 8 * ty + 4 * half + i, at = m * p.n_out + n;
+      if (m >= p.M) continue;
+      float a[4], b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        a[j] = i & 1 ? acc[0][i >> 1][j].y : acc[0][i >> 1][j].x;
+        b[j] = i & 1 ? acc[1][i >> 1][j].y : acc[1][i >> 1][j].x;
+      }
+      const float4 v = make_float4(a[0] + pb.x, a[1] + pb.y, a[2] + pb.z, a[3] + pb.w), g = make_float4(b[0] + gb.x, b[1] + gb.y, b[2] + gb.z, b[3] + gb.w);
+      if (p.P != nullptr) { store_four(p.P + at, v); store_four(p.G + at, g); }
+      const float keep = !OUT && p.mask ? to_f32(static_cast<const T*>(p.mask)[m]) : 1.f;
+      const float4 r = make_float4(v.x * sigmoidf_acc(g.x) * keep, v.y * sigmoidf_acc(g.y) * keep, v.z * sigmoidf_acc(g.z) * keep, v.w * sigmoidf_acc(g.w) * keep);
+      if constexpr (OUT) store_four(static_cast<T*>(p.out) + at, r);
+      else store_four(p.ab + at, r);
+    }
+  }
+}
+
+// Rows of up to 256 channels in whole 16-byte pieces; wider or odd ones go through one stage per kernel.
+template <typename T>
+static bool fused_fits(const TriMulDesc* d, const void* x, const TriMulWeights* w, void* out) {
+  const size_t v = 4 * sizeof(T);
+  for (const void* p : {x, static_cast<const void*>(out), w->p_in_b, w->g_in_b, w->p_out_b, w->g_out_b, w->norm_in_w, w->norm_in_b, w->p_in_w, w->g_in_w, w->norm_out_w, w->norm_out_b, w->p_out_w, w->g_out_w})
+    if (reinterpret_cast<uintptr_t>(p) % v != 0) return false;
+  return d->C % 4 == 0 && d->Ch % 4 == 0 && d->C <= kFusedMax && d->Ch <= kFusedMax;
+}
+
+template <typename T, bool OUT>
+static int fused_start(const FusedP& p, bool tf32, cudaStream_t st) {
+  const auto kern = tf32 ? fused_kernel<T, OUT, kCanTf32<T>> : fused_kernel<T, OUT, false>;
+  const int rows = std::max(128, OUT ? std::max(p.C, p.Ch) : p.C);   // the row tile, at least as large as the halves' exchange
+  const size_t smem = (size_t)64 * sizeof(float) * ((OUT ? p.C + p.Ch : 2 * p.C) + rows);
+  TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const double M = (double)p.M;
+  KernelTimer kt(OUT ? "simt_fused_out" : "simt_fused_in", st, 2.0 * M * p.n_out * (p.C + (OUT ? p.Ch : p.C)),
+                 OUT ? M * (2.0 * p.C * sizeof(T) + 4.0 * p.Ch) : M * (p.C * sizeof(T) + 8.0 * p.Ch));
+  const int blocks = cdiv(p.n_out, 64), room = std::max(1, (smem <= 113 * 1024 ? 2 : 1) * sm_count() / blocks);
+  kern<<<dim3(blocks, (unsigned)std::min<long long>((p.M + 63) / 64, room)), 256, smem, st>>>(p);
+  TRI_LAUNCH_OK();
+  return 0;
+}
+
 template <typename T>
 static int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out,
                      void* saved, void* ws, size_t ws_size, cudaStream_t st) {
@@ -486,19 +826,29 @@ static int forward_t(const TriMulDesc* d, const void* x, const void* mask, const
   if (saved) { Arena sa(saved, saved_bytes(d)); carve_saved(sa, d, &s); }
   else carve_saved(a, d, &s);
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
-  TRI_TRY(convert_weights<T>(st, d, w, mask, &f));
+  const bool fused = fused_fits<T>(d, x, w, out);
+  FusedP fp{};
+  if (fused) {
+    fp.x = x; fp.mask = mask; fp.norm_in_w = w->norm_in_w; fp.norm_in_b = w->norm_in_b; fp.norm_out_w = w->norm_out_w; fp.norm_out_b = w->norm_out_b;
+    fp.p_w = w->p_in_w; fp.p_b = w->p_in_b; fp.g_w = w->g_in_w; fp.g_b = w->g_in_b;
+    fp.M = M; fp.C = C; fp.Ch = Ch; fp.n_out = 2 * Ch; fp.eps = d->eps; fp.ab = s.ab;
+    if (saved) { fp.z = s.z; fp.mean = s.mean_in; fp.rstd = s.rstd_in; fp.P = s.P; fp.G = s.G; }
+    TRI_TRY((fused_start<T, false>(fp, tf32, st)));
+  } else {
+    TRI_TRY(convert_weights<T>(st, d, w, mask, &f));
 
-  {
-    KernelTimer kt("simt_ln_fwd", st, 0.0, (double)M * C * (sizeof(T) + 4.0));
-    ln_fwd_kernel<T><<<cdiv(M, 8), 256, 0, st>>>((const T*)x, f.norm_in_w, f.norm_in_b, d->eps, M, C, s.z, s.mean_in, s.rstd_in);
-    TRI_LAUNCH_OK();
-  }
-  TRI_TRY(gemm(st, tf32, linear_p(s.z, C, f.p_in_w, f.p_in_b, s.P, 2 * Ch, M, 2 * Ch, C)));
-  TRI_TRY(gemm(st, tf32, linear_p(s.z, C, f.g_in_w, f.g_in_b, s.G, 2 * Ch, M, 2 * Ch, C)));
-  {
-    KernelTimer kt("simt_gate_in", st, 0.0, 24.0 * M * Ch);
-    gate_in_kernel<<<EW_GRID(M * 2 * Ch)>>>(s.P, s.G, f.mask, M, 2 * Ch, s.ab);
-    TRI_LAUNCH_OK();
+    {
+      KernelTimer kt("simt_ln_fwd", st, 0.0, (double)M * C * (sizeof(T) + 4.0));
+      ln_fwd_kernel<T><<<cdiv(M, 8), 256, 0, st>>>((const T*)x, f.norm_in_w, f.norm_in_b, d->eps, M, C, s.z, s.mean_in, s.rstd_in);
+      TRI_LAUNCH_OK();
+    }
+    TRI_TRY(gemm(st, tf32, linear_p(s.z, C, f.p_in_w, f.p_in_b, s.P, 2 * Ch, M, 2 * Ch, C)));
+    TRI_TRY(gemm(st, tf32, linear_p(s.z, C, f.g_in_w, f.g_in_b, s.G, 2 * Ch, M, 2 * Ch, C)));
+    {
+      KernelTimer kt("simt_gate_in", st, 0.0, 24.0 * M * Ch);
+      gate_in_kernel<<<EW_GRID(M * 2 * Ch)>>>(s.P, s.G, f.mask, M, 2 * Ch, s.ab);
+      TRI_LAUNCH_OK();
+    }
   }
   ContractP cp{};
   cp.X = s.ab; cp.Y = s.ab; cp.O = s.t; cp.N = N; cp.Ch = Ch;
@@ -507,6 +857,12 @@ static int forward_t(const TriMulDesc* d, const void* x, const void* mask, const
   if (d->direction == TRI_OUTGOING) { cp.xs_p = N; cp.xs_r = 1; cp.ys_q = N; cp.ys_r = 1; }
   else { cp.xs_p = 1; cp.xs_r = N; cp.ys_q = 1; cp.ys_r = N; }
   TRI_TRY(contract(st, tf32, d->B, cp));
+  if (fused) {
+    fp.p_w = w->p_out_w; fp.p_b = w->p_out_b; fp.g_w = w->g_out_w; fp.g_b = w->g_out_b; fp.n_out = C; fp.t = s.t; fp.out = out;
+    if (saved) { fp.mean = s.mean_out; fp.rstd = s.rstd_out; fp.P = s.y; fp.G = s.go; }
+    fp.ab = nullptr; fp.z = nullptr;
+    return fused_start<T, true>(fp, tf32, st);
+  }
   // LayerNormed contraction output: P is dead by now in inference, so it doubles as scratch there;
   // with a saved block P must survive, and the workspace region that would have held it is free.
   float* u_buf = saved ? a.take<float>((size_t)M * Ch) : s.P;
