@@ -221,6 +221,12 @@ int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z
   return tc::attn_project_bias(d, plane, z, ln_w, ln_b, w_bias, bias, ws, (cudaStream_t)stream);
 }
 
+int tri_gate_mul(int dtype, int64_t n, const void* a, const void* gate, void* out, tri_stream_t stream) {
+  if (dtype < TRI_F32 || dtype > TRI_F16) return fail(TRI_ERR_ARG, "bad dtype %d", dtype);
+  if (n < 0 || (n > 0 && (!a || !gate || !out))) return fail(TRI_ERR_ARG, "a, gate and out must not be null");
+  return n == 0 ? 0 : tc::gate_mul(dtype, n, a, gate, out, (cudaStream_t)stream);
+}
+
 size_t tri_mul_saved_bytes(const TriMulDesc* d) {
   if (check_mul(d) != 0) return 0;
   return tc::mul_supported(d) ? tc::mul_saved_bytes(d) : simt::saved_bytes(d);

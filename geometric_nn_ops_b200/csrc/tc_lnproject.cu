@@ -28,10 +28,11 @@ constexpr int kTile = 2 * kSub;             // 128 x 128 16-bit values
 constexpr int kHeads = 16;                  // columns of the heads' product
 constexpr int kHTile = 2 * kHeads * 128;    // their weights: two 64-channel halves
 constexpr uint32_t kHCol = 384;             // their TMEM columns
+constexpr int kMaxStages = 5;               // z tiles in flight
 
 struct Args {
   long long M;
-  int tiles, blocks, heads;
+  int tiles, blocks, heads, stages;
   long long plane;       // pixels per batch entry of the head-major output
   float eps;
   const void* gamma;
@@ -40,6 +41,10 @@ struct Args {
   int* err;
 };
 
+__device__ __forceinline__ void next_stage(int& b, uint32_t& phase, int stages) {
+  if (++b == stages) { b = 0; phase ^= 1; }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmW,
@@ -47,26 +52,27 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
   constexpr int KIND = ElemTraits<T>::kind;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint8_t* sZ = smem;                       // [2] z tiles
-  uint8_t* sH = sZ + 2 * kTile;
+  uint8_t* sZ = smem;                       // [stages] z tiles
+  uint8_t* sH = sZ + g.stages * kTile;
   uint8_t* sO = sH + kHTile;                // an output block, if there are any
   uint8_t* sW = sO + (g.blocks > 0 ? kTile : 0);
   T* s_gamma = reinterpret_cast<T*>(sW + g.blocks * kTile);
   T* s_beta = s_gamma + 128;
   uint64_t* wfull = reinterpret_cast<uint64_t*>(s_beta + 128);
-  uint64_t* zfull = wfull + 1;              // [2] tile landed
-  uint64_t* znorm = zfull + 2;              // [2] tile normalised (8 warps)
-  uint64_t* zempty = znorm + 2;             // [2] the tile's products are done
-  uint64_t* tfull = zempty + 2;             // [4] block complete (3: heads)
+  uint64_t* zfull = wfull + 1;              // [stages] tile landed
+  uint64_t* znorm = zfull + kMaxStages;     // [stages] tile normalised (8 warps)
+  uint64_t* zempty = znorm + kMaxStages;    // [stages] the tile's products are done
+  uint64_t* tfull = zempty + kMaxStages;    // [4] block complete (3: heads)
   uint64_t* tempty = tfull + 4;             // [4] block read (8 warps; heads: 4)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(wfull, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(&zfull[b], 1); mbar_init(&znorm[b], 8); mbar_init(&zempty[b], 1); }
+    for (int b = 0; b < g.stages; ++b) { mbar_init(&zfull[b], 1); mbar_init(&znorm[b], 8); mbar_init(&zempty[b], 1); }
     for (int b = 0; b < 4; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], b < 3 ? 8 : 4); }
     mbar_fence_init();
+    if (blockIdx.x == 0) *g.err = 0;        // a wait gives up seconds after this
   }
   if (threadIdx.x < 128) {
     s_gamma[threadIdx.x] = g.gamma ? reinterpret_cast<const T*>(g.gamma)[threadIdx.x] : from_f32<T>(1.f);
@@ -86,10 +92,10 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         tma_load_3d(sH + kb * (kHTile / 2), &tmH, wfull, kb * 64, 0, 0);
         for (int blk = 0; blk < g.blocks; ++blk) tma_load_3d(sW + blk * kTile + kb * kSub, &tmW, wfull, kb * 64, blk * 128, 0);
       }
-      int i = 0;
-      for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
-        const int b = i & 1;
-        if (!mbar_wait(&zempty[b], ((i >> 1) & 1) ^ 1, g.err, 70)) break;
+      int b = 0;
+      uint32_t ph = 0;
+      for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, next_stage(b, ph, g.stages)) {
+        if (!mbar_wait(&zempty[b], ph ^ 1, g.err, 70)) break;
         mbar_expect_tx(&zfull[b], kTile);
         for (int kb = 0; kb < 2; ++kb) tma_load_3d(sZ + b * kTile + kb * kSub, &tmZ, &zfull[b], kb * 64, tile * 128, 0);
       }
@@ -101,10 +107,10 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
       const uint32_t idesc = make_idesc(KIND, 128, 128, false, false), idesc_h = make_idesc(KIND, 128, kHeads, false, false);
       const uint32_t z_base = smem_u32(sZ), w_base = smem_u32(sW), h_base = smem_u32(sH);
       bool ok = mbar_wait(wfull, 0, g.err, 71);
-      int i = 0;
-      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
-        const int b = i & 1;
-        if (!mbar_wait(&znorm[b], (i >> 1) & 1, g.err, 72)) break;
+      int i = 0, b = 0;
+      uint32_t ph = 0;
+      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i, next_stage(b, ph, g.stages)) {
+        if (!mbar_wait(&znorm[b], ph, g.err, 72)) break;
         for (int n = 0; n <= g.blocks && ok; ++n) {
           const int blk = n < g.blocks ? n : 3;
           if (!mbar_wait(&tempty[blk], (i & 1) ^ 1, g.err, 73)) { ok = false; break; }
@@ -133,42 +139,36 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     const uint32_t sw = (uint32_t)((r & 7) ^ (half << 2)) << 4;
     const T* gam = s_gamma + half * 64;
     const T* bet = s_beta + half * 64;
-    int i = 0;
-    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
-      const int b = i & 1;
-      const bool landed = mbar_wait(&zfull[b], (i >> 1) & 1, g.err, 74);
+    const bool shifted = g.beta != nullptr;
+    int b = 0;
+    uint32_t ph = 0;
+    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, next_stage(b, ph, g.stages)) {
+      const bool landed = mbar_wait(&zfull[b], ph, g.err, 74);
       if (!__all_sync(0xffffffffu, landed)) break;
       const uint32_t rowp = smem_u32(sZ + b * kTile + half * kSub + r * 128);
       auto unpack = [](const uint4& w, float2 (&v)[4]) {
         v[0] = unpack2<T>(w.x); v[1] = unpack2<T>(w.y); v[2] = unpack2<T>(w.z); v[3] = unpack2<T>(w.w);
       };
-      // the half row stays packed in registers: mean, then the squares about it, then the result
-      uint4 w[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) w[c] = lds128(rowp + ((c << 4) ^ sw));
-      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+      // the half row stays in registers: mean, then the squares about it, then the result
+      float2 v[8][4], s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        float2 v[4];
-        unpack(w[c], v);
-        s0 = __fadd2_rn(s0, __fadd2_rn(v[0], v[1]));
-        s1 = __fadd2_rn(s1, __fadd2_rn(v[2], v[3]));
+        unpack(lds128(rowp + ((c << 4) ^ sw)), v[c]);
+        s0 = __fadd2_rn(s0, __fadd2_rn(v[c][0], v[c][1]));
+        s1 = __fadd2_rn(s1, __fadd2_rn(v[c][2], v[c][3]));
       }
       float mu = (s0.x + s0.y) + (s1.x + s1.y);
       mu = (mu + __shfl_xor_sync(0xffffffffu, mu, 1)) * (1.0f / 128);
       const float2 nmu = make_float2(-mu, -mu);
       s0 = s1 = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float2 v[4];
-        unpack(w[c], v);
+      for (int c = 0; c < 8; ++c)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          v[e] = __fadd2_rn(v[e], nmu);
-          if (e & 1) s1 = __ffma2_rn(v[e], v[e], s1);
-          else s0 = __ffma2_rn(v[e], v[e], s0);
+          v[c][e] = __fadd2_rn(v[c][e], nmu);
+          if (e & 1) s1 = __ffma2_rn(v[c][e], v[c][e], s1);
+          else s0 = __ffma2_rn(v[c][e], v[c][e], s0);
         }
-      }
       float var = (s0.x + s0.y) + (s1.x + s1.y);
       var = (var + __shfl_xor_sync(0xffffffffu, var, 1)) * (1.0f / 128);
       const float rs = 1.0f / sqrtf(var + g.eps);
@@ -176,17 +176,18 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int ch = (c ^ (half << 2)) * 8;
-        float2 v[4], gm[4], bt[4];
-        unpack(w[c], v);
+        float2 gm[4];
         unpack(*reinterpret_cast<const uint4*>(gam + ch), gm);
-        unpack(*reinterpret_cast<const uint4*>(bet + ch), bt);
-        uint32_t o[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 y = __ffma2_rn(__fmul2_rn(__fadd2_rn(v[e], nmu), rs2), gm[e], bt[e]);
-          o[e] = pack2<T>(y.x, y.y);
+        for (int e = 0; e < 4; ++e) v[c][e] = __fmul2_rn(__fmul2_rn(v[c][e], rs2), gm[e]);
+        if (shifted) {
+          float2 bt[4];
+          unpack(*reinterpret_cast<const uint4*>(bet + ch), bt);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[c][e] = __fadd2_rn(v[c][e], bt[e]);
         }
-        sts128(rowp + ((c << 4) ^ sw), o[0], o[1], o[2], o[3]);
+        sts128(rowp + ((c << 4) ^ sw), pack2<T>(v[c][0].x, v[c][0].y), pack2<T>(v[c][1].x, v[c][1].y), pack2<T>(v[c][2].x, v[c][2].y),
+               pack2<T>(v[c][3].x, v[c][3].y));
       }
       fence_proxy_async_smem();   // the tile is read next by tcgen05.mma
       __syncwarp();
@@ -277,7 +278,9 @@ int launch(cudaStream_t st, const LnProject& p) {
     TRI_TRY(make_tmap_3d(&tw, p.w_qkv, 2, f16, wd, ws, box, false));
     TRI_TRY(make_tmap_3d(&to, p.qkv, 2, f16, od, os, box, false));
   }
-  const size_t smem = 1024 + 2 * kTile + kHTile + (a.blocks > 0 ? (1 + a.blocks) * kTile : 0) + 512 + 16 * 8;
+  // Two z tiles beside 96 KB of weights; five without, to cover the latency of DRAM.
+  a.stages = a.blocks > 0 ? 2 : kMaxStages;
+  const size_t smem = 1024 + a.stages * kTile + kHTile + (a.blocks > 0 ? (1 + a.blocks) * kTile : 0) + 512 + (2 + 3 * kMaxStages + 8) * 8;
   auto kern = ln_project_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const double unit = 256.0 * p.M;

@@ -39,6 +39,7 @@ struct Api {
   decltype(&tri_attn_fwd) attn_fwd;
   decltype(&tri_attn_bwd) attn_bwd;
   decltype(&tri_attn_project_bias) attn_project_bias;
+  decltype(&tri_gate_mul) gate_mul;
   decltype(&tri_mul_saved_bytes) mul_saved_bytes;
   decltype(&tri_mul_ws_bytes) mul_ws_bytes;
   decltype(&tri_mul_fwd) mul_fwd;
@@ -54,7 +55,7 @@ void bind(const std::string& path) {
   };
   get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
   get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
-  get(api.attn_project_bias, "tri_attn_project_bias");
+  get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul");
   get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
   get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
 }
@@ -126,14 +127,15 @@ TriAttnDesc attn_desc(const Tensor& q, const Tensor& k, const Tensor& v, const T
 struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, S, N]
 
 // q, k, v [B, S, N, H, D], bias [B, 1, H, N, N], mask [B, S, 1, 1, N]
+// (`rows`: o contiguous in that order of axes, else laid out like q)
 AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias_, const Tensor& mask_, double scale,
-                      int64_t precision) {
+                      int64_t precision, bool rows) {
   AttnCall c;
   c.q = inner_contiguous(q_); c.k = inner_contiguous(k_); c.v = inner_contiguous(v_);
   if (bias_.defined()) c.bias = inner_contiguous(bias_);
   const int64_t B = c.q.size(0), S = c.q.size(1), N = c.q.size(2), H = c.q.size(3);
   if (mask_.defined()) c.mask = mask_.reshape({B, S, N}).contiguous();
-  c.o = like(c.q);
+  c.o = rows ? at::empty(c.q.sizes(), c.q.options()) : like(c.q);
   c.stats = at::empty({2, B, S, H, N}, c.q.options().dtype(at::kFloat));
   const TriAttnDesc d = attn_desc(c.q, c.k, c.v, c.o, c.bias, c.mask, scale, precision);
   const c10::cuda::CUDAGuard guard(c.q.device());
@@ -152,8 +154,8 @@ Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); 
 
 struct AttnFn : torch::autograd::Function<AttnFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& bias,
-                               const OptTensor& mask, double scale, int64_t precision) {
-    const AttnCall c = attn_forward(q, k, v, or_undefined(bias), or_undefined(mask), scale, precision);
+                               const OptTensor& mask, double scale, int64_t precision, bool rows) {
+    const AttnCall c = attn_forward(q, k, v, or_undefined(bias), or_undefined(mask), scale, precision, rows);
     ctx->save_for_backward({c.q, c.k, c.v, c.bias, c.mask, c.o, c.stats});
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["precision"] = precision;
@@ -178,7 +180,7 @@ struct AttnFn : torch::autograd::Function<AttnFn> {
                     ptr(ws), n, st), "tri_attn_bwd");
     check_device(ws, reinterpret_cast<cudaStream_t>(st));
     if (dbias.defined()) dbias = dbias.to(bias.scalar_type()).view({B, 1, H, N, N});
-    return {dq, dk, dv, dbias, Tensor(), Tensor(), Tensor()};
+    return {dq, dk, dv, dbias, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -191,6 +193,17 @@ Tensor rank5(const Tensor& t) {
     return t.reshape(s);
   }
   return t.reshape({-1, s[s.size() - 4], s[s.size() - 3], s[s.size() - 2], s[s.size() - 1]});
+}
+
+// o and the statistics, recorded for the backward where a gradient is wanted
+std::pair<Tensor, Tensor> attn_any(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias, const Tensor& mask, double scale,
+                                   int64_t precision, bool rows) {
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()))) {
+    const variable_list r = AttnFn::apply(q, k, v, opt(bias), opt(mask), scale, precision, rows);
+    return {r[0], r[1]};
+  }
+  const AttnCall c = attn_forward(q, k, v, bias, mask, scale, precision, rows);
+  return {c.o, c.stats};
 }
 
 py::object attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& bias_, const OptTensor& mask_,
@@ -216,14 +229,7 @@ py::object attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
     mask = mask.expand({B, S, 1, 1, N});
   }
   const double scale = scale_.has_value() ? *scale_ : 1.0 / std::sqrt((double)q.size(4));
-  Tensor o, stats;
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()))) {
-    const variable_list r = AttnFn::apply(q, k, v, opt(bias), opt(mask), scale, precision);
-    o = r[0]; stats = r[1];
-  } else {
-    const AttnCall c = attn_forward(q, k, v, bias, mask, scale, precision);
-    o = c.o; stats = c.stats;
-  }
+  auto [o, stats] = attn_any(q, k, v, bias, mask, scale, precision, false);
   if (!canonical) o = o.reshape(q_.sizes());
   if (!return_aux) return py::cast(o);
   const Tensor m = stats.select(0, 0);
@@ -377,25 +383,56 @@ Tensor multiplicative_update(const Tensor& x, const OptTensor& mask_, bool outgo
 
 // ---------------------------------------------------------------------------------------------------- pair bias
 
-// z [B, U, V, 128] -> LayerNorm (weight only) -> projection to H <= 16 heads -> [B, H, U, V], without gradients; None where
-// the kernel does not take the call (mixed or other types, other channel counts, gradients or autocast in force)
-py::object pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
+// z [B, U, V, Zc] -> LayerNorm (weight only) -> projection to H heads -> [B, H, U, V].  One kernel where it has the shape (16-bit
+// types, 128 channels, at most 16 heads) and neither gradients nor autocast are in force, else torch's operations.
+bool pair_bias_fits(const Tensor& z, const OptTensor& ln_w, const Tensor& w) {
   const auto dt = z.scalar_type();
   const bool fits = z.is_cuda() && z.dim() == 4 && (dt == at::kBFloat16 || dt == at::kHalf) && z.size(3) == 128 && w.dim() == 2 &&
                     w.size(1) == 128 && w.size(0) >= 1 && w.size(0) <= 16 && w.scalar_type() == dt && w.device() == z.device() &&
                     (!ln_w.has_value() || (ln_w->scalar_type() == dt && ln_w->dim() == 1 && ln_w->size(0) == 128 && ln_w->device() == z.device()));
   const bool grad = at::GradMode::is_enabled() && (z.requires_grad() || w.requires_grad() || (ln_w.has_value() && ln_w->requires_grad()));
-  const int64_t plane = z.dim() == 4 ? z.size(1) * z.size(2) : 0, M = fits ? z.size(0) * plane : 0;
-  if (!fits || grad || M < 1 || M >= (1LL << 31) - 128 || at::autocast::is_autocast_enabled(at::kCUDA)) return py::none();
+  return fits && !grad && z.numel() >= 128 && z.numel() / 128 < (1LL << 31) - 128 && !at::autocast::is_autocast_enabled(at::kCUDA);
+}
+Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
+  if (!pair_bias_fits(z, ln_w, w))
+    return at::linear(at::layer_norm(z, {z.size(-1)}, ln_w, {}, eps), w).permute({0, 3, 1, 2}).contiguous();
   TriAttnProjDesc d{};
-  d.M = M; d.C = 128; d.H = (int32_t)w.size(0); d.dtype = dtype_code(z); d.eps = (float)eps;
+  d.M = z.numel() / 128; d.C = 128; d.H = (int32_t)w.size(0); d.dtype = dtype_code(z); d.eps = (float)eps;
   const c10::cuda::CUDAGuard guard(z.device());
   const Tensor zc = aligned(z), wc = aligned(w), lw = ln_w.has_value() ? ln_w->contiguous() : Tensor(), ws = bytes(256, z);
   const Tensor out = at::empty({z.size(0), w.size(0), z.size(1), z.size(2)}, z.options());
   const tri_stream_t st = stream_of(z);
-  ok(api.attn_project_bias(&d, plane, ptr(zc), ptr(lw), nullptr, ptr(wc), ptr(out), ptr(ws), st), "tri_attn_project_bias");
+  ok(api.attn_project_bias(&d, z.size(1) * z.size(2), ptr(zc), ptr(lw), nullptr, ptr(wc), ptr(out), ptr(ws), st), "tri_attn_project_bias");
   check_device(ws, reinterpret_cast<cudaStream_t>(st));
-  return py::cast(out);
+  return out;
+}
+
+// o * sigmoid(gate)
+Tensor gated(const Tensor& o, const Tensor& gate) {
+  const bool grad = at::GradMode::is_enabled() && (o.requires_grad() || gate.requires_grad());
+  if (grad || !o.is_contiguous() || !gate.is_contiguous() || o.scalar_type() != gate.scalar_type() || o.sizes() != gate.sizes())
+    return o * at::sigmoid(gate);
+  const c10::cuda::CUDAGuard guard(o.device());
+  const Tensor out = at::empty(o.sizes(), o.options());
+  ok(api.gate_mul(dtype_code(o), o.numel(), ptr(o), ptr(gate), ptr(out), stream_of(o)), "tri_gate_mul");
+  return out;
+}
+
+// The whole of attention_pair_bias where its softmax core runs on the kernels (the Python function decides); returns the
+// output and the projected bias.  About fifteen torch calls, which took 100 us from Python and whose kernels take a third of that.
+std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& z,
+                                              const Tensor& g_w, const OptTensor& g_b, const Tensor& o_w, const OptTensor& o_b,
+                                              const OptTensor& z_w, const OptTensor& ln_w, const OptTensor& mask_, double scale, double eps,
+                                              int64_t precision) {
+  const int64_t BM = q.size(0), H = q.size(1), U = q.size(2), D = q.size(3), B = z.size(0), M = BM / B;
+  const Tensor pz = z_w.has_value() ? pair_bias(z, ln_w, *z_w, eps) : z;
+  // (BM, H, U, D) -> rows = multiplicity: [B, M, U, H, D] as a strided view (no copy)
+  auto rows = [&](const Tensor& t) { return inner_contiguous(t.reshape({B, M, H, U, D}).transpose(2, 3)); };
+  Tensor mask;
+  if (mask_.has_value()) mask = at::ne(*mask_, 0).reshape({B, -1, 1, 1, U}).expand({B, M, 1, 1, U});
+  const Tensor bias = (pz.scalar_type() == q.scalar_type() ? pz : pz.to(q.scalar_type())).unsqueeze(1).expand({B, 1, H, U, U});
+  const Tensor o = attn_any(rows(q), rows(k), rows(v), bias, mask, scale, precision, true).first.reshape({BM, U, H * D}).to(s.scalar_type());
+  return {at::linear(gated(o, at::linear(s, g_w, g_b)), o_w, o_b), pz};
 }
 
 }  // namespace
@@ -405,4 +442,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention", &attention);
   m.def("multiplicative_update", &multiplicative_update);
   m.def("pair_bias", &pair_bias);
+  m.def("pair_bias_fits", &pair_bias_fits);
+  m.def("attention_pair_bias", &attention_pair_bias);
 }

@@ -11,24 +11,20 @@ Viewed as triangle attention, a batch entry is ``B``, the multiplicity ``M`` (th
 share a batch entry) is the row axis, and the per-head bias ``(B, H, U, V)`` is the pair bias shared by all
 rows.  Every other case (cross attention with U != V, an explicit ``inf`` other than the dtype's sentinel, CPU
 tensors, fp64) is evaluated with the same torch operations the reference uses, on whatever device the tensors
-live.  The LayerNorm and projection of ``z`` before the core, and the gate and output projection after it, are
-torch operations in both cases.
+live.  Around the core, the gate and output projections are torch linears; the LayerNorm and projection of ``z``
+and the gating are kernels of this package where no gradient is recorded and they have the shape.
 """
 
 import torch
 import torch.nn.functional as F
 
-from .. import _lib
+from .. import _lib, _precision
 from ._masking import mask_val
-from ._triattn import _DTYPES, triangle_attention_b200
+from ._triattn import _DTYPES
 
 
 def _pair_bias(z, ln_z_weight, proj_z_weight, eps):
     """``(B, U, V, Zc)`` -> LayerNorm (weight only) -> ``Zc -> H`` projection -> ``(B, H, U, V)`` contiguous."""
-    if z.is_cuda:   # one kernel where no gradient is recorded and it has the shape (16-bit types, 128 channels, H <= 16)
-        pz = _lib.host().pair_bias(z, ln_z_weight, proj_z_weight, eps)
-        if pz is not None:
-            return pz
     zn = F.layer_norm(z, z.shape[-1:], ln_z_weight, None, eps)
     return F.linear(zn, proj_z_weight).permute(0, 3, 1, 2).contiguous()
 
@@ -43,17 +39,6 @@ def _core_torch(q, k, v, pz, mask, scale, inf, B, M):
         sentinel = mask_val(logits.dtype) if inf is None else inf
         logits = logits + (keep.to(logits.dtype) - 1.0) * sentinel
     return torch.matmul(torch.softmax(logits, dim=-1), vm).reshape(BM, H, U, DH)
-
-
-def _core_kernel(q, k, v, pz, mask, scale, B, M):
-    BM, H, U, DH = q.shape
-    # (BM, H, U, DH) -> rows = multiplicity: [B, M, U, H, DH] as a strided view (no copy)
-    as_rows = lambda t: t.reshape(B, M, H, U, DH).transpose(2, 3)  # noqa: E731
-    keep = None
-    if mask is not None:
-        keep = (mask != 0).reshape(B, -1, 1, 1, U).expand(B, M, 1, 1, U)
-    o = triangle_attention_b200(as_rows(q), as_rows(k), as_rows(v), pz.unsqueeze(1), keep, scale)
-    return o.transpose(2, 3).reshape(BM, H, U, DH)
 
 
 def attention_pair_bias(s, q, k, v, z, *, proj_g_weight, proj_o_weight, proj_z_weight=None, ln_z_weight=None,
@@ -82,14 +67,16 @@ def attention_pair_bias(s, q, k, v, z, *, proj_g_weight, proj_o_weight, proj_z_w
         raise ValueError(f"mask batch {mask.shape[0]} must be B={B} or BM={BM}")
     if scale is None:
         scale = DH ** -0.5
-    pz = z if z_is_projected else _pair_bias(z, ln_z_weight, proj_z_weight, eps)
-
     on_kernel = (q.is_cuda and U == V and q.dtype in _DTYPES and k.dtype == q.dtype and v.dtype == q.dtype
                  and DH <= 128 and (inf is None or float(inf) == mask_val(q.dtype)))
     if on_kernel:
-        o = _core_kernel(q, k, v, pz.to(q.dtype), mask, float(scale), B, M)
-    else:
-        o = _core_torch(q, k, v, pz, mask, scale, inf, B, M)
+        precision = _precision.matmul_precision(fp32_operands=q.dtype == torch.float32)
+        out, pz = _lib.host().attention_pair_bias(
+            s, q, k, v, z, proj_g_weight, proj_g_bias, proj_o_weight, proj_o_bias, None if z_is_projected else proj_z_weight, ln_z_weight,
+            mask, float(scale), float(eps), _lib.PREC_TF32 if precision == _precision.TF32 else _lib.PREC_IEEE)
+        return out, (pz if return_z_proj else None)
+    pz = z if z_is_projected else _pair_bias(z, ln_z_weight, proj_z_weight, eps)
+    o = _core_torch(q, k, v, pz, mask, scale, inf, B, M)
     o = o.transpose(1, 2).reshape(BM, U, H * DH).to(s.dtype)
     gate = torch.sigmoid(F.linear(s, proj_g_weight, proj_g_bias))
     out = F.linear(o * gate, proj_o_weight, proj_o_bias)

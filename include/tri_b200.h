@@ -144,6 +144,9 @@ int tri_attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w /
 int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z, const void* ln_w /*nullable*/,
                           const void* ln_b /*nullable*/, const void* w_bias, void* bias, void* ws, tri_stream_t stream);
 
+/* out[i] = a[i] * sigmoid(gate[i]), i < n, in `dtype` (fp32 arithmetic). */
+int tri_gate_mul(int dtype, int64_t n, const void* a, const void* gate, void* out, tri_stream_t stream);
+
 /* ------------------------------------------------------------------------ */
 /* Triangle multiplicative update                                           */
 /* ------------------------------------------------------------------------ */

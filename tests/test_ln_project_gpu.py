@@ -51,6 +51,23 @@ def test_projection(H, D, pixels):
 def test_pair_bias_leaves_other_calls_to_torch():
     from geometric_nn_ops_b200 import _lib
     z, ln, w, _ = _operands(1, 4, 4, 4, 0, torch.bfloat16, 0)
-    f = _lib.host().pair_bias
-    assert f(z.float(), ln.float(), w.float(), 1e-5) is None and f(z, ln, w.requires_grad_(), 1e-5) is None
-    assert f(z[..., :64].contiguous(), ln[:64], w.detach()[:, :64], 1e-5) is None
+    fits = _lib.host().pair_bias_fits
+    assert fits(z, ln, w) and fits(z, None, w)
+    assert not fits(z.float(), ln.float(), w.float()) and not fits(z, ln, w.requires_grad_())
+    assert not fits(z[..., :64].contiguous(), ln[:64], w.detach()[:, :64])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=str)
+@pytest.mark.parametrize("n,offset", [(1, 0), (7, 0), (2048, 0), (5000, 0), (4096, 1)])
+def test_gate_mul(n, offset, dtype):
+    import ctypes
+
+    from geometric_nn_ops_b200 import _lib
+    g = torch.Generator().manual_seed(n)
+    a, gate = ((torch.randn(n + offset, generator=g) * 3).to(dtype).cuda()[offset:] for _ in range(2))
+    out = torch.full((n + 8,), 7.0, dtype=dtype, device="cuda")
+    code = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}[dtype]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(_lib.load().tri_gate_mul(code, n, p(a), p(gate), p(out), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "tri_gate_mul")
+    want = (a.float() * torch.sigmoid(gate.float())).to(dtype)
+    assert torch.allclose(out[:n].float(), want.float(), rtol=1e-6 if dtype == torch.float32 else 8e-3, atol=1e-6) and (out[n:] == 7).all()
