@@ -250,10 +250,21 @@ int tri_mul_fwd(const TriMulDesc* d, const void* x, const void* mask, const TriM
   if (!x || !out || !ws) return fail(TRI_ERR_ARG, "x, out and ws must not be null");
   if (tc::mul_supported(d)) {
     set_path("tcgen05");
-    return tc::mul_forward(d, x, mask, w, out, saved, ws, ws_bytes, (cudaStream_t)stream);
+    return tc::mul_forward(d, x, mask, w, nullptr, out, saved, ws, ws_bytes, (cudaStream_t)stream);
   }
   set_path("simt");
   return simt::forward(d, x, mask, w, out, saved, ws, ws_bytes, (cudaStream_t)stream);
+}
+
+int tri_mul_fwd_residual(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out,
+                         void* ws, size_t ws_bytes, tri_stream_t stream) {
+  TRI_TRY(check_mul(d));
+  TRI_TRY(check_mul_weights(w));
+  if (!x || !residual || !out || !ws) return fail(TRI_ERR_ARG, "x, residual, out and ws must not be null");
+  if (!tc::mul_residual_supported(d) || reinterpret_cast<uintptr_t>(residual) % 16 != 0)
+    return fail(TRI_ERR_UNSUPPORTED, "the residual form needs a 16-bit type, one batch entry, 128 channels and N a multiple of eight");
+  set_path("tcgen05");
+  return tc::mul_forward(d, x, mask, w, residual, out, nullptr, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 int tri_mul_bwd(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* saved,

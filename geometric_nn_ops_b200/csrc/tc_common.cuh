@@ -289,6 +289,11 @@ template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w)
 template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
   return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
+// a + b of two pairs of 16-bit values, rounded once
+template <typename T> __device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
+  const float2 s = __fadd2_rn(unpack2<T>(a), unpack2<T>(b));
+  return pack2<T>(s.x, s.y);
+}
 // reciprocal of a value of at least one (infinity gives zero): without the scaling that a general quotient carries for
 // denormal and huge divisors
 __device__ __forceinline__ float rcp_approx(float x) {

@@ -350,8 +350,26 @@ struct OutArgs {
   float* mean;
   float* rstd;
   void* out;
+  const void* residual;
   int* err;
 };
+
+// One step of the transposition of 4 x 4 pieces of 16 bytes over four lanes: piece p of lane l meets piece p ^ B of lane l ^ B.
+template <int B>
+__device__ __forceinline__ void swap_pieces(uint32_t (&w)[16], int lane) {
+  const bool up = (lane & B) != 0;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    if (p & B) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint32_t &lo = w[4 * p + e], &hi = w[4 * (p | B) + e];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, B);
+      if (up) lo = got;
+      else hi = got;
+    }
+  }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -555,7 +573,6 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
   } else {
     // ------------------------------------------------------------------ gate epilogue: thread = pixel
     const int quarter = warp & 3, j = (warp - 6) >> 2;   // TMEM lane quarter; 32-channel chunk of the output row
-    const int row = quarter * 32 + lane;
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const int acc = i & 1;
@@ -563,31 +580,46 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       if (!__all_sync(0xffffffffu, done)) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 256;
-      const long long m = (long long)tile * 128 + row;
-      T* orow = reinterpret_cast<T*>(g.out) + m * 128;
+      uint32_t w[16];
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         float y[16], gt[16];
         ld16x2_f(t_row + j * 32 + hf * 16, t_row + 128 + j * 32 + hf * 16, y, gt);
-        if (m < g.M) {
-          float o[16];
 #pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const int c = j * 32 + hf * 16 + e;
-            float2 yv = make_float2(y[e], y[e + 1]), gv = make_float2(gt[e], gt[e + 1]);
-            if (g.bias != nullptr) {
-              yv = __fadd2_rn(yv, *reinterpret_cast<const float2*>(g.bias + c));
-              gv = __fadd2_rn(gv, *reinterpret_cast<const float2*>(g.bias + 128 + c));
-            }
-            const float2 r = __fmul2_rn(yv, sigmoid2(gv));
-            o[e] = r.x; o[e + 1] = r.y;
+        for (int e = 0; e < 16; e += 2) {
+          const int c = j * 32 + hf * 16 + e;
+          float2 yv = make_float2(y[e], y[e + 1]), gv = make_float2(gt[e], gt[e + 1]);
+          if (g.bias != nullptr) {
+            yv = __fadd2_rn(yv, *reinterpret_cast<const float2*>(g.bias + c));
+            gv = __fadd2_rn(gv, *reinterpret_cast<const float2*>(g.bias + 128 + c));
           }
-          store16<T>(orow + j * 32 + hf * 16, o);
+          const float2 r = __fmul2_rn(yv, sigmoid2(gv));
+          w[hf * 8 + e / 2] = pack2<T>(r.x, r.y);
         }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
+      // four lanes exchange their 16-byte pieces, so that a request writes 64 bytes of eight rows and not 16 of 32
+      swap_pieces<1>(w, lane);
+      swap_pieces<2>(w, lane);
+      const long long m0 = (long long)tile * 128 + quarter * 32 + (lane & ~3);
+      if (m0 < g.M) {   // M is a multiple of four
+        const long long at = (m0 * 128 + j * 32) / 8 + (lane & 3);
+        uint4 r[4];
+        if (g.residual != nullptr) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) r[q] = __ldg(reinterpret_cast<const uint4*>(g.residual) + at + q * 16);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            w[4 * q] = add2<T>(w[4 * q], r[q].x); w[4 * q + 1] = add2<T>(w[4 * q + 1], r[q].y);
+            w[4 * q + 2] = add2<T>(w[4 * q + 2], r[q].z); w[4 * q + 3] = add2<T>(w[4 * q + 3], r[q].w);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          (reinterpret_cast<uint4*>(g.out) + at)[q * 16] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+      }
     }
   }
   tc_fence_before_sync();
@@ -614,7 +646,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   TRI_TRY(make_tmap_3d(&tmWg, p.w_gate, 2, f16, wd, wsd, box, false));
   OutArgs a;
   a.M = p.M; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps; a.gamma = p.gamma; a.beta = p.beta;
-  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.err = p.err;
+  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.err = p.err;
   constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 8 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_out_kernel<T>;

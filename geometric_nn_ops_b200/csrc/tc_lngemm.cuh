@@ -50,6 +50,7 @@ struct LnGateOut {
   float* mean;               // [M]
   float* rstd;               // [M]
   void* out;                 // [M, 128]
+  const void* residual = nullptr;   // [M, 128], added to the (rounded) result, or null
   int* err;
 };
 

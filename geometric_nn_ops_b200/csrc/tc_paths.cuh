@@ -17,7 +17,8 @@ int attn_backward(const TriAttnDesc* d, const void* q, const void* k, const void
 bool mul_supported(const TriMulDesc* d);
 size_t mul_saved_bytes(const TriMulDesc* d);
 size_t mul_ws_bytes(const TriMulDesc* d, int is_bwd);
-int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out,
+bool mul_residual_supported(const TriMulDesc* d);   // mul_forward takes a residual
+int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out,
                 void* saved, void* ws, size_t ws_size, cudaStream_t st);
 int mul_backward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* saved,
                  const void* d_out, void* dx, const TriMulWeightGrads* g, void* ws, size_t ws_size, cudaStream_t st);

@@ -747,7 +747,7 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
 // ---- phase 3: t -> u (LayerNorm over channels), out = (u Wo^T + bo) * sigmoid(z Wgo^T + bgo) --------------
 template <typename T>
 int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* z, const TriMulWeights* w,
-                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true) {
+                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true, const void* residual = nullptr) {
   const long long M = gm.M;
   if (u_channel_major(gm)) {
     // one batch entry, 16-bit dtype: t is normalised in shared memory as the MMA's MN-major operand; u (kept for
@@ -756,7 +756,7 @@ int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* 
     f.dtype = gm.dtype; f.M = M; f.eps = gm.eps; f.t_cm = t_cm; f.z = z;
     f.gamma = w->norm_out_w; f.beta = w->norm_out_b; f.w_out = w->p_out_w; f.w_gate = w->g_out_w;
     f.bias_out = (w->p_out_b || w->g_out_b) ? pr.bias_out : nullptr;
-    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.err = pr.err;
+    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.err = pr.err;
     return ln_gate_out(st, f);
   }
   {
@@ -1011,7 +1011,7 @@ void carve_bwd(Arena& a, const Geom& gm, BwdBufs* w) {
 }
 
 template <typename T>
-int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out, void* saved,
+int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
               void* ws, size_t ws_size, cudaStream_t st) {
   const Geom gm = geom_of(d);
   Arena a(ws, ws_size);
@@ -1025,7 +1025,7 @@ int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMul
   TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b));
   const bool incoming = d->direction == TRI_INCOMING;
   TRI_TRY(contraction(st, d->dtype, d->B * CW, d->N, s.a, incoming, s.b, incoming, s.t, pr.err, "tc_gemm_contract"));
-  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr);
+  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual);
 }
 
 template <typename T>
@@ -1203,7 +1203,7 @@ int pad_mask(cudaStream_t st, const TriMulDesc* d, const void* src, void* dst) {
 }
 
 template <typename T>
-int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out, void* saved, void* ws,
+int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void*, void* out, void* saved, void* ws,
                    size_t ws_size, cudaStream_t st) {
   const TriMulDesc p = whole(d);
   const size_t inner = align_up(mul_ws_bytes(&p, 0));   // first, so that the status word is the workspace's first
@@ -1214,7 +1214,7 @@ int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const T
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
   TRI_TRY(pad_pixels(st, d, true, x, b.x));
   TRI_TRY(pad_mask<T>(st, d, mask, b.mask));
-  TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, b.io, saved, ws, inner, st));
+  TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, nullptr, b.io, saved, ws, inner, st));
   return pad_pixels(st, d, false, b.io, out);
 }
 
@@ -1297,12 +1297,14 @@ int mul_shard_phase(const TriMulShardDesc* d, int phase, const TriMulShardBufs* 
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
 }
 
-int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out, void* saved,
+bool mul_residual_supported(const TriMulDesc* d) { return mul_supported(d) && !ragged(d) && u_channel_major(geom_of(d)); }
+
+int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
                 void* ws, size_t ws_size, cudaStream_t st) {
   switch (d->dtype) {
-    case TRI_F32: return (ragged(d) ? ragged_forward<float> : forward_t<float>)(d, x, mask, w, out, saved, ws, ws_size, st);
-    case TRI_BF16: return (ragged(d) ? ragged_forward<__nv_bfloat16> : forward_t<__nv_bfloat16>)(d, x, mask, w, out, saved, ws, ws_size, st);
-    case TRI_F16: return (ragged(d) ? ragged_forward<__half> : forward_t<__half>)(d, x, mask, w, out, saved, ws, ws_size, st);
+    case TRI_F32: return (ragged(d) ? ragged_forward<float> : forward_t<float>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_BF16: return (ragged(d) ? ragged_forward<__nv_bfloat16> : forward_t<__nv_bfloat16>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_F16: return (ragged(d) ? ragged_forward<__half> : forward_t<__half>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
   }
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
 }

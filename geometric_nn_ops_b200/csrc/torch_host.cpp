@@ -43,6 +43,7 @@ struct Api {
   decltype(&tri_mul_saved_bytes) mul_saved_bytes;
   decltype(&tri_mul_ws_bytes) mul_ws_bytes;
   decltype(&tri_mul_fwd) mul_fwd;
+  decltype(&tri_mul_fwd_residual) mul_fwd_residual;
   decltype(&tri_mul_bwd) mul_bwd;
 } api;
 
@@ -55,6 +56,7 @@ void bind(const std::string& path) {
   };
   get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
   get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
+  get(api.mul_fwd_residual, "tri_mul_fwd_residual");
   get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul");
   get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
   get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
@@ -127,15 +129,16 @@ TriAttnDesc attn_desc(const Tensor& q, const Tensor& k, const Tensor& v, const T
 struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, S, N]
 
 // q, k, v [B, S, N, H, D], bias [B, 1, H, N, N], mask [B, S, 1, 1, N]
-// (`rows`: o contiguous in that order of axes, else laid out like q)
+// (`rows`: o contiguous in that order of axes, else laid out like q; or like `model`)
 AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias_, const Tensor& mask_, double scale,
-                      int64_t precision, bool rows) {
+                      int64_t precision, bool rows, const Tensor& model = Tensor()) {
   AttnCall c;
   c.q = inner_contiguous(q_); c.k = inner_contiguous(k_); c.v = inner_contiguous(v_);
   if (bias_.defined()) c.bias = inner_contiguous(bias_);
   const int64_t B = c.q.size(0), S = c.q.size(1), N = c.q.size(2), H = c.q.size(3);
   if (mask_.defined()) c.mask = mask_.reshape({B, S, N}).contiguous();
-  c.o = rows ? at::empty(c.q.sizes(), c.q.options()) : like(c.q);
+  c.o = model.defined() ? at::empty_strided(model.sizes(), model.strides(), c.q.options())
+                        : (rows ? at::empty(c.q.sizes(), c.q.options()) : like(c.q));
   c.stats = at::empty({2, B, S, H, N}, c.q.options().dtype(at::kFloat));
   const TriAttnDesc d = attn_desc(c.q, c.k, c.v, c.o, c.bias, c.mask, scale, precision);
   const c10::cuda::CUDAGuard guard(c.q.device());
@@ -183,6 +186,16 @@ struct AttnFn : torch::autograd::Function<AttnFn> {
     return {dq, dk, dv, dbias, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
+
+// residual + attention, laid out like the residual; q, k, v, residual [B, S, N, H, D], bias [B, 1, H, N, N]; inference only
+Tensor attention_residual(const Tensor& residual, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias, const Tensor& mask,
+                          int64_t precision) {
+  TORCH_CHECK(residual.is_cuda() && residual.sizes() == q.sizes() && residual.scalar_type() == q.scalar_type() &&
+              residual.is_non_overlapping_and_dense() && residual.stride(-1) == 1, "residual must be dense and of q's shape and dtype");
+  const at::NoGradGuard no_grad;
+  // (the sum in the kernel's epilogue was slower, 0.25 ms per 1024 x 1024 x 4 x 32 call against 0.12: its softmax warps wait for it)
+  return attn_forward(q, k, v, bias, mask, 1.0 / std::sqrt((double)q.size(4)), precision, false, residual).o.add_(residual);
+}
 
 // leading axes folded (or added) to rank 5
 Tensor rank5(const Tensor& t) {
@@ -260,7 +273,9 @@ TriMulWeights weight_ptrs(const Weights& w) {
 
 struct MulCall { TriMulDesc d; Tensor x, mask, saved, out; Weights w; };
 
-MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights, bool outgoing, double eps, int64_t precision, bool keep) {
+// `residual`: out is x + update
+MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights, bool outgoing, double eps, int64_t precision, bool keep,
+                    bool residual = false) {
   TORCH_CHECK(x.is_cuda(), "triangle_multiplicative_update needs CUDA tensors: there is no CPU implementation");
   MulCall c{};
   c.d.dtype = dtype_code(x);
@@ -290,7 +305,13 @@ MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights,
   c.out = at::empty(c.x.sizes(), c.x.options());
   const TriMulWeights w = weight_ptrs(c.w);
   const tri_stream_t st = stream_of(x);
-  ok(api.mul_fwd(&c.d, ptr(c.x), ptr(c.mask), &w, ptr(c.out), ptr(c.saved), ptr(ws), n, st), "tri_mul_fwd");
+  bool add = residual;
+  if (add) {
+    const int code = api.mul_fwd_residual(&c.d, ptr(c.x), ptr(c.mask), &w, ptr(c.x), ptr(c.out), ptr(ws), n, st);
+    if (code != TRI_ERR_UNSUPPORTED) { ok(code, "tri_mul_fwd_residual"); add = false; }
+  }
+  if (!residual || add) ok(api.mul_fwd(&c.d, ptr(c.x), ptr(c.mask), &w, ptr(c.out), ptr(c.saved), ptr(ws), n, st), "tri_mul_fwd");
+  if (add) c.out.add_(c.x);
   check_device(ws, reinterpret_cast<cudaStream_t>(st));
   return c;
 }
@@ -381,6 +402,16 @@ Tensor multiplicative_update(const Tensor& x, const OptTensor& mask_, bool outgo
   return mul_forward(x, mask, w, outgoing, eps, precision, /*keep=*/false).out.reshape(x.sizes());
 }
 
+// x + update, inference only
+Tensor multiplicative_update_residual(const Tensor& x, const OptTensor& mask, bool outgoing, double eps, int64_t precision,
+                                      const std::vector<OptTensor>& weights) {
+  TORCH_CHECK(weights.size() == kWeights, "expected ", kWeights, " weights");
+  Weights w;
+  for (int i = 0; i < kWeights; ++i) w[i] = or_undefined(weights[i]);
+  const at::NoGradGuard no_grad;
+  return mul_forward(x, or_undefined(mask), w, outgoing, eps, precision, /*keep=*/false, /*residual=*/true).out.reshape(x.sizes());
+}
+
 // ---------------------------------------------------------------------------------------------------- pair bias
 
 // z [B, U, V, Zc] -> LayerNorm (weight only) -> projection to H heads -> [B, H, U, V].  One kernel where it has the shape (16-bit
@@ -441,6 +472,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bind", &bind);
   m.def("attention", &attention);
   m.def("multiplicative_update", &multiplicative_update);
+  m.def("attention_residual", &attention_residual);
+  m.def("multiplicative_update_residual", &multiplicative_update_residual);
   m.def("pair_bias", &pair_bias);
   m.def("pair_bias_fits", &pair_bias_fits);
   m.def("attention_pair_bias", &attention_pair_bias);

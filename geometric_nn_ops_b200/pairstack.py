@@ -24,7 +24,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
-from . import sharded
+from . import _lib, sharded
 from .triangle import attention_input_projection, triangle_attention, triangle_multiplicative_update
 
 HEADS, HEAD_DIM = 4, 32
@@ -126,9 +126,31 @@ def _attention_update(z, pair_mask, w, group):
     return o.reshape(B, R, N, HEADS * HEAD_DIM)
 
 
+def _block_on_kernels(z, pair_mask, w):
+    """:func:`pair_block` on one GPU without gradients: the updates' residual sums are made in their epilogues, and the
+    ending-node attention writes in ``z``'s order through a transposed view, so that its sum is a plain one."""
+    host = _lib.host()
+    for outgoing, tw in ((True, w.trimul_out), (False, w.trimul_in)):
+        z = host.multiplicative_update_residual(z, pair_mask, outgoing, 1e-5, _lib.PREC_IEEE, [tw.get(n) for n in _lib.WEIGHT_NAMES])
+    B, N = z.shape[:2]
+    keep = pair_mask != 0
+    for ending, aw in ((False, w.attn_start), (True, w.attn_end)):
+        q, k, v, bias = project_attention_inputs(z, aw)
+        zh, m = z.view(B, N, N, HEADS, HEAD_DIM), keep
+        if ending:     # the kernels take the strides; only the bias and the mask, both small, are copied transposed
+            q, k, v, zh = (t.transpose(1, 2) for t in (q, k, v, zh))
+            bias, m = bias.transpose(2, 3).contiguous(), keep.transpose(1, 2)
+        zh = host.attention_residual(zh, q, k, v, bias.unsqueeze(1), m.reshape(B, N, 1, 1, N), _lib.PREC_IEEE)
+        z = (zh.transpose(1, 2) if ending else zh).view(z.shape)
+    return z
+
+
 def pair_block(z, pair_mask, w: BlockWeights, group=None):
     """One block on ``z`` ``[B, R, N, C]`` (R = N on one GPU, N/P rows when sharded), ``pair_mask`` ``[B, R, N]``."""
     multi = group is not None and sharded._world(group)[0] > 1
+    if (not multi and z.is_cuda and z.dtype in (torch.bfloat16, torch.float16) and z.shape[-1] == HEADS * HEAD_DIM and z.is_contiguous()
+            and not torch.is_grad_enabled()):
+        return _block_on_kernels(z, pair_mask, w)
     for direction, tw in (("outgoing", w.trimul_out), ("incoming", w.trimul_in)):
         if multi:
             z = z + sharded.sharded_triangle_multiplicative_update(z, direction, pair_mask, group=group, **tw)

@@ -185,6 +185,10 @@ size_t tri_mul_ws_bytes(const TriMulDesc* d, int is_bwd);
 int tri_mul_fwd(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w,
                 void* out, void* saved /*nullable*/, void* ws, size_t ws_bytes,
                 tri_stream_t stream);
+/* out = residual + update (each rounded to `dtype`), nothing kept for a backward.  TRI_ERR_UNSUPPORTED, before anything is
+ * launched, unless `dtype` has 16 bits, B = 1, C = Ch = 128 and N is a multiple of eight. */
+int tri_mul_fwd_residual(const TriMulDesc* d, const void* x, const void* mask /*nullable*/, const TriMulWeights* w, const void* residual,
+                         void* out, void* ws, size_t ws_bytes, tri_stream_t stream);
 
 /* Backward of the above.  The reference has no kernel for it: it differentiates
  * trimul_torch with autograd (geometric_nn_ops_torch/triangle/_trimul.py:31-36). */
