@@ -661,17 +661,22 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
 // =================================================================================================================
 // gate_in_bwd: dP = d sig(G) mask, dG = d P sig (1 - sig) mask for d = da, db, with P and G recomputed from z
 // =================================================================================================================
-// 576 threads: warp 0 TMA, warp 1 tcgen05.mma, warps 2-17 the gate epilogue (thread = channel of the half, 16 of the
-// tile's 64 pixels).  As in ln_gate_in the weights stay in shared memory and a z tile feeds the products of both halves,
-// so z is read once.  The gradient tile of a half ([128 channels x 64 pixels]) comes by TMA; the epilogue copies it to
+// 576 threads: warp 0 TMA, warp 1 tcgen05.mma, warps 2-17 the gate epilogue (thread = channel of the half, a quarter of
+// the tile's pixels).  A tile is 128 bytes of pixels: 64 of 16 bits or 32 of fp32.  As in ln_gate_in the weights stay in
+// shared memory; with 16-bit types a z tile feeds the products of both halves, so z is read once.  The fp32 weights of one
+// half fill the same space, so there a CTA has one half and its neighbour the other, on the same tiles (z comes from L2
+// the second time).  The gradient tile of a half ([128 channels x 128 bytes]) comes by TMA; the epilogue copies it to
 // registers at once, so that its buffer takes the next tile's during the arithmetic.  dP and dG leave through a staging
 // tile each and a TMA store: whole 128-byte lines.  Written by the threads, a request carried 32 bytes (a channel's rows
 // lie a plane apart), 4096 of them per 128 pixels, and the load / store pipe held the kernel at 0.29 ms for 768 x 768
 // pixels; with the gradients read that way too (the batched GEMM's form) it took 0.365.  Now 0.22, floor by bytes 0.16.
+// fp32 with TF32 products, 512 x 512 pixels: 0.41 ms in the GEMM's form, 0.18 here, floor 0.14.
 constexpr int kBwdThreads = 576;
 constexpr int kBwdMaskRing = 4;           // as kMaskRing
-constexpr int kBSub = 8192;               // [64 rows x 128 bytes]
-constexpr uint32_t kBTile = 16384;        // z tile: two 64-channel halves; gradient or output tile of a half
+constexpr uint32_t kBTile = 16384;        // z tile: kKb blocks of [kPx rows x 128 bytes]; gradient or output tile of a half
+template <typename T> struct BwdGeo {
+  static constexpr int kHalves = sizeof(T) == 2 ? 2 : 1, kPx = 128 / sizeof(T), kKb = sizeof(T), kBSub = kPx * 128, kE = kPx / 4;
+};
 
 struct BwdArgs {
   long long M;
@@ -682,25 +687,40 @@ struct BwdArgs {
   int* err;
 };
 
+// 16 bytes of a tile row as pairs
+template <typename T, int N> __device__ __forceinline__ void unpack_piece(const uint4& w, float2 (&v)[N]) {
+  if constexpr (sizeof(T) == 4) {
+    v[0] = make_float2(__uint_as_float(w.x), __uint_as_float(w.y));
+    v[1] = make_float2(__uint_as_float(w.z), __uint_as_float(w.w));
+  } else {
+    unpack8p<T>(w, v);
+  }
+}
+template <typename T, int N> __device__ __forceinline__ uint4 pack_piece(const float2 (&v)[N]) {
+  if constexpr (sizeof(T) == 4) return make_uint4(__float_as_uint(v[0].x), __float_as_uint(v[0].y), __float_as_uint(v[1].x), __float_as_uint(v[1].y));
+  else return pack8p<T>(v);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmW,
                    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmO, const BwdArgs g) {
-  constexpr int KIND = ElemTraits<T>::kind;
+  using G = BwdGeo<T>;
+  constexpr int KIND = ElemTraits<T>::kind, kH = G::kHalves, kKb = G::kKb;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
   uint8_t* sZ = smem + kWBytes;            // [2] z tiles
-  uint8_t* sG = sZ + 2 * kBTile;           // [half] gradient tile
+  uint8_t* sG = sZ + 2 * kBTile;           // [2] gradient tiles (of the halves in turn)
   uint8_t* sO = sG + 2 * kBTile;           // dP, dG of a half
-  uint8_t* sM = sO + 2 * kBTile;           // [kBwdMaskRing] x 64 mask values
+  uint8_t* sM = sO + 2 * kBTile;           // [kBwdMaskRing] x 128 bytes of mask values
   uint64_t* wfull = reinterpret_cast<uint64_t*>(sM + kBwdMaskRing * 128);
   uint64_t* zfull = wfull + 1;             // [2]
   uint64_t* zempty = zfull + 2;            // [2] both halves' products of the tile are done
-  uint64_t* gfull = zempty + 2;            // [half] gradient tile (half a: with the tile's mask)
-  uint64_t* gempty = gfull + 2;            // [half] ... copied to registers by all 16 epilogue warps
-  uint64_t* tfull = gempty + 2;            // [tile & 1][half] accumulator complete
+  uint64_t* gfull = zempty + 2;            // [2] gradient tile (the tile's first: with its mask)
+  uint64_t* gempty = gfull + 2;            // [2] ... copied to registers by all 16 epilogue warps
+  uint64_t* tfull = gempty + 2;            // [4] accumulator of an item complete
   uint64_t* tempty = tfull + 4;            // ... read by all 16 epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 4);
 
@@ -717,29 +737,34 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  // items: the halves this CTA has, of tiles tile0, tile0 + step, ...; half_of(hh): the hh-th of them
+  const int tile0 = kH == 2 ? blockIdx.x : blockIdx.x >> 1, step = kH == 2 ? gridDim.x : gridDim.x >> 1;
+  auto half_of = [&](int hh) { return kH == 2 ? hh : (int)(blockIdx.x & 1); };
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
       mbar_expect_tx(wfull, kWBytes);
-      for (int blk = 0; blk < 4; ++blk)
-        for (int kb = 0; kb < 2; ++kb) tma_load_3d(sW + (blk * 2 + kb) * kSub, &tmW, wfull, kb * 64, blk * 128, 0);
+      for (int blk = 0; blk < 2 * kH; ++blk)
+        for (int kb = 0; kb < kKb; ++kb)
+          tma_load_3d(sW + (blk * kKb + kb) * kSub, &tmW, wfull, kb * G::kPx, (half_of(blk >> 1) * 2 + (blk & 1)) * 128, 0);
       bool ok = true;
       auto load_z = [&](int i, int tile) {
         const int b = i & 1;
         if (!mbar_wait(&zempty[b], ((i >> 1) & 1) ^ 1, g.err, 60)) { ok = false; return; }
         mbar_expect_tx(&zfull[b], kBTile);
-        for (int kb = 0; kb < 2; ++kb) tma_load_3d(sZ + b * kBTile + kb * kBSub, &tmZ, &zfull[b], kb * 64, tile * 64, 0);
+        for (int kb = 0; kb < kKb; ++kb) tma_load_3d(sZ + b * kBTile + kb * G::kBSub, &tmZ, &zfull[b], kb * G::kPx, tile * G::kPx, 0);
       };
-      if ((int)blockIdx.x < g.tiles) load_z(0, blockIdx.x);
-      int i = 0;
-      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
-        if (tile + (int)gridDim.x < g.tiles) load_z(i + 1, tile + gridDim.x);   // one tile ahead
-        for (int half = 0; half < 2 && ok; ++half) {
-          if (!mbar_wait(&gempty[half], (i & 1) ^ 1, g.err, 61)) { ok = false; break; }
-          const bool with_mask = half == 0 && g.mask != nullptr;
-          mbar_expect_tx(&gfull[half], kBTile + (with_mask ? 128 : 0));
-          tma_load_3d(sG + half * kBTile, half == 0 ? &tmA : &tmB, &gfull[half], tile * 64, 0, 0);
-          if (with_mask) bulk_load(sM + (i % kBwdMaskRing) * 128, static_cast<const uint8_t*>(g.mask) + (long long)tile * 128, 128, &gfull[0]);
+      if (tile0 < g.tiles) load_z(0, tile0);
+      int i = 0, it = 0;
+      for (int tile = tile0; tile < g.tiles && ok; tile += step, ++i) {
+        if (tile + step < g.tiles) load_z(i + 1, tile + step);   // one tile ahead
+        for (int hh = 0; hh < kH && ok; ++hh, ++it) {
+          const int b = it & 1;
+          if (!mbar_wait(&gempty[b], ((it >> 1) & 1) ^ 1, g.err, 61)) { ok = false; break; }
+          const bool with_mask = hh == 0 && g.mask != nullptr;
+          mbar_expect_tx(&gfull[b], kBTile + (with_mask ? 128 : 0));
+          tma_load_3d(sG + b * kBTile, half_of(hh) == 0 ? &tmA : &tmB, &gfull[b], tile * G::kPx, 0, 0);
+          if (with_mask) bulk_load(sM + (i % kBwdMaskRing) * 128, static_cast<const uint8_t*>(g.mask) + (long long)tile * 128, 128, &gfull[b]);
         }
       }
     }
@@ -747,26 +772,26 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      const uint32_t idesc = make_idesc(KIND, 128, 64, false, false);
+      const uint32_t idesc = make_idesc(KIND, 128, G::kPx, false, false);
       const uint32_t w_base = smem_u32(sW), z_base = smem_u32(sZ);
       bool ok = mbar_wait(wfull, 0, g.err, 62);
-      int i = 0;
-      for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i) {
+      int i = 0, it = 0;
+      for (int tile = tile0; tile < g.tiles && ok; tile += step, ++i) {
         const int b = i & 1;
         if (!mbar_wait(&zfull[b], (i >> 1) & 1, g.err, 63)) break;
-        for (int half = 0; half < 2 && ok; ++half) {
-          const int acc = b * 2 + half;
-          if (!mbar_wait(&tempty[acc], ((i >> 1) & 1) ^ 1, g.err, 64)) { ok = false; break; }
+        for (int hh = 0; hh < kH && ok; ++hh, ++it) {
+          const int acc = it & 3;
+          if (!mbar_wait(&tempty[acc], ((it >> 2) & 1) ^ 1, g.err, 64)) { ok = false; break; }
           tc_fence_after_sync();
 #pragma unroll
           for (int pg = 0; pg < 2; ++pg) {   // P block, G block of this half
             const uint32_t d_addr = tmem_base + acc * 128 + pg * 64;
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb)
+            for (int kb = 0; kb < kKb; ++kb)
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks) {
-                const uint64_t ad = make_smem_desc(w_base + ((half * 2 + pg) * 2 + kb) * kSub + ks * 32, 16, 1024);
-                const uint64_t bd = make_smem_desc(z_base + b * kBTile + kb * kBSub + ks * 32, 16, 1024);
+                const uint64_t ad = make_smem_desc(w_base + ((hh * 2 + pg) * kKb + kb) * kSub + ks * 32, 16, 1024);
+                const uint64_t bd = make_smem_desc(z_base + b * kBTile + kb * G::kBSub + ks * 32, 16, 1024);
                 umma<KIND>(d_addr, ad, bd, idesc, (kb == 0 && ks == 0) ? 0u : 1u);
               }
           }
@@ -778,65 +803,77 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
-    const int quarter = warp & 3, j = (warp - 2) >> 2;   // TMEM lane quarter; 16-pixel part of the tile
+    const int quarter = warp & 3, j = (warp - 2) >> 2;   // TMEM lane quarter; kE-pixel part of the tile
     const int row = quarter * 32 + lane;
     const uint32_t at = row * 128, c0 = ((j * 2) ^ (row & 7)) << 4, c1 = ((j * 2 + 1) ^ (row & 7)) << 4;   // this thread's two pieces of a tile row
     const bool masked = g.mask != nullptr;
-    int i = 0;
+    int i = 0, it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
+    for (int tile = tile0; tile < g.tiles; tile += step, ++i) {
       const uint4* mrow = reinterpret_cast<const uint4*>(sM + (i % kBwdMaskRing) * 128 + j * 32);
-      for (int half = 0; half < 2; ++half) {
-        const int acc = (i & 1) * 2 + half;
-        const uint8_t* gt_row = sG + half * kBTile + at;
-        ok = mbar_wait(&gfull[half], i & 1, g.err, 65) && ok;
+      for (int hh = 0; hh < kH; ++hh, ++it) {
+        const int half = half_of(hh), acc = it & 3, b = it & 1;
+        const uint8_t* gt_row = sG + b * kBTile + at;
+        ok = mbar_wait(&gfull[b], (it >> 1) & 1, g.err, 65) && ok;
         const uint4 d[2] = {*reinterpret_cast<const uint4*>(gt_row + c0), *reinterpret_cast<const uint4*>(gt_row + c1)};
         // The arrival must not pass the loads, which queue behind other accesses of this warp: its address takes in what
         // they returned (and-ed with an argument that is zero), so the warp cannot issue it before they are complete.
         __syncwarp();
-        if (lane == 0) mbar_arrive(&gempty[half] + ((d[0].w | d[1].w) & g.zero));
-        ok = mbar_wait(&tfull[acc], (i >> 1) & 1, g.err, 66) && ok;
+        if (lane == 0) mbar_arrive(&gempty[b] + ((d[0].w | d[1].w) & g.zero));
+        ok = mbar_wait(&tfull[acc], (it >> 2) & 1, g.err, 66) && ok;
         tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * 16;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * G::kE;
         float bp = 0.f, bg = 0.f;
         if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
         const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
-        float p[16], gt[16];
-        ld16x2_f(t_row, t_row + 64, p, gt);
+        float p[G::kE], gt[G::kE];
+        if constexpr (G::kE == 16) {
+          ld16x2_f(t_row, t_row + 64, p, gt);
+        } else {
+          uint32_t rp[8], rg[8];
+          tmem_ld_32x8(t_row, rp);
+          tmem_ld_32x8(t_row + 64, rg);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { p[e] = __uint_as_float(rp[e]); gt[e] = __uint_as_float(rg[e]); }
+        }
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[acc]);
-        Raw8<T> o0[2], o1[2];
+        // two pieces of 16 bytes: kE pixels as float2 pairs, dP and dG in place of the gradient
+        constexpr int kPair = G::kE / 4;   // per piece
+        uint4 o0[2], o1[2];
 #pragma unroll
         for (int uu = 0; uu < 2; ++uu) {
-          float2 dv[4], mk[4];
-          unpack8p<T>(d[uu], dv);
+          float2 dv[kPair], mk[kPair], dg[kPair];
+          unpack_piece<T>(d[uu], dv);
           if (masked) {
-            unpack8p<T>(mrow[uu], mk);
+            unpack_piece<T>(mrow[uu], mk);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) dv[k] = __fmul2_rn(dv[k], mk[k]);
+            for (int k = 0; k < kPair; ++k) dv[k] = __fmul2_rn(dv[k], mk[k]);
           }
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int e = uu * 8 + 2 * k;
+          for (int k = 0; k < kPair; ++k) {
+            const int e = uu * 2 * kPair + 2 * k;
             const float2 sg = sigmoid2(make_float2(gt[e], gt[e + 1]), nbg2);
-            const float2 dp = __fmul2_rn(dv[k], sg);
+            dv[k] = __fmul2_rn(dv[k], sg);
             const float2 oms = __ffma2_rn(sg, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
-            putraw8(o0[uu], k, dp);
-            putraw8(o1[uu], k, __fmul2_rn(__fmul2_rn(dp, __fadd2_rn(make_float2(p[e], p[e + 1]), bp2)), oms));
+            dg[k] = __fmul2_rn(__fmul2_rn(dv[k], __fadd2_rn(make_float2(p[e], p[e + 1]), bp2)), oms);
           }
+          o0[uu] = pack_piece<T>(dv);
+          o1[uu] = pack_piece<T>(dg);
         }
         if (threadIdx.x == 64) bulk_wait_group_read0();   // the previous half's stores have left the staging tiles
         named_barrier(1, 512);
-        *reinterpret_cast<uint4*>(sO + at + c0) = o0[0].w[0];
-        *reinterpret_cast<uint4*>(sO + at + c1) = o0[1].w[0];
-        *reinterpret_cast<uint4*>(sO + kBTile + at + c0) = o1[0].w[0];
-        *reinterpret_cast<uint4*>(sO + kBTile + at + c1) = o1[1].w[0];
+        *reinterpret_cast<uint4*>(sO + at + c0) = o0[0];
+        *reinterpret_cast<uint4*>(sO + at + c1) = o0[1];
+        *reinterpret_cast<uint4*>(sO + kBTile + at + c0) = o1[0];
+        *reinterpret_cast<uint4*>(sO + kBTile + at + c1) = o1[1];
         fence_proxy_async_smem();
         named_barrier(2, 512);
         if (threadIdx.x == 64 && ok) {
-          tma_store_3d(&tmO, sO, tile * 64, half * 256, 0);
-          tma_store_3d(&tmO, sO + kBTile, tile * 64, half * 256 + 128, 0);
+          tma_store_3d(&tmO, sO, tile * G::kPx, half * 256, 0);
+          tma_store_3d(&tmO, sO + kBTile, tile * G::kPx, half * 256 + 128, 0);
           bulk_commit_group();
         }
       }
@@ -859,20 +896,22 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   const uint64_t zd[3] = {128, M, 1}, zs[2] = {128, 128 * M};
   const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
   const uint64_t gd[3] = {M, 128, 1}, od[3] = {M, 512, 1}, gs[2] = {M, 512 * M};
-  const uint32_t zbox[3] = {64, 64, 1}, box[3] = {64, 128, 1};
-  TRI_TRY(make_tmap_3d(&tmZ, p.z, 2, f16, zd, zs, zbox, false));
-  TRI_TRY(make_tmap_3d(&tmW, p.wcat, 2, f16, wd, wsd, box, false));
-  TRI_TRY(make_tmap_3d(&tmA, p.da_cm, 2, f16, gd, gs, box, false));
-  TRI_TRY(make_tmap_3d(&tmB, p.db_cm, 2, f16, gd, gs, box, false));
-  TRI_TRY(make_tmap_3d(&tmO, p.dpg, 2, f16, od, gs, box, false));
+  using G = BwdGeo<T>;
+  constexpr int E = sizeof(T);
+  const uint32_t zbox[3] = {G::kPx, G::kPx, 1}, box[3] = {G::kPx, 128, 1};
+  TRI_TRY(make_tmap_3d(&tmZ, p.z, E, f16, zd, zs, zbox, false));
+  TRI_TRY(make_tmap_3d(&tmW, p.wcat, E, f16, wd, wsd, box, false));
+  TRI_TRY(make_tmap_3d(&tmA, p.da_cm, E, f16, gd, gs, box, false));
+  TRI_TRY(make_tmap_3d(&tmB, p.db_cm, E, f16, gd, gs, box, false));
+  TRI_TRY(make_tmap_3d(&tmO, p.dpg, E, f16, od, gs, box, false));
   BwdArgs a;
-  a.M = p.M; a.tiles = (int)(p.M / 64); a.bias = p.bias_cat; a.mask = p.mask; a.zero = 0; a.err = p.err;
+  a.M = p.M; a.tiles = (int)(p.M / G::kPx); a.bias = p.bias_cat; a.mask = p.mask; a.zero = 0; a.err = p.err;
   constexpr size_t smem = 1024 + kWBytes + 6 * kBTile + kBwdMaskRing * 128 + 17 * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = gate_in_bwd_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = std::min(a.tiles, sm_count());
-  KernelTimer kt("tc_gate_in_bwd", st, 0.0, 7.0 * p.M * 128 * 2);
+  const int grid = G::kHalves == 2 ? std::min(a.tiles, sm_count()) : 2 * std::min(a.tiles, sm_count() / 2);
+  KernelTimer kt("tc_gate_in_bwd", st, 0.0, 7.0 * p.M * 128 * E);
   kern<<<grid, kBwdThreads, smem, st>>>(tmZ, tmW, tmA, tmB, tmO, a);
   TRI_LAUNCH_OK();
   return 0;
@@ -882,11 +921,12 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
 
 // one batch entry (its channel planes are M pixels apart), whole tiles (any square of a multiple of eight)
 bool gate_in_bwd_supported(int dtype, long long M, long long plane) {
-  return (dtype == TRI_BF16 || dtype == TRI_F16) && M > 0 && M == plane && M % 64 == 0 && M < (1LL << 31) - 128;
+  return (dtype == TRI_BF16 || dtype == TRI_F16 || dtype == TRI_F32) && M > 0 && M == plane && M % 64 == 0 && M < (1LL << 31) - 128;
 }
 
 int gate_in_bwd(cudaStream_t st, const GateInBwd& p) {
   if (!gate_in_bwd_supported(p.dtype, p.M, p.M)) return fail(TRI_ERR_ARG, "gate_in_bwd: unsupported shape or dtype");
+  if (p.dtype == TRI_F32) return launch_bwd<float>(st, p);
   return p.dtype == TRI_BF16 ? launch_bwd<__nv_bfloat16>(st, p) : launch_bwd<__half>(st, p);
 }
 

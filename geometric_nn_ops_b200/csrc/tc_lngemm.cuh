@@ -60,7 +60,7 @@ int ln_gate_out(cudaStream_t st, const LnGateOut& p);
 
 // Input gate backward: dP, dG of both halves from the recomputed projections of z and the gradients of a and b.
 struct GateInBwd {
-  int dtype;                 // TRI_BF16 / TRI_F16
+  int dtype;                 // fp32: TF32 products
   long long M;               // pixels (one batch entry)
   const void* z;             // [M, 128]
   const void* wcat;          // [512, 128]: rows [Wp_a; Wg_a; Wp_b; Wg_b]

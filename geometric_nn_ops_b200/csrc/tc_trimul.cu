@@ -33,7 +33,7 @@ namespace {
 constexpr int CW = 128;        // channel width this path is built for
 constexpr int kPersist = 592;  // blocks of the persistent memory-bound kernels (4 per SM)
 constexpr int kLnCmBlocks = 592;    // ln_cm: 4 per SM (64 registers per thread hold the next tile's loads)
-constexpr int kLnCmBwdBlocks = 444; // ln_cm_bwd: 3 per SM (80 registers: next tile, eight pixels' gradients and statistics)
+constexpr int kLnCmBwdBlocks = 296; // ln_cm_bwd: 2 per SM (128 registers: next tile, eight pixels' gradients and statistics; 85 spill with fp32)
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256, 4) ln_cm_kernel(const T* t_cm, const T* g
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, 3) ln_cm_bwd_kernel(const T* du, const T* t_cm, const float* mean,
+__global__ void __launch_bounds__(256, 2) ln_cm_bwd_kernel(const T* du, const T* t_cm, const float* mean,
                                                             const float* rstd, const T* gamma, long long M,
                                                             long long NN, T* dt_cm, float* pg, float* pb) {
   __shared__ float tile[TP * TROW];
@@ -366,21 +366,25 @@ __global__ void __launch_bounds__(256, 3) ln_cm_bwd_kernel(const T* du, const T*
   if (gamma) load4(gamma + lane * 4, gm);
   const long long tiles = (M + TP - 1) / TP;
   CmRegs<T> next;
-  if ((long long)blockIdx.x < tiles) fetch_cm_tile(next, t_cm, (long long)blockIdx.x * TP, M, NN);
-  for (long long tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
-    const long long m0 = tl * TP;
-    __syncthreads();                       // the previous tile has been stored from shared memory
-    put_cm_tile(tile, next);
-    // this warp's eight pixels: their upstream gradients and statistics, fetched together instead of one pixel at a
-    // time in front of their use (eight exposed load latencies per tile)
-    Raw4<T> d8[TP / 8];
-    float mu8[TP / 8], rs8[TP / 8];
+  // this warp's pixels of a tile: their upstream gradients and statistics, fetched together, for the next tile as soon as
+  // this one's are used up (0.146 -> 0.081 ms, without the spills at 512 x 512 pixels of fp32; fetched in front of their use they exposed a
+  // DRAM latency per tile)
+  Raw4<T> d8[TP / 8];
+  float mu8[TP / 8], rs8[TP / 8];
+  auto fetch_rows = [&](long long m0) {
 #pragma unroll
     for (int i = 0; i < TP / 8; ++i) {
       const long long m = m0 + warp + 8 * i;
       mu8[i] = 0.f; rs8[i] = 0.f;
       if (m < M) { d8[i] = ldraw4<T>(du + m * CW + lane * 4); mu8[i] = mean[m]; rs8[i] = rstd[m]; }
     }
+  };
+  if ((long long)blockIdx.x < tiles) fetch_rows((long long)blockIdx.x * TP);
+  if ((long long)blockIdx.x < tiles) fetch_cm_tile(next, t_cm, (long long)blockIdx.x * TP, M, NN);
+  for (long long tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
+    const long long m0 = tl * TP;
+    __syncthreads();                       // the previous tile has been stored from shared memory
+    put_cm_tile(tile, next);
     __syncthreads();
     if (tl + gridDim.x < tiles) fetch_cm_tile(next, t_cm, (tl + gridDim.x) * TP, M, NN);   // in flight during the arithmetic
 #pragma unroll
@@ -404,6 +408,7 @@ __global__ void __launch_bounds__(256, 3) ln_cm_bwd_kernel(const T* du, const T*
 #pragma unroll
       for (int k = 0; k < 4; ++k) tile[tile_at(pl, lane * 4 + k)] = rs * (dh[k] - s1 - th[k] * s2);
     }
+    if (tl + gridDim.x < tiles) fetch_rows((tl + gridDim.x) * TP);
     __syncthreads();
     store_cm_tile(tile, dt_cm, m0, M, NN);
   }
