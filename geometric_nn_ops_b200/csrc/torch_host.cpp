@@ -84,6 +84,15 @@ void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 Tensor bytes(size_t n, const Tensor& like) {
   return at::empty({(int64_t)std::max<size_t>(n, 1)}, like.options().dtype(at::kByte));
 }
+// Without gradients the torch calls of a function need no autograd bookkeeping (about half a microsecond each).  Tensors that are
+// handed out must not be views made under this.
+struct NoRecord {
+  std::optional<at::AutoDispatchBelowADInplaceOrView> guard;
+  explicit NoRecord(bool on) { if (on) guard.emplace(); }
+};
+bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
+bool wants_grad(const OptTensor& t) { return t.has_value() && t->requires_grad(); }
+
 tri_stream_t stream_of(const Tensor& t) {
   return reinterpret_cast<tri_stream_t>(c10::cuda::getCurrentCUDAStream(t.get_device()).stream());
 }
@@ -131,7 +140,8 @@ struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, 
 // q, k, v [B, S, N, H, D], bias [B, 1, H, N, N], mask [B, S, 1, 1, N]
 // (`rows`: o contiguous in that order of axes, else laid out like q; or like `model`)
 AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias_, const Tensor& mask_, double scale,
-                      int64_t precision, bool rows, const Tensor& model = Tensor()) {
+                      int64_t precision, bool rows, bool record = false, const Tensor& model = Tensor()) {
+  const NoRecord fast(!record);   // (views that are saved for a backward share their base's version counter)
   AttnCall c;
   c.q = inner_contiguous(q_); c.k = inner_contiguous(k_); c.v = inner_contiguous(v_);
   if (bias_.defined()) c.bias = inner_contiguous(bias_);
@@ -158,7 +168,7 @@ Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); 
 struct AttnFn : torch::autograd::Function<AttnFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& bias,
                                const OptTensor& mask, double scale, int64_t precision, bool rows) {
-    const AttnCall c = attn_forward(q, k, v, or_undefined(bias), or_undefined(mask), scale, precision, rows);
+    const AttnCall c = attn_forward(q, k, v, or_undefined(bias), or_undefined(mask), scale, precision, rows, /*record=*/true);
     ctx->save_for_backward({c.q, c.k, c.v, c.bias, c.mask, c.o, c.stats});
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["precision"] = precision;
@@ -194,7 +204,7 @@ Tensor attention_residual(const Tensor& residual, const Tensor& q, const Tensor&
               residual.is_non_overlapping_and_dense() && residual.stride(-1) == 1, "residual must be dense and of q's shape and dtype");
   const at::NoGradGuard no_grad;
   // (the sum in the kernel's epilogue was slower, 0.25 ms per 1024 x 1024 x 4 x 32 call against 0.12: its softmax warps wait for it)
-  return attn_forward(q, k, v, bias, mask, 1.0 / std::sqrt((double)q.size(4)), precision, false, residual).o.add_(residual);
+  return attn_forward(q, k, v, bias, mask, 1.0 / std::sqrt((double)q.size(4)), precision, false, false, residual).o.add_(residual);
 }
 
 // leading axes folded (or added) to rank 5
@@ -224,25 +234,29 @@ py::object attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
   TORCH_CHECK(q_.is_cuda(), "triangle_attention needs CUDA tensors: there is no CPU implementation");
   dtype_code(q_);
   const bool canonical = q_.dim() == 5;
-  const Tensor q = rank5(q_);
-  Tensor k = rank5(k_), v = rank5(v_), bias, mask;
-  if (k.scalar_type() != q.scalar_type()) k = k.to(q.scalar_type());
-  if (v.scalar_type() != q.scalar_type()) v = v.to(q.scalar_type());
-  const int64_t B = q.size(0), S = q.size(1), N = q.size(2), H = q.size(3);
-  if (bias_.has_value()) {
-    bias = *bias_;
-    if (bias.dim() == 4) bias = bias.unsqueeze(-4);
-    else if (bias.dim() > 5) bias = rank5(bias);
-    bias = bias.expand({B, 1, H, N, N});
-    if (bias.scalar_type() != q.scalar_type()) bias = bias.to(q.scalar_type());
+  Tensor o, stats;
+  {
+    const NoRecord fast(!at::GradMode::is_enabled() || !(wants_grad(q_) || wants_grad(k_) || wants_grad(v_) || wants_grad(bias_)));
+    const Tensor q = rank5(q_);
+    Tensor k = rank5(k_), v = rank5(v_), bias, mask;
+    if (k.scalar_type() != q.scalar_type()) k = k.to(q.scalar_type());
+    if (v.scalar_type() != q.scalar_type()) v = v.to(q.scalar_type());
+    const int64_t B = q.size(0), S = q.size(1), N = q.size(2), H = q.size(3);
+    if (bias_.has_value()) {
+      bias = *bias_;
+      if (bias.dim() == 4) bias = bias.unsqueeze(-4);
+      else if (bias.dim() > 5) bias = rank5(bias);
+      bias = bias.expand({B, 1, H, N, N});
+      if (bias.scalar_type() != q.scalar_type()) bias = bias.to(q.scalar_type());
+    }
+    if (mask_.has_value()) {
+      mask = *mask_;
+      if (mask.dim() > 5) mask = rank5(mask);
+      mask = mask.expand({B, S, 1, 1, N});
+    }
+    const double scale = scale_.has_value() ? *scale_ : 1.0 / std::sqrt((double)q.size(4));
+    std::tie(o, stats) = attn_any(q, k, v, bias, mask, scale, precision, false);
   }
-  if (mask_.has_value()) {
-    mask = *mask_;
-    if (mask.dim() > 5) mask = rank5(mask);
-    mask = mask.expand({B, S, 1, 1, N});
-  }
-  const double scale = scale_.has_value() ? *scale_ : 1.0 / std::sqrt((double)q.size(4));
-  auto [o, stats] = attn_any(q, k, v, bias, mask, scale, precision, false);
   if (!canonical) o = o.reshape(q_.sizes());
   if (!return_aux) return py::cast(o);
   const Tensor m = stats.select(0, 0);
@@ -277,6 +291,7 @@ struct MulCall { TriMulDesc d; Tensor x, mask, saved, out; Weights w; };
 MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights, bool outgoing, double eps, int64_t precision, bool keep,
                     bool residual = false) {
   TORCH_CHECK(x.is_cuda(), "triangle_multiplicative_update needs CUDA tensors: there is no CPU implementation");
+  const NoRecord fast(!keep);   // as in attn_forward
   MulCall c{};
   c.d.dtype = dtype_code(x);
   for (int i : {2, 4, 8, 10}) TORCH_CHECK_VALUE(weights[i].defined(), kNames[i], " is required");
@@ -456,6 +471,11 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
                                               const OptTensor& z_w, const OptTensor& ln_w, const OptTensor& mask_, double scale, double eps,
                                               int64_t precision) {
   const int64_t BM = q.size(0), H = q.size(1), U = q.size(2), D = q.size(3), B = z.size(0), M = BM / B;
+  bool grad = false;
+  if (at::GradMode::is_enabled())
+    for (const Tensor* t : {&s, &q, &k, &v, &z, &g_w, &o_w}) grad = grad || t->requires_grad();
+  grad = grad || (at::GradMode::is_enabled() && (wants_grad(g_b) || wants_grad(o_b) || wants_grad(z_w) || wants_grad(ln_w)));
+  const NoRecord fast(!grad);
   const Tensor pz = z_w.has_value() ? pair_bias(z, ln_w, *z_w, eps) : z;
   // (BM, H, U, D) -> rows = multiplicity: [B, M, U, H, D] as a strided view (no copy)
   auto rows = [&](const Tensor& t) { return inner_contiguous(t.reshape({B, M, H, U, D}).transpose(2, 3)); };
@@ -463,7 +483,14 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
   if (mask_.has_value()) mask = at::ne(*mask_, 0).reshape({B, -1, 1, 1, U}).expand({B, M, 1, 1, U});
   const Tensor bias = (pz.scalar_type() == q.scalar_type() ? pz : pz.to(q.scalar_type())).unsqueeze(1).expand({B, 1, H, U, U});
   const Tensor o = attn_any(rows(q), rows(k), rows(v), bias, mask, scale, precision, true).first.reshape({BM, U, H * D}).to(s.scalar_type());
-  return {at::linear(gated(o, at::linear(s, g_w, g_b)), o_w, o_b), pz};
+  if (grad || s.dim() != 3 || !s.is_contiguous() || g_w.dim() != 2 || o_w.dim() != 2)
+    return {at::linear(gated(o, at::linear(s, g_w, g_b)), o_w, o_b), pz};
+  // the same products on two dimensions
+  auto linear = [](const Tensor& x, const Tensor& w, const OptTensor& b) { return b.has_value() ? at::addmm(*b, x, w.t()) : at::mm(x, w.t()); };
+  const Tensor gate = linear(s.view({-1, s.size(2)}), g_w, g_b);
+  Tensor out = linear(gated(o.reshape({-1, H * D}), gate), o_w, o_b);
+  out.unsafeGetTensorImpl()->set_sizes_contiguous({BM, U, o_w.size(0)});   // (a view made here would go untracked)
+  return {out, pz};
 }
 
 }  // namespace
