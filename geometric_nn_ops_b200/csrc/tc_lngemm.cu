@@ -47,6 +47,7 @@ struct Args {
   void* b_cm;
   float* mean;
   float* rstd;
+  int pitch;            // 0, or the padded side: x has its own
   int staged;           // a / b leave through shared memory by TMA (planes of whole 64-pixel chunks)
   int* err;
 };
@@ -111,7 +112,15 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int b = i % kXBufs;
         if (!mbar_wait(&xempty[b], ((i / kXBufs) & 1) ^ 1, g.err, 10)) break;
         mbar_expect_tx(&xfull[b], kXBytes);
-        for (int kb = 0; kb < 2; ++kb) tma_load_3d(sX + b * kXBytes + kb * kSub, &tmX, &xfull[b], kb * 64, tile * 128, 0);
+        if (g.pitch == 0) {
+          for (int kb = 0; kb < 2; ++kb) tma_load_3d(sX + b * kXBytes + kb * kSub, &tmX, &xfull[b], kb * 64, tile * 128, 0);
+        } else {   // eight pixels of a row at a time (the pitch is a multiple of eight), zeros where x ends
+          int row = tile * 128 / g.pitch, col = tile * 128 - row * g.pitch;
+          for (int e = 0; e < 16; ++e) {
+            for (int kb = 0; kb < 2; ++kb) tma_load_3d(sX + b * kXBytes + kb * kSub + e * 1024, &tmX, &xfull[b], kb * 64, col, row);
+            if ((col += 8) == g.pitch) { col = 0; ++row; }
+          }
+        }
       }
     }
     __syncwarp();
@@ -299,10 +308,17 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
   const uint32_t box[3] = {64, 128, 1};
   const bool f16 = p.dtype == TRI_F16;
-  TRI_TRY(make_tmap_3d(&tmX, p.x, 2, f16, xd, xs, box, false));
+  if (p.n > 0) {
+    const uint64_t n = (uint64_t)p.n, nd[3] = {128, n, n}, ns[2] = {128, 128 * n};
+    const uint32_t nbox[3] = {64, 8, 1};
+    TRI_TRY(make_tmap_3d(&tmX, p.x, 2, f16, nd, ns, nbox, false));
+  } else {
+    TRI_TRY(make_tmap_3d(&tmX, p.x, 2, f16, xd, xs, box, false));
+  }
   TRI_TRY(make_tmap_3d(&tmW, p.wcat, 2, f16, wd, wsd, box, false));
   TRI_TRY(make_tmap_3d(&tmZ, p.z, 2, f16, xd, xs, box, false));
   Args a;
+  a.pitch = p.n > 0 ? p.pitch : 0;
   a.staged = p.plane % 64 == 0;
   tmA = tmB = tmX;
   if (a.staged) {
@@ -351,6 +367,7 @@ struct OutArgs {
   float* rstd;
   void* out;
   const void* residual;
+  int n, pitch;
   int* err;
 };
 
@@ -604,7 +621,14 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       swap_pieces<1>(w, lane);
       swap_pieces<2>(w, lane);
       const long long m0 = (long long)tile * 128 + quarter * 32 + (lane & ~3);
-      if (m0 < g.M) {   // M is a multiple of four
+      if (g.n > 0) {    // out has its own side: the four pixels lie in one row (the pitch is a multiple of eight)
+        const int prow = (int)m0 / g.pitch, col = (int)m0 - prow * g.pitch;
+        const long long at = (((long long)prow * g.n + col) * 128 + j * 32) / 8 + (lane & 3);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (prow < g.n && col + q < g.n)
+            (reinterpret_cast<uint4*>(g.out) + at)[q * 16] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+      } else if (m0 < g.M) {   // M is a multiple of four
         const long long at = (m0 * 128 + j * 32) / 8 + (lane & 3);
         uint4 r[4];
         if (g.residual != nullptr) {
@@ -646,7 +670,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   TRI_TRY(make_tmap_3d(&tmWg, p.w_gate, 2, f16, wd, wsd, box, false));
   OutArgs a;
   a.M = p.M; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps; a.gamma = p.gamma; a.beta = p.beta;
-  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.err = p.err;
+  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.n = p.n; a.pitch = p.pitch; a.err = p.err;
   constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 8 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_out_kernel<T>;

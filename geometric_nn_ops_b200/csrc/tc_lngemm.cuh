@@ -19,6 +19,7 @@ struct LnGateIn {
   long long M, plane;        // pixels in all; pixels per batch entry (channel-plane stride of a / b)
   float eps;
   const void* x;             // [M, 128]
+  int n = 0, pitch = 0;      // n > 0 (one batch entry): x is [n, n, 128], the pixels [pitch, pitch] are zero beyond it
   const void* gamma;         // [128] or null
   const void* beta;          // [128] or null
   const void* wcat;          // [512, 128]: rows [Wp_a; Wg_a; Wp_b; Wg_b]
@@ -51,6 +52,7 @@ struct LnGateOut {
   float* rstd;               // [M]
   void* out;                 // [M, 128]
   const void* residual = nullptr;   // [M, 128], added to the (rounded) result, or null
+  int n = 0, pitch = 0;      // n > 0 (no residual): out is [n, n, 128] of the pixels [pitch, pitch]
   int* err;
 };
 

@@ -723,7 +723,7 @@ void gate_in_operands(GemmPlan* p, const Geom& gm, const Prep& pr, const void* z
 template <typename T>
 int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* mask, const TriMulWeights* w,
                   const Prep& pr, void* z, float* mean_in, float* rstd_in, void* a_cm, void* b_cm,
-                  void* const* peer_ab = nullptr, int peer_world = 0, int peer_rank = 0) {
+                  void* const* peer_ab = nullptr, int peer_world = 0, int peer_rank = 0, int n = 0) {
   const long long M = gm.M;
   if (peer_ab == nullptr && ln_gate_in_supported(gm.dtype, M, gm.plane)) {
     // 16-bit dtypes: one kernel normalises each x tile in shared memory and feeds both halves' products from it
@@ -731,7 +731,7 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
     f.dtype = gm.dtype; f.M = M; f.plane = gm.plane; f.eps = gm.eps;
     f.x = x; f.gamma = w->norm_in_w; f.beta = w->norm_in_b; f.wcat = pr.wcat;
     f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr; f.mask = mask;
-    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.err = pr.err;
+    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.n = n; f.pitch = n > 0 ? (n + 7) / 8 * 8 : 0; f.err = pr.err;
     return ln_gate_in(st, f);
   }
   {
@@ -752,7 +752,7 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
 // ---- phase 3: t -> u (LayerNorm over channels), out = (u Wo^T + bo) * sigmoid(z Wgo^T + bgo) --------------
 template <typename T>
 int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* z, const TriMulWeights* w,
-                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true, const void* residual = nullptr) {
+                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true, const void* residual = nullptr, int n = 0) {
   const long long M = gm.M;
   if (u_channel_major(gm)) {
     // one batch entry, 16-bit dtype: t is normalised in shared memory as the MMA's MN-major operand; u (kept for
@@ -761,7 +761,7 @@ int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* 
     f.dtype = gm.dtype; f.M = M; f.eps = gm.eps; f.t_cm = t_cm; f.z = z;
     f.gamma = w->norm_out_w; f.beta = w->norm_out_b; f.w_out = w->p_out_w; f.w_gate = w->g_out_w;
     f.bias_out = (w->p_out_b || w->g_out_b) ? pr.bias_out : nullptr;
-    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.err = pr.err;
+    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.n = n; f.pitch = n > 0 ? (n + 7) / 8 * 8 : 0; f.err = pr.err;
     return ln_gate_out(st, f);
   }
   {
@@ -1015,9 +1015,10 @@ void carve_bwd(Arena& a, const Geom& gm, BwdBufs* w) {
   w->partial = a.take<float>(partial_floats());
 }
 
+// n > 0: x and out are [n, n, 128] inside the padded problem d (only where the fused 16-bit kernels run)
 template <typename T>
 int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
-              void* ws, size_t ws_size, cudaStream_t st) {
+              void* ws, size_t ws_size, cudaStream_t st, int n = 0) {
   const Geom gm = geom_of(d);
   Arena a(ws, ws_size);
   Prep pr;
@@ -1027,10 +1028,10 @@ int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMul
   else carve_saved(a, gm, &s);
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
   TRI_TRY(run_prep<T>(st, w, pr));
-  TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b));
+  TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b, nullptr, 0, 0, n));
   const bool incoming = d->direction == TRI_INCOMING;
   TRI_TRY(contraction(st, d->dtype, d->B * CW, d->N, s.a, incoming, s.b, incoming, s.t, pr.err, "tc_gemm_contract"));
-  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual);
+  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual, n);
 }
 
 template <typename T>
@@ -1208,7 +1209,7 @@ int pad_mask(cudaStream_t st, const TriMulDesc* d, const void* src, void* dst) {
 }
 
 template <typename T>
-int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void*, void* out, void* saved, void* ws,
+int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* /*residual*/, void* out, void* saved, void* ws,
                    size_t ws_size, cudaStream_t st) {
   const TriMulDesc p = whole(d);
   const size_t inner = align_up(mul_ws_bytes(&p, 0));   // first, so that the status word is the workspace's first
@@ -1217,8 +1218,10 @@ int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const T
   PadBufs b;
   carve_pad(a, &p, 0, &b);
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
-  TRI_TRY(pad_pixels(st, d, true, x, b.x));
   TRI_TRY(pad_mask<T>(st, d, mask, b.mask));
+  // the fused kernels read and write rows of their own pitch; the others work on padded copies (11 of 74 us at 203 residues)
+  if (u_channel_major(geom_of(&p))) return forward_t<T>(&p, x, b.mask, w, nullptr, out, saved, ws, inner, st, d->N);
+  TRI_TRY(pad_pixels(st, d, true, x, b.x));
   TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, nullptr, b.io, saved, ws, inner, st));
   return pad_pixels(st, d, false, b.io, out);
 }
@@ -1307,9 +1310,9 @@ bool mul_residual_supported(const TriMulDesc* d) { return mul_supported(d) && !r
 int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
                 void* ws, size_t ws_size, cudaStream_t st) {
   switch (d->dtype) {
-    case TRI_F32: return (ragged(d) ? ragged_forward<float> : forward_t<float>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
-    case TRI_BF16: return (ragged(d) ? ragged_forward<__nv_bfloat16> : forward_t<__nv_bfloat16>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
-    case TRI_F16: return (ragged(d) ? ragged_forward<__half> : forward_t<__half>)(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_F32: return ragged(d) ? ragged_forward<float>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<float>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_BF16: return ragged(d) ? ragged_forward<__nv_bfloat16>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<__nv_bfloat16>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_F16: return ragged(d) ? ragged_forward<__half>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<__half>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
   }
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
 }
