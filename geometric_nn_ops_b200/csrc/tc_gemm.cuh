@@ -183,6 +183,48 @@ template <typename T> __device__ __forceinline__ void store16(T* p, const float*
                : "memory");
 }
 
+// One step of the transposition of 4 x 4 pieces of 16 bytes over four lanes: piece p of lane l meets piece p ^ B of lane l ^ B.
+template <int B>
+__device__ __forceinline__ void swap_pieces(uint32_t (&w)[16], int lane) {
+  const bool up = (lane & B) != 0;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    if (p & B) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint32_t &lo = w[4 * p + e], &hi = w[4 * (p | B) + e];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, B);
+      if (up) lo = got;
+      else hi = got;
+    }
+  }
+}
+
+// 16 channels of this lane's pixel m (channels c ..) into rows of 128 floats; lanes are consecutive pixels, M a multiple of four
+__device__ __forceinline__ void store_rows4(float* out, const float (&v)[16], int m, int M, int c, int lane) {
+  uint32_t w[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(v[e]);
+  swap_pieces<1>(w, lane);
+  swap_pieces<2>(w, lane);
+  if (m >= M) return;
+  uint4* dst = reinterpret_cast<uint4*>(out + (long long)(m & ~3) * 128 + c) + (lane & 3);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) dst[q * 32] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+}
+// pieces that were read from rows m & ~3 .. (one of four lanes' columns each) into 16 channels of this lane's row
+template <typename T>
+__device__ __forceinline__ void swap_rows(Raw8<T>& a, Raw8<T>& b, int lane) {
+  if constexpr (sizeof(T) == 4) {
+    uint32_t w[16] = {a.w[0].x, a.w[0].y, a.w[0].z, a.w[0].w, a.w[1].x, a.w[1].y, a.w[1].z, a.w[1].w,
+                      b.w[0].x, b.w[0].y, b.w[0].z, b.w[0].w, b.w[1].x, b.w[1].y, b.w[1].z, b.w[1].w};
+    swap_pieces<1>(w, lane);
+    swap_pieces<2>(w, lane);
+    a.w[0] = make_uint4(w[0], w[1], w[2], w[3]); a.w[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    b.w[0] = make_uint4(w[8], w[9], w[10], w[11]); b.w[1] = make_uint4(w[12], w[13], w[14], w[15]);
+  }
+}
+
 template <typename TOUT>
 __device__ __forceinline__ void store_row32(TOUT* dst, const float (&v)[32], int valid, bool vec_ok) {
   if (valid >= 32 && vec_ok) {
@@ -410,8 +452,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               if constexpr (sizeof(TIN) == 2) {   // rows of 256 bytes: 32-byte loads are aligned
                 ldraw16<TIN>(dout + (grp * CPG + jj) * 32 + u * 8, dst[jj][u], dst[jj][u + 1]);
               } else {
-                dst[jj][u] = ldraw8<TIN>(dout + (grp * CPG + jj) * 32 + u * 8);
-                dst[jj][u + 1] = ldraw8<TIN>(dout + (grp * CPG + jj) * 32 + u * 8 + 8);
+                // (each lane a quarter of four rows' 16 channels: swap_rows gives it its own row's)
+                const uint4* src = reinterpret_cast<const uint4*>(dout - (long long)(lane & 3) * 128 + (grp * CPG + jj) * 32 + u * 8) + (lane & 3);
+                dst[jj][u].w[0] = __ldg(src); dst[jj][u].w[1] = __ldg(src + 32);
+                dst[jj][u + 1].w[0] = __ldg(src + 64); dst[jj][u + 1].w[1] = __ldg(src + 96);
               }
             }
         }
@@ -527,8 +571,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           for (int hf = 0; hf < 2; ++hf) {
             float y[16], gt[16];
             ld16x2_f(t_row + j * 32 + hf * 16, t_row + 128 + j * 32 + hf * 16, y, gt);
-            if (m < g.M) {
+            {
               float r0[16], r1[16];
+              if constexpr (EPI == EPI_GATE_OUT_BWD && sizeof(TIN) == 4) swap_rows(dpre[jj][hf * 2], dpre[jj][hf * 2 + 1], lane);
 #pragma unroll
               for (int uu = 0; uu < 2; ++uu) {
                 float2 d[4];
@@ -555,16 +600,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 }
               }
               // 16 channels of this pixel: one 32-byte store for 16-bit outputs (rows are 256 bytes, so it is aligned)
+              // fp32: four lanes exchange their pieces, so that a request covers 64 bytes of eight rows and not 16 of 32
               if constexpr (sizeof(TOUT) == 2) {
-                store16<TOUT>(o0 + j * 32 + hf * 16, r0);
-                if constexpr (EPI == EPI_GATE_OUT_BWD) store16<TOUT>(o1 + j * 32 + hf * 16, r1);
-              } else {
-                store8<TOUT>(o0 + j * 32 + hf * 16, r0);
-                store8<TOUT>(o0 + j * 32 + hf * 16 + 8, r0 + 8);
-                if constexpr (EPI == EPI_GATE_OUT_BWD) {
-                  store8<TOUT>(o1 + j * 32 + hf * 16, r1);
-                  store8<TOUT>(o1 + j * 32 + hf * 16 + 8, r1 + 8);
+                if (m < g.M) {
+                  store16<TOUT>(o0 + j * 32 + hf * 16, r0);
+                  if constexpr (EPI == EPI_GATE_OUT_BWD) store16<TOUT>(o1 + j * 32 + hf * 16, r1);
                 }
+              } else {
+                store_rows4(reinterpret_cast<float*>(g.out0), r0, m, g.M, j * 32 + hf * 16, lane);
+                if constexpr (EPI == EPI_GATE_OUT_BWD) store_rows4(reinterpret_cast<float*>(g.out1), r1, m, g.M, j * 32 + hf * 16, lane);
               }
             }
           }

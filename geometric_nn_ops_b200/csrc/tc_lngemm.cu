@@ -371,23 +371,6 @@ struct OutArgs {
   int* err;
 };
 
-// One step of the transposition of 4 x 4 pieces of 16 bytes over four lanes: piece p of lane l meets piece p ^ B of lane l ^ B.
-template <int B>
-__device__ __forceinline__ void swap_pieces(uint32_t (&w)[16], int lane) {
-  const bool up = (lane & B) != 0;
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    if (p & B) continue;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      uint32_t &lo = w[4 * p + e], &hi = w[4 * (p | B) + e];
-      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, B);
-      if (up) lo = got;
-      else hi = got;
-    }
-  }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ CUtensorMap tmZ,
