@@ -490,6 +490,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         // row = channel of half tm; columns: P for pixels n0..n0+127, then G for the same pixels
         const uint32_t n0 = (uint32_t)tn * 128, plane = (uint32_t)g.plane, np0 = n0 % plane;
         const bool wide16 = sizeof(TOUT) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0 && (g.ld_out & 15) == 0;
+        // fp32: 16 pixels of four channels, exchanged between four lanes (64 bytes of eight rows per request, not 16 of 32)
+        const bool wide4 = EPI == EPI_GATE_IN && sizeof(TOUT) == 4 && (g.plane & 15) == 0 && (g.N & 15) == 0 && g.peer_world == 0;
         const TIN* mask = reinterpret_cast<const TIN*>(g.aux);
         float bp = 0.f, bg = 0.f;
         if (g.bias0 != nullptr) { bp = g.bias0[tm * 256 + row]; bg = g.bias0[tm * 256 + 128 + row]; }
@@ -534,7 +536,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                   putraw8(o1[uu], i, dg);
                 }
               }
-              if (!wide16) {
+              if (!wide16 && !wide4) {
                 TOUT* dst = dst0 + off + uu * 8;
                 if constexpr (EPI == EPI_GATE_IN) {
                   if (np0 + off + uu * 8 >= plane) dst = gate_in_dst<TOUT>(g, tm, m8 / plane, row, m8 % plane);
@@ -543,6 +545,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                   straw8<TOUT>(dst, o0[uu]);
                   straw8<TOUT>(dst + 128 * g.ld_out, o1[uu]);
                 }
+              }
+            }
+            if constexpr (sizeof(TOUT) == 4 && EPI == EPI_GATE_IN) {
+              if (wide4 && n0 + off < (uint32_t)g.N) {
+                TOUT* dst = np0 + off >= plane ? gate_in_dst<TOUT>(g, tm, (n0 + off) / plane, row, (n0 + off) % plane) : dst0 + off;
+                swap_rows(o0[0], o0[1], lane);
+                uint4* at = reinterpret_cast<uint4*>(dst - (long long)(lane & 3) * g.plane) + (lane & 3);
+                const long long step = g.plane / 4;
+                at[0] = o0[0].w[0]; at[step] = o0[0].w[1]; at[2 * step] = o0[1].w[0]; at[3 * step] = o0[1].w[1];
               }
             }
             if constexpr (sizeof(TOUT) == 2) {
