@@ -225,6 +225,29 @@ __device__ __forceinline__ void swap_rows(Raw8<T>& a, Raw8<T>& b, int lane) {
   }
 }
 
+// 32 columns of this lane's row, rows `ld` apart, all four rows of a lane group valid or none: the lanes exchange their 16-byte
+// pieces, so that a request covers 64 bytes of eight rows
+template <typename TOUT>
+__device__ __forceinline__ void store_rows32(TOUT* dst, const float (&v)[32], long long ld, bool valid, int lane) {
+  constexpr int E = 16 / sizeof(TOUT), H = sizeof(TOUT) / 2;   // elements of a piece; groups of four pieces
+  TOUT* at = dst + (lane & 3) * (E - ld);
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    uint32_t w[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      if constexpr (sizeof(TOUT) == 4) w[e] = __float_as_uint(v[h * 16 + e]);
+      else w[e] = pack2<TOUT>(v[2 * e], v[2 * e + 1]);
+    }
+    swap_pieces<1>(w, lane);
+    swap_pieces<2>(w, lane);
+    if (valid) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(at + q * ld + h * 4 * E) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+    }
+  }
+}
+
 template <typename TOUT>
 __device__ __forceinline__ void store_row32(TOUT* dst, const float (&v)[32], int valid, bool vec_ok) {
   if (valid >= 32 && vec_ok) {
@@ -484,7 +507,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) if (n + i < g.N) v[i] += g.bias0[n + i];
           }
-          if (m < g.M && n < g.N) store_row32<TOUT>(out + n, v, g.N - n, vec_ok);
+          if ((g.M & 3) == 0 && vec_ok && g.N - n >= 32) store_rows32<TOUT>(out + n, v, g.ld_out, m < g.M, lane);
+          else if (m < g.M && n < g.N) store_row32<TOUT>(out + n, v, g.N - n, vec_ok);
         }
       } else if constexpr (EPI == EPI_GATE_IN || EPI == EPI_GATE_IN_BWD) {
         // row = channel of half tm; columns: P for pixels n0..n0+127, then G for the same pixels
