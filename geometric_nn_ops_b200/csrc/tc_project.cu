@@ -1,5 +1,6 @@
-// Fused attention-input projection for the pair stack: LayerNorm(z) and the q / k / v / pair-bias projections in two
-// launches, written in the layouts the triangle-attention kernels read.
+// Fused attention-input projection for the pair stack: LayerNorm(z) and the q / k / v / pair-bias projections, written in the
+// layouts the triangle-attention kernels read.  16-bit types up to 384 columns take one kernel (tc_lnproject.cu), the others
+// these two launches:
 //
 //   ln_bias_kernel   z [M, 128] -> zn = LayerNorm(z) [M, 128] (input dtype), and the pair bias
 //                    bias[h][m] = sum_c zn[m][c] Wb[h][c] for h < H, computed from the fp32 row while it is in

@@ -85,7 +85,7 @@ def _fused_weights(w):
 def project_attention_inputs(z, w):
     """``z`` ``[B, R, N, C]`` (R rows) -> q, k, v ``[B, R, N, H, D]`` and this rows' bias ``[B, H, R, N]``.
 
-    On the GPU with C = 128 this is the library's fused projection (one LayerNorm + bias kernel, one GEMM); the
+    On the GPU with C = 128 this is the library's fused projection kernel; the
     torch composition below it defines what that computes and serves every other case."""
     if z.is_cuda and z.shape[-1] == 128 and z.dtype in (torch.bfloat16, torch.float16) and not torch.is_grad_enabled():
         w_qkv, w_bias = _fused_weights(w)

@@ -1,8 +1,8 @@
 """Fused input projection of triangle attention in a pair stack: LayerNorm(z) -> q, k, v and the pair bias.
 
-Two launches of the CUDA library (``tri_attn_project``): a LayerNorm kernel that also projects the per-head pair
-bias while the normalised row is in registers, and one tcgen05 GEMM that writes q, k and v side by side in a single
-``[pixels, 3*H*D]`` buffer.  The returned q, k, v are strided views of that buffer in the ``[B, rows, N, H, D]``
+One kernel of the CUDA library (``tri_attn_project``) for 16-bit types -- LayerNorm in shared memory, tcgen05 products
+with resident weights -- or two (a LayerNorm + bias kernel and a GEMM) for TF32 and wide projections.  q, k and v are written
+side by side in a single ``[pixels, 3*H*D]`` buffer.  The returned q, k, v are strided views of that buffer in the ``[B, rows, N, H, D]``
 layout :func:`triangle_attention` takes (its kernels read strides, so nothing is copied), and the bias comes back
 head-major, ready to be used as ``[B, 1, H, N, N]``.
 
