@@ -59,10 +59,10 @@ template <int HD> struct Geo {
   static constexpr int SMEM = OFF_BAR + 256 + 1024;      // + alignment slack
 };
 
-// additive key-mask terms of every (batch, row): 0 for a kept key, -sentinel for a masked key, -inf beyond N; rows of
+// additive key-mask terms of every (batch, row): 0 for a kept key, -1e9 for a masked key, -inf beyond N; rows of
 // npad.  Also clears the error word of the launches that follow.
 __global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b, int64_t st_s, int B, int S, int N, int npad,
-                                  float sentinel, float* __restrict__ out, int* err) {
+                                  float* __restrict__ out, int* err) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx == 0) *err = 0;
   if (idx >= (long long)B * S * npad) return;
@@ -71,7 +71,7 @@ __global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b
   const int s = bs % S, b = bs / S;
   float v = 0.f;
   if (k >= N) v = -INFINITY;
-  else if (mask != nullptr) v = sentinel * ((mask[b * st_b + s * st_s + k] ? 1.0f : 0.0f) - 1.0f);
+  else if (mask != nullptr) v = kMaskSentinel * ((mask[b * st_b + s * st_s + k] ? 1.0f : 0.0f) - 1.0f);
   out[idx] = v;
 }
 
@@ -1365,7 +1365,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     KernelTimer kt("tc_attn_delta", st, 0.0, 2.0 * tensor_bytes);
     {
       const long long n = (long long)d->B * d->n_seq * npad;
-      mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, kMaskSentinel, mask_terms, err);
+      mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, mask_terms, err);
       TRI_LAUNCH_OK();
     }
     if (npad != d->n_res) TRI_CUDA_OK(cudaMemsetAsync(prep, 0, 3 * prep_plane * sizeof(float), st));
@@ -1495,7 +1495,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0;
   {
     const long long n = (long long)d->B * d->n_seq * a.npad;
-    mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, a.npad, rows ? kMaskLog2 : kMaskSentinel, mask_terms, err);
+    mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, a.npad, mask_terms, err);
     TRI_LAUNCH_OK();
   }
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;

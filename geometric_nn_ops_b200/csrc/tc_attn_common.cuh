@@ -9,7 +9,6 @@ namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMaskSentinel = 1e9f;
-constexpr float kMaskLog2 = 1442695040.0f;   // the sentinel in units of log 2
 
 // byte offset of 16-byte chunk `g` (0..15, 8 elements each) of row r inside a [128 x 128] two-block SW128 tile
 __device__ __forceinline__ int sw128_chunk(int r, int g) {

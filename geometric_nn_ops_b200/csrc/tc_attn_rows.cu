@@ -5,12 +5,18 @@
 // of 64 keys; the bias tile of a step comes to shared memory once for the three of them.  Otherwise a group is on its
 // own: its Q, K, V tiles, its 160 TMEM columns and the lane that issues its copies and products.
 //
-// Per step and thread (one query row, 64 keys), sixteen logits at a time, in units of log 2:
-//   x = bias log2e + (S scale log2e + mask term) -> P = 2^(x - m), 16 bit -> O += P V.
+// Per step and thread (one query row, 64 keys), sixteen logits at a time:
+//   x = (S scale + mask term) + bias -> P = 2^(x log2e - m log2e), 16 bit -> O += P V.
+// The logits are rounded as the backward rounds them, in natural units: beside a bias of -1e8 a row's other terms are lost
+// to both, and in units of log 2 the type's lowest value would overflow.
 // One sweep without a maximum: P is formed against the reference m of the row (the largest of its first four logits to
 // start with).  P, its sum and O are floating point, so a reference that lags the maximum by a factor of up to kTooBig
 // loses nothing; the sum of a step shows whether a row has outgrown it, and then O and the sum are rescaled and the step
 // is done again.  S stays in TMEM until the check: P is stored over it afterwards.
+// m log2e is rounded, so every P of a row carries the factor 2^r, r = m log2e - fl(m log2e), which the statistics take out
+// again: 1 within 2^-12 where |m| is below 2^11.  A warp with a row where it is not (masked, or held up, by its bias or its
+// mask) does its first step again, and from then on forms P from the differences, 2^((x - m) log2e): one more packed
+// instruction per two logits.
 //
 // S is double buffered and P(c) takes the columns of S(c).  After P(c) the issuing lane sends P V(c) and S(c + 2),
 // which run in that order, so S(c + 1) is there before a thread asks for it and one arrival per step (p_ready) is all
@@ -22,6 +28,7 @@
 // pipe, against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
 // also read 2 bytes of bias per logit from L2; here 0.67).
 #include <algorithm>
+#include <type_traits>
 
 #include "tc_attn_common.cuh"
 #include "tc_attn_rows.cuh"
@@ -38,14 +45,14 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 struct RowsArgs {
   int B, S, N, H, D;
-  float scale2;              // scale * log2e
+  float scale;
   void* o;
   int64_t o_st[4];
   float* stats;              // [2][B][S][H][N]: row maximum, log row sum
   const float* mask_terms;
   int npad;
   int bias_b_mul;
-  int rows_per_item;         // groups in use (fewer where a quad per CTA would leave SMs idle)
+  int rows_per_item;         // groups in use (fewer where a triple per CTA would leave SMs idle)
   uint32_t idesc_s, idesc_pv;
   int* err;
 };
@@ -87,13 +94,13 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint8_t* smem = align1024(smem_raw);
   GroupBars* bars = reinterpret_cast<GroupBars*>(smem + M::OFF_BAR);
   uint64_t* b_full = reinterpret_cast<uint64_t*>(bars + kGroups);   // [kBiasStages]
-  uint64_t* b_free = b_full + kBiasStages;                          // [kBiasStages]: 16 warps
+  uint64_t* b_free = b_full + kBiasStages;                          // [kBiasStages]: the softmax warps of the groups in use
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_free + kBiasStages);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qblocks = (a.N + 127) / 128, nk = (a.N + 63) / 64;
-  const int R = a.rows_per_item, squads = (a.S + R - 1) / R;
-  const long long items = (long long)qblocks * a.H * squads * a.B;
+  const int R = a.rows_per_item, triples = (a.S + R - 1) / R;
+  const long long items = (long long)qblocks * a.H * triples * a.B;
   const int my_items = blockIdx.x < items ? (int)((items - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
   struct Item { int q0, h, s0, b; };
   auto item_of = [&](int n) {
@@ -101,8 +108,8 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     Item it;
     it.q0 = (int)(z % (unsigned)qblocks) * 128; z /= (unsigned)qblocks;
     it.h = (int)(z % (unsigned)a.H); z /= (unsigned)a.H;
-    it.s0 = (int)(z % (unsigned)squads) * R;
-    it.b = (int)(z / (unsigned)squads);
+    it.s0 = (int)(z % (unsigned)triples) * R;
+    it.b = (int)(z / (unsigned)triples);
     return it;
   };
 
@@ -232,7 +239,11 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     GroupBars& gb = bars[g];
     const uint32_t t_row = tmem_base + g * COLS + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t mask_s = smem_u32(smem + M::OFF_M) + g * 256, bias_row = smem_u32(smem + M::OFF_BIAS) + r * 128 + ((r & 7) << 4);
-    const float2 sc2 = splat(a.scale2), l2e2 = splat(kLog2e);
+    const float2 sc2 = splat(a.scale), l2e2 = splat(kLog2e);
+    // the exponent r of the factor that P carries against the reference m (see the top), and whether a row goes without
+    auto residue = [](float m) { return fmaf(m, kLog2e, -(m * kLog2e)); };
+    auto large = [&](float m) { return !(fabsf(residue(m)) <= 0.000244140625f); };
+    auto factor = [&](float m) { return large(m) ? 0.0f : residue(m); };
     int c = 0, bstg = 0;
     uint32_t bph = 0;
     bool early_s = false, early_b = false;
@@ -260,13 +271,11 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             (reinterpret_cast<uint4*>(a.o) + po)[h] = pk;
           }
         }
-        // Natural units.  The largest of the steps' sums over 64 keys is 1 to 64 times the largest P, so that m plus
-        // log2(sum / 64) lies at most 6 below the row's maximum; m itself is one of the logits.  A fully masked row keeps
-        // the sentinel's exact value, which the backward forms again.
-        const bool masked = pm < -1e8f;
-        const float lift = masked ? 0.f : fmaxf(__log2f(pseen) - 6.0f, 0.f);
-        a.stats[pstat] = masked ? fmaf(pm + kMaskLog2, kLn2, -kMaskSentinel) : (pm + lift) * kLn2;
-        a.stats[(long long)a.B * a.S * a.H * a.N + pstat] = logf(pl) - lift * kLn2;
+        // The largest of the steps' sums over 64 keys is 1 to 64 times the largest P, so that m plus log(sum / 64) lies at
+        // most 6 ln 2 below the row's maximum.  What m takes on of that (nothing, beside a large m) leaves the logarithm.
+        const float top = pm + fmaxf(__log2f(pseen) - 6.0f, 0.f) * kLn2;
+        a.stats[pstat] = top;
+        a.stats[(long long)a.B * a.S * a.H * a.N + pstat] = (logf(pl) - factor(pm) * kLn2) - (top - pm);
       }
     };
     for (int n = 0; g < R && n < my_items && ok; ++n) {
@@ -283,6 +292,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       float m = -INFINITY, l = 0.f;   // reference, sum of P
       float seen = 0.f;               // largest sum of a step against this reference
+      bool by_diff = false;           // P from differences (the same for the whole warp)
       for (int j = 0; j < nk; ++j, ++c) {
         if (!early_s && !mbar_wait(&gb.mma[c & 1], (c >> 1) & 1, a.err, 58)) ok = false;
         if (!early_b && !mbar_wait(&b_full[bstg], bph, a.err, 57)) ok = false;
@@ -299,45 +309,60 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
-              if constexpr (HB) v = __ffma2_rn(unpack2<T>(bw[i]), l2e2, v);
+              if constexpr (HB) v = __fadd2_rn(v, unpack2<T>(bw[i]));
               x[u * 4 + i] = v;
             }
           }
         };
-        auto exps = [&](const float2 (&x)[8], float2 nm, uint32_t* w, float2& sum) {
+        auto subtract = [](float2 (&x)[8], float m) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = __fadd2_rn(x[i], splat(-m));
+        };
+        auto exps = [&](const float2 (&x)[8], float2 nm2, uint32_t* w, float2& sum) {   // P = 2^(x log2e + nm2)
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const float2 e = __fadd2_rn(x[i], nm);
+            const float2 e = __ffma2_rn(x[i], l2e2, nm2);
             const float2 p = make_float2(ex2_approx(e.x), ex2_approx(e.y));
             sum = __fadd2_rn(sum, p);
             w[i] = pack2<T>(p.x, p.y);
           }
         };
-        // P = 2^(x - m) of this thread's 64 keys and their sum
+        // P of this thread's 64 keys and their sum
         float2 ps = make_float2(0.f, 0.f);
         uint32_t pw[32], ra[16], rb[16];
-        auto chunk = [&](uint32_t (&cur)[16], uint32_t (&nxt)[16], int q) {   // sixteen keys; the next sixteen on their way
+        auto chunk = [&](auto diff, uint32_t (&cur)[16], uint32_t (&nxt)[16], int q) {   // sixteen keys; the next sixteen on their way
           ld_wait16(cur);
           if (q < 3) tmem_ld_32x16(t_s + (q + 1) * 16, nxt);
           float2 x[8];
           logits(cur, q, x);
-          if (q == 0) m = j > 0 ? m : fmaxf(fmaxf(x[0].x, x[0].y), fmaxf(x[1].x, x[1].y));   // (key 0 is in range: finite)
-          exps(x, splat(-m), pw + q * 8, ps);
+          if constexpr (diff.value) {
+            subtract(x, m);
+            exps(x, splat(factor(m)), pw + q * 8, ps);
+          } else {
+            if (q == 0) m = j > 0 ? m : fmaxf(fmaxf(x[0].x, x[0].y), fmaxf(x[1].x, x[1].y));
+            exps(x, splat(-(m * kLog2e)), pw + q * 8, ps);
+          }
         };
-        tmem_ld_32x16(t_s, ra);
-        chunk(ra, rb, 0);
-        chunk(rb, ra, 1);
-        chunk(ra, rb, 2);
-        chunk(rb, ra, 3);
+        auto sweep = [&](auto diff) {
+          tmem_ld_32x16(t_s, ra);
+          chunk(diff, ra, rb, 0);
+          chunk(diff, rb, ra, 1);
+          chunk(diff, ra, rb, 2);
+          chunk(diff, rb, ra, 3);
+        };
+        if (by_diff) sweep(std::true_type{});
+        else sweep(std::false_type{});
         // whether the next step's S and bias tile are there: asked now, needed at the top
         early_s = mbar_test(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1);
         early_b = mbar_test(&b_full[bstg + 1 == kBiasStages ? 0 : bstg + 1], bstg + 1 == kBiasStages ? bph ^ 1 : bph);
         float sum = ps.x + ps.y;
-        if (!__any_sync(0xffffffffu, !(sum < kTooBig))) {
+        const bool redo = __any_sync(0xffffffffu, !(sum < kTooBig) || (j == 0 && large(m)));
+        if (!redo) {
           tmem_st_32x32(t_s, pw);   // over the S values this warp has read: 64 keys as 32 packed columns
         } else {
-          // Some row of the warp outgrew its reference: take the maximum of the step, scale by 2^(m - m_new) the sum and O
-          // (once P V of the step before is done), and form P again.  (Sixteen keys' P end before the next sixteen's S.)
+          // Some row of the warp outgrew its reference, or starts from a large one: take the maximum of the step, scale the sum and O by
+          // 2^((m - m_new) log2e) and the quotient of the factors (once P V of the step before is done), and form P again.
+          // (Sixteen keys' P end before the next sixteen's S.)
           float top = m;
 #pragma unroll 1
           for (int q = 0; q < 4; ++q) {
@@ -348,7 +373,8 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
             for (int i = 0; i < 8; ++i) top = fmax3(top, x[i].x, x[i].y);
           }
-          const float alpha = ex2_approx(m - top);
+          top = fmaxf(top, -3.402823466e38f);   // (no finite logit yet: P = 2^-inf)
+          const float fac = factor(top), alpha = ex2_approx((m - top) * kLog2e + (fac - factor(m)));
           m = top;
           l *= alpha;
           if (j > 0) {
@@ -372,13 +398,15 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             tmem_ld_32x16(t_s + q * 16, ra);
             ld_wait16(ra);
             logits(ra, q, x);
-            exps(x, splat(-m), w, ps);
+            subtract(x, m);
+            exps(x, splat(fac), w, ps);
             tmem_st_32x8(t_s + q * 8, w);
           }
           sum = ps.x + ps.y;
         }
         l += sum;
         seen = fmaxf(seen, sum);
+        if (redo) by_diff = __any_sync(0xffffffffu, large(m));
         if (j == 0 && pend) finish(c - 1);   // the row before this one
         tmem_st_wait();
         tc_fence_before_sync();
@@ -420,7 +448,7 @@ int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void
   TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, 32));
   RowsArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D;
-  a.scale2 = d->scale * kLog2e;
+  a.scale = d->scale;
   a.o = o;
   for (int i = 0; i < 4; ++i) a.o_st[i] = d->o_st[i];
   a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;

@@ -13,7 +13,7 @@ int qkv_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, const in
 // its offsets are 32-bit: rows of statistics, and O in units of 8 elements
 bool attn_fwd_rows_fits(const TriAttnDesc* d);
 // tbias: map over the bias with boxes of 128 queries x 64 keys, or null.  mask_terms: [B][S][npad] additive key-mask
-// terms in units of log 2 (0, -kMaskLog2, -inf beyond N).
+// terms (0, -1e9, -inf beyond N).
 int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void* v, const CUtensorMap* tbias,
                   bool bias_batched, void* o, float* stats, const float* mask_terms, int* err, cudaStream_t st);
 
