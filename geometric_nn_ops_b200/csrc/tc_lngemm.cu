@@ -47,7 +47,8 @@ struct Args {
   void* b_cm;
   float* mean;
   float* rstd;
-  int pitch;            // 0, or the padded side: x has its own
+  int n, pitch;         // as in LnGateIn
+  int own_pitch;
   int staged;           // a / b leave through shared memory by TMA (planes of whole 64-pixel chunks)
   int* err;
 };
@@ -112,7 +113,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int b = i % kXBufs;
         if (!mbar_wait(&xempty[b], ((i / kXBufs) & 1) ^ 1, g.err, 10)) break;
         mbar_expect_tx(&xfull[b], kXBytes);
-        if (g.pitch == 0) {
+        if (!g.own_pitch) {
           for (int kb = 0; kb < 2; ++kb) tma_load_3d(sX + b * kXBytes + kb * kSub, &tmX, &xfull[b], kb * 64, tile * 128, 0);
         } else {   // eight pixels of a row at a time (the pitch is a multiple of eight), zeros where x ends
           int row = tile * 128 / g.pitch, col = tile * 128 - row * g.pitch;
@@ -187,7 +188,8 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       const float ms = ((s0.x + s0.y) + (s1.x + s1.y)) * (1.0f / 128);          // mean - K
       const float mu = ms - nk.x;
       const float var = fmaxf(((q0.x + q0.y) + (q1.x + q1.y)) * (1.0f / 128) - ms * ms, 0.f);
-      const float rs = 1.0f / sqrtf(var + g.eps);
+      const long long m = (long long)tile * 128 + r;
+      const float rs = pixel_rstd(var, g.eps, m, g.n, g.pitch);
       const float2 nmu = make_float2(-mu, -mu);
       const float2 rs2 = make_float2(rs, rs);
 #pragma unroll 4
@@ -202,7 +204,6 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         for (int e = 0; e < 4; ++e) o[e] = __ffma2_rn(__fadd2_rn(v[e], nmu), __fmul2_rn(rs2, gm[e]), bt[e]);
         *p = pack8p<T>(o);
       }
-      const long long m = (long long)tile * 128 + r;
       if (m < g.M) {
         g.mean[m] = mu; g.rstd[m] = rs;
         if (mask != nullptr) s_mask[(i % kMaskRing) * 128 + r] = mask[m];
@@ -308,7 +309,7 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
   const uint32_t box[3] = {64, 128, 1};
   const bool f16 = p.dtype == TRI_F16;
-  if (p.n > 0) {
+  if (p.own_pitch) {
     const uint64_t n = (uint64_t)p.n, nd[3] = {128, n, n}, ns[2] = {128, 128 * n};
     const uint32_t nbox[3] = {64, 8, 1};
     TRI_TRY(make_tmap_3d(&tmX, p.x, 2, f16, nd, ns, nbox, false));
@@ -318,7 +319,7 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   TRI_TRY(make_tmap_3d(&tmW, p.wcat, 2, f16, wd, wsd, box, false));
   TRI_TRY(make_tmap_3d(&tmZ, p.z, 2, f16, xd, xs, box, false));
   Args a;
-  a.pitch = p.n > 0 ? p.pitch : 0;
+  a.n = p.n; a.pitch = p.pitch; a.own_pitch = p.own_pitch;
   a.staged = p.plane % 64 == 0;
   tmA = tmB = tmX;
   if (a.staged) {
@@ -367,7 +368,7 @@ struct OutArgs {
   float* rstd;
   void* out;
   const void* residual;
-  int n, pitch;
+  int n, pitch, own_pitch;   // as in LnGateOut
   int* err;
 };
 
@@ -536,10 +537,10 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
         float dev = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) dev = fmaf(pm[k] - m, pm[k] - m, dev);
-        const float rs = 1.0f / sqrtf((m2 + 16.f * dev) * (1.0f / 128) + g.eps);
+        const long long px = (long long)tile * 128 + tid;
+        const float rs = pixel_rstd((m2 + 16.f * dev) * (1.0f / 128), g.eps, px, g.n, g.pitch);
         s_mean[tid] = m;
         s_rstd[tid] = rs;
-        const long long px = (long long)tile * 128 + tid;
         if (px < g.M) { g.mean[px] = m; g.rstd[px] = rs; }
       }
       mbar_arrive(&nsync[1]);
@@ -604,7 +605,7 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       swap_pieces<1>(w, lane);
       swap_pieces<2>(w, lane);
       const long long m0 = (long long)tile * 128 + quarter * 32 + (lane & ~3);
-      if (g.n > 0) {    // out has its own side: the four pixels lie in one row (the pitch is a multiple of eight)
+      if (g.own_pitch) {    // out has its own side: the four pixels lie in one row (the pitch is a multiple of eight)
         const int prow = (int)m0 / g.pitch, col = (int)m0 - prow * g.pitch;
         const long long at = (((long long)prow * g.n + col) * 128 + j * 32) / 8 + (lane & 3);
 #pragma unroll
@@ -653,7 +654,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   TRI_TRY(make_tmap_3d(&tmWg, p.w_gate, 2, f16, wd, wsd, box, false));
   OutArgs a;
   a.M = p.M; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps; a.gamma = p.gamma; a.beta = p.beta;
-  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.n = p.n; a.pitch = p.pitch; a.err = p.err;
+  a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.n = p.n; a.pitch = p.pitch; a.own_pitch = p.own_pitch; a.err = p.err;
   constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 8 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_out_kernel<T>;

@@ -14,12 +14,27 @@
 namespace tri {
 namespace tc {
 
+// Does pixel px of planes of [pitch, pitch] pixels that hold [n, n] lie beyond them?  (n = 0: nothing does)
+__device__ __forceinline__ bool pad_pixel(long long px, int n, int pitch) {
+  if (n == 0) return false;
+  const long long plane = (long long)pitch * pitch;
+  const int p = (int)(px % plane);
+  return p / pitch >= n || p % pitch >= n;
+}
+// 1 / sqrt(var + eps) of pixel px.  A pad's variance is zero, and with eps = 0 its infinity, times its zeros, would reach every
+// pixel through the contraction: 0 there, so that a pad is normalised to the bias as with any other eps.
+__device__ __forceinline__ float pixel_rstd(float var, float eps, long long px, int n, int pitch) {
+  const float rs = 1.0f / sqrtf(var + eps);
+  return isinf(rs) && pad_pixel(px, n, pitch) ? 0.0f : rs;
+}
+
 struct LnGateIn {
   int dtype;                 // TRI_BF16 / TRI_F16
   long long M, plane;        // pixels in all; pixels per batch entry (channel-plane stride of a / b)
   float eps;
   const void* x;             // [M, 128]
-  int n = 0, pitch = 0;      // n > 0 (one batch entry): x is [n, n, 128], the pixels [pitch, pitch] are zero beyond it
+  int n = 0, pitch = 0;      // n > 0: planes of [pitch, pitch] pixels hold [n, n]; x is zero beyond
+  bool own_pitch = false;    // x is [n, n, 128] (one batch entry) and not [M, 128]
   const void* gamma;         // [128] or null
   const void* beta;          // [128] or null
   const void* wcat;          // [512, 128]: rows [Wp_a; Wg_a; Wp_b; Wg_b]
@@ -52,7 +67,8 @@ struct LnGateOut {
   float* rstd;               // [M]
   void* out;                 // [M, 128]
   const void* residual = nullptr;   // [M, 128], added to the (rounded) result, or null
-  int n = 0, pitch = 0;      // n > 0 (no residual): out is [n, n, 128] of the pixels [pitch, pitch]
+  int n = 0, pitch = 0;      // n > 0: the pixels [pitch, pitch] hold [n, n], t is zero beyond
+  bool own_pitch = false;    // out is [n, n, 128] (no residual) and not [M, 128]
   int* err;
 };
 

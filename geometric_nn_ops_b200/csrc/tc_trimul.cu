@@ -125,7 +125,7 @@ constexpr int kLnRowPairs = 4;   // row pairs per warp and pass (8 rows)
 
 template <typename T>
 __global__ void __launch_bounds__(256) ln_rows_kernel(const T* __restrict__ x, const T* gamma, const T* beta, float eps,
-                                                       long long M, T* __restrict__ z, float* mean, float* rstd) {
+                                                       long long M, T* __restrict__ z, float* mean, float* rstd, int n, int pitch) {
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long long row0 = (blockIdx.x * 8LL + (threadIdx.x >> 5)) * (2 * kLnRowPairs) + half;
   float gm[8], bt[8];
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) ln_rows_kernel(const T* __restrict__ x, c
     float q = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) { v[p][i] -= mu; q += v[p][i] * v[p][i]; }
-    const float rs = 1.0f / sqrtf(half_warp_sum(q) * (1.0f / CW) + eps);
+    const float rs = pixel_rstd(half_warp_sum(q) * (1.0f / CW), eps, row, n, pitch);
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[p][i] = v[p][i] * rs * gm[i] + bt[i];
     if (row < M) {
@@ -321,7 +321,7 @@ __device__ __forceinline__ void store_cm_tile(const float* tile, T* dst, long lo
 // bytes per lane (256 or 512 contiguous bytes per warp).
 template <typename T>
 __global__ void __launch_bounds__(256, 4) ln_cm_kernel(const T* t_cm, const T* gamma, const T* beta, float eps,
-                                                        long long M, long long NN, T* u, float* mean, float* rstd) {
+                                                        long long M, long long NN, T* u, float* mean, float* rstd, int n, int pitch) {
   __shared__ float tile[TP * TROW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float gm[4] = {1.f, 1.f, 1.f, 1.f}, bt[4] = {0.f, 0.f, 0.f, 0.f};
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256, 4) ln_cm_kernel(const T* t_cm, const T* g
       float q = 0.f;
 #pragma unroll
       for (int k = 0; k < 4; ++k) { v[k] -= mu; q += v[k] * v[k]; }
-      const float rs = 1.0f / sqrtf(warp_sum(q) * (1.0f / CW) + eps);
+      const float rs = pixel_rstd(warp_sum(q) * (1.0f / CW), eps, m, n, pitch);
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = v[k] * rs * gm[k] + bt[k];
       store4(u + m * CW + lane * 4, v);
@@ -637,6 +637,7 @@ struct Geom {
   int dtype;
   float eps;
   long long M, plane;
+  int n = 0, pitch = 0;      // n > 0: the planes of [pitch, pitch] pixels hold [n, n] and pads
   bool sharded = false;      // a row shard of a multi-GPU op (other streams' kernels run beside this one's)
   size_t es() const { return dtype == TRI_F32 ? 4 : 2; }
   double unit() const { return (double)M * CW * es(); }
@@ -723,7 +724,7 @@ void gate_in_operands(GemmPlan* p, const Geom& gm, const Prep& pr, const void* z
 template <typename T>
 int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* mask, const TriMulWeights* w,
                   const Prep& pr, void* z, float* mean_in, float* rstd_in, void* a_cm, void* b_cm,
-                  void* const* peer_ab = nullptr, int peer_world = 0, int peer_rank = 0, int n = 0) {
+                  void* const* peer_ab = nullptr, int peer_world = 0, int peer_rank = 0, bool own_pitch = false) {
   const long long M = gm.M;
   if (peer_ab == nullptr && ln_gate_in_supported(gm.dtype, M, gm.plane)) {
     // 16-bit dtypes: one kernel normalises each x tile in shared memory and feeds both halves' products from it
@@ -731,13 +732,13 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
     f.dtype = gm.dtype; f.M = M; f.plane = gm.plane; f.eps = gm.eps;
     f.x = x; f.gamma = w->norm_in_w; f.beta = w->norm_in_b; f.wcat = pr.wcat;
     f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr; f.mask = mask;
-    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.n = n; f.pitch = n > 0 ? (n + 7) / 8 * 8 : 0; f.err = pr.err;
+    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.err = pr.err;
     return ln_gate_in(st, f);
   }
   {
     KernelTimer kt("tc_ln_rows", st, 0.0, 2.0 * gm.unit());
     ln_rows_kernel<T><<<cdiv(M, 8 * 2 * kLnRowPairs), 256, 0, st>>>((const T*)x, (const T*)w->norm_in_w, (const T*)w->norm_in_b, gm.eps,
-                                                  M, (T*)z, mean_in, rstd_in);
+                                                  M, (T*)z, mean_in, rstd_in, gm.n, gm.pitch);
     TRI_LAUNCH_OK();
   }
   GemmPlan p;
@@ -752,7 +753,7 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
 // ---- phase 3: t -> u (LayerNorm over channels), out = (u Wo^T + bo) * sigmoid(z Wgo^T + bgo) --------------
 template <typename T>
 int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* z, const TriMulWeights* w,
-                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true, const void* residual = nullptr, int n = 0) {
+                 const Prep& pr, void* u, float* mean_out, float* rstd_out, void* out, bool keep_u = true, const void* residual = nullptr, bool own_pitch = false) {
   const long long M = gm.M;
   if (u_channel_major(gm)) {
     // one batch entry, 16-bit dtype: t is normalised in shared memory as the MMA's MN-major operand; u (kept for
@@ -761,13 +762,13 @@ int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* 
     f.dtype = gm.dtype; f.M = M; f.eps = gm.eps; f.t_cm = t_cm; f.z = z;
     f.gamma = w->norm_out_w; f.beta = w->norm_out_b; f.w_out = w->p_out_w; f.w_gate = w->g_out_w;
     f.bias_out = (w->p_out_b || w->g_out_b) ? pr.bias_out : nullptr;
-    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.n = n; f.pitch = n > 0 ? (n + 7) / 8 * 8 : 0; f.err = pr.err;
+    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.err = pr.err;
     return ln_gate_out(st, f);
   }
   {
     KernelTimer kt("tc_ln_cm", st, 0.0, 2.0 * gm.unit());
     ln_cm_kernel<T><<<kLnCmBlocks, 256, 0, st>>>((const T*)t_cm, (const T*)w->norm_out_w, (const T*)w->norm_out_b, gm.eps,
-                                              M, gm.plane, (T*)u, mean_out, rstd_out);
+                                              M, gm.plane, (T*)u, mean_out, rstd_out, gm.n, gm.pitch);
     TRI_LAUNCH_OK();
   }
   GemmPlan p;
@@ -1015,11 +1016,12 @@ void carve_bwd(Arena& a, const Geom& gm, BwdBufs* w) {
   w->partial = a.take<float>(partial_floats());
 }
 
-// n > 0: x and out are [n, n, 128] inside the padded problem d (only where the fused 16-bit kernels run)
+// n > 0: the padded problem d holds [n, n] pixels; own_pitch: x and out are [n, n, 128] (only where the fused 16-bit kernels run)
 template <typename T>
 int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
-              void* ws, size_t ws_size, cudaStream_t st, int n = 0) {
-  const Geom gm = geom_of(d);
+              void* ws, size_t ws_size, cudaStream_t st, int n = 0, bool own_pitch = false) {
+  Geom gm = geom_of(d);
+  if (n > 0) { gm.n = n; gm.pitch = d->N; }
   Arena a(ws, ws_size);
   Prep pr;
   carve_prep(a, gm.es(), &pr);
@@ -1028,10 +1030,10 @@ int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMul
   else carve_saved(a, gm, &s);
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
   TRI_TRY(run_prep<T>(st, w, pr));
-  TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b, nullptr, 0, 0, n));
+  TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b, nullptr, 0, 0, own_pitch));
   const bool incoming = d->direction == TRI_INCOMING;
   TRI_TRY(contraction(st, d->dtype, d->B * CW, d->N, s.a, incoming, s.b, incoming, s.t, pr.err, "tc_gemm_contract"));
-  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual, n);
+  return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual, own_pitch);
 }
 
 template <typename T>
@@ -1220,9 +1222,9 @@ int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const T
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
   TRI_TRY(pad_mask<T>(st, d, mask, b.mask));
   // the fused kernels read and write rows of their own pitch; the others work on padded copies (11 of 74 us at 203 residues)
-  if (u_channel_major(geom_of(&p))) return forward_t<T>(&p, x, b.mask, w, nullptr, out, saved, ws, inner, st, d->N);
+  if (u_channel_major(geom_of(&p))) return forward_t<T>(&p, x, b.mask, w, nullptr, out, saved, ws, inner, st, d->N, true);
   TRI_TRY(pad_pixels(st, d, true, x, b.x));
-  TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, nullptr, b.io, saved, ws, inner, st));
+  TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, nullptr, b.io, saved, ws, inner, st, d->N));
   return pad_pixels(st, d, false, b.io, out);
 }
 
