@@ -291,6 +291,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
           }
         }
+        fence_proxy_async_smem();   // the bias tile and mask terms have been read: TMA writes the next ones over them
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_free[c & 3]);
@@ -1187,6 +1188,7 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
         }
       }
+      fence_proxy_async_smem();   // (TMA writes the row's statistics and mask terms over)
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_free[j & 3]);   // accumulators, statistics and mask terms of the row are consumed

@@ -821,13 +821,16 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
       const uint4* mrow = reinterpret_cast<const uint4*>(sM + (i % kBwdMaskRing) * 128 + j * 32);
       for (int hh = 0; hh < kH; ++hh, ++it) {
         const int half = half_of(hh), acc = it & 3, b = it & 1;
-        const uint8_t* gt_row = sG + b * kBTile + at;
+        const uint32_t gt_row = smem_u32(sG + b * kBTile) + at;
         ok = mbar_wait(&gfull[b], (it >> 1) & 1, g.err, 65) && ok;
-        const uint4 d[2] = {*reinterpret_cast<const uint4*>(gt_row + c0), *reinterpret_cast<const uint4*>(gt_row + c1)};
-        // The arrival must not pass the loads, which queue behind other accesses of this warp: its address takes in what
-        // they returned (and-ed with an argument that is zero), so the warp cannot issue it before they are complete.
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&gempty[b] + ((d[0].w | d[1].w) & g.zero));
+        __syncwarp();   // (the wait is a loop of each lane's own)
+        const uint4 d[2] = {lds128(gt_row + c0), lds128(gt_row + c1)};
+        // After the arrival TMA may write the buffer.  These loads are of the generic proxy and its writes of the async proxy,
+        // which an mbarrier alone does not order: each lane fences its own loads.  And nothing here consumes them before the
+        // arrival, so its address takes in what all lanes' loads returned (and-ed with an argument that is zero).
+        fence_proxy_async_smem();
+        const uint32_t got = __reduce_or_sync(0xffffffffu, d[0].w | d[1].w);
+        if (lane == 0) mbar_arrive(&gempty[b] + (got & g.zero));
         ok = mbar_wait(&tfull[acc], (it >> 2) & 1, g.err, 66) && ok;
         tc_fence_after_sync();
         const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * G::kE;

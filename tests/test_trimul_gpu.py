@@ -239,3 +239,16 @@ def test_headline_size_pixels_against_oracle(tmu):
     got = out[0][rows][:, rows]
     cos_min, fro, mar = _tol(torch.bfloat16, "ieee")
     util.check_close("out", got, want, cos_min, fro, mar)
+
+
+@pytest.mark.parametrize("n", [136, 264])
+@pytest.mark.parametrize("dtype,precision", [(torch.bfloat16, "ieee"), (torch.float32, "tf32")], ids=lambda v: str(v).replace("torch.", ""))
+def test_gate_gradients_from_reused_tiles(tmu, n, dtype, precision):
+    """Several tiles per CTA, whose gradient buffers TMA fills again while the epilogue runs: the same bits on every pass."""
+    x, mask, w, d_out = util.trimul_inputs(1, n, 128, 128, dtype, seed=n)
+    with util.matmul_precision(precision):
+        _, first = util.trimul_fwd_bwd(tmu, x, mask, w, "outgoing", d_out)
+        for _ in range(8):
+            _, again = util.trimul_fwd_bwd(tmu, x, mask, w, "outgoing", d_out)
+            for name in first:
+                assert torch.equal(again[name], first[name]), name
