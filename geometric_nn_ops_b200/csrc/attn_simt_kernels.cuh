@@ -434,6 +434,7 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_fwd_kernel(const 
         float x = mn[mb][hi];
         x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
         x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+        x = fmaxf(x, -3.402823466e38f);   // no key with a finite logit yet: P = exp(-inf), not exp(-inf + inf)
         const float alpha = exp_of<TF32>(m[mb][hi] - x);
         m[mb][hi] = x;
         float sum = 0.f;
