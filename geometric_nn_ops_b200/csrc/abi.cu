@@ -93,11 +93,20 @@ static int check_mul(const TriMulDesc* d) {
 }
 
 // What the tensor-core attention kernels need beyond the descriptor: q, k, v and dO, which they reach through tensor
-// maps, start on a 16-byte boundary.  Anything else runs on the CUDA-core kernels, which take any pointer and stride.
-static bool attn_operands_fit_tma(std::initializer_list<const void*> ptrs) {
+// maps, start on a 16-byte boundary, and so do the results, which they write (and read back) in 16-byte pieces.  Anything else
+// runs on the CUDA-core kernels, which take any pointer and stride.
+static bool aligned_to(size_t bytes, std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)
-    if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
+    if (reinterpret_cast<uintptr_t>(p) % bytes != 0) return false;
   return true;
+}
+// The multiplicative update on the tensor cores has no other path to take (its saved block is laid out for this one): what its
+// kernels read or write in pieces starts on a piece.  Norm weights are read four or eight at a time, the mask eight at a time,
+// except in the 16-bit forward's first kernel; ragged sides copy the mask.
+static int check_mul_alignment(const TriMulDesc* d, const void* mask, std::initializer_list<const void*> tensors, std::initializer_list<const void*> norms) {
+  const bool mask_ok = d->N % 8 != 0 || aligned_to(16, {mask});
+  if (aligned_to(16, tensors) && aligned_to(d->dtype == TRI_F32 ? 16 : 8, norms) && mask_ok) return 0;
+  return fail(TRI_ERR_ARG, "the tensor-core multiplicative update needs tensors that start on 16-byte boundaries");
 }
 
 }  // namespace tri
@@ -157,7 +166,7 @@ int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void*
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_bytes, tri_stream_t stream) {
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse) return fail(TRI_ERR_ARG, "q, k, v, o and lse must not be null");
-  if (tc::attn_fwd_supported(d) && attn_operands_fit_tma({q, k, v})) {
+  if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o})) {
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -171,7 +180,7 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse || !d_o || !dq || !dk || !dv || !ws)
     return fail(TRI_ERR_ARG, "q, k, v, o, lse, d_o, dq, dk, dv and ws must not be null");
-  if (tc::attn_bwd_supported(d) && attn_operands_fit_tma({q, k, v, d_o})) {
+  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias})) {
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);
@@ -249,6 +258,8 @@ int tri_mul_fwd(const TriMulDesc* d, const void* x, const void* mask, const TriM
   TRI_TRY(check_mul_weights(w));
   if (!x || !out || !ws) return fail(TRI_ERR_ARG, "x, out and ws must not be null");
   if (tc::mul_supported(d)) {
+    if (d->dtype == TRI_F32) TRI_TRY(check_mul_alignment(d, mask, {x, out, saved, ws}, {w->norm_in_w, w->norm_in_b, w->norm_out_w, w->norm_out_b}));
+    else TRI_TRY(check_mul_alignment(d, nullptr, {x, out, saved, ws}, {d->B > 1 ? w->norm_out_w : nullptr, d->B > 1 ? w->norm_out_b : nullptr}));
     set_path("tcgen05");
     return tc::mul_forward(d, x, mask, w, nullptr, out, saved, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -263,6 +274,7 @@ int tri_mul_fwd_residual(const TriMulDesc* d, const void* x, const void* mask, c
   if (!x || !residual || !out || !ws) return fail(TRI_ERR_ARG, "x, residual, out and ws must not be null");
   if (!tc::mul_residual_supported(d) || reinterpret_cast<uintptr_t>(residual) % 16 != 0)
     return fail(TRI_ERR_UNSUPPORTED, "the residual form needs a 16-bit type, one batch entry, 128 channels and N a multiple of eight");
+  TRI_TRY(check_mul_alignment(d, nullptr, {x, out, ws}, {}));
   set_path("tcgen05");
   return tc::mul_forward(d, x, mask, w, residual, out, nullptr, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -275,6 +287,7 @@ int tri_mul_bwd(const TriMulDesc* d, const void* x, const void* mask, const TriM
   if (!x || !saved || !d_out || !dx || !g || !ws)
     return fail(TRI_ERR_ARG, "x, saved, d_out, dx, grads and ws must not be null");
   if (tc::mul_supported(d)) {
+    TRI_TRY(check_mul_alignment(d, mask, {x, saved, d_out, dx, ws, w->norm_in_w}, {w->norm_out_w}));
     set_path("tcgen05");
     return tc::mul_backward(d, x, mask, w, saved, d_out, dx, g, ws, ws_bytes, (cudaStream_t)stream);
   }

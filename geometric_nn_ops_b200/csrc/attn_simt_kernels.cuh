@@ -739,6 +739,7 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dbias_kernel(
     }
   }
   float* out = a.dbias + (((long long)chunk * d.B + b) * d.H + h) * n * (long long)n;
+  const bool pairs = (n & 1) == 0 && (reinterpret_cast<uintptr_t>(a.dbias) & 7) == 0;
 #pragma unroll
   for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dbias_kernel(
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
         const int left = n - (k0 + nb * 8 + 2 * c);
-        if (left >= 2 && (n & 1) == 0) {
+        if (left >= 2 && pairs) {
           *reinterpret_cast<float2*>(row + nb * 8) = make_float2(acc[mb][nb][hi * 2], acc[mb][nb][hi * 2 + 1]);
         } else {
           if (left >= 1) row[nb * 8] = acc[mb][nb][hi * 2];

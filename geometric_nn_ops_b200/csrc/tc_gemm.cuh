@@ -467,13 +467,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       } else if constexpr (EPI == EPI_GATE_OUT_BWD) {
         const int m = tm * kBM + row;
         const TIN* dout = reinterpret_cast<const TIN*>(g.aux) + (long long)m * 128;
+        const bool wide = (reinterpret_cast<uintptr_t>(g.aux) & 31) == 0;   // (rows of 256 bytes; the caller's tensor may start between)
         if (m < g.M) {
 #pragma unroll
           for (int jj = 0; jj < CPG; ++jj)
 #pragma unroll
             for (int u = 0; u < 4; u += 2) {
-              if constexpr (sizeof(TIN) == 2) {   // rows of 256 bytes: 32-byte loads are aligned
-                ldraw16<TIN>(dout + (grp * CPG + jj) * 32 + u * 8, dst[jj][u], dst[jj][u + 1]);
+              if constexpr (sizeof(TIN) == 2) {
+                const TIN* src = dout + (grp * CPG + jj) * 32 + u * 8;
+                if (wide) {
+                  ldraw16<TIN>(src, dst[jj][u], dst[jj][u + 1]);
+                } else {
+                  dst[jj][u] = ldraw8<TIN>(src);
+                  dst[jj][u + 1] = ldraw8<TIN>(src + 8);
+                }
               } else {
                 // (each lane a quarter of four rows' 16 channels: swap_rows gives it its own row's)
                 const uint4* src = reinterpret_cast<const uint4*>(dout - (long long)(lane & 3) * 128 + (grp * CPG + jj) * 32 + u * 8) + (lane & 3);
@@ -495,7 +502,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       if constexpr (EPI == EPI_STORE) {
         const int m = tm * kBM + row, n0 = tn * BN;
         TOUT* out = reinterpret_cast<TOUT*>(g.out0) + bz * g.batch_out + (long long)m * g.ld_out;
-        const bool vec_ok = (g.ld_out * sizeof(TOUT)) % 16 == 0 && (g.batch_out * sizeof(TOUT)) % 16 == 0;
+        const bool vec_ok = (g.ld_out * sizeof(TOUT)) % 16 == 0 && (g.batch_out * sizeof(TOUT)) % 16 == 0 && (reinterpret_cast<uintptr_t>(g.out0) & 15) == 0;
         constexpr int CH = BN / 32 / NGRP;  // 32-column chunks per group
 #pragma unroll 1
         for (int jj = 0; jj < CH; ++jj) {
@@ -634,11 +641,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                   }
                 }
               }
-              // 16 channels of this pixel: one 32-byte store for 16-bit outputs (rows are 256 bytes, so it is aligned)
-              // fp32: four lanes exchange their pieces, so that a request covers 64 bytes of eight rows and not 16 of 32
+              // 16 channels of this pixel: one 32-byte store for 16-bit outputs (rows are 256 bytes; two where the caller's tensor
+              // starts between them).  fp32: four lanes exchange their pieces, so that a request covers 64 bytes of eight rows and not 16 of 32
               if constexpr (sizeof(TOUT) == 2) {
                 if (m < g.M) {
-                  store16<TOUT>(o0 + j * 32 + hf * 16, r0);
+                  TOUT* at = o0 + j * 32 + hf * 16;
+                  if (EPI == EPI_GATE_OUT_BWD || (reinterpret_cast<uintptr_t>(at) & 31) == 0) {
+                    store16<TOUT>(at, r0);
+                  } else {
+                    store8<TOUT>(at, r0);
+                    store8<TOUT>(at + 8, r0 + 8);
+                  }
                   if constexpr (EPI == EPI_GATE_OUT_BWD) store16<TOUT>(o1 + j * 32 + hf * 16, r1);
                 }
               } else {

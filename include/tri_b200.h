@@ -17,6 +17,10 @@
  *    tri_last_error() returns a thread-local message for the last failure.
  *  - Strides are in ELEMENTS.  The innermost (head-dim / channel) axis is
  *    always contiguous.
+ *  - Attention takes any alignment (tensors off a 16-byte boundary run on the
+ *    CUDA-core kernels).  The multiplicative update on the tensor cores wants
+ *    x, out, d_out, dx, the weights, saved and ws on 16-byte boundaries, and
+ *    returns TRI_ERR_ARG otherwise.
  */
 #ifndef TRI_B200_H_
 #define TRI_B200_H_

@@ -1,0 +1,82 @@
+"""Tensors that start off the boundaries the kernels' wide accesses like: views into a flat buffer, and pointers through the C ABI."""
+
+import ctypes
+
+import pytest
+import torch
+
+from tests import util
+
+pytestmark = pytest.mark.gpu
+
+
+def _at(t, elements):
+    """A copy of t that starts `elements` into its storage."""
+    flat = torch.empty(t.numel() + 64, dtype=t.dtype, device=t.device)
+    out = flat[elements:elements + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=str)
+@pytest.mark.parametrize("B,n", [(1, 40), (2, 24)])
+def test_update_gradient_on_16_but_not_32_bytes(B, n, dtype):
+    from geometric_nn_ops_b200.triangle import trimul_b200
+    x, mask, w, d_out = util.trimul_inputs(B, n, 128, 128, dtype, seed=n)
+    out, want = util.trimul_fwd_bwd(trimul_b200, x, mask, w, "outgoing", d_out)
+    out8, got = util.trimul_fwd_bwd(trimul_b200, _at(x, 8), mask, w, "outgoing", _at(d_out, 8))
+    assert _at(d_out, 8).data_ptr() % 32 == 16 and torch.equal(out8, out)
+    for name in want:
+        assert torch.equal(got[name], want[name]), name
+
+
+def _p(t):
+    return None if t is None else ctypes.c_void_p(t.data_ptr())
+
+
+def test_attention_results_off_16_bytes():
+    """Results that cannot be written in 16-byte pieces come from the CUDA-core kernels."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import _triattn
+    lib = _lib.load()
+    t, mask, d_o = util.attn_inputs(1, 4, 64, 2, 32, torch.bfloat16, seed=1)
+    q, k, v, bias = t["q"], t["k"], t["v"], t["bias"]
+    m = mask.reshape(1, 4, 64).contiguous().view(torch.uint8)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def call(off):
+        new = lambda like, n: _at(torch.zeros_like(like), n)  # noqa: E731
+        o, (dq, dk, dv) = new(q, off), (new(q, off) for _ in range(3))
+        dbias = _at(torch.zeros(1, 2, 64, 64, device="cuda"), off)
+        lse = torch.empty(2, 1, 4, 2, 64, device="cuda")
+        d = _triattn._desc(q, k, v, o, bias, m, 32 ** -0.5, "ieee")
+        d.do_st = d.dq_st = d.dk_st = d.dv_st = _triattn._st4(q)
+        ws = torch.empty(max(lib.tri_attn_ws_bytes(ctypes.byref(d), b) for b in (0, 1)), dtype=torch.uint8, device="cuda")
+        _lib.check(lib.tri_attn_fwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(bias), _p(m), _p(o), _p(lse), _p(ws), ws.numel(), stream), "fwd")
+        path = [_lib.last_path()]
+        _lib.check(lib.tri_attn_bwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(bias), _p(m), _p(o), _p(lse), _p(d_o), _p(dq), _p(dk), _p(dv),
+                                    _p(dbias), _p(ws), ws.numel(), stream), "bwd")
+        torch.cuda.synchronize()
+        return path + [_lib.last_path()], {"o": o, "dq": dq, "dk": dk, "dv": dv, "dbias": dbias}
+
+    path, want = call(0)
+    assert path == ["tcgen05", "tcgen05"]
+    path, got = call(1)
+    assert path == ["simt", "simt"]
+    cos_min, fro = util.ATTN_TOL[torch.bfloat16, "ieee"]
+    for name in want:
+        util.check_close(name, got[name], util.f64(want[name]), cos_min, fro)
+
+
+def test_update_refuses_results_off_16_bytes():
+    from geometric_nn_ops_b200 import _lib
+    lib = _lib.load()
+    x, mask, w, _ = util.trimul_inputs(1, 16, 128, 128, torch.bfloat16, seed=1)
+    d = _lib.TriMulDesc(1, 16, 128, 128, _lib.BF16, _lib.PREC_IEEE, _lib.OUTGOING, 1e-5)
+    wp = _lib.TriMulWeights(**{_lib.abi_field(n): (t.data_ptr() if t is not None else None) for n, t in ((n, w.get(n)) for n in _lib.WEIGHT_NAMES)})
+    ws = torch.empty(lib.tri_mul_ws_bytes(ctypes.byref(d), 0), dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    call = lambda out: lib.tri_mul_fwd(ctypes.byref(d), _p(x), _p(mask), ctypes.byref(wp), _p(out), None, _p(ws), ws.numel(), stream)  # noqa: E731
+    assert call(_at(torch.empty_like(x), 4)) == -1 and b"16-byte" in lib.tri_last_error()
+    assert call(_at(torch.empty_like(x), 8)) == 0
+    torch.cuda.synchronize()
