@@ -159,14 +159,15 @@ int tri_profile_summary(char* buf, size_t cap) {
 
 size_t tri_attn_ws_bytes(const TriAttnDesc* d, int is_bwd) {
   if (check_attn(d) != 0) return 0;
-  return std::max(tc::attn_ws_bytes(d, is_bwd), simt::attn_ws_bytes(d, is_bwd));
+  const size_t n = simt::attn_ws_bytes(d, is_bwd);
+  return d->dtype == TRI_F32 ? n : std::max(n, tc::attn_ws_bytes(d, is_bwd));
 }
 
 int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_bytes, tri_stream_t stream) {
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse) return fail(TRI_ERR_ARG, "q, k, v, o and lse must not be null");
-  if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o})) {
+  if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o}) && tc::attn_bias_has_room(d, bias, ws_bytes, 0)) {
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -180,7 +181,7 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse || !d_o || !dq || !dk || !dv || !ws)
     return fail(TRI_ERR_ARG, "q, k, v, o, lse, d_o, dq, dk, dv and ws must not be null");
-  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias})) {
+  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias}) && tc::attn_bias_has_room(d, bias, ws_bytes, 1)) {
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);

@@ -1285,16 +1285,18 @@ constexpr int kDbiasRowChunks = 8;   // at most this many row chunks (the worksp
 
 // Can a tensor map reach the bias as it is?  Otherwise the tensor-core kernels read a copy with padded rows: rows whose
 // length or start is not a multiple of 16 bytes (any N that is not a multiple of eight), broadcast heads or queries.
-bool bias_fits_tma(const TriAttnDesc* d, const void* bias) {
-  return (reinterpret_cast<uintptr_t>(bias) & 15) == 0 && d->bias_st[0] % 8 == 0 && d->bias_st[1] % 8 == 0 && d->bias_st[2] % 8 == 0 &&
-         (d->bias_st[1] != 0 || d->H == 1) && (d->bias_st[2] != 0 || d->n_res == 1);
+bool bias_strides_fit_tma(const TriAttnDesc* d) {
+  return d->bias_st[0] % 8 == 0 && d->bias_st[1] % 8 == 0 && d->bias_st[2] % 8 == 0 && (d->bias_st[1] != 0 || d->H == 1) &&
+         (d->bias_st[2] != 0 || d->n_res == 1);
 }
+bool bias_fits_tma(const TriAttnDesc* d, const void* bias) { return (reinterpret_cast<uintptr_t>(bias) & 15) == 0 && bias_strides_fit_tma(d); }
 int bias_pitch(const TriAttnDesc* d) { return (d->n_res + 7) / 8 * 8; }
-size_t bias_copy_bytes(const TriAttnDesc* d) { return align_up((size_t)d->B * d->H * d->n_res * bias_pitch(d) * 2); }
+int bias_batches(const TriAttnDesc* d) { return d->bias_st[0] != 0 ? d->B : 1; }
+size_t bias_copy_bytes(const TriAttnDesc* d) { return align_up((size_t)bias_batches(d) * d->H * d->n_res * bias_pitch(d) * 2); }
 
 // boxes of `rows` queries x 64 keys over the bias itself or its copy (or of keys x queries over the transposed copy)
 int bias_map(CUtensorMap* out, const void* bias, const void* copy, const TriAttnDesc* d, int rows) {
-  const uint64_t nb = d->bias_st[0] != 0 ? (uint64_t)d->B : 1, pitch = bias_pitch(d);
+  const uint64_t nb = bias_batches(d), pitch = bias_pitch(d);
   const uint64_t dims[4] = {(uint64_t)d->n_res, (uint64_t)d->n_res, (uint64_t)d->H, nb};
   const uint64_t own[3] = {(uint64_t)d->bias_st[2], (uint64_t)d->bias_st[1], (uint64_t)d->bias_st[0]};
   const uint64_t packed[3] = {pitch, pitch * d->n_res, nb > 1 ? pitch * d->n_res * d->H : 0};
@@ -1314,8 +1316,7 @@ __global__ void pad_bias_kernel(const uint16_t* __restrict__ in, int64_t st_b, i
 }
 
 int launch_pad_bias(const TriAttnDesc* d, const void* bias, void* copy, cudaStream_t st) {
-  const int nb = d->bias_st[0] != 0 ? d->B : 1;
-  const long long rows = (long long)nb * d->H * d->n_res;
+  const long long rows = (long long)bias_batches(d) * d->H * d->n_res;
   pad_bias_kernel<<<cdiv(rows, 4), dim3(64, 4), 0, st>>>(static_cast<const uint16_t*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2],
                                                           d->n_res, d->H, bias_pitch(d), rows, static_cast<uint16_t*>(copy));
   TRI_LAUNCH_OK();
@@ -1389,8 +1390,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 128, HD));
   TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 128, HD));
   if (bias) {   // the dK/dV pass (thread = key) reads a transposed copy of the bias: [b][h][key][query]
-    const int nb = d->bias_st[0] != 0 ? d->B : 1;
-    transpose_bias_kernel<<<dim3(cdiv(d->n_res, 64), cdiv(d->n_res, 64), nb * d->H), dim3(32, 8), 0, st>>>(
+    transpose_bias_kernel<<<dim3(cdiv(d->n_res, 64), cdiv(d->n_res, 64), bias_batches(d) * d->H), dim3(32, 8), 0, st>>>(
         static_cast<const uint16_t*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2], d->n_res, d->H, bias_pitch(d),
         static_cast<uint16_t*>(bias_t));
     TRI_LAUNCH_OK();
@@ -1563,15 +1563,25 @@ static size_t attn_dq_part_bytes(const TriAttnDesc* d) {
   return align_up(attn_npad(d) / 128 * (size_t)d->B * d->n_seq * d->n_res * d->H * d->D * 2);
 }
 
-size_t attn_ws_bytes(const TriAttnDesc* d, int is_bwd) {
-  if (!is_bwd)   // additive key-mask terms, copy of the bias
-    return 512 + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)) + bias_copy_bytes(d);
+// everything but the padded copy of the bias, which comes last
+static size_t attn_ws_base(const TriAttnDesc* d, int is_bwd) {
+  if (!is_bwd) return 512 + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));   // additive key-mask terms
   return 512 + align_up((size_t)d->B * d->n_seq * d->H * d->n_res * sizeof(float)) +
          align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float)) +
-         2 * bias_copy_bytes(d) +                                    // transposed copy of the bias, and a padded one
+         bias_copy_bytes(d) +                                                            // transposed copy of the bias
          align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)) +   // padded per-row constants
          align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)) +              // additive key-mask terms
          attn_dq_part_bytes(d);                                                          // merged pass: dQ per key block
+}
+
+// (The descriptor does not say where the bias starts: a copy for that reason alone is not counted here, see attn_bias_has_room.)
+size_t attn_ws_bytes(const TriAttnDesc* d, int is_bwd) {
+  return attn_ws_base(d, is_bwd) + (bias_strides_fit_tma(d) ? 0 : bias_copy_bytes(d));
+}
+
+// a bias that a copy was planned for or that needs none, or a workspace with room for one
+bool attn_bias_has_room(const TriAttnDesc* d, const void* bias, size_t ws_size, int is_bwd) {
+  return bias == nullptr || bias_fits_tma(d, bias) || !bias_strides_fit_tma(d) || ws_size >= attn_ws_base(d, is_bwd) + bias_copy_bytes(d);
 }
 
 int attn_forward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
@@ -1579,7 +1589,7 @@ int attn_forward(const TriAttnDesc* d, const void* q, const void* k, const void*
   if (ws == nullptr || ws_size < attn_ws_bytes(d, 0)) return fail(TRI_ERR_WORKSPACE, "attention forward workspace too small");
   int* err = static_cast<int*>(ws);
   float* mt = reinterpret_cast<float*>(static_cast<char*>(ws) + 512);
-  void* bc = reinterpret_cast<char*>(mt) + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));
+  void* bc = static_cast<char*>(ws) + attn_ws_base(d, 0);
   if (d->dtype == TRI_BF16) {
     if (d->D <= 32) return fwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, err, mt, bc, st);
     return fwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, err, mt, bc, st);
@@ -1597,10 +1607,10 @@ int attn_backward(const TriAttnDesc* d, const void* q, const void* k, const void
   float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + 512 +
                                          align_up((size_t)d->B * d->n_seq * d->H * d->n_res * sizeof(float)));
   void* bias_t = reinterpret_cast<char*>(part) + align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float));
-  void* bias_c = static_cast<char*>(bias_t) + bias_copy_bytes(d);
-  float* prep = reinterpret_cast<float*>(static_cast<char*>(bias_c) + bias_copy_bytes(d));
+  float* prep = reinterpret_cast<float*>(static_cast<char*>(bias_t) + bias_copy_bytes(d));
   float* mterms = reinterpret_cast<float*>(reinterpret_cast<char*>(prep) + align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)));
   void* dq_part = reinterpret_cast<char*>(mterms) + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));
+  void* bias_c = static_cast<char*>(ws) + attn_ws_base(d, 1);
   if (d->dtype == TRI_BF16) {
     if (d->D <= 32) return bwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);
     return bwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);

@@ -8,6 +8,7 @@ namespace tc {
 bool attn_fwd_supported(const TriAttnDesc* d);
 bool attn_bwd_supported(const TriAttnDesc* d);
 size_t attn_ws_bytes(const TriAttnDesc* d, int is_bwd);
+bool attn_bias_has_room(const TriAttnDesc* d, const void* bias, size_t ws_size, int is_bwd);
 int attn_forward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_size, cudaStream_t st);
 int attn_backward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,

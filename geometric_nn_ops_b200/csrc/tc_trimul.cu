@@ -1158,13 +1158,18 @@ TriMulDesc whole(const TriMulDesc* d) {
 }
 bool ragged(const TriMulDesc* d) { return d->N % 8 != 0; }
 
-struct PadBufs { void *x, *mask, *io, *dx; };   // io: out (forward), d_out (backward)
+struct PadBufs { void *mask, *x, *io, *dx; };   // io: out (forward), d_out (backward)
+// the fused forward reads and writes rows of their own pitch and copies only the mask
+bool pads_mask_only(const Geom& gm, int is_bwd) { return !is_bwd && u_channel_major(gm); }
 void carve_pad(Arena& a, const TriMulDesc* d, int is_bwd, PadBufs* b) {
   const Geom gm = geom_of(d);
-  b->x = a.take<char>((size_t)gm.M * CW * gm.es());
+  const size_t unit = (size_t)gm.M * CW * gm.es();
+  *b = PadBufs{};
   b->mask = a.take<char>((size_t)gm.M * gm.es());
-  b->io = a.take<char>((size_t)gm.M * CW * gm.es());
-  b->dx = is_bwd ? a.take<char>((size_t)gm.M * CW * gm.es()) : nullptr;
+  if (pads_mask_only(gm, is_bwd)) return;
+  b->x = a.take<char>(unit);
+  b->io = a.take<char>(unit);
+  if (is_bwd) b->dx = a.take<char>(unit);
 }
 
 // pixels [B, n, n] of `vec` 16-byte pieces each <-> [B, np, np] with zeros beyond n; PAD copies in, otherwise out
@@ -1211,7 +1216,7 @@ int pad_mask(cudaStream_t st, const TriMulDesc* d, const void* src, void* dst) {
 }
 
 template <typename T>
-int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* /*residual*/, void* out, void* saved, void* ws,
+int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, void* out, void* saved, void* ws,
                    size_t ws_size, cudaStream_t st) {
   const TriMulDesc p = whole(d);
   const size_t inner = align_up(mul_ws_bytes(&p, 0));   // first, so that the status word is the workspace's first
@@ -1221,8 +1226,8 @@ int ragged_forward(const TriMulDesc* d, const void* x, const void* mask, const T
   carve_pad(a, &p, 0, &b);
   if (!a.ok()) return fail(TRI_ERR_WORKSPACE, "trimul forward workspace too small: need %zu, got %zu", a.off, ws_size);
   TRI_TRY(pad_mask<T>(st, d, mask, b.mask));
-  // the fused kernels read and write rows of their own pitch; the others work on padded copies (11 of 74 us at 203 residues)
-  if (u_channel_major(geom_of(&p))) return forward_t<T>(&p, x, b.mask, w, nullptr, out, saved, ws, inner, st, d->N, true);
+  // the others work on padded copies (11 of 74 us at 203 residues)
+  if (pads_mask_only(geom_of(&p), 0)) return forward_t<T>(&p, x, b.mask, w, nullptr, out, saved, ws, inner, st, d->N, true);
   TRI_TRY(pad_pixels(st, d, true, x, b.x));
   TRI_TRY(forward_t<T>(&p, b.x, b.mask, w, nullptr, b.io, saved, ws, inner, st, d->N));
   return pad_pixels(st, d, false, b.io, out);
@@ -1312,9 +1317,9 @@ bool mul_residual_supported(const TriMulDesc* d) { return mul_supported(d) && !r
 int mul_forward(const TriMulDesc* d, const void* x, const void* mask, const TriMulWeights* w, const void* residual, void* out, void* saved,
                 void* ws, size_t ws_size, cudaStream_t st) {
   switch (d->dtype) {
-    case TRI_F32: return ragged(d) ? ragged_forward<float>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<float>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
-    case TRI_BF16: return ragged(d) ? ragged_forward<__nv_bfloat16>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<__nv_bfloat16>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
-    case TRI_F16: return ragged(d) ? ragged_forward<__half>(d, x, mask, w, residual, out, saved, ws, ws_size, st) : forward_t<__half>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_F32: return ragged(d) ? ragged_forward<float>(d, x, mask, w, out, saved, ws, ws_size, st) : forward_t<float>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_BF16: return ragged(d) ? ragged_forward<__nv_bfloat16>(d, x, mask, w, out, saved, ws, ws_size, st) : forward_t<__nv_bfloat16>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
+    case TRI_F16: return ragged(d) ? ragged_forward<__half>(d, x, mask, w, out, saved, ws, ws_size, st) : forward_t<__half>(d, x, mask, w, residual, out, saved, ws, ws_size, st);
   }
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
 }

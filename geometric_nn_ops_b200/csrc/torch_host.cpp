@@ -131,8 +131,16 @@ TriAttnDesc attn_desc(const Tensor& q, const Tensor& k, const Tensor& v, const T
   d.dtype = dtype_code(q); d.precision = (int)precision; d.scale = (float)scale;
   st4(d.q_st, q); st4(d.k_st, k); st4(d.v_st, v); st4(d.o_st, o);
   if (bias.defined()) { d.bias_st[0] = bias.stride(0); d.bias_st[1] = bias.stride(2); d.bias_st[2] = bias.stride(3); }
+  else d.bias_st[1] = d.bias_st[2] = 8;   // (strides that need no copy: no room for one)
   if (mask.defined()) { d.mask_st[0] = mask.stride(0); d.mask_st[1] = mask.stride(1); }
   return d;
+}
+
+// the workspace of a call; a bias that starts off a 16-byte boundary is copied into it
+size_t attn_ws_bytes(const TriAttnDesc& d, const Tensor& bias, int is_bwd) {
+  const size_t n = api.attn_ws_bytes(&d, is_bwd);
+  if (!bias.defined() || reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0) return n;
+  return n + (size_t)2 * d.B * d.H * d.n_res * (d.n_res + 7) + 256;
 }
 
 struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, S, N]
@@ -152,7 +160,7 @@ AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, cons
   c.stats = at::empty({2, B, S, H, N}, c.q.options().dtype(at::kFloat));
   const TriAttnDesc d = attn_desc(c.q, c.k, c.v, c.o, c.bias, c.mask, scale, precision);
   const c10::cuda::CUDAGuard guard(c.q.device());
-  const size_t n = api.attn_ws_bytes(&d, 0);
+  const size_t n = attn_ws_bytes(d, c.bias, 0);
   const Tensor ws = bytes(n, c.q);
   const tri_stream_t st = stream_of(c.q);
   ok(api.attn_fwd(&d, ptr(c.q), ptr(c.k), ptr(c.v), ptr(c.bias), static_cast<const uint8_t*>(ptr(c.mask)), ptr(c.o),
@@ -185,7 +193,7 @@ struct AttnFn : torch::autograd::Function<AttnFn> {
     TriAttnDesc d = attn_desc(q, k, v, o, bias, mask, ctx->saved_data["scale"].toDouble(), ctx->saved_data["precision"].toInt());
     st4(d.do_st, d_o); st4(d.dq_st, dq); st4(d.dk_st, dk); st4(d.dv_st, dv);
     const c10::cuda::CUDAGuard guard(q.device());
-    const size_t n = api.attn_ws_bytes(&d, 1);
+    const size_t n = attn_ws_bytes(d, bias, 1);
     const Tensor ws = bytes(n, q);
     const tri_stream_t st = stream_of(q);
     ok(api.attn_bwd(&d, ptr(q), ptr(k), ptr(v), ptr(bias), static_cast<const uint8_t*>(ptr(mask)), ptr(o),

@@ -102,6 +102,8 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
                  const void* d_o, void* dq, void* dk, void* dv, float* dbias /*nullable*/,
                  void* ws, size_t ws_bytes, tri_stream_t stream);
 
+/* Enough for every bias that starts on a 16-byte boundary.  One that does not is copied if the workspace has another
+ * 2 * B * H * n_res * (n_res + 7) + 256 bytes (16-bit dtypes), and read by the CUDA-core kernels otherwise. */
 size_t tri_attn_ws_bytes(const TriAttnDesc* d, int is_bwd);
 
 /* Attention backward for callers that cannot provide a workspace.  (No counterpart in the reference,

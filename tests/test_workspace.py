@@ -1,0 +1,71 @@
+"""Workspaces hold what a call needs: no copy of a bias that is read in place, one of a bias that all batch entries share."""
+
+import ctypes
+
+import pytest
+import torch
+
+from tests import util
+
+
+def _attn_bytes(B, S, N, H, D, bias_st, is_bwd=0):
+    from geometric_nn_ops_b200 import _lib
+    d = _lib.TriAttnDesc()
+    d.B, d.n_seq, d.n_res, d.H, d.D, d.dtype, d.scale = B, S, N, H, D, _lib.BF16, 1.0
+    d.bias_st = (ctypes.c_int64 * 3)(*bias_st)
+    return _lib.load().tri_attn_ws_bytes(ctypes.byref(d), is_bwd)
+
+
+@pytest.mark.parametrize("is_bwd", [0, 1])
+def test_attention_bias_copies(is_bwd):
+    in_place = _attn_bytes(4, 64, 256, 4, 32, (4 * 256 * 256, 256 * 256, 256), is_bwd)
+    shared = _attn_bytes(4, 64, 256, 4, 32, (0, 256 * 256, 256), is_bwd)
+    broadcast = _attn_bytes(4, 64, 256, 4, 32, (0, 0, 0), is_bwd)
+    plane = 4 * 256 * 256 * 2
+    assert broadcast - shared == plane                        # heads and queries without a stride: one padded copy
+    assert in_place - shared == (3 * plane if is_bwd else 0)  # the backward's transposed copies
+    if not is_bwd:
+        assert shared < 4 * 64 * 256 * 4 + 4096               # the mask terms and little else
+
+
+def test_ragged_update_forward():
+    from geometric_nn_ops_b200 import _lib
+    size = lambda n: _lib.load().tri_mul_ws_bytes(ctypes.byref(_lib.TriMulDesc(1, n, 128, 128, _lib.BF16, 0, 0, 1e-5)), 0)  # noqa: E731
+    assert size(203) - size(208) <= 208 * 208 * 2 + 1024      # a padded mask, no padded x and out
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room", [True, False])
+def test_attention_bias_off_16_bytes(room):
+    """A bias that starts off a 16-byte boundary: copied where the workspace has room, else read by the CUDA-core kernels."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import _triattn, triangle_attention
+    t, mask, d_out = util.attn_inputs(1, 4, 136, 2, 32, torch.bfloat16, seed=3)
+    want, g_want = util.attn_fwd_bwd(triangle_attention, t, mask, None, d_out)
+    flat = torch.empty(t["bias"].numel() + 1, dtype=torch.bfloat16, device="cuda")
+    bias = flat[1:].view(t["bias"].shape).copy_(t["bias"])
+    if room:
+        leaves = {n: t[n].clone().requires_grad_() for n in ("q", "k", "v")}
+        flat.requires_grad_()
+        view = flat[1:].view(t["bias"].shape)
+        out = triangle_attention(leaves["q"], leaves["k"], leaves["v"], view, mask)
+        got = torch.autograd.grad(out, [*leaves.values(), view], grad_outputs=d_out)
+        torch.cuda.synchronize()
+        assert _lib.last_path() == "tcgen05" and torch.equal(out, want)
+        for name, g in zip(("q", "k", "v", "bias"), got):
+            assert torch.equal(g, g_want[name]), name
+        return
+    lib, q = _lib.load(), t["q"]
+    m = mask.reshape(1, 4, 136).contiguous().view(torch.uint8)
+    o, lse = torch.empty_like(q), torch.empty(2, 1, 4, 2, 136, device="cuda")
+    d = _triattn._desc(q, t["k"], t["v"], o, bias, m, 32 ** -0.5, "ieee")
+    ws = torch.empty(lib.tri_attn_ws_bytes(ctypes.byref(d), 0), dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(lib.tri_attn_fwd(ctypes.byref(d), _p(q), _p(t["k"]), _p(t["v"]), _p(bias), _p(m), _p(o), _p(lse), _p(ws), ws.numel(), stream), "fwd")
+    torch.cuda.synchronize()
+    assert _lib.last_path() == "simt"
+    util.check_close("out", o, util.f64(want), *util.ATTN_TOL[torch.bfloat16, "ieee"])
