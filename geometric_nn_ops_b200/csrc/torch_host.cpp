@@ -496,9 +496,8 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
   // the same products on two dimensions
   auto linear = [](const Tensor& x, const Tensor& w, const OptTensor& b) { return b.has_value() ? at::addmm(*b, x, w.t()) : at::mm(x, w.t()); };
   const Tensor gate = linear(s.view({-1, s.size(2)}), g_w, g_b);
-  Tensor out = linear(gated(o.reshape({-1, H * D}), gate), o_w, o_b);
-  out.unsafeGetTensorImpl()->set_sizes_contiguous({BM, U, o_w.size(0)});   // (a view made here would go untracked)
-  return {out, pz};
+  const Tensor out = linear(gated(o.reshape({-1, H * D}), gate), o_w, o_b);
+  return {at::_unsafe_view(out, {BM, U, o_w.size(0)}), pz};   // (the product's own storage, and no view of a tensor that is kept)
 }
 
 }  // namespace
