@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <optional>
 #include <vector>
 
@@ -90,8 +91,18 @@ struct NoRecord {
   std::optional<at::AutoDispatchBelowADInplaceOrView> guard;
   explicit NoRecord(bool on) { if (on) guard.emplace(); }
 };
-bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
-bool wants_grad(const OptTensor& t) { return t.has_value() && t->requires_grad(); }
+// Is a derivative taken through any of these: recorded for a backward, or carried along in forward mode?
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
+bool wants_grad(std::initializer_list<const Tensor*> tensors) {
+  const bool mode = at::GradMode::is_enabled();
+  for (const Tensor* t : tensors)
+    if ((mode && t->defined() && t->requires_grad()) || has_tangent(*t)) return true;
+  return false;
+}
+void refuse_tangents(std::initializer_list<const Tensor*> tensors, const char* op) {
+  for (const Tensor* t : tensors) TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(*t), op, " has no forward-mode derivative");
+}
+Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 
 tri_stream_t stream_of(const Tensor& t) {
   return reinterpret_cast<tri_stream_t>(c10::cuda::getCurrentCUDAStream(t.get_device()).stream());
@@ -171,7 +182,6 @@ AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, cons
 
 // (an autograd Function takes an absent tensor as an empty optional; needs_input_grad counts the tensors that are there)
 OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
-Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 
 struct AttnFn : torch::autograd::Function<AttnFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& bias,
@@ -210,6 +220,7 @@ Tensor attention_residual(const Tensor& residual, const Tensor& q, const Tensor&
                           int64_t precision) {
   TORCH_CHECK(residual.is_cuda() && residual.sizes() == q.sizes() && residual.scalar_type() == q.scalar_type() &&
               residual.is_non_overlapping_and_dense() && residual.stride(-1) == 1, "residual must be dense and of q's shape and dtype");
+  refuse_tangents({&residual, &q, &k, &v, &bias}, "triangle_attention");
   const at::NoGradGuard no_grad;
   // (the sum in the kernel's epilogue was slower, 0.25 ms per 1024 x 1024 x 4 x 32 call against 0.12: its softmax warps wait for it)
   return attn_forward(q, k, v, bias, mask, 1.0 / std::sqrt((double)q.size(4)), precision, false, false, residual).o.add_(residual);
@@ -229,7 +240,8 @@ Tensor rank5(const Tensor& t) {
 // o and the statistics, recorded for the backward where a gradient is wanted
 std::pair<Tensor, Tensor> attn_any(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& bias, const Tensor& mask, double scale,
                                    int64_t precision, bool rows) {
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()))) {
+  refuse_tangents({&q, &k, &v, &bias}, "triangle_attention");
+  if (wants_grad({&q, &k, &v, &bias})) {
     const variable_list r = AttnFn::apply(q, k, v, opt(bias), opt(mask), scale, precision, rows);
     return {r[0], r[1]};
   }
@@ -244,14 +256,14 @@ py::object attention(const Tensor& q_, const Tensor& k_, const Tensor& v_, const
   const bool canonical = q_.dim() == 5;
   Tensor o, stats;
   {
-    const NoRecord fast(!at::GradMode::is_enabled() || !(wants_grad(q_) || wants_grad(k_) || wants_grad(v_) || wants_grad(bias_)));
+    Tensor bias = or_undefined(bias_), mask;
+    const NoRecord fast(!wants_grad({&q_, &k_, &v_, &bias}));
     const Tensor q = rank5(q_);
-    Tensor k = rank5(k_), v = rank5(v_), bias, mask;
+    Tensor k = rank5(k_), v = rank5(v_);
     if (k.scalar_type() != q.scalar_type()) k = k.to(q.scalar_type());
     if (v.scalar_type() != q.scalar_type()) v = v.to(q.scalar_type());
     const int64_t B = q.size(0), S = q.size(1), N = q.size(2), H = q.size(3);
-    if (bias_.has_value()) {
-      bias = *bias_;
+    if (bias.defined()) {
       if (bias.dim() == 4) bias = bias.unsqueeze(-4);
       else if (bias.dim() > 5) bias = rank5(bias);
       bias = bias.expand({B, 1, H, N, N});
@@ -412,14 +424,15 @@ Tensor multiplicative_update(const Tensor& x, const OptTensor& mask_, bool outgo
                              const std::vector<OptTensor>& weights) {
   TORCH_CHECK(weights.size() == kWeights, "expected ", kWeights, " weights");
   Weights w;
-  bool grad = x.requires_grad();
+  const Tensor mask = or_undefined(mask_);
+  refuse_tangents({&x, &mask}, "triangle_multiplicative_update");
+  bool grad = wants_grad({&x});
   for (int i = 0; i < kWeights; ++i) {
-    if (!weights[i].has_value()) continue;
-    w[i] = *weights[i];
-    grad = grad || w[i].requires_grad();
+    w[i] = or_undefined(weights[i]);
+    refuse_tangents({&w[i]}, "triangle_multiplicative_update");
+    grad = grad || wants_grad({&w[i]});
   }
-  const Tensor mask = mask_.has_value() ? *mask_ : Tensor();
-  if (at::GradMode::is_enabled() && grad)
+  if (grad)
     return MulFn::apply(x, mask_, weights[0], weights[1], weights[2], weights[3], weights[4], weights[5], weights[6], weights[7], weights[8],
                         weights[9], weights[10], weights[11], outgoing, eps, precision);
   return mul_forward(x, mask, w, outgoing, eps, precision, /*keep=*/false).out.reshape(x.sizes());
@@ -430,7 +443,11 @@ Tensor multiplicative_update_residual(const Tensor& x, const OptTensor& mask, bo
                                       const std::vector<OptTensor>& weights) {
   TORCH_CHECK(weights.size() == kWeights, "expected ", kWeights, " weights");
   Weights w;
-  for (int i = 0; i < kWeights; ++i) w[i] = or_undefined(weights[i]);
+  refuse_tangents({&x}, "triangle_multiplicative_update");
+  for (int i = 0; i < kWeights; ++i) {
+    w[i] = or_undefined(weights[i]);
+    refuse_tangents({&w[i]}, "triangle_multiplicative_update");
+  }
   const at::NoGradGuard no_grad;
   return mul_forward(x, or_undefined(mask), w, outgoing, eps, precision, /*keep=*/false, /*residual=*/true).out.reshape(x.sizes());
 }
@@ -444,8 +461,8 @@ bool pair_bias_fits(const Tensor& z, const OptTensor& ln_w, const Tensor& w) {
   const bool fits = z.is_cuda() && z.dim() == 4 && (dt == at::kBFloat16 || dt == at::kHalf) && z.size(3) == 128 && w.dim() == 2 &&
                     w.size(1) == 128 && w.size(0) >= 1 && w.size(0) <= 16 && w.scalar_type() == dt && w.device() == z.device() &&
                     (!ln_w.has_value() || (ln_w->scalar_type() == dt && ln_w->dim() == 1 && ln_w->size(0) == 128 && ln_w->device() == z.device()));
-  const bool grad = at::GradMode::is_enabled() && (z.requires_grad() || w.requires_grad() || (ln_w.has_value() && ln_w->requires_grad()));
-  return fits && !grad && z.numel() >= 128 && z.numel() / 128 < (1LL << 31) - 128 && !at::autocast::is_autocast_enabled(at::kCUDA);
+  const Tensor lw = or_undefined(ln_w);
+  return fits && !wants_grad({&z, &w, &lw}) && z.numel() >= 128 && z.numel() / 128 < (1LL << 31) - 128 && !at::autocast::is_autocast_enabled(at::kCUDA);
 }
 Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
   if (!pair_bias_fits(z, ln_w, w))
@@ -463,8 +480,7 @@ Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double
 
 // o * sigmoid(gate)
 Tensor gated(const Tensor& o, const Tensor& gate) {
-  const bool grad = at::GradMode::is_enabled() && (o.requires_grad() || gate.requires_grad());
-  if (grad || !o.is_contiguous() || !gate.is_contiguous() || o.scalar_type() != gate.scalar_type() || o.sizes() != gate.sizes())
+  if (wants_grad({&o, &gate}) || !o.is_contiguous() || !gate.is_contiguous() || o.scalar_type() != gate.scalar_type() || o.sizes() != gate.sizes())
     return o * at::sigmoid(gate);
   const c10::cuda::CUDAGuard guard(o.device());
   const Tensor out = at::empty(o.sizes(), o.options());
@@ -479,10 +495,8 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
                                               const OptTensor& z_w, const OptTensor& ln_w, const OptTensor& mask_, double scale, double eps,
                                               int64_t precision) {
   const int64_t BM = q.size(0), H = q.size(1), U = q.size(2), D = q.size(3), B = z.size(0), M = BM / B;
-  bool grad = false;
-  if (at::GradMode::is_enabled())
-    for (const Tensor* t : {&s, &q, &k, &v, &z, &g_w, &o_w}) grad = grad || t->requires_grad();
-  grad = grad || (at::GradMode::is_enabled() && (wants_grad(g_b) || wants_grad(o_b) || wants_grad(z_w) || wants_grad(ln_w)));
+  const Tensor gb = or_undefined(g_b), ob = or_undefined(o_b), zw = or_undefined(z_w), lw = or_undefined(ln_w);
+  const bool grad = wants_grad({&s, &q, &k, &v, &z, &g_w, &o_w, &gb, &ob, &zw, &lw});
   const NoRecord fast(!grad);
   const Tensor pz = z_w.has_value() ? pair_bias(z, ln_w, *z_w, eps) : z;
   // (BM, H, U, D) -> rows = multiplicity: [B, M, U, H, D] as a strided view (no copy)
