@@ -1533,10 +1533,12 @@ int qkv_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, const in
   return make_tmap(out, p, d->dtype, 5, dims, str, box, width * 2);
 }
 
-// Logits from which on odd lengths (and head dims other than 32 and 64) come here.  These kernels are the faster ones down
-// to the smallest sizes measured (forward and backward of 16 rows of 100 residues, 4 heads of 32: 43 us against 331; 8 rows
-// of 8, 2 heads of 8: 31 against 61); below the lines the gain is tens of microseconds, and the exact-fp32 kernels keep
-// what the tests hold them to there.  N = 301, forward and backward: 10.0 ms on the CUDA cores, 0.45 here.
+// Logits from which on odd lengths (and head dims other than 32 and 64) come here.  Below, calls stay on the CUDA-core kernels,
+// which keep P and dS in fp32 (bf16, 203 residues: outputs within 1.7e-3 of fp64, 2.3e-3 here; gradients 1.8e-3 and 3.0e-3).
+// The lines lie just above the largest shapes that the tests hold to those kernels (16 rows of 100 residues, 4 heads: 640,000
+// logits; 8 rows of 8, 2 heads of 8), not where the times cross.  Forward alone, us on the CUDA cores / here: 53 x 53 residues,
+// 4 heads 14 / 18; 16 x 100 16 / 16; 1 x 201, 16 heads 31 / 16.  All kernels of forward and backward: 137 / 67, 132 / 61,
+// 156 / 65; 8 x 8, 2 heads of 8 93 / 55.  At 301 x 301 it is 10 ms against 0.45.
 constexpr double kMinRagged = 655360.0, kMinPaddedDim = 4096.0;
 
 bool attn_fwd_supported(const TriAttnDesc* d) {

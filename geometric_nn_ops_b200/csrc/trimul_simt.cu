@@ -274,12 +274,14 @@ static int contract_start(cudaStream_t st, bool tf32, int B, const ContractP& p)
   return 0;
 }
 
-// The largest tile that still makes a CTA for every SM.
+// The largest tile that still makes a CTA for every SM; of the two smaller ones the larger from 100 CTAs on.  128 channels, fp32,
+// us with 16 x 8, 8 x 8 and 4 x 4 pixels a warp: N = 96 (72 CTAs of 8 x 8) 39, 25, 19; N = 104 (112) 42, 26, 29; N = 128 (128) 48,
+// 29, 37; N = 192 (144 CTAs of 16 x 8) 69, 64, 93; N = 256 (256) 164, 150, 206.
 static int contract(cudaStream_t st, bool tf32, int B, ContractP p) {
   p.vec = p.ldx % 4 == 0 && p.ldy % 4 == 0 && p.xoff % 4 == 0 && p.yoff % 4 == 0 && p.Ch % 4 == 0;
   const long long planes = (long long)B * cdiv(p.Ch, 32);
   if (planes * cdiv(p.N, 32) * cdiv(p.N, 32) >= 148) return contract_start<16, 8>(st, tf32, B, p);
-  if (planes * cdiv(p.N, 32) * cdiv(p.N, 16) >= 120) return contract_start<8, 8>(st, tf32, B, p);
+  if (planes * cdiv(p.N, 32) * cdiv(p.N, 16) >= 100) return contract_start<8, 8>(st, tf32, B, p);
   return contract_start<4, 4>(st, tf32, B, p);
 }
 
