@@ -160,6 +160,10 @@ struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, 
 // (`rows`: o contiguous in that order of axes, else laid out like q; or like `model`)
 AttnCall attn_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& bias_, const Tensor& mask_, double scale,
                       int64_t precision, bool rows, bool record = false, const Tensor& model = Tensor()) {
+  TORCH_CHECK_VALUE(q_.dim() == 5 && k_.sizes() == q_.sizes() && v_.sizes() == q_.sizes(),
+                    "q, k and v must have one shape, got ", q_.sizes(), ", ", k_.sizes(), " and ", v_.sizes());
+  TORCH_CHECK_VALUE(k_.device() == q_.device() && v_.device() == q_.device() && (!bias_.defined() || bias_.device() == q_.device()) &&
+                    (!mask_.defined() || mask_.device() == q_.device()), "q, k, v, bias and mask must be on one device");
   const NoRecord fast(!record);   // (views that are saved for a backward share their base's version counter)
   AttnCall c;
   c.q = inner_contiguous(q_); c.k = inner_contiguous(k_); c.v = inner_contiguous(v_);
@@ -315,6 +319,9 @@ MulCall mul_forward(const Tensor& x, const Tensor& mask, const Weights& weights,
   MulCall c{};
   c.d.dtype = dtype_code(x);
   for (int i : {2, 4, 8, 10}) TORCH_CHECK_VALUE(weights[i].defined(), kNames[i], " is required");
+  for (int i = 0; i < kWeights; ++i)
+    TORCH_CHECK_VALUE(!weights[i].defined() || weights[i].device() == x.device(), kNames[i], " is on ", weights[i].device(), ", x on ", x.device());
+  TORCH_CHECK_VALUE(!mask.defined() || mask.device() == x.device(), "mask is on ", mask.device(), ", x on ", x.device());
   TORCH_CHECK_VALUE(x.dim() >= 3 && x.size(-2) == x.size(-3), "x must be [*, N, N, C], got ", x.sizes());
   const int64_t N = x.size(-2), C = x.size(-1);
   c.x = aligned(x.dim() == 4 ? x : x.reshape({-1, N, N, C}));

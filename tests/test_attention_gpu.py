@@ -322,3 +322,14 @@ def test_rows_and_residues_swapped_in_memory_bit_exact(ta):
     for a, b in zip(g1[:3], g0[:3]):
         assert torch.equal(a.transpose(1, 2), b)
     assert torch.equal(g1[3], g0[3])
+
+
+@pytest.mark.parametrize("name", ["k", "v"])
+@pytest.mark.parametrize("cut", [lambda t: t[:, :, :24], lambda t: t[:1], lambda t: t[..., :8], lambda t: t.cpu()],
+                         ids=["residues", "batch", "head dim", "device"])
+def test_operands_that_do_not_match_are_refused(ta, name, cut):
+    """The kernels address k and v by q's sizes: a smaller tensor would be read beyond its end."""
+    t, mask, _ = util.attn_inputs(2, 3, 40, 2, 16, torch.bfloat16, seed=3)
+    t[name] = cut(t[name])
+    with pytest.raises(ValueError, match="one shape|one device"):
+        ta(t["q"], t["k"], t["v"], t["bias"], mask)

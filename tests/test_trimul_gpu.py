@@ -252,3 +252,14 @@ def test_gate_gradients_from_reused_tiles(tmu, n, dtype, precision):
             _, again = util.trimul_fwd_bwd(tmu, x, mask, w, "outgoing", d_out)
             for name in first:
                 assert torch.equal(again[name], first[name]), name
+
+
+@pytest.mark.parametrize("name", ["mask", "p_in_weight", "norm_out_bias"])
+def test_operands_on_another_device_are_refused(tmu, name):
+    x, mask, w, _ = util.trimul_inputs(1, 16, 128, 128, torch.bfloat16, seed=1)
+    if name == "mask":
+        mask = mask.cpu()
+    else:
+        w[name] = w[name].cpu()
+    with pytest.raises(ValueError, match=name):
+        tmu(x, "outgoing", mask, **w)
