@@ -674,7 +674,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
 // shared memory; with 16-bit types a z tile feeds the products of both halves, so z is read once.  The fp32 weights of one
 // half fill the same space, so there a CTA has one half and its neighbour the other, on the same tiles (z comes from L2
 // the second time).  The gradient tile of a half ([128 channels x 128 bytes]) comes by TMA; the epilogue copies it to
-// registers at once, so that its buffer takes the next tile's during the arithmetic.  dP and dG leave through a staging
+// registers first, so that its buffer takes the next tile's during the arithmetic.  dP and dG leave through a staging
 // tile each and a TMA store: whole 128-byte lines.  Written by the threads, a request carried 32 bytes (a channel's rows
 // lie a plane apart), 4096 of them per 128 pixels, and the load / store pipe held the kernel at 0.29 ms for 768 x 768
 // pixels; with the gradients read that way too (the batched GEMM's form) it took 0.365.  Now 0.22, floor by bytes 0.16.
@@ -691,7 +691,6 @@ struct BwdArgs {
   int tiles;
   const float* bias;
   const void* mask;
-  uint32_t zero;        // 0
   int* err;
 };
 
@@ -823,14 +822,7 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
         const int half = half_of(hh), acc = it & 3, b = it & 1;
         const uint32_t gt_row = smem_u32(sG + b * kBTile) + at;
         ok = mbar_wait(&gfull[b], (it >> 1) & 1, g.err, 65) && ok;
-        __syncwarp();   // (the wait is a loop of each lane's own)
         const uint4 d[2] = {lds128(gt_row + c0), lds128(gt_row + c1)};
-        // After the arrival TMA may write the buffer.  These loads are of the generic proxy and its writes of the async proxy,
-        // which an mbarrier alone does not order: each lane fences its own loads.  And nothing here consumes them before the
-        // arrival, so its address takes in what all lanes' loads returned (and-ed with an argument that is zero).
-        fence_proxy_async_smem();
-        const uint32_t got = __reduce_or_sync(0xffffffffu, d[0].w | d[1].w);
-        if (lane == 0) mbar_arrive(&gempty[b] + (got & g.zero));
         ok = mbar_wait(&tfull[acc], (it >> 2) & 1, g.err, 66) && ok;
         tc_fence_after_sync();
         const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * G::kE;
@@ -848,9 +840,13 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
 #pragma unroll
           for (int e = 0; e < 8; ++e) { p[e] = __uint_as_float(rp[e]); gt[e] = __uint_as_float(rg[e]); }
         }
+        // After these arrivals the next products go to the accumulator and TMA writes the gradient buffer.  The buffer's loads are
+        // of the generic proxy and TMA's writes of the async proxy, which an mbarrier alone does not order: each lane fences its
+        // own loads, here, where they have long returned (right behind them the fence cost 11 of 226 us at 768 x 768 pixels).
+        fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[acc]);
+        if (lane == 0) { mbar_arrive(&tempty[acc]); mbar_arrive(&gempty[b]); }
         // two pieces of 16 bytes: kE pixels as float2 pairs, dP and dG in place of the gradient
         constexpr int kPair = G::kE / 4;   // per piece
         uint4 o0[2], o1[2];
@@ -916,7 +912,7 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   TRI_TRY(make_tmap_3d(&tmB, p.db_cm, E, f16, gd, gs, box, false));
   TRI_TRY(make_tmap_3d(&tmO, p.dpg, E, f16, od, gs, box, false));
   BwdArgs a;
-  a.M = p.M; a.tiles = (int)(p.M / G::kPx); a.bias = p.bias_cat; a.mask = p.mask; a.zero = 0; a.err = p.err;
+  a.M = p.M; a.tiles = (int)(p.M / G::kPx); a.bias = p.bias_cat; a.mask = p.mask; a.err = p.err;
   constexpr size_t smem = 1024 + kWBytes + 6 * kBTile + kBwdMaskRing * 128 + 17 * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = gate_in_bwd_kernel<T>;
