@@ -4,8 +4,8 @@
 
 One step = triangle_attention fwd+bwd (B=1, N=768, H=4, D=32, bf16, pair bias + key mask) plus
 triangle_multiplicative_update fwd+bwd in both directions (N=768, C=C_hidden=128, bf16), i.e. the
-configuration the metric in BASELINE.json is quoted on.  Inputs are seeded synthetic tensors with the
-shapes and distributions BASELINE.json lists.  Prints ONE JSON line (rank 0).
+configuration the metric is quoted on.  Inputs are seeded synthetic tensors of those shapes.  Prints ONE JSON line
+(rank 0).
 
 value      TFLOP/s over the timed steps with inputs resident in HBM (CUDA events, max over ranks).
 e2e        the same metric through the public API with HOST (pinned) buffers: every step copies the
@@ -109,7 +109,7 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------------------------------------------
-# synthetic inputs (host, fp32 draw -> bf16), BASELINE.json distributions
+# synthetic inputs (host, fp32 draw -> bf16)
 # ------------------------------------------------------------------------------------------------
 def host_inputs(n, seed, torch, rows=None):
     """Inputs for one rank.  ``rows`` = (i0, i1) restricts the row axis (multi-GPU sharding)."""

@@ -1,6 +1,6 @@
 """``bench.py --workload stack``: the 4-block pair stack, bf16 inference, on 1..8 GPUs (rows sharded).
 
-BASELINE configuration: B=1, N=1024, c_z=128, four blocks with weights from seeds 0..3, z ~ N(0, 1), the last 64
+Configuration: B=1, N=1024, c_z=128, four blocks with weights from seeds 0..3, z ~ N(0, 1), the last 64
 residues masked out.  Before timing, the same code runs a reduced size (N=128 per 8 ranks or fewer) and is
 checked against the CPU oracle composition (oracle/pairstack_oracle.py); a mismatch ends the run non-zero.
 Prints one JSON line with the whole-stack time, TFLOP/s over the algorithmic forward FLOPs, and the split of

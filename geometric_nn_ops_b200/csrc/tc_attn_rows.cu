@@ -24,8 +24,8 @@
 // waiting warps' polling took half of all issue slots.
 //
 // What bounds it: the exponentials (16 per clock and SM: 8 clocks of a sub-partition per 32), then the waits a row's four
-// warps, which run on four sub-partitions, have for one another.  N = 768, 4 heads, bf16: 0.73 ms, 58 % of the exponential
-// pipe, against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
+// warps, which run on four sub-partitions, have for one another.  N = 768, 4 heads, bf16: 0.72 ms, 59 % of the exponential
+// pipe (which also converts), against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
 // also read 2 bytes of bias per logit from L2; here 0.67).
 #include <algorithm>
 #include <type_traits>

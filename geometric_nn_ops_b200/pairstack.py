@@ -45,7 +45,7 @@ class BlockWeights:
 
 
 def make_block_weights(seed, c=128, dtype=torch.bfloat16, device="cpu"):
-    """Random weights of one block drawn on the CPU from ``seed`` (BASELINE distributions: LayerNorm weights
+    """Random weights of one block drawn on the CPU from ``seed`` (LayerNorm weights
     1 + N(0, 0.02), LayerNorm biases N(0, 0.02), projections N(0, 1/sqrt(fan_in)), no projection biases)."""
     g = torch.Generator().manual_seed(seed)
     rn = lambda *s, sc=1.0: torch.randn(*s, generator=g) * sc  # noqa: E731
