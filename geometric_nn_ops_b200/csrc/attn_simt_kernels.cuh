@@ -262,12 +262,15 @@ __device__ __forceinline__ void cols_product(float (&acc)[MB][DB / 32][4][4], co
   }
 }
 
-// s = bias of this warp's rows (queries) and NB * 8 keys from k0, zero where there is none.  A tile inside the plane whose
-// rows start on pairs is read without a test per element (rows beyond the last query repeat it: nothing of them is kept).
-template <typename T, int MB, int NB>
+// s = bias (ADD: s += bias) of this warp's rows (queries) and NB * 8 keys from k0, zero where there is none.  A tile inside the
+// plane whose rows start on pairs is read without a test per element (rows beyond the last query repeat it: nothing of them is
+// kept).  TF32 products start from the bias.  Exact ones start from zero and take it afterwards, in one rounding, as the
+// reference does: a sum that starts from it rounds every term beside it (errors four to eight times larger from a bias of 10 on).
+template <typename T, int MB, int NB, bool ADD>
 __device__ __forceinline__ void bias_tile(float (&s)[MB][NB][4], const T* bias, long long row_st, int q0, int k0, int n, bool pairs) {
   const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
   const bool fast = bias != nullptr && pairs && k0 + NB * 8 <= n;
+  auto put = [](float& x, float v) { x = ADD ? x + v : v; };
 #pragma unroll
   for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
@@ -278,27 +281,27 @@ __device__ __forceinline__ void bias_tile(float (&s)[MB][NB][4], const T* bias, 
         for (int nb = 0; nb < NB; ++nb) {
           if constexpr (sizeof(T) == 4) {
             const float2 v = __ldg(reinterpret_cast<const float2*>(row + nb * 8));
-            s[mb][nb][hi * 2] = v.x;
-            s[mb][nb][hi * 2 + 1] = v.y;
+            put(s[mb][nb][hi * 2], v.x);
+            put(s[mb][nb][hi * 2 + 1], v.y);
           } else {
             union { uint32_t u; T h[2]; } v;
             v.u = __ldg(reinterpret_cast<const uint32_t*>(row + nb * 8));
-            s[mb][nb][hi * 2] = to_f32(v.h[0]);
-            s[mb][nb][hi * 2 + 1] = to_f32(v.h[1]);
+            put(s[mb][nb][hi * 2], to_f32(v.h[0]));
+            put(s[mb][nb][hi * 2 + 1], to_f32(v.h[1]));
           }
         }
       } else {
         const int left = bias != nullptr ? n - k0 - 2 * c : 0;
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-          s[mb][nb][hi * 2] = nb * 8 < left ? to_f32(row[nb * 8]) : 0.f;
-          s[mb][nb][hi * 2 + 1] = nb * 8 + 1 < left ? to_f32(row[nb * 8 + 1]) : 0.f;
+          put(s[mb][nb][hi * 2], nb * 8 < left ? to_f32(row[nb * 8]) : 0.f);
+          put(s[mb][nb][hi * 2 + 1], nb * 8 + 1 < left ? to_f32(row[nb * 8 + 1]) : 0.f);
         }
       }
     }
 }
 // ... with the keys as this warp's rows and NB * 8 queries from q0
-template <typename T, int MB, int NB>
+template <typename T, int MB, int NB, bool ADD>
 __device__ __forceinline__ void bias_tile_t(float (&s)[MB][NB][4], const T* bias, long long row_st, int key0, int q0, int n) {
   const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
   const T* col = bias + (bias != nullptr ? (q0 + 2 * c) * row_st + key0 + r : 0);
@@ -311,7 +314,9 @@ __device__ __forceinline__ void bias_tile_t(float (&s)[MB][NB][4], const T* bias
 #pragma unroll
       for (int i = 0; i < 2 * MB; ++i) {
         const bool live = fast || (bias != nullptr && key0 + r + i * 8 < n && q0 + nb * 8 + 2 * c + e < n);
-        s[i >> 1][nb][(i & 1) * 2 + e] = live ? to_f32(__ldg(at + i * 8)) : 0.f;
+        const float v = live ? to_f32(__ldg(at + i * 8)) : 0.f;
+        float& x = s[i >> 1][nb][(i & 1) * 2 + e];
+        x = ADD ? x + v : v;
       }
     }
 }
@@ -410,9 +415,10 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_fwd_kernel(const 
     settle<T, DB, NT, TF32, false>(tV, 1.f);
     __syncthreads();
     if (k0 + NT < n) issue(k0 + NT, b ^ 1);
-    float s[MB][NB][4];
-    bias_tile<T, MB, NB>(s, bias, d.bias_st[2], z.m0 + warp * 16 * MB, k0, n, a.pair_bias != 0);
+    float s[MB][NB][4] = {};
+    if constexpr (TF32) bias_tile<T, MB, NB, false>(s, bias, d.bias_st[2], z.m0 + warp * 16 * MB, k0, n, a.pair_bias != 0);
     rows_product<DB, MB, NB, TF32>(s, sQ, tK);
+    if constexpr (!TF32) bias_tile<T, MB, NB, true>(s, bias, d.bias_st[2], z.m0 + warp * 16 * MB, k0, n, a.pair_bias != 0);
     float mn[MB][2];
 #pragma unroll
     for (int mb = 0; mb < MB; ++mb) mn[mb][0] = m[mb][0], mn[mb][1] = m[mb][1];
@@ -556,18 +562,23 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dkdv_kernel(c
     __syncthreads();
     if (q0 + NT < n) issue(q0 + NT, b ^ 1);
     const float* st = sS + b * 3 * NT + 2 * c;
-    float s[MB][NB][4], dp[MB][NB][4];
-    bias_tile_t<T, MB, NB>(s, bias, d.bias_st[2], key0, q0, n);
+    float s[MB][NB][4] = {}, dp[MB][NB][4] = {};
+    if constexpr (TF32) bias_tile_t<T, MB, NB, false>(s, bias, d.bias_st[2], key0, q0, n);
     rows_product<DB, MB, NB, TF32>(s, sK, tQ);
+    if constexpr (!TF32) bias_tile_t<T, MB, NB, true>(s, bias, d.bias_st[2], key0, q0, n);
+    auto minus_delta = [&] {
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-      const float2 dl = *reinterpret_cast<const float2*>(st + 2 * NT + nb * 8);
+      for (int nb = 0; nb < NB; ++nb) {
+        const float2 dl = *reinterpret_cast<const float2*>(st + 2 * NT + nb * 8);
 #pragma unroll
-      for (int mb = 0; mb < MB; ++mb)
+        for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dp[mb][nb][i] = i & 1 ? -dl.y : -dl.x;
-    }
+          for (int i = 0; i < 4; ++i) dp[mb][nb][i] -= i & 1 ? dl.y : dl.x;
+      }
+    };
+    if constexpr (TF32) minus_delta();
     rows_product<DB, MB, NB, TF32>(dp, sV, tG);
+    if constexpr (!TF32) minus_delta();
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
       const float2 mx = *reinterpret_cast<const float2*>(st + nb * 8), ll = *reinterpret_cast<const float2*>(st + NT + nb * 8);
@@ -644,16 +655,21 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dq_kernel(con
     settle<T, DB, NT, TF32, false>(tV, 1.f);
     __syncthreads();
     if (k0 + NT < n) issue(k0 + NT, b ^ 1);
-    float s[MB][NB][4], dp[MB][NB][4];
-    bias_tile<T, MB, NB>(s, bias, d.bias_st[2], q0, k0, n, a.pair_bias != 0);
+    float s[MB][NB][4] = {}, dp[MB][NB][4] = {};
+    if constexpr (TF32) bias_tile<T, MB, NB, false>(s, bias, d.bias_st[2], q0, k0, n, a.pair_bias != 0);
     rows_product<DB, MB, NB, TF32>(s, sQ, tK);
+    if constexpr (!TF32) bias_tile<T, MB, NB, true>(s, bias, d.bias_st[2], q0, k0, n, a.pair_bias != 0);
+    auto minus_delta = [&] {
 #pragma unroll
-    for (int mb = 0; mb < MB; ++mb)
+      for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
+        for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dp[mb][nb][i] = -dl[mb][i >> 1];
+          for (int i = 0; i < 4; ++i) dp[mb][nb][i] -= dl[mb][i >> 1];
+    };
+    if constexpr (TF32) minus_delta();
     rows_product<DB, MB, NB, TF32>(dp, sG, tV);
+    if constexpr (!TF32) minus_delta();
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
       const float2 t = *reinterpret_cast<const float2*>(sM + b * NT + nb * 8 + 2 * c);
@@ -707,7 +723,7 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dbias_kernel(
       sM[buf * NT + threadIdx.x] = mask_term(a.mask == nullptr ? nullptr : a.mask + b * d.mask_st[0] + s * d.mask_st[1], k0 + threadIdx.x, n);
   };
   float acc[MB][NB][4] = {}, bt[MB][NB][4], mx[MB][2], ll[MB][2], dl[MB][2];
-  bias_tile<T, MB, NB>(bt, bias, d.bias_st[2], q0, k0, n, a.pair_bias != 0);
+  bias_tile<T, MB, NB, false>(bt, bias, d.bias_st[2], q0, k0, n, a.pair_bias != 0);
   if (s_begin < s_end) issue(s_begin, 0);
   for (int s = s_begin, buf = 0; s < s_end; ++s, buf ^= 1) {
     const uint32_t tQ = base + buf * kStage, tG = tQ + MT * DB * 4, tK = tG + MT * DB * 4, tV = tK + NT * DB * 4;
@@ -725,9 +741,17 @@ __global__ void __launch_bounds__(kCta, DB == 32 ? 3 : 1) attn_bwd_dbias_kernel(
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { p[mb][nb][i] = bt[mb][nb][i]; dp[mb][nb][i] = -dl[mb][i >> 1]; }
+        for (int i = 0; i < 4; ++i) { p[mb][nb][i] = TF32 ? bt[mb][nb][i] : 0.f; dp[mb][nb][i] = TF32 ? -dl[mb][i >> 1] : 0.f; }
     rows_product<DB, MB, NB, TF32>(p, tQ, tK);
     rows_product<DB, MB, NB, TF32>(dp, tG, tV);
+    if constexpr (!TF32) {
+#pragma unroll
+      for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { p[mb][nb][i] += bt[mb][nb][i]; dp[mb][nb][i] -= dl[mb][i >> 1]; }
+    }
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
       const float2 t = *reinterpret_cast<const float2*>(sM + buf * NT + nb * 8 + 2 * c);

@@ -33,3 +33,19 @@ def test_against_oracle(shape, precision):
     util.check_close("out", out, o_ref, cos_min, fro, worst)
     for name, val in grads.items():
         util.check_close("grad_" + name, val, g_ref[name], cos_min, fro, worst)
+
+
+@pytest.mark.parametrize("shape", [(1, 6, 128, 4, 32), (1, 5, 101, 2, 64), (1, 4, 70, 2, 128)], ids=str)
+def test_bias_is_added_in_one_rounding(shape):
+    """A bias near 100 under every logit: exact fp32 products must not start from it.  fp32 numbers there lie 2^-17 apart, so that
+    bias and mask in one rounding each leave a logit, and with it P, right to 2^-18 = 4e-6 each way; a sum that rounds
+    after every term beside the bias was off by 1e-5 and more."""
+    from geometric_nn_ops_b200.triangle import triangle_attention
+    t, mask, d_out = util.attn_inputs(*shape, torch.float32, seed=2, keep=0.95)
+    t["bias"] = t["bias"] * 0.5 + 100
+    with util.matmul_precision("ieee"):
+        out, grads = util.attn_fwd_bwd(triangle_attention, t, mask, None, d_out)
+    o_ref, g_ref = util.attn_oracle(t, mask, None, d_out)
+    util.check_close("out", out, o_ref, 1 - 1e-9, 4e-6)
+    for name, val in grads.items():
+        util.check_close("grad_" + name, val, g_ref[name], 1 - 1e-9, 4e-6)
