@@ -16,8 +16,8 @@
 // whatever the number of rows) was the shared-memory pipe, and for dbias an idle chip.  What bounds these is instruction
 // issue: about half of the slots at 12 warps per SM (168 registers per thread; the 32-wide tiles are compiled for three CTAs),
 // of which the matrix instructions are a small part; in the exact kernels the FMAs are.  At 256 x 256 x 4 heads x 32 with
-// TF32 (exact): forward 0.66 -> 0.13 ms (0.65 -> 0.33), dK and dV 1.11 -> 0.22 (0.55), dQ 0.85 -> 0.17 (0.39), dbias
-// 5.6 -> 0.22 (0.37), delta 0.072 -> 0.025.
+// TF32 (exact): forward 0.66 -> 0.13 ms (0.65 -> 0.34), dK and dV 1.11 -> 0.22 (0.55), dQ 0.85 -> 0.17 (0.40), dbias
+// 5.6 -> 0.23 (0.40), delta 0.072 -> 0.025.
 #pragma once
 
 #include "attn_simt.cuh"
