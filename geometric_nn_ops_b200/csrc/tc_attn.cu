@@ -64,7 +64,11 @@ template <int HD> struct Geo {
 __global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b, int64_t st_s, int B, int S, int N, int npad,
                                   float* __restrict__ out, int* err) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx == 0) *err = 0;
+  if (idx == 0) {
+    *err = 0;
+    __threadfence();   // before the kernels that follow may start
+  }
+  dependent_trigger();
   if (idx >= (long long)B * S * npad) return;
   const int k = idx % npad;
   const long long bs = idx / npad;
@@ -145,6 +149,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   constexpr uint32_t COL_O = 128;   // O_0 at [128, 128 + HD), O_1 at [128 + HD, 128 + 2 HD)
   // With head dim 32 the 256 TMEM columns have room for P itself (two 16-bit values per column) and P V reads it
@@ -529,6 +534,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   constexpr uint32_t COL_DP = 64, COL_DV = 128, COL_DK = 128 + HD;
   // With head dim 32 the 256 TMEM columns have room for P^T and dS^T themselves (two 16-bit values per column), and
@@ -859,6 +865,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   constexpr uint32_t COL_DP = 64, COL_DQ = 128, COL_DS = 128 + HD;   // dS: 64 keys as 32 packed columns
   bool ok = true;
@@ -1095,6 +1102,7 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   bool ok = true;
 
@@ -1251,6 +1259,7 @@ __global__ void attn_delta_tc_kernel(TriAttnDesc d, const T* o, const T* d_o, co
 // block order in fp32; 8 elements per thread.
 template <typename T>
 __global__ void attn_dq_sum_kernel(const T* __restrict__ part, int nparts, long long plane, TriAttnDesc d, T* __restrict__ dq) {
+  dependent_trigger();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= plane / 8) return;
   const int dc = d.D / 8;
@@ -1307,6 +1316,7 @@ int bias_map(CUtensorMap* out, const void* bias, const void* copy, const TriAttn
 // one row of the bias per block row: 16-bit elements to rows of `pitch`
 __global__ void pad_bias_kernel(const uint16_t* __restrict__ in, int64_t st_b, int64_t st_h, int64_t st_q, int n, int H, int pitch,
                                 long long rows, uint16_t* __restrict__ out) {
+  dependent_trigger();
   const long long row = blockIdx.x * (long long)blockDim.y + threadIdx.y;   // (batch, head, query)
   const int q = row % n;
   const long long bh = row / n;
@@ -1327,6 +1337,7 @@ int launch_pad_bias(const TriAttnDesc* d, const void* bias, void* copy, cudaStre
 __global__ void transpose_bias_kernel(const uint16_t* __restrict__ in, int64_t st_b, int64_t st_h, int64_t st_q, int n, int H,
                                       int pitch, uint16_t* __restrict__ out) {
   __shared__ uint16_t tile[64][66];
+  dependent_trigger();
   const int bh = blockIdx.z, b = bh / H, h = bh % H;
   const uint16_t* src = in + b * st_b + h * st_h;
   uint16_t* dst = out + (int64_t)bh * n * pitch;
@@ -1413,7 +1424,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     TRI_TRY(set_dyn_smem(kern, GeoC<HD>::SMEM));   // per-device attribute: set on every launch
     KernelTimer kt(kMerge ? "tc_attn_bwd_dkdvdq" : "tc_attn_bwd_dkdv", st, (kMerge ? 10.0 : 8.0) * pairs * d->D,
                    (kMerge ? 7.0 : 6.0) * tensor_bytes);
-    kern<<<(unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoC<HD>::SMEM, st>>>(tq, tdo, tk, tv, tb, a);
+    launch_dependent(kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoC<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
   }
   if (kMerge) {
@@ -1440,7 +1451,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     auto kern = bias ? attn_bwd_dq_kernel<T, HD, true> : attn_bwd_dq_kernel<T, HD, false>;
     TRI_TRY(set_dyn_smem(kern, GeoQ<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dq", st, 2.0 * pairs * d->D, 5.0 * tensor_bytes);
-    kern<<<(unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoQ<HD>::SMEM, st>>>(tq, tdo, tk, tv, tb, a);
+    launch_dependent(kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoQ<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
   }
   // ---- dbias ---------------------------------------------------------------------------------
@@ -1459,7 +1470,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     auto kern = attn_bwd_dbias_kernel<T, HD>;   // (K / V maps with 64-key boxes and the bias map are those of the dQ pass)
     TRI_TRY(set_dyn_smem(kern, GeoB<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor_bytes);
-    kern<<<(unsigned)((long long)qblocks * kblocks * d->B * d->H * chunks), 320, GeoB<HD>::SMEM, st>>>(tq, tdo, tk, tv, tb, a);
+    launch_dependent(kern, (unsigned)((long long)qblocks * kblocks * d->B * d->H * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     if (chunks > 1) {   // fixed-order sum of the row-chunk partials
       sum_partials_kernel<<<cdiv(nb, 256), 256, 0, st>>>(dbias_partial, chunks, nb, dbias);
@@ -1519,7 +1530,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto kern = bias != nullptr ? attn_fwd_tc_kernel<T, HD, true> : attn_fwd_tc_kernel<T, HD, false>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<HD>::SMEM));
-  kern<<<(unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st>>>(tq, tk, tv, tb, a);
+  launch_dependent(kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
   TRI_LAUNCH_OK();
   return 0;
 }

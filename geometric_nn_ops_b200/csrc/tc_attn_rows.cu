@@ -127,12 +127,14 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_trigger();   // (q, k, v are the caller's: only the mask terms and a copied bias come from the kernels before)
   constexpr uint32_t COLS = 160, COL_O = 128;   // a group's columns: S / P of even and odd steps at 0 and 64, O
   bool ok = true;
 
   if (warp == 5 * kGroups) {
     // ------------------------------------ bias tiles and mask terms --------------------------------
     if (lane == 0) {
+      dependent_wait();
       int stg = 0;
       uint32_t ph = 0;
       for (int n = 0; n < my_items && ok; ++n) {
@@ -466,7 +468,7 @@ int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto launch = [&](auto kern, const CUtensorMap& tb) {
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem::SMEM));
-    kern<<<(unsigned)std::min<long long>(items, sm_count()), kThreads, RowsSmem::SMEM, st>>>(tq, tk, tv, tb, a);
+    launch_dependent(kern, (unsigned)std::min<long long>(items, sm_count()), kThreads, RowsSmem::SMEM, st, tq, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     return 0;
   };

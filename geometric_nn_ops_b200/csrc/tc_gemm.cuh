@@ -343,6 +343,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
 
   const int total = g.batches * g.tiles_m * g.tiles_n;
   const int kb_total = g.kblocks0 + g.kblocks1;

@@ -101,6 +101,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -336,7 +337,7 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(a.tiles, sm_count());
   KernelTimer kt("tc_ln_gate_in", st, 2.0 * p.M * 128 * 512, 4.0 * p.M * 128 * 2);
-  kern<<<grid, kThreads, smem, st>>>(tmX, tmW, tmZ, tmA, tmB, a);
+  launch_dependent(kern, grid, kThreads, smem, st, tmX, tmW, tmZ, tmA, tmB, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -416,15 +417,19 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // the weights are the caller's and come while the contraction drains
+  if (warp == 0 && elect_one()) {
+    mbar_expect_tx(wfull, kOWBytes);
+    for (int kb = 0; kb < 2; ++kb) {
+      tma_load_3d(sW + kb * kSub, &tmWo, wfull, kb * 64, 0, 0);
+      tma_load_3d(sW + (2 + kb) * kSub, &tmWg, wfull, kb * 64, 0, 0);
+    }
+  }
+  dependent_enter();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(wfull, kOWBytes);
-      for (int kb = 0; kb < 2; ++kb) {
-        tma_load_3d(sW + kb * kSub, &tmWo, wfull, kb * 64, 0, 0);
-        tma_load_3d(sW + (2 + kb) * kSub, &tmWg, wfull, kb * 64, 0, 0);
-      }
       int i = 0;
       for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
         const int b = i % kOBufs;
@@ -661,7 +666,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(a.tiles, sm_count());
   KernelTimer kt("tc_ln_gate_out", st, 2.0 * p.M * 128 * 256, (p.u_cm ? 4.0 : 3.0) * p.M * 128 * 2);
-  kern<<<grid, kThreads, smem, st>>>(tmT, tmZ, tmWo, tmWg, a);
+  launch_dependent(kern, grid, kThreads, smem, st, tmT, tmZ, tmWo, tmWg, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -743,6 +748,7 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependent_enter();
 
   // items: the halves this CTA has, of tiles tile0, tile0 + step, ...; half_of(hh): the hh-th of them
   const int tile0 = kH == 2 ? blockIdx.x : blockIdx.x >> 1, step = kH == 2 ? gridDim.x : gridDim.x >> 1;
@@ -919,7 +925,7 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = G::kHalves == 2 ? std::min(a.tiles, sm_count()) : 2 * std::min(a.tiles, sm_count() / 2);
   KernelTimer kt("tc_gate_in_bwd", st, 0.0, 7.0 * p.M * 128 * E);
-  kern<<<grid, kBwdThreads, smem, st>>>(tmZ, tmW, tmA, tmB, tmO, a);
+  launch_dependent(kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
   TRI_LAUNCH_OK();
   return 0;
 }

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(256) ln_bias_kernel(const T* __restrict__ z, c
                                                        long long M, const T* __restrict__ wb, int H, T* __restrict__ zn,
                                                        T* __restrict__ bias) {
   __shared__ float sWb[H4 ? 1 : kMaxHeads][CW];
+  dependent_trigger();
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   float wr[4][8];
   if constexpr (H4) {

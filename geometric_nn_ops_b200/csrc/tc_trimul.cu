@@ -70,7 +70,11 @@ template <typename T>
 __global__ void prep_weights_kernel(const T* wp, const T* wg, const T* bp, const T* bg, const T* bo, const T* bgo,
                                     T* wcat, float* bias_cat, float* bias_out, int* err) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx == 0) *err = 0;   // the error word of the launches that follow
+  if (idx == 0) {
+    *err = 0;   // the error word of the launches that follow
+    __threadfence();
+  }
+  dependent_trigger();
   if (idx < 4 * CW * CW) {
     const int r = idx / CW, k = idx % CW, blk = r / CW, c = r % CW;
     const T* src = (blk & 1) ? wg : wp;
@@ -126,6 +130,7 @@ constexpr int kLnRowPairs = 4;   // row pairs per warp and pass (8 rows)
 template <typename T>
 __global__ void __launch_bounds__(256) ln_rows_kernel(const T* __restrict__ x, const T* gamma, const T* beta, float eps,
                                                        long long M, T* __restrict__ z, float* mean, float* rstd, int n, int pitch) {
+  dependent_trigger();
   const int lane = threadIdx.x & 31, sub = lane & 15, half = lane >> 4;
   const long long row0 = (blockIdx.x * 8LL + (threadIdx.x >> 5)) * (2 * kLnRowPairs) + half;
   float gm[8], bt[8];
@@ -323,6 +328,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4) ln_cm_kernel(const T* t_cm, const T* gamma, const T* beta, float eps,
                                                         long long M, long long NN, T* u, float* mean, float* rstd, int n, int pitch) {
   __shared__ float tile[TP * TROW];
+  dependent_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float gm[4] = {1.f, 1.f, 1.f, 1.f}, bt[4] = {0.f, 0.f, 0.f, 0.f};
   if (gamma) load4(gamma + lane * 4, gm);
@@ -575,6 +581,7 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_multi_kernel(const Redu
   const int o = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int j = ((blockIdx.x - jobs.first[job]) * 32 + o) * 4;   // n is a multiple of 128
   const float* partial = jobs.partial[job] + j;
+  dependent_trigger();
   float4 a[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
