@@ -207,7 +207,13 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       }
       if (m < g.M) {
         g.mean[m] = mu; g.rstd[m] = rs;
-        if (mask != nullptr) s_mask[(i % kMaskRing) * 128 + r] = mask[m];
+        T* keep = s_mask + (i % kMaskRing) * 128 + r;
+        if (g.own_pitch) {   // the mask in its own pitch too, zero at the pixels beyond n
+          const int py = (int)((uint32_t)m / (uint32_t)g.pitch), px = (int)m - py * g.pitch;
+          *keep = py < g.n && px < g.n ? (mask != nullptr ? mask[py * g.n + px] : from_f32<T>(1.f)) : from_f32<T>(0.f);
+        } else if (mask != nullptr) {
+          *keep = mask[m];
+        }
       }
       fence_proxy_async_smem();   // the tile is read next by tcgen05.mma and by the TMA store
       __syncwarp();
@@ -229,7 +235,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
     const int quarter = warp & 3, j = (warp - 6) >> 2;   // TMEM lane quarter; 32-pixel chunk of the tile
     const int row = quarter * 32 + lane;
-    const bool masked = g.mask != nullptr, staged = g.staged != 0;
+    const bool masked = g.mask != nullptr || g.own_pitch, staged = g.staged != 0;
     const uint32_t plane = (uint32_t)g.plane, M = (uint32_t)g.M;
     // staging: the 64-pixel chunk of warps j, j ^ 1 and its issuing thread
     uint8_t* orow = sO + (j >> 1) * kSub + row * 128;

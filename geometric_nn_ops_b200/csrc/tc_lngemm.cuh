@@ -34,7 +34,7 @@ struct LnGateIn {
   float eps;
   const void* x;             // [M, 128]
   int n = 0, pitch = 0;      // n > 0: planes of [pitch, pitch] pixels hold [n, n]; x is zero beyond
-  bool own_pitch = false;    // x is [n, n, 128] (one batch entry) and not [M, 128]
+  bool own_pitch = false;    // x is [n, n, 128] and the mask [n, n] (one batch entry), not [M, 128] and [M]
   const void* gamma;         // [128] or null
   const void* beta;          // [128] or null
   const void* wcat;          // [512, 128]: rows [Wp_a; Wg_a; Wp_b; Wg_b]
