@@ -20,6 +20,7 @@
 // bias and the finite -1e9 key-mask sentinel are added in fp32; keys beyond N_res get -inf.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "tc_attn_common.cuh"
 #include "tc_attn_rows.cuh"
@@ -60,16 +61,19 @@ template <int HD> struct Geo {
 };
 
 // additive key-mask terms of every (batch, row): 0 for a kept key, -1e9 for a masked key, -inf beyond N; rows of
-// npad.  Also clears the error word of the launches that follow.
+// npad.  With n_flags > 0 (the backward) a second plane holds them times log2(e), and the flags of the rows are cleared.
+// Also clears the error word of the launches that follow.
 __global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b, int64_t st_s, int B, int S, int N, int npad,
-                                  float* __restrict__ out, int* err) {
+                                  float* __restrict__ out, int* err, int* __restrict__ flags, long long n_flags) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx == 0) {
     *err = 0;
     __threadfence();   // before the kernels that follow may start
   }
   dependent_trigger();
-  if (idx >= (long long)B * S * npad) return;
+  const long long n = (long long)B * S * npad;
+  for (long long i = idx; i < n_flags; i += (long long)gridDim.x * blockDim.x) flags[i] = 0;
+  if (idx >= n) return;
   const int k = idx % npad;
   const long long bs = idx / npad;
   const int s = bs % S, b = bs / S;
@@ -77,6 +81,7 @@ __global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b
   if (k >= N) v = -INFINITY;
   else if (mask != nullptr) v = kMaskSentinel * ((mask[b * st_b + s * st_s + k] ? 1.0f : 0.0f) - 1.0f);
   out[idx] = v;
+  if (n_flags > 0) out[n + idx] = v * kLog2e;
 }
 
 // 320 threads.  Warps 0-7 do the softmax arithmetic: thread (r, hh) owns query row r and the 64-key half hh of each
@@ -433,7 +438,10 @@ struct AttnBwdArgs {
   const float* prep;     // [3][B][S][H][npad]: -m, -log l * log2e, -delta, zero in the padding
   long long prep_plane;  // B*S*H*npad
   int npad;              // N rounded up to 128
-  const float* mask_terms;   // [B][S][npad] additive key-mask terms (0, -1e9, or -inf beyond N)
+  const float* mask_terms;   // [2][B][S][npad] additive key-mask terms (0, -1e9, or -inf beyond N); the same times log2(e)
+  long long mask_plane;      // B*S*npad
+  const uint4* aug;          // [B][S][H][npad] row constants as eight 16-bit factors (see RowFactors)
+  const int* large;          // [B][S][H] whether a query of the row goes without them
   const uint8_t* mask;
   int64_t mask_st[2];
   int bias_b_mul;        // 0 when the bias is broadcast over the batch
@@ -448,6 +456,56 @@ struct AttnBwdArgs {
   int* err;
 };
 
+// Row constants through the products.  With c = -(m + log l) / scale and -delta of a query as further channels of Q and dO,
+// against ones for every key, S and dP arrive as (x - m - log l) / scale without bias and mask, and as dP - delta: a logit
+// then takes two packed instructions up to the exponential, and no statistics are read beside it.  (As fp32 vectors in shared
+// memory they were six of the seven loads of eight logits in the dK/dV pass, and it followed the load pipe: 66 % at N = 768.)
+// A factor pair carries 24 bits: three 16-bit terms whose products with the key side's constants add up to the value.
+//   query: {c1, c2, c3, d1, d2, d3, 0, 0}     key, for S: {1, 1, 1, 0 ...}     for dP: {0, 0, 0, k1, k2, k3, 0, 0}
+// bf16 has fp32's range: k = 1.  fp16 takes delta in steps of 2^-48 up to 31: k = 2^-11, 2^-22, 2^-24.
+// A product of 16 channels reads two 16-byte columns per row; the second one of the key side is zero, and the second one of
+// the query side is the next eight rows' first (128 bytes of zeros follow the last).
+// Rows (batch, row, head) in which a query has |m| > 256, or a value out of range, are flagged, and their CTAs (dbias: steps)
+// take differences in natural units instead, as the forward does where logits are large.
+struct RowFactors {
+  static constexpr int kBlock = 384;            // one 8-row block of equal rows, read with a row-group stride of 16 bytes
+  static constexpr int kBytes = 3 * kBlock;     // for S | for dP | zeros
+  static constexpr uint32_t HI_KEY = desc_hi(16, 0), HI_QUERY = desc_hi(128, 0);   // no swizzle
+  __device__ static uint32_t key_s(uint32_t at) { return desc_lo(at, 2 * kBlock); }
+  __device__ static uint32_t key_dp(uint32_t at) { return desc_lo(at + kBlock, kBlock); }
+  __device__ static uint32_t query(uint32_t at) { return desc_lo(at, 128); }
+  template <typename T> __device__ static void fill(uint8_t* key, int tid) {   // kBytes / 16 threads
+    if (tid >= kBytes / 16) return;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (tid < kBlock / 16) { v.x = pack2<T>(1.f, 1.f); v.y = pack2<T>(1.f, 0.f); }
+    else if (tid < 2 * kBlock / 16) {
+      constexpr bool bf = ElemIsBf16<T>::value;
+      v.y = pack2<T>(0.f, bf ? 1.f : 0x1p-11f);
+      v.z = pack2<T>(bf ? 1.f : 0x1p-22f, bf ? 1.f : 0x1p-24f);
+    }
+    reinterpret_cast<uint4*>(key)[tid] = v;
+  }
+  // the terms of v for factors 1 / s1, 1 / s2, 1 / s3 (powers of two)
+  template <typename T> __device__ static void split(float v, float s1, float s2, float s3, float (&t)[3]) {
+    t[0] = to_f32(from_f32<T>(v * s1));
+    v -= t[0] / s1;
+    t[1] = to_f32(from_f32<T>(v * s2));
+    v -= t[1] / s2;
+    t[2] = to_f32(from_f32<T>(v * s3));
+  }
+  template <typename T> __device__ static bool fits(float m, float c, float d) {
+    constexpr bool bf = ElemIsBf16<T>::value;
+    return fabsf(m) <= 256.f && fabsf(c) <= (bf ? 1e30f : 6e4f) && fabsf(d) <= (bf ? 1e30f : 31.f);
+  }
+  template <typename T> __device__ static uint4 pack(float c, float d) {
+    constexpr bool bf = ElemIsBf16<T>::value;
+    float a[3], b[3];
+    split<T>(c, 1.f, 1.f, 1.f, a);
+    split<T>(d, bf ? 1.f : 0x1p11f, bf ? 1.f : 0x1p22f, bf ? 1.f : 0x1p24f, b);
+    return make_uint4(pack2<T>(a[0], a[1]), pack2<T>(a[2], b[0]), pack2<T>(b[1], b[2]), 0u);
+  }
+};
+
 template <int HD> struct GeoC {
   static constexpr int RB = HD * 2;
   static constexpr int TK = 128 * RB;   // K / V tile
@@ -455,7 +513,8 @@ template <int HD> struct GeoC {
   static constexpr uint32_t LAYOUT = RB == 128 ? 2 : 4;
   static constexpr uint32_t SBO = 8 * RB;
   static constexpr int NQ = 3;                      // query-tile stages: tiles are fetched two steps ahead
-  static constexpr int ST = 3 * 64 * 4;             // one stage of row statistics: -m, -log l log2e, -delta for 64 queries
+  static constexpr int ST = 64 * 16 + 128;          // one stage of row constants: factors of 64 queries and zeros behind them, or
+                                                    // (flagged rows) -m, -log l log2e, -delta
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = OFF_K + TK;
   static constexpr int OFF_Q = OFF_V + TK;          // [NQ]
@@ -463,8 +522,9 @@ template <int HD> struct GeoC {
   static constexpr int OFF_PT = OFF_DO + NQ * TQ;   // [2] x [128 keys x 64 queries] SW128: the transposed bias tile arrives
                                                     // here and each thread overwrites its part with P^T
   static constexpr int OFF_DST = OFF_PT + 2 * 16384;    // [2] x dS^T, same shape
-  static constexpr int OFF_ST = OFF_DST + 2 * 16384;    // [NQ] statistics stages
-  static constexpr int OFF_BAR = OFF_ST + NQ * ST;
+  static constexpr int OFF_ST = OFF_DST + 2 * 16384;    // [NQ] row constants
+  static constexpr int OFF_KEY = OFF_ST + NQ * ST;
+  static constexpr int OFF_BAR = OFF_KEY + RowFactors::kBytes;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
 };
 
@@ -499,7 +559,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint8_t* sDO = smem + G::OFF_DO;
   uint8_t* sPT = smem + G::OFF_PT;
   uint8_t* sDST = smem + G::OFF_DST;
-  float* sStats = reinterpret_cast<float*>(smem + G::OFF_ST);   // [NQ][3][64]
+  uint8_t* sRow = smem + G::OFF_ST;   // [NQ] row constants
   uint64_t* bar_kv = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);
   uint64_t* bar_in = bar_kv + 1;     // [NQ]
   uint64_t* bar_bias = bar_kv + 4;   // [2]
@@ -529,12 +589,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(bar_free, 8); mbar_init(bar_p, 8);
     mbar_fence_init();
   }
+  RowFactors::fill<T>(smem + G::OFF_KEY, tid);
+  if (tid >= 288 && tid < 288 + G::NQ * 8) reinterpret_cast<uint4*>(sRow + (tid - 288) / 8 * G::ST + 1024)[(tid - 288) % 8] = make_uint4(0, 0, 0, 0);
+  fence_proxy_async_smem();
   if (warp == 0) tmem_alloc(tmem_slot, 256);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   dependent_enter();
+  const bool folded = a.large[((long long)b * a.S + s) * a.H + h] == 0;   // the row's constants come with the products
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   constexpr uint32_t COL_DP = 64, COL_DV = 128, COL_DK = 128 + HD;
   // With head dim 32 the 256 TMEM columns have room for P^T and dS^T themselves (two 16-bit values per column), and
@@ -549,16 +613,21 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 9) {
     if (lane == 0) {
       // ---------------------------------- TMA copies ---------------------------------------------
-      const float* prep_row = a.prep + ((((long long)b * a.S + s) * a.H + h) * (long long)a.npad);
+      const long long row0 = (((long long)b * a.S + s) * a.H + h) * (long long)a.npad;
+      const float* prep_row = a.prep + row0;
       auto load_step = [&](int step) {
         const int stg = step % G::NQ;
-        float* st = sStats + stg * 192;
-        mbar_expect_tx(&bar_in[stg], 2 * G::TQ + G::ST);
+        float* st = reinterpret_cast<float*>(sRow + stg * G::ST);
+        mbar_expect_tx(&bar_in[stg], 2 * G::TQ + (folded ? 1024 : 768));
         tma_load_5d(sQ + stg * G::TQ, &tmQ, &bar_in[stg], 0, h, step * 64, s, b);
         tma_load_5d(sDO + stg * G::TQ, &tmDO, &bar_in[stg], 0, h, step * 64, s, b);
-        bulk_load(st, prep_row + step * 64, 256, &bar_in[stg]);
-        bulk_load(st + 64, prep_row + a.prep_plane + step * 64, 256, &bar_in[stg]);
-        bulk_load(st + 128, prep_row + 2 * a.prep_plane + step * 64, 256, &bar_in[stg]);
+        if (folded) {
+          bulk_load(st, a.aug + row0 + step * 64, 1024, &bar_in[stg]);
+        } else {
+          bulk_load(st, prep_row + step * 64, 256, &bar_in[stg]);
+          bulk_load(st + 64, prep_row + a.prep_plane + step * 64, 256, &bar_in[stg]);
+          bulk_load(st + 128, prep_row + 2 * a.prep_plane + step * 64, 256, &bar_in[stg]);
+        }
       };
       auto load_bias = [&](int step) {
         uint64_t* bb = &bar_bias[step & 1];
@@ -591,6 +660,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t pt_lo = desc_lo(smem_u32(sPT), 16), dst_lo = desc_lo(smem_u32(sDST), 16);
       const uint32_t dsmn_lo = desc_lo(smem_u32(sDST), 16384);      // dS of a tile pair as [m = query, k = key]: MN-major A
       const uint32_t kmn_lo = desc_lo(smem_u32(sK), 128 * G::RB);   // K as [n = d, k = key]: MN-major B
+      const uint32_t key_s = RowFactors::key_s(smem_u32(smem + G::OFF_KEY)), key_dp = RowFactors::key_dp(smem_u32(smem + G::OFF_KEY));
+      const uint32_t row_lo = RowFactors::query(smem_u32(sRow));
       // S^T = K Q^T and dP^T = V dO^T of one 64-query tile
       auto issue_scores = [&](int step) {
         const int stg = step % G::NQ;
@@ -603,6 +674,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
           umma<KIND_F16>(tmem_base + COL_DP, desc_join(v_lo + ks * 2, HI_KMAJ), desc_join(do_lo + so + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
+        if (folded) {
+          const uint64_t rows = desc_join(row_lo + stg * (G::ST >> 4), RowFactors::HI_QUERY);
+          umma<KIND_F16>(tmem_base, desc_join(key_s, RowFactors::HI_KEY), rows, a.idesc_a, 1);
+          umma<KIND_F16>(tmem_base + COL_DP, desc_join(key_dp, RowFactors::HI_KEY), rows, a.idesc_a, 1);
+        }
         umma_commit(bar_s);
       };
       ok = mbar_wait(bar_kv, 0, a.err, 31);
@@ -645,7 +721,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     float mb = 0.f;
     if (kj >= a.N) mb = -INFINITY;
     else if (a.mask != nullptr) mb = kMaskSentinel * ((a.mask[b * a.mask_st[0] + s * a.mask_st[1] + kj] ? 1.0f : 0.0f) - 1.0f);
-    const float2 sc2 = splat(a.scale), mk2 = splat(mb), l2e2 = splat(kLog2e);
+    const float2 sc2 = splat(a.scale), mk2 = splat(mb), l2e2 = splat(kLog2e), scl2 = splat(a.scale * kLog2e), mkl2 = splat(mb * kLog2e);
     // MERGE: fetch the dQ accumulator of query-tile pair `pair` (row r = query 128 pair + r, this thread's half of the
     // head dim) and store it, unscaled, as this key block's partial.  tcgen05.ld is warp-wide: every thread loads.
     auto store_dq_pair = [&](int pair) {
@@ -672,23 +748,36 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int stg = j & 1, qstg = j % G::NQ;
       ok = mbar_wait(bar_s, j & 1, a.err, 33) && ok;
       tc_fence_after_sync();
-      ok = mbar_wait(&bar_in[qstg], (j / G::NQ) & 1, a.err, 32) && ok;   // the tile's row statistics
+      if (!folded) ok = mbar_wait(&bar_in[qstg], (j / G::NQ) & 1, a.err, 32) && ok;   // the tile's row statistics
       if (HB) ok = mbar_wait(&bar_bias[stg], (j >> 1) & 1, a.err, 34) && ok;
 
-      // packed fp32x2 arithmetic: P = 2^((x - m) log2e - log l log2e), dS = P (dP - delta); thread = key, columns = queries
+      // packed fp32x2 arithmetic: P = 2^((x - m) log2e - log l log2e), dS = P (dP - delta); thread = key, columns = queries.
+      // Folded: the accumulators hold (scale q k - m - log l) / scale and dP - delta.
       const uint32_t sPTj = smem_u32(sPT) + stg * 16384;     // holds the transposed bias tile now, P^T when this step is done
       const uint32_t sDSTj = smem_u32(sDST) + stg * 16384;   // (its last readers, tile j-2's products, finished before S^T(j) did)
-      const uint32_t st_a = smem_u32(sStats) + qstg * 768;   // -m, -log l log2e, -delta of 64 queries, 256 bytes each
+      const uint32_t st_a = smem_u32(sRow) + qstg * G::ST;   // -m, -log l log2e, -delta of 64 queries, 256 bytes each
       const int c = hh;
       uint32_t pw[16], dw[16];
       // 16 of this thread's 32 queries
-      auto half = [&](const uint32_t (&rs)[16], const uint32_t (&rp)[16], int h2) {
+      auto half = [&](auto fold, const uint32_t (&rs)[16], const uint32_t (&rp)[16], int h2) {
 #pragma unroll
         for (int uu = 0; uu < 2; ++uu) {
           const int u = h2 * 2 + uu;
           uint4 raw = make_uint4(0, 0, 0, 0);
           if constexpr (HB) raw = lds128(sPTj + sw128_chunk1(r, c * 4 + u));
           const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
+          if constexpr (fold.value) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 t = HB ? __ffma2_rn(unpack2<T>(bw[i]), l2e2, mkl2) : mkl2;
+              const float2 e = __ffma2_rn(pair(rs[uu * 8 + 2 * i], rs[uu * 8 + 2 * i + 1]), scl2, t);
+              const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+              const float2 ds = __fmul2_rn(pp, pair(rp[uu * 8 + 2 * i], rp[uu * 8 + 2 * i + 1]));
+              pw[u * 4 + i] = pack2<T>(pp.x, pp.y);
+              dw[u * 4 + i] = pack2<T>(ds.x, ds.y);
+            }
+            continue;
+          }
           const uint32_t at = st_a + (c * 8 + u * 2) * 16;
           const float4 m0 = lds128f(at), m1 = lds128f(at + 16);
           const float4 l0 = lds128f(at + 256), l1 = lds128f(at + 272);
@@ -706,10 +795,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             pw[u * 4 + i] = pack2<T>(pp.x, pp.y);
             dw[u * 4 + i] = pack2<T>(ds.x, ds.y);
           }
-          if constexpr (!TMEM_A) {
-            sts128(sPTj + sw128_chunk1(r, c * 4 + u), pw[u * 4], pw[u * 4 + 1], pw[u * 4 + 2], pw[u * 4 + 3]);
-            sts128(sDSTj + sw128_chunk1(r, c * 4 + u), dw[u * 4], dw[u * 4 + 1], dw[u * 4 + 2], dw[u * 4 + 3]);
-          }
         }
       };
       // the second half's TMEM loads are in flight while the first half is computed
@@ -719,12 +804,21 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tmem_ld_wait();
       tmem_ld_32x16(t_row + hh * 32 + 16, rsB);
       tmem_ld_32x16(t_row + COL_DP + hh * 32 + 16, rpB);
-      half(rsA, rpA, 0);
+      if (folded) half(std::true_type{}, rsA, rpA, 0);
+      else half(std::false_type{}, rsA, rpA, 0);
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_free);   // this warp holds its logits: the accumulators can take the next tile
-      half(rsB, rpB, 1);
+      if (folded) half(std::true_type{}, rsB, rpB, 1);
+      else half(std::false_type{}, rsB, rpB, 1);
+      if constexpr (!TMEM_A) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          sts128(sPTj + sw128_chunk1(r, c * 4 + u), pw[u * 4], pw[u * 4 + 1], pw[u * 4 + 2], pw[u * 4 + 3]);
+          sts128(sDSTj + sw128_chunk1(r, c * 4 + u), dw[u * 4], dw[u * 4 + 1], dw[u * 4 + 2], dw[u * 4 + 3]);
+        }
+      }
       if constexpr (TMEM_A) {
         if (j > 0) ok = mbar_wait(&bar_acc[(j - 1) & 3], ((j - 1) >> 2) & 1, a.err, 35) && ok;   // the previous tile's products have read theirs
         tc_fence_after_sync();
@@ -1049,11 +1143,13 @@ template <int HD> struct GeoB {
   static constexpr uint32_t LAYOUT = RB == 128 ? 2 : 4;
   static constexpr uint32_t SBO = 8 * RB;
   static constexpr int NS = 3;                           // row stages
-  static constexpr int STAT = 2048;                      // -m, -log l log2e, -delta of 128 queries; 64 mask terms; padding
-                                                         // (stages stay 1024-byte aligned for the swizzled tiles)
+  static constexpr int OFF_MASK = 2048 + 128;            // factors of 128 queries and zeros behind them, or (flagged rows)
+                                                         // -m, -log l log2e, -delta; then 64 mask terms
+  static constexpr int STAT = 3072;                      // (stages stay 1024-byte aligned for the swizzled tiles)
   static constexpr int STAGE = 2 * TA + 2 * TB + STAT;
   static constexpr int OFF_BIAS = NS * STAGE;            // [128 queries x 64 keys] SW128, loaded once
-  static constexpr int OFF_BAR = OFF_BIAS + 16384;
+  static constexpr int OFF_KEY = OFF_BIAS + 16384;
+  static constexpr int OFF_BAR = OFF_KEY + RowFactors::kBytes;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
 };
 
@@ -1097,6 +1193,9 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int i = 0; i < 4; ++i) mbar_init(&bar_free[i], 8);
     mbar_fence_init();
   }
+  RowFactors::fill<T>(smem + G::OFF_KEY, tid);
+  if (tid >= 288 && tid < 288 + G::NS * 8) reinterpret_cast<uint4*>(stage_stat((tid - 288) / 8) + 512)[(tid - 288) % 8] = make_uint4(0, 0, 0, 0);
+  fence_proxy_async_smem();
   if (warp == 0) tmem_alloc(tmem_slot, 256);
   tc_fence_before_sync();
   __syncthreads();
@@ -1105,23 +1204,30 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   dependent_enter();
   const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
   bool ok = true;
+  const int* large = a.large + ((long long)b * a.S + s_lo) * a.H + h;   // flags of the rows, H apart
 
   if (warp == 9) {
     if (lane == 0) {
       // ---------------------------------- TMA copies ---------------------------------------------
       auto load_step = [&](int step) {
         const int stg = step % G::NS, s = s_lo + step;
-        const float* prow = a.prep + ((((long long)b * a.S + s) * a.H + h) * (long long)a.npad) + q0;
+        const long long row0 = (((long long)b * a.S + s) * a.H + h) * (long long)a.npad + q0;
+        const float* prow = a.prep + row0;
+        const bool folded = large[(long long)step * a.H] == 0;
         float* st = stage_stat(stg);
-        mbar_expect_tx(&bar_in[stg], 2 * G::TA + 2 * G::TB + 3 * 512 + 256);
+        mbar_expect_tx(&bar_in[stg], 2 * G::TA + 2 * G::TB + (folded ? 2048 : 3 * 512) + 256);
         tma_load_5d(stage_q(stg), &tmQ, &bar_in[stg], 0, h, q0, s, b);
         tma_load_5d(stage_do(stg), &tmDO, &bar_in[stg], 0, h, q0, s, b);
         tma_load_5d(stage_k(stg), &tmK, &bar_in[stg], 0, h, k0, s, b);
         tma_load_5d(stage_v(stg), &tmV, &bar_in[stg], 0, h, k0, s, b);
-        bulk_load(st, prow, 512, &bar_in[stg]);
-        bulk_load(st + 128, prow + a.prep_plane, 512, &bar_in[stg]);
-        bulk_load(st + 256, prow + 2 * a.prep_plane, 512, &bar_in[stg]);
-        bulk_load(st + 384, a.mask_terms + ((long long)b * a.S + s) * a.npad + k0, 256, &bar_in[stg]);
+        if (folded) {
+          bulk_load(st, a.aug + row0, 2048, &bar_in[stg]);
+        } else {
+          bulk_load(st, prow, 512, &bar_in[stg]);
+          bulk_load(st + 128, prow + a.prep_plane, 512, &bar_in[stg]);
+          bulk_load(st + 256, prow + 2 * a.prep_plane, 512, &bar_in[stg]);
+        }
+        bulk_load(st + G::OFF_MASK / 4, a.mask_terms + (folded ? a.mask_plane : 0) + ((long long)b * a.S + s) * a.npad + k0, 256, &bar_in[stg]);
       };
       if (nsteps > 0) {   // (a CTA with no rows must not leave a copy in flight)
         mbar_expect_tx(bar_once, 16384);
@@ -1138,8 +1244,13 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // ---------------------------------- MMA issue ----------------------------------------------
       constexpr uint32_t HI_KMAJ = desc_hi(G::SBO, G::LAYOUT);
       const uint32_t base_lo = desc_lo(smem_u32(smem), 16);
+      const uint32_t key_s = RowFactors::key_s(smem_u32(smem + G::OFF_KEY)), key_dp = RowFactors::key_dp(smem_u32(smem + G::OFF_KEY));
+      const uint32_t row_lo = RowFactors::query(smem_u32(stage_stat(0)));
+      int flag = nsteps > 0 ? large[0] : 0;
       for (int j = 0; j < nsteps && ok; ++j) {
         const int stg = j % G::NS, buf = j & 1;
+        const bool folded = flag == 0;
+        if (j + 1 < nsteps) flag = large[(long long)(j + 1) * a.H];
         if (j >= 2) ok = mbar_wait(&bar_free[(j - 2) & 3], ((j - 2) >> 2) & 1, a.err, 42) && ok;   // TMEM buffer is free
         ok = mbar_wait(&bar_in[stg], (j / G::NS) & 1, a.err, 43) && ok;
         tc_fence_after_sync();
@@ -1151,6 +1262,11 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
           umma<KIND_F16>(tmem_base + buf * 128 + 64, desc_join(do_lo + ks * 2, HI_KMAJ), desc_join(v_lo + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
+        if (folded) {
+          const uint64_t rows = desc_join(row_lo + stg * (G::STAGE >> 4), RowFactors::HI_QUERY);
+          umma<KIND_F16>(tmem_base + buf * 128, rows, desc_join(key_s, RowFactors::HI_KEY), a.idesc_a, 1);
+          umma<KIND_F16>(tmem_base + buf * 128 + 64, rows, desc_join(key_dp, RowFactors::HI_KEY), a.idesc_a, 1);
+        }
         umma_commit(&bar_s[buf]);
       }
     }
@@ -1159,16 +1275,14 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     float acc[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    const float2 sc2 = splat(a.scale), l2e2 = splat(kLog2e);
+    const float2 sc2 = splat(a.scale), l2e2 = splat(kLog2e), scl2 = splat(a.scale * kLog2e);
     if (nsteps > 0) ok = mbar_wait(bar_once, 0, a.err, 21);
 
-    for (int j = 0; j < nsteps; ++j) {
-      const int stg = j % G::NS, buf = j & 1;
-      ok = mbar_wait(&bar_in[stg], (j / G::NS) & 1, a.err, 43) && ok;   // statistics and mask terms of the row
-      const uint32_t st_a = smem_u32(stage_stat(stg)) + r * 4, mb_a = smem_u32(stage_stat(stg)) + 1536 + hh * 128;
-      const float2 nm2 = splat(lds32f(st_a)), nl2 = splat(lds32f(st_a + 512)), nd2 = splat(lds32f(st_a + 1024));
-      ok = mbar_wait(&bar_s[buf], (j >> 1) & 1, a.err, 24) && ok;
-      tc_fence_after_sync();
+    // a row's share of the sum
+    auto add_row = [&](auto fold, int stg, int buf) {
+      const uint32_t st_a = smem_u32(stage_stat(stg)) + r * 4, mb_a = smem_u32(stage_stat(stg)) + G::OFF_MASK + hh * 128;
+      float2 nm2, nl2, nd2;
+      if constexpr (!fold.value) { nm2 = splat(lds32f(st_a)); nl2 = splat(lds32f(st_a + 512)); nd2 = splat(lds32f(st_a + 1024)); }
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t rs[16], rp[16];
@@ -1184,18 +1298,34 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                                 make_float2(mB.z, mB.w)};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            float2 x = __ffma2_rn(pair(rs[u * 8 + 2 * i], rs[u * 8 + 2 * i + 1]), sc2, mk[i]);
-            x = __fadd2_rn(x, unpack2<T>(bw[i]));
-            const float2 e = __ffma2_rn(__fadd2_rn(x, nm2), l2e2, nl2);
-            const float2 p = make_float2(ex2_approx(e.x), ex2_approx(e.y));
-            const float2 ds = __fmul2_rn(p, __fadd2_rn(pair(rp[u * 8 + 2 * i], rp[u * 8 + 2 * i + 1]), nd2));
+            const float2 s2 = pair(rs[u * 8 + 2 * i], rs[u * 8 + 2 * i + 1]), d2 = pair(rp[u * 8 + 2 * i], rp[u * 8 + 2 * i + 1]);
             const int k = c * 16 + u * 8 + 2 * i;
-            const float2 t = __fadd2_rn(make_float2(acc[k], acc[k + 1]), ds);
+            const float2 sum = make_float2(acc[k], acc[k + 1]);
+            float2 t;
+            if constexpr (fold.value) {
+              const float2 e = __ffma2_rn(s2, scl2, __ffma2_rn(unpack2<T>(bw[i]), l2e2, mk[i]));
+              t = __ffma2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), d2, sum);
+            } else {
+              const float2 x = __fadd2_rn(__ffma2_rn(s2, sc2, mk[i]), unpack2<T>(bw[i]));
+              const float2 e = __ffma2_rn(__fadd2_rn(x, nm2), l2e2, nl2);
+              t = __fadd2_rn(sum, __fmul2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), __fadd2_rn(d2, nd2)));
+            }
             acc[k] = t.x;
             acc[k + 1] = t.y;
           }
         }
       }
+    };
+    int flag = nsteps > 0 ? large[0] : 0;
+    for (int j = 0; j < nsteps; ++j) {
+      const int stg = j % G::NS, buf = j & 1;
+      const bool folded = flag == 0;
+      if (j + 1 < nsteps) flag = large[(long long)(j + 1) * a.H];
+      ok = mbar_wait(&bar_in[stg], (j / G::NS) & 1, a.err, 43) && ok;   // statistics and mask terms of the row
+      ok = mbar_wait(&bar_s[buf], (j >> 1) & 1, a.err, 24) && ok;
+      tc_fence_after_sync();
+      if (folded) add_row(std::true_type{}, stg, buf);
+      else add_row(std::false_type{}, stg, buf);
       fence_proxy_async_smem();   // (TMA writes the row's statistics and mask terms over)
       tc_fence_before_sync();
       __syncwarp();
@@ -1227,32 +1357,44 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
 }
 
-// delta[b,s,h,i] = sum_d dO * O; also the per-row constants of the backward passes in the form their packed
-// arithmetic adds (prep[0] = -m, prep[1] = -log l * log2e, prep[2] = -delta), rows padded to npad entries.
+// delta[b,s,h,i] = sum_d dO * O (written where the dQ pass reads it); the row constants of the backward passes as factors (see
+// RowFactors), and for flagged rows in the form their packed arithmetic adds (prep[0] = -m, prep[1] = -log l * log2e,
+// prep[2] = -delta); rows padded to npad entries with zeros.  A block has 128 queries of a (batch, row), all heads of a query
+// one after the other: they share its cache lines.
 template <typename T>
-__global__ void attn_delta_tc_kernel(TriAttnDesc d, const T* o, const T* d_o, const float* stats, float* delta,
-                                     float* prep, int npad) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long total = (long long)d.B * d.n_seq * d.H * d.n_res;
-  if (idx >= total) return;
-  const int i = idx % d.n_res; long long z = idx / d.n_res;
-  const int h = z % d.H; z /= d.H;
-  const int s = z % d.n_seq; const int b = z / d.n_seq;
-  const T* orow = o + b * d.o_st[0] + s * d.o_st[1] + i * d.o_st[2] + h * d.o_st[3];
-  const T* grow = d_o + b * d.do_st[0] + s * d.do_st[1] + i * d.do_st[2] + h * d.do_st[3];
-  float acc = 0.f;
-  for (int g = 0; g < d.D / 8; ++g) {
-    float x[8], y[8];
-    unpack8<T>(reinterpret_cast<const uint4*>(orow)[g], x);
-    unpack8<T>(reinterpret_cast<const uint4*>(grow)[g], y);
+__global__ void __launch_bounds__(128) attn_delta_tc_kernel(TriAttnDesc d, const T* o, const T* d_o, const float* stats, float* delta,
+                                                            float* prep, uint4* aug, int* large, int npad) {
+  const unsigned chunks = npad / 128, bs = blockIdx.x / chunks;
+  const int i = (blockIdx.x - bs * chunks) * 128 + threadIdx.x;
+  const unsigned b = bs / (unsigned)d.n_seq, s = bs - b * (unsigned)d.n_seq;
+  const long long plane = (long long)d.B * d.n_seq * d.H * npad, total = (long long)d.B * d.n_seq * d.H * d.n_res;
+  const bool in = i < d.n_res;
+  const T* orow = o + b * d.o_st[0] + s * d.o_st[1] + i * d.o_st[2];
+  const T* grow = d_o + b * d.do_st[0] + s * d.do_st[1] + i * d.do_st[2];
+#pragma unroll 2
+  for (int h = 0; h < d.H; ++h) {
+    const long long row = (long long)bs * d.H + h, at = row * npad + i, idx = row * d.n_res + i;
+    float acc = 0.f, m = 0.f, ll = 0.f;
+    if (in) {
+      m = stats[idx];
+      ll = stats[total + idx];
+      for (int g = 0; g < d.D / 8; ++g) {
+        float x[8], y[8];
+        unpack8<T>(reinterpret_cast<const uint4*>(orow + h * d.o_st[3])[g], x);
+        unpack8<T>(reinterpret_cast<const uint4*>(grow + h * d.do_st[3])[g], y);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc = fmaf(x[e], y[e], acc);
+        for (int e = 0; e < 8; ++e) acc = fmaf(x[e], y[e], acc);
+      }
+      if (delta != nullptr) delta[idx] = acc;
+    }
+    const float c = in ? -(m + ll) / d.scale : 0.f;
+    const bool fits = RowFactors::fits<T>(m, c, acc);
+    if (!fits) large[row] = 1;
+    aug[at] = fits ? RowFactors::pack<T>(c, -acc) : make_uint4(0, 0, 0, 0);
+    prep[at] = -m;
+    prep[plane + at] = -ll * kLog2e;
+    prep[2 * plane + at] = -acc;
   }
-  delta[idx] = acc;
-  const long long pi = (idx / d.n_res) * npad + i, plane = (total / d.n_res) * npad;
-  prep[pi] = -stats[idx];
-  prep[plane + pi] = -stats[total + idx] * kLog2e;
-  prep[2 * plane + pi] = -acc;
 }
 
 // dq = scale * sum over key blocks of the merged pass's partials ([nparts][B][S][N][H][D] contiguous), added in key
@@ -1369,7 +1511,7 @@ template <typename T, int HD>
 int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
                const uint8_t* mask, const void* o, const float* stats, const void* d_o, void* dq, void* dk, void* dv,
                float* dbias, int* err, float* delta, float* dbias_partial, void* bias_t, void* bias_c, float* prep, float* mask_terms,
-               void* dq_part, cudaStream_t st) {
+               uint4* aug, int* large, void* dq_part, cudaStream_t st) {
   const long long rows = (long long)d->B * d->n_seq * d->H * d->n_res;
   const double pairs = (double)rows * d->n_res;
   const double tensor_bytes = 2.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D;
@@ -1379,17 +1521,19 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     KernelTimer kt("tc_attn_delta", st, 0.0, 2.0 * tensor_bytes);
     {
       const long long n = (long long)d->B * d->n_seq * npad;
-      mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, mask_terms, err);
+      mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, mask_terms, err,
+                                                      large, (long long)d->B * d->n_seq * d->H);
       TRI_LAUNCH_OK();
     }
-    if (npad != d->n_res) TRI_CUDA_OK(cudaMemsetAsync(prep, 0, 3 * prep_plane * sizeof(float), st));
-    attn_delta_tc_kernel<T><<<cdiv(rows, 256), 256, 0, st>>>(*d, (const T*)o, (const T*)d_o, stats, delta, prep, npad);
+    attn_delta_tc_kernel<T><<<(unsigned)(d->B * (long long)d->n_seq * (npad / 128)), 128, 0, st>>>(
+        *d, (const T*)o, (const T*)d_o, stats, HD == 32 ? nullptr : delta, prep, aug, large, npad);
     TRI_LAUNCH_OK();
   }
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   AttnBwdArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D; a.scale = d->scale;
-  a.stats = stats; a.delta = delta; a.prep = prep; a.prep_plane = prep_plane; a.npad = npad; a.mask_terms = mask_terms; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
+  a.stats = stats; a.delta = delta; a.prep = prep; a.prep_plane = prep_plane; a.npad = npad; a.mask_terms = mask_terms; a.mask_plane = (long long)d->B * d->n_seq * npad;
+  a.aug = aug; a.large = large; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
   a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0; a.err = err;
   a.row_chunks = 1;
   const int qblocks = (d->n_res + 127) / 128;
@@ -1508,7 +1652,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0;
   {
     const long long n = (long long)d->B * d->n_seq * a.npad;
-    mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, a.npad, mask_terms, err);
+    mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, a.npad, mask_terms, err, nullptr, 0);
     TRI_LAUNCH_OK();
   }
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
@@ -1583,7 +1727,9 @@ static size_t attn_ws_base(const TriAttnDesc* d, int is_bwd) {
          align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float)) +
          bias_copy_bytes(d) +                                                            // transposed copy of the bias
          align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)) +   // padded per-row constants
-         align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)) +              // additive key-mask terms
+         align_up(2 * (size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)) +          // additive key-mask terms
+         align_up((size_t)d->B * d->n_seq * d->H * attn_npad(d) * 16) +                  // row constants as factors
+         align_up((size_t)d->B * d->n_seq * d->H * sizeof(int)) +                        // rows that go without them
          attn_dq_part_bytes(d);                                                          // merged pass: dQ per key block
 }
 
@@ -1622,14 +1768,16 @@ int attn_backward(const TriAttnDesc* d, const void* q, const void* k, const void
   void* bias_t = reinterpret_cast<char*>(part) + align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float));
   float* prep = reinterpret_cast<float*>(static_cast<char*>(bias_t) + bias_copy_bytes(d));
   float* mterms = reinterpret_cast<float*>(reinterpret_cast<char*>(prep) + align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)));
-  void* dq_part = reinterpret_cast<char*>(mterms) + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));
+  uint4* aug = reinterpret_cast<uint4*>(reinterpret_cast<char*>(mterms) + align_up(2 * (size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)));
+  int* large = reinterpret_cast<int*>(reinterpret_cast<char*>(aug) + align_up((size_t)d->B * d->n_seq * d->H * attn_npad(d) * 16));
+  void* dq_part = reinterpret_cast<char*>(large) + align_up((size_t)d->B * d->n_seq * d->H * sizeof(int));
   void* bias_c = static_cast<char*>(ws) + attn_ws_base(d, 1);
   if (d->dtype == TRI_BF16) {
-    if (d->D <= 32) return bwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);
-    return bwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);
+    if (d->D <= 32) return bwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
+    return bwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
   }
-  if (d->D <= 32) return bwd_launch<__half, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);
-  return bwd_launch<__half, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, dq_part, st);
+  if (d->D <= 32) return bwd_launch<__half, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
+  return bwd_launch<__half, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
 }
 
 }  // namespace tc
