@@ -456,6 +456,13 @@ struct AttnBwdArgs {
   int* err;
 };
 
+// tcgen05.wait::ld that the registers of two loads pass through, so that no use of them can move above it
+__device__ __forceinline__ void ld_wait8x2(uint32_t (&v)[8], uint32_t (&w)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(w[0]),
+                 "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])::"memory");
+}
+
 // Row constants through the products.  With c = -(m + log l) / scale and -delta of a query as further channels of Q and dO,
 // against ones for every key, S and dP arrive as (x - m - log l) / scale without bias and mask, and as dP - delta: a logit
 // then takes two packed instructions up to the exponential, and no statistics are read beside it.  (As fp32 vectors in shared
@@ -1137,26 +1144,29 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------------------
-// dbias pass: one CTA per (row chunk, batch, head, 128-query block, 64-key block) looping over the rows of its chunk
+// dbias pass: one CTA per (row chunk, batch, head, 64-query block, 128-key block) looping over the rows of its chunk
 // in order and summing dS = P (dP - delta) in registers (no atomics: the sum over rows has a fixed order; the chunks'
 // partial sums are added by sum_partials_kernel).  320 threads: warps 0-7 do the arithmetic (thread (r, hh) owns
-// query r and key half hh), warp 8 issues the MMAs, warp 9 the TMA copies.  S and dP are double buffered in TMEM,
+// key r and query half hh), warp 8 issues the MMAs, warp 9 the TMA copies.  S^T and dP^T are double buffered in TMEM,
 // so the products of the next two rows run under the arithmetic of this one.
+// Thread = key: what varies over a thread's queries comes with the products (RowFactors), the mask is one value per row and
+// the bias, the same for all rows, stays in registers: nothing but the accumulators is read in the loop.
+// With thread = query, the bias tile and the rows' mask terms were read for every row: 0.81 -> 0.70 ms at N = 768, 4 heads.
 //   bar_s[2]    MMA -> threads        S, dP of a row are in TMEM buffer (row & 1)
 //   bar_free[4] threads -> MMA, TMA   the row's accumulators, statistics and mask terms have been read
 // ------------------------------------------------------------------------------------------------
 template <int HD> struct GeoB {
   static constexpr int RB = HD * 2;
-  static constexpr int TA = 128 * RB;                    // Q / dO tile
-  static constexpr int TB = 64 * RB;                     // K / V tile
+  static constexpr int TA = 128 * RB;                    // K / V tile
+  static constexpr int TB = 64 * RB;                     // Q / dO tile
   static constexpr uint32_t LAYOUT = RB == 128 ? 2 : 4;
   static constexpr uint32_t SBO = 8 * RB;
   static constexpr int NS = 3;                           // row stages
-  static constexpr int OFF_MASK = 2048 + 128;            // factors of 128 queries and zeros behind them, or (flagged rows)
-                                                         // -m, -log l log2e, -delta; then 64 mask terms
-  static constexpr int STAT = 3072;                      // (stages stay 1024-byte aligned for the swizzled tiles)
+  static constexpr int OFF_MASK = 1024 + 128;            // factors of 64 queries and zeros behind them, or (flagged rows)
+                                                         // -m, -log l log2e, -delta; then 128 mask terms
+  static constexpr int STAT = 2048;                      // (stages stay 1024-byte aligned for the swizzled tiles)
   static constexpr int STAGE = 2 * TA + 2 * TB + STAT;
-  static constexpr int OFF_BIAS = NS * STAGE;            // [128 queries x 64 keys] SW128, loaded once
+  static constexpr int OFF_BIAS = NS * STAGE;            // [128 keys x 64 queries] SW128, loaded once
   static constexpr int OFF_KEY = OFF_BIAS + 16384;
   static constexpr int OFF_BAR = OFF_KEY + RowFactors::kBytes;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
@@ -1176,14 +1186,14 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint64_t* bar_s = bar_once + 4;      // [2]
   uint64_t* bar_free = bar_once + 6;   // [4]: row j arrives on bar_free[j & 3]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_once + 10);
-  auto stage_q = [&](int stg) { return smem + stg * G::STAGE; };
-  auto stage_do = [&](int stg) { return smem + stg * G::STAGE + G::TA; };
-  auto stage_k = [&](int stg) { return smem + stg * G::STAGE + 2 * G::TA; };
-  auto stage_v = [&](int stg) { return smem + stg * G::STAGE + 2 * G::TA + G::TB; };
+  auto stage_k = [&](int stg) { return smem + stg * G::STAGE; };
+  auto stage_v = [&](int stg) { return smem + stg * G::STAGE + G::TA; };
+  auto stage_q = [&](int stg) { return smem + stg * G::STAGE + 2 * G::TA; };
+  auto stage_do = [&](int stg) { return smem + stg * G::STAGE + 2 * G::TA + G::TB; };
   auto stage_stat = [&](int stg) { return reinterpret_cast<float*>(smem + stg * G::STAGE + 2 * G::TA + 2 * G::TB); };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid & 127, hh = (tid >> 7) & 1;
-  const int qblocks = (a.N + 127) / 128, kblocks = (a.N + 63) / 64;
+  const int qblocks = (a.N + 63) / 64, kblocks = (a.N + 127) / 128;
   int z = blockIdx.x;
   const int kvb = z % kblocks; z /= kblocks;
   const int qb = z % qblocks; z /= qblocks;
@@ -1193,7 +1203,7 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int per = (a.S + a.row_chunks - 1) / a.row_chunks;
   const int s_lo = rc * per;
   const int nsteps = max(0, min(a.S, s_lo + per) - s_lo);
-  const int q0 = qb * 128, k0 = kvb * 64;
+  const int q0 = qb * 64, k0 = kvb * 128;
 
   if (tid == 0) {
     mbar_init(bar_once, 1);
@@ -1203,7 +1213,7 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_fence_init();
   }
   RowFactors::fill<T>(smem + G::OFF_KEY, tid);
-  if (tid >= 288 && tid < 288 + G::NS * 8) reinterpret_cast<uint4*>(stage_stat((tid - 288) / 8) + 512)[(tid - 288) % 8] = make_uint4(0, 0, 0, 0);
+  if (tid >= 288 && tid < 288 + G::NS * 8) reinterpret_cast<uint4*>(stage_stat((tid - 288) / 8) + 256)[(tid - 288) % 8] = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   if (warp == 0) tmem_alloc(tmem_slot, 256);
   tc_fence_before_sync();
@@ -1224,23 +1234,23 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const float* prow = a.prep + row0;
         const bool folded = large[(long long)step * a.H] == 0;
         float* st = stage_stat(stg);
-        mbar_expect_tx(&bar_in[stg], 2 * G::TA + 2 * G::TB + (folded ? 2048 : 3 * 512) + 256);
+        mbar_expect_tx(&bar_in[stg], 2 * G::TA + 2 * G::TB + (folded ? 1024 : 3 * 256) + 512);
         tma_load_5d(stage_q(stg), &tmQ, &bar_in[stg], 0, h, q0, s, b);
         tma_load_5d(stage_do(stg), &tmDO, &bar_in[stg], 0, h, q0, s, b);
         tma_load_5d(stage_k(stg), &tmK, &bar_in[stg], 0, h, k0, s, b);
         tma_load_5d(stage_v(stg), &tmV, &bar_in[stg], 0, h, k0, s, b);
         if (folded) {
-          bulk_load(st, a.aug + row0, 2048, &bar_in[stg]);
+          bulk_load(st, a.aug + row0, 1024, &bar_in[stg]);
         } else {
-          bulk_load(st, prow, 512, &bar_in[stg]);
-          bulk_load(st + 128, prow + a.prep_plane, 512, &bar_in[stg]);
-          bulk_load(st + 256, prow + 2 * a.prep_plane, 512, &bar_in[stg]);
+          bulk_load(st, prow, 256, &bar_in[stg]);
+          bulk_load(st + 64, prow + a.prep_plane, 256, &bar_in[stg]);
+          bulk_load(st + 128, prow + 2 * a.prep_plane, 256, &bar_in[stg]);
         }
-        bulk_load(st + G::OFF_MASK / 4, a.mask_terms + (folded ? a.mask_plane : 0) + ((long long)b * a.S + s) * a.npad + k0, 256, &bar_in[stg]);
+        bulk_load(st + G::OFF_MASK / 4, a.mask_terms + (folded ? a.mask_plane : 0) + ((long long)b * a.S + s) * a.npad + k0, 512, &bar_in[stg]);
       };
       if (nsteps > 0) {   // (a CTA with no rows must not leave a copy in flight)
         mbar_expect_tx(bar_once, 16384);
-        tma_load_4d(sBias, &tmBias, bar_once, k0, q0, h, b * a.bias_b_mul);
+        tma_load_4d(sBias, &tmBias, bar_once, q0, k0, h, b * a.bias_b_mul);   // transposed copy: queries inner
       }
       for (int st = 0; st < G::NS && st < nsteps; ++st) load_step(st);
       for (int j = 0; j + G::NS < nsteps && ok; ++j) {
@@ -1263,18 +1273,18 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (j >= 2) ok = mbar_wait(&bar_free[(j - 2) & 3], ((j - 2) >> 2) & 1, a.err, 42) && ok;   // TMEM buffer is free
         ok = mbar_wait(&bar_in[stg], (j / G::NS) & 1, a.err, 43) && ok;
         tc_fence_after_sync();
-        const uint32_t q_lo = base_lo + stg * (G::STAGE >> 4), do_lo = q_lo + (G::TA >> 4), k_lo = do_lo + (G::TA >> 4),
-                       v_lo = k_lo + (G::TB >> 4);
+        const uint32_t k_lo = base_lo + stg * (G::STAGE >> 4), v_lo = k_lo + (G::TA >> 4), q_lo = v_lo + (G::TA >> 4),
+                       do_lo = q_lo + (G::TB >> 4);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
-          umma<KIND_F16>(tmem_base + buf * 128, desc_join(q_lo + ks * 2, HI_KMAJ), desc_join(k_lo + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
+          umma<KIND_F16>(tmem_base + buf * 128, desc_join(k_lo + ks * 2, HI_KMAJ), desc_join(q_lo + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
-          umma<KIND_F16>(tmem_base + buf * 128 + 64, desc_join(do_lo + ks * 2, HI_KMAJ), desc_join(v_lo + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
+          umma<KIND_F16>(tmem_base + buf * 128 + 64, desc_join(v_lo + ks * 2, HI_KMAJ), desc_join(do_lo + ks * 2, HI_KMAJ), a.idesc_a, ks > 0);
         if (folded) {
           const uint64_t rows = desc_join(row_lo + stg * (G::STAGE >> 4), RowFactors::HI_QUERY);
-          umma<KIND_F16>(tmem_base + buf * 128, rows, desc_join(key_s, RowFactors::HI_KEY), a.idesc_a, 1);
-          umma<KIND_F16>(tmem_base + buf * 128 + 64, rows, desc_join(key_dp, RowFactors::HI_KEY), a.idesc_a, 1);
+          umma<KIND_F16>(tmem_base + buf * 128, desc_join(key_s, RowFactors::HI_KEY), rows, a.idesc_a, 1);
+          umma<KIND_F16>(tmem_base + buf * 128 + 64, desc_join(key_dp, RowFactors::HI_KEY), rows, a.idesc_a, 1);
         }
         umma_commit(&bar_s[buf]);
       }
@@ -1286,44 +1296,49 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     const float2 sc2 = splat(a.scale), l2e2 = splat(kLog2e), scl2 = splat(a.scale * kLog2e);
     if (nsteps > 0) ok = mbar_wait(bar_once, 0, a.err, 21);
+    uint4 bias[4];   // of this thread's key and 32 queries
+#pragma unroll
+    for (int u = 0; u < 4; ++u) bias[u] = nsteps > 0 ? lds128(smem_u32(sBias) + sw128_chunk1(r, hh * 4 + u)) : make_uint4(0, 0, 0, 0);
 
-    // a row's share of the sum
+    // a row's share of the sum, eight queries at a time with the next eight on their way
     auto add_row = [&](auto fold, int stg, int buf) {
-      const uint32_t st_a = smem_u32(stage_stat(stg)) + r * 4, mb_a = smem_u32(stage_stat(stg)) + G::OFF_MASK + hh * 128;
-      float2 nm2, nl2, nd2;
-      if constexpr (!fold.value) { nm2 = splat(lds32f(st_a)); nl2 = splat(lds32f(st_a + 512)); nd2 = splat(lds32f(st_a + 1024)); }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t rs[16], rp[16];
-        tmem_ld_32x16(t_row + buf * 128 + hh * 32 + c * 16, rs);
-        tmem_ld_32x16(t_row + buf * 128 + 64 + hh * 32 + c * 16, rp);
-        tmem_ld_wait();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint4 raw = lds128(smem_u32(sBias) + sw128_chunk1(r, hh * 4 + c * 2 + u));   // same tile for every row
-          const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
-          const float4 mA = lds128f(mb_a + (c * 4 + u * 2) * 16), mB = lds128f(mb_a + (c * 4 + u * 2 + 1) * 16);
-          const float2 mk[4] = {make_float2(mA.x, mA.y), make_float2(mA.z, mA.w), make_float2(mB.x, mB.y),
-                                make_float2(mB.z, mB.w)};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 s2 = pair(rs[u * 8 + 2 * i], rs[u * 8 + 2 * i + 1]), d2 = pair(rp[u * 8 + 2 * i], rp[u * 8 + 2 * i + 1]);
-            const int k = c * 16 + u * 8 + 2 * i;
-            const float2 sum = make_float2(acc[k], acc[k + 1]);
-            float2 t;
-            if constexpr (fold.value) {
-              const float2 e = __ffma2_rn(s2, scl2, __ffma2_rn(unpack2<T>(bw[i]), l2e2, mk[i]));
-              t = __ffma2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), d2, sum);
-            } else {
-              const float2 x = __fadd2_rn(__ffma2_rn(s2, sc2, mk[i]), unpack2<T>(bw[i]));
-              const float2 e = __ffma2_rn(__fadd2_rn(x, nm2), l2e2, nl2);
-              t = __fadd2_rn(sum, __fmul2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), __fadd2_rn(d2, nd2)));
-            }
-            acc[k] = t.x;
-            acc[k + 1] = t.y;
-          }
+      const uint32_t st_a = smem_u32(stage_stat(stg)), t_s = t_row + buf * 128 + hh * 32;
+      const float2 mk2 = splat(lds32f(st_a + G::OFF_MASK + r * 4));   // (in units of log 2 where folded)
+      auto eight = [&](uint32_t (&rs)[8], uint32_t (&rp)[8], uint32_t (&ns)[8], uint32_t (&np)[8], int u) {
+        ld_wait8x2(rs, rp);
+        if (u < 3) {
+          tmem_ld_32x8(t_s + (u + 1) * 8, ns);
+          tmem_ld_32x8(t_s + 64 + (u + 1) * 8, np);
         }
-      }
+        const uint32_t bw[4] = {bias[u].x, bias[u].y, bias[u].z, bias[u].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 s2 = pair(rs[2 * i], rs[2 * i + 1]), d2 = pair(rp[2 * i], rp[2 * i + 1]);
+          const int k = u * 8 + 2 * i;
+          const float2 sum = make_float2(acc[k], acc[k + 1]);
+          float2 t;
+          if constexpr (fold.value) {
+            const float2 e = __ffma2_rn(s2, scl2, __ffma2_rn(unpack2<T>(bw[i]), l2e2, mk2));
+            t = __ffma2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), d2, sum);
+          } else {
+            const uint32_t at = st_a + (hh * 32 + k) * 4;
+            const float2 nm = make_float2(lds32f(at), lds32f(at + 4)), nl = make_float2(lds32f(at + 256), lds32f(at + 260)),
+                         nd = make_float2(lds32f(at + 512), lds32f(at + 516));
+            const float2 x = __fadd2_rn(__ffma2_rn(s2, sc2, mk2), unpack2<T>(bw[i]));
+            const float2 e = __ffma2_rn(__fadd2_rn(x, nm), l2e2, nl);
+            t = __fadd2_rn(sum, __fmul2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), __fadd2_rn(d2, nd)));
+          }
+          acc[k] = t.x;
+          acc[k + 1] = t.y;
+        }
+      };
+      uint32_t sA[8], pA[8], sB[8], pB[8];
+      tmem_ld_32x8(t_s, sA);
+      tmem_ld_32x8(t_s + 64, pA);
+      eight(sA, pA, sB, pB, 0);
+      eight(sB, pB, sA, pA, 1);
+      eight(sA, pA, sB, pB, 2);
+      eight(sB, pB, sA, pA, 3);
     };
     int flag = nsteps > 0 ? large[0] : 0;
     for (int j = 0; j < nsteps; ++j) {
@@ -1342,20 +1357,14 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (!ok) break;
     }
 
-    const int qi = q0 + r;
-    if (qi < a.N && ok) {
-      float* row = reinterpret_cast<float*>(a.out0) + (long long)rc * a.B * a.H * a.N * a.N +
-                   (((long long)b * a.H + h) * a.N + qi) * a.N + k0 + hh * 32;
-      const int valid = a.N - k0 - hh * 32;
-      if (valid >= 32 && (a.N % 4) == 0) {
+    const int kj = k0 + r;
+    if (kj < a.N && ok) {   // a query at a time: lanes are consecutive keys
+      float* at = reinterpret_cast<float*>(a.out0) + (long long)rc * a.B * a.H * a.N * a.N +
+                  (((long long)b * a.H + h) * a.N + q0 + hh * 32) * a.N + kj;
+      const int valid = a.N - q0 - hh * 32;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          reinterpret_cast<float4*>(row)[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (i < valid) row[i] = acc[i];
-      }
+      for (int i = 0; i < 32; ++i)
+        if (i < valid) at[(long long)i * a.N] = acc[i];
     }
   }
   tc_fence_before_sync();
@@ -1587,20 +1596,21 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     TRI_LAUNCH_OK();
   }
   // ---- dQ ------------------------------------------------------------------------------------
-  TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, HD));
-  TRI_TRY(qkv_tile_map(&tdo, d_o, d, d->do_st, 128, HD));
-  TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, HD));
-  TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, HD));
-  if (bias && (!kMerge || dbias != nullptr)) {
-    const bool own = bias_fits_tma(d, bias);
-    if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
-    TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
-  }
-  a.out0 = dq; a.out1 = nullptr;
-  for (int i = 0; i < 4; ++i) a.out0_st[i] = d->dq_st[i];
-  a.idesc_a = make_idesc(kind, 128, 64, false, false);
-  a.idesc_b = make_idesc(kind, 128, HD, false, true);
   if (!kMerge) {
+    CUtensorMap tq, tdo, tk, tv, tb;   // (the dK/dV pass's serve the dbias pass too)
+    TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, HD));
+    TRI_TRY(qkv_tile_map(&tdo, d_o, d, d->do_st, 128, HD));
+    TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, HD));
+    TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, HD));
+    if (bias) {
+      const bool own = bias_fits_tma(d, bias);
+      if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
+      TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
+    } else {
+      tb = tq;
+    }
+    a.out0 = dq; a.out1 = nullptr;
+    for (int i = 0; i < 4; ++i) a.out0_st[i] = d->dq_st[i];
     auto kern = bias ? attn_bwd_dq_kernel<T, HD, true> : attn_bwd_dq_kernel<T, HD, false>;
     TRI_TRY(set_dyn_smem(kern, GeoQ<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dq", st, 2.0 * pairs * d->D, 5.0 * tensor_bytes);
@@ -1609,21 +1619,24 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   }
   // ---- dbias ---------------------------------------------------------------------------------
   if (dbias != nullptr) {
-    // Row chunks only as far as they are needed to fill the GPU (two CTAs per SM): with enough (batch, head, query
-    // block, key block) combinations one CTA sums all rows and no partial sums are written or added.
-    const long long combos = (long long)qblocks * ((d->n_res + 63) / 64) * d->B * d->H, slots = 2LL * sm_count();
+    // Row chunks until the CTAs fill the GPU, as few as give the fewest rows in a row: rounds of CTAs times rows of a chunk.  (One
+    // round more for the last few CTAs costs as much as the rounds before: 301 residues, 60 tiles, 5 chunks 113 us, 4 chunks 84.)
+    const int qtiles = (d->n_res + 63) / 64;
+    const long long combos = (long long)qblocks * qtiles * d->B * d->H, slots = (HD == 32 ? 2LL : 1LL) * sm_count();
     int chunks = 1;
-    if (combos * 10 < slots * 9) chunks = (int)std::min<long long>(kDbiasRowChunks, (slots + combos - 1) / combos);
-    chunks = std::max(1, std::min(chunks, d->n_seq / 2));
+    long long best = -1;
+    for (int ch = 1; ch <= std::min(kDbiasRowChunks, std::max(1, d->n_seq / 2)); ++ch) {
+      const long long steps = (combos * ch + slots - 1) / slots * cdiv(d->n_seq, ch);
+      if (best < 0 || steps * 10 < best * 9) { best = steps; chunks = ch; }   // (each chunk costs a partial sum)
+    }
     const long long nb = (long long)d->B * d->H * d->n_res * d->n_res;
-    const int kblocks = (d->n_res + 63) / 64;
     a.row_chunks = chunks;
     a.out0 = chunks > 1 ? dbias_partial : dbias;
     a.idesc_a = make_idesc(kind, 128, 64, false, false);
-    auto kern = attn_bwd_dbias_kernel<T, HD>;   // (K / V maps with 64-key boxes and the bias map are those of the dQ pass)
+    auto kern = attn_bwd_dbias_kernel<T, HD>;   // (with the dK/dV pass's maps)
     TRI_TRY(set_dyn_smem(kern, GeoB<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor_bytes);
-    launch_dependent(kern, (unsigned)((long long)qblocks * kblocks * d->B * d->H * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
+    launch_dependent(kern, (unsigned)(combos * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     if (chunks > 1) {   // fixed-order sum of the row-chunk partials
       sum_partials_kernel<<<cdiv(nb, 256), 256, 0, st>>>(dbias_partial, chunks, nb, dbias);
