@@ -554,6 +554,10 @@ template <int HD> struct GeoC {
 // blocks' partials in fixed order.  A last tile without a partner is paired with a buffer of zeros.
 // The MMA warp runs its code as a whole, so that descriptors stay in uniform registers (a lone lane took 900 clocks to issue a
 // tile's products), and dQ is fetched after a tile's arrival on bar_p, beside its products: 1.56 -> 1.45 ms at N = 768.
+// Accumulators are read eight queries at a time, the next eight on their way (the wait for a tile's first half had been 600 of
+// 4100 clocks), and dQ leaves as 32-byte sectors: 1.45 -> 1.36 ms.  From there on a sustained training step at N = 768 runs at the
+// board's power limit (1.8 GHz).  A persistent form (items as one stream) was slower, 1.47 -> 1.58 ms: K and V have no second
+// buffer, and the two CTAs of an SM no longer change places.
 template <typename T, int HD, bool HB, bool MERGE>
 __global__ void __launch_bounds__(320, 2)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
@@ -747,14 +751,17 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (qi < a.N && ok) {
         T* dst = reinterpret_cast<T*>(a.dq_part) + kvb * a.dq_part_plane +
                  ((((long long)b * a.S + s) * a.N + qi) * a.H + h) * a.D + hh * 16;
+        uint32_t w[8];
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          uint4 pk;
-          pk.x = pack2<T>(__uint_as_float(v[g * 8 + 0]), __uint_as_float(v[g * 8 + 1]));
-          pk.y = pack2<T>(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3]));
-          pk.z = pack2<T>(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
-          pk.w = pack2<T>(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]));
-          if (hh * 16 + g * 8 < a.D) reinterpret_cast<uint4*>(dst)[g] = pk;
+        for (int i = 0; i < 8; ++i) w[i] = pack2<T>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        if (a.D == 32) {   // a whole 32-byte sector
+          asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                       "r"(w[5]), "r"(w[6]), "r"(w[7])
+                       : "memory");
+        } else {
+#pragma unroll
+          for (int g = 0; g < 2; ++g)
+            if (hh * 16 + g * 8 < a.D) reinterpret_cast<uint4*>(dst)[g] = make_uint4(w[g * 4], w[g * 4 + 1], w[g * 4 + 2], w[g * 4 + 3]);
         }
       }
     };
@@ -773,26 +780,32 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t st_a = smem_u32(sRow) + qstg * G::ST;   // -m, -log l log2e, -delta of 64 queries, 256 bytes each
       const int c = hh;
       uint32_t pw[16], dw[16];
-      // 16 of this thread's 32 queries
-      auto half = [&](auto fold, const uint32_t (&rs)[16], const uint32_t (&rp)[16], int h2) {
+      // this thread's 32 queries, eight at a time with the next eight's accumulators on their way
+      const uint32_t t_s = t_row + hh * 32, t_d = t_row + COL_DP + hh * 32;
+      auto eight = [&](auto fold, uint32_t (&rs)[8], uint32_t (&rp)[8], uint32_t (&ns)[8], uint32_t (&np)[8], int u) {
+        ld_wait8x2(rs, rp);
+        if (u < 3) {
+          tmem_ld_32x8(t_s + (u + 1) * 8, ns);
+          tmem_ld_32x8(t_d + (u + 1) * 8, np);
+        } else {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_free);   // this warp holds its logits: the accumulators can take the next tile
+        }
+        uint4 raw = make_uint4(0, 0, 0, 0);
+        if constexpr (HB) raw = lds128(sPTj + sw128_chunk1(r, c * 4 + u));
+        const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
+        if constexpr (fold.value) {
 #pragma unroll
-        for (int uu = 0; uu < 2; ++uu) {
-          const int u = h2 * 2 + uu;
-          uint4 raw = make_uint4(0, 0, 0, 0);
-          if constexpr (HB) raw = lds128(sPTj + sw128_chunk1(r, c * 4 + u));
-          const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
-          if constexpr (fold.value) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 t = HB ? __ffma2_rn(unpack2<T>(bw[i]), l2e2, mkl2) : mkl2;
-              const float2 e = __ffma2_rn(pair(rs[uu * 8 + 2 * i], rs[uu * 8 + 2 * i + 1]), scl2, t);
-              const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
-              const float2 ds = __fmul2_rn(pp, pair(rp[uu * 8 + 2 * i], rp[uu * 8 + 2 * i + 1]));
-              pw[u * 4 + i] = pack2<T>(pp.x, pp.y);
-              dw[u * 4 + i] = pack2<T>(ds.x, ds.y);
-            }
-            continue;
+          for (int i = 0; i < 4; ++i) {
+            const float2 t = HB ? __ffma2_rn(unpack2<T>(bw[i]), l2e2, mkl2) : mkl2;
+            const float2 e = __ffma2_rn(pair(rs[2 * i], rs[2 * i + 1]), scl2, t);
+            const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+            const float2 ds = __fmul2_rn(pp, pair(rp[2 * i], rp[2 * i + 1]));
+            pw[u * 4 + i] = pack2<T>(pp.x, pp.y);
+            dw[u * 4 + i] = pack2<T>(ds.x, ds.y);
           }
+        } else {
           const uint32_t at = st_a + (c * 8 + u * 2) * 16;
           const float4 m0 = lds128f(at), m1 = lds128f(at + 16);
           const float4 l0 = lds128f(at + 256), l1 = lds128f(at + 272);
@@ -802,31 +815,27 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const float2 nd[4] = {make_float2(d0.x, d0.y), make_float2(d0.z, d0.w), make_float2(d1.x, d1.y), make_float2(d1.z, d1.w)};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            float2 x = __ffma2_rn(pair(rs[uu * 8 + 2 * i], rs[uu * 8 + 2 * i + 1]), sc2, mk2);
+            float2 x = __ffma2_rn(pair(rs[2 * i], rs[2 * i + 1]), sc2, mk2);
             if constexpr (HB) x = __fadd2_rn(x, unpack2<T>(bw[i]));
             const float2 e = __ffma2_rn(__fadd2_rn(x, nm[i]), l2e2, nl[i]);
             const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
-            const float2 ds = __fmul2_rn(pp, __fadd2_rn(pair(rp[uu * 8 + 2 * i], rp[uu * 8 + 2 * i + 1]), nd[i]));
+            const float2 ds = __fmul2_rn(pp, __fadd2_rn(pair(rp[2 * i], rp[2 * i + 1]), nd[i]));
             pw[u * 4 + i] = pack2<T>(pp.x, pp.y);
             dw[u * 4 + i] = pack2<T>(ds.x, ds.y);
           }
         }
       };
-      // the second half's TMEM loads are in flight while the first half is computed
-      uint32_t rsA[16], rpA[16], rsB[16], rpB[16];
-      tmem_ld_32x16(t_row + hh * 32, rsA);
-      tmem_ld_32x16(t_row + COL_DP + hh * 32, rpA);
-      tmem_ld_wait();
-      tmem_ld_32x16(t_row + hh * 32 + 16, rsB);
-      tmem_ld_32x16(t_row + COL_DP + hh * 32 + 16, rpB);
-      if (folded) half(std::true_type{}, rsA, rpA, 0);
-      else half(std::false_type{}, rsA, rpA, 0);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_free);   // this warp holds its logits: the accumulators can take the next tile
-      if (folded) half(std::true_type{}, rsB, rpB, 1);
-      else half(std::false_type{}, rsB, rpB, 1);
+      auto tile = [&](auto fold) {
+        uint32_t sA[8], pA[8], sB[8], pB[8];
+        tmem_ld_32x8(t_s, sA);
+        tmem_ld_32x8(t_d, pA);
+        eight(fold, sA, pA, sB, pB, 0);
+        eight(fold, sB, pB, sA, pA, 1);
+        eight(fold, sA, pA, sB, pB, 2);
+        eight(fold, sB, pB, sA, pA, 3);
+      };
+      if (folded) tile(std::true_type{});
+      else tile(std::false_type{});
       if constexpr (!TMEM_A) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
