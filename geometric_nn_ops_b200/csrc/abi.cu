@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "tc_gemm.cuh"
 #include "tc_lnproject.cuh"
+#include "tc_attn_tf32.cuh"
 #include "tc_paths.cuh"
 #include "trimul_simt.cuh"
 
@@ -160,7 +161,8 @@ int tri_profile_summary(char* buf, size_t cap) {
 size_t tri_attn_ws_bytes(const TriAttnDesc* d, int is_bwd) {
   if (check_attn(d) != 0) return 0;
   const size_t n = simt::attn_ws_bytes(d, is_bwd);
-  return d->dtype == TRI_F32 ? n : std::max(n, tc::attn_ws_bytes(d, is_bwd));
+  if (d->dtype == TRI_F32) return tc::attn_tf32_supported(d, is_bwd) ? std::max(n, tc::attn_tf32_ws_bytes(d, is_bwd)) : n;
+  return std::max(n, tc::attn_ws_bytes(d, is_bwd));
 }
 
 int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
@@ -170,6 +172,10 @@ int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o}) && tc::attn_bias_has_room(d, bias, ws_bytes, 0)) {
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
+  }
+  if (tc::attn_tf32_supported(d, 0) && aligned_to(16, {q, k, v, o}) && ws != nullptr && ws_bytes >= tc::attn_tf32_ws_bytes(d, 0)) {
+    set_path("tcgen05");
+    return tc::attn_tf32_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
   set_path("simt");
   return simt::attn_forward(d, q, k, v, bias, mask, o, lse, (cudaStream_t)stream);
@@ -185,6 +191,10 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);
+  }
+  if (tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
+    set_path("tcgen05");
+    return tc::attn_tf32_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes, (cudaStream_t)stream);
   }
   set_path("simt");
   return simt::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,

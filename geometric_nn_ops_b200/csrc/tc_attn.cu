@@ -24,6 +24,7 @@
 
 #include "tc_attn_common.cuh"
 #include "tc_attn_rows.cuh"
+#include "tc_attn_tf32.cuh"
 #include "tc_paths.cuh"
 
 namespace tri {
@@ -254,7 +255,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int kk = 0; kk < 8; ++kk) {   // O_half += P[:, half] V[half]: keys 64 * (kk >> 2) + 16 * (kk & 3) ...
           const uint64_t vd = desc_join(vmn_lo + so + kk * G::RB, HI_KMAJ);
           const uint32_t accf = (j > 0 || (kk & 3) > 0) ? 1u : 0u;
-          if constexpr (TMEM_P) umma_ts_f16(tmem_base + COL_O + (kk >> 2) * HD, tmem_base + COL_P + kk * 8, vd, a.idesc_pv, accf);
+          if constexpr (TMEM_P) umma_ts<KIND_F16>(tmem_base + COL_O + (kk >> 2) * HD, tmem_base + COL_P + kk * 8, vd, a.idesc_pv, accf);
           else umma<KIND_F16>(tmem_base + COL_O + (kk >> 2) * HD, desc_join(p_lo + po + (kk >> 2) * 1024 + (kk & 3) * 2, HI_P), vd, a.idesc_pv, accf);
         }
         umma_commit(&bar_pv[stg]);
@@ -455,13 +456,6 @@ struct AttnBwdArgs {
   int row_chunks;              // MODE_DBIAS: the row loop is split into this many CTAs, each writing its own partial
   int* err;
 };
-
-// tcgen05.wait::ld that the registers of two loads pass through, so that no use of them can move above it
-__device__ __forceinline__ void ld_wait8x2(uint32_t (&v)[8], uint32_t (&w)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(w[0]),
-                 "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])::"memory");
-}
 
 // Row constants through the products.  With c = -(m + log l) / scale and -delta of a query as further channels of Q and dO,
 // against ones for every key, S and dP arrive as (x - m - log l) / scale without bias and mask, and as dP - delta: a logit
@@ -712,14 +706,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int kk = 0; kk < 4; ++kk) {   // dV += P^T dO   (B = dO as [n = d, k = query]: MN-major)
             const uint64_t bd = desc_join(domn_lo + so + kk * G::RB, HI_KMAJ);
             const uint32_t accf = (j > 0 || kk > 0) ? 1u : 0u;
-            if constexpr (TMEM_A) umma_ts_f16(tmem_base + COL_DV, tmem_base + COL_PT + kk * 8, bd, a.idesc_b, accf);
+            if constexpr (TMEM_A) umma_ts<KIND_F16>(tmem_base + COL_DV, tmem_base + COL_PT + kk * 8, bd, a.idesc_b, accf);
             else umma<KIND_F16>(tmem_base + COL_DV, desc_join(pt_lo + bo + kk * 2, HI_PT), bd, a.idesc_b, accf);
           }
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {   // dK += dS^T Q
             const uint64_t bd = desc_join(qmn_lo + so + kk * G::RB, HI_KMAJ);
             const uint32_t accf = (j > 0 || kk > 0) ? 1u : 0u;
-            if constexpr (TMEM_A && !MERGE) umma_ts_f16(tmem_base + COL_DK, tmem_base + COL_DST + kk * 8, bd, a.idesc_b, accf);
+            if constexpr (TMEM_A && !MERGE) umma_ts<KIND_F16>(tmem_base + COL_DK, tmem_base + COL_DST + kk * 8, bd, a.idesc_b, accf);
             else umma<KIND_F16>(tmem_base + COL_DK, desc_join(dst_lo + bo + kk * 2, HI_PT), bd, a.idesc_b, accf);
           }
           if constexpr (MERGE) {
@@ -1048,7 +1042,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t so = (j % G::NS) * (G::TB >> 4);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)   // dQ += dS K   (A = dS from TMEM, B = K as [n = d, k = key]: MN-major)
-          umma_ts_f16(tmem_base + COL_DQ, tmem_base + COL_DS + kk * 8, desc_join(kmn_lo + so + kk * G::RB, HI_KMAJ), a.idesc_b,
+          umma_ts<KIND_F16>(tmem_base + COL_DQ, tmem_base + COL_DS + kk * 8, desc_join(kmn_lo + so + kk * G::RB, HI_KMAJ), a.idesc_b,
                       (j > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&bar_dq[j & 3]);
       }
@@ -1546,12 +1540,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   const long long prep_plane = (long long)d->B * d->n_seq * d->H * npad;
   {
     KernelTimer kt("tc_attn_delta", st, 0.0, 2.0 * tensor_bytes);
-    {
-      const long long n = (long long)d->B * d->n_seq * npad;
-      mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, mask_terms, err,
-                                                      large, (long long)d->B * d->n_seq * d->H);
-      TRI_LAUNCH_OK();
-    }
+    TRI_TRY(launch_mask_terms(d, mask, mask_terms, err, large, st));
     attn_delta_tc_kernel<T><<<(unsigned)(d->B * (long long)d->n_seq * (npad / 128)), 128, 0, st>>>(
         *d, (const T*)o, (const T*)d_o, stats, HD == 32 ? nullptr : delta, prep, aug, large, npad);
     TRI_LAUNCH_OK();
@@ -1681,11 +1670,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   a.o = o; for (int i = 0; i < 4; ++i) a.o_st[i] = d->o_st[i];
   a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
   a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0;
-  {
-    const long long n = (long long)d->B * d->n_seq * a.npad;
-    mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, a.npad, mask_terms, err, nullptr, 0);
-    TRI_LAUNCH_OK();
-  }
+  TRI_TRY(launch_mask_terms(d, mask, mask_terms, err, nullptr, st));
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   a.idesc_s = make_idesc(kind, 128, 128, false, false);
   a.idesc_pv = make_idesc(kind, 128, HD, false, true);
@@ -1695,7 +1680,12 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
     TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
   }
-  if (rows) return attn_fwd_rows(d, q, k, v, bias ? &tb : nullptr, a.bias_b_mul != 0, o, stats, mask_terms, err, st);
+  if (rows) {
+    TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, 32));
+    TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, 32));
+    TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, 32));
+    return attn_fwd_rows(d, tq, tk, tv, bias ? &tb : nullptr, a.bias_b_mul != 0, o, stats, mask_terms, err, st);
+  }
   TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, HD));
   TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 128, HD));
   TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 128, HD));
@@ -1711,6 +1701,15 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
 }
 
 }  // namespace
+
+int launch_mask_terms(const TriAttnDesc* d, const uint8_t* mask, float* out, int* err, int* flags, cudaStream_t st) {
+  const int npad = (d->n_res + 127) / 128 * 128;
+  const long long n = (long long)d->B * d->n_seq * npad;
+  mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, out, err, flags,
+                                                  flags != nullptr ? (long long)d->B * d->n_seq * d->H : 0LL);
+  TRI_LAUNCH_OK();
+  return 0;
+}
 
 int qkv_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, const int64_t* st, int rows, int width) {
   const uint64_t dims[5] = {(uint64_t)d->D, (uint64_t)d->H, (uint64_t)d->n_res, (uint64_t)d->n_seq, (uint64_t)d->B};

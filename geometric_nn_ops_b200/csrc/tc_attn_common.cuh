@@ -18,6 +18,13 @@ __device__ __forceinline__ int sw128_chunk(int r, int g) {
 template <typename T> struct ElemIsBf16 { static constexpr bool value = false; };
 template <> struct ElemIsBf16<__nv_bfloat16> { static constexpr bool value = true; };
 
+// tcgen05.wait::ld that the registers of two loads pass through, so that no use of them can move above it
+__device__ __forceinline__ void ld_wait8x2(uint32_t (&v)[8], uint32_t (&w)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(w[0]),
+                 "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])::"memory");
+}
+
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;

@@ -1,4 +1,5 @@
-// Forward triangle attention, 16-bit types, head dim up to 32: three rows of the pair tensor share a pair-bias tile.
+// Forward triangle attention, 16-bit types and fp32 with TF32 products, head dim up to 32: three rows of the pair tensor
+// (fp32: two) share a pair-bias tile.
 //
 // The pair bias depends on (head, query, key) only, so rows s .. s+2 of one head and 128-query block read the same
 // bias tiles.  A CTA takes such a triple: three groups of four softmax warps, one row each, walk the key axis in steps
@@ -38,9 +39,32 @@ namespace tc {
 
 namespace {
 
-constexpr int kGroups = 3;                  // rows per CTA
-constexpr int kBiasStages = 4;
-constexpr int kThreads = (4 * kGroups + kGroups + 1) * 32;   // softmax warps, issuing warps, one warp for the bias tiles
+// fp32: tiles are twice as large, which leaves room for two rows per CTA; operands were rounded to TF32 before, P is as it is
+// stored.  P takes one column per key and so replaces S in place; V is read across its rows, which 32-bit operands can only be
+// in the swizzle with 32-byte atoms.
+template <typename T> struct RowsCfg {
+  static constexpr bool F32 = sizeof(T) == 4;
+  static constexpr int kGroups = F32 ? 2 : 3;      // rows per CTA
+  static constexpr int kBiasStages = F32 ? 2 : 4;
+  static constexpr int kThreads = (4 * kGroups + kGroups + 1) * 32;   // softmax warps, issuing warps, one warp for the bias tiles
+  static constexpr int kQ = F32 ? 2 : 3;           // Q buffers (two suffice where a row has two key steps)
+  static constexpr int RB = 32 * sizeof(T);        // bytes of a Q, K or V row
+  static constexpr int TQ = 128 * RB, TK = 64 * RB, TB = 128 * 64 * sizeof(T);   // bytes: Q tile, K or V tile, bias tile
+  static constexpr int OFF_BIAS = 0;
+  static constexpr int OFF_Q = OFF_BIAS + kBiasStages * TB;     // [group][kQ]
+  static constexpr int OFF_K = OFF_Q + kGroups * kQ * TQ;       // [group][3]
+  static constexpr int OFF_V = OFF_K + kGroups * 3 * TK;        // [group][3]
+  static constexpr int OFF_M = OFF_V + kGroups * 3 * TK;        // [bias stage][group] x 64 mask terms
+  static constexpr int OFF_BAR = OFF_M + kBiasStages * kGroups * 256;
+  static constexpr int SMEM = OFF_BAR + 1024 + 1024;
+  static constexpr int PC = F32 ? 64 : 32;         // columns of P: a step's 64 keys
+  static constexpr int KS = F32 ? 4 : 2;           // products of a step's S: 32 channels, 32 bytes each
+  static constexpr int KV = F32 ? 8 : 4;           // ... of its P V: 64 keys
+  static constexpr uint32_t HI = F32 ? desc_hi(8 * 128, 2) : desc_hi(8 * 64, 4);        // Q, K: SWIZZLE_128B, SWIZZLE_64B
+  static constexpr uint32_t HI_V = F32 ? desc_hi(512, 1) : desc_hi(8 * 64, 4);          // V across its rows
+  static constexpr int kind = F32 ? KIND_TF32 : KIND_F16;
+  static constexpr int kVec = 16 / (int)sizeof(T); // elements of a 16-byte piece
+};
 constexpr float kLn2 = 0.6931471805599453f;
 
 struct RowsArgs {
@@ -55,17 +79,6 @@ struct RowsArgs {
   int rows_per_item;         // groups in use (fewer where a triple per CTA would leave SMs idle)
   uint32_t idesc_s, idesc_pv;
   int* err;
-};
-
-struct RowsSmem {
-  static constexpr int TQ = 128 * 64, TK = 64 * 64, TB = 128 * 128;   // bytes: Q tile, K or V tile, bias tile
-  static constexpr int OFF_BIAS = 0;
-  static constexpr int OFF_Q = OFF_BIAS + kBiasStages * TB;     // [group][3]
-  static constexpr int OFF_K = OFF_Q + kGroups * 3 * TQ;        // [group][3]
-  static constexpr int OFF_V = OFF_K + kGroups * 3 * TK;        // [group][3]
-  static constexpr int OFF_M = OFF_V + kGroups * 3 * TK;        // [bias stage][group] x 64 mask terms
-  static constexpr int OFF_BAR = OFF_M + kBiasStages * kGroups * 256;
-  static constexpr int SMEM = OFF_BAR + 1024 + 1024;
 };
 
 // barriers of one group
@@ -85,11 +98,12 @@ __device__ __forceinline__ void ld_wait16(uint32_t (&v)[16]) {
 }
 
 template <typename T, bool HB>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(RowsCfg<T>::kThreads, 1)
 attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias, const RowsArgs a) {
-  using M = RowsSmem;
-  constexpr float kTooBig = ElemIsBf16<T>::value ? 1.152921504606847e18f : 32768.0f;   // 2^60; fp16 tops out at 2^16
+  using M = RowsCfg<T>;
+  constexpr int kGroups = M::kGroups, kBiasStages = M::kBiasStages;
+  constexpr float kTooBig = std::is_same<T, __half>::value ? 32768.0f : 1.152921504606847e18f;   // fp16 tops out at 2^16; 2^60
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   GroupBars* bars = reinterpret_cast<GroupBars*>(smem + M::OFF_BAR);
@@ -127,8 +141,10 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  dependent_trigger();   // (q, k, v are the caller's: only the mask terms and a copied bias come from the kernels before)
-  constexpr uint32_t COLS = 160, COL_O = 128;   // a group's columns: S / P of even and odd steps at 0 and 64, O
+  dependent_trigger();
+  if constexpr (M::F32) dependent_wait();   // (else q, k, v are the caller's: only mask terms and a copied bias come from before)
+  constexpr uint32_t COLS = M::F32 ? 224 : 160, COL_O = 128, COL_LO = 160;   // a group's columns: S / P of even and odd steps at
+                                                                             // 0 and 64, O, (fp32) what P's upper bits leave
   bool ok = true;
 
   if (warp == 5 * kGroups) {
@@ -147,6 +163,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int g = 0; g < rows; ++g)
             bulk_load(smem + M::OFF_M + (stg * kGroups + g) * 256, a.mask_terms + ((long long)it.b * a.S + it.s0 + g) * a.npad + j * 64, 256, &b_full[stg]);
           if (HB) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB, &tmBias, &b_full[stg], j * 64, it.q0, it.h, it.b * a.bias_b_mul);
+          if (HB && M::F32) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB + M::TB / 2, &tmBias, &b_full[stg], j * 64 + 32, it.q0, it.h, it.b * a.bias_b_mul);
           if (++stg == kBiasStages) { stg = 0; ph ^= 1; }
         }
       }
@@ -157,13 +174,12 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int g = warp - 4 * kGroups;
     if (g < R) {
       GroupBars& gb = bars[g];
-      uint8_t* sQ = smem + M::OFF_Q + g * 3 * M::TQ;
+      uint8_t* sQ = smem + M::OFF_Q + g * M::kQ * M::TQ;
       uint8_t* sK = smem + M::OFF_K + g * 3 * M::TK;
       uint8_t* sV = smem + M::OFF_V + g * 3 * M::TK;
       const uint32_t t0 = tmem_base + g * COLS;
       const bool leader = elect_one();
-      constexpr uint32_t HI = desc_hi(8 * 64, 4);   // 64-byte rows, SWIZZLE_64B
-      const uint32_t q_lo = desc_lo(smem_u32(sQ), 16), k_lo = desc_lo(smem_u32(sK), 16), v_lo = desc_lo(smem_u32(sV), 64 * 64);
+      const uint32_t q_lo = desc_lo(smem_u32(sQ), 16), k_lo = desc_lo(smem_u32(sK), 16), v_lo = desc_lo(smem_u32(sV), 64 * M::RB);
       int total = 0;                        // steps of this group: rows beyond S are left out
       for (int n = 0; n < my_items; ++n) total += item_of(n).s0 + g < a.S ? nk : 0;
       // a position in the group's stream: item, key step, ring stage, Q buffer
@@ -176,7 +192,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (++u.stg == 3) u.stg = 0;
         if (++u.j == nk) {
           u.j = 0;
-          if (++u.q == 3) u.q = 0;
+          if (++u.q == M::kQ) u.q = 0;
           if (u.left > 0) { u.it = item_of(++u.n); start(u); }
         }
       };
@@ -199,10 +215,10 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint32_t s_q = q_lo + sq * (M::TQ >> 4), s_k = k_lo + sk * (M::TK >> 4);
         if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-            umma<KIND_F16>(t, desc_join(s_q + ks * 2, HI), desc_join(s_k + ks * 2, HI), a.idesc_s, ks > 0);
+          for (int ks = 0; ks < M::KS; ++ks)
+            umma<M::kind>(t, desc_join(s_q + ks * 2, M::HI), desc_join(s_k + ks * 2, M::HI), a.idesc_s, ks > 0);
         }
-        if (++sj == nk) { sj = 0; if (++sq == 3) sq = 0; }
+        if (++sj == nk) { sj = 0; if (++sq == M::kQ) sq = 0; }
         if (++sk == 3) sk = 0;
       };
       for (int c = 0; c < 2 && c < total; ++c) load(&gb.first[c], true, false);
@@ -225,8 +241,12 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_after_sync();
         if (leader) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ts_f16(t0 + COL_O, tp + kk * 8, desc_join(v_at + kk * 64, HI), a.idesc_pv, kk > 0 ? 1u : first);
+          for (int kk = 0; kk < M::KV; ++kk)
+            umma_ts<M::kind>(t0 + COL_O, tp + kk * 8, desc_join(v_at + kk * 64, M::HI_V), a.idesc_pv, kk > 0 ? 1u : first);
+          if constexpr (M::F32) {
+#pragma unroll
+            for (int kk = 0; kk < M::KV; ++kk) umma_ts<M::kind>(t0 + COL_O, t0 + COL_LO + kk * 8, desc_join(v_at + kk * 64, M::HI_V), a.idesc_pv, 1u);
+          }
         }
         if (more) issue_s(tp);               // into the columns P V(c) reads: products of one thread run in order
         if (leader) umma_commit(&gb.mma[c & 1]);
@@ -252,7 +272,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // the row that is finished but for its last P V: statistics, where its results go
     bool pend = false;
     float pm = 0.f, pl = 0.f, pseen = 0.f;
-    int po = -1, pstat = 0;   // O row in units of 8 elements, -1 where the query is beyond N; row of the statistics
+    int po = -1, pstat = 0;   // O row in 16-byte pieces, -1 where the query is beyond N; row of the statistics
     // O and the statistics of the row, once P V of its last step `cl` is done; no later P V can have been issued yet
     auto finish = [&](int cl) {
       if (!mbar_wait(&gb.mma[cl & 1], ((cl >> 1) + 1) & 1, a.err, 59)) ok = false;
@@ -265,8 +285,12 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (po >= 0 && ok) {
         const float inv = 1.0f / pl;
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          if (h * 8 < a.D) {
+        for (int h = 0; h < 32 / M::kVec; ++h) {
+          if (h * M::kVec >= a.D) continue;
+          if constexpr (M::F32) {
+            auto f = [&](int i) { return __uint_as_float(o[h >> 2][(h & 3) * 4 + i]) * inv; };
+            (reinterpret_cast<float4*>(a.o) + po)[h] = make_float4(f(0), f(1), f(2), f(3));
+          } else {
             uint4 pk;
             auto f = [&](int i) { return __uint_as_float(o[h >> 1][(h & 1) * 8 + i]) * inv; };
             pk.x = pack2<T>(f(0), f(1)); pk.y = pack2<T>(f(2), f(3)); pk.z = pack2<T>(f(4), f(5)); pk.w = pack2<T>(f(6), f(7));
@@ -305,13 +329,21 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int u = 0; u < 2; ++u) {
             const float4 mA = lds128f(mrow + (q * 4 + u * 2) * 16), mB = lds128f(mrow + (q * 4 + u * 2 + 1) * 16);
             const float2 mk[4] = {make_float2(mA.x, mA.y), make_float2(mA.z, mA.w), make_float2(mB.x, mB.y), make_float2(mB.z, mB.w)};
-            uint4 raw = make_uint4(0, 0, 0, 0);
-            if constexpr (HB) raw = lds128(brow ^ ((q * 2 + u) << 4));   // (128-byte rows, 16-byte chunks swizzled by the row)
-            const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
+            // (bias: 128-byte rows, 16-byte chunks swizzled by the row; fp32: two tiles of 32 keys)
+            uint4 raw = make_uint4(0, 0, 0, 0), more = raw;
+            if constexpr (HB && M::F32) {
+              const uint32_t at = brow + (q >> 1) * (M::TB / 2), g = (q & 1) * 4 + u * 2;
+              raw = lds128(at ^ (g << 4));
+              more = lds128(at ^ ((g + 1) << 4));
+            } else if constexpr (HB) {
+              raw = lds128(brow ^ ((q * 2 + u) << 4));
+            }
+            const uint32_t bw[8] = {raw.x, raw.y, raw.z, raw.w, more.x, more.y, more.z, more.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
-              if constexpr (HB) v = __fadd2_rn(v, unpack2<T>(bw[i]));
+              if constexpr (HB && M::F32) v = __fadd2_rn(v, pair(bw[2 * i], bw[2 * i + 1]));
+              else if constexpr (HB) v = __fadd2_rn(v, unpack2<T>(bw[i]));
               x[u * 4 + i] = v;
             }
           }
@@ -326,12 +358,31 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             const float2 e = __ffma2_rn(x[i], l2e2, nm2);
             const float2 p = make_float2(ex2_approx(e.x), ex2_approx(e.y));
             sum = __fadd2_rn(sum, p);
-            w[i] = pack2<T>(p.x, p.y);
+            if constexpr (M::F32) {
+              w[2 * i] = __float_as_uint(p.x);
+              w[2 * i + 1] = __float_as_uint(p.y);
+            } else {
+              w[i] = pack2<T>(p.x, p.y);
+            }
           }
+        };
+        // fp32: sixteen P as their upper 19 bits, what a product reads of them, and the rest: P V is the sum of two products
+        auto store_split = [&](uint32_t t_s, const uint32_t* w, int q) {
+          uint32_t hi[16], lo[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            hi[2 * i] = w[2 * i] & 0xffffe000u;
+            hi[2 * i + 1] = w[2 * i + 1] & 0xffffe000u;
+            const float2 r = __fadd2_rn(pair(w[2 * i], w[2 * i + 1]), pair(hi[2 * i] ^ 0x80000000u, hi[2 * i + 1] ^ 0x80000000u));
+            lo[2 * i] = __float_as_uint(r.x);
+            lo[2 * i + 1] = __float_as_uint(r.y);
+          }
+          tmem_st_32x16(t_s + q * 16, hi);
+          tmem_st_32x16(t_row + COL_LO + q * 16, lo);
         };
         // P of this thread's 64 keys and their sum
         float2 ps = make_float2(0.f, 0.f);
-        uint32_t pw[32], ra[16], rb[16];
+        uint32_t pw[M::PC], ra[16], rb[16];
         auto chunk = [&](auto diff, uint32_t (&cur)[16], uint32_t (&nxt)[16], int q) {   // sixteen keys; the next sixteen on their way
           ld_wait16(cur);
           if (q < 3) tmem_ld_32x16(t_s + (q + 1) * 16, nxt);
@@ -339,10 +390,10 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           logits(cur, q, x);
           if constexpr (diff.value) {
             subtract(x, m);
-            exps(x, splat(factor(m)), pw + q * 8, ps);
+            exps(x, splat(factor(m)), pw + q * (M::PC / 4), ps);
           } else {
             if (q == 0) m = j > 0 ? m : fmaxf(fmaxf(x[0].x, x[0].y), fmaxf(x[1].x, x[1].y));
-            exps(x, splat(-(m * kLog2e)), pw + q * 8, ps);
+            exps(x, splat(-(m * kLog2e)), pw + q * (M::PC / 4), ps);
           }
         };
         auto sweep = [&](auto diff) {
@@ -357,10 +408,22 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // whether the next step's S and bias tile are there: asked now, needed at the top
         early_s = mbar_test(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1);
         early_b = mbar_test(&b_full[bstg + 1 == kBiasStages ? 0 : bstg + 1], bstg + 1 == kBiasStages ? bph ^ 1 : bph);
+        // (fp32: the rest of P has one buffer, and P V of the step before reads it; its commit is the next step's S)
+        if (M::F32 && c > 0 && !early_s) {
+          early_s = mbar_wait(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1, a.err, 58);
+          ok = early_s && ok;
+          tc_fence_after_sync();
+        }
         float sum = ps.x + ps.y;
         const bool redo = __any_sync(0xffffffffu, !(sum < kTooBig) || (j == 0 && large(m)));
         if (!redo) {
-          tmem_st_32x32(t_s, pw);   // over the S values this warp has read: 64 keys as 32 packed columns
+          // over the S values this warp has read: 64 keys as 32 packed columns, or 64
+          if constexpr (M::F32) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) store_split(t_s, pw + q * 16, q);
+          } else {
+            tmem_st_32x32(t_s, pw);
+          }
         } else {
           // Some row of the warp outgrew its reference, or starts from a large one: take the maximum of the step, scale the sum and O by
           // 2^((m - m_new) log2e) and the quotient of the factors (once P V of the step before is done), and form P again.
@@ -396,13 +459,14 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll 1
           for (int q = 0; q < 4; ++q) {
             float2 x[8];
-            uint32_t w[8];
+            uint32_t w[M::PC / 4];
             tmem_ld_32x16(t_s + q * 16, ra);
             ld_wait16(ra);
             logits(ra, q, x);
             subtract(x, m);
             exps(x, splat(fac), w, ps);
-            tmem_st_32x8(t_s + q * 8, w);
+            if constexpr (M::F32) store_split(t_s, w, q);
+            else tmem_st_32x8(t_s + q * 8, w);
           }
           sum = ps.x + ps.y;
         }
@@ -422,7 +486,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       pend = true; pm = m; pl = l; pseen = seen;
       const int qi = it.q0 + r, s = it.s0 + g;
-      po = qi < a.N ? (int)((it.b * a.o_st[0] + s * a.o_st[1] + qi * a.o_st[2] + it.h * a.o_st[3]) >> 3) : -1;
+      po = qi < a.N ? (int)((it.b * a.o_st[0] + s * a.o_st[1] + qi * a.o_st[2] + it.h * a.o_st[3]) / M::kVec) : -1;
       pstat = ((it.b * a.S + s) * a.H + it.h) * a.N + qi;
     }
     if (pend && ok) finish(c - 1);
@@ -438,16 +502,13 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }  // namespace
 
 bool attn_fwd_rows_fits(const TriAttnDesc* d) {
+  const int vec = d->dtype == TRI_F32 ? 4 : 8;
   const int64_t last = (d->B - 1) * d->o_st[0] + (d->n_seq - 1) * d->o_st[1] + (d->n_res - 1) * d->o_st[2] + (d->H - 1) * d->o_st[3];
-  return (int64_t)d->B * d->n_seq * d->H * d->n_res < (int64_t)1 << 31 && last / 8 < ((int64_t)1 << 31) - 8;
+  return (int64_t)d->B * d->n_seq * d->H * d->n_res < (int64_t)1 << 31 && last / vec < ((int64_t)1 << 31) - 8;
 }
 
-int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void* v, const CUtensorMap* tbias,
+int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap* tbias,
                   bool bias_batched, void* o, float* stats, const float* mask_terms, int* err, cudaStream_t st) {
-  CUtensorMap tq, tk, tv;
-  TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, 32));
-  TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, 32));
-  TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, 32));
   RowsArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D;
   a.scale = d->scale;
@@ -456,25 +517,29 @@ int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void
   a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
   a.bias_b_mul = bias_batched ? 1 : 0;
   a.err = err;
-  const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
+  const int kind = d->dtype == TRI_F32 ? KIND_TF32 : d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   a.idesc_s = make_idesc(kind, 128, 64, false, false);
   a.idesc_pv = make_idesc(kind, 128, 32, false, true);
   const long long combos = (long long)((d->n_res + 127) / 128) * d->H * d->B;
-  int rows = kGroups;
+  int rows = d->dtype == TRI_F32 ? RowsCfg<float>::kGroups : RowsCfg<__half>::kGroups;
   while (rows > 1 && combos * cdiv(d->n_seq, rows) < sm_count()) --rows;   // fewer rows per CTA before an SM stays idle
   a.rows_per_item = rows;
   const long long items = combos * cdiv(d->n_seq, rows);
   const double pairs = (double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res;
-  KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
-  auto launch = [&](auto kern, const CUtensorMap& tb) {
-    TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem::SMEM));
-    launch_dependent(kern, (unsigned)std::min<long long>(items, sm_count()), kThreads, RowsSmem::SMEM, st, tq, tk, tv, tb, a);
+  KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, (double)dtype_size(d->dtype) * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
+  auto launch = [&](auto elem, auto kern, const CUtensorMap& tb) {
+    using M = RowsCfg<decltype(elem)>;
+    TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::SMEM));
+    launch_dependent(kern, (unsigned)std::min<long long>(items, sm_count()), M::kThreads, M::SMEM, st, tq, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     return 0;
   };
-  if (d->dtype == TRI_BF16)
-    return tbias ? launch(attn_fwd_rows_kernel<__nv_bfloat16, true>, *tbias) : launch(attn_fwd_rows_kernel<__nv_bfloat16, false>, tq);
-  return tbias ? launch(attn_fwd_rows_kernel<__half, true>, *tbias) : launch(attn_fwd_rows_kernel<__half, false>, tq);
+  auto start = [&](auto elem) {
+    using T = decltype(elem);
+    return tbias ? launch(elem, attn_fwd_rows_kernel<T, true>, *tbias) : launch(elem, attn_fwd_rows_kernel<T, false>, tq);
+  };
+  if (d->dtype == TRI_F32) return start(float());
+  return d->dtype == TRI_BF16 ? start(__nv_bfloat16()) : start(__half());
 }
 
 }  // namespace tc

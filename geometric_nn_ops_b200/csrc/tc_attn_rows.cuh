@@ -10,11 +10,12 @@ namespace tc {
 // `width` channels (32 or 64), zero beyond D
 int qkv_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, const int64_t* st, int rows, int width);
 
-// its offsets are 32-bit: rows of statistics, and O in units of 8 elements
+// its offsets are 32-bit: rows of statistics, and O in 16-byte pieces
 bool attn_fwd_rows_fits(const TriAttnDesc* d);
-// tbias: map over the bias with boxes of 128 queries x 64 keys, or null.  mask_terms: [B][S][npad] additive key-mask
+// Boxes: tq 128 queries, tk and tv 64 keys of 32 channels; fp32: operands rounded to TF32, tv in the swizzle with 32-byte atoms,
+// more than 64 residues.  tbias: 128 queries x 64 keys (fp32: x 32), or null.  mask_terms: [B][S][npad] additive key-mask
 // terms (0, -1e9, -inf beyond N).
-int attn_fwd_rows(const TriAttnDesc* d, const void* q, const void* k, const void* v, const CUtensorMap* tbias,
+int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap* tbias,
                   bool bias_batched, void* o, float* stats, const float* mask_terms, int* err, cudaStream_t st);
 
 }  // namespace tc
