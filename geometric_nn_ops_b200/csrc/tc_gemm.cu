@@ -118,6 +118,10 @@ static int launch_in(cudaStream_t st, int epi, int bn, bool out_f32, const CUten
     if (bn == 256) return launch_t<TIN, TIN, 256, EPI_STORE>(st, maps, g, p);
     return launch_t<TIN, TIN, 128, EPI_STORE>(st, maps, g, p);
   }
+  if (epi == EPI_GATE_MUL) {
+    if constexpr (sizeof(TIN) == 2) return launch_t<TIN, TIN, 128, EPI_GATE_MUL>(st, maps, g, p);
+    return fail(TRI_ERR_ARG, "the gated product is for 16-bit types");
+  }
   if (bn != 256) return fail(TRI_ERR_ARG, "gate epilogues need 256-column tiles");
   if (epi == EPI_GATE_IN) return launch_t<TIN, TIN, 256, EPI_GATE_IN>(st, maps, g, p);
   if (epi == EPI_GATE_OUT) return launch_t<TIN, TIN, 256, EPI_GATE_OUT>(st, maps, g, p);

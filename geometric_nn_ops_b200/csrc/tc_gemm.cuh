@@ -31,9 +31,10 @@ enum Epilogue {
                          //   half-plane[c][px] = (P+bp)*sigmoid(G+bg)*mask[px]
   EPI_GATE_OUT = 2,      // rows = pixels, cols [y(128) | g(128)]: out0[m][c] = (y+b)*sigmoid(g+b)
   EPI_GATE_OUT_BWD = 3,  // same cols, aux = d_out: out0 = d_out*sig, out1 = d_out*(y+b)*sig*(1-sig)
-  EPI_GATE_IN_BWD = 4    // transposed like GATE_IN; aux2/aux3 = channel-major d(a), d(b); aux = mask;
+  EPI_GATE_IN_BWD = 4,   // transposed like GATE_IN; aux2/aux3 = channel-major d(a), d(b); aux = mask;
                          //   d = d(half)[c][px]*mask;  out0 is channel-major [512][M]:
                          //   row half*256+c = d*sig(G),  row half*256+128+c = d*P*sig*(1-sig)
+  EPI_GATE_MUL = 5       // out0[m][n] = aux[m][n] * sigmoid(acc); aux alone comes from the kernels before
 };
 
 constexpr int kBM = 128;
@@ -41,7 +42,7 @@ constexpr int kStageA = kBM * 128;  // bytes
 // warp 0 producer, warp 1 MMA, then the epilogue warps: 16 for the gate epilogues, whose per-element arithmetic (sigmoid,
 // products) is latency-bound with fewer warps per scheduler, 8 for the plain store.  (Gate-in backward on 8 warps with the
 // gradients fetched a tile ahead into registers: 0.381 ms per launch at 768 x 768 pixels against 0.365.)
-constexpr int gemm_epi_warps(int epi) { return epi == 0 ? 8 : 16; }
+constexpr int gemm_epi_warps(int epi) { return epi == EPI_STORE || epi == EPI_GATE_MUL ? 8 : 16; }
 constexpr int gemm_threads(int epi) { return 64 + 32 * gemm_epi_warps(epi); }
 
 struct GemmArgs {
@@ -343,7 +344,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  dependent_enter();
+  if constexpr (EPI == EPI_GATE_MUL) dependent_trigger();   // (the epilogue waits)
+  else dependent_enter();
 
   const int total = g.batches * g.tiles_m * g.tiles_n;
   const int kb_total = g.kblocks0 + g.kblocks1;
@@ -439,6 +441,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     const int row = quarter * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
+    if constexpr (EPI == EPI_GATE_MUL) dependent_wait();
     // The backward gate epilogues read a gradient tile from global memory, just before they wait for the product.
     constexpr bool kGradTile = EPI == EPI_GATE_IN_BWD || EPI == EPI_GATE_OUT_BWD;
     auto fetch_grad = [&](int t, Raw8<TIN> (&dst)[CPG][4]) {
@@ -500,7 +503,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       if (!mbar_wait(&tfull[acc], acc_phase, g.err, 4)) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      if constexpr (EPI == EPI_STORE) {
+      if constexpr (EPI == EPI_STORE || EPI == EPI_GATE_MUL) {
         const int m = tm * kBM + row, n0 = tn * BN;
         TOUT* out = reinterpret_cast<TOUT*>(g.out0) + bz * g.batch_out + (long long)m * g.ld_out;
         const bool vec_ok = (g.ld_out * sizeof(TOUT)) % 16 == 0 && (g.batch_out * sizeof(TOUT)) % 16 == 0 && (reinterpret_cast<uintptr_t>(g.out0) & 15) == 0;
@@ -514,6 +517,21 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           if (g.bias0 != nullptr) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) if (n + i < g.N) v[i] += g.bias0[n + i];
+          }
+          if constexpr (EPI == EPI_GATE_MUL) {   // (N is a multiple of eight)
+            const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const TIN*>(g.aux) + (long long)m * g.ld_out + n);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (m >= g.M || n + u * 8 >= g.N) continue;
+              const uint4 x = src[u];
+              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 r = __fmul2_rn(unpack2<TIN>(w[i]), sigmoid2(make_float2(v[u * 8 + 2 * i], v[u * 8 + 2 * i + 1])));
+                v[u * 8 + 2 * i] = r.x;
+                v[u * 8 + 2 * i + 1] = r.y;
+              }
+            }
           }
           if ((g.M & 3) == 0 && vec_ok && g.N - n >= 32) store_rows32<TOUT>(out + n, v, g.ld_out, m < g.M, lane);
           else if (m < g.M && n < g.N) store_row32<TOUT>(out + n, v, g.N - n, vec_ok);

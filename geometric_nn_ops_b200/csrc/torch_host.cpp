@@ -41,6 +41,7 @@ struct Api {
   decltype(&tri_attn_bwd) attn_bwd;
   decltype(&tri_attn_project_bias) attn_project_bias;
   decltype(&tri_gate_mul) gate_mul;
+  decltype(&tri_gated_linear) gated_linear;
   decltype(&tri_mul_saved_bytes) mul_saved_bytes;
   decltype(&tri_mul_ws_bytes) mul_ws_bytes;
   decltype(&tri_mul_fwd) mul_fwd;
@@ -58,7 +59,7 @@ void bind(const std::string& path) {
   get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
   get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
   get(api.mul_fwd_residual, "tri_mul_fwd_residual");
-  get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul");
+  get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul"); get(api.gated_linear, "tri_gated_linear");
   get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
   get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
 }
@@ -471,7 +472,8 @@ bool pair_bias_fits(const Tensor& z, const OptTensor& ln_w, const Tensor& w) {
   const Tensor lw = or_undefined(ln_w);
   return fits && !wants_grad({&z, &w, &lw}) && z.numel() >= 128 && z.numel() / 128 < (1LL << 31) - 128 && !at::autocast::is_autocast_enabled(at::kCUDA);
 }
-Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
+// (`status`: the kernel's workspace, whose first word later kernels on the stream may report to; undefined where torch ran)
+Tensor pair_bias_of(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps, Tensor* status) {
   if (!pair_bias_fits(z, ln_w, w))
     return at::linear(at::layer_norm(z, {z.size(-1)}, ln_w, {}, eps), w).permute({0, 3, 1, 2}).contiguous();
   TriAttnProjDesc d{};
@@ -482,7 +484,23 @@ Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double
   const tri_stream_t st = stream_of(z);
   ok(api.attn_project_bias(&d, z.size(1) * z.size(2), ptr(zc), ptr(lw), nullptr, ptr(wc), ptr(out), ptr(ws), st), "tri_attn_project_bias");
   check_device(ws, reinterpret_cast<cudaStream_t>(st));
+  *status = ws;
   return out;
+}
+Tensor pair_bias(const Tensor& z, const OptTensor& ln_w, const Tensor& w, double eps) {
+  Tensor status;
+  return pair_bias_of(z, ln_w, w, eps, &status);
+}
+
+// Whether (o * sigmoid(s g_w^T)) o_w^T can run as two products of this package: dense operands of one 16-bit type, no biases.
+bool gated_linear_fits(const Tensor& s, const Tensor& o, const Tensor& g_w, const Tensor& o_w) {
+  const auto dt = s.scalar_type();
+  if ((dt != at::kBFloat16 && dt != at::kHalf) || s.numel() == 0 || g_w.size(1) != s.size(-1) || g_w.size(0) != o.size(-1) ||
+      o_w.size(1) != o.size(-1) || s.numel() / s.size(-1) != o.numel() / o.size(-1) || s.numel() / s.size(-1) >= (1LL << 31) - 128)
+    return false;
+  for (const Tensor* t : {&s, &o, &g_w, &o_w})
+    if (t->scalar_type() != dt || t->device() != s.device() || !t->is_contiguous() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) return false;
+  return g_w.size(1) % 8 == 0 && g_w.size(0) % 8 == 0 && o_w.size(0) % 8 == 0 && o_w.size(0) > 0;
 }
 
 // o * sigmoid(gate)
@@ -505,7 +523,8 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
   const Tensor gb = or_undefined(g_b), ob = or_undefined(o_b), zw = or_undefined(z_w), lw = or_undefined(ln_w);
   const bool grad = wants_grad({&s, &q, &k, &v, &z, &g_w, &o_w, &gb, &ob, &zw, &lw});
   const NoRecord fast(!grad);
-  const Tensor pz = z_w.has_value() ? pair_bias(z, ln_w, *z_w, eps) : z;
+  Tensor status;
+  const Tensor pz = z_w.has_value() ? pair_bias_of(z, ln_w, *z_w, eps, &status) : z;
   // (BM, H, U, D) -> rows = multiplicity: [B, M, U, H, D] as a strided view (no copy)
   auto rows = [&](const Tensor& t) { return inner_contiguous(t.reshape({B, M, H, U, D}).transpose(2, 3)); };
   Tensor mask;
@@ -514,6 +533,16 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
   const Tensor o = attn_any(rows(q), rows(k), rows(v), bias, mask, scale, precision, true).first.reshape({BM, U, H * D}).to(s.scalar_type());
   if (grad || s.dim() != 3 || !s.is_contiguous() || g_w.dim() != 2 || o_w.dim() != 2)
     return {at::linear(gated(o, at::linear(s, g_w, g_b)), o_w, o_b), pz};
+  if (status.defined() && !g_b.has_value() && !o_b.has_value() && gated_linear_fits(s, o, g_w, o_w)) {
+    const c10::cuda::CUDAGuard guard(s.device());
+    const int64_t W = H * D, N = o_w.size(0);
+    const Tensor gated = at::empty({BM, U, W}, s.options()), out = at::empty({BM, U, N}, s.options());
+    const tri_stream_t st = stream_of(s);
+    ok(api.gated_linear(dtype_code(s), BM * U, (int32_t)s.size(2), (int32_t)W, (int32_t)N, ptr(s), ptr(g_w), ptr(o), ptr(o_w), ptr(gated), ptr(out),
+                        ptr(status), st), "tri_gated_linear");
+    check_device(status, reinterpret_cast<cudaStream_t>(st));
+    return {out, pz};
+  }
   // the same products on two dimensions
   auto linear = [](const Tensor& x, const Tensor& w, const OptTensor& b) { return b.has_value() ? at::addmm(*b, x, w.t()) : at::mm(x, w.t()); };
   const Tensor gate = linear(s.view({-1, s.size(2)}), g_w, g_b);

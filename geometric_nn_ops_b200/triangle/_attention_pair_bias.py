@@ -11,8 +11,8 @@ Viewed as triangle attention, a batch entry is ``B``, the multiplicity ``M`` (th
 share a batch entry) is the row axis, and the per-head bias ``(B, H, U, V)`` is the pair bias shared by all
 rows.  Every other case (cross attention with U != V, an explicit ``inf`` other than the dtype's sentinel, CPU
 tensors, fp64) is evaluated with the same torch operations the reference uses, on whatever device the tensors
-live.  Around the core, the gate and output projections are torch linears; the LayerNorm and projection of ``z``
-and the gating are kernels of this package where no gradient is recorded and they have the shape.
+live.  Around the core, where no gradient is recorded and they have the shape, the LayerNorm and projection of
+``z`` and the two products with the gate (16-bit types, no biases) are kernels of this package; else they are torch's.
 """
 
 import torch

@@ -153,6 +153,12 @@ int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z
 /* out[i] = a[i] * sigmoid(gate[i]), i < n, in `dtype` (fp32 arithmetic). */
 int tri_gate_mul(int dtype, int64_t n, const void* a, const void* gate, void* out, tri_stream_t stream);
 
+/* out[M][N] = (o * sigmoid(s w_gate^T)) w_out^T for a 16-bit type: s [M][K], w_gate [W][K], o and the scratch tensor `gated`
+ * [M][W], w_out [N][W], all contiguous and 16-byte aligned; K, W and N multiples of eight.  `status` is the first word of a
+ * workspace whose call (the one that wrote o, say) came before on this stream; a timeout is reported there. */
+int tri_gated_linear(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
+                     const void* w_out, void* gated, void* out, void* status, tri_stream_t stream);
+
 /* ------------------------------------------------------------------------ */
 /* Triangle multiplicative update                                           */
 /* ------------------------------------------------------------------------ */
