@@ -5,7 +5,7 @@
 // accesses and warp-shuffle reductions.  Intermediates are stored in the input dtype.
 //
 // Data layout in HBM (M = B*N*N pixels, NN = N*N):
-//   z, u, dy, dgo, du, dz   pixel-major   [M, 128]
+//   z, u, dy, dgo, du       pixel-major   [M, 128]
 //   dPG                     channel-major [512, M], rows [dP_a | dG_a | dP_b | dG_b]
 //   a, b, t, dt, da, db     channel-major [B, 128, N, N]: one N x N plane per channel, so the per-channel
 //                           contraction is a plain batched GEMM and both directions (and all four
@@ -15,7 +15,7 @@
 //           -> GEMM[u Wo^T | z Wgo^T, gate-out epilogue -> out]
 // backward: GEMM[gate-out bwd epilogue -> dy,dgo] -> split-K GEMMs dWo,dWgo -> GEMM du -> ln_cm_bwd -> dt
 //           -> 2 contraction GEMMs -> GEMM[z Wcat^T | gate-in bwd epilogue -> dPG] -> split-K GEMM dWcat
-//           -> GEMM[dPG Wcat + dgo Wgo -> dz] -> ln_rows_bwd -> dx
+//           -> GEMM[dPG Wcat + dgo Wgo -> dz, LayerNorm backward -> dx]
 // Math follows trimul_torch (geometric_nn_ops_torch/triangle/_reference/trimul.py:57-97).
 #include <algorithm>
 #include <cstdlib>
@@ -165,67 +165,6 @@ __global__ void __launch_bounds__(256) ln_rows_kernel(const T* __restrict__ x, c
       store8v(z + row * CW + sub * 8, v[p]);
       if (sub == 0) { mean[row] = mu; rstd[row] = rs; }
     }
-  }
-}
-
-// dx = rstd * (dhat - mean(dhat) - xhat * mean(dhat*xhat)); per-block partial dgamma / dbeta
-template <typename T>
-__global__ void __launch_bounds__(256, 4) ln_rows_bwd_kernel(const T* __restrict__ dz, const T* __restrict__ x,
-                                                           const float* __restrict__ mean, const float* __restrict__ rstd,
-                                                           const T* gamma, long long M, T* __restrict__ dx, float* pg,
-                                                           float* pb) {
-  __shared__ float sg[16][CW], sb[16][CW];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 15, half = lane >> 4;
-  constexpr int RP = 1;   // row pairs per warp and pass (more would cost the registers of a fourth resident block)
-  float gm[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) gm[i] = 1.f;
-  if (gamma) load8v(gamma + sub * 8, gm);
-  float ag[8] = {}, ab[8] = {};
-  for (long long base = (blockIdx.x * 8LL + warp) * (2 * RP); base < M; base += gridDim.x * 8LL * (2 * RP)) {
-    float xv[RP][8], dv[RP][8], mu[RP], rs[RP];
-#pragma unroll
-    for (int p = 0; p < RP; ++p) {
-      const long long row = base + 2 * p + half;
-      if (row < M) {
-        load8v(x + row * CW + sub * 8, xv[p]);
-        load8v(dz + row * CW + sub * 8, dv[p]);
-        mu[p] = mean[row]; rs[p] = rstd[row];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { xv[p][i] = 0.f; dv[p][i] = 0.f; }
-        mu[p] = 0.f; rs[p] = 0.f;
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < RP; ++p) {
-      const long long row = base + 2 * p + half;
-      float s1 = 0.f, s2 = 0.f, dh[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        xv[p][i] = (xv[p][i] - mu[p]) * rs[p];
-        dh[i] = dv[p][i] * gm[i];
-        s1 += dh[i];
-        s2 += dh[i] * xv[p][i];
-        ag[i] += dv[p][i] * xv[p][i];
-        ab[i] += dv[p][i];
-      }
-      s1 = half_warp_sum(s1) * (1.0f / CW);
-      s2 = half_warp_sum(s2) * (1.0f / CW);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) dh[i] = rs[p] * (dh[i] - s1 - xv[p][i] * s2);
-      if (row < M) store8v(dx + row * CW + sub * 8, dh);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { sg[warp * 2 + half][sub * 8 + i] = ag[i]; sb[warp * 2 + half][sub * 8 + i] = ab[i]; }
-  __syncthreads();
-  if (threadIdx.x < CW) {
-    float g = 0.f, b = 0.f;
-#pragma unroll
-    for (int w = 0; w < 16; ++w) { g += sg[w][threadIdx.x]; b += sb[w][threadIdx.x]; }
-    pg[blockIdx.x * CW + threadIdx.x] = g;
-    pb[blockIdx.x * CW + threadIdx.x] = b;
   }
 }
 
@@ -946,8 +885,11 @@ template <typename T>
 int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void* mask, const void* z,
                       const void* da_cm, const void* db_cm, const void* dgo, const float* mean_in,
                       const float* rstd_in, const TriMulWeights* w, const Prep& pr, const TriMulWeightGrads* g,
-                      void* dpg, void* dz, void* dx, float* partial) {
+                      void* dpg, void* dx, float* partial) {
   const long long M = gm.M;
+  const int blocks = std::min(cdiv(M, 128), sm_count());
+  float* pg = partial + kWgradPartialFloats;
+  float* pb = pg + (size_t)kPersist * CW;
   int nparts = 0;
   if (gate_in_bwd_supported(gm.dtype, M, gm.plane) && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) {
     GateInBwd f;
@@ -970,25 +912,16 @@ int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void
     TRI_LAUNCH_OK();
   }
   {
-    GemmPlan p;   // dz = dPG Wcat + dgo Wgo
+    GemmPlan p;   // dz = dPG Wcat + dgo Wgo, and from it dx (LayerNorm's backward) in the epilogue
     p.a[0] = rows_operand(dpg, 4 * CW, M, false);
     p.a[0].mn_major = true; p.a[0].inner = M; p.a[0].outer = 4 * CW; p.a[0].st_outer = M;   // A(m = pixel, k = row of dPG): m contiguous
     p.b[0] = rows_operand(pr.wcat, CW, 4 * CW, true);   // B(n = c, k = row of Wcat): n contiguous
     p.a[1] = rows_operand(dgo, CW, M, false);
     p.b[1] = rows_operand(w->g_out_w, CW, CW, true);
     p.M = (int)M; p.N = CW; p.K0 = 4 * CW; p.K1 = CW; p.seg1_col = 0;
-    p.out0 = dz; p.ld_out = CW;
-    p.name = "tc_gemm_dz"; p.flops = 2.0 * M * CW * 5 * CW; p.bytes = 6.0 * gm.unit();
-    TRI_TRY(launch_gemm(st, gm.dtype, EPI_STORE, 128, false, p, pr.err));
-  }
-  const int blocks = (int)std::min<long long>(kPersist, (M + 7) / 8);
-  float* pg = partial + kWgradPartialFloats;
-  float* pb = pg + (size_t)kPersist * CW;
-  {
-    KernelTimer kt("tc_ln_rows_bwd", st, 0.0, 3.0 * gm.unit());
-    ln_rows_bwd_kernel<T><<<blocks, 256, 0, st>>>((const T*)dz, (const T*)x, mean_in, rstd_in, (const T*)w->norm_in_w,
-                                                  M, (T*)dx, pg, pb);
-    TRI_LAUNCH_OK();
+    p.out0 = dx; p.x = x; p.gamma = w->norm_in_w; p.mean = mean_in; p.rstd = rstd_in; p.sum_g = pg; p.sum_b = pb;
+    p.name = "tc_gemm_dx"; p.flops = 2.0 * M * CW * 5 * CW; p.bytes = 7.0 * gm.unit();
+    TRI_TRY(launch_gemm(st, gm.dtype, EPI_LN_BWD, 128, false, p, pr.err));
   }
   return reduce_many(st, {{partial, nparts, 4 * CW * CW, g->p_in_w, g->g_in_w, CW},
                           {pg, blocks, CW, g->norm_in_w}, {pb, blocks, CW, g->norm_in_b}});
@@ -1014,12 +947,12 @@ void carve_saved(Arena& a, const Geom& gm, SavedT* s) {
   s->mean_out = a.take<float>(M); s->rstd_out = a.take<float>(M);
 }
 
-struct BwdBufs { void *dy, *dgo, *du, *dt, *da, *db, *dpg, *dz; float* partial; };
+struct BwdBufs { void *dy, *dgo, *du, *dt, *da, *db, *dpg; float* partial; };
 void carve_bwd(Arena& a, const Geom& gm, BwdBufs* w) {
   const size_t unit = (size_t)gm.M * CW * gm.es();
   w->dy = a.take<char>(unit); w->dgo = a.take<char>(unit); w->du = a.take<char>(unit);
   w->dt = a.take<char>(unit); w->da = a.take<char>(unit); w->db = a.take<char>(unit);
-  w->dpg = a.take<char>(4 * unit); w->dz = a.take<char>(unit);
+  w->dpg = a.take<char>(4 * unit);
   w->partial = a.take<float>(partial_floats());
 }
 
@@ -1067,7 +1000,7 @@ int backward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMu
     TRI_TRY(contraction(st, dt, planes, n, s.b, false, b.dt, false, b.da, pr.err, "tc_gemm_contract_bwd")); // da[k,i] = sum_j b[k,j] dt[i,j]
     TRI_TRY(contraction(st, dt, planes, n, s.a, false, b.dt, true, b.db, pr.err, "tc_gemm_contract_bwd"));  // db[k,j] = sum_i a[k,i] dt[i,j]
   }
-  return phase_project_bwd<T>(st, gm, x, mask, s.z, b.da, b.db, b.dgo, s.mean_in, s.rstd_in, w, pr, g, b.dpg, b.dz, dx,
+  return phase_project_bwd<T>(st, gm, x, mask, s.z, b.da, b.db, b.dgo, s.mean_in, s.rstd_in, w, pr, g, b.dpg, dx,
                               b.partial);
 }
 
@@ -1091,12 +1024,12 @@ void carve_shard_saved(Arena& a, const Geom& gm, ShardSaved* s) {
   s->mean_out = a.take<float>(M); s->rstd_out = a.take<float>(M);
 }
 
-struct ShardWs { void *dy, *du, *dpg, *dz; float* partial; };
+struct ShardWs { void *dy, *du, *dpg; float* partial; };
 void carve_shard_ws(Arena& a, const Geom& gm, int phase, ShardWs* w) {
   const size_t unit = (size_t)gm.M * CW * gm.es();
   *w = ShardWs{};
   if (phase == TRI_PHASE_OUTPUT_BWD) { w->dy = a.take<char>(unit); w->du = a.take<char>(unit); }
-  if (phase == TRI_PHASE_PROJECT_BWD) { w->dpg = a.take<char>(4 * unit); w->dz = a.take<char>(unit); }
+  if (phase == TRI_PHASE_PROJECT_BWD) w->dpg = a.take<char>(4 * unit);
   if (phase >= TRI_PHASE_OUTPUT_BWD) w->partial = a.take<float>(partial_floats());
 }
 
@@ -1133,7 +1066,7 @@ int shard_phase_t(const TriMulShardDesc* d, int phase, const TriMulShardBufs* bf
     case TRI_PHASE_PROJECT_BWD:
       if (!bf->x || !bf->a_cm || !bf->b_cm || !bf->dx || !bf->g) return fail(TRI_ERR_ARG, "project backward needs x, a_cm, b_cm (gradients), dx, g");
       return phase_project_bwd<T>(st, gm, bf->x, bf->mask, s.z, bf->a_cm, bf->b_cm, s.dgo, s.mean_in, s.rstd_in, bf->w,
-                                  pr, bf->g, sw.dpg, sw.dz, bf->dx, sw.partial);
+                                  pr, bf->g, sw.dpg, bf->dx, sw.partial);
   }
   return fail(TRI_ERR_ARG, "bad phase %d", phase);
 }
