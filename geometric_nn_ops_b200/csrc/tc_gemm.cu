@@ -94,7 +94,7 @@ static int operand_map(CUtensorMap* out, const Operand& o, int dtype, int rows_b
 template <typename TIN, typename TOUT, int BN, int EPI>
 static int launch_t(cudaStream_t st, const CUtensorMap* maps, const GemmArgs& g, const GemmPlan& p) {
   constexpr int STAGES = gemm_stages(EPI, BN, sizeof(TIN));
-  constexpr size_t smem = 1024 + (size_t)STAGES * (kStageA + BN * 128) + gemm_extra(EPI, sizeof(TIN)) + (2 * STAGES + 6) * 8 + 16;
+  constexpr size_t smem = 1024 + (size_t)STAGES * (kStageA + BN * 128) + gemm_extra(EPI, sizeof(TIN)) + (2 * STAGES + 8) * 8 + 16;
   auto kern = tc_gemm_kernel<TIN, TOUT, BN, EPI, STAGES>;
   // The opt-in to more than 48 KB of dynamic shared memory is a per-device attribute: set it on every launch
   // (a host-side call of about a microsecond) instead of remembering it process-wide.
@@ -123,6 +123,7 @@ static int launch_in(cudaStream_t st, int epi, int bn, bool out_f32, const CUten
     return fail(TRI_ERR_ARG, "the gated product is for 16-bit types");
   }
   if (epi == EPI_LN_BWD) return launch_t<TIN, TIN, 128, EPI_LN_BWD>(st, maps, g, p);
+  if (epi == EPI_LN_BWD_T) return launch_t<TIN, TIN, 128, EPI_LN_BWD_T>(st, maps, g, p);
   if (bn != 256) return fail(TRI_ERR_ARG, "gate epilogues need 256-column tiles");
   if (epi == EPI_GATE_IN) return launch_t<TIN, TIN, 256, EPI_GATE_IN>(st, maps, g, p);
   if (epi == EPI_GATE_OUT) return launch_t<TIN, TIN, 256, EPI_GATE_OUT>(st, maps, g, p);
@@ -158,9 +159,10 @@ int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const
   }
   g.out0 = p.out0; g.out1 = p.out1; g.ld_out = p.ld_out; g.batch_out = p.batch_out;
   g.bias0 = p.bias0; g.aux = p.aux; g.aux2 = p.aux2; g.aux3 = p.aux3; g.plane = p.plane; g.err = err;
-  if (epi == EPI_LN_BWD) {
-    if (p.N != 128 || bn != 128) return fail(TRI_ERR_ARG, "the LayerNorm epilogue needs rows of 128 channels");
-    const uint64_t dims[3] = {128, (uint64_t)p.M, 1}, str[2] = {128, 128 * (uint64_t)p.M};
+  if (epi_is_ln(epi)) {
+    const bool rows = epi == EPI_LN_BWD;
+    if ((rows ? p.N : p.M) != 128 || bn != 128 || p.N % 4 != 0) return fail(TRI_ERR_ARG, "the LayerNorm epilogues need 128 channels");
+    const uint64_t inner = rows ? 128 : p.N, outer = rows ? p.M : 128, dims[3] = {inner, outer, 1}, str[2] = {inner, inner * outer};
     const uint32_t box[3] = {128u / es, kBM, 1};
     TRI_TRY(make_tmap(&g.tmX, p.x, dtype, 3, dims, str, box, 128));
     TRI_TRY(make_tmap(&g.tmDx, p.out0, dtype, 3, dims, str, box, 128));

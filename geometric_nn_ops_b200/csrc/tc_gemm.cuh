@@ -35,9 +35,11 @@ enum Epilogue {
                          //   d = d(half)[c][px]*mask;  out0 is channel-major [512][M]:
                          //   row half*256+c = d*sig(G),  row half*256+128+c = d*P*sig*(1-sig)
   EPI_GATE_MUL = 5,      // out0[m][n] = aux[m][n] * sigmoid(acc); aux alone comes from the kernels before
-  EPI_LN_BWD = 6         // rows of 128 channels: acc = d(LayerNorm(x)); dx = rstd (gamma acc - mean(gamma acc) - xhat mean(gamma acc xhat)),
+  EPI_LN_BWD = 6,        // rows of 128 channels: acc = d(LayerNorm(x)); dx = rstd (gamma acc - mean(gamma acc) - xhat mean(gamma acc xhat)),
                          //   and per CTA the sums over rows of acc xhat and acc
+  EPI_LN_BWD_T = 7       // the same with the 128 channels as rows and pixels as columns; x and dx [128][N]
 };
+constexpr bool epi_is_ln(int epi) { return epi == EPI_LN_BWD || epi == EPI_LN_BWD_T; }
 
 constexpr int kBM = 128;
 constexpr int kStageA = kBM * 128;  // bytes
@@ -46,10 +48,18 @@ constexpr int kStageA = kBM * 128;  // bytes
 // gradients fetched a tile ahead into registers: 0.381 ms per launch at 768 x 768 pixels against 0.365.)
 constexpr int gemm_epi_warps(int epi) { return epi == EPI_STORE || epi == EPI_GATE_MUL ? 8 : 16; }
 constexpr int gemm_threads(int epi) { return 64 + 32 * gemm_epi_warps(epi); }
-// operand stages; EPI_LN_BWD keeps room for an x tile, its rows' sums and gamma.  (Two x tiles and four stages of a 16-bit type:
-// 215 us per launch at 768 x 768 pixels against 206: the operands' prefetch is worth more.)
-constexpr int gemm_stages(int epi, int bn, int es) { return bn == 256 ? 4 : epi != EPI_LN_BWD ? 6 : es == 2 ? 5 : 4; }
-constexpr int gemm_extra(int epi, int es) { return epi == EPI_LN_BWD ? 128 * 128 * es + 2 * 4 * 128 * 8 + 512 : 0; }
+// Operand stages and x tiles.  EPI_LN_BWD has ten (fp32: twenty) blocks of K per tile, and stages are worth more than a second x
+// tile (768 x 768 pixels, bf16: 215 us per launch with four and two, 206 with five and one); EPI_LN_BWD_T has two (four), and it is
+// the other way round (191 us with five and one, 137 with four and two; fp32 at 512 x 512 116 with four and one, 91 with two and two).
+constexpr int gemm_stages(int epi, int bn, int es) {
+  return epi == EPI_LN_BWD_T ? (es == 2 ? 4 : 2) : bn == 256 ? 4 : !epi_is_ln(epi) ? 6 : es == 2 ? 5 : 4;
+}
+constexpr int gemm_x_tiles(int epi) { return epi == EPI_LN_BWD_T ? 2 : 1; }
+// (x tiles, partial sums; gamma, or the totals of 16 warps' columns and the tiles' pixels' statistics)
+constexpr int gemm_extra(int epi, int es) {
+  const int nx = gemm_x_tiles(epi);
+  return !epi_is_ln(epi) ? 0 : nx * 128 * 128 * es + 2 * 4 * 128 * 8 + (epi == EPI_LN_BWD ? 512 : 16 * 256 + nx * 2 * 512);
+}
 
 
 struct GemmArgs {
@@ -436,6 +446,131 @@ __device__ __forceinline__ void ln_bwd_rows(const GemmArgs& g, uint8_t* sX, floa
   if (t == 0) bulk_wait_group0();
 }
 
+// Epilogue EPI_LN_BWD_T: thread = channel, 32 of the tile's 128 pixels.  Here the sums over channels go across the lanes of a warp
+// and the four warps of a pixel chunk, and the sums over pixels stay in the thread.  xhat is formed twice: its registers would not
+// fit beside the accumulators and the sums under way.  No early return, as above.
+// At 768 x 768 pixels, bf16: 137 us per launch for 3 tensors (69 at the copy rate), against 55 + 117 with du between two kernels;
+// fp32 (TF32) at 512 x 512 91 against 47 + 101.
+template <typename T>
+__device__ __forceinline__ void ln_bwd_cols(const GemmArgs& g, uint8_t* sX, float2* s_part, float2* s_tot, const float* s_stat, uint64_t* tfull,
+                                            uint64_t* tempty, uint64_t* xfull, uint64_t* xempty, uint32_t tmem_base, int total, int warp, int lane) {
+  constexpr int ES = sizeof(T), PIECES = 32 * ES / 16, PE = 16 / ES;     // 16-byte pieces of a thread's pixels, elements of one
+  constexpr int NX = gemm_x_tiles(EPI_LN_BWD_T), XBYTES = 128 * 128 * ES;
+  const int quarter = warp & 3, grp = (warp - 2) >> 2, row = quarter * 32 + lane, t = (warp - 2) * 32 + lane;
+  const float gamma = g.gamma ? to_f32(static_cast<const T*>(g.gamma)[row]) : 1.f;
+  const uint32_t xa0 = smem_u32(sX) + (ES == 2 ? grp >> 1 : grp) * 16384 + row * 128, piece0 = ES == 2 ? (grp & 1) * 4 : 0, sw = row & 7;
+  float2* tot = s_tot + (warp - 2) * 32;
+  float acc_g = 0.f, acc_b = 0.f;
+  int acc = 0, i = 0;
+  uint32_t acc_phase = 0;
+  uint32_t xa = xa0;
+  const float *s_mu = s_stat + grp * 32, *s_rs = s_mu + 128;
+  // xhat of a piece's pixels
+  auto hats = [&](int p, float (&xh)[PE]) {
+    const uint4 raw = lds128(xa + (((piece0 + p) ^ sw) << 4));
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int e = 0; e < PE; e += 4) {
+      const float4 mu = *reinterpret_cast<const float4*>(s_mu + p * PE + e), rs = *reinterpret_cast<const float4*>(s_rs + p * PE + e);
+      float x[4];
+      if constexpr (ES == 2) {
+        const float2 a = unpack2<T>(w[e / 2]), b = unpack2<T>(w[e / 2 + 1]);
+        x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = __uint_as_float(w[k]);
+      }
+      xh[e] = (x[0] - mu.x) * rs.x; xh[e + 1] = (x[1] - mu.y) * rs.y; xh[e + 2] = (x[2] - mu.z) * rs.z; xh[e + 3] = (x[3] - mu.w) * rs.w;
+    }
+  };
+  for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++i) {
+    const int b = i % NX;
+    xa = xa0 + b * XBYTES;
+    s_mu = s_stat + b * 256 + grp * 32;
+    s_rs = s_mu + 128;
+    mbar_wait(&xfull[b], (i / NX) & 1, g.err, 7);
+    mbar_wait(&tfull[acc], acc_phase, g.err, 4);
+    tc_fence_after_sync();
+    float v[32];
+    ld32_f(tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + grp * 32, v);
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&tempty[acc]);
+    float2 mine;       // this warp's channels' sums for pixel grp 32 + lane
+    {
+      float a[32];
+#pragma unroll
+      for (int c = 0; c < 32; ++c) { acc_b += v[c]; a[c] = v[c] * gamma; }
+      mine.x = sum_lanes32(a, lane);
+    }
+    {
+      float a[32];
+#pragma unroll
+      for (int p = 0; p < PIECES; ++p) {
+        float xh[PE];
+        hats(p, xh);
+#pragma unroll
+        for (int e = 0; e < PE; ++e) {
+          const float d = v[p * PE + e] * xh[e];
+          acc_g += d;
+          a[p * PE + e] = d * gamma;
+        }
+      }
+      mine.y = sum_lanes32(a, lane);
+    }
+    float2* part = s_part + (i & 1) * 512 + grp * 32 + lane;     // (the set of two tiles ago: every warp has met the others since it was read)
+    part[quarter * 128] = mine;
+    named_barrier(1 + grp, 128);
+    float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { const float2 p = part[q * 128]; sum.x += p.x; sum.y += p.y; }
+    __syncwarp();
+    tot[lane] = make_float2(sum.x * (1.0f / 128), sum.y * (1.0f / 128));
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      float xh[PE], o[PE];
+      hats(p, xh);
+#pragma unroll
+      for (int e = 0; e < PE; e += 2) {
+        const float4 m = *reinterpret_cast<const float4*>(tot + p * PE + e);    // two pixels
+        const float2 rs = *reinterpret_cast<const float2*>(s_rs + p * PE + e);
+        o[e] = rs.x * (v[p * PE + e] * gamma - m.x - xh[e] * m.y);
+        o[e + 1] = rs.y * (v[p * PE + e + 1] * gamma - m.z - xh[e + 1] * m.w);
+      }
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if constexpr (ES == 2) w[k] = pack2<T>(o[2 * k], o[2 * k + 1]);
+        else w[k] = __float_as_uint(o[k]);
+      }
+      sts128(xa + (((piece0 + p) ^ sw) << 4), w[0], w[1], w[2], w[3]);
+    }
+    fence_proxy_async_smem();
+    named_barrier(5, 512);
+    if (t == 0) {
+      for (int c = 0; c < ES; ++c) tma_store_3d(&g.tmDx, sX + b * XBYTES + c * 16384, tile * 128 + c * (128 / ES), 0, 0);
+      bulk_commit_group();
+      bulk_wait_group_read0();
+      mbar_arrive(&xempty[b]);
+    }
+    __syncwarp();
+    acc ^= 1;
+    if (acc == 0) acc_phase ^= 1;
+  }
+  // this thread's channel, its 32 of each tile's pixels
+  named_barrier(5, 512);
+  s_part[grp * 128 + row] = make_float2(acc_g, acc_b);
+  named_barrier(5, 512);
+  if (t < 128) {
+    float2 s = s_part[t];
+    for (int q = 1; q < 4; ++q) { const float2 p = s_part[q * 128 + t]; s.x += p.x; s.y += p.y; }
+    g.sum_g[blockIdx.x * 128 + t] = s.x;
+    g.sum_b[blockIdx.x * 128 + t] = s.y;
+  }
+  if (t == 0) bulk_wait_group0();
+}
+
 template <typename TIN, typename TOUT, int BN, int EPI, int STAGES>
 __global__ void __launch_bounds__(gemm_threads(EPI), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
@@ -455,30 +590,35 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * kStageA;
-  // LN_BWD: the x tile, two sets of the rows' partial sums, gamma
-  [[maybe_unused]] constexpr int XBYTES = 128 * 128 * ES;
+  // LN_BWD: the x tile, two sets of partial sums, gamma; LN_BWD_T: ..., 16 warps' totals, the pixels' mean and rstd
+  [[maybe_unused]] constexpr int XBYTES = 128 * 128 * ES, NX = gemm_x_tiles(EPI);
   uint8_t* sX = sB + STAGES * STAGE_B;
-  [[maybe_unused]] float2* s_part = reinterpret_cast<float2*>(sX + XBYTES);     // [2][4][128]
+  [[maybe_unused]] float2* s_part = reinterpret_cast<float2*>(sX + NX * XBYTES);     // [2][4][128]
   [[maybe_unused]] float* s_gamma = reinterpret_cast<float*>(s_part + 2 * 4 * 128);
+  [[maybe_unused]] float2* s_tot = s_part + 2 * 4 * 128;
+  [[maybe_unused]] float* s_stat = reinterpret_cast<float*>(s_tot + 16 * 32);      // [NX][2][128]
   uint64_t* full = reinterpret_cast<uint64_t*>(sX + gemm_extra(EPI, ES));
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + 2;
-  [[maybe_unused]] uint64_t* xfull = tempty + 2;     // x tile landed
-  [[maybe_unused]] uint64_t* xempty = xfull + 1;     // ... and its dx has been read by the store
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2 + (EPI == EPI_LN_BWD ? 2 : 0));
+  [[maybe_unused]] uint64_t* xfull = tempty + 2;     // [2] x tile landed
+  [[maybe_unused]] uint64_t* xempty = xfull + 2;     // [2] ... and its dx has been read by the store
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2 + (epi_is_ln(EPI) ? 4 : 0));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], gemm_epi_warps(EPI)); }
-    if constexpr (EPI == EPI_LN_BWD) {
-      mbar_init(xfull, 1);
-      mbar_init(xempty, 1);
+    if constexpr (epi_is_ln(EPI)) {
+      for (int b = 0; b < 2; ++b) { mbar_init(&xfull[b], 1); mbar_init(&xempty[b], 1); }
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmA0);
     tma_prefetch_desc(&tmB0);
+  }
+  if constexpr (EPI == EPI_LN_BWD_T) {   // what a last tile's copies leave unwritten is read beside zeros
+    if (threadIdx.x < NX * 256) s_stat[threadIdx.x] = 0.f;
+    fence_proxy_async_smem();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 2 * BN);
   tc_fence_before_sync();
@@ -534,11 +674,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if constexpr (EPI == EPI_LN_BWD) {   // (after the operands: the tile before may still hold the buffer)
-          const uint32_t i = (tile - blockIdx.x) / gridDim.x;
-          if (!ok || !mbar_wait(xempty, (i & 1) ^ 1, g.err, 6)) break;
-          mbar_expect_tx(xfull, XBYTES);
-          for (int c = 0; c < ES; ++c) tma_load_3d(sX + c * 16384, &g.tmX, xfull, c * CE, tm * kBM, 0);
+        if constexpr (epi_is_ln(EPI)) {   // (after the operands: the tile before may still hold the buffer)
+          const uint32_t i = (tile - blockIdx.x) / gridDim.x, b = i % NX;
+          uint64_t* bar = &xfull[b];
+          if (!ok || !mbar_wait(&xempty[b], ((i / NX) & 1) ^ 1, g.err, 6)) break;
+          const uint32_t stat = EPI == EPI_LN_BWD_T ? 4 * min(128, g.N - n0) : 0;   // (N is a multiple of four)
+          mbar_expect_tx(bar, XBYTES + 2 * stat);
+          for (int c = 0; c < ES; ++c)
+            tma_load_3d(sX + b * XBYTES + c * 16384, &g.tmX, bar, EPI == EPI_LN_BWD ? c * CE : n0 + c * CE, EPI == EPI_LN_BWD ? tm * kBM : 0, 0);
+          if constexpr (EPI == EPI_LN_BWD_T) {
+            bulk_load(s_stat + b * 256, g.mean + n0, stat, bar);
+            bulk_load(s_stat + b * 256 + 128, g.rstd + n0, stat, bar);
+          }
         }
       }
     }
@@ -591,6 +738,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     if constexpr (EPI == EPI_GATE_MUL) dependent_wait();
     if constexpr (EPI == EPI_LN_BWD) {
       ln_bwd_rows<TIN>(g, sX, s_part, s_gamma, tfull, tempty, xfull, xempty, tmem_base, total, warp, lane);
+    } else if constexpr (EPI == EPI_LN_BWD_T) {
+      ln_bwd_cols<TIN>(g, sX, s_part, s_tot, s_stat, tfull, tempty, xfull, xempty, tmem_base, total, warp, lane);
     } else {
     // The backward gate epilogues read a gradient tile from global memory, just before they wait for the product.
     constexpr bool kGradTile = EPI == EPI_GATE_IN_BWD || EPI == EPI_GATE_OUT_BWD;
