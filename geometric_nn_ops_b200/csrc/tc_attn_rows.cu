@@ -39,8 +39,8 @@ namespace tc {
 
 namespace {
 
-// fp32: tiles are twice as large, which leaves room for two rows per CTA; operands were rounded to TF32 before, P is as it is
-// stored.  P takes one column per key and so replaces S in place; V is read across its rows, which 32-bit operands can only be
+// fp32: tiles are twice as large, which leaves room for two rows per CTA; operands were rounded to TF32 before, P goes into the
+// product as two TF32 terms.  P takes one column per key and so replaces S in place; V is read across its rows, which 32-bit operands can only be
 // in the swizzle with 32-byte atoms.
 template <typename T> struct RowsCfg {
   static constexpr bool F32 = sizeof(T) == 4;
@@ -63,7 +63,7 @@ template <typename T> struct RowsCfg {
   static constexpr uint32_t HI = F32 ? desc_hi(8 * 128, 2) : desc_hi(8 * 64, 4);        // Q, K: SWIZZLE_128B, SWIZZLE_64B
   static constexpr uint32_t HI_V = F32 ? desc_hi(512, 1) : desc_hi(8 * 64, 4);          // V across its rows
   static constexpr int kind = F32 ? KIND_TF32 : KIND_F16;
-  static constexpr int kVec = 16 / (int)sizeof(T); // elements of a 16-byte piece
+  static constexpr int kVecBits = F32 ? 2 : 3, kVec = 1 << kVecBits;   // elements of a 16-byte piece
 };
 constexpr float kLn2 = 0.6931471805599453f;
 
@@ -286,15 +286,16 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const float inv = 1.0f / pl;
 #pragma unroll
         for (int h = 0; h < 32 / M::kVec; ++h) {
-          if (h * M::kVec >= a.D) continue;
-          if constexpr (M::F32) {
-            auto f = [&](int i) { return __uint_as_float(o[h >> 2][(h & 3) * 4 + i]) * inv; };
-            (reinterpret_cast<float4*>(a.o) + po)[h] = make_float4(f(0), f(1), f(2), f(3));
-          } else {
-            uint4 pk;
-            auto f = [&](int i) { return __uint_as_float(o[h >> 1][(h & 1) * 8 + i]) * inv; };
-            pk.x = pack2<T>(f(0), f(1)); pk.y = pack2<T>(f(2), f(3)); pk.z = pack2<T>(f(4), f(5)); pk.w = pack2<T>(f(6), f(7));
-            (reinterpret_cast<uint4*>(a.o) + po)[h] = pk;
+          if (h * M::kVec < a.D) {
+            if constexpr (M::F32) {
+              auto f = [&](int i) { return __uint_as_float(o[h >> 2][(h & 3) * 4 + i]) * inv; };
+              (reinterpret_cast<float4*>(a.o) + po)[h] = make_float4(f(0), f(1), f(2), f(3));
+            } else {
+              uint4 pk;
+              auto f = [&](int i) { return __uint_as_float(o[h >> 1][(h & 1) * 8 + i]) * inv; };
+              pk.x = pack2<T>(f(0), f(1)); pk.y = pack2<T>(f(2), f(3)); pk.z = pack2<T>(f(4), f(5)); pk.w = pack2<T>(f(6), f(7));
+              (reinterpret_cast<uint4*>(a.o) + po)[h] = pk;
+            }
           }
         }
         // The largest of the steps' sums over 64 keys is 1 to 64 times the largest P, so that m plus log(sum / 64) lies at
@@ -329,21 +330,29 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int u = 0; u < 2; ++u) {
             const float4 mA = lds128f(mrow + (q * 4 + u * 2) * 16), mB = lds128f(mrow + (q * 4 + u * 2 + 1) * 16);
             const float2 mk[4] = {make_float2(mA.x, mA.y), make_float2(mA.z, mA.w), make_float2(mB.x, mB.y), make_float2(mB.z, mB.w)};
-            // (bias: 128-byte rows, 16-byte chunks swizzled by the row; fp32: two tiles of 32 keys)
-            uint4 raw = make_uint4(0, 0, 0, 0), more = raw;
-            if constexpr (HB && M::F32) {
-              const uint32_t at = brow + (q >> 1) * (M::TB / 2), g = (q & 1) * 4 + u * 2;
-              raw = lds128(at ^ (g << 4));
-              more = lds128(at ^ ((g + 1) << 4));
-            } else if constexpr (HB) {
-              raw = lds128(brow ^ ((q * 2 + u) << 4));
+            if constexpr (M::F32) {    // (bias: two tiles of 32 keys, 128-byte rows, 16-byte chunks swizzled by the row)
+              uint4 b0 = make_uint4(0, 0, 0, 0), b1 = b0;
+              if constexpr (HB) {
+                const uint32_t at = brow + (q >> 1) * (M::TB / 2), g = (q & 1) * 4 + u * 2;
+                b0 = lds128(at ^ (g << 4));
+                b1 = lds128(at ^ ((g + 1) << 4));
+              }
+              const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
+                if constexpr (HB) v = __fadd2_rn(v, pair(bw[2 * i], bw[2 * i + 1]));
+                x[u * 4 + i] = v;
+              }
+              continue;
             }
-            const uint32_t bw[8] = {raw.x, raw.y, raw.z, raw.w, more.x, more.y, more.z, more.w};
+            uint4 raw = make_uint4(0, 0, 0, 0);
+            if constexpr (HB && !M::F32) raw = lds128(brow ^ ((q * 2 + u) << 4));   // (128-byte rows, 16-byte chunks swizzled by the row)
+            const uint32_t bw[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
-              if constexpr (HB && M::F32) v = __fadd2_rn(v, pair(bw[2 * i], bw[2 * i + 1]));
-              else if constexpr (HB) v = __fadd2_rn(v, unpack2<T>(bw[i]));
+              if constexpr (HB && !M::F32) v = __fadd2_rn(v, unpack2<T>(bw[i]));
               x[u * 4 + i] = v;
             }
           }
@@ -486,7 +495,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       pend = true; pm = m; pl = l; pseen = seen;
       const int qi = it.q0 + r, s = it.s0 + g;
-      po = qi < a.N ? (int)((it.b * a.o_st[0] + s * a.o_st[1] + qi * a.o_st[2] + it.h * a.o_st[3]) / M::kVec) : -1;
+      po = qi < a.N ? (int)((it.b * a.o_st[0] + s * a.o_st[1] + qi * a.o_st[2] + it.h * a.o_st[3]) >> M::kVecBits) : -1;
       pstat = ((it.b * a.S + s) * a.H + it.h) * a.N + qi;
     }
     if (pend && ok) finish(c - 1);
