@@ -71,7 +71,11 @@ inline int fail(int code, const char* fmt, ...) {
 // while others run are packed onto the SMs that have room and keep the little L1 that is left there (with every kernel started
 // so: fp32 update at 64 x 64 pixels 53.3 -> 55.3 us, bf16 update with gradients at 768 1806 -> 1835).  As it is, us before and
 // after: attention at 64, 256 residues 14.1 -> 13.6, 45.2 -> 42.8, with gradients at 301 469 -> 460; update at 203 61.4 -> 55.1,
-// with gradients at 384 497 -> 483; from 512 on no difference.
+// with gradients at 384 497 -> 483.
+// And only the short ones: `us` is what the kernel takes at least, by its bytes or its exponentials.  The few us of a ramp do
+// not show beside a long kernel, and with every kernel of the pair stack at 1024 residues (86 us and more each, at the power limit
+// throughout) started early, its pass took 0.5 to 1 % longer: 23.24-23.34 -> 23.40-23.60 ms.  The kernels that gained take at
+// least 1 to 40 us; between that and 70 neither start is measurably better.
 __device__ __forceinline__ void dependent_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependent_enter() {
@@ -79,13 +83,17 @@ __device__ __forceinline__ void dependent_enter() {
   dependent_wait();
 }
 
+constexpr double kEarlyStartUs = 60.0;
+inline double us_of_bytes(double bytes) { return bytes / 6.5e6; }        // the measured copy rate
+inline double us_of_logits(double logits) { return logits / 4.6e6; }     // one exponential each, 16 per clock and SM
+
 template <typename... K, typename... A>
-inline void launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_dependent(double us, void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = 1;
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = us < kEarlyStartUs ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, K(args)...);   // (errors: TRI_LAUNCH_OK)
 }
 

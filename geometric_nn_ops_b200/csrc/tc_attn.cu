@@ -4,8 +4,8 @@
 // tile row, each owning half of the tile's columns), warp 8 issues every tcgen05.mma and warp 9 every TMA / bulk
 // copy.  The three sides meet only on mbarriers, so the serial issue code never sits between the arithmetic warps'
 // steps, and score products for the next tile are issued as soon as the accumulators have been read into registers.
-// The arithmetic is packed fp32x2 (fma.rn.f32x2 and friends); row constants arrive in the form it adds
-// (-m, -log l * log2e, -delta), and additive key-mask terms (0, -1e9, -inf beyond N) come from a small array
+// The arithmetic is packed fp32x2 (fma.rn.f32x2 and friends); row constants of the backward come as
+// extra channels of the products (RowFactors), and additive key-mask terms (0, -1e9, -inf beyond N) from a small array
 // prepared once per call.  With head dim 32 the probabilities (forward) and dS / P^T / dS^T (backward) never touch
 // shared memory: they are stored packed into TMEM and read from there as the A operand of the next product, which
 // halves the shared-memory traffic that otherwise bounds these kernels.
@@ -15,7 +15,7 @@
 //   S = Q K^T (TMEM) -> x = scale*S + mask + bias -> running maximum -> P = 2^((x - m) log2e) -> O_half += P V.
 //   Each half of the key tile keeps its own maximum, sum and O accumulator (merged at the end); O stays in TMEM
 //   and is rescaled only when a maximum grows by more than 8 ln 2.
-// Backward: three deterministic passes, each recomputing P from the saved statistics (see below).
+// Backward: deterministic passes, two with head dim 32 and three otherwise, each recomputing P from the saved statistics (see below).
 // Semantics follow triangle_attention_torch (geometric_nn_ops_torch/triangle/_reference/triangle_attention.py:28-44):
 // bias and the finite -1e9 key-mask sentinel are added in fp32; keys beyond N_res get -inf.
 #include <algorithm>
@@ -421,13 +421,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // =================================================================================================
-// Backward.  Three deterministic passes, each recomputing P from the saved statistics:
+// Backward.  Deterministic passes, each recomputing P from the saved statistics (with head dim 32 the first gives dQ too):
 //   dK/dV : one CTA per (b, row, head, 128-key block), thread = key.  Per 64-query tile:
 //           S^T = K Q^T and dP^T = V dO^T (TMEM), P^T and dS^T packed (TMEM or smem), dV += P^T dO, dK += dS^T Q.
 //           The bias is read from a transposed copy so that a thread's queries are contiguous.
 //   dQ    : one CTA per (b, row, head, 128-query block), thread = query.  Per 64-key tile:
 //           S = Q K^T, dP = dO V^T, dS packed into TMEM, dQ += dS K.
-//   dbias : one CTA per (row chunk, b, head, 128-query block, 64-key block) looping over its rows in order and
+//   dbias : one CTA per (row chunk, b, head, 64-query block, 128-key block) looping over its rows in order and
 //           summing dS in registers (no atomics: fixed order), S / dP double buffered in TMEM.
 // P = exp((x - m) - log l), dS = P * (dP - delta), delta = sum_d dO*O (computed by a small kernel first).
 // =================================================================================================
@@ -1584,7 +1584,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     TRI_TRY(set_dyn_smem(kern, GeoC<HD>::SMEM));   // per-device attribute: set on every launch
     KernelTimer kt(kMerge ? "tc_attn_bwd_dkdvdq" : "tc_attn_bwd_dkdv", st, (kMerge ? 10.0 : 8.0) * pairs * d->D,
                    (kMerge ? 7.0 : 6.0) * tensor_bytes);
-    launch_dependent(kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoC<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoC<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
   }
   if (kMerge) {
@@ -1612,7 +1612,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     auto kern = bias ? attn_bwd_dq_kernel<T, HD, true> : attn_bwd_dq_kernel<T, HD, false>;
     TRI_TRY(set_dyn_smem(kern, GeoQ<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dq", st, 2.0 * pairs * d->D, 5.0 * tensor_bytes);
-    launch_dependent(kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoQ<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, (unsigned)((long long)qblocks * d->B * d->n_seq * d->H), 320, GeoQ<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
   }
   // ---- dbias ---------------------------------------------------------------------------------
@@ -1634,7 +1634,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     auto kern = attn_bwd_dbias_kernel<T, HD>;   // (with the dK/dV pass's maps)
     TRI_TRY(set_dyn_smem(kern, GeoB<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor_bytes);
-    launch_dependent(kern, (unsigned)(combos * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, (unsigned)(combos * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     if (chunks > 1) {   // fixed-order sum of the row-chunk partials
       sum_partials_kernel<<<cdiv(nb, 256), 256, 0, st>>>(dbias_partial, chunks, nb, dbias);
@@ -1695,7 +1695,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto kern = bias != nullptr ? attn_fwd_tc_kernel<T, HD, true> : attn_fwd_tc_kernel<T, HD, false>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<HD>::SMEM));
-  launch_dependent(kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
+  launch_dependent(us_of_logits(pairs), kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
   TRI_LAUNCH_OK();
   return 0;
 }

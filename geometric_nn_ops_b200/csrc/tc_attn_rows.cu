@@ -539,7 +539,7 @@ int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap
   auto launch = [&](auto elem, auto kern, const CUtensorMap& tb) {
     using M = RowsCfg<decltype(elem)>;
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::SMEM));
-    launch_dependent(kern, (unsigned)std::min<long long>(items, sm_count()), M::kThreads, M::SMEM, st, tq, tk, tv, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, (unsigned)std::min<long long>(items, sm_count()), M::kThreads, M::SMEM, st, tq, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     return 0;
   };

@@ -1,7 +1,8 @@
 // Triangle attention on the tensor cores for fp32 with TF32 products, head dim up to 32 (tcgen05 kind::tf32, TMEM, TMA).
 //
 // The operands of a product are rounded to TF32 (nearest), as the CUDA-core path does: q, k, v and dO once per call into
-// copies in the workspace, P and dS when they are stored.  Everything else is fp32.
+// copies in the workspace, P and dS of the backward when they are stored; the forward's P is multiplied as two TF32 terms.
+// Everything else is fp32.
 //   forward   the row-sharing kernel of tc_attn_rows.cu on the rounded copies
 //   dK / dV   one item per (batch, row, head, 128-key block), thread = key: S^T = K Q^T, dP^T = V dO^T per 64-query tile,
 //             dV += P^T dO, dK += dS^T Q
@@ -827,7 +828,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     auto kern = bias ? attn_bwd_tf32_kernel<true, true> : attn_bwd_tf32_kernel<true, false>;
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GeoT<true>::SMEM));
     KernelTimer kt("tc_attn_bwd_dkdv", st, 8.0 * pairs * d->D, 6.0 * tensor);
-    launch_dependent(kern, grid, kThreads, GeoT<true>::SMEM, st, a0, a1, b0, b1, l0, l1, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, grid, kThreads, GeoT<true>::SMEM, st, a0, a1, b0, b1, l0, l1, tb, a);
     TRI_LAUNCH_OK();
   }
   // ---- dQ: stationary Q, dO; streamed K, V ------------------------------------------------------
@@ -845,7 +846,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     auto kern = bias ? attn_bwd_tf32_kernel<false, true> : attn_bwd_tf32_kernel<false, false>;
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GeoT<false>::SMEM));
     KernelTimer kt("tc_attn_bwd_dq", st, 6.0 * pairs * d->D, 5.0 * tensor);
-    launch_dependent(kern, grid, kThreads, GeoT<false>::SMEM, st, a0, a1, b0, b1, l0, l0, tb, a);
+    launch_dependent(us_of_logits(pairs), kern, grid, kThreads, GeoT<false>::SMEM, st, a0, a1, b0, b1, l0, l0, tb, a);
     TRI_LAUNCH_OK();
   }
   // ---- dbias ------------------------------------------------------------------------------------
@@ -862,7 +863,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     a.out[0] = chunks > 1 ? w.part : dbias;
     TRI_CUDA_OK(cudaFuncSetAttribute(attn_bwd_dbias_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GeoTB::SMEM));
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor);
-    launch_dependent(attn_bwd_dbias_tf32_kernel, (unsigned)(combos * chunks), kThreads, GeoTB::SMEM, st, tk, tv, tq, tdo, w.bias_t, pitch_of(d), a);
+    launch_dependent(us_of_logits(pairs), attn_bwd_dbias_tf32_kernel, (unsigned)(combos * chunks), kThreads, GeoTB::SMEM, st, tk, tv, tq, tdo, w.bias_t, pitch_of(d), a);
     TRI_LAUNCH_OK();
     if (chunks > 1) {
       add_chunks_kernel<<<cdiv(n, 256), 256, 0, st>>>(w.part, chunks, n, dbias);

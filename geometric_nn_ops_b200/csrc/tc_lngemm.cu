@@ -342,8 +342,9 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   auto kern = ln_gate_in_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(a.tiles, sm_count());
-  KernelTimer kt("tc_ln_gate_in", st, 2.0 * p.M * 128 * 512, 4.0 * p.M * 128 * 2);
-  launch_dependent(kern, grid, kThreads, smem, st, tmX, tmW, tmZ, tmA, tmB, a);
+  const double bytes = 4.0 * p.M * 128 * 2;
+  KernelTimer kt("tc_ln_gate_in", st, 2.0 * p.M * 128 * 512, bytes);
+  launch_dependent(us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmX, tmW, tmZ, tmA, tmB, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -671,8 +672,9 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   auto kern = ln_gate_out_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(a.tiles, sm_count());
-  KernelTimer kt("tc_ln_gate_out", st, 2.0 * p.M * 128 * 256, (p.u_cm ? 4.0 : 3.0) * p.M * 128 * 2);
-  launch_dependent(kern, grid, kThreads, smem, st, tmT, tmZ, tmWo, tmWg, a);
+  const double bytes = (p.u_cm ? 4.0 : 3.0) * p.M * 128 * 2;
+  KernelTimer kt("tc_ln_gate_out", st, 2.0 * p.M * 128 * 256, bytes);
+  launch_dependent(us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmT, tmZ, tmWo, tmWg, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -930,8 +932,9 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   auto kern = gate_in_bwd_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = G::kHalves == 2 ? std::min(a.tiles, sm_count()) : 2 * std::min(a.tiles, sm_count() / 2);
-  KernelTimer kt("tc_gate_in_bwd", st, 0.0, 7.0 * p.M * 128 * E);
-  launch_dependent(kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
+  const double bytes = 7.0 * p.M * 128 * E;
+  KernelTimer kt("tc_gate_in_bwd", st, 0.0, bytes);
+  launch_dependent(us_of_bytes(bytes), kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
   TRI_LAUNCH_OK();
   return 0;
 }
