@@ -545,7 +545,7 @@ template <int HD> struct GeoC {
 // after every second tile one product dQ_pair[128 queries x D] = dS_pair K reads the pair MN-major (M = queries) with
 // K as the MN-major B operand, into the TMEM columns dS^T no longer needs.  The arithmetic warps fetch that
 // accumulator one step later and store it, unscaled, as this key block's partial; attn_dq_sum_kernel adds the key
-// blocks' partials in fixed order.  A last tile without a partner is paired with a buffer of zeros.
+// blocks' partials in fixed order.  A last tile without a partner is paired with a buffer of zeros and has columns of its own.
 // The MMA warp runs its code as a whole, so that descriptors stay in uniform registers (a lone lane took 900 clocks to issue a
 // tile's products), and dQ is fetched after a tile's arrival on bar_p, beside its products: 1.56 -> 1.45 ms at N = 768.
 // Accumulators are read eight queries at a time, the next eight on their way (the wait for a tile's first half had been 600 of
@@ -614,6 +614,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   constexpr bool TMEM_A = HD == 32;
   constexpr uint32_t COL_PT = 192, COL_DST = 224;
   constexpr uint32_t COL_DQ = COL_DST;   // MERGE: dS^T lives in shared memory and its columns hold the dQ accumulator
+  // A last tile without a partner: its product follows its own arrivals on bar_p, behind which the dQ before it may still be read.
+  // It goes to the columns of S, which every warp has read (bar_free) and no further product wants.
+  constexpr uint32_t COL_DQ_LAST = 0;
   static_assert(!MERGE || TMEM_A, "the merged pass is built for head dim 32");
   bool ok = true;
 
@@ -720,7 +723,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             if ((j & 1) || j == nsteps - 1) {   // a pair of query tiles is complete: dQ_pair = dS_pair K (16 keys per product)
 #pragma unroll
               for (int ks = 0; ks < 8; ++ks)
-                umma<KIND_F16>(tmem_base + COL_DQ, desc_join(dsmn_lo + ks * 128, HI_PT), desc_join(kmn_lo + ks * G::RB, HI_KMAJ),
+                umma<KIND_F16>(tmem_base + (j & 1 ? COL_DQ : COL_DQ_LAST), desc_join(dsmn_lo + ks * 128, HI_PT), desc_join(kmn_lo + ks * G::RB, HI_KMAJ),
                                a.idesc_c, ks > 0);
             }
           }
@@ -737,9 +740,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const float2 sc2 = splat(a.scale), mk2 = splat(mb), l2e2 = splat(kLog2e), scl2 = splat(a.scale * kLog2e), mkl2 = splat(mb * kLog2e);
     // MERGE: fetch the dQ accumulator of query-tile pair `pair` (row r = query 128 pair + r, this thread's half of the
     // head dim) and store it, unscaled, as this key block's partial.  tcgen05.ld is warp-wide: every thread loads.
-    auto store_dq_pair = [&](int pair) {
+    auto store_dq_pair = [&](int pair, uint32_t col) {
       uint32_t v[16];
-      tmem_ld_32x16(t_row + COL_DQ + hh * 16, v);
+      tmem_ld_32x16(t_row + col + hh * 16, v);
       tmem_ld_wait();
       const int qi = pair * 128 + r;
       if (qi < a.N && ok) {
@@ -862,14 +865,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_p);
       if (!ok) break;
-      // the pair before this tile: its dQ product is done (bar_acc above), the next one waits for this warp's next arrival
+      // The pair before this tile: its dQ product is done (bar_acc above).  The next one into its columns is that of tile j + 1, which
+      // waits for this warp's arrival there; a tile j without a partner has columns of its own.
       if constexpr (MERGE) {
-        if (j >= 2 && (j & 1) == 0) store_dq_pair(j / 2 - 1);
+        if (j >= 2 && (j & 1) == 0) store_dq_pair(j / 2 - 1, COL_DQ);
       }
     }
     ok = mbar_wait(&bar_acc[(nsteps - 1) & 3], ((nsteps - 1) >> 2) & 1, a.err, 36) && ok;
     tc_fence_after_sync();
-    if constexpr (MERGE) store_dq_pair((nsteps - 1) / 2);   // the last pair
+    if constexpr (MERGE) store_dq_pair((nsteps - 1) / 2, nsteps & 1 ? COL_DQ_LAST : COL_DQ);   // the last pair
     {
       const bool st_ok = kj < a.N && ok && hh == 0;
       T* krow = reinterpret_cast<T*>(a.out0) + b * a.out0_st[0] + s * a.out0_st[1] + kj * a.out0_st[2] + h * a.out0_st[3];

@@ -53,3 +53,23 @@ def test_backward(shape, dtype, d_scale, shift):
         slack = 2.0 ** -25 * want.numel() ** 0.5 / float(want.norm()) if dtype == torch.float16 else 0.0   # fp16's smallest step
         err = float((got - want).norm() / want.norm())
         assert err <= limit + slack, f"{name}: {err:.2e} > {limit + slack:.2e}"
+
+
+# odd numbers of 64-query tiles: the last one's dQ product has no partner, and its own columns
+@pytest.mark.parametrize("n", [136, 192, 301, 320, 64])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+def test_unpaired_last_tile(n, dtype):
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import triangle_attention
+    t, mask, d_out = util.attn_inputs(1, 96, n, 4, 32, dtype, seed=n, keep=0.9)
+    _, grads = util.attn_fwd_bwd(triangle_attention, t, mask, 0.2, d_out)
+    torch.cuda.synchronize()
+    assert _lib.last_path() == "tcgen05"
+    limit = 4 * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
+    for name, want in _reference(t, mask, d_out, 0.2).items():
+        err = float((grads[name].double() - want).norm() / want.norm())
+        assert err <= limit, f"{name}: {err:.2e} > {limit:.2e}"
+    for _ in range(40):
+        _, again = util.attn_fwd_bwd(triangle_attention, t, mask, 0.2, d_out)
+        for name, first in grads.items():
+            assert torch.equal(again[name], first), name
