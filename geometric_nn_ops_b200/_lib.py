@@ -107,6 +107,7 @@ EXPORTS = {
     "tri_mul_fwd_residual": (c_int, [POINTER(TriMulDesc)] + [c_void_p] * 2 + [POINTER(TriMulWeights)] + [c_void_p] * 3 + [c_size_t, c_void_p]),
     "tri_gate_mul": (c_int, [c_int, c_int64] + [c_void_p] * 4),
     "tri_gated_linear": (c_int, [c_int, c_int64, c_int32, c_int32, c_int32] + [c_void_p] * 8),
+    "tri_gated_linear_after": (c_int, [c_int, c_int64, c_int32, c_int32, c_int32] + [c_void_p] * 8),
     "tri_attn_project_bias": (c_int, [POINTER(TriAttnProjDesc), c_int64] + [c_void_p] * 7),
     "tri_attn_project": (c_int, [POINTER(TriAttnProjDesc)] + [c_void_p] * 8 + [c_size_t, c_void_p]),
     "tri_mul_saved_bytes": (c_size_t, [POINTER(TriMulDesc)]),

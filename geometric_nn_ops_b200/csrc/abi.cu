@@ -241,14 +241,24 @@ int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z
   return tc::attn_project_bias(d, plane, z, ln_w, ln_b, w_bias, bias, ws, (cudaStream_t)stream);
 }
 
-int tri_gated_linear(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
-                     const void* w_out, void* gated, void* out, void* status, tri_stream_t stream) {
+static int gated_linear(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
+                        const void* w_out, void* gated, void* out, void* status, bool after, tri_stream_t stream) {
   if (!s || !w_gate || !o || !w_out || !gated || !out || !status) return fail(TRI_ERR_ARG, "null pointer");
   if (dtype != TRI_BF16 && dtype != TRI_F16) return fail(TRI_ERR_UNSUPPORTED, "16-bit types only");
   if (M < 1 || M > 2147483647LL - 128 || K < 8 || W < 8 || N < 8 || K % 8 || W % 8 || N % 8 || !aligned_to(16, {s, w_gate, o, w_out, gated, out}))
     return fail(TRI_ERR_ARG, "bad extent or alignment: M %lld, K %d, W %d, N %d", (long long)M, K, W, N);
   set_path("tcgen05");
-  return tc::gated_linear(dtype, M, K, W, N, s, w_gate, o, w_out, gated, out, static_cast<int*>(status), (cudaStream_t)stream);
+  return tc::gated_linear(dtype, M, K, W, N, s, w_gate, o, w_out, gated, out, static_cast<int*>(status), after, (cudaStream_t)stream);
+}
+
+int tri_gated_linear(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
+                     const void* w_out, void* gated, void* out, void* status, tri_stream_t stream) {
+  return gated_linear(dtype, M, K, W, N, s, w_gate, o, w_out, gated, out, status, false, stream);
+}
+
+int tri_gated_linear_after(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
+                           const void* w_out, void* gated, void* out, void* status, tri_stream_t stream) {
+  return gated_linear(dtype, M, K, W, N, s, w_gate, o, w_out, gated, out, status, true, stream);
 }
 
 int tri_gate_mul(int dtype, int64_t n, const void* a, const void* gate, void* out, tri_stream_t stream) {

@@ -66,7 +66,8 @@ inline int fail(int code, const char* fmt, ...) {
 // and this one waits until all kernels before it are complete and their results visible.  (Each of them has waited in the same
 // way before it ends, so nothing older is in flight either.)
 // The first kernel of a call is launched plainly: once it runs, all work before the call is complete, and the later ones may
-// read the caller's tensors, which no kernel of the chain writes, without waiting.
+// read the caller's tensors, which no kernel of the chain writes, without waiting.  (tri_gated_linear_after continues the chain of
+// the call before it, and says so.)
 // Only the tensor-core kernels are started so.  They fill an SM by their shared memory, whereas CTAs of a small kernel that come
 // while others run are packed onto the SMs that have room and keep the little L1 that is left there (with every kernel started
 // so: fp32 update at 64 x 64 pixels 53.3 -> 55.3 us, bf16 update with gradients at 768 1806 -> 1835).  As it is, us before and
@@ -83,7 +84,7 @@ __device__ __forceinline__ void dependent_enter() {
   dependent_wait();
 }
 
-constexpr double kEarlyStartUs = 60.0;
+constexpr double kEarlyStartUs = 60.0, kLaunchPlainly = kEarlyStartUs;
 inline double us_of_bytes(double bytes) { return bytes / 6.5e6; }        // the measured copy rate
 inline double us_of_logits(double logits) { return logits / 4.6e6; }     // one exponential each, 16 per clock and SM
 

@@ -625,7 +625,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (EPI == EPI_GATE_MUL) dependent_trigger();   // (the epilogue waits)
+  if constexpr (EPI == EPI_GATE_MUL) dependent_trigger();   // (the epilogue waits; s and the weights were there before o's call)
   else dependent_enter();
 
   const int total = g.batches * g.tiles_m * g.tiles_n;
@@ -1029,6 +1029,7 @@ struct GemmPlan {
   long long plane = 0;
   void* const* peer_out = nullptr;   // GATE_IN: per-rank exchange buffers (see GemmArgs)
   int peer_world = 0, peer_rank = 0, peer_batches = 0;
+  bool first = false;                // no kernel of this call came before: launched plainly
   const char* name = "tc_gemm";
   double flops = 0, bytes = 0;
 };

@@ -37,7 +37,7 @@ int attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w, cons
                  const void* w_bias, void* qkv, void* bias, void* ws, size_t ws_size, cudaStream_t st);
 int gate_mul(int dtype, long long n, const void* a, const void* gate, void* out, cudaStream_t st);
 int gated_linear(int dtype, long long M, int K, int W, int N, const void* s, const void* w_gate, const void* o, const void* w_out, void* gated,
-                 void* out, int* status, cudaStream_t st);
+                 void* out, int* status, bool after, cudaStream_t st);
 // LayerNorm and the pair bias alone (tri_attn_project_bias)
 int attn_project_bias(const TriAttnProjDesc* d, long long plane, const void* z, const void* ln_w, const void* ln_b, const void* w_bias,
                       void* bias, void* ws, cudaStream_t st);

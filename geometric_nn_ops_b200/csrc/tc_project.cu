@@ -221,15 +221,16 @@ int attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w, cons
   return fail(TRI_ERR_ARG, "bad dtype %d", d->dtype);
 }
 
-// out = (o * sigmoid(s Wg^T)) Wo^T: the first product's epilogue gates o, and only that epilogue waits for o's kernel.  384 tokens,
-// 768 channels, bf16, whole op: 55 -> 47 us, against two library products and a gating kernel (the host was what it waited for).
+// out = (o * sigmoid(s Wg^T)) Wo^T: the first product's epilogue gates o.  `after`: only that epilogue waits for the call that wrote
+// o, and s and w_gate were there before that call.  384 tokens, 768 channels, bf16, whole op: 55 -> 47 us, against two library
+// products and a gating kernel (the host was what it waited for).
 int gated_linear(int dtype, long long M, int K, int W, int N, const void* s, const void* w_gate, const void* o, const void* w_out, void* gated,
-                 void* out, int* status, cudaStream_t st) {
+                 void* out, int* status, bool after, cudaStream_t st) {
   auto product = [&](int epi, const void* a, const void* w, int k, int n, const void* aux, void* to, const char* name) {
     GemmPlan p;
     p.a[0].ptr = a; p.a[0].mn_major = false; p.a[0].inner = k; p.a[0].outer = M; p.a[0].batch = 1; p.a[0].st_outer = k;
     p.b[0].ptr = w; p.b[0].mn_major = false; p.b[0].inner = k; p.b[0].outer = n; p.b[0].batch = 1; p.b[0].st_outer = k;
-    p.M = (int)M; p.N = n; p.K0 = k; p.out0 = to; p.ld_out = n; p.aux = aux;
+    p.M = (int)M; p.N = n; p.K0 = k; p.out0 = to; p.ld_out = n; p.aux = aux; p.first = epi == EPI_GATE_MUL && !after;
     p.name = name; p.flops = 2.0 * M * k * n; p.bytes = 2.0 * (M * (double)(k + n) + (double)k * n);
     return launch_gemm(st, dtype, epi, 128, false, p, status);
   };

@@ -41,7 +41,7 @@ struct Api {
   decltype(&tri_attn_bwd) attn_bwd;
   decltype(&tri_attn_project_bias) attn_project_bias;
   decltype(&tri_gate_mul) gate_mul;
-  decltype(&tri_gated_linear) gated_linear;
+  decltype(&tri_gated_linear_after) gated_linear_after;
   decltype(&tri_mul_saved_bytes) mul_saved_bytes;
   decltype(&tri_mul_ws_bytes) mul_ws_bytes;
   decltype(&tri_mul_fwd) mul_fwd;
@@ -59,7 +59,7 @@ void bind(const std::string& path) {
   get(api.last_error, "tri_last_error"); get(api.last_path, "tri_last_path"); get(api.ws_status, "tri_ws_status");
   get(api.attn_ws_bytes, "tri_attn_ws_bytes"); get(api.attn_fwd, "tri_attn_fwd"); get(api.attn_bwd, "tri_attn_bwd");
   get(api.mul_fwd_residual, "tri_mul_fwd_residual");
-  get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul"); get(api.gated_linear, "tri_gated_linear");
+  get(api.attn_project_bias, "tri_attn_project_bias"); get(api.gate_mul, "tri_gate_mul"); get(api.gated_linear_after, "tri_gated_linear_after");
   get(api.mul_saved_bytes, "tri_mul_saved_bytes"); get(api.mul_ws_bytes, "tri_mul_ws_bytes");
   get(api.mul_fwd, "tri_mul_fwd"); get(api.mul_bwd, "tri_mul_bwd");
 }
@@ -538,8 +538,9 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
     const int64_t W = H * D, N = o_w.size(0);
     const Tensor gated = at::empty({BM, U, W}, s.options()), out = at::empty({BM, U, N}, s.options());
     const tri_stream_t st = stream_of(s);
-    ok(api.gated_linear(dtype_code(s), BM * U, (int32_t)s.size(2), (int32_t)W, (int32_t)N, ptr(s), ptr(g_w), ptr(o), ptr(o_w), ptr(gated), ptr(out),
-                        ptr(status), st), "tri_gated_linear");
+    // (nothing is queued between the attention, which wrote o, and this: o is its output as it came, s and the weights the caller's)
+    ok(api.gated_linear_after(dtype_code(s), BM * U, (int32_t)s.size(2), (int32_t)W, (int32_t)N, ptr(s), ptr(g_w), ptr(o), ptr(o_w), ptr(gated),
+                              ptr(out), ptr(status), st), "tri_gated_linear_after");
     check_device(status, reinterpret_cast<cudaStream_t>(st));
     return {out, pz};
   }

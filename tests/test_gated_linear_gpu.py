@@ -34,6 +34,69 @@ def test_gated_linear(dtype, M, K, W, N):
     assert float((out[:M].double() - ref).norm() / ref.norm()) <= limit
 
 
+def _operands(M, W, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rn = lambda *s, sc=1.0: (torch.randn(*s, generator=g, device="cuda") * sc).to(dtype)  # noqa: E731
+    return rn(M, W), rn(M, W), rn(W, W, sc=W ** -0.5), rn(W, W, sc=3 * W ** -0.5)
+
+
+def _call(f, M, W, s, wg, o, wo, gated, out, status):
+    from geometric_nn_ops_b200 import _lib
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(f(_lib.BF16, M, W, W, W, p(s), p(wg), p(o), p(wo), p(gated), p(out), p(status),
+                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "tri_gated_linear")
+
+
+@pytest.mark.parametrize("M,W", [(128, 256), (2048, 768), (9000, 256)])
+def test_chained_calls(M, W):
+    """s is what the call before wrote: nothing of it is read before that call is done."""
+    from geometric_nn_ops_b200 import _lib
+    f = _lib.load().tri_gated_linear
+    s, o, wg, wo = _operands(M, W)
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+
+    def chain(wait):
+        bufs = [torch.full_like(s, float("nan")) for _ in range(8)]
+        gated = [torch.empty_like(o) for _ in range(8)]
+        torch.cuda.synchronize()
+        x = s
+        for out, scratch in zip(bufs, gated):
+            _call(f, M, W, x, wg, o, wo, scratch, out, status)
+            if wait:
+                torch.cuda.synchronize()
+            x = out
+        torch.cuda.synchronize()
+        return bufs
+
+    want = chain(True)
+    for _ in range(20):
+        for got, ref in zip(chain(False), want):
+            assert torch.equal(got, ref)
+    assert int(status[0]) == 0
+
+
+def test_behind_the_call_that_wrote_o():
+    """The early form: o is what the call before wrote, s and the weights are older."""
+    from geometric_nn_ops_b200 import _lib
+    lib, M, W = _lib.load(), 2048, 768
+    s, o, wg, wo = _operands(M, W)
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    mid, out, g1, g2 = (torch.full_like(s, float("nan")) for _ in range(4))
+    want = torch.empty_like(out)
+    _call(lib.tri_gated_linear, M, W, s, wg, o, wo, g1, mid, status)
+    torch.cuda.synchronize()
+    _call(lib.tri_gated_linear, M, W, s, wg, mid, wo, g2, want, status)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        mid.fill_(float("nan"))
+        out.fill_(float("nan"))
+        _call(lib.tri_gated_linear, M, W, s, wg, o, wo, g1, mid, status)
+        _call(lib.tri_gated_linear_after, M, W, s, wg, mid, wo, g2, out, status)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert int(status[0]) == 0
+
+
 def test_refusals():
     from geometric_nn_ops_b200 import _lib
     t = torch.zeros(64, dtype=torch.bfloat16, device="cuda")
