@@ -550,6 +550,7 @@ int tri_bgemm(const TriGemmDesc* d, const void* a, const void* b, void* c, void*
   p.b[0].batch = d->batch; p.b[0].st_outer = d->ldb; p.b[0].st_batch = d->batch_b;
   p.M = d->M; p.N = d->N; p.K0 = d->K; p.batches = d->batch;
   p.out0 = c; p.ld_out = d->ldc; p.batch_out = d->batch_c;
+  p.first = true;
   p.name = "tc_bgemm";
   p.flops = 2.0 * d->batch * d->M * (double)d->N * d->K;
   const double es = d->dtype == TRI_F32 ? 4.0 : 2.0;

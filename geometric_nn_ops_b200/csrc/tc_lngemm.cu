@@ -344,7 +344,7 @@ int launch(cudaStream_t st, const LnGateIn& p) {
   const int grid = std::min(a.tiles, sm_count());
   const double bytes = 4.0 * p.M * 128 * 2;
   KernelTimer kt("tc_ln_gate_in", st, 2.0 * p.M * 128 * 512, bytes);
-  launch_dependent(us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmX, tmW, tmZ, tmA, tmB, a);
+  launch_dependent(p.first ? kLaunchPlainly : us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmX, tmW, tmZ, tmA, tmB, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -674,7 +674,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   const int grid = std::min(a.tiles, sm_count());
   const double bytes = (p.u_cm ? 4.0 : 3.0) * p.M * 128 * 2;
   KernelTimer kt("tc_ln_gate_out", st, 2.0 * p.M * 128 * 256, bytes);
-  launch_dependent(us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmT, tmZ, tmWo, tmWg, a);
+  launch_dependent(p.first ? kLaunchPlainly : us_of_bytes(bytes), kern, grid, kThreads, smem, st, tmT, tmZ, tmWo, tmWg, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -934,7 +934,7 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   const int grid = G::kHalves == 2 ? std::min(a.tiles, sm_count()) : 2 * std::min(a.tiles, sm_count() / 2);
   const double bytes = 7.0 * p.M * 128 * E;
   KernelTimer kt("tc_gate_in_bwd", st, 0.0, bytes);
-  launch_dependent(us_of_bytes(bytes), kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
+  launch_dependent(p.first ? kLaunchPlainly : us_of_bytes(bytes), kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
   TRI_LAUNCH_OK();
   return 0;
 }

@@ -45,6 +45,7 @@ struct LnGateIn {
   float* rstd;               // [M]
   void* a_cm;                // [B, 128, plane]
   void* b_cm;
+  bool first = false;        // no kernel of this call came before: launched plainly
   int* err;                  // device status word (zeroed by the caller)
 };
 
@@ -69,6 +70,7 @@ struct LnGateOut {
   const void* residual = nullptr;   // [M, 128], added to the (rounded) result, or null
   int n = 0, pitch = 0;      // n > 0: the pixels [pitch, pitch] hold [n, n], t is zero beyond
   bool own_pitch = false;    // out is [n, n, 128] (no residual) and not [M, 128]
+  bool first = false;        // as above
   int* err;
 };
 
@@ -87,6 +89,7 @@ struct GateInBwd {
   const void* da_cm;         // [128, M]
   const void* db_cm;
   void* dpg;                 // [512, M]: rows [dP_a; dG_a; dP_b; dG_b]
+  bool first = false;        // as above
   int* err;
 };
 bool gate_in_bwd_supported(int dtype, long long M, long long plane);

@@ -490,7 +490,12 @@ struct Geom {
   double unit() const { return (double)M * CW * es(); }
 };
 
-struct Prep { int* err; void* wcat; float* bias_cat; float* bias_out; };
+struct Prep {
+  int* err;
+  void* wcat;
+  float *bias_cat, *bias_out;
+  bool first = false;   // the weights were prepared by an earlier call: the phase's first kernel is the call's
+};
 
 void carve_prep_weights(Arena& a, size_t es, Prep* p) {
   p->wcat = a.take<char>(4 * CW * CW * es);
@@ -541,9 +546,10 @@ int contraction(cudaStream_t st, int dtype, int planes, int n, const void* a, bo
 }
 
 template <typename T>
-int run_prep(cudaStream_t st, const TriMulWeights* w, const Prep& pr, bool weights_ready = false) {
+int run_prep(cudaStream_t st, const TriMulWeights* w, Prep& pr, bool weights_ready = false) {
   if (weights_ready) {   // the caller kept the prepared weights of an earlier phase of the same call
     TRI_CUDA_OK(cudaMemsetAsync(pr.err, 0, 256, st));
+    pr.first = true;
     return 0;
   }
   KernelTimer kt("tc_prep_weights", st, 0.0, 0.0);
@@ -579,7 +585,7 @@ int phase_project(cudaStream_t st, const Geom& gm, const void* x, const void* ma
     f.dtype = gm.dtype; f.M = M; f.plane = gm.plane; f.eps = gm.eps;
     f.x = x; f.gamma = w->norm_in_w; f.beta = w->norm_in_b; f.wcat = pr.wcat;
     f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr; f.mask = mask;
-    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.err = pr.err;
+    f.z = z; f.mean = mean_in; f.rstd = rstd_in; f.a_cm = a_cm; f.b_cm = b_cm; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.first = pr.first; f.err = pr.err;
     return ln_gate_in(st, f);
   }
   {
@@ -609,7 +615,7 @@ int phase_output(cudaStream_t st, const Geom& gm, const void* t_cm, const void* 
     f.dtype = gm.dtype; f.M = M; f.eps = gm.eps; f.t_cm = t_cm; f.z = z;
     f.gamma = w->norm_out_w; f.beta = w->norm_out_b; f.w_out = w->p_out_w; f.w_gate = w->g_out_w;
     f.bias_out = (w->p_out_b || w->g_out_b) ? pr.bias_out : nullptr;
-    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.err = pr.err;
+    f.u_cm = keep_u ? u : nullptr; f.mean = mean_out; f.rstd = rstd_out; f.out = out; f.residual = residual; f.n = gm.n; f.pitch = gm.pitch; f.own_pitch = own_pitch; f.first = pr.first; f.err = pr.err;
     return ln_gate_out(st, f);
   }
   {
@@ -721,6 +727,7 @@ int phase_output_bwd(cudaStream_t st, const Geom& gm, const void* d_out, const v
     p.b[1] = rows_operand(w->g_out_w, CW, CW, false);
     p.M = (int)M; p.N = CW; p.K0 = CW; p.K1 = CW; p.seg1_col = CW;
     p.out0 = dy; p.out1 = dgo; p.aux = d_out; p.bias0 = (w->p_out_b || w->g_out_b) ? pr.bias_out : nullptr;
+    p.first = pr.first;
     p.name = "tc_gemm_gate_out_bwd"; p.flops = 0.0; p.bytes = 5.0 * gm.unit();  // recompute: no algorithmic flops
     TRI_TRY(launch_gemm(st, gm.dtype, EPI_GATE_OUT_BWD, 256, false, p, pr.err));
   }
@@ -788,13 +795,13 @@ int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void
   if (gate_in_bwd_supported(gm.dtype, M, gm.plane) && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) {
     GateInBwd f;
     f.dtype = gm.dtype; f.M = M; f.z = z; f.wcat = pr.wcat; f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr;
-    f.mask = mask; f.da_cm = da_cm; f.db_cm = db_cm; f.dpg = dpg; f.err = pr.err;
+    f.mask = mask; f.da_cm = da_cm; f.db_cm = db_cm; f.dpg = dpg; f.first = pr.first; f.err = pr.err;
     TRI_TRY(gate_in_bwd(st, f));
   } else {
     GemmPlan p;   // input gate backward fused into the recomputed projection GEMM
     gate_in_operands(&p, gm, pr, z);
     p.out0 = dpg; p.ld_out = M; p.bias0 = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr;
-    p.aux = mask; p.aux2 = da_cm; p.aux3 = db_cm; p.plane = gm.plane;
+    p.aux = mask; p.aux2 = da_cm; p.aux3 = db_cm; p.plane = gm.plane; p.first = pr.first;
     p.name = "tc_gemm_gate_in_bwd"; p.flops = 0.0; p.bytes = 7.0 * gm.unit();
     TRI_TRY(launch_gemm(st, gm.dtype, EPI_GATE_IN_BWD, 256, false, p, pr.err));
   }
