@@ -94,7 +94,8 @@ static int check_mul(const TriMulDesc* d) {
 }
 
 // What the tensor-core attention kernels need beyond the descriptor: q, k, v and dO, which they reach through tensor
-// maps, start on a 16-byte boundary, and so do the results, which they write (and read back) in 16-byte pieces.  Anything else
+// maps, start on a 16-byte boundary, and so do the results, which they write (and read back) in 16-byte pieces.  The workspace holds
+// operands of tensor maps and bulk copies (16 bytes), and the 16-bit backward stores 32-byte sectors into it.  Anything else
 // runs on the CUDA-core kernels, which take any pointer and stride.
 static bool aligned_to(size_t bytes, std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)
@@ -169,11 +170,11 @@ int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void*
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_bytes, tri_stream_t stream) {
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse) return fail(TRI_ERR_ARG, "q, k, v, o and lse must not be null");
-  if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o}) && tc::attn_bias_has_room(d, bias, ws_bytes, 0)) {
+  if (tc::attn_fwd_supported(d) && aligned_to(16, {q, k, v, o, ws}) && tc::attn_bias_has_room(d, bias, ws_bytes, 0)) {
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
-  if (tc::attn_tf32_supported(d, 0) && aligned_to(16, {q, k, v, o}) && ws != nullptr && ws_bytes >= tc::attn_tf32_ws_bytes(d, 0)) {
+  if (tc::attn_tf32_supported(d, 0) && aligned_to(16, {q, k, v, o, ws}) && ws != nullptr && ws_bytes >= tc::attn_tf32_ws_bytes(d, 0)) {
     set_path("tcgen05");
     return tc::attn_tf32_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -187,12 +188,12 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse || !d_o || !dq || !dk || !dv || !ws)
     return fail(TRI_ERR_ARG, "q, k, v, o, lse, d_o, dq, dk, dv and ws must not be null");
-  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias}) && tc::attn_bias_has_room(d, bias, ws_bytes, 1)) {
+  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias}) && aligned_to(32, {ws}) && tc::attn_bias_has_room(d, bias, ws_bytes, 1)) {
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);
   }
-  if (tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
+  if (tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, ws}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
     set_path("tcgen05");
     return tc::attn_tf32_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes, (cudaStream_t)stream);
   }

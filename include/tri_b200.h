@@ -17,8 +17,9 @@
  *    tri_last_error() returns a thread-local message for the last failure.
  *  - Strides are in ELEMENTS.  The innermost (head-dim / channel) axis is
  *    always contiguous.
- *  - Attention takes any alignment (tensors off a 16-byte boundary run on the
- *    CUDA-core kernels).  The multiplicative update on the tensor cores wants
+ *  - Attention takes any alignment (tensors off a 16-byte boundary, or a ws off
+ *    a 32-byte boundary, run on the CUDA-core kernels; there ws is on a 4-byte
+ *    boundary at least).  The multiplicative update on the tensor cores wants
  *    x, out, d_out, dx, the weights, saved and ws on 16-byte boundaries, and
  *    returns TRI_ERR_ARG otherwise.
  */

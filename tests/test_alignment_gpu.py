@@ -80,3 +80,38 @@ def test_update_refuses_results_off_16_bytes():
     assert call(_at(torch.empty_like(x), 4)) == -1 and b"16-byte" in lib.tri_last_error()
     assert call(_at(torch.empty_like(x), 8)) == 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype,precision,S,N,offset,paths", [
+    (torch.bfloat16, "ieee", 4, 136, 0, ["tcgen05", "tcgen05"]), (torch.bfloat16, "ieee", 4, 136, 16, ["tcgen05", "simt"]),
+    (torch.bfloat16, "ieee", 4, 136, 8, ["simt", "simt"]), (torch.bfloat16, "ieee", 4, 136, 4, ["simt", "simt"]),
+    (torch.float32, "tf32", 80, 256, 16, ["tcgen05", "tcgen05"]), (torch.float32, "tf32", 80, 256, 4, ["simt", "simt"])],
+    ids=lambda v: str(v).replace("torch.", "") if not isinstance(v, list) else "-".join(v))
+def test_attention_workspace_off_its_boundary(dtype, precision, S, N, offset, paths):
+    """A workspace that the tensor-core kernels cannot use is served by the CUDA-core kernels."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import _triattn, triangle_attention
+    lib, H = _lib.load(), 4
+    t, mask, d_o = util.attn_inputs(1, S, N, H, 32, dtype, seed=2)
+    with util.matmul_precision(precision):
+        want, g_want = util.attn_fwd_bwd(triangle_attention, t, mask, None, d_o)
+    q, k, v, bias = t["q"], t["k"], t["v"], t["bias"]
+    m = mask.reshape(1, S, N).contiguous().view(torch.uint8)
+    o, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+    dbias, lse = torch.empty(1, H, N, N, device="cuda"), torch.empty(2, 1, S, H, N, device="cuda")
+    d = _triattn._desc(q, k, v, o, bias, m, 32 ** -0.5, precision)
+    d.do_st = d.dq_st = d.dk_st = d.dv_st = _triattn._st4(q)
+    n = max(lib.tri_attn_ws_bytes(ctypes.byref(d), b) for b in (0, 1))
+    ws = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    assert ws.data_ptr() % 32 == 0
+    at, stream = ctypes.c_void_p(ws.data_ptr() + offset), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(lib.tri_attn_fwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(bias), _p(m), _p(o), _p(lse), at, n, stream), "fwd")
+    path = [_lib.last_path()]
+    _lib.check(lib.tri_attn_bwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(bias), _p(m), _p(o), _p(lse), _p(d_o), _p(dq), _p(dk), _p(dv),
+                                _p(dbias), at, n, stream), "bwd")
+    torch.cuda.synchronize()
+    assert path + [_lib.last_path()] == paths
+    cos_min, fro = util.ATTN_TOL[dtype, precision]
+    for name, got, ref in (("out", o, want.detach()), ("dq", dq, g_want["q"]), ("dk", dk, g_want["k"]), ("dv", dv, g_want["v"]),
+                           ("dbias", dbias, g_want["bias"].reshape(dbias.shape))):
+        util.check_close(name, got, util.f64(ref), cos_min, fro)
