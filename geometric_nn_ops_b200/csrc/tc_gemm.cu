@@ -168,6 +168,8 @@ int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const
     TRI_TRY(make_tmap(&g.tmDx, p.out0, dtype, 3, dims, str, box, 128));
     g.gamma = p.gamma; g.mean = p.mean; g.rstd = p.rstd; g.sum_g = p.sum_g; g.sum_b = p.sum_b;
   }
+  auto on = [](const void* q, int bytes) { return reinterpret_cast<uintptr_t>(q) % bytes == 0; };
+  g.wide = on(p.out0, 32) && on(p.out1, 32) && on(p.aux2, 32) && on(p.aux3, 32);
   g.peer_world = 0; g.peer_rank = 0; g.peer_cs = 128; g.peer_batches = 0;
   for (int i = 0; i < 16; ++i) g.peer_out[i] = nullptr;
   if (p.peer_out != nullptr && p.peer_world > 1) {
@@ -175,7 +177,8 @@ int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const
       return fail(TRI_ERR_ARG, "peer outputs need the gate-in epilogue and a rank count that divides 128 (at most 16)");
     g.peer_world = p.peer_world; g.peer_rank = p.peer_rank; g.peer_cs = 128 / p.peer_world; g.peer_batches = p.peer_batches;
     for (int i = 0; i < p.peer_world; ++i) {
-      if (p.peer_out[i] == nullptr) return fail(TRI_ERR_ARG, "null peer output buffer");
+      if (p.peer_out[i] == nullptr || !on(p.peer_out[i], 16)) return fail(TRI_ERR_ARG, "a peer output buffer is null or off a 16-byte boundary");
+      g.wide = g.wide && on(p.peer_out[i], 32);
       g.peer_out[i] = p.peer_out[i];
     }
   }

@@ -82,6 +82,7 @@ struct GemmArgs {
   const void* aux2;              // GATE_IN_BWD: channel-major gradient of the a half
   const void* aux3;              //              ... of the b half
   long long plane;               // GATE_IN(_BWD): pixels per batch entry; channel-major plane stride
+  bool wide;                     // out0, out1, aux2, aux3 and the peers' buffers start on 32-byte boundaries
   // GATE_IN with peer_world > 0: channel c of half tm goes to GPU c / peer_cs, into its buffer
   // [2 * peer_batches][peer_cs][peer_world][plane] at (tm * peer_batches + batch, c % peer_cs, peer_rank)
   void* peer_out[16];
@@ -750,7 +751,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         const TIN* dplane = reinterpret_cast<const TIN*>(tm == 0 ? g.aux2 : g.aux3);
         const uint32_t t0 = (uint32_t)tn * 128, plane = (uint32_t)g.plane, tb0 = t0 / plane, tp0 = t0 - tb0 * plane;
         const TIN* base = dplane + ((long long)tb0 * 128 + row) * g.plane + tp0;
-        const bool wide = sizeof(TIN) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0;   // 16-pixel groups: aligned, never split
+        const bool wide = sizeof(TIN) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0 && g.wide;   // 16-pixel groups: aligned, never split
 #pragma unroll
         for (int jj = 0; jj < CPG; ++jj)
 #pragma unroll
@@ -838,7 +839,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       } else if constexpr (EPI == EPI_GATE_IN || EPI == EPI_GATE_IN_BWD) {
         // row = channel of half tm; columns: P for pixels n0..n0+127, then G for the same pixels
         const uint32_t n0 = (uint32_t)tn * 128, plane = (uint32_t)g.plane, np0 = n0 % plane;
-        const bool wide16 = sizeof(TOUT) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0 && (g.ld_out & 15) == 0;
+        const bool wide16 = sizeof(TOUT) == 2 && (g.plane & 15) == 0 && (g.N & 15) == 0 && (g.ld_out & 15) == 0 && g.wide;
         // fp32: 16 pixels of four channels, exchanged between four lanes (64 bytes of eight rows per request, not 16 of 32)
         const bool wide4 = EPI == EPI_GATE_IN && sizeof(TOUT) == 4 && (g.plane & 15) == 0 && (g.N & 15) == 0 && g.peer_world == 0;
         const TIN* mask = reinterpret_cast<const TIN*>(g.aux);
@@ -959,18 +960,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                   }
                 }
               }
-              // 16 channels of this pixel: one 32-byte store for 16-bit outputs (rows are 256 bytes; two where the caller's tensor
-              // starts between them).  fp32: four lanes exchange their pieces, so that a request covers 64 bytes of eight rows and not 16 of 32
+              // 16 channels of this pixel: one 32-byte store for 16-bit outputs (two where the tensors start between).  fp32: four lanes exchange their pieces, so that a request covers 64 bytes of eight rows and not 16 of 32
               if constexpr (sizeof(TOUT) == 2) {
                 if (m < g.M) {
                   TOUT* at = o0 + j * 32 + hf * 16;
-                  if (EPI == EPI_GATE_OUT_BWD || (reinterpret_cast<uintptr_t>(at) & 31) == 0) {
+                  TOUT* at1 = o1 + j * 32 + hf * 16;
+                  if (g.wide) {
                     store16<TOUT>(at, r0);
+                    if constexpr (EPI == EPI_GATE_OUT_BWD) store16<TOUT>(at1, r1);
                   } else {
                     store8<TOUT>(at, r0);
                     store8<TOUT>(at + 8, r0 + 8);
+                    if constexpr (EPI == EPI_GATE_OUT_BWD) { store8<TOUT>(at1, r1); store8<TOUT>(at1 + 8, r1 + 8); }
                   }
-                  if constexpr (EPI == EPI_GATE_OUT_BWD) store16<TOUT>(o1 + j * 32 + hf * 16, r1);
                 }
               } else {
                 store_rows4(reinterpret_cast<float*>(g.out0), r0, m, g.M, j * 32 + hf * 16, lane);

@@ -115,3 +115,34 @@ def test_attention_workspace_off_its_boundary(dtype, precision, S, N, offset, pa
     for name, got, ref in (("out", o, want.detach()), ("dq", dq, g_want["q"]), ("dk", dk, g_want["k"]), ("dv", dv, g_want["v"]),
                            ("dbias", dbias, g_want["bias"].reshape(dbias.shape))):
         util.check_close(name, got, util.f64(ref), cos_min, fro)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=str)
+@pytest.mark.parametrize("B,n", [(1, 64), (2, 32), (1, 43)])
+def test_update_scratch_on_16_but_not_32_bytes(B, n, dtype):
+    """ws and the saved block hold the gradients that the gate epilogues read and write in wide pieces."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle._trimul import _DTYPES
+    lib = _lib.load()
+    x, mask, w, d_out = util.trimul_inputs(B, n, 128, 128, dtype, seed=n)
+    d = _lib.TriMulDesc(B, n, 128, 128, _DTYPES[dtype], _lib.PREC_TF32 if dtype == torch.float32 else _lib.PREC_IEEE, _lib.OUTGOING, 1e-5)
+    wp = _lib.TriMulWeights(**{_lib.abi_field(k): t.data_ptr() for k, t in w.items()})
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sizes = [lib.tri_mul_saved_bytes(ctypes.byref(d)), lib.tri_mul_ws_bytes(ctypes.byref(d), 0), lib.tri_mul_ws_bytes(ctypes.byref(d), 1)]
+
+    def call(offset):
+        saved, ws, ws_bwd = (torch.zeros(s + 64, dtype=torch.uint8, device="cuda") for s in sizes)
+        at = [ctypes.c_void_p(t.data_ptr() + offset) for t in (saved, ws, ws_bwd)]
+        out, dx = torch.empty_like(x), torch.empty_like(x)
+        grads = {k: torch.empty(t.shape, device="cuda") for k, t in w.items()}
+        g = _lib.TriMulWeightGrads(**{_lib.abi_field(k): t.data_ptr() for k, t in grads.items()})
+        _lib.check(lib.tri_mul_fwd(ctypes.byref(d), _p(x), _p(mask), ctypes.byref(wp), _p(out), at[0], at[1], sizes[1], stream), "fwd")
+        _lib.check(lib.tri_mul_bwd(ctypes.byref(d), _p(x), _p(mask), ctypes.byref(wp), at[0], _p(d_out), _p(dx), ctypes.byref(g), at[2], sizes[2],
+                                   stream), "bwd")
+        torch.cuda.synchronize()
+        assert all(int(t[sizes[i] + offset:].sum()) == 0 and int(t[:offset].sum()) == 0 for i, t in enumerate((saved, ws, ws_bwd)))
+        return {"out": out, "dx": dx, **grads}
+
+    want, got = call(0), call(16)
+    for name in want:
+        assert torch.equal(got[name], want[name]), name
