@@ -136,6 +136,9 @@ template <typename T>
 int project_t(const TriAttnProjDesc* d, const void* z, const void* ln_w, const void* ln_b, const void* w_qkv,
               const void* w_bias, void* qkv, void* bias, void* ws, cudaStream_t st) {
   const long long M = d->M;
+  // (w_bias: the four-head form reads it in pieces)
+  for (const void* p : {z, ln_w, ln_b, w_qkv, static_cast<const void*>(ws), d->H == 4 ? w_bias : nullptr})
+    if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return fail(TRI_ERR_ARG, "the fused projection needs tensors that start on 16-byte boundaries");
   int* err = static_cast<int*>(ws);
   void* zn = static_cast<char*>(ws) + 256;
   TRI_CUDA_OK(cudaMemsetAsync(ws, 0, 256, st));

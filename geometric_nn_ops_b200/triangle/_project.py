@@ -16,6 +16,7 @@ import torch
 
 from .. import _lib, _precision
 from ._triattn import _DTYPES
+from ._trimul import _aligned
 
 
 def attention_input_projection(z, w_qkv, w_bias, heads, ln_weight=None, ln_bias=None, eps=1e-5):
@@ -43,7 +44,7 @@ def attention_input_projection(z, w_qkv, w_bias, heads, ln_weight=None, ln_bias=
     ws_bytes = lib.tri_attn_project_ws_bytes(ctypes.byref(d))
     if ws_bytes == 0:
         raise RuntimeError("attention_input_projection: " + lib.tri_last_error().decode(errors="replace"))
-    cv = lambda t: None if t is None else t.detach().to(z.dtype).contiguous()  # noqa: E731
+    cv = lambda t: None if t is None else _aligned(t.detach().to(z.dtype))  # noqa: E731
     zc, wq, wb, lw, lb = cv(z), cv(w_qkv), cv(w_bias), cv(ln_weight), cv(ln_bias)
     qkv = torch.empty(B, R, N, 3, heads, D, dtype=z.dtype, device=z.device)
     bias = torch.empty(heads, B, R, N, dtype=z.dtype, device=z.device)

@@ -133,7 +133,8 @@ int tri_attn_bwd_noalloc(const TriAttnDesc* d, const void* q, const void* k, con
  * No counterpart in the reference, whose attention takes pre-projected tensors
  * (geometric_nn_ops_torch/triangle/_triattn.py:36-44); callers there run a LayerNorm, four linears and a permute.
  * z: [M, C] contiguous, C = 128; ln_w / ln_b: [C] or NULL; w_qkv: [3*H*D, C]; w_bias: [H, C], H <= 8; everything in
- * `dtype` (fp32 needs precision tf32: tensor-core path only).  Forward only. */
+ * `dtype` (fp32 needs precision tf32: tensor-core path only).  z, the weights, qkv and ws start on 16-byte boundaries (else
+ * TRI_ERR_ARG).  Forward only. */
 typedef struct TriAttnProjDesc {
   int64_t M;
   int32_t C, H, D;

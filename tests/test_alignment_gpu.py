@@ -146,3 +146,31 @@ def test_update_scratch_on_16_but_not_32_bytes(B, n, dtype):
     want, got = call(0), call(16)
     for name in want:
         assert torch.equal(got[name], want[name]), name
+
+
+@pytest.mark.parametrize("dtype,H,D", [(torch.float32, 4, 32), (torch.float32, 3, 16), (torch.bfloat16, 4, 32), (torch.bfloat16, 8, 32)], ids=str)
+def test_projection_of_views_off_16_bytes(dtype, H, D):
+    """z and weights that are views into a flat buffer: copied by the Python entry, refused by the C entry before a launch."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import attention_input_projection
+    g = torch.Generator().manual_seed(H)
+    rn = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()  # noqa: E731
+    args = [rn(1, 5, 40, 128), rn(3 * H * D, 128), rn(H, 128), rn(128), rn(128)]
+    call = lambda z, wq, wb, lw, lb: attention_input_projection(z, wq, wb, H, lw, lb)  # noqa: E731
+    with util.matmul_precision("tf32"), torch.no_grad():
+        want = call(*args)
+        for got, ref in zip(call(*(_at(t, 1) for t in args)), want):
+            assert torch.equal(got, ref)
+    if dtype == torch.bfloat16 and H == 4:
+        return      # the one-kernel form: its norm weights are read one at a time
+    z, wq, wb, lw, lb = args
+    d = _lib.TriAttnProjDesc(200, 128, H, D, _lib.F32 if dtype == torch.float32 else _lib.BF16, _lib.PREC_TF32, 1e-5)
+    n = _lib.load().tri_attn_project_ws_bytes(ctypes.byref(d))
+    ws = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    qkv, bias = torch.empty(200, 3 * H * D, dtype=dtype, device="cuda"), torch.empty(H, 200, dtype=dtype, device="cuda")
+    before = _lib.launch_count()
+    for i in range(5):
+        p = [_p(_at(t, 1) if j == i else t) for j, t in enumerate((z, lw, lb, wq))]
+        at = ctypes.c_void_p(ws.data_ptr() + (4 if i == 4 else 0))
+        assert _lib.load().tri_attn_project(ctypes.byref(d), *p, _p(wb), _p(qkv), _p(bias), at, n, None) == -1
+    assert _lib.launch_count() == before
