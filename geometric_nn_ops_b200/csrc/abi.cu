@@ -336,6 +336,28 @@ static int check_shard(const TriMulShardDesc* d) {
   return 0;
 }
 
+// What a phase reads or writes in pieces, as for the whole update (the peers' buffers: launch_gemm).
+static int check_shard_alignment(const TriMulShardDesc* d, int phase, const TriMulShardBufs* b, const void* ws) {
+  const bool peers = b->peer_ab != nullptr && b->peer_world > 1, f32 = d->dtype == TRI_F32;
+  bool ok = aligned_to(16, {b->saved, b->prep, ws});
+  switch (phase) {
+    case TRI_PHASE_PROJECT:   // (16-bit types read the norm weights and the mask one at a time, unless the epilogue stores to peers)
+      ok = ok && aligned_to(16, {b->x, peers ? nullptr : b->a_cm, peers ? nullptr : b->b_cm}) &&
+           ((!f32 && !peers) || aligned_to(16, {b->w->norm_in_w, b->w->norm_in_b, b->mask}));
+      break;
+    case TRI_PHASE_OUTPUT:
+      ok = ok && aligned_to(16, {b->t_cm, b->out}) && aligned_to(f32 ? 16 : d->B > 1 ? 8 : 1, {b->w->norm_out_w, b->w->norm_out_b});
+      break;
+    case TRI_PHASE_OUTPUT_BWD:
+      ok = ok && aligned_to(16, {b->d_out, b->t_cm, b->dt_cm}) && (d->B == 1 || aligned_to(f32 ? 16 : 8, {b->w->norm_out_w}));
+      break;
+    case TRI_PHASE_PROJECT_BWD:
+      ok = ok && aligned_to(16, {b->x, b->mask, b->a_cm, b->b_cm, b->dx});
+      break;
+  }
+  return ok ? 0 : fail(TRI_ERR_ARG, "the phases of the sharded update need tensors that start on 16-byte boundaries");
+}
+
 size_t tri_mul_shard_saved_bytes(const TriMulShardDesc* d) {
   return check_shard(d) != 0 ? 0 : tc::mul_shard_saved_bytes(d);
 }
@@ -353,6 +375,7 @@ int tri_mul_shard_phase(const TriMulShardDesc* d, int phase, const TriMulShardBu
   TRI_TRY(check_shard(d));
   if (!bufs || !bufs->w || !bufs->saved || !ws) return fail(TRI_ERR_ARG, "bufs, weights, saved and ws must not be null");
   TRI_TRY(check_mul_weights(bufs->w));
+  TRI_TRY(check_shard_alignment(d, phase, bufs, ws));
   set_path("tcgen05");
   return tc::mul_shard_phase(d, phase, bufs, ws, ws_bytes, (cudaStream_t)stream);
 }

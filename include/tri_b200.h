@@ -230,7 +230,8 @@ int tri_mul_bwd(const TriMulDesc* d, const void* x, const void* mask, const TriM
  *   PROJECT_BWD  gradients da, db passed in a_cm, b_cm -> dx, gradients of norm_in / p_in / g_in (partial)
  * `saved` (tri_mul_shard_saved_bytes) carries z, u, dgo and the LayerNorm statistics between phases.
  * Weight gradients are per-rank partial sums: all-reduce them.  Tensor-core path only
- * (C = Ch = 128, N % 8 == 0, bf16 / fp16, or fp32 with precision tf32). */
+ * (C = Ch = 128, N % 8 == 0, bf16 / fp16, or fp32 with precision tf32).  Tensors, weights, saved, prep and ws start on 16-byte
+ * boundaries, as for the whole update. */
 typedef struct TriMulShardDesc {
   int32_t B, rows, N, C, Ch;
   int32_t dtype, precision;

@@ -42,6 +42,31 @@ class _Shard:
         self.bufs.prep_ready = 1     # every later phase is a call whose first kernel is the phase's own
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=str)
+def test_tensors_off_16_bytes_are_refused(dtype):
+    from geometric_nn_ops_b200 import _lib
+    x, mask, w, d_out = util.trimul_inputs(1, 32, 128, 128, dtype, seed=1)
+    s = _Shard(x[:, :16].contiguous(), mask[:, :16].contiguous(), w, _lib.PREC_TF32)
+    room = torch.zeros(1 << 24, dtype=torch.uint8, device="cuda")
+    launches = _lib.launch_count()
+    names = {_lib.PHASE_PROJECT: ["x", "saved", "prep", "a_cm", "b_cm"] + (["mask"] if dtype == torch.float32 else []),
+             _lib.PHASE_OUTPUT: ["saved", "t_cm", "out"], _lib.PHASE_OUTPUT_BWD: ["saved", "t_cm", "d_out", "dt_cm"],
+             _lib.PHASE_PROJECT_BWD: ["x", "mask", "saved", "a_cm", "b_cm", "dx"]}
+    for name in ("a_cm", "b_cm", "t_cm", "out", "d_out", "dt_cm", "dx"):
+        setattr(s.bufs, name, room.data_ptr())
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for phase, tensors in names.items():
+        for name in tensors + ["ws"]:
+            aligned, off = (0, 8) if name == "ws" else (getattr(s.bufs, name), 0)
+            if name != "ws":
+                setattr(s.bufs, name, aligned + 8)
+            at = ctypes.c_void_p(room.data_ptr() + off)
+            assert s.lib.tri_mul_shard_phase(ctypes.byref(s.d), phase, ctypes.byref(s.bufs), at, room.numel() - 16, stream) == -1, (phase, name)
+            if name != "ws":
+                setattr(s.bufs, name, aligned)
+    assert _lib.launch_count() == launches
+
+
 @pytest.mark.parametrize("direction", ["outgoing", "incoming"])
 @pytest.mark.parametrize("dtype,precision,B,n", [(torch.bfloat16, "ieee", 1, 64), (torch.float16, "ieee", 2, 48), (torch.float32, "tf32", 1, 48),
                                                  (torch.bfloat16, "ieee", 1, 264)], ids=lambda v: str(v).replace("torch.", ""))
