@@ -418,9 +418,11 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         early_s = mbar_test(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1);
         early_b = mbar_test(&b_full[bstg + 1 == kBiasStages ? 0 : bstg + 1], bstg + 1 == kBiasStages ? bph ^ 1 : bph);
         // (fp32: the rest of P has one buffer, and P V of the step before reads it; its commit is the next step's S)
-        if (M::F32 && c > 0 && !early_s) {
-          early_s = mbar_wait(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1, a.err, 58);
-          ok = early_s && ok;
+        if (M::F32 && c > 0) {
+          if (!early_s) {
+            early_s = mbar_wait(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1, a.err, 58);
+            ok = early_s && ok;
+          }
           tc_fence_after_sync();
         }
         float sum = ps.x + ps.y;
