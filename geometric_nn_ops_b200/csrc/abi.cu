@@ -188,12 +188,13 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
   TRI_TRY(check_attn(d));
   if (!q || !k || !v || !o || !lse || !d_o || !dq || !dk || !dv || !ws)
     return fail(TRI_ERR_ARG, "q, k, v, o, lse, d_o, dq, dk, dv and ws must not be null");
-  if (tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias}) && aligned_to(32, {ws}) && tc::attn_bias_has_room(d, bias, ws_bytes, 1)) {
+  const bool tensor_cores = dbias == nullptr || bias != nullptr;   // (their dbias passes read the bias)
+  if (tensor_cores && tc::attn_bwd_supported(d) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, dbias}) && aligned_to(32, {ws}) && tc::attn_bias_has_room(d, bias, ws_bytes, 1)) {
     set_path("tcgen05");
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);
   }
-  if (tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, ws}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
+  if (tensor_cores && tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, ws}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
     set_path("tcgen05");
     return tc::attn_tf32_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes, (cudaStream_t)stream);
   }

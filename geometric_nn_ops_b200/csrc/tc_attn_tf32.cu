@@ -850,7 +850,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     TRI_LAUNCH_OK();
   }
   // ---- dbias ------------------------------------------------------------------------------------
-  if (dbias != nullptr && bias != nullptr) {
+  if (dbias != nullptr) {
     const long long combos = (long long)blocks * nq * d->B * d->H;
     int chunks = 1;
     long long best = -1;

@@ -78,7 +78,7 @@ int tri_profile_summary(char* buf, size_t cap);
  * the logits, plane 1 is log(sum_j exp(logit_j - m)); the log-sum-exp is their sum.  They are kept
  * apart because a fully masked row has m = -1e9, where adding the second term would round it away.
  * dbias: fp32 [B, H, n_res, n_res]
- * contiguous, summed over rows. */
+ * contiguous, summed over rows (without a bias: the gradient at zero, on the CUDA-core kernels). */
 typedef struct TriAttnDesc {
   int32_t B, n_seq, n_res, H, D;
   int32_t dtype;      /* TRI_F32 / TRI_BF16 / TRI_F16 */

@@ -333,3 +333,36 @@ def test_operands_that_do_not_match_are_refused(ta, name, cut):
     t[name] = cut(t[name])
     with pytest.raises(ValueError, match="one shape|one device"):
         ta(t["q"], t["k"], t["v"], t["bias"], mask)
+
+
+@pytest.mark.parametrize("dtype,precision,S,N", [(torch.bfloat16, "ieee", 4, 72), (torch.float32, "tf32", 80, 256), (torch.float32, "ieee", 3, 20)],
+                         ids=lambda v: str(v).replace("torch.", ""))
+def test_bias_gradient_without_a_bias(ta, dtype, precision, S, N):
+    """Through the C ABI: dbias asked for and bias null gives the gradient at a bias of zero."""
+    import ctypes
+
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import _triattn
+    lib, H = _lib.load(), 4
+    t, mask, d_o = util.attn_inputs(1, S, N, H, 32, dtype, seed=8, with_bias=False)
+    zero = dict(t, bias=torch.zeros(1, 1, H, N, N, dtype=dtype, device="cuda"))
+    with util.matmul_precision(precision):
+        _, want = util.attn_fwd_bwd(ta, zero, mask, None, d_o)
+    q, k, v = t["q"], t["k"], t["v"]
+    m = mask.reshape(1, S, N).contiguous().view(torch.uint8)
+    o, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+    dbias, lse = torch.full((1, H, N, N), float("nan"), device="cuda"), torch.empty(2, 1, S, H, N, device="cuda")
+    d = _triattn._desc(q, k, v, o, None, m, 32 ** -0.5, precision)
+    d.do_st = d.dq_st = d.dk_st = d.dv_st = _triattn._st4(q)
+    n = max(lib.tri_attn_ws_bytes(ctypes.byref(d), b) for b in (0, 1))
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    p = lambda x: None if x is None else ctypes.c_void_p(x.data_ptr())  # noqa: E731
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(lib.tri_attn_fwd(ctypes.byref(d), p(q), p(k), p(v), None, p(m), p(o), p(lse), p(ws), n, stream), "fwd")
+    _lib.check(lib.tri_attn_bwd(ctypes.byref(d), p(q), p(k), p(v), None, p(m), p(o), p(lse), p(d_o), p(dq), p(dk), p(dv), p(dbias), p(ws), n, stream),
+               "bwd")
+    torch.cuda.synchronize()
+    assert _lib.last_path() == "simt"
+    cos_min, fro, _ = _tol(dtype, precision)
+    for name, got in (("q", dq), ("k", dk), ("v", dv), ("bias", dbias)):
+        util.check_close("grad_" + name, got, util.f64(want[name].reshape(got.shape)), cos_min, fro)
