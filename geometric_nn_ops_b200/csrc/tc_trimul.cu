@@ -511,6 +511,9 @@ void carve_prep(Arena& a, size_t es, Prep* p) {
 // transposes t), pixel-major [M, 128] otherwise.  Forward and backward decide from the same geometry.
 bool u_channel_major(const Geom& gm) { return ln_gate_out_supported(gm.dtype, gm.M, gm.plane); }
 
+// With one batch entry the product that forms du ends in the LayerNorm's backward; with more, a tile of pixels crosses planes.
+bool du_in_memory(const Geom& gm) { return gm.M != gm.plane; }
+
 constexpr int kSplitK = 148;
 // The partials of one backward phase live side by side until the phase's single reduction launch: the split-K
 // weight-gradient partials (dWcat, or dWo | dWgo) first, then the LayerNorm weight / bias partials.
@@ -748,7 +751,7 @@ int phase_output_bwd(cudaStream_t st, const Geom& gm, const void* d_out, const v
     TRI_TRY(reduce_to(st, scratch, nparts, CW, g->g_out_b));
   }
   float* pg = partial + kWgradPartialFloats;
-  if (gm.M == gm.plane) {
+  if (!du_in_memory(gm)) {
     // One batch entry: du^T = Wo^T dy^T, channel-major like t and dt, and the LayerNorm's backward in the epilogue.
     const int blocks = std::min(cdiv(M, 128), sm_count());
     float* pb = pg + (size_t)kPersist * CW;
@@ -851,7 +854,7 @@ void carve_saved(Arena& a, const Geom& gm, SavedT* s) {
 struct BwdBufs { void *dy, *dgo, *du, *dt, *da, *db, *dpg; float* partial; };
 void carve_bwd(Arena& a, const Geom& gm, BwdBufs* w) {
   const size_t unit = (size_t)gm.M * CW * gm.es();
-  w->dy = a.take<char>(unit); w->dgo = a.take<char>(unit); w->du = a.take<char>(unit);
+  w->dy = a.take<char>(unit); w->dgo = a.take<char>(unit); w->du = a.take<char>(du_in_memory(gm) ? unit : 0);
   w->dt = a.take<char>(unit); w->da = a.take<char>(unit); w->db = a.take<char>(unit);
   w->dpg = a.take<char>(4 * unit);
   w->partial = a.take<float>(partial_floats());
@@ -929,7 +932,7 @@ struct ShardWs { void *dy, *du, *dpg; float* partial; };
 void carve_shard_ws(Arena& a, const Geom& gm, int phase, ShardWs* w) {
   const size_t unit = (size_t)gm.M * CW * gm.es();
   *w = ShardWs{};
-  if (phase == TRI_PHASE_OUTPUT_BWD) { w->dy = a.take<char>(unit); w->du = a.take<char>(unit); }
+  if (phase == TRI_PHASE_OUTPUT_BWD) { w->dy = a.take<char>(unit); w->du = a.take<char>(du_in_memory(gm) ? unit : 0); }
   if (phase == TRI_PHASE_PROJECT_BWD) w->dpg = a.take<char>(4 * unit);
   if (phase >= TRI_PHASE_OUTPUT_BWD) w->partial = a.take<float>(partial_floats());
 }

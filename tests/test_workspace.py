@@ -34,6 +34,18 @@ def test_ragged_update_forward():
     assert size(203) - size(208) <= 208 * 208 * 2 + 1024      # a padded mask, no padded x and out
 
 
+def test_update_backward():
+    from geometric_nn_ops_b200 import _lib
+    lib = _lib.load()
+    size = lambda b: lib.tri_mul_ws_bytes(ctypes.byref(_lib.TriMulDesc(b, 256, 128, 128, _lib.BF16, 0, 0, 1e-5)), 1)  # noqa: E731
+    unit = 256 * 256 * 128 * 2
+    # per pixel and channel: dy, dgo, dt, da, db, four of dPG; du for batches only, where the LayerNorm's backward reads it
+    fixed = size(1) - 9 * unit
+    assert 0 < fixed < 48 << 20 and size(2) == fixed + 2 * 10 * unit
+    phase = lambda b: lib.tri_mul_shard_ws_bytes(ctypes.byref(_lib.TriMulShardDesc(b, 256, 256, 128, 128, _lib.BF16, 0, 1e-5)), _lib.PHASE_OUTPUT_BWD)  # noqa: E731
+    assert phase(2) - phase(1) == 3 * unit
+
+
 def _p(t):
     return ctypes.c_void_p(t.data_ptr())
 
