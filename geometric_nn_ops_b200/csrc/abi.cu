@@ -174,7 +174,7 @@ int tri_attn_fwd(const TriAttnDesc* d, const void* q, const void* k, const void*
     set_path("tcgen05");
     return tc::attn_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
-  if (tc::attn_tf32_supported(d, 0) && aligned_to(16, {q, k, v, o, ws}) && ws != nullptr && ws_bytes >= tc::attn_tf32_ws_bytes(d, 0)) {
+  if (tc::attn_tf32_supported(d, 0) && aligned_to(16, {q, k, v, o, ws}) && ws != nullptr && tc::attn_tf32_has_room(d, bias, ws_bytes, 0)) {
     set_path("tcgen05");
     return tc::attn_tf32_forward(d, q, k, v, bias, mask, o, lse, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -194,7 +194,7 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
     return tc::attn_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes,
                              (cudaStream_t)stream);
   }
-  if (tensor_cores && tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, ws}) && ws_bytes >= tc::attn_tf32_ws_bytes(d, 1)) {
+  if (tensor_cores && tc::attn_tf32_supported(d, 1) && aligned_to(16, {q, k, v, d_o, o, dq, dk, dv, ws}) && tc::attn_tf32_has_room(d, bias, ws_bytes, 1)) {
     set_path("tcgen05");
     return tc::attn_tf32_backward(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, ws, ws_bytes, (cudaStream_t)stream);
   }

@@ -1457,8 +1457,6 @@ __global__ void sum_partials_kernel(const float* partial, int nparts, long long 
   out[i] = s;
 }
 
-constexpr int kDbiasRowChunks = 8;   // at most this many row chunks (the workspace holds one partial sum per chunk)
-
 // Can a tensor map reach the bias as it is?  Otherwise the tensor-core kernels read a copy with padded rows: rows whose
 // length or start is not a multiple of 16 bytes (any N that is not a multiple of eight), broadcast heads or queries.
 bool bias_strides_fit_tma(const TriAttnDesc* d) {
@@ -1532,11 +1530,34 @@ int set_dyn_smem(KernelT kern, int bytes) {
   return 0;
 }
 
+struct BwdWs {
+  int* err;
+  float *delta, *part, *prep, *mask_terms;
+  uint4* aug;
+  int* large;
+  void *bias_t, *dq_part;
+  void* bias_c;        // padded copy of the bias, behind the rest
+};
+int dbias_slots(const TriAttnDesc* d) { return (d->D <= 32 ? 2 : 1) * sm_count(); }   // CTAs of the dbias pass at a time
+void carve_bwd(Arena& a, const TriAttnDesc* d, BwdWs* w) {
+  const size_t rows = (size_t)d->B * d->n_seq * d->H, npad = ((size_t)d->n_res + 127) / 128 * 128;
+  const bool merged = d->D <= 32;
+  w->err = a.take<int>(128);
+  w->delta = a.take<float>(merged ? 0 : rows * d->n_res);                        // read by the dQ pass
+  w->part = a.take<float>(dbias_partial_bytes(d, dbias_slots(d)) / sizeof(float));
+  w->bias_t = a.take<char>(bias_copy_bytes(d));                                  // transposed copy of the bias
+  w->prep = a.take<float>(3 * rows * npad);                                      // padded per-row constants
+  w->mask_terms = a.take<float>(2 * (size_t)d->B * d->n_seq * npad);             // additive key-mask terms
+  w->aug = a.take<uint4>(rows * npad);                                           // row constants as factors
+  w->large = a.take<int>(rows);                                                  // rows that go without them
+  w->dq_part = a.take<uint16_t>(merged ? npad / 128 * rows * d->n_res * d->D : 0);   // merged pass: dQ per 128-key block
+  w->bias_c = a.take<char>(0);
+}
+
 template <typename T, int HD>
 int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias,
                const uint8_t* mask, const void* o, const float* stats, const void* d_o, void* dq, void* dk, void* dv,
-               float* dbias, int* err, float* delta, float* dbias_partial, void* bias_t, void* bias_c, float* prep, float* mask_terms,
-               uint4* aug, int* large, void* dq_part, cudaStream_t st) {
+               float* dbias, const BwdWs& w, cudaStream_t st) {
   const long long rows = (long long)d->B * d->n_seq * d->H * d->n_res;
   const double pairs = (double)rows * d->n_res;
   const double tensor_bytes = 2.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D;
@@ -1544,17 +1565,17 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   const long long prep_plane = (long long)d->B * d->n_seq * d->H * npad;
   {
     KernelTimer kt("tc_attn_delta", st, 0.0, 2.0 * tensor_bytes);
-    TRI_TRY(launch_mask_terms(d, mask, mask_terms, err, large, st));
+    TRI_TRY(launch_mask_terms(d, mask, w.mask_terms, w.err, w.large, st));
     attn_delta_tc_kernel<T><<<(unsigned)(d->B * (long long)d->n_seq * (npad / 128)), 128, 0, st>>>(
-        *d, (const T*)o, (const T*)d_o, stats, HD == 32 ? nullptr : delta, prep, aug, large, npad);
+        *d, (const T*)o, (const T*)d_o, stats, HD == 32 ? nullptr : w.delta, w.prep, w.aug, w.large, npad);
     TRI_LAUNCH_OK();
   }
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   AttnBwdArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D; a.scale = d->scale;
-  a.stats = stats; a.delta = delta; a.prep = prep; a.prep_plane = prep_plane; a.npad = npad; a.mask_terms = mask_terms; a.mask_plane = (long long)d->B * d->n_seq * npad;
-  a.aug = aug; a.large = large; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
-  a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0; a.err = err;
+  a.stats = stats; a.delta = w.delta; a.prep = w.prep; a.prep_plane = prep_plane; a.npad = npad; a.mask_terms = w.mask_terms; a.mask_plane = (long long)d->B * d->n_seq * npad;
+  a.aug = w.aug; a.large = w.large; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
+  a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0; a.err = w.err;
   a.row_chunks = 1;
   const int qblocks = (d->n_res + 127) / 128;
   CUtensorMap tq, tdo, tk, tv, tb;
@@ -1567,9 +1588,9 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   if (bias) {   // the dK/dV pass (thread = key) reads a transposed copy of the bias: [b][h][key][query]
     transpose_bias_kernel<<<dim3(cdiv(d->n_res, 64), cdiv(d->n_res, 64), bias_batches(d) * d->H), dim3(32, 8), 0, st>>>(
         static_cast<const uint16_t*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2], d->n_res, d->H, bias_pitch(d),
-        static_cast<uint16_t*>(bias_t));
+        static_cast<uint16_t*>(w.bias_t));
     TRI_LAUNCH_OK();
-    TRI_TRY(bias_map(&tb, bias, bias_t, d, 128));
+    TRI_TRY(bias_map(&tb, bias, w.bias_t, d, 128));
   } else {
     tb = tq;
   }
@@ -1582,7 +1603,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   // TMEM columns to spare for the dQ accumulator and keeps the separate dQ pass.
   constexpr bool kMerge = HD == 32;
   const long long dq_plane = (long long)d->B * d->n_seq * d->n_res * d->H * d->D;
-  a.dq_part = dq_part; a.dq_part_plane = dq_plane;
+  a.dq_part = w.dq_part; a.dq_part_plane = dq_plane;
   {
     auto kern = bias ? attn_bwd_dkdv_kernel<T, HD, true, kMerge> : attn_bwd_dkdv_kernel<T, HD, false, kMerge>;
     TRI_TRY(set_dyn_smem(kern, GeoC<HD>::SMEM));   // per-device attribute: set on every launch
@@ -1593,7 +1614,7 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   }
   if (kMerge) {
     KernelTimer kt("tc_attn_dq_sum", st, 0.0, (qblocks + 1.0) * tensor_bytes);
-    attn_dq_sum_kernel<T><<<cdiv(dq_plane / 8, 256), 256, 0, st>>>(static_cast<const T*>(dq_part), qblocks, dq_plane, *d,
+    attn_dq_sum_kernel<T><<<cdiv(dq_plane / 8, 256), 256, 0, st>>>(static_cast<const T*>(w.dq_part), qblocks, dq_plane, *d,
                                                                static_cast<T*>(dq));
     TRI_LAUNCH_OK();
   }
@@ -1606,8 +1627,8 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
     TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, HD));
     if (bias) {
       const bool own = bias_fits_tma(d, bias);
-      if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
-      TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
+      if (!own) TRI_TRY(launch_pad_bias(d, bias, w.bias_c, st));
+      TRI_TRY(bias_map(&tb, bias, own ? nullptr : w.bias_c, d, 128));
     } else {
       tb = tq;
     }
@@ -1621,29 +1642,17 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   }
   // ---- dbias ---------------------------------------------------------------------------------
   if (dbias != nullptr) {
-    // Row chunks until the CTAs fill the GPU, as few as give the fewest rows in a row: rounds of CTAs times rows of a chunk.  (One
-    // round more for the last few CTAs costs as much as the rounds before: 301 residues, 60 tiles, 5 chunks 113 us, 4 chunks 84.)
-    const int qtiles = (d->n_res + 63) / 64;
-    const long long combos = (long long)qblocks * qtiles * d->B * d->H, slots = (HD == 32 ? 2LL : 1LL) * sm_count();
-    int chunks = 1;
-    long long best = -1;
-    for (int ch = 1; ch <= std::min(kDbiasRowChunks, std::max(1, d->n_seq / 2)); ++ch) {
-      const long long steps = (combos * ch + slots - 1) / slots * cdiv(d->n_seq, ch);
-      if (best < 0 || steps * 10 < best * 9) { best = steps; chunks = ch; }   // (each chunk costs a partial sum)
-    }
-    const long long nb = (long long)d->B * d->H * d->n_res * d->n_res;
+    const int chunks = dbias_row_chunks(d, dbias_slots(d));
+    const long long combos = (long long)qblocks * cdiv(d->n_res, 64) * d->B * d->H, nb = (long long)d->B * d->H * d->n_res * d->n_res;
     a.row_chunks = chunks;
-    a.out0 = chunks > 1 ? dbias_partial : dbias;
+    a.out0 = chunks > 1 ? w.part : dbias;
     a.idesc_a = make_idesc(kind, 128, 64, false, false);
     auto kern = attn_bwd_dbias_kernel<T, HD>;   // (with the dK/dV pass's maps)
     TRI_TRY(set_dyn_smem(kern, GeoB<HD>::SMEM));
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor_bytes);
     launch_dependent(us_of_logits(pairs), kern, (unsigned)(combos * chunks), 320, GeoB<HD>::SMEM, st, tq, tdo, tk, tv, tb, a);
     TRI_LAUNCH_OK();
-    if (chunks > 1) {   // fixed-order sum of the row-chunk partials
-      sum_partials_kernel<<<cdiv(nb, 256), 256, 0, st>>>(dbias_partial, chunks, nb, dbias);
-      TRI_LAUNCH_OK();
-    }
+    if (chunks > 1) TRI_TRY(launch_sum_partials(w.part, chunks, nb, dbias, st));
   }
   return 0;
 }
@@ -1715,6 +1724,30 @@ int launch_mask_terms(const TriAttnDesc* d, const uint8_t* mask, float* out, int
   return 0;
 }
 
+// Row chunks until the CTAs fill the GPU, as few as give the fewest rows in a row: rounds of CTAs times rows of a chunk.  (One
+// round more for the last few CTAs costs as much as the rounds before: 301 residues, 60 tiles, 5 chunks 113 us, 4 chunks 84.)
+int dbias_row_chunks(const TriAttnDesc* d, int slots) {
+  const long long combos = (long long)cdiv(d->n_res, 128) * cdiv(d->n_res, 64) * d->B * d->H;
+  int chunks = 1;
+  long long best = -1;
+  for (int ch = 1; ch <= std::min(8, std::max(1, d->n_seq / 2)); ++ch) {
+    const long long steps = (combos * ch + slots - 1) / slots * cdiv(d->n_seq, ch);
+    if (best < 0 || steps * 10 < best * 9) { best = steps; chunks = ch; }   // (each chunk costs a partial sum)
+  }
+  return chunks;
+}
+
+size_t dbias_partial_bytes(const TriAttnDesc* d, int slots) {
+  const int chunks = dbias_row_chunks(d, slots);
+  return chunks > 1 ? align_up((size_t)chunks * d->B * d->H * d->n_res * d->n_res * sizeof(float)) : 0;
+}
+
+int launch_sum_partials(const float* partial, int chunks, long long n, float* out, cudaStream_t st) {
+  sum_partials_kernel<<<cdiv(n, 256), 256, 0, st>>>(partial, chunks, n, out);
+  TRI_LAUNCH_OK();
+  return 0;
+}
+
 int qkv_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, const int64_t* st, int rows, int width) {
   const uint64_t dims[5] = {(uint64_t)d->D, (uint64_t)d->H, (uint64_t)d->n_res, (uint64_t)d->n_seq, (uint64_t)d->B};
   const uint64_t str[4] = {(uint64_t)st[3], (uint64_t)st[2], (uint64_t)st[1], (uint64_t)st[0]};
@@ -1748,23 +1781,14 @@ bool attn_bwd_supported(const TriAttnDesc* d) {
 }
 
 static size_t attn_npad(const TriAttnDesc* d) { return ((size_t)d->n_res + 127) / 128 * 128; }
-// partial dQ of the merged dK/dV + dQ pass (head dim 32 only): one 16-bit tensor of q's size per 128-key block
-static size_t attn_dq_part_bytes(const TriAttnDesc* d) {
-  if (d->D > 32) return 0;
-  return align_up(attn_npad(d) / 128 * (size_t)d->B * d->n_seq * d->n_res * d->H * d->D * 2);
-}
 
 // everything but the padded copy of the bias, which comes last
 static size_t attn_ws_base(const TriAttnDesc* d, int is_bwd) {
   if (!is_bwd) return 512 + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));   // additive key-mask terms
-  return 512 + align_up((size_t)d->B * d->n_seq * d->H * d->n_res * sizeof(float)) +
-         align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float)) +
-         bias_copy_bytes(d) +                                                            // transposed copy of the bias
-         align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)) +   // padded per-row constants
-         align_up(2 * (size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)) +          // additive key-mask terms
-         align_up((size_t)d->B * d->n_seq * d->H * attn_npad(d) * 16) +                  // row constants as factors
-         align_up((size_t)d->B * d->n_seq * d->H * sizeof(int)) +                        // rows that go without them
-         attn_dq_part_bytes(d);                                                          // merged pass: dQ per key block
+  Arena a(nullptr, 0);
+  BwdWs w;
+  carve_bwd(a, d, &w);
+  return a.off;
 }
 
 // (The descriptor does not say where the bias starts: a copy for that reason alone is not counted here, see attn_bias_has_room.)
@@ -1795,23 +1819,15 @@ int attn_backward(const TriAttnDesc* d, const void* q, const void* k, const void
                   const uint8_t* mask, const void* o, const float* lse, const void* d_o, void* dq, void* dk,
                   void* dv, float* dbias, void* ws, size_t ws_size, cudaStream_t st) {
   if (ws == nullptr || ws_size < attn_ws_bytes(d, 1)) return fail(TRI_ERR_WORKSPACE, "attention backward workspace too small");
-  int* err = static_cast<int*>(ws);
-  float* delta = reinterpret_cast<float*>(static_cast<char*>(ws) + 512);
-  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + 512 +
-                                         align_up((size_t)d->B * d->n_seq * d->H * d->n_res * sizeof(float)));
-  void* bias_t = reinterpret_cast<char*>(part) + align_up((size_t)kDbiasRowChunks * d->B * d->H * d->n_res * d->n_res * sizeof(float));
-  float* prep = reinterpret_cast<float*>(static_cast<char*>(bias_t) + bias_copy_bytes(d));
-  float* mterms = reinterpret_cast<float*>(reinterpret_cast<char*>(prep) + align_up(3 * (size_t)d->B * d->n_seq * d->H * attn_npad(d) * sizeof(float)));
-  uint4* aug = reinterpret_cast<uint4*>(reinterpret_cast<char*>(mterms) + align_up(2 * (size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float)));
-  int* large = reinterpret_cast<int*>(reinterpret_cast<char*>(aug) + align_up((size_t)d->B * d->n_seq * d->H * attn_npad(d) * 16));
-  void* dq_part = reinterpret_cast<char*>(large) + align_up((size_t)d->B * d->n_seq * d->H * sizeof(int));
-  void* bias_c = static_cast<char*>(ws) + attn_ws_base(d, 1);
+  Arena a(ws, ws_size);
+  BwdWs w;
+  carve_bwd(a, d, &w);
   if (d->dtype == TRI_BF16) {
-    if (d->D <= 32) return bwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
-    return bwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
+    if (d->D <= 32) return bwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, w, st);
+    return bwd_launch<__nv_bfloat16, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, w, st);
   }
-  if (d->D <= 32) return bwd_launch<__half, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
-  return bwd_launch<__half, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, err, delta, part, bias_t, bias_c, prep, mterms, aug, large, dq_part, st);
+  if (d->D <= 32) return bwd_launch<__half, 32>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, w, st);
+  return bwd_launch<__half, 64>(d, q, k, v, bias, mask, o, lse, d_o, dq, dk, dv, dbias, w, st);
 }
 
 }  // namespace tc

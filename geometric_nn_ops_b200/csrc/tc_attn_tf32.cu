@@ -155,14 +155,6 @@ __global__ void copy_bias_kernel(const float* __restrict__ in, int64_t st_b, int
   }
 }
 
-__global__ void add_chunks_kernel(const float* partial, int nparts, long long n, float* out) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += partial[p * n + i];
-  out[i] = s;
-}
-
 // ---------------------------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------------------------
@@ -662,17 +654,15 @@ attn_bwd_dbias_tf32_kernel(const __grid_constant__ CUtensorMap tmK, const __grid
 // ---------------------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------------------
-constexpr int kRowChunks = 8;
-
 int pitch_of(const TriAttnDesc* d) { return (d->n_res + 3) / 4 * 4; }
 int batches_of(const TriAttnDesc* d) { return d->bias_st[0] != 0 ? d->B : 1; }
 size_t tensor_floats(const TriAttnDesc* d) { return (size_t)d->B * d->n_seq * d->n_res * d->H * d->D; }
 size_t bias_floats(const TriAttnDesc* d) { return (size_t)batches_of(d) * d->H * d->n_res * pitch_of(d); }
 int npad_of(const TriAttnDesc* d) { return (d->n_res + 127) / 128 * 128; }
-bool own_bias(const TriAttnDesc* d, const void* bias) {
-  return reinterpret_cast<uintptr_t>(bias) % 16 == 0 && d->bias_st[0] % 4 == 0 && d->bias_st[1] % 4 == 0 && d->bias_st[2] % 4 == 0 &&
-         (d->bias_st[1] != 0 || d->H == 1) && d->bias_st[2] != 0;
+bool bias_strides_fit(const TriAttnDesc* d) {
+  return d->bias_st[0] % 4 == 0 && d->bias_st[1] % 4 == 0 && d->bias_st[2] % 4 == 0 && (d->bias_st[1] != 0 || d->H == 1) && d->bias_st[2] != 0;
 }
+bool own_bias(const TriAttnDesc* d, const void* bias) { return reinterpret_cast<uintptr_t>(bias) % 16 == 0 && bias_strides_fit(d); }
 
 struct TfWs {
   int* err;
@@ -680,11 +670,12 @@ struct TfWs {
   float4* aug;
   int* large;
 };
-void carve(Arena& a, const TriAttnDesc* d, int is_bwd, TfWs* w) {
+// bias_copy: the bias is not read in place
+void carve(Arena& a, const TriAttnDesc* d, int is_bwd, bool bias_copy, TfWs* w) {
   const size_t t = tensor_floats(d), rows = (size_t)d->B * d->n_seq * d->H, np = npad_of(d);
   w->err = a.take<int>(64);
   w->q = a.take<float>(t); w->k = a.take<float>(t); w->v = a.take<float>(t);
-  w->bias = a.take<float>(bias_floats(d));
+  w->bias = a.take<float>(bias_copy ? bias_floats(d) : 0);
   w->mask = a.take<float>((is_bwd ? 2 : 1) * (size_t)d->B * d->n_seq * np);
   if (!is_bwd) return;
   w->d_o = a.take<float>(t);
@@ -692,7 +683,7 @@ void carve(Arena& a, const TriAttnDesc* d, int is_bwd, TfWs* w) {
   w->prep = a.take<float>(3 * rows * np);
   w->aug = a.take<float4>(2 * rows * np);
   w->large = a.take<int>(rows);
-  w->part = a.take<float>((size_t)kRowChunks * d->B * d->H * d->n_res * d->n_res);
+  w->part = a.take<float>(dbias_partial_bytes(d, sm_count()) / sizeof(float));
 }
 
 // boxes of `rows` residues of a rounded copy; `across` for a product that reads it across its rows
@@ -755,18 +746,23 @@ bool attn_tf32_supported(const TriAttnDesc* d, int is_bwd) {
   return attn_fwd_rows_fits(d);
 }
 
-size_t attn_tf32_ws_bytes(const TriAttnDesc* d, int is_bwd) {
+static size_t ws_bytes(const TriAttnDesc* d, int is_bwd, bool bias_copy) {
   Arena a(nullptr, 0);
   TfWs w;
-  carve(a, d, is_bwd, &w);
+  carve(a, d, is_bwd, bias_copy, &w);
   return a.off;
+}
+// (The descriptor does not say where the bias starts: a copy for that reason alone is not counted here.)
+size_t attn_tf32_ws_bytes(const TriAttnDesc* d, int is_bwd) { return ws_bytes(d, is_bwd, !bias_strides_fit(d)); }
+bool attn_tf32_has_room(const TriAttnDesc* d, const void* bias, size_t ws_size, int is_bwd) {
+  return ws_size >= ws_bytes(d, is_bwd, !bias_strides_fit(d) || (bias != nullptr && !own_bias(d, bias)));
 }
 
 int attn_tf32_forward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias, const uint8_t* mask, void* o, float* stats,
                       void* ws, size_t ws_size, cudaStream_t st) {
   Arena ar(ws, ws_size);
   TfWs w;
-  carve(ar, d, 0, &w);
+  carve(ar, d, 0, bias != nullptr && !own_bias(d, bias), &w);
   if (ws == nullptr || !ar.ok()) return fail(TRI_ERR_WORKSPACE, "attention forward workspace too small");
   TRI_TRY(launch_mask_terms(d, mask, w.mask, w.err, nullptr, st));
   TRI_TRY(round_qkv(d, q, k, v, w, st));
@@ -786,7 +782,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
                        const float* stats, const void* d_o, void* dq, void* dk, void* dv, float* dbias, void* ws, size_t ws_size, cudaStream_t st) {
   Arena ar(ws, ws_size);
   TfWs w;
-  carve(ar, d, 1, &w);
+  carve(ar, d, 1, bias != nullptr && !own_bias(d, bias), &w);
   if (ws == nullptr || !ar.ok()) return fail(TRI_ERR_WORKSPACE, "attention backward workspace too small");
   TRI_TRY(launch_mask_terms(d, mask, w.mask, w.err, w.large, st));
   TRI_TRY(round_qkv(d, q, k, v, w, st));
@@ -852,12 +848,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
   // ---- dbias ------------------------------------------------------------------------------------
   if (dbias != nullptr) {
     const long long combos = (long long)blocks * nq * d->B * d->H;
-    int chunks = 1;
-    long long best = -1;
-    for (int ch = 1; ch <= std::min(kRowChunks, std::max(1, d->n_seq / 2)); ++ch) {   // as in tc_attn.cu
-      const long long steps = (combos * ch + sm_count() - 1) / sm_count() * cdiv(d->n_seq, ch);
-      if (best < 0 || steps * 10 < best * 9) { best = steps; chunks = ch; }
-    }
+    const int chunks = dbias_row_chunks(d, sm_count());
     const long long n = (long long)d->B * d->H * d->n_res * d->n_res;
     a.row_chunks = chunks;
     a.out[0] = chunks > 1 ? w.part : dbias;
@@ -865,10 +856,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     KernelTimer kt("tc_attn_bwd_dbias", st, 0.0, 4.0 * tensor);
     launch_dependent(us_of_logits(pairs), attn_bwd_dbias_tf32_kernel, (unsigned)(combos * chunks), kThreads, GeoTB::SMEM, st, tk, tv, tq, tdo, w.bias_t, pitch_of(d), a);
     TRI_LAUNCH_OK();
-    if (chunks > 1) {
-      add_chunks_kernel<<<cdiv(n, 256), 256, 0, st>>>(w.part, chunks, n, dbias);
-      TRI_LAUNCH_OK();
-    }
+    if (chunks > 1) TRI_TRY(launch_sum_partials(w.part, chunks, n, dbias, st));
   }
   return 0;
 }

@@ -152,7 +152,7 @@ TriAttnDesc attn_desc(const Tensor& q, const Tensor& k, const Tensor& v, const T
 size_t attn_ws_bytes(const TriAttnDesc& d, const Tensor& bias, int is_bwd) {
   const size_t n = api.attn_ws_bytes(&d, is_bwd);
   if (!bias.defined() || reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0) return n;
-  return n + (size_t)2 * d.B * d.H * d.n_res * (d.n_res + 7) + 256;
+  return n + (size_t)bias.element_size() * d.B * d.H * d.n_res * (d.n_res + 7) + 256;
 }
 
 struct AttnCall { Tensor q, k, v, bias, mask, o, stats; };   // mask: bytes [B, S, N]

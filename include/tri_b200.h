@@ -104,7 +104,9 @@ int tri_attn_bwd(const TriAttnDesc* d, const void* q, const void* k, const void*
                  void* ws, size_t ws_bytes, tri_stream_t stream);
 
 /* Enough for every bias that starts on a 16-byte boundary.  One that does not is copied if the workspace has another
- * 2 * B * H * n_res * (n_res + 7) + 256 bytes (16-bit dtypes), and read by the CUDA-core kernels otherwise. */
+ * itemsize * B * H * n_res * (n_res + 7) + 256 bytes, and read by the CUDA-core kernels otherwise.  The backward's size depends on
+ * the number of multiprocessors of the current device: query it with the device of the call current.
+ * fp32 with precision tf32: from 2e7 (backward: 5e6) logits on, head dim up to 32, it holds copies of q, k, v (and d_o). */
 size_t tri_attn_ws_bytes(const TriAttnDesc* d, int is_bwd);
 
 /* Attention backward for callers that cannot provide a workspace.  (No counterpart in the reference,
