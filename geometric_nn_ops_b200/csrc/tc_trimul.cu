@@ -370,6 +370,8 @@ __global__ void __launch_bounds__(256, 2) ln_cm_bwd_kernel(const T* du, const T*
   }
 }
 
+// Column sums of a pixel-major [M, W] tensor, for the output biases' gradients: partial[block][c] over the block's share of the
+// rows, in order.
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_kernel(const T* X, long long M, int W, float* partial) {
   const long long per = (M + gridDim.x - 1) / gridDim.x;

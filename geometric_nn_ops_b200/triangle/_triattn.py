@@ -58,7 +58,9 @@ def triangle_attention_b200(q, k, v, bias=None, mask=None, scale=None, dynamic=F
     ``return_aux=True`` returns ``(out, lse, max)``: the log-sum-exp and the maximum of each query's
     logits, fp32 ``[B, N_seq, H, N_res, 1]`` (the cuequivariance ``(B, N, H, Q, 1)`` layout), not differentiable.
     ``lse`` is exact.  ``max`` is the reference point the kernel used for the exponentials: the exact row maximum on
-    the CUDA-core path; on the tensor-core path a value between ``max - 8 ln 2`` and ``max``.  (The reference's kernels
+    the CUDA-core path; on the tensor-core path a value between ``max - 8 ln 2`` and ``max``.  That path serves 16-bit
+    types, and fp32 with TF32 products (head dim up to 32) from 2e7 logits, B * N_seq * H * N_res**2, on; fp32 at "ieee" is
+    always exact.  (The reference's kernels
     do not expose them and its cuequivariance shim raises for ``return_aux``,
     ``cuequivariance_ops_torch/triangle_attention.py:34-38``; these kernels write them anyway.)
     """
@@ -75,7 +77,8 @@ def triangle_attention(q, k, v, bias=None, mask=None, scale=None, dynamic=False,
         scale: softmax scale, default ``D ** -0.5``.
 
     Returns a tensor of q's shape and dtype; with ``return_aux=True`` also the log-sum-exp and the
-    maximum of every query's logits (fp32, ``[B, N_seq, H, N_res, 1]``).  fp32 matmuls follow
+    maximum of every query's logits (fp32, ``[B, N_seq, H, N_res, 1]``).  The maximum is exact for fp32 at "ieee"; for
+    16-bit types and TF32 it may lie up to ``8 ln 2`` below it (see :func:`triangle_attention_b200`).  fp32 matmuls follow
     ``torch.backends.cuda.matmul.fp32_precision``.
     """
     if mask is not None and mask.dtype != torch.bool:
