@@ -76,7 +76,8 @@ inline int fail(int code, const char* fmt, ...) {
 // And only the short ones: `us` is what the kernel takes at least, by its bytes or its exponentials.  The few us of a ramp do
 // not show beside a long kernel, and with every kernel of the pair stack at 1024 residues (86 us and more each, at the power limit
 // throughout) started early, its pass took 0.5 to 1 % longer: 23.24-23.34 -> 23.40-23.60 ms.  The kernels that gained take at
-// least 1 to 40 us; between that and 70 neither start is measurably better.
+// least 1 to 40 us; between that and 70 neither start is measurably better: the update with gradients at 384, 768 and (TF32) 512, whose
+// gate kernels lie above the line, takes 450.8, 1711 and 1436 us with it and 450.7, 1710 and 1436 with every kernel started early.
 __device__ __forceinline__ void dependent_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependent_enter() {
