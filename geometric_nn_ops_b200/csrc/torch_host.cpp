@@ -538,7 +538,7 @@ std::pair<Tensor, Tensor> attention_pair_bias(const Tensor& s, const Tensor& q, 
     const int64_t W = H * D, N = o_w.size(0);
     const Tensor gated = at::empty({BM, U, W}, s.options()), out = at::empty({BM, U, N}, s.options());
     const tri_stream_t st = stream_of(s);
-    // (nothing is queued between the attention, which wrote o, and this: o is its output as it came, s and the weights the caller's)
+    // (the last call of the library is the attention, and s and the weights are the caller's: older than it)
     ok(api.gated_linear_after(dtype_code(s), BM * U, (int32_t)s.size(2), (int32_t)W, (int32_t)N, ptr(s), ptr(g_w), ptr(o), ptr(o_w), ptr(gated),
                               ptr(out), ptr(status), st), "tri_gated_linear_after");
     check_device(status, reinterpret_cast<cudaStream_t>(st));

@@ -164,9 +164,9 @@ int tri_gate_mul(int dtype, int64_t n, const void* a, const void* gate, void* ou
 int tri_gated_linear(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
                      const void* w_out, void* gated, void* out, void* status, tri_stream_t stream);
 
-/* The same directly behind the call of this library that wrote o, with no other work between the two on the stream: the first
- * product starts while that call still runs and waits for it only where it needs o.  s and w_gate must have been complete before
- * THAT call, not merely before this one. */
+/* The same, begun while the last call of this library on the stream (the one that wrote o, say) still runs: the first product
+ * waits for what is queued before it only where it needs o.  s and w_gate must have been complete before THAT call, not merely
+ * before this one. */
 int tri_gated_linear_after(int dtype, int64_t M, int32_t K, int32_t W, int32_t N, const void* s, const void* w_gate, const void* o,
                            const void* w_out, void* gated, void* out, void* status, tri_stream_t stream);
 
