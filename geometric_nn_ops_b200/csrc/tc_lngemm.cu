@@ -680,23 +680,38 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
 }
 
 // =================================================================================================================
-// gate_in_bwd: dP = d sig(G) mask, dG = d P sig (1 - sig) mask for d = da, db, with P and G recomputed from z
+// gate_in_bwd: dP = d sig(G) mask, dG = d P sig (1 - sig) mask for d = da, db, with P and G recomputed from z, and the
+// gradients of the input weights, dP^T z and dG^T z
 // =================================================================================================================
-// 576 threads: warp 0 TMA, warp 1 tcgen05.mma, warps 2-17 the gate epilogue (thread = channel of the half, a quarter of
-// the tile's pixels).  A tile is 128 bytes of pixels: 64 of 16 bits or 32 of fp32.  As in ln_gate_in the weights stay in
-// shared memory; with 16-bit types a z tile feeds the products of both halves, so z is read once.  The fp32 weights of one
-// half fill the same space, so there a CTA has one half and its neighbour the other, on the same tiles (z comes from L2
-// the second time).  The gradient tile of a half ([128 channels x 128 bytes]) comes by TMA; the epilogue copies it to
-// registers first, so that its buffer takes the next tile's during the arithmetic.  dP and dG leave through a staging
-// tile each and a TMA store: whole 128-byte lines.  Written by the threads, a request carried 32 bytes (a channel's rows
-// lie a plane apart), 4096 of them per 128 pixels, and the load / store pipe held the kernel at 0.29 ms for 768 x 768
-// pixels; with the gradients read that way too (the batched GEMM's form) it took 0.365.  Now 0.22, floor by bytes 0.16.
-// fp32 with TF32 products, 512 x 512 pixels: 0.41 ms in the GEMM's form, 0.18 here, floor 0.14.
-constexpr int kBwdThreads = 576;
-constexpr int kBwdMaskRing = 4;           // as kMaskRing
-constexpr uint32_t kBTile = 16384;        // z tile: kKb blocks of [kPx rows x 128 bytes]; gradient or output tile of a half
+// 608 threads: warp 0 TMA, warp 1 tcgen05.mma for the projections, warps 2-17 the gate epilogue (thread = channel of the
+// half, half of the tile's pixels), warp 18 tcgen05.mma for the weights' gradients and the stores.  A tile is 128 bytes of
+// pixels: 64 of 16 bits or 32 of fp32.  As in ln_gate_in the weights stay in shared memory, here those of one half: a CTA has
+// one half and its neighbour the other, on the same tiles (z comes from L2 the second time).
+// dP and dG leave through a staging tile each and a TMA store: whole 128-byte lines.  Written by the threads, a request
+// carried 32 bytes (a channel's rows lie a plane apart), 4096 of them per 128 pixels, and the load / store pipe held the
+// kernel at 0.29 ms for 768 x 768 pixels.
+// The staging tiles are the weight gradients' operands as they lie (channels x pixels, K = pixels), z's tile the other one
+// (MN-major; fp32 has that form in the 32-byte-atom swizzle only and loads the tile a second time).  The sums stay in 256 TMEM
+// columns for the life of the CTA, so nothing reads dP, dG and z again for them.  (Two halves per CTA, which would read z once,
+// need 512 columns for the sums alone.)
+// What bounds it is the chain of an item: gradients from DRAM 2000 to 3500 cycles after they are asked for, products,
+// sigmoids, products and store, 2700 cycles per item, no unit above half of its rate.  Hence two sets of eight epilogue warps
+// on alternate tiles, an issuing warp for each kind of product (with one, the next tile's projections waited for this one's dP
+// and dG), and with fp32 the gradients by the threads themselves, an item ahead, which leaves their shared memory to z and a
+// third staging tile; for 16 bits that took longer (258 us against 238), and so did a third or fourth gradient tile in place of
+// a staging tile (244 to 261).  Launches in us, with the product over pixels that the sums were before: bf16 768 x 768 256 + 140
+// -> 230, 384 x 384 63 + 44 -> 62; fp32 with TF32 products 512 x 512 205 + 127 -> 245.
+constexpr int kBwdThreads = 608;
+constexpr uint32_t kBTile = 16384;        // z tile: kKb blocks of [kPx rows x 128 bytes]; output tile of a half
 template <typename T> struct BwdGeo {
-  static constexpr int kHalves = sizeof(T) == 2 ? 2 : 1, kPx = 128 / sizeof(T), kKb = sizeof(T), kBSub = kPx * 128, kE = kPx / 4;
+  static constexpr bool kZt = sizeof(T) == 4;                  // a second copy of the z tile, MN-major
+  static constexpr int kPx = 128 / sizeof(T), kKb = sizeof(T), kBSub = kPx * 128, kE = kPx / 2;   // kE: an epilogue thread's pixels
+  static constexpr bool kGradTiles = sizeof(T) == 2;           // the gradients by TMA; fp32: by the threads
+  static constexpr int kZ = kZt ? 2 : 4, kG = kGradTiles ? 2 : 0, kO = kZt ? 3 : 4;   // z tiles; gradient tiles; staging tiles
+  static constexpr int kAcc = 128 / kPx;                       // accumulators [P | G] in 256 columns
+  static constexpr uint32_t kW = 2 * kKb * kSub;               // weights of a half
+  static constexpr uint32_t kTiles = kZ + kZt + kG + kO;
+  static constexpr size_t smem = 1024 + kW + kTiles * kBTile + 16 * 64 + (2 * (kZ + 1 + kG + kO + kAcc) + 2) * 8 + 16;
 };
 
 struct BwdArgs {
@@ -704,6 +719,9 @@ struct BwdArgs {
   int tiles;
   const float* bias;
   const void* mask;
+  const uint8_t *da, *db;
+  bool wide;            // da and db start on 32-byte boundaries
+  float* partial;       // [CTA pairs][512][128], or null
   int* err;
 };
 
@@ -721,34 +739,52 @@ template <typename T, int N> __device__ __forceinline__ uint4 pack_piece(const f
   else return pack8p<T>(v);
 }
 
+__device__ __forceinline__ void ldg256(const void* p, uint4& lo, uint4& hi) {
+  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
+               : "l"(p));
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmW,
+gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmZt, const __grid_constant__ CUtensorMap tmW,
                    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmO, const BwdArgs g) {
   using G = BwdGeo<T>;
-  constexpr int KIND = ElemTraits<T>::kind, kH = G::kHalves, kKb = G::kKb;
+  constexpr int KIND = ElemTraits<T>::kind, kKb = G::kKb, kZ = G::kZ, kG = G::kG, kO = G::kO, kAcc = G::kAcc;
+  constexpr bool kZt = G::kZt;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
-  uint8_t* sZ = smem + kWBytes;            // [2] z tiles
-  uint8_t* sG = sZ + 2 * kBTile;           // [2] gradient tiles (of the halves in turn)
-  uint8_t* sO = sG + 2 * kBTile;           // dP, dG of a half
-  uint8_t* sM = sO + 2 * kBTile;           // [kBwdMaskRing] x 128 bytes of mask values
-  uint64_t* wfull = reinterpret_cast<uint64_t*>(sM + kBwdMaskRing * 128);
-  uint64_t* zfull = wfull + 1;             // [2]
-  uint64_t* zempty = zfull + 2;            // [2] both halves' products of the tile are done
-  uint64_t* gfull = zempty + 2;            // [2] gradient tile (the tile's first: with its mask)
-  uint64_t* gempty = gfull + 2;            // [2] ... copied to registers by all 16 epilogue warps
-  uint64_t* tfull = gempty + 2;            // [4] accumulator of an item complete
-  uint64_t* tempty = tfull + 4;            // ... read by all 16 epilogue warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 4);
+  uint8_t* sZ = smem + G::kW;              // [kZ] z tiles
+  uint8_t* sT = sZ + kZ * kBTile;          // fp32: the z tile as an MN-major operand
+  uint8_t* sG = sT + kZt * kBTile;         // [kG] gradient tiles
+  uint8_t* sO = sG + kG * kBTile;          // [kO] dP, dG of an item and the next
+  uint8_t* sM = sO + kO * kBTile;          // [16 warps] mask of the warp's pixels
+  uint64_t* wfull = reinterpret_cast<uint64_t*>(sM + 16 * 64);
+  uint64_t* zfull = wfull + 1;             // [kZ]
+  uint64_t* zempty = zfull + kZ;           // [kZ] the products that read the tile are done
+  uint64_t* ztfull = zempty + kZ;          // the second copy
+  uint64_t* ztempty = ztfull + 1;
+  uint64_t* gfull = ztempty + 1;           // [kG] gradient tile
+  uint64_t* gempty = gfull + kG;           // [kG] ... copied to registers by its set's 8 epilogue warps
+  uint64_t* ofull = gempty + kG;           // [kO] staging tile written by its set's 8 epilogue warps
+  uint64_t* oempty = ofull + kO;           // [kO] ... read: by the products (commit) and by the store
+  uint64_t* tfull = oempty + kO;           // [kAcc] accumulator of an item complete
+  uint64_t* tempty = tfull + kAcc;         // [kAcc] ... read by its set's 8 epilogue warps
+  uint64_t* sums = tempty + kAcc;          // all products are done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sums + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(wfull, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(&zfull[b], 1); mbar_init(&zempty[b], 1); mbar_init(&gfull[b], 1); mbar_init(&gempty[b], 16); }
-    for (int b = 0; b < 4; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 16); }
+    for (int b = 0; b < kZ; ++b) { mbar_init(&zfull[b], 1); mbar_init(&zempty[b], 1); }
+    mbar_init(ztfull, 1);
+    mbar_init(ztempty, 1);
+    for (int b = 0; b < kG; ++b) { mbar_init(&gfull[b], 1); mbar_init(&gempty[b], 8); }
+    for (int b = 0; b < kO; ++b) { mbar_init(&ofull[b], 8); mbar_init(&oempty[b], 2); }
+    for (int b = 0; b < kAcc; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 8); }
+    mbar_init(sums, 1);
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -758,118 +794,180 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   dependent_enter();
 
-  // items: the halves this CTA has, of tiles tile0, tile0 + step, ...; half_of(hh): the hh-th of them
-  const int tile0 = kH == 2 ? blockIdx.x : blockIdx.x >> 1, step = kH == 2 ? gridDim.x : gridDim.x >> 1;
-  auto half_of = [&](int hh) { return kH == 2 ? hh : (int)(blockIdx.x & 1); };
+  const int tile0 = blockIdx.x >> 1, step = gridDim.x >> 1, half = blockIdx.x & 1;
+  const int items = tile0 < g.tiles ? (g.tiles - tile0 + step - 1) / step : 0;
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(wfull, kWBytes);
-      for (int blk = 0; blk < 2 * kH; ++blk)
-        for (int kb = 0; kb < kKb; ++kb)
-          tma_load_3d(sW + (blk * kKb + kb) * kSub, &tmW, wfull, kb * G::kPx, (half_of(blk >> 1) * 2 + (blk & 1)) * 128, 0);
-      bool ok = true;
-      auto load_z = [&](int i, int tile) {
-        const int b = i & 1;
-        if (!mbar_wait(&zempty[b], ((i >> 1) & 1) ^ 1, g.err, 60)) { ok = false; return; }
+      mbar_expect_tx(wfull, G::kW);
+      for (int blk = 0; blk < 2; ++blk)
+        for (int kb = 0; kb < kKb; ++kb) tma_load_3d(sW + (blk * kKb + kb) * kSub, &tmW, wfull, kb * G::kPx, (half * 2 + blk) * 128, 0);
+      auto load_z = [&](int i) {
+        const int b = i % kZ;
+        if (!mbar_wait(&zempty[b], ((i / kZ) & 1) ^ 1, g.err, 60)) return false;
         mbar_expect_tx(&zfull[b], kBTile);
-        for (int kb = 0; kb < kKb; ++kb) tma_load_3d(sZ + b * kBTile + kb * G::kBSub, &tmZ, &zfull[b], kb * G::kPx, tile * G::kPx, 0);
+        for (int kb = 0; kb < kKb; ++kb) tma_load_3d(sZ + b * kBTile + kb * G::kBSub, &tmZ, &zfull[b], kb * G::kPx, (tile0 + i * step) * G::kPx, 0);
+        return true;
       };
-      if (tile0 < g.tiles) load_z(0, tile0);
-      int i = 0, it = 0;
-      for (int tile = tile0; tile < g.tiles && ok; tile += step, ++i) {
-        if (tile + step < g.tiles) load_z(i + 1, tile + step);   // one tile ahead
-        for (int hh = 0; hh < kH && ok; ++hh, ++it) {
-          const int b = it & 1;
-          if (!mbar_wait(&gempty[b], ((it >> 1) & 1) ^ 1, g.err, 61)) { ok = false; break; }
-          const bool with_mask = hh == 0 && g.mask != nullptr;
-          mbar_expect_tx(&gfull[b], kBTile + (with_mask ? 128 : 0));
-          tma_load_3d(sG + b * kBTile, half_of(hh) == 0 ? &tmA : &tmB, &gfull[b], tile * G::kPx, 0, 0);
-          if (with_mask) bulk_load(sM + (i % kBwdMaskRing) * 128, static_cast<const uint8_t*>(g.mask) + (long long)tile * 128, 128, &gfull[b]);
+      bool ok = true;
+      if constexpr (kZt) {
+        for (int i = 0; i < items + 1 && ok; ++i) {   // the second copy of an item behind the first copy of the next
+          if (i < items) ok = load_z(i);
+          if (i == 0 || !ok) continue;
+          ok = mbar_wait(ztempty, i & 1, g.err, 67);   // (i - 1: the item)
+          if (!ok) break;
+          mbar_expect_tx(ztfull, kBTile);
+          for (int c = 0; c < 4; ++c) tma_load_3d(sT + c * G::kBSub, &tmZt, ztfull, c * 32, (tile0 + (i - 1) * step) * G::kPx, 0);
+        }
+      } else {
+        for (int i = 0; i < items && ok; ++i) {
+          ok = load_z(i) && mbar_wait(&gempty[i % kG], ((i / kG) & 1) ^ 1, g.err, 61);
+          if (!ok) break;
+          mbar_expect_tx(&gfull[i % kG], kBTile);
+          tma_load_3d(sG + i % kG * kBTile, half == 0 ? &tmA : &tmB, &gfull[i % kG], (tile0 + i * step) * G::kPx, 0, 0);
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ MMA issuer: the projections
     if (elect_one()) {
       const uint32_t idesc = make_idesc(KIND, 128, G::kPx, false, false);
       const uint32_t w_base = smem_u32(sW), z_base = smem_u32(sZ);
       bool ok = mbar_wait(wfull, 0, g.err, 62);
-      int i = 0, it = 0;
-      for (int tile = tile0; tile < g.tiles && ok; tile += step, ++i) {
-        const int b = i & 1;
-        if (!mbar_wait(&zfull[b], (i >> 1) & 1, g.err, 63)) break;
-        for (int hh = 0; hh < kH && ok; ++hh, ++it) {
-          const int acc = it & 3;
-          if (!mbar_wait(&tempty[acc], ((it >> 2) & 1) ^ 1, g.err, 64)) { ok = false; break; }
+      for (int i = 0; i < items && ok; ++i) {
+        const int b = i % kZ, acc = i % kAcc;
+        if (!mbar_wait(&zfull[b], (i / kZ) & 1, g.err, 63)) break;
+        if (!mbar_wait(&tempty[acc], ((i / kAcc) & 1) ^ 1, g.err, 64)) break;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int pg = 0; pg < 2; ++pg) {   // P block, G block
+          const uint32_t d_addr = tmem_base + (acc * 2 + pg) * G::kPx;
+#pragma unroll
+          for (int kb = 0; kb < kKb; ++kb)
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+              const uint64_t ad = make_smem_desc(w_base + (pg * kKb + kb) * kSub + ks * 32, 16, 1024);
+              const uint64_t bd = make_smem_desc(z_base + b * kBTile + kb * G::kBSub + ks * 32, 16, 1024);
+              umma<KIND>(d_addr, ad, bd, idesc, (kb == 0 && ks == 0) ? 0u : 1u);
+            }
+        }
+        umma_commit(&tfull[acc]);
+        if constexpr (kZt) umma_commit(&zempty[b]);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 18) {
+    // ------------------------------------------------------------------ MMA issuer: the weights' gradients, and the staging tiles' stores
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc(KIND, 128, 128, false, true);
+      const uint32_t z_base = smem_u32(sZ), t_base = smem_u32(sT), o_base = smem_u32(sO);
+      bool ok = true;
+      for (int i = 0; i < items && ok; ++i) {
+        if (kZt) ok = mbar_wait(ztfull, i & 1, g.err, 69);
+#pragma unroll
+        for (int pg = 0; pg < 2; ++pg) {
+          const int n = 2 * i + pg, ob = n % kO;
+          ok = ok && mbar_wait(&ofull[ob], (n / kO) & 1, g.err, 68);
+          if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
-          for (int pg = 0; pg < 2; ++pg) {   // P block, G block of this half
-            const uint32_t d_addr = tmem_base + acc * 128 + pg * 64;
-#pragma unroll
-            for (int kb = 0; kb < kKb; ++kb)
-#pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                const uint64_t ad = make_smem_desc(w_base + ((hh * 2 + pg) * kKb + kb) * kSub + ks * 32, 16, 1024);
-                const uint64_t bd = make_smem_desc(z_base + b * kBTile + kb * G::kBSub + ks * 32, 16, 1024);
-                umma<KIND>(d_addr, ad, bd, idesc, (kb == 0 && ks == 0) ? 0u : 1u);
-              }
+          for (int ks = 0; ks < 4; ++ks) {
+            const uint64_t ad = make_smem_desc(o_base + ob * kBTile + ks * 32, 16, 1024);
+            const uint64_t bd = kZt ? make_smem_desc(t_base + ks * 8 * 128, G::kBSub, 512, 1)
+                                    : make_smem_desc(z_base + (i % kZ) * kBTile + ks * 16 * 128, G::kBSub, 1024);
+            umma<KIND>(tmem_base + 256 + pg * 128, ad, bd, idesc, (i == 0 && ks == 0) ? 0u : 1u);
           }
-          umma_commit(&tfull[acc]);
+          umma_commit(&oempty[ob]);
+          if (pg == 1) umma_commit(kZt ? ztempty : &zempty[i % kZ]);
+          tma_store_3d(&tmO, sO + ob * kBTile, (tile0 + i * step) * G::kPx, half * 256 + pg * 128, 0);
+          bulk_commit_group();
+          if (n > 0) {   // the store before this one has left shared memory
+            bulk_wait_group_read1();
+            mbar_arrive(&oempty[(n - 1) % kO]);
+          }
         }
-        if (ok) umma_commit(&zempty[b]);
       }
+      if (ok) umma_commit(sums);
+      bulk_wait_group0();
     }
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
-    const int quarter = warp & 3, j = (warp - 2) >> 2;   // TMEM lane quarter; kE-pixel part of the tile
-    const int row = quarter * 32 + lane;
-    const uint32_t at = row * 128, c0 = ((j * 2) ^ (row & 7)) << 4, c1 = ((j * 2 + 1) ^ (row & 7)) << 4;   // this thread's two pieces of a tile row
+    const int quarter = warp & 3, j = (warp - 2) >> 2, set = j >> 1;   // TMEM lane quarter; part of the 256 columns of sums
+    const int row = quarter * 32 + lane, px0 = (j & 1) * G::kE;
+    const uint32_t at = row * 128, sw = row & 7, piece0 = (j & 1) * 4;   // this thread's four pieces of a tile row
     const bool masked = g.mask != nullptr;
-    int i = 0, it = 0;
-    bool ok = true;
-    for (int tile = tile0; tile < g.tiles; tile += step, ++i) {
-      const uint4* mrow = reinterpret_cast<const uint4*>(sM + (i % kBwdMaskRing) * 128 + j * 32);
-      for (int hh = 0; hh < kH; ++hh, ++it) {
-        const int half = half_of(hh), acc = it & 3, b = it & 1;
-        const uint32_t gt_row = smem_u32(sG + b * kBTile) + at;
-        ok = mbar_wait(&gfull[b], (it >> 1) & 1, g.err, 65) && ok;
-        const uint4 d[2] = {lds128(gt_row + c0), lds128(gt_row + c1)};
-        ok = mbar_wait(&tfull[acc], (it >> 2) & 1, g.err, 66) && ok;
-        tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 128 + j * G::kE;
-        float bp = 0.f, bg = 0.f;
-        if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
-        const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
-        float p[G::kE], gt[G::kE];
-        if constexpr (G::kE == 16) {
-          ld16x2_f(t_row, t_row + 64, p, gt);
+    float bp = 0.f, bg = 0.f;
+    if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
+    const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+    constexpr int kPair = 16 / sizeof(T) / 2;   // pairs of pixels in a piece
+    // one pixel's mask of the set's next item, on its way for an item's time, and with fp32 this thread's 64 bytes of the gradients
+    uint4 dn[4];
+    T mn = from_f32<T>(1.f);
+    auto fetch = [&](int i) {
+      const long long px = (long long)(tile0 + i * step) * G::kPx + px0;
+      if constexpr (!G::kGradTiles) {
+        const uint8_t* src = (half == 0 ? g.da : g.db) + ((long long)row * g.M + px) * sizeof(T);
+        if (g.wide) {
+          ldg256(src, dn[0], dn[1]);
+          ldg256(src + 32, dn[2], dn[3]);
         } else {
-          uint32_t rp[8], rg[8];
-          tmem_ld_32x8(t_row, rp);
-          tmem_ld_32x8(t_row + 64, rg);
-          tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) { p[e] = __uint_as_float(rp[e]); gt[e] = __uint_as_float(rg[e]); }
+          for (int u = 0; u < 4; ++u) dn[u] = __ldg(reinterpret_cast<const uint4*>(src) + u);
         }
-        // After these arrivals the next products go to the accumulator and TMA writes the gradient buffer.  The buffer's loads are
-        // of the generic proxy and TMA's writes of the async proxy, which an mbarrier alone does not order: each lane fences its
-        // own loads, here, where they have long returned (right behind them the fence cost 11 of 226 us at 768 x 768 pixels).
-        fence_proxy_async_smem();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&tempty[acc]); mbar_arrive(&gempty[b]); }
-        // two pieces of 16 bytes: kE pixels as float2 pairs, dP and dG in place of the gradient
-        constexpr int kPair = G::kE / 4;   // per piece
-        uint4 o0[2], o1[2];
+      }
+      if (masked && lane < G::kE) mn = static_cast<const T*>(g.mask)[px + lane];
+    };
+    if (set < items) fetch(set);
+    T* const wmask = reinterpret_cast<T*>(sM + (warp - 2) * 64);
+    bool ok = true;
+    for (int i = set; i < items; i += 2) {
+      const int acc = i % kAcc;
+      uint4 d[4];
+      if constexpr (G::kGradTiles) {
+        ok = mbar_wait(&gfull[i % G::kG], (i / G::kG) & 1, g.err, 65) && ok;
 #pragma unroll
-        for (int uu = 0; uu < 2; ++uu) {
+        for (int u = 0; u < 4; ++u) d[u] = lds128(smem_u32(sG + i % G::kG * kBTile) + at + (((piece0 + u) ^ sw) << 4));
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) d[u] = dn[u];
+      }
+      if (masked && lane < G::kE) wmask[lane] = mn;
+      __syncwarp();
+      if (i + 2 < items) fetch(i + 2);
+      ok = mbar_wait(&tfull[acc], (i / kAcc) & 1, g.err, 66) && ok;
+      tc_fence_after_sync();
+      const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * 2 * G::kPx + px0;
+      uint8_t* const so0 = sO + 2 * i % kO * kBTile + at;
+      uint8_t* const so1 = sO + (2 * i + 1) % kO * kBTile + at;
+#pragma unroll
+      for (int h = 0; h < G::kE / 16; ++h) {       // 16 pixels at a time
+        float p[16], gt[16];
+        ld16x2_f(t_row + h * 16, t_row + G::kPx + h * 16, p, gt);
+        if constexpr (G::kGradTiles) {
+          if (h == 0) {
+            // TMA writes the gradient buffer after this arrival.  The buffer's loads are of the generic proxy and TMA's writes of the
+            // async proxy, which an mbarrier alone does not order: each lane fences its own loads, here, where they have long returned
+            // (right behind them the fence cost 11 of 226 us at 768 x 768 pixels).
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&gempty[i % G::kG]);
+          }
+        }
+        if (h == G::kE / 16 - 1) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[acc]);
+        }
+        constexpr int kPieces = 16 * sizeof(T) / 16;
+#pragma unroll
+        for (int uu = 0; uu < kPieces; ++uu) {
+          const int u = h * kPieces + uu;
           float2 dv[kPair], mk[kPair], dg[kPair];
-          unpack_piece<T>(d[uu], dv);
+          unpack_piece<T>(d[u], dv);
           if (masked) {
-            unpack_piece<T>(mrow[uu], mk);
+            unpack_piece<T>(reinterpret_cast<const uint4*>(wmask)[u], mk);
 #pragma unroll
             for (int k = 0; k < kPair; ++k) dv[k] = __fmul2_rn(dv[k], mk[k]);
           }
@@ -881,25 +979,32 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
             const float2 oms = __ffma2_rn(sg, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
             dg[k] = __fmul2_rn(__fmul2_rn(dv[k], __fadd2_rn(make_float2(p[e], p[e + 1]), bp2)), oms);
           }
-          o0[uu] = pack_piece<T>(dv);
-          o1[uu] = pack_piece<T>(dg);
-        }
-        if (threadIdx.x == 64) bulk_wait_group_read0();   // the previous half's stores have left the staging tiles
-        named_barrier(1, 512);
-        *reinterpret_cast<uint4*>(sO + at + c0) = o0[0];
-        *reinterpret_cast<uint4*>(sO + at + c1) = o0[1];
-        *reinterpret_cast<uint4*>(sO + kBTile + at + c0) = o1[0];
-        *reinterpret_cast<uint4*>(sO + kBTile + at + c1) = o1[1];
-        fence_proxy_async_smem();
-        named_barrier(2, 512);
-        if (threadIdx.x == 64 && ok) {
-          tma_store_3d(&tmO, sO, tile * G::kPx, half * 256, 0);
-          tma_store_3d(&tmO, sO + kBTile, tile * G::kPx, half * 256 + 128, 0);
-          bulk_commit_group();
+          if (u == 0) {   // the tiles' last products and stores have read them
+            const int n0 = 2 * i, n1 = 2 * i + 1;
+            ok = mbar_wait(&oempty[n0 % kO], ((n0 / kO) & 1) ^ 1, g.err, 70) && ok;
+            ok = mbar_wait(&oempty[n1 % kO], ((n1 / kO) & 1) ^ 1, g.err, 72) && ok;
+          }
+          const uint32_t c = ((piece0 + u) ^ sw) << 4;
+          *reinterpret_cast<uint4*>(so0 + c) = pack_piece<T>(dv);
+          *reinterpret_cast<uint4*>(so1 + c) = pack_piece<T>(dg);
         }
       }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&ofull[2 * i % kO]); mbar_arrive(&ofull[(2 * i + 1) % kO]); }
     }
-    if (threadIdx.x == 64) bulk_wait_group0();
+    // the sums: this thread's row of dP and of dG, a quarter of the 256 columns
+    if (g.partial != nullptr && items > 0) {
+      ok = mbar_wait(sums, 0, g.err, 71) && ok;
+      tc_fence_after_sync();
+      float* dst = g.partial + ((long long)tile0 * 512 + half * 256 + (j >> 1) * 128 + row) * 128 + (j & 1) * 64;
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 32) {
+        float v[32];
+        ld32_f(tmem_base + ((uint32_t)(quarter * 32) << 16) + 256 + j * 64 + c, v);
+        store_rows32<float>(dst + c, v, 128, ok, lane);
+      }
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -912,7 +1017,7 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
 template <typename T>
 int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   const uint64_t M = (uint64_t)p.M;
-  CUtensorMap tmZ, tmW, tmA, tmB, tmO;
+  CUtensorMap tmZ, tmZt, tmW, tmA, tmB, tmO;
   const bool f16 = p.dtype == TRI_F16;
   const uint64_t zd[3] = {128, M, 1}, zs[2] = {128, 128 * M};
   const uint64_t wd[3] = {128, 512, 1}, wsd[2] = {128, 128 * 512};
@@ -921,25 +1026,35 @@ int launch_bwd(cudaStream_t st, const GateInBwd& p) {
   constexpr int E = sizeof(T);
   const uint32_t zbox[3] = {G::kPx, G::kPx, 1}, box[3] = {G::kPx, 128, 1};
   TRI_TRY(make_tmap_3d(&tmZ, p.z, E, f16, zd, zs, zbox, false));
+  tmZt = tmZ;
+  if (G::kZt) TRI_TRY(make_tmap_3d(&tmZt, p.z, E, f16, zd, zs, zbox, true));
   TRI_TRY(make_tmap_3d(&tmW, p.wcat, E, f16, wd, wsd, box, false));
-  TRI_TRY(make_tmap_3d(&tmA, p.da_cm, E, f16, gd, gs, box, false));
-  TRI_TRY(make_tmap_3d(&tmB, p.db_cm, E, f16, gd, gs, box, false));
+  tmA = tmB = tmW;
+  if (G::kGradTiles) {
+    TRI_TRY(make_tmap_3d(&tmA, p.da_cm, E, f16, gd, gs, box, false));
+    TRI_TRY(make_tmap_3d(&tmB, p.db_cm, E, f16, gd, gs, box, false));
+  }
   TRI_TRY(make_tmap_3d(&tmO, p.dpg, E, f16, od, gs, box, false));
   BwdArgs a;
-  a.M = p.M; a.tiles = (int)(p.M / G::kPx); a.bias = p.bias_cat; a.mask = p.mask; a.err = p.err;
-  constexpr size_t smem = 1024 + kWBytes + 6 * kBTile + kBwdMaskRing * 128 + 17 * 8 + 16;
-  static_assert(smem <= 232448, "shared memory of one CTA");
+  a.M = p.M; a.tiles = (int)(p.M / G::kPx); a.bias = p.bias_cat; a.mask = p.mask; a.da = static_cast<const uint8_t*>(p.da_cm); a.db = static_cast<const uint8_t*>(p.db_cm);
+  a.wide = ((reinterpret_cast<uintptr_t>(p.da_cm) | reinterpret_cast<uintptr_t>(p.db_cm)) & 31) == 0;
+  a.partial = p.partial; a.err = p.err;
+  static_assert(G::smem <= 232448, "shared memory of one CTA");
   auto kern = gate_in_bwd_kernel<T>;
-  TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = G::kHalves == 2 ? std::min(a.tiles, sm_count()) : 2 * std::min(a.tiles, sm_count() / 2);
+  TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem));
   const double bytes = 7.0 * p.M * 128 * E;
-  KernelTimer kt("tc_gate_in_bwd", st, 0.0, bytes);
-  launch_dependent(p.first ? kLaunchPlainly : us_of_bytes(bytes), kern, grid, kBwdThreads, smem, st, tmZ, tmW, tmA, tmB, tmO, a);
+  KernelTimer kt("tc_gate_in_bwd", st, 2.0 * p.M * 128 * 512, bytes);
+  launch_dependent(p.first ? kLaunchPlainly : us_of_bytes(bytes), kern, 2 * gate_in_bwd_parts(p.dtype, p.M), kBwdThreads, G::smem, st, tmZ, tmZt, tmW,
+                   tmA, tmB, tmO, a);
   TRI_LAUNCH_OK();
   return 0;
 }
 
 }  // namespace
+
+int gate_in_bwd_parts(int dtype, long long M) {
+  return (int)std::max(1LL, std::min(M / (dtype == TRI_F32 ? 32 : 64), (long long)sm_count() / 2));
+}
 
 // one batch entry (its channel planes are M pixels apart), whole tiles (any square of a multiple of eight)
 bool gate_in_bwd_supported(int dtype, long long M, long long plane) {

@@ -6,7 +6,8 @@
 //   ln_gate_out  t (channel-major) -> u = LayerNorm over channels, normalised in shared memory in the layout the
 //                contraction left it in (the MMA reads it as an MN-major operand, so nothing is transposed), then
 //                out = (u Wo^T + bo) * sigmoid(z Wgo^T + bgo); u is kept channel-major for the backward pass.
-//   gate_in_bwd  z, da, db -> dP, dG of both halves (no LayerNorm: the same kernel shape with resident weights).
+//   gate_in_bwd  z, da, db -> dP, dG of both halves and the input weights' gradients (no LayerNorm: the same kernel shape with
+//                resident weights).
 #pragma once
 
 #include "tc_common.cuh"
@@ -78,7 +79,8 @@ struct LnGateOut {
 bool ln_gate_out_supported(int dtype, long long M, long long plane);
 int ln_gate_out(cudaStream_t st, const LnGateOut& p);
 
-// Input gate backward: dP, dG of both halves from the recomputed projections of z and the gradients of a and b.
+// Input gate backward: dP, dG of both halves from the recomputed projections of z and the gradients of a and b, and their
+// products with z summed over the pixels.
 struct GateInBwd {
   int dtype;                 // fp32: TF32 products
   long long M;               // pixels (one batch entry)
@@ -89,10 +91,12 @@ struct GateInBwd {
   const void* da_cm;         // [128, M]
   const void* db_cm;
   void* dpg;                 // [512, M]: rows [dP_a; dG_a; dP_b; dG_b]
+  float* partial;            // [gate_in_bwd_parts][512, 128]: parts of dPG z, or null
   bool first = false;        // as above
   int* err;
 };
 bool gate_in_bwd_supported(int dtype, long long M, long long plane);
+int gate_in_bwd_parts(int dtype, long long M);   // one for every two SMs at most
 int gate_in_bwd(cudaStream_t st, const GateInBwd& p);
 
 }  // namespace tc

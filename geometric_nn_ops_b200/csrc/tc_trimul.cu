@@ -796,12 +796,14 @@ int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void
   const int blocks = std::min(cdiv(M, 128), sm_count());
   float* pg = partial + kWgradPartialFloats;
   float* pb = pg + (size_t)kPersist * CW;
+  const bool want_w = g->p_in_w || g->g_in_w;   // reduced at the end of the phase together with the LayerNorm partials
   int nparts = 0;
   if (gate_in_bwd_supported(gm.dtype, M, gm.plane) && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) {
     GateInBwd f;
     f.dtype = gm.dtype; f.M = M; f.z = z; f.wcat = pr.wcat; f.bias_cat = (w->p_in_b || w->g_in_b) ? pr.bias_cat : nullptr;
-    f.mask = mask; f.da_cm = da_cm; f.db_cm = db_cm; f.dpg = dpg; f.first = pr.first; f.err = pr.err;
+    f.mask = mask; f.da_cm = da_cm; f.db_cm = db_cm; f.dpg = dpg; f.partial = want_w ? partial : nullptr; f.first = pr.first; f.err = pr.err;
     TRI_TRY(gate_in_bwd(st, f));
+    if (want_w) nparts = gate_in_bwd_parts(gm.dtype, M);
   } else {
     GemmPlan p;   // input gate backward fused into the recomputed projection GEMM
     gate_in_operands(&p, gm, pr, z);
@@ -809,9 +811,8 @@ int phase_project_bwd(cudaStream_t st, const Geom& gm, const void* x, const void
     p.aux = mask; p.aux2 = da_cm; p.aux3 = db_cm; p.plane = gm.plane; p.first = pr.first;
     p.name = "tc_gemm_gate_in_bwd"; p.flops = 0.0; p.bytes = 7.0 * gm.unit();
     TRI_TRY(launch_gemm(st, gm.dtype, EPI_GATE_IN_BWD, 256, false, p, pr.err));
+    if (want_w) TRI_TRY(split_k_grad(st, gm, dpg, 4 * CW, z, partial, pr.err, "tc_gemm_wgrad", &nparts, /*lhs_channel_major=*/true));
   }
-  if (g->p_in_w || g->g_in_w)   // reduced at the end of the phase together with the LayerNorm partials
-    TRI_TRY(split_k_grad(st, gm, dpg, 4 * CW, z, partial, pr.err, "tc_gemm_wgrad", &nparts, /*lhs_channel_major=*/true));
   if (g->p_in_b || g->g_in_b) {
     KernelTimer kt("tc_rowsum", st, 0.0, 4.0 * gm.unit());
     rowsum_wcat_kernel<T><<<4 * CW, 256, 0, st>>>((const T*)dpg, M, g->p_in_b, g->g_in_b);

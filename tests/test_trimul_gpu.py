@@ -263,3 +263,16 @@ def test_operands_on_another_device_are_refused(tmu, name):
         w[name] = w[name].cpu()
     with pytest.raises(ValueError, match=name):
         tmu(x, "outgoing", mask, **w)
+
+
+@pytest.mark.parametrize("n", [8, 72, 104])
+@pytest.mark.parametrize("dtype,precision", [m for m in MODES if m != (torch.float32, "ieee")], ids=lambda v: str(v).replace("torch.", ""))
+def test_input_weight_gradients_over_few_tiles(tmu, n, dtype, precision):
+    """The sums of the input gate's backward: one tile (fp32: two) for all CTAs, CTAs with one or two, and with two or three
+    (fp32: three to five), so that every buffer is used, and not used, a second time."""
+    x, mask, w, d_out = util.trimul_inputs(1, n, 128, 128, dtype, seed=n)
+    with util.matmul_precision(precision):
+        _, grads = util.trimul_fwd_bwd(tmu, x, mask, w, "outgoing", d_out)
+    _, g_ref = util.trimul_oracle(x, mask, w, "outgoing", d_out)
+    for name in ("x", "p_in_weight", "g_in_weight"):
+        util.check_close("grad_" + name, grads[name], g_ref[name], *_tol(dtype, precision))
