@@ -38,8 +38,8 @@ struct AttnArgs {
   void* o;
   int64_t o_st[4];
   float* stats;          // [2][B][S][H][N]: row max, log row sum
-  const float* mask_terms;   // [B][S][npad] additive key-mask terms (0, -1e9, or -inf beyond N)
-  int npad;                  // N rounded up to 128
+  const uint8_t* mask;   // [B][S][N] key masks, or null
+  int64_t mask_st[2];
   int bias_b_mul;        // 0 when the bias is broadcast over the batch
   uint32_t idesc_s, idesc_pv;
   int* err;
@@ -61,28 +61,15 @@ template <int HD> struct Geo {
   static constexpr int SMEM = OFF_BAR + 256 + 1024;      // + alignment slack
 };
 
-// additive key-mask terms of every (batch, row): 0 for a kept key, -1e9 for a masked key, -inf beyond N; rows of
-// npad.  With n_flags > 0 (the backward) a second plane holds them times log2(e), and the flags of the rows are cleared.
-// Also clears the error word of the launches that follow.
-__global__ void mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b, int64_t st_s, int B, int S, int N, int npad,
-                                  float* __restrict__ out, int* err, int* __restrict__ flags, long long n_flags) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx == 0) {
-    *err = 0;
-    __threadfence();   // before the kernels that follow may start
-  }
+__global__ void __launch_bounds__(256) mask_terms_kernel(const uint8_t* __restrict__ mask, int64_t st_b, int64_t st_s, int B, int S, int N, int npad,
+                                                         float* __restrict__ out, int* err) {
   dependent_trigger();
-  const long long n = (long long)B * S * npad;
-  for (long long i = idx; i < n_flags; i += (long long)gridDim.x * blockDim.x) flags[i] = 0;
-  if (idx >= n) return;
-  const int k = idx % npad;
-  const long long bs = idx / npad;
-  const int s = bs % S, b = bs / S;
-  float v = 0.f;
-  if (k >= N) v = -INFINITY;
-  else if (mask != nullptr) v = kMaskSentinel * ((mask[b * st_b + s * st_s + k] ? 1.0f : 0.0f) - 1.0f);
-  out[idx] = v;
-  if (n_flags > 0) out[n + idx] = v * kLog2e;
+  const long long idx = blockIdx.x * 256LL + threadIdx.x;
+  if (idx == 0) *err = 0;
+  if (idx >= (long long)B * S * npad) return;
+  const int k = (int)(idx % npad);
+  const long long bs = idx / npad, b = bs / S, s = bs - b * S;
+  out[idx] = mask_term(mask != nullptr && k < N ? mask[b * st_b + s * st_s + k] : 1u, k < N);
 }
 
 // 320 threads.  Warps 0-7 do the softmax arithmetic: thread (r, hh) owns query row r and the 64-key half hh of each
@@ -149,6 +136,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(bar_s, 1); mbar_init(bar_p, 8);
     for (int i = 0; i < 4; ++i) mbar_init(&bar_free[i], 8);
     mbar_fence_init();
+    *a.err = 0;   // (by every CTA: its waits read the word.  One that gives up does so two seconds after all have started)
   }
   if (warp == 0) tmem_alloc(tmem_slot, 256);
   tc_fence_before_sync();
@@ -166,60 +154,75 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   bool ok = true;
 
   if (warp == 9) {
-    if (lane == 0) {
-      // ---------------------------------- TMA copies ---------------------------------------------
-      auto load_q = [&](int n) {
-        const Item it = item_of(n);
-        mbar_expect_tx(bar_q, G::TILE);
-        tma_load_5d(sQ, &tmQ, bar_q, 0, it.h, it.q0, it.s, it.b);
-      };
-      // tile c of the stream: item `it`, key tile t of that item
-      auto load_k = [&](int c, const Item& it, int t) {
-        const int stg = c & 1;
-        mbar_expect_tx(&bar_k[stg], G::TILE + 512);
-        tma_load_5d(sK + stg * G::TILE, &tmK, &bar_k[stg], 0, it.h, t * 128, it.s, it.b);
-        bulk_load(sMb + stg * 128, a.mask_terms + ((long long)it.b * a.S + it.s) * a.npad + t * 128, 512, &bar_k[stg]);
-      };
-      auto load_v = [&](int c, const Item& it, int t) {
-        const int stg = c & 1;
-        mbar_expect_tx(&bar_v[stg], G::TILE);
-        tma_load_5d(sV + stg * G::TILE, &tmV, &bar_v[stg], 0, it.h, t * 128, it.s, it.b);
-      };
-      auto load_bias = [&](int c, const Item& it, int t) {
-        uint64_t* bb = &bar_bias[c & 1];
-        uint8_t* dst = sP + (c & 1) * 32768;
-        mbar_expect_tx(bb, 32768);
-        tma_load_4d(dst, &tmBias, bb, t * 128, it.q0, it.h, it.b * a.bias_b_mul);
-        tma_load_4d(dst + 16384, &tmBias, bb, t * 128 + 64, it.q0, it.h, it.b * a.bias_b_mul);
-      };
-      // (la_n, la_t): item and key tile of the stream position being loaded, two tiles ahead of the consumers
-      int la_n = 0, la_t = 0;
-      Item la = item_of(0);
-      auto advance = [&]() {
-        if (++la_t == nt) { la_t = 0; ++la_n; if (la_n < my_items) la = item_of(la_n); }
-      };
-      if (total > 0) load_q(0);
-      for (int c = 0; c < 2 && c < total; ++c) {
-        load_k(c, la, la_t);
-        if (HB) load_bias(c, la, la_t);
-        load_v(c, la, la_t);
-        advance();
+    // ---------------------------------- TMA copies, mask terms -----------------------------------
+    // The warp runs together: a lane writes the terms of four keys of a tile, lane 0 issues the copies.
+    auto load_q = [&](int n) {
+      if (lane != 0) return;
+      const Item it = item_of(n);
+      mbar_expect_tx(bar_q, G::TILE);
+      tma_load_5d(sQ, &tmQ, bar_q, 0, it.h, it.q0, it.s, it.b);
+    };
+    uint32_t kept[4];
+    auto fetch_mask = [&](const Item& it, int t) {   // of key tile t, in time for its load_k
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = t * 128 + lane * 4 + e;
+        kept[e] = a.mask != nullptr && k < a.N ? a.mask[it.b * a.mask_st[0] + it.s * a.mask_st[1] + k] : 1u;
       }
-      int jt = 0, n_cur = 0;   // key tile and item of stream position c
-      for (int c = 0; c < total && ok; ++c) {
-        ok = mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16) && ok;   // S(c) has been read: its K stage and mask terms are free
-        if (++jt == nt) {                                    // ... and it was the item's last use of Q
-          jt = 0;
-          if (++n_cur < my_items) load_q(n_cur);
-        }
-        if (c + 2 < total) {
-          load_k(c + 2, la, la_t);
-          if (HB && TMEM_P) load_bias(c + 2, la, la_t);      // the bias tile has been read too and P does not replace it
-          ok = mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, a.err, 15) && ok;   // P V(c) done: its V stage and P buffer are free
-          if (HB && !TMEM_P) load_bias(c + 2, la, la_t);
-          load_v(c + 2, la, la_t);
-          advance();
-        }
+    };
+    // tile c of the stream: item `it`, key tile t of that item
+    auto load_k = [&](int c, const Item& it, int t) {
+      const int stg = c & 1, k = t * 128 + lane * 4;
+      reinterpret_cast<float4*>(sMb + stg * 128)[lane] = make_float4(mask_term(kept[0], k < a.N), mask_term(kept[1], k + 1 < a.N),
+                                                                     mask_term(kept[2], k + 2 < a.N), mask_term(kept[3], k + 3 < a.N));
+      __syncwarp();
+      if (lane != 0) return;
+      mbar_expect_tx(&bar_k[stg], G::TILE);
+      tma_load_5d(sK + stg * G::TILE, &tmK, &bar_k[stg], 0, it.h, t * 128, it.s, it.b);
+    };
+    auto load_v = [&](int c, const Item& it, int t) {
+      if (lane != 0) return;
+      const int stg = c & 1;
+      mbar_expect_tx(&bar_v[stg], G::TILE);
+      tma_load_5d(sV + stg * G::TILE, &tmV, &bar_v[stg], 0, it.h, t * 128, it.s, it.b);
+    };
+    auto load_bias = [&](int c, const Item& it, int t) {
+      if (lane != 0) return;
+      uint64_t* bb = &bar_bias[c & 1];
+      uint8_t* dst = sP + (c & 1) * 32768;
+      mbar_expect_tx(bb, 32768);
+      tma_load_4d(dst, &tmBias, bb, t * 128, it.q0, it.h, it.b * a.bias_b_mul);
+      tma_load_4d(dst + 16384, &tmBias, bb, t * 128 + 64, it.q0, it.h, it.b * a.bias_b_mul);
+    };
+    // (la_n, la_t): item and key tile of the stream position being loaded, two tiles ahead of the consumers
+    int la_n = 0, la_t = 0;
+    Item la = item_of(0);
+    auto advance = [&]() {
+      if (++la_t == nt) { la_t = 0; ++la_n; if (la_n < my_items) la = item_of(la_n); }
+    };
+    if (total > 0) load_q(0);
+    for (int c = 0; c < 2 && c < total; ++c) {
+      fetch_mask(la, la_t);
+      load_k(c, la, la_t);
+      if (HB) load_bias(c, la, la_t);
+      load_v(c, la, la_t);
+      advance();
+    }
+    int jt = 0, n_cur = 0;   // key tile and item of stream position c
+    for (int c = 0; c < total && ok; ++c) {
+      if (c + 2 < total) fetch_mask(la, la_t);
+      ok = mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16) && ok;   // S(c) has been read: its K stage and mask terms are free
+      if (++jt == nt) {                                    // ... and it was the item's last use of Q
+        jt = 0;
+        if (++n_cur < my_items) load_q(n_cur);
+      }
+      if (c + 2 < total) {
+        load_k(c + 2, la, la_t);
+        if (HB && TMEM_P) load_bias(c + 2, la, la_t);      // the bias tile has been read too and P does not replace it
+        ok = mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, a.err, 15) && ok;   // P V(c) done: its V stage and P buffer are free
+        if (HB && !TMEM_P) load_bias(c + 2, la, la_t);
+        load_v(c + 2, la, la_t);
+        advance();
       }
     }
   } else if (warp == 8) {
@@ -1382,66 +1385,141 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
 }
 
-// delta[b,s,h,i] = sum_d dO * O (written where the dQ pass reads it); the row constants of the backward passes as factors (see
-// RowFactors), and for flagged rows in the form their packed arithmetic adds (prep[0] = -m, prep[1] = -log l * log2e,
-// prep[2] = -delta); rows padded to npad entries with zeros.  A block has 128 queries of a (batch, row), all heads of a query
-// one after the other: they share its cache lines.
+// What the backward passes read besides the tensors, in one launch.
+//   delta[b,s,h,i] = sum_d dO * O (written where the dQ pass reads it); the row constants as factors (see RowFactors), and for flagged
+//   rows in the form their packed arithmetic adds (prep[0] = -m, prep[1] = -log l * log2e, prep[2] = -delta); padded to npad entries
+//   with zeros.  A block has a (batch, row, head), a warp 32 of its queries at a time, four lanes to a query: a request covers rows of
+//   64 bytes whole.
+//   The key-mask terms of a (batch, row), by its first head's block: 0 for a kept key, -1e9 for a masked one, -inf beyond N; and in a
+//   second plane times log2(e).
+//   The first blocks transpose the bias instead: out[b][h][k][q] = bias[b][h][q][k], a 64 x 64 tile each.
+// One launch in place of four.  At 301 x 301 residues, 4 heads of 32: 22 us against 18 + 3 + 9 and the gaps between them; at 768 x 768
+// 97 against 88 + 5 + 11, where the bytes are 60: what it waits for is the load, sum, exchange and store of an item, with 24 warps an SM
+// on it (three blocks; two 127).  Also clears the error word.
+struct PrepareArgs {
+  const float* stats;
+  float *delta, *prep, *mask_terms;
+  uint4* aug;
+  int* large;
+  int* err;
+  const uint8_t* mask;
+  const uint16_t* bias;
+  uint16_t* bias_t;
+  int npad, pitch, tiles, transposes;   // tiles of a side of the bias; blocks that transpose
+};
 template <typename T>
-__global__ void __launch_bounds__(128) attn_delta_tc_kernel(TriAttnDesc d, const T* o, const T* d_o, const float* stats, float* delta,
-                                                            float* prep, uint4* aug, int* large, int npad) {
-  const unsigned chunks = npad / 128, bs = blockIdx.x / chunks;
-  const int i = (blockIdx.x - bs * chunks) * 128 + threadIdx.x;
-  const unsigned b = bs / (unsigned)d.n_seq, s = bs - b * (unsigned)d.n_seq;
-  const long long plane = (long long)d.B * d.n_seq * d.H * npad, total = (long long)d.B * d.n_seq * d.H * d.n_res;
-  const bool in = i < d.n_res;
-  const T* orow = o + b * d.o_st[0] + s * d.o_st[1] + i * d.o_st[2];
-  const T* grow = d_o + b * d.do_st[0] + s * d.do_st[1] + i * d.do_st[2];
-#pragma unroll 2
-  for (int h = 0; h < d.H; ++h) {
-    const long long row = (long long)bs * d.H + h, at = row * npad + i, idx = row * d.n_res + i;
-    float acc = 0.f, m = 0.f, ll = 0.f;
-    if (in) {
-      m = stats[idx];
-      ll = stats[total + idx];
-      for (int g = 0; g < d.D / 8; ++g) {
-        float x[8], y[8];
-        unpack8<T>(reinterpret_cast<const uint4*>(orow + h * d.o_st[3])[g], x);
-        unpack8<T>(reinterpret_cast<const uint4*>(grow + h * d.do_st[3])[g], y);
+__global__ void __launch_bounds__(256, 3) attn_prepare_kernel(const TriAttnDesc d, const T* o, const T* d_o, const PrepareArgs a) {
+  __shared__ uint16_t tile[64][66];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = d.n_res;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
+  if ((int)blockIdx.x < a.transposes) {
+    unsigned z = blockIdx.x;
+    const int k0 = (int)(z % (unsigned)a.tiles) * 64; z /= (unsigned)a.tiles;
+    const int q0 = (int)(z % (unsigned)a.tiles) * 64, bh = (int)(z / (unsigned)a.tiles);
+    const uint16_t* src = a.bias + bh / d.H * d.bias_st[0] + bh % d.H * d.bias_st[1];
+    uint16_t* dst = a.bias_t + (int64_t)bh * N * a.pitch;
+    for (int i = warp; i < 64; i += 8)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc = fmaf(x[e], y[e], acc);
-      }
-      if (delta != nullptr) delta[idx] = acc;
+      for (int e = 0; e < 64; e += 32)
+        if (q0 + i < N && k0 + lane + e < N) tile[i][lane + e] = src[(q0 + i) * d.bias_st[2] + k0 + lane + e];
+    __syncthreads();
+    for (int i = warp; i < 64; i += 8)
+#pragma unroll
+      for (int e = 0; e < 64; e += 32)
+        if (k0 + i < N && q0 + lane + e < N) dst[(int64_t)(k0 + i) * a.pitch + q0 + lane + e] = tile[lane + e][i];
+    return;
+  }
+  const unsigned row = blockIdx.x - a.transposes, bs = row / (unsigned)d.H, h = row - bs * (unsigned)d.H;
+  const unsigned b = bs / (unsigned)d.n_seq, s = bs - b * (unsigned)d.n_seq;
+  const long long planes = (long long)d.B * d.n_seq, plane = planes * d.H * a.npad, total = planes * d.H * N;
+  if (h == 0) {
+    for (int k = threadIdx.x; k < a.npad; k += 256) {
+      const float v = mask_term(a.mask != nullptr && k < N ? a.mask[b * d.mask_st[0] + s * d.mask_st[1] + k] : 1u, k < N);
+      a.mask_terms[(long long)bs * a.npad + k] = v;
+      a.mask_terms[(planes + bs) * a.npad + k] = v * kLog2e;
     }
+  }
+  const T* ob = o + b * d.o_st[0] + s * d.o_st[1] + h * d.o_st[3];
+  const T* gb = d_o + b * d.do_st[0] + s * d.do_st[1] + h * d.do_st[3];
+  const int pieces = d.D / 8;
+  int flag = 0;
+  for (int n0 = warp * 32; n0 < a.npad; n0 += 256) {
+    const int i = n0 + lane;   // this lane's query once the sums are there
+    const long long at = (long long)row * a.npad + i, idx = (long long)row * N + i;
+    const bool in = i < N;
+    const float m = in ? a.stats[idx] : 0.f, ll = in ? a.stats[total + idx] : 0.f;
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = lane & 3; c < pieces; c += 4) {
+      uint4 x[4], y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int n = n0 + e * 8 + (lane >> 2);
+        x[e] = y[e] = make_uint4(0, 0, 0, 0);
+        if (n < N) {
+          x[e] = reinterpret_cast<const uint4*>(ob + n * d.o_st[2])[c];
+          y[e] = reinterpret_cast<const uint4*>(gb + n * d.do_st[2])[c];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float u[8], w[8];
+        unpack8<T>(x[e], u);
+        unpack8<T>(y[e], w);
+#pragma unroll
+        for (int f = 0; f < 8; ++f) part[e] = fmaf(u[f], w[f], part[e]);
+      }
+    }
+    __syncwarp();
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      part[e] += __shfl_xor_sync(0xffffffffu, part[e], 1);
+      part[e] += __shfl_xor_sync(0xffffffffu, part[e], 2);
+      const float v = __shfl_sync(0xffffffffu, part[e], (lane & 7) * 4);
+      if (lane >> 3 == e) acc = v;
+    }
+    if (in && a.delta != nullptr) a.delta[idx] = acc;
     const float c = in ? -(m + ll) / d.scale : 0.f;
     const bool fits = RowFactors::fits<T>(m, c, acc);
-    if (!fits) large[row] = 1;
-    aug[at] = fits ? RowFactors::pack<T>(c, -acc) : make_uint4(0, 0, 0, 0);
-    prep[at] = -m;
-    prep[plane + at] = -ll * kLog2e;
-    prep[2 * plane + at] = -acc;
+    if (!fits) flag = 1;
+    a.aug[at] = fits ? RowFactors::pack<T>(c, -acc) : make_uint4(0, 0, 0, 0);
+    a.prep[at] = -m;
+    a.prep[plane + at] = -ll * kLog2e;
+    a.prep[2 * plane + at] = -acc;
   }
+  flag = __syncthreads_or(flag);
+  if (threadIdx.x == 0) a.large[row] = flag;
 }
 
 // dq = scale * sum over key blocks of the merged pass's partials ([nparts][B][S][N][H][D] contiguous), added in key
 // block order in fp32; 8 elements per thread.
+// (Rows are counted in 32 bits: 2^31 of them would not fit the device.  With the divisions in 64 bits and a load at a time
+// 22.5 us at 301 x 301 residues, 4 heads of 32, 18.9 now; the bytes are 14.)
 template <typename T>
-__global__ void attn_dq_sum_kernel(const T* __restrict__ part, int nparts, long long plane, TriAttnDesc d, T* __restrict__ dq) {
+__global__ void __launch_bounds__(256) attn_dq_sum_kernel(const T* __restrict__ part, int nparts, long long plane, TriAttnDesc d, T* __restrict__ dq) {
   dependent_trigger();
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long c = blockIdx.x * 256LL + threadIdx.x;
   if (c >= plane / 8) return;
-  const int dc = d.D / 8;
-  long long z = c;
-  const int d8 = z % dc; z /= dc;
-  const int h = z % d.H; z /= d.H;
-  const int q = z % d.n_res; z /= d.n_res;
-  const int s = z % d.n_seq; const int b = z / d.n_seq;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int p = 0; p < nparts; ++p) {
+  auto add = [&](const uint4& w) {
     float v[8];
-    unpack8<T>(*reinterpret_cast<const uint4*>(part + p * plane + c * 8), v);
+    unpack8<T>(w, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] += v[e];
+  };
+  const uint4* src = reinterpret_cast<const uint4*>(part) + c;
+  const long long step = plane / 8;
+  int p = 0;
+  for (; p + 3 <= nparts; p += 3, src += 3 * step) {
+    const uint4 w0 = src[0], w1 = src[step], w2 = src[2 * step];
+    add(w0); add(w1); add(w2);
   }
+  for (; p < nparts; ++p, src += step) add(*src);
+  const unsigned dc = d.D / 8;
+  unsigned z = (unsigned)(c / dc);
+  const unsigned d8 = (unsigned)(c - (long long)z * dc), h = z % (unsigned)d.H; z /= (unsigned)d.H;
+  const unsigned q = z % (unsigned)d.n_res; z /= (unsigned)d.n_res;
+  const unsigned b = z / (unsigned)d.n_seq, s = z - b * (unsigned)d.n_seq;
   uint4 pk;
   pk.x = pack2<T>(acc[0] * d.scale, acc[1] * d.scale); pk.y = pack2<T>(acc[2] * d.scale, acc[3] * d.scale);
   pk.z = pack2<T>(acc[4] * d.scale, acc[5] * d.scale); pk.w = pack2<T>(acc[6] * d.scale, acc[7] * d.scale);
@@ -1498,32 +1576,6 @@ int launch_pad_bias(const TriAttnDesc* d, const void* bias, void* copy, cudaStre
   return 0;
 }
 
-// out[b][h][k][q] = bias[b][h][q][k] for 16-bit elements (the dK/dV pass reads keys as rows)
-__global__ void transpose_bias_kernel(const uint16_t* __restrict__ in, int64_t st_b, int64_t st_h, int64_t st_q, int n, int H,
-                                      int pitch, uint16_t* __restrict__ out) {
-  __shared__ uint16_t tile[64][66];
-  dependent_trigger();
-  const int bh = blockIdx.z, b = bh / H, h = bh % H;
-  const uint16_t* src = in + b * st_b + h * st_h;
-  uint16_t* dst = out + (int64_t)bh * n * pitch;
-  const int q0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
-  for (int i = threadIdx.y; i < 64; i += blockDim.y) {
-    const int q = q0 + i;
-    for (int jj = threadIdx.x; jj < 64; jj += 32) {
-      const int k = k0 + jj;
-      tile[i][jj] = (q < n && k < n) ? src[q * st_q + k] : (uint16_t)0;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 64; i += blockDim.y) {
-    const int k = k0 + i;
-    for (int jj = threadIdx.x; jj < 64; jj += 32) {
-      const int q = q0 + jj;
-      if (k < n && q < n) dst[(int64_t)k * pitch + q] = tile[jj][i];
-    }
-  }
-}
-
 template <typename KernelT>
 int set_dyn_smem(KernelT kern, int bytes) {
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -1565,9 +1617,14 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   const long long prep_plane = (long long)d->B * d->n_seq * d->H * npad;
   {
     KernelTimer kt("tc_attn_delta", st, 0.0, 2.0 * tensor_bytes);
-    TRI_TRY(launch_mask_terms(d, mask, w.mask_terms, w.err, w.large, st));
-    attn_delta_tc_kernel<T><<<(unsigned)(d->B * (long long)d->n_seq * (npad / 128)), 128, 0, st>>>(
-        *d, (const T*)o, (const T*)d_o, stats, HD == 32 ? nullptr : w.delta, w.prep, w.aug, w.large, npad);
+    PrepareArgs p;
+    p.stats = stats; p.delta = HD == 32 ? nullptr : w.delta; p.prep = w.prep; p.mask_terms = w.mask_terms; p.aug = w.aug; p.large = w.large;
+    p.err = w.err; p.mask = mask; p.bias = static_cast<const uint16_t*>(bias); p.bias_t = static_cast<uint16_t*>(w.bias_t);
+    p.npad = npad; p.pitch = bias_pitch(d); p.tiles = cdiv(d->n_res, 64);
+    p.transposes = bias != nullptr ? p.tiles * p.tiles * bias_batches(d) * d->H : 0;
+    const long long planes = (long long)d->B * d->n_seq;
+    const long long blocks = p.transposes + planes * d->H;
+    attn_prepare_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(*d, (const T*)o, (const T*)d_o, p);
     TRI_LAUNCH_OK();
   }
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
@@ -1586,10 +1643,6 @@ int bwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 128, HD));
   TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 128, HD));
   if (bias) {   // the dK/dV pass (thread = key) reads a transposed copy of the bias: [b][h][key][query]
-    transpose_bias_kernel<<<dim3(cdiv(d->n_res, 64), cdiv(d->n_res, 64), bias_batches(d) * d->H), dim3(32, 8), 0, st>>>(
-        static_cast<const uint16_t*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2], d->n_res, d->H, bias_pitch(d),
-        static_cast<uint16_t*>(w.bias_t));
-    TRI_LAUNCH_OK();
     TRI_TRY(bias_map(&tb, bias, w.bias_t, d, 128));
   } else {
     tb = tq;
@@ -1681,23 +1734,22 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   AttnArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D; a.scale = d->scale;
   a.o = o; for (int i = 0; i < 4; ++i) a.o_st[i] = d->o_st[i];
-  a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
+  a.stats = stats; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
   a.bias_b_mul = d->bias_st[0] != 0 ? 1 : 0;
-  TRI_TRY(launch_mask_terms(d, mask, mask_terms, err, nullptr, st));
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   a.idesc_s = make_idesc(kind, 128, 128, false, false);
   a.idesc_pv = make_idesc(kind, 128, HD, false, true);
   a.err = err;
-  if (bias != nullptr) {
-    const bool own = bias_fits_tma(d, bias);
-    if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
-    TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
-  }
+  const bool own = bias == nullptr || bias_fits_tma(d, bias);   // (else a copy with padded rows is the first kernel)
+  if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
+  if (bias != nullptr) TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
   if (rows) {
+    const bool terms = wants_mask_terms(d);
+    if (terms) TRI_TRY(launch_mask_terms(d, mask, mask_terms, err, st));
     TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, 32));
     TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 64, 32));
     TRI_TRY(qkv_tile_map(&tv, v, d, d->v_st, 64, 32));
-    return attn_fwd_rows(d, tq, tk, tv, bias ? &tb : nullptr, a.bias_b_mul != 0, o, stats, mask_terms, err, st);
+    return attn_fwd_rows(d, tq, tk, tv, bias ? &tb : nullptr, a.bias_b_mul != 0, mask, terms ? mask_terms : nullptr, o, stats, err, own && !terms, st);
   }
   TRI_TRY(qkv_tile_map(&tq, q, d, d->q_st, 128, HD));
   TRI_TRY(qkv_tile_map(&tk, k, d, d->k_st, 128, HD));
@@ -1708,18 +1760,19 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto kern = bias != nullptr ? attn_fwd_tc_kernel<T, HD, true> : attn_fwd_tc_kernel<T, HD, false>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<HD>::SMEM));
-  launch_dependent(us_of_logits(pairs), kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
+  launch_dependent(own ? kLaunchPlainly : us_of_logits(pairs), kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
   TRI_LAUNCH_OK();
   return 0;
 }
 
 }  // namespace
 
-int launch_mask_terms(const TriAttnDesc* d, const uint8_t* mask, float* out, int* err, int* flags, cudaStream_t st) {
+bool wants_mask_terms(const TriAttnDesc* d) {
+  return us_of_logits((double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res) >= kEarlyStartUs;
+}
+int launch_mask_terms(const TriAttnDesc* d, const uint8_t* mask, float* out, int* err, cudaStream_t st) {
   const int npad = (d->n_res + 127) / 128 * 128;
-  const long long n = (long long)d->B * d->n_seq * npad;
-  mask_terms_kernel<<<cdiv(n, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, out, err, flags,
-                                                  flags != nullptr ? (long long)d->B * d->n_seq * d->H : 0LL);
+  mask_terms_kernel<<<cdiv((long long)d->B * d->n_seq * npad, 256), 256, 0, st>>>(mask, d->mask_st[0], d->mask_st[1], d->B, d->n_seq, d->n_res, npad, out, err);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -1780,11 +1833,10 @@ bool attn_bwd_supported(const TriAttnDesc* d) {
          strides_ok(d, d->dv_st) && d->n_seq <= 65535;
 }
 
-static size_t attn_npad(const TriAttnDesc* d) { return ((size_t)d->n_res + 127) / 128 * 128; }
-
 // everything but the padded copy of the bias, which comes last
 static size_t attn_ws_base(const TriAttnDesc* d, int is_bwd) {
-  if (!is_bwd) return 512 + align_up((size_t)d->B * d->n_seq * attn_npad(d) * sizeof(float));   // additive key-mask terms
+  // (the status word, the key-mask terms)
+  if (!is_bwd) return 512 + (wants_mask_terms(d) ? align_up((size_t)d->B * d->n_seq * ((d->n_res + 127) / 128 * 128) * sizeof(float)) : 0);
   Arena a(nullptr, 0);
   BwdWs w;
   carve_bwd(a, d, &w);

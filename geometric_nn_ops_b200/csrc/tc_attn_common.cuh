@@ -15,6 +15,9 @@ __device__ __forceinline__ int sw128_chunk(int r, int g) {
   return (g >> 3) * 16384 + r * 128 + (((g & 7) ^ (r & 7)) << 4);
 }
 
+// the additive term of a key: 0 where it is kept, -1e9 where it is masked, -inf beyond the row
+__device__ __forceinline__ float mask_term(uint32_t kept, bool in) { return !in ? -INFINITY : kept != 0 ? 0.0f : -kMaskSentinel; }
+
 template <typename T> struct ElemIsBf16 { static constexpr bool value = false; };
 template <> struct ElemIsBf16<__nv_bfloat16> { static constexpr bool value = true; };
 
@@ -33,6 +36,15 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 }
 __device__ __forceinline__ float2 pair(uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); }
 __device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
+
+// a pair plus the 16-bit pair of a word, as two additions that widen their operand on the way
+template <typename T> __device__ __forceinline__ float2 add_wide(float2 x, uint32_t w) {
+  if constexpr (ElemIsBf16<T>::value)
+    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; add.rn.f32.bf16 %0, lo, %0; add.rn.f32.bf16 %1, hi, %1; }" : "+f"(x.x), "+f"(x.y) : "r"(w));
+  else
+    asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %2; add.rn.f32.f16 %0, lo, %0; add.rn.f32.f16 %1, hi, %1; }" : "+f"(x.x), "+f"(x.y) : "r"(w));
+  return x;
+}
 
 template <typename T>
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {

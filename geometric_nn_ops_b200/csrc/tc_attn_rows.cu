@@ -24,9 +24,10 @@
 // that the softmax warps owe.  With S single buffered each step waited about 600 clocks for the next product, and the
 // waiting warps' polling took half of all issue slots.
 //
-// What bounds it: the exponentials (16 per clock and SM: 8 clocks of a sub-partition per 32), then the waits a row's four
-// warps, which run on four sub-partitions, have for one another.  N = 768, 4 heads, bf16: 0.72 ms, 59 % of the exponential
-// pipe (which also converts), against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
+// What bounds it: the instructions of a step (about 330 per warp, three warps to a sub-partition), then the waits a row's four warps,
+// which run on four sub-partitions, have for one another.  A quarter of the exponentials as polynomials on the FMA pipe: 714 -> 784 us.
+// The bias added by two additions that widen it, in place of two conversions and a packed addition: 714 -> 689.  N = 768, 4
+// heads, bf16: 0.69 ms, 62 % of the exponential pipe (which also converts), against 1.05 ms and 41 % for the kernel with two CTAs per SM, two threads per row and a maximum per step (which
 // also read 2 bytes of bias per logit from L2; here 0.67).
 #include <algorithm>
 #include <type_traits>
@@ -73,12 +74,14 @@ struct RowsArgs {
   void* o;
   int64_t o_st[4];
   float* stats;              // [2][B][S][H][N]: row maximum, log row sum
-  const float* mask_terms;
+  const float* mask_terms;   // [B][S][npad] (mask_term), or null: made here
   int npad;
   int bias_b_mul;
   int rows_per_item;         // groups in use (fewer where a triple per CTA would leave SMs idle)
   uint32_t idesc_s, idesc_pv;
   int* err;
+  const uint8_t* mask;       // [B][S][N], or null
+  int64_t mask_st[2];
 };
 
 // barriers of one group
@@ -97,7 +100,8 @@ __device__ __forceinline__ void ld_wait16(uint32_t (&v)[16]) {
                  "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 
-template <typename T, bool HB>
+// TERMS: the mask terms were made before
+template <typename T, bool HB, bool TERMS>
 __global__ void __launch_bounds__(RowsCfg<T>::kThreads, 1)
 attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias, const RowsArgs a) {
@@ -133,7 +137,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int i = 0; i < 3; ++i) mbar_init(&bars[g].in[i], 1);
       mbar_init(&bars[g].mma[0], 1); mbar_init(&bars[g].mma[1], 1); mbar_init(&bars[g].p_ready[0], 4); mbar_init(&bars[g].p_ready[1], 4);
     }
-    for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_free[i], 4 * R); }
+    for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], TERMS ? 1 : 2); mbar_init(&b_free[i], 4 * R); }
     mbar_fence_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
@@ -142,30 +146,101 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   dependent_trigger();
-  if constexpr (M::F32) dependent_wait();   // (else q, k, v are the caller's: only mask terms and a copied bias come from before)
+  if constexpr (M::F32) dependent_wait();   // (else q, k, v are the caller's: only a copied bias comes from before)
   constexpr uint32_t COLS = M::F32 ? 224 : 160, COL_O = 128, COL_LO = 160;   // a group's columns: S / P of even and odd steps at
                                                                              // 0 and 64, O, (fp32) what P's upper bits leave
   bool ok = true;
+  // 512 threads of 128 registers: the issuing warps give some of theirs to the softmax warps (12 x 152 + 4 x 56 = 16 x 128), whose step
+  // did not fit: 721 -> 714 us at N = 768, 4 heads (with the additions of `add_wide` 730 at 144 and 72, 695 at 152 and 48, 689 so;
+  // at 160 and 32 the issuing warps spill: 775).
+  if constexpr (!M::F32) {
+    static_assert(M::kThreads == 512 && kGroups == 3);
+    if (warp >= 4 * kGroups) regs_dec<56>();
+    else regs_inc<152>();
+  }
 
   if (warp == 5 * kGroups) {
     // ------------------------------------ bias tiles and mask terms --------------------------------
-    if (lane == 0) {
+    if constexpr (TERMS) {
+      if (lane == 0) {
+        dependent_wait();
+        int stg = 0;
+        uint32_t ph = 0;
+        for (int n = 0; n < my_items && ok; ++n) {
+          const Item it = item_of(n);
+          for (int j = 0; j < nk; ++j) {
+            ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51);
+            if (!ok) break;
+            const int rows = min(R, a.S - it.s0);
+            mbar_expect_tx(&b_full[stg], (HB ? M::TB : 0) + rows * 256);
+            for (int g = 0; g < rows; ++g)
+              bulk_load(smem + M::OFF_M + (stg * kGroups + g) * 256, a.mask_terms + ((long long)it.b * a.S + it.s0 + g) * a.npad + j * 64, 256, &b_full[stg]);
+            if (HB) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB, &tmBias, &b_full[stg], j * 64, it.q0, it.h, it.b * a.bias_b_mul);
+            if (HB && M::F32) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB + M::TB / 2, &tmBias, &b_full[stg], j * 64 + 32, it.q0, it.h, it.b * a.bias_b_mul);
+            if (++stg == kBiasStages) { stg = 0; ph ^= 1; }
+          }
+        }
+      }
+    } else {
+      // The terms of short calls are made here, which saves a launch: eight lanes have the 64 keys of a row's step, eight keys each;
+      // their mask bytes are fetched a step ahead, as three aligned words of which the funnel shift takes the eight bytes.  The
+      // softmax warps of the sub-partition miss the instructions: N = 768 took 761 us so and 729 with terms made before, launch
+      // included; N = 256 42.3 and 42.9.
+      if (lane == 0) *a.err = 0;   // (by every CTA: its waits read the word.  One that gives up does so two seconds after all have started)
       dependent_wait();
       int stg = 0;
-      uint32_t ph = 0;
+      uint32_t ph = 0, w[3] = {};
+      const int g = lane >> 3, k_lane = (lane & 7) * 8;
+      const bool owner = lane < 8 * kGroups;
+      const uint8_t* row = nullptr;
+      auto row_of = [&](const Item& it) {
+        const bool live = a.mask != nullptr && owner && g < R && it.s0 + g < a.S;
+        return live ? a.mask + it.b * a.mask_st[0] + (it.s0 + g) * a.mask_st[1] + k_lane : nullptr;
+      };
+      auto fetch = [&](int j) {
+        w[0] = w[1] = w[2] = 0x01010101u;
+        if (row == nullptr) return;
+        const uint8_t* at = row + j * 64;
+        const int off = (int)(reinterpret_cast<uintptr_t>(at) & 3), left = a.N - j * 64 - k_lane + off;   // bytes from the first word on
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(at - off);
+        if (left > off) w[0] = p[0];
+        if (left > 4) w[1] = p[1];
+        if (left > 8 && off > 0) w[2] = p[2];
+      };
+      Item it = item_of(0);
+      if (my_items > 0) { row = row_of(it); fetch(0); }
       for (int n = 0; n < my_items && ok; ++n) {
-        const Item it = item_of(n);
+        const Item after = item_of(n + 1 < my_items ? n + 1 : n);
         for (int j = 0; j < nk; ++j) {
           ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51);
           if (!ok) break;
-          const int rows = min(R, a.S - it.s0);
-          mbar_expect_tx(&b_full[stg], (HB ? M::TB : 0) + rows * 256);
-          for (int g = 0; g < rows; ++g)
-            bulk_load(smem + M::OFF_M + (stg * kGroups + g) * 256, a.mask_terms + ((long long)it.b * a.S + it.s0 + g) * a.npad + j * 64, 256, &b_full[stg]);
-          if (HB) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB, &tmBias, &b_full[stg], j * 64, it.q0, it.h, it.b * a.bias_b_mul);
-          if (HB && M::F32) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB + M::TB / 2, &tmBias, &b_full[stg], j * 64 + 32, it.q0, it.h, it.b * a.bias_b_mul);
+          if (lane == 0) {
+            mbar_expect_tx(&b_full[stg], HB ? M::TB : 0);
+            if (HB) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB, &tmBias, &b_full[stg], j * 64, it.q0, it.h, it.b * a.bias_b_mul);
+            if (HB && M::F32) tma_load_4d(smem + M::OFF_BIAS + stg * M::TB + M::TB / 2, &tmBias, &b_full[stg], j * 64 + 32, it.q0, it.h, it.b * a.bias_b_mul);
+          }
+          const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(row) & 3) * 8;
+          const uint32_t lo = __funnelshift_r(w[0], w[1], sh), hi = __funnelshift_r(w[1], w[2], sh);
+          float term[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) term[e] = ((e < 4 ? lo : hi) & (0xffu << (8 * (e & 3)))) != 0 ? 0.0f : -kMaskSentinel;
+          if (j * 64 + 64 > a.N) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (j * 64 + k_lane + e >= a.N) term[e] = -INFINITY;
+          }
+          if (owner) {
+            float4* to = reinterpret_cast<float4*>(smem + M::OFF_M + (stg * kGroups + g) * 256 + k_lane * 4);
+            to[0] = make_float4(term[0], term[1], term[2], term[3]);
+            to[1] = make_float4(term[4], term[5], term[6], term[7]);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&b_full[stg]);
+          if (j + 1 == nk) row = row_of(after);
+          fetch(j + 1 < nk ? j + 1 : 0);
           if (++stg == kBiasStages) { stg = 0; ph ^= 1; }
         }
+        it = after;
       }
     }
   } else if (warp >= 4 * kGroups) {
@@ -352,7 +427,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float2 v = __ffma2_rn(pair(cur[u * 8 + 2 * i], cur[u * 8 + 2 * i + 1]), sc2, mk[i]);
-              if constexpr (HB && !M::F32) v = __fadd2_rn(v, unpack2<T>(bw[i]));
+              if constexpr (HB && !M::F32) v = add_wide<T>(v, bw[i]);
               x[u * 4 + i] = v;
             }
           }
@@ -519,13 +594,14 @@ bool attn_fwd_rows_fits(const TriAttnDesc* d) {
 }
 
 int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap* tbias,
-                  bool bias_batched, void* o, float* stats, const float* mask_terms, int* err, cudaStream_t st) {
+                  bool bias_batched, const uint8_t* mask, const float* mask_terms, void* o, float* stats, int* err, bool first, cudaStream_t st) {
   RowsArgs a;
   a.B = d->B; a.S = d->n_seq; a.N = d->n_res; a.H = d->H; a.D = d->D;
   a.scale = d->scale;
   a.o = o;
   for (int i = 0; i < 4; ++i) a.o_st[i] = d->o_st[i];
-  a.stats = stats; a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
+  a.stats = stats; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
+  a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
   a.bias_b_mul = bias_batched ? 1 : 0;
   a.err = err;
   const int kind = d->dtype == TRI_F32 ? KIND_TF32 : d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
@@ -541,13 +617,14 @@ int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap
   auto launch = [&](auto elem, auto kern, const CUtensorMap& tb) {
     using M = RowsCfg<decltype(elem)>;
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::SMEM));
-    launch_dependent(us_of_logits(pairs), kern, (unsigned)std::min<long long>(items, sm_count()), M::kThreads, M::SMEM, st, tq, tk, tv, tb, a);
+    launch_dependent(first ? kLaunchPlainly : us_of_logits(pairs), kern, (unsigned)std::min<long long>(items, sm_count()), M::kThreads, M::SMEM, st, tq, tk, tv, tb, a);
     TRI_LAUNCH_OK();
     return 0;
   };
   auto start = [&](auto elem) {
     using T = decltype(elem);
-    return tbias ? launch(elem, attn_fwd_rows_kernel<T, true>, *tbias) : launch(elem, attn_fwd_rows_kernel<T, false>, tq);
+    if (mask_terms != nullptr) return tbias ? launch(elem, attn_fwd_rows_kernel<T, true, true>, *tbias) : launch(elem, attn_fwd_rows_kernel<T, false, true>, tq);
+    return tbias ? launch(elem, attn_fwd_rows_kernel<T, true, false>, *tbias) : launch(elem, attn_fwd_rows_kernel<T, false, false>, tq);
   };
   if (d->dtype == TRI_F32) return start(float());
   return d->dtype == TRI_BF16 ? start(__nv_bfloat16()) : start(__half());

@@ -65,13 +65,13 @@ struct TfFactors {
 // preparation
 // ---------------------------------------------------------------------------------------------
 struct RoundArgs {
-  const float* src[4];
-  int64_t st[4][4];     // strides of (batch, row, residue, head)
-  float* dst[4];        // [B][S][N][H][D]
+  const float* src[3];
+  int64_t st[3][4];     // strides of (batch, row, residue, head)
+  float* dst[3];        // [B][S][N][H][D]
   int S, N, H, D;
   unsigned rows;        // B S N H
 };
-// a row of up to 32 channels by eight lanes; blockIdx.y = tensor
+// forward: a row of up to 32 channels by eight lanes; blockIdx.y = tensor
 __global__ void __launch_bounds__(256) round_copies_kernel(const RoundArgs a) {
   dependent_trigger();
   const unsigned row = blockIdx.x * 32u + (threadIdx.x >> 3);   // (fewer than 2^31)
@@ -85,74 +85,117 @@ __global__ void __launch_bounds__(256) round_copies_kernel(const RoundArgs a) {
   *reinterpret_cast<float4*>(a.dst[t] + (long long)row * a.D + c) = make_float4(round_tf32(v.x), round_tf32(v.y), round_tf32(v.z), round_tf32(v.w));
 }
 
-// dO rounded, and the row constants of the backward: factors, and for flagged rows prep = -m | -log l log2e | -delta
-struct ConstArgs {
-  const float *o, *d_o, *stats;
-  int64_t o_st[4], do_st[4];
-  float* d_o_r;
+// backward, in one launch: q, k, v and dO rounded, the row constants as factors and (for flagged rows) as prep = -m | -log l log2e |
+// -delta, the key-mask terms (0, -1e9, -inf beyond N; in a second plane times log2(e)), the bias transposed.  A block has a (batch, row,
+// head), a warp 32 queries at a time, eight lanes to a row of up to 32 channels; the first blocks transpose a tile of 32 x 32 each.  Bound by
+// the bytes: N = 256, 4 heads of 32, 56 us, 48 by the copy rate, as four kernels 35 + 26 + 3 + 4 and their gaps.
+struct PrepareArgs {
+  const float *q, *k, *v, *o, *d_o, *stats, *bias;
+  float *q_r, *k_r, *v_r, *d_o_r;   // [B][S][N][H][D]
+  float* bias_t;
   float4* aug;          // [2][B][S][H][npad]
   float* prep;          // [3][B][S][H][npad]
-  int* large;
-  int B, S, N, H, D, npad;
-  float scale;
+  float* mask_terms;    // [2][B][S][npad]
+  int* large;           // [B][S][H]
+  int* err;             // cleared
+  const uint8_t* mask;
+  int npad, pitch, tiles, transposes;   // tiles of a side of the bias; blocks that transpose
 };
-__global__ void __launch_bounds__(256) row_constants_kernel(const ConstArgs a) {
-  dependent_trigger();
-  const unsigned row = blockIdx.x * 32u + (threadIdx.x >> 3), rows = (unsigned)a.B * a.S * a.npad * a.H;   // (fewer than 2^31)
-  const int lane8 = threadIdx.x & 7, ch = lane8 * 4;
-  const bool live = row < rows;
-  unsigned w = live ? row : 0;
-  const int h = (int)(w % (unsigned)a.H); w /= (unsigned)a.H;
-  const int n = (int)(w % (unsigned)a.npad); w /= (unsigned)a.npad;
-  const int s = (int)(w % (unsigned)a.S), b = (int)(w / (unsigned)a.S);
-  const long long z = w;    // (batch, row)
-  const bool in = live && n < a.N;
-  float acc = 0.f;
-  if (in && ch < a.D) {
-    const float4 x = *reinterpret_cast<const float4*>(a.o + b * a.o_st[0] + s * a.o_st[1] + n * a.o_st[2] + h * a.o_st[3] + ch);
-    const float4 y = *reinterpret_cast<const float4*>(a.d_o + b * a.do_st[0] + s * a.do_st[1] + n * a.do_st[2] + h * a.do_st[3] + ch);
-    acc = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w)));
-    *reinterpret_cast<float4*>(a.d_o_r + ((z * a.N + n) * a.H + h) * a.D + ch) =
-        make_float4(round_tf32(y.x), round_tf32(y.y), round_tf32(y.z), round_tf32(y.w));
-  }
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (!live || lane8 != 0) return;
-  const long long r = z * a.H + h, plane = (long long)a.B * a.S * a.H * a.npad, at = r * a.npad + n, total = (long long)a.B * a.S * a.H * a.N;
-  const float m = in ? a.stats[r * a.N + n] : 0.f, ll = in ? a.stats[total + r * a.N + n] : 0.f;
-  const float c = in ? -(m + ll) / a.scale : 0.f;
-  const bool fits = TfFactors::fits(m, c, acc);
-  if (!fits) a.large[r] = 1;
-  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-  if (fits) TfFactors::pack(c, -acc, lo, hi);
-  a.aug[at] = lo;
-  a.aug[plane + at] = hi;
-  a.prep[at] = -m;
-  a.prep[plane + at] = -ll * kLog2e;
-  a.prep[2 * plane + at] = -acc;
-}
-
-// out[b][h][k][q] = bias[b][h][q][k], or (keep) the rows themselves, to rows of `pitch`
-__global__ void copy_bias_kernel(const float* __restrict__ in, int64_t st_b, int64_t st_h, int64_t st_q, int n, int H, int pitch, bool transpose,
-                                 float* __restrict__ out) {
+__global__ void __launch_bounds__(256, 3) prepare_bwd_kernel(const TriAttnDesc d, const PrepareArgs a) {
   __shared__ float tile[32][33];
   dependent_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = d.n_res;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
+  if ((int)blockIdx.x < a.transposes) {
+    unsigned z = blockIdx.x;
+    const int k0 = (int)(z % (unsigned)a.tiles) * 32; z /= (unsigned)a.tiles;
+    const int q0 = (int)(z % (unsigned)a.tiles) * 32, bh = (int)(z / (unsigned)a.tiles);
+    const float* src = a.bias + bh / d.H * d.bias_st[0] + bh % d.H * d.bias_st[1];
+    float* dst = a.bias_t + (int64_t)bh * N * a.pitch;
+    for (int i = warp; i < 32; i += 8)
+      if (q0 + i < N && k0 + lane < N) tile[i][lane] = src[(q0 + i) * d.bias_st[2] + k0 + lane];
+    __syncthreads();
+    for (int i = warp; i < 32; i += 8)
+      if (k0 + i < N && q0 + lane < N) dst[(int64_t)(k0 + i) * a.pitch + q0 + lane] = tile[lane][i];
+    return;
+  }
+  const unsigned row = blockIdx.x - a.transposes, bs = row / (unsigned)d.H, h = row - bs * (unsigned)d.H;
+  const unsigned b = bs / (unsigned)d.n_seq, s = bs - b * (unsigned)d.n_seq;
+  const long long planes = (long long)d.B * d.n_seq, plane = planes * d.H * a.npad, total = planes * d.H * N;
+  if (h == 0) {
+    for (int k = threadIdx.x; k < a.npad; k += 256) {
+      const float v = mask_term(a.mask != nullptr && k < N ? a.mask[b * d.mask_st[0] + s * d.mask_st[1] + k] : 1u, k < N);
+      a.mask_terms[(long long)bs * a.npad + k] = v;
+      a.mask_terms[(planes + bs) * a.npad + k] = v * kLog2e;
+    }
+  }
+  const int ch = (lane & 7) * 4;
+  const bool on = ch < d.D;
+  const float *qb = a.q + b * d.q_st[0] + s * d.q_st[1] + h * d.q_st[3] + ch, *kb = a.k + b * d.k_st[0] + s * d.k_st[1] + h * d.k_st[3] + ch,
+              *vb = a.v + b * d.v_st[0] + s * d.v_st[1] + h * d.v_st[3] + ch, *ob = a.o + b * d.o_st[0] + s * d.o_st[1] + h * d.o_st[3] + ch,
+              *gb = a.d_o + b * d.do_st[0] + s * d.do_st[1] + h * d.do_st[3] + ch;
+  int flag = 0;
+  for (int n0 = warp * 32; n0 < a.npad; n0 += 256) {
+    const int i = n0 + lane;   // this lane's query once the sums are there
+    const long long at = (long long)row * a.npad + i;
+    const bool in = i < N;
+    const float m = in ? a.stats[(long long)row * N + i] : 0.f, ll = in ? a.stats[total + (long long)row * N + i] : 0.f;
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float4 x[2][5];
+      float part[2] = {0.f, 0.f};
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const int n = n0 + (e + f) * 4 + (lane >> 3);
+        if (!(on && n < N)) continue;
+        x[f][0] = *reinterpret_cast<const float4*>(ob + n * d.o_st[2]);
+        x[f][1] = *reinterpret_cast<const float4*>(gb + n * d.do_st[2]);
+        x[f][2] = *reinterpret_cast<const float4*>(qb + n * d.q_st[2]);
+        x[f][3] = *reinterpret_cast<const float4*>(kb + n * d.k_st[2]);
+        x[f][4] = *reinterpret_cast<const float4*>(vb + n * d.v_st[2]);
+      }
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const int n = n0 + (e + f) * 4 + (lane >> 3);
+        if (!(on && n < N)) continue;
+        part[f] = fmaf(x[f][0].x, x[f][1].x, fmaf(x[f][0].y, x[f][1].y, fmaf(x[f][0].z, x[f][1].z, x[f][0].w * x[f][1].w)));
+        const long long to = (((long long)bs * N + n) * d.H + h) * d.D + ch;
+        float* const dst[4] = {a.d_o_r, a.q_r, a.k_r, a.v_r};
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          *reinterpret_cast<float4*>(dst[w] + to) = make_float4(round_tf32(x[f][w + 1].x), round_tf32(x[f][w + 1].y), round_tf32(x[f][w + 1].z), round_tf32(x[f][w + 1].w));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) part[f] += __shfl_xor_sync(0xffffffffu, part[f], o);
+        const float v = __shfl_sync(0xffffffffu, part[f], (lane & 3) * 8);
+        if (lane >> 2 == e + f) acc = v;
+      }
+    }
+    const float c = in ? -(m + ll) / d.scale : 0.f;
+    const bool fits = TfFactors::fits(m, c, acc);
+    if (!fits) flag = 1;
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+    if (fits) TfFactors::pack(c, -acc, lo, hi);
+    a.aug[at] = lo;
+    a.aug[plane + at] = hi;
+    a.prep[at] = -m;
+    a.prep[plane + at] = -ll * kLog2e;
+    a.prep[2 * plane + at] = -acc;
+  }
+  flag = __syncthreads_or(flag);
+  if (threadIdx.x == 0) a.large[row] = flag;
+}
+
+// the bias in rows of `pitch`
+__global__ void copy_bias_kernel(const float* __restrict__ in, int64_t st_b, int64_t st_h, int64_t st_q, int n, int H, int pitch, float* __restrict__ out) {
+  dependent_trigger();
   const int bh = blockIdx.z, b = bh / H, h = bh % H;
-  const float* src = in + b * st_b + h * st_h;
-  float* dst = out + (int64_t)bh * n * pitch;
-  const int q0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int q = q0 + i, k = k0 + threadIdx.x;
-    const float v = q < n && k < n ? src[q * st_q + k] : 0.f;
-    if (transpose) tile[i][threadIdx.x] = v;
-    else if (q < n && k < n) dst[(int64_t)q * pitch + k] = v;
-  }
-  if (!transpose) return;
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int k = k0 + i, q = q0 + threadIdx.x;
-    if (k < n && q < n) dst[(int64_t)k * pitch + q] = tile[threadIdx.x][i];
-  }
+  const int q = blockIdx.y * 8 + threadIdx.y, k = blockIdx.x * 32 + threadIdx.x;
+  if (q < n && k < n) out[((int64_t)bh * n + q) * pitch + k] = in[b * st_b + h * st_h + q * st_q + k];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -676,7 +719,7 @@ void carve(Arena& a, const TriAttnDesc* d, int is_bwd, bool bias_copy, TfWs* w) 
   w->err = a.take<int>(64);
   w->q = a.take<float>(t); w->k = a.take<float>(t); w->v = a.take<float>(t);
   w->bias = a.take<float>(bias_copy ? bias_floats(d) : 0);
-  w->mask = a.take<float>((is_bwd ? 2 : 1) * (size_t)d->B * d->n_seq * np);
+  w->mask = a.take<float>((is_bwd ? 2 : wants_mask_terms(d) ? 1 : 0) * (size_t)d->B * d->n_seq * np);
   if (!is_bwd) return;
   w->d_o = a.take<float>(t);
   w->bias_t = a.take<float>(bias_floats(d));
@@ -700,27 +743,9 @@ int bias_tile_map(CUtensorMap* out, const void* p, const TriAttnDesc* d, bool ow
   const uint32_t box[4] = {32, 128, 1, 1};
   return make_tmap(out, p, TRI_F32, 4, dims, own ? mine : packed, box, 128);
 }
-int copy_bias(const TriAttnDesc* d, const void* bias, bool transpose, float* out, cudaStream_t st) {
-  const int t = cdiv(d->n_res, 32);
-  copy_bias_kernel<<<dim3(t, t, batches_of(d) * d->H), dim3(32, 8), 0, st>>>(static_cast<const float*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2],
-                                                                             d->n_res, d->H, pitch_of(d), transpose, out);
-  TRI_LAUNCH_OK();
-  return 0;
-}
-int round_qkv(const TriAttnDesc* d, const void* q, const void* k, const void* v, const TfWs& w, cudaStream_t st) {
-  RoundArgs r;
-  const void* src[3] = {q, k, v};
-  const int64_t* strides[3] = {d->q_st, d->k_st, d->v_st};
-  float* dst[3] = {w.q, w.k, w.v};
-  for (int i = 0; i < 3; ++i) {
-    r.src[i] = static_cast<const float*>(src[i]);
-    r.dst[i] = dst[i];
-    for (int e = 0; e < 4; ++e) r.st[i][e] = strides[i][e];
-  }
-  r.S = d->n_seq; r.N = d->n_res; r.H = d->H; r.D = d->D;
-  r.rows = (unsigned)d->B * d->n_seq * d->n_res * d->H;
-  KernelTimer kt("tc_attn_round", st, 0.0, 24.0 * tensor_floats(d));
-  round_copies_kernel<<<dim3(cdiv(r.rows, 32), 3), 256, 0, st>>>(r);
+int copy_bias(const TriAttnDesc* d, const void* bias, float* out, cudaStream_t st) {
+  copy_bias_kernel<<<dim3(cdiv(d->n_res, 32), cdiv(d->n_res, 8), batches_of(d) * d->H), dim3(32, 8), 0, st>>>(
+      static_cast<const float*>(bias), d->bias_st[0], d->bias_st[1], d->bias_st[2], d->n_res, d->H, pitch_of(d), out);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -764,18 +789,34 @@ int attn_tf32_forward(const TriAttnDesc* d, const void* q, const void* k, const 
   TfWs w;
   carve(ar, d, 0, bias != nullptr && !own_bias(d, bias), &w);
   if (ws == nullptr || !ar.ok()) return fail(TRI_ERR_WORKSPACE, "attention forward workspace too small");
-  TRI_TRY(launch_mask_terms(d, mask, w.mask, w.err, nullptr, st));
-  TRI_TRY(round_qkv(d, q, k, v, w, st));
+  {
+    RoundArgs r;
+    const void* src[3] = {q, k, v};
+    const int64_t* strides[3] = {d->q_st, d->k_st, d->v_st};
+    float* dst[3] = {w.q, w.k, w.v};
+    for (int i = 0; i < 3; ++i) {
+      r.src[i] = static_cast<const float*>(src[i]);
+      r.dst[i] = dst[i];
+      for (int e = 0; e < 4; ++e) r.st[i][e] = strides[i][e];
+    }
+    r.S = d->n_seq; r.N = d->n_res; r.H = d->H; r.D = d->D;
+    r.rows = (unsigned)d->B * d->n_seq * d->n_res * d->H;
+    KernelTimer kt("tc_attn_round", st, 0.0, 24.0 * tensor_floats(d));
+    round_copies_kernel<<<dim3(cdiv(r.rows, 32), 3), 256, 0, st>>>(r);
+    TRI_LAUNCH_OK();
+  }
+  const bool terms = wants_mask_terms(d);
+  if (terms) TRI_TRY(launch_mask_terms(d, mask, w.mask, w.err, st));
   CUtensorMap tq, tk, tv, tb;
   TRI_TRY(copy_map(&tq, w.q, d, 128, false));
   TRI_TRY(copy_map(&tk, w.k, d, 64, false));
   TRI_TRY(copy_map(&tv, w.v, d, 64, true));
   if (bias != nullptr) {
     const bool own = own_bias(d, bias);
-    if (!own) TRI_TRY(copy_bias(d, bias, false, w.bias, st));
+    if (!own) TRI_TRY(copy_bias(d, bias, w.bias, st));
     TRI_TRY(bias_tile_map(&tb, own ? bias : w.bias, d, own));
   }
-  return attn_fwd_rows(d, tq, tk, tv, bias ? &tb : nullptr, d->bias_st[0] != 0, o, stats, w.mask, w.err, st);
+  return attn_fwd_rows(d, tq, tk, tv, bias ? &tb : nullptr, d->bias_st[0] != 0, mask, terms ? w.mask : nullptr, o, stats, w.err, false, st);
 }
 
 int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias, const uint8_t* mask, const void* o,
@@ -784,18 +825,19 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
   TfWs w;
   carve(ar, d, 1, bias != nullptr && !own_bias(d, bias), &w);
   if (ws == nullptr || !ar.ok()) return fail(TRI_ERR_WORKSPACE, "attention backward workspace too small");
-  TRI_TRY(launch_mask_terms(d, mask, w.mask, w.err, w.large, st));
-  TRI_TRY(round_qkv(d, q, k, v, w, st));
   const int npad = npad_of(d), blocks = npad / 128, nq = cdiv(d->n_res, 64);
   const double pairs = (double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res, tensor = 4.0 * tensor_floats(d);
   {
-    ConstArgs c;
-    c.o = static_cast<const float*>(o); c.d_o = static_cast<const float*>(d_o); c.stats = stats;
-    for (int i = 0; i < 4; ++i) { c.o_st[i] = d->o_st[i]; c.do_st[i] = d->do_st[i]; }
-    c.d_o_r = w.d_o; c.aug = w.aug; c.prep = w.prep; c.large = w.large;
-    c.B = d->B; c.S = d->n_seq; c.N = d->n_res; c.H = d->H; c.D = d->D; c.npad = npad; c.scale = d->scale;
-    KernelTimer kt("tc_attn_delta", st, 0.0, 3.0 * tensor);
-    row_constants_kernel<<<cdiv((long long)d->B * d->n_seq * npad * d->H, 32), 256, 0, st>>>(c);
+    PrepareArgs p;
+    p.q = static_cast<const float*>(q); p.k = static_cast<const float*>(k); p.v = static_cast<const float*>(v);
+    p.o = static_cast<const float*>(o); p.d_o = static_cast<const float*>(d_o); p.stats = stats; p.bias = static_cast<const float*>(bias);
+    p.q_r = w.q; p.k_r = w.k; p.v_r = w.v; p.d_o_r = w.d_o; p.bias_t = w.bias_t; p.aug = w.aug; p.prep = w.prep; p.mask_terms = w.mask;
+    p.large = w.large; p.err = w.err; p.mask = mask; p.npad = npad; p.pitch = pitch_of(d);
+    p.tiles = cdiv(d->n_res, 32);
+    p.transposes = bias != nullptr ? p.tiles * p.tiles * batches_of(d) * d->H : 0;
+    const long long planes = (long long)d->B * d->n_seq;
+    KernelTimer kt("tc_attn_prepare", st, 0.0, 9.0 * tensor);
+    prepare_bwd_kernel<<<(unsigned)(p.transposes + planes * d->H), 256, 0, st>>>(*d, p);
     TRI_LAUNCH_OK();
   }
   TfBwdArgs a;
@@ -810,7 +852,6 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
   CUtensorMap a0, a1, b0, b1, l0, l1, tb;
   // ---- dK, dV: stationary K, V; streamed Q, dO -------------------------------------------------
   if (bias != nullptr) {
-    TRI_TRY(copy_bias(d, bias, true, w.bias_t, st));
     TRI_TRY(bias_tile_map(&tb, w.bias_t, d, false));
   }
   TRI_TRY(copy_map(&a0, w.k, d, 128, false)); TRI_TRY(copy_map(&a1, w.v, d, 128, false));
@@ -830,7 +871,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
   // ---- dQ: stationary Q, dO; streamed K, V ------------------------------------------------------
   if (bias != nullptr) {
     const bool own = own_bias(d, bias);
-    if (!own) TRI_TRY(copy_bias(d, bias, false, w.bias, st));
+    if (!own) TRI_TRY(copy_bias(d, bias, w.bias, st));
     TRI_TRY(bias_tile_map(&tb, own ? bias : w.bias, d, own));
   }
   TRI_TRY(copy_map(&a0, w.q, d, 128, false)); TRI_TRY(copy_map(&a1, w.d_o, d, 128, false));

@@ -15,9 +15,6 @@ int attn_tf32_forward(const TriAttnDesc* d, const void* q, const void* k, const 
 int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const void* v, const void* bias, const uint8_t* mask, const void* o,
                        const float* stats, const void* d_o, void* dq, void* dk, void* dv, float* dbias, void* ws, size_t ws_size, cudaStream_t st);
 
-// the additive key-mask terms of a call (see mask_terms_kernel); `flags` [B][S][H]: cleared, and the terms times log2(e) follow
-int launch_mask_terms(const TriAttnDesc* d, const uint8_t* mask, float* out, int* err, int* flags, cudaStream_t st);
-
 // The row chunks of a dbias pass (64 queries x 128 keys per CTA) on `slots` CTAs at a time, the bytes of their partial sums
 // (none for one chunk), and their sum in fixed order.
 int dbias_row_chunks(const TriAttnDesc* d, int slots);

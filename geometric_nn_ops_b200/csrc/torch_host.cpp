@@ -196,12 +196,13 @@ struct AttnFn : torch::autograd::Function<AttnFn> {
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["precision"] = precision;
     ctx->mark_non_differentiable({c.stats});
+    ctx->set_materialize_grads(false);   // (no zeros for the statistics)
     return {c.o, c.stats};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     const Tensor &q = s[0], &k = s[1], &v = s[2], &bias = s[3], &mask = s[4], &o = s[5], &stats = s[6];
-    const Tensor d_o = inner_contiguous(grads[0]);
+    const Tensor d_o = grads[0].defined() ? inner_contiguous(grads[0]) : at::zeros_like(o);
     const int64_t B = q.size(0), N = q.size(2), H = q.size(3);
     Tensor dq = like(q), dk = like(k), dv = like(v), dbias;
     if (bias.defined() && ctx->needs_input_grad(3)) dbias = at::empty({B, H, N, N}, q.options().dtype(at::kFloat));
