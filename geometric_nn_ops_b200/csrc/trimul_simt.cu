@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(256) contract_kernel(ContractP p) {
       }
     }
   };
+  dependent_trigger();
   auto issue = [&](int r0, int buf) {
 #pragma unroll
     for (int e = 0; e < R * PT / 32; ++e, X += x_step) copy(xd + buf * L::kStage * 4 + e * 32 * 128, X, r0 + xr + e * (32 / PT) < p.N, p.X);
@@ -570,7 +571,9 @@ static GemmP linear_t_p(const float* D, int ldd, const float* W, float* out, lon
 // CTA have half of each contraction and exchange half of their sums.  Two CTAs share an SM; one's loads and LayerNorm run
 // under the other's products.  The FMAs are packed in pairs: 1.2 clocks per 32 of them against 1.4 for single ones.
 //   One stage per kernel -- 9 conversions, 2 LayerNorms, 4 GEMMs of 16 us and two gates -- took 116 us of the 183 us of a
-// 64 x 64 x 128 fp32 call; these take 22 and 19 us of 52 (and 0.60 and 0.38 ms at 384 x 384, against 2.1 ms).
+// 64 x 64 x 128 fp32 call; these take 21 and 13 us of 45 (and 0.59 and 0.37 ms at 384 x 384, against 2.1 ms).  The output stage took 19
+// of 53 in tiles of 64 pixels, which make 128 CTAs there, launched behind the contraction.  Of the 21 the products are 11 (75 % of
+// the FMA rate, 22 k cycles on an SM with two CTAs); weights, LayerNorm and the gate take 1.5 to 2 each.
 struct FusedP {
   const void *x, *mask, *norm_in_w, *norm_in_b, *p_w, *p_b, *g_w, *g_b, *norm_out_w, *norm_out_b;
   const float* t;                                   // output stage: the contraction
@@ -601,101 +604,128 @@ __device__ __forceinline__ float4 round_four(float4 v) {
   return v;
 }
 
-// Four rows' values at four consecutive k, transposed into a tile [K][64]: the 16-byte chunk of four rows is XORed with k / 4,
-// which keeps the lanes of a warp (consecutive k / 4) apart.
+// Four rows' values at four consecutive k, transposed into a tile [K][R] of 64 or 32 rows: the 16-byte chunk of four rows is XORed with
+// k / 4, which keeps the lanes of a warp (consecutive k / 4) apart.
+template <int R>
 __device__ __forceinline__ void put_transposed(float* tile, int k, int row0, const float4& v0, const float4& v1, const float4& v2, const float4& v3) {
-  float* to = tile + k * 64 + (((row0 >> 2) ^ (k >> 2 & 7)) << 2);
+  float* to = tile + k * R + (((row0 >> 2) ^ (k >> 2 & 7)) << 2);
   *reinterpret_cast<float4*>(to) = make_float4(v0.x, v1.x, v2.x, v3.x);
-  *reinterpret_cast<float4*>(to + 64) = make_float4(v0.y, v1.y, v2.y, v3.y);
-  *reinterpret_cast<float4*>(to + 128) = make_float4(v0.z, v1.z, v2.z, v3.z);
-  *reinterpret_cast<float4*>(to + 192) = make_float4(v0.w, v1.w, v2.w, v3.w);
+  *reinterpret_cast<float4*>(to + R) = make_float4(v0.y, v1.y, v2.y, v3.y);
+  *reinterpret_cast<float4*>(to + 2 * R) = make_float4(v0.z, v1.z, v2.z, v3.z);
+  *reinterpret_cast<float4*>(to + 3 * R) = make_float4(v0.w, v1.w, v2.w, v3.w);
 }
 
-// 64 rows of W [n_out, K] from row n0 into shared memory as [K][64], zero beyond n_out
+// 64 rows of W [n_out, K] and of G [n_out, C] from row n0 into shared memory as [K][64] and [C][64], zero beyond n_out; a warp has eight
+// rows of each, four of both at a time
 template <typename T, bool TF32>
-__device__ __forceinline__ void stage_weights(float* dst, const T* W, int n0, int n_out, int K) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int r0 = warp * 8 + i * 4;
-    for (int k = lane * 4; k < K; k += 128) {
-      float4 v[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        v[r] = round_four<TF32>(n0 + r0 + r < n_out ? load_four(W + (long long)(n0 + r0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f));
-      put_transposed(dst, k, r0, v[0], v[1], v[2], v[3]);
-    }
-  }
-}
-
-// 64 rows of X [M, K] from row m0, LayerNormed, into shared memory as [K][64]; a warp has eight rows, four at a time
-template <typename TX, typename T, bool TF32>
-__device__ __forceinline__ void stage_normalised(float* dst, const TX* X, const T* gamma, const T* beta, float eps, long long m0, long long M,
-                                                 int K, float* z, float* mean, float* rstd) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ __forceinline__ void stage_weights(float* dst_w, float* dst_g, const T* W, const T* G, int n0, int n_out, int K, int C) {
+  const int lane = threadIdx.x & 31;
+  for (int k = lane * 4; k < max(K, C); k += 128) {
 #pragma unroll 1
-  for (int i = 0; i < 2; ++i) {
-    const int r0 = warp * 8 + i * 4;
-    float4 v[4][2];
-    float s[4], mu[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      s[r] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int k = (lane + 32 * j) * 4;
-        v[r][j] = k < K && m0 + r0 + r < M ? load_four(X + (m0 + r0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        s[r] += (v[r][j].x + v[r][j].y) + (v[r][j].z + v[r][j].w);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      mu[r] = warp_sum(s[r]) / K;
-      s[r] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        if ((lane + 32 * j) * 4 < K) {
-          float4& x = v[r][j];
-          x = make_float4(x.x - mu[r], x.y - mu[r], x.z - mu[r], x.w - mu[r]);
-          s[r] += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      s[r] = 1.0f / sqrtf(warp_sum(s[r]) / K + eps);
-      if (mean != nullptr && m0 + r0 + r < M && lane == 0) { mean[m0 + r0 + r] = mu[r]; rstd[m0 + r0 + r] = s[r]; }
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int k = (lane + 32 * j) * 4;
-      if (k >= K) continue;
-      const float4 g = gamma ? load_four(gamma + k) : make_float4(1.f, 1.f, 1.f, 1.f), o = beta ? load_four(beta + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r0 = (threadIdx.x >> 5) * 8, end = r0 + 8; r0 < end; r0 += 4) {
+      float4 v[2][4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        float4& x = v[r][j];
-        x = make_float4(x.x * s[r] * g.x + o.x, x.y * s[r] * g.y + o.y, x.z * s[r] * g.z + o.z, x.w * s[r] * g.w + o.w);
-        if (z != nullptr && m0 + r0 + r < M) *reinterpret_cast<float4*>(z + (m0 + r0 + r) * K + k) = x;
-        x = round_four<TF32>(x);
+        const bool in = n0 + r0 + r < n_out;
+        v[0][r] = in && k < K ? load_four(W + (long long)(n0 + r0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[1][r] = in && k < C ? load_four(G + (long long)(n0 + r0 + r) * C + k) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      put_transposed(dst, k, r0, v[0][j], v[1][j], v[2][j], v[3][j]);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) { v[0][r] = round_four<TF32>(v[0][r]); v[1][r] = round_four<TF32>(v[1][r]); }
+      if (k < K) put_transposed<64>(dst_w, k, r0, v[0][0], v[0][1], v[0][2], v[0][3]);
+      if (k < C) put_transposed<64>(dst_g, k, r0, v[1][0], v[1][1], v[1][2], v[1][3]);
     }
   }
 }
 
-// acc[w][i][j] += A^T B[w] over k_begin .. k_end, for pixels 2 i, 2 i + 1 of the eight in chunks ch, ch + 1 of A's rows and
-// channel j of chunk cn of each of W weight blocks
-template <int W>
-__device__ __forceinline__ void dot_tile(float2 (&acc)[W][4][4], const float* A, const float* B, int K, int k_begin, int k_end, int ch, int cn) {
+// N rows of up to 128 J channels, a lane with four channels of every 128; and their LayerNorm's weight and bias
+template <int N, int J> struct Rows { float4 v[N][J]; };
+template <int J> struct Affine {
+  float4 g[J], b[J];
+  template <typename T> __device__ __forceinline__ void load(const T* gamma, const T* beta, int K) {
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = ((threadIdx.x & 31) + 32 * j) * 4;
+      g[j] = gamma && k < K ? load_four(gamma + k) : make_float4(1.f, 1.f, 1.f, 1.f);
+      b[j] = beta && k < K ? load_four(beta + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+};
+// rows of X [M, K] from row m
+template <int N, int J, typename TX>
+__device__ __forceinline__ void load_rows(Rows<N, J>& x, const TX* X, long long m, long long M, int K) {
+#pragma unroll
+  for (int r = 0; r < N; ++r)
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = ((threadIdx.x & 31) + 32 * j) * 4;
+      x.v[r][j] = k < K && m + r < M ? load_four(X + (m + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+// ... LayerNormed into rows r0 .. of a tile [K][R]; z, mean, rstd [M ..]: null, or written
+template <int R, bool TF32, int N, int J>
+__device__ __forceinline__ void put_normalised(Rows<N, J>& x, const Affine<J>& w, float* dst, int r0, float eps, long long m, long long M, int K, float* z,
+                                               float* mean, float* rstd) {
+  const int lane = threadIdx.x & 31;
+  float s[N], mu[N];
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    s[r] = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) s[r] += (x.v[r][j].x + x.v[r][j].y) + (x.v[r][j].z + x.v[r][j].w);
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    mu[r] = warp_sum(s[r]) / K;
+    s[r] = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if ((lane + 32 * j) * 4 < K) {
+        float4& v = x.v[r][j];
+        v = make_float4(v.x - mu[r], v.y - mu[r], v.z - mu[r], v.w - mu[r]);
+        s[r] += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    s[r] = 1.0f / sqrtf(warp_sum(s[r]) / K + eps);
+    if (mean != nullptr && m + r < M && lane == 0) { mean[m + r] = mu[r]; rstd[m + r] = s[r]; }
+  }
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const int k = (lane + 32 * j) * 4;
+    if (k >= K) continue;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      float4& v = x.v[r][j];
+      v = make_float4(v.x * s[r] * w.g[j].x + w.b[j].x, v.y * s[r] * w.g[j].y + w.b[j].y, v.z * s[r] * w.g[j].z + w.b[j].z, v.w * s[r] * w.g[j].w + w.b[j].w);
+      if (z != nullptr && m + r < M) *reinterpret_cast<float4*>(z + (m + r) * K + k) = v;
+      v = round_four<TF32>(v);
+    }
+#pragma unroll
+    for (int r = 0; r < N; r += 4) put_transposed<R>(dst, k, r0 + r, x.v[r][j], x.v[r + 1][j], x.v[r + 2][j], x.v[r + 3][j]);
+  }
+}
+
+// acc[w][i][j] += A^T B[w] over k_begin .. k_end, for pixels 2 i, 2 i + 1 of those in A's chunks of four from ch on (R = 64: two, 32: one)
+// and channel j of chunk cn of each of W weight blocks
+template <int W, int R>
+__device__ __forceinline__ void dot_tile(float2 (&acc)[W][R / 16][4], const float* A, const float* B, int K, int k_begin, int k_end, int ch, int cn) {
 #pragma unroll 1
   for (int k4 = k_begin; k4 < k_end; k4 += 4) {
     const int sw = k4 >> 2 & 7;
-    const float* a0 = A + k4 * 64 + ((ch ^ sw) << 2);
-    const float* a1 = A + k4 * 64 + (((ch + 1) ^ sw) << 2);
+    const float* a0 = A + k4 * R + ((ch ^ sw) << 2);
+    const float* a1 = A + k4 * R + (((ch + 1) ^ sw) << 2);
     const float* b0 = B + k4 * 64 + ((cn ^ sw) << 2);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float4 x = *reinterpret_cast<const float4*>(a0 + e * 64), y = *reinterpret_cast<const float4*>(a1 + e * 64);
-      const float2 a[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), make_float2(y.z, y.w)};
+      float2 a[R / 16];
+      const float4 x = *reinterpret_cast<const float4*>(a0 + e * R);
+      a[0] = make_float2(x.x, x.y); a[1] = make_float2(x.z, x.w);
+      if constexpr (R == 64) {
+        const float4 y = *reinterpret_cast<const float4*>(a1 + e * R);
+        a[2] = make_float2(y.x, y.y); a[3] = make_float2(y.z, y.w);
+      }
 #pragma unroll
       for (int w = 0; w < W; ++w) {
         const float4 b = *reinterpret_cast<const float4*>(b0 + (w * K + e) * 64);
@@ -703,7 +733,7 @@ __device__ __forceinline__ void dot_tile(float2 (&acc)[W][4][4], const float* A,
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) acc[w][i][j] = __ffma2_rn(a[i], bb[j], acc[w][i][j]);
+          for (int i = 0; i < R / 16; ++i) acc[w][i][j] = __ffma2_rn(a[i], bb[j], acc[w][i][j]);
       }
     }
   }
@@ -723,57 +753,93 @@ __device__ __forceinline__ void store_four(T* p, float4 v) {
 // where the second half of a contraction over K starts
 __device__ __forceinline__ int split(int K) { return (K / 4 + 1) / 2 * 4; }
 
-// OUT: the output stage (first product on the LayerNormed contraction), else the input stage (both on z)
-template <typename T, bool OUT, bool TF32>
+// OUT: the output stage (first product on the LayerNormed contraction), else the input stage (both on z).  R: pixels of a tile; rows of
+// up to 128 J channels
+template <typename T, bool OUT, bool TF32, int R, int J>
 __global__ void __launch_bounds__(256, 2) fused_kernel(const FusedP p) {
   extern __shared__ __align__(16) float sm[];
   const int C = p.C, K0 = OUT ? p.Ch : p.C, n0 = blockIdx.x * 64;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = warp >> 2, t = threadIdx.x & 127;
-  const int ty = (warp >> 1 & 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);   // pixels 8 ty .., channels 4 tx ..
+  const int ty = (warp >> 1 & 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);   // pixels R / 8 ty .., channels 4 tx ..
+  constexpr int kChunks = R / 32, kPairs = R / 16;   // of the pixels of a thread
+  constexpr int kRows = J == 1 ? R / 8 : 4;          // a warp's rows in registers at a time
   const bool first = blockIdx.x == 0;
-  const T *gin = static_cast<const T*>(p.norm_in_w), *bin = static_cast<const T*>(p.norm_in_b);
-  float *sW = sm, *sG = sW + 64 * K0, *sA = sG + 64 * C;
-  stage_weights<T, TF32>(sW, static_cast<const T*>(p.p_w), n0, p.n_out, K0);
-  stage_weights<T, TF32>(sG, static_cast<const T*>(p.g_w), n0, p.n_out, C);
-  const int n = n0 + 4 * tx;
+  const T* px = static_cast<const T*>(p.x);
+  float *sW = sm, *sG = sW + 64 * K0, *sA = sG + 64 * C, *sZ = OUT && R == 32 ? sA + R * K0 : sA;   // (32 pixels: both rows' tiles at once)
+  const int n = n0 + 4 * tx, r0 = warp * (R / 8);
   float4 pb = make_float4(0.f, 0.f, 0.f, 0.f), gb = pb;
+  stage_weights<T, TF32>(sW, sG, static_cast<const T*>(p.p_w), static_cast<const T*>(p.g_w), n0, p.n_out, K0, C);
   if (n < p.n_out && p.p_b) pb = load_four(static_cast<const T*>(p.p_b) + n);
   if (n < p.n_out && p.g_b) gb = load_four(static_cast<const T*>(p.g_b) + n);
-  for (long long m0 = blockIdx.y * 64LL; m0 < p.M; m0 += gridDim.y * 64LL) {
-    float2 acc[2][4][4] = {};
-    __syncthreads();
-    if constexpr (OUT) {
-      stage_normalised<float, T, TF32>(sA, p.t, static_cast<const T*>(p.norm_out_w), static_cast<const T*>(p.norm_out_b), p.eps, m0, p.M, K0,
-                                       nullptr, first ? p.mean : nullptr, p.rstd);
-      __syncthreads();
-      dot_tile<1>(reinterpret_cast<float2(&)[1][4][4]>(acc[0]), sA, sW, K0, half ? split(K0) : 0, half ? K0 : split(K0), 2 * ty, tx);
-      __syncthreads();
-      stage_normalised<T, T, TF32>(sA, static_cast<const T*>(p.x), gin, bin, p.eps, m0, p.M, C, nullptr, nullptr, nullptr);
-      __syncthreads();
-      dot_tile<1>(reinterpret_cast<float2(&)[1][4][4]>(acc[1]), sA, sG, C, half ? split(C) : 0, half ? C : split(C), 2 * ty, tx);
-    } else {
-      stage_normalised<T, T, TF32>(sA, static_cast<const T*>(p.x), gin, bin, p.eps, m0, p.M, C, first ? p.z : nullptr, first ? p.mean : nullptr,
-                                   p.rstd);
-      __syncthreads();
-      dot_tile<2>(acc, sA, sW, C, half ? split(C) : 0, half ? C : split(C), 2 * ty, tx);
+  // LayerNormed rows of the tile from m0 on
+  auto put_x = [&](long long m0, float* z, float* mean, float* rstd) {
+#pragma unroll 1
+    for (int i = 0; i < R / 8; i += kRows) {
+      Rows<kRows, J> x;
+      Affine<J> w;
+      load_rows(x, px, m0 + r0 + i, p.M, C);
+      w.load(static_cast<const T*>(p.norm_in_w), static_cast<const T*>(p.norm_in_b), C);
+      put_normalised<R, TF32>(x, w, sZ, r0 + i, p.eps, m0 + r0 + i, p.M, C, z, mean, rstd);
     }
-    // each half keeps four of the eight pixels: it hands the other four's sums over through the row tile
+  };
+  auto put_t = [&](long long m0) {
+#pragma unroll 1
+    for (int i = 0; i < R / 8; i += kRows) {
+      Rows<kRows, J> x;
+      Affine<J> w;
+      load_rows(x, p.t, m0 + r0 + i, p.M, K0);
+      w.load(static_cast<const T*>(p.norm_out_w), static_cast<const T*>(p.norm_out_b), K0);
+      put_normalised<R, TF32>(x, w, sA, r0 + i, p.eps, m0 + r0 + i, p.M, K0, nullptr, first ? p.mean : nullptr, p.rstd);
+    }
+  };
+  // t is the kernel's before, all else is the caller's
+  if (OUT && R == 32) put_x(blockIdx.y * (long long)R, nullptr, nullptr, nullptr);
+  if (OUT && R == 32) dependent_wait();
+  for (long long m0 = blockIdx.y * (long long)R; m0 < p.M; m0 += gridDim.y * (long long)R) {
+    float2 acc[2][kPairs][4];
+    auto clear = [&](int w) {   // (late: the rows on their way need the registers)
+#pragma unroll
+      for (int x = 0; x < 4 * kPairs; ++x) acc[w][x >> 2][x & 3] = make_float2(0.f, 0.f);
+    };
+    const bool again = m0 != blockIdx.y * (long long)R;
+    if (again) __syncthreads();
+    if constexpr (OUT) {
+      if (R == 32 && again) put_x(m0, nullptr, nullptr, nullptr);
+      put_t(m0);
+      __syncthreads();
+      clear(0);
+      dot_tile<1, R>(reinterpret_cast<float2(&)[1][kPairs][4]>(acc[0]), sA, sW, K0, half ? split(K0) : 0, half ? K0 : split(K0), kChunks * ty, tx);
+      if (R == 64) {
+        __syncthreads();
+        put_x(m0, nullptr, nullptr, nullptr);
+        __syncthreads();
+      }
+      clear(1);
+      dot_tile<1, R>(reinterpret_cast<float2(&)[1][kPairs][4]>(acc[1]), sZ, sG, C, half ? split(C) : 0, half ? C : split(C), kChunks * ty, tx);
+    } else {
+      put_x(m0, first ? p.z : nullptr, first ? p.mean : nullptr, p.rstd);
+      __syncthreads();
+      clear(0);
+      clear(1);
+      dot_tile<2, R>(acc, sA, sW, C, half ? split(C) : 0, half ? C : split(C), kChunks * ty, tx);
+    }
+    // each half keeps half of the pixels: it hands the others' sums over through the row tile
     __syncthreads();
     float2* swap = reinterpret_cast<float2*>(sA);
+    constexpr int kHand = 4 * kPairs;   // pairs of both products that change hands
+    auto sum = [&](int x, bool upper) -> float2& { return acc[x / (kHand / 2)][(upper ? kPairs / 2 : 0) + x / 4 % (kPairs / 2)][x % 4]; };
 #pragma unroll
-    for (int x = 0; x < 16; ++x) swap[(half * 16 + x) * 128 + t] = half ? acc[x >> 3][x >> 2 & 1][x & 3] : acc[x >> 3][2 + (x >> 2 & 1)][x & 3];
+    for (int x = 0; x < kHand; ++x) swap[(half * kHand + x) * 128 + t] = half ? sum(x, false) : sum(x, true);
     __syncthreads();
 #pragma unroll
-    for (int x = 0; x < 16; ++x) {
-      const float2 o = swap[((half ^ 1) * 16 + x) * 128 + t];
-      float2& mine = acc[x >> 3][x >> 2 & 1][x & 3];
-      const float2 own = half ? acc[x >> 3][2 + (x >> 2 & 1)][x & 3] : mine;
-      mine = half ? __fadd2_rn(o, own) : __fadd2_rn(own, o);
+    for (int x = 0; x < kHand; ++x) {
+      const float2 o = swap[((half ^ 1) * kHand + x) * 128 + t], own = half ? sum(x, true) : sum(x, false);
+      sum(x, false) = half ? __fadd2_rn(o, own) : __fadd2_rn(own, o);
     }
     if (n >= p.n_out) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long long m = m0 + 8 * ty + 4 * half + i, at = m * p.n_out + n;
+    for (int i = 0; i < R / 16; ++i) {
+      const long long m = m0 + R / 8 * ty + R / 16 * half + i, at = m * p.n_out + n;
       if (m >= p.M) continue;
       float a[4], b[4];
 #pragma unroll
@@ -800,19 +866,31 @@ static bool fused_fits(const TriMulDesc* d, const void* x, const TriMulWeights* 
   return d->C % 4 == 0 && d->Ch % 4 == 0 && d->C <= kFusedMax && d->Ch <= kFusedMax;
 }
 
-template <typename T, bool OUT>
-static int fused_start(const FusedP& p, bool tf32, cudaStream_t st) {
-  const auto kern = tf32 ? fused_kernel<T, OUT, kCanTf32<T>> : fused_kernel<T, OUT, false>;
-  const int rows = std::max(128, OUT ? std::max(p.C, p.Ch) : p.C);   // the row tile, at least as large as the halves' exchange
-  const size_t smem = (size_t)64 * sizeof(float) * ((OUT ? p.C + p.Ch : 2 * p.C) + rows);
+template <typename T, bool OUT, int R, int J>
+static int fused_launch(const FusedP& p, bool tf32, cudaStream_t st) {
+  const auto kern = tf32 ? fused_kernel<T, OUT, kCanTf32<T>, R, J> : fused_kernel<T, OUT, false, R, J>;
+  // the row tile (of 32 pixels: tiles), at least as large as the halves' exchange
+  const int rows = OUT && R == 32 ? std::max(128, p.C + p.Ch) : std::max(128, OUT ? std::max(p.C, p.Ch) : p.C);
+  const size_t smem = sizeof(float) * (64 * (size_t)(OUT ? p.C + p.Ch : 2 * p.C) + (size_t)R * rows);
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const double M = (double)p.M;
-  KernelTimer kt(OUT ? "simt_fused_out" : "simt_fused_in", st, 2.0 * M * p.n_out * (p.C + (OUT ? p.Ch : p.C)),
-                 OUT ? M * (2.0 * p.C * sizeof(T) + 4.0 * p.Ch) : M * (p.C * sizeof(T) + 8.0 * p.Ch));
+  const double M = (double)p.M, fma = M * p.n_out * (p.C + (OUT ? p.Ch : p.C));
+  KernelTimer kt(OUT ? "simt_fused_out" : "simt_fused_in", st, 2.0 * fma, OUT ? M * (2.0 * p.C * sizeof(T) + 4.0 * p.Ch) : M * (p.C * sizeof(T) + 8.0 * p.Ch));
   const int blocks = cdiv(p.n_out, 64), room = std::max(1, (smem <= 113 * 1024 ? 2 : 1) * sm_count() / blocks);
-  kern<<<dim3(blocks, (unsigned)std::min<long long>((p.M + 63) / 64, room)), 256, smem, st>>>(p);
+  // The output stage of a small call starts early: weights and x are staged under the contraction, which leaves the room (64 x 64 pixels:
+  // 13 us behind it instead of 21).  With larger ones, early CTAs take their places unevenly (203 x 203: 404 -> 407 us).
+  launch_dependent(OUT && R == 32 ? 0.0 : kLaunchPlainly, kern, dim3(blocks, (unsigned)std::min<long long>((p.M + R - 1) / R, room)), 256, smem, st, p);
   TRI_LAUNCH_OK();
   return 0;
+}
+template <typename T, bool OUT>
+static int fused_start(const FusedP& p, bool tf32, cudaStream_t st) {
+  const bool narrow = p.C <= 128 && p.Ch <= 128;
+  // output stage: tiles of 32 pixels where those of 64 would not make two CTAs for an SM
+  if (OUT && (p.M + 63) / 64 * cdiv(p.n_out, 64) <= sm_count()) {
+    constexpr int R = OUT ? 32 : 64;
+    return narrow ? fused_launch<T, OUT, R, 1>(p, tf32, st) : fused_launch<T, OUT, R, 2>(p, tf32, st);
+  }
+  return narrow ? fused_launch<T, OUT, 64, 1>(p, tf32, st) : fused_launch<T, OUT, 64, 2>(p, tf32, st);
 }
 
 template <typename T>

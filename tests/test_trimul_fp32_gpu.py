@@ -14,6 +14,8 @@ CASES = [  # B, N, C, Ch
     (3, 21, 68, 132),     # channels that are no multiple of a 64-wide block
     (2, 11, 30, 20),      # channels that are no multiple of four: one stage per kernel
     (1, 10, 264, 40),     # rows too wide for the fused kernels
+    (1, 68, 128, 128), (1, 69, 128, 128),   # output stage in tiles of 32 pixels, of 64
+    (1, 33, 132, 256), (1, 60, 256, 128),   # rows of more than 128 channels, tiles of 32 and of 64
 ]
 
 
