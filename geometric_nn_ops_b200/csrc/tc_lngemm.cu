@@ -1,23 +1,25 @@
 // LayerNorm fused into the two projection kernels of the triangle multiplicative update (see tc_lngemm.cuh).
 //
-// ln_gate_in.  One persistent CTA per SM, 704 threads:
+// ln_gate_in.  One persistent CTA per SM, 832 threads:
 //   warp 0       TMA: the concatenated weights once (128 KB, resident), then one 128-pixel x tile per step into one of
-//                two 32 KB buffers
+//                two 32 KB buffers; stores each tile as z once it is normalised
 //   warp 1       tcgen05.mma: per tile and half (a, b) the P and G products, M = the half's 128 channels, N = 128
-//                pixels, into one of two 256-column accumulators (the halves alternate, so the epilogue of one half
-//                runs under the products of the other)
-//   warps 2-5    LayerNorm: thread = pixel row; normalises the row in place (two passes over it in shared memory:
-//                statistics, result), writes the statistics, releases the tile to the MMA warp and
-//                stores it as z with one TMA store per 64-channel half.  (With two warps owning two rows each the
-//                kernel ran at the pace of this role: 9.4 us per tile against 5.4 for the two gate epilogues.)
-//   warps 6-21   gate epilogue, thread = channel holding consecutive pixels (the order of the channel-major a / b)
+//                pixels, into the half's 256-column accumulator
+//   warps 2-9    LayerNorm: thread = half of a pixel row; normalises it in place (two passes over it in shared memory:
+//                statistics, result), writes the statistics and releases the tile to the MMA warp and to the store.
+//   warps 10-25  gate epilogue, thread = channel holding consecutive pixels (the order of the channel-major a / b); a set of
+//                eight warps for each half, so that one set's waits and stores run beside the other's arithmetic
 //
 // Against the two-kernel form (LayerNorm kernel, then the gate GEMM reading z once per half) x is read once, z is
 // written from shared memory and never read back here, and the weights stay in shared memory.  a and b leave through
 // shared memory too, by TMA in whole 128-byte lines; the epilogue threads' own stores carried 32 bytes per request, a
 // channel's rows lying a plane apart.  Per launch at 768 x 768 pixels: 0.24 ms for the pair of kernels, 0.197 for this one
-// at first, 0.164 with a reciprocal instead of a quotient in the sigmoid, pairwise conversions and the mask read once per
-// tile, and 0.148 with the staged stores; floor by bytes 0.092.
+// at first, 0.165 with a reciprocal instead of a quotient in the sigmoid, pairwise conversions, the mask read once per
+// tile and staged stores, and 0.145 with eight LayerNorm warps (four took 5.3 k cycles a tile, one of them 2 k more for the store of
+// z, where a tile takes 8.5 k in all) and the epilogue in two sets (as one, 4.8 k cycles of arithmetic, 1.4 of staging and 1.3 of
+// waiting followed one another); floor by bytes 0.092.  What bounds it is the path of shared memory and TMEM: MMA operands, accumulators,
+// the LayerNorm's passes and the tiles' ways in and out take about 6.6 k of the 7.4 k cycles of a tile at 128 bytes each.  (One reciprocal for
+// two sigmoids changes nothing; rows kept in registers between the passes spill at 72 a thread.)
 // Every mbarrier wait is bounded; a timeout lands in *err and all roles drain.
 #include "tc_lngemm.cuh"
 
@@ -28,7 +30,7 @@ namespace tc {
 
 namespace {
 
-constexpr int kThreads = 704;
+constexpr int kThreads = 832, kLnWarps = 8, kEpi0 = 2 + kLnWarps;   // warps: TMA, MMA, LayerNorm, 16 for the gate epilogue
 constexpr int kSub = 16384;                 // one [128 rows x 128 bytes] swizzled sub-tile
 constexpr uint32_t kWBytes = 8 * kSub;      // (Pa, Ga, Pb, Gb) x (k 0..63, k 64..127)
 constexpr uint32_t kXBytes = 2 * kSub;      // one pixel tile: two 64-channel halves
@@ -77,16 +79,16 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint64_t* wfull = reinterpret_cast<uint64_t*>(s_mask + kMaskRing * 128);
   uint64_t* xfull = wfull + 1;            // [kXBufs] tile landed (TMA bytes)
   uint64_t* xnorm = xfull + kXBufs;       // [kXBufs] tile normalised (one arrival per LayerNorm warp)
-  uint64_t* xempty = xnorm + kXBufs;      // [kXBufs] tile consumed: the products (commit) and the z store (its reads) are done
+  uint64_t* xempty = xnorm + kXBufs;      // [kXBufs] the tile's products are done (commit)
   uint64_t* tfull = xempty + kXBufs;      // [2] accumulator of half h complete
-  uint64_t* tempty = tfull + 2;     // [2] accumulator of half h read by all 16 epilogue warps
+  uint64_t* tempty = tfull + 2;     // [2] accumulator of half h read by its eight epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(wfull, 1);
-    for (int b = 0; b < kXBufs; ++b) { mbar_init(&xfull[b], 1); mbar_init(&xnorm[b], 4); mbar_init(&xempty[b], 2); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 16); }
+    for (int b = 0; b < kXBufs; ++b) { mbar_init(&xfull[b], 1); mbar_init(&xnorm[b], kLnWarps); mbar_init(&xempty[b], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 8); }
     mbar_fence_init();
     tma_prefetch_desc(&tmX);
     tma_prefetch_desc(&tmW);
@@ -104,15 +106,29 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   dependent_enter();
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------------ TMA producer; z leaves from the normalised tiles
     if (elect_one()) {
       mbar_expect_tx(wfull, kWBytes);
       for (int blk = 0; blk < 4; ++blk)
         for (int kb = 0; kb < 2; ++kb) tma_load_3d(sW + (blk * 2 + kb) * kSub, &tmW, wfull, kb * 64, blk * 128, 0);
+      // z of the k-th tile, once its rows are normalised; the buffer is free when the store has read it and the products are done
+      auto store_z = [&](int k) {
+        const int b = k % kXBufs, tile = blockIdx.x + k * gridDim.x;
+        if (!mbar_wait(&xnorm[b], (k / kXBufs) & 1, g.err, 15)) return false;
+        tma_store_3d(&tmZ, sX + b * kXBytes, 0, tile * 128, 0);
+        tma_store_3d(&tmZ, sX + b * kXBytes + kSub, 64, tile * 128, 0);
+        bulk_commit_group();
+        return true;
+      };
       int i = 0;
+      bool ok = true;
       for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
         const int b = i % kXBufs;
-        if (!mbar_wait(&xempty[b], ((i / kXBufs) & 1) ^ 1, g.err, 10)) break;
+        if (i >= kXBufs) {
+          ok = store_z(i - kXBufs);
+          bulk_wait_group_read0();
+          if (!ok || !(ok = mbar_wait(&xempty[b], ((i / kXBufs) & 1) ^ 1, g.err, 10))) break;
+        }
         mbar_expect_tx(&xfull[b], kXBytes);
         if (!g.own_pitch) {
           for (int kb = 0; kb < 2; ++kb) tma_load_3d(sX + b * kXBytes + kb * kSub, &tmX, &xfull[b], kb * 64, tile * 128, 0);
@@ -124,6 +140,8 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           }
         }
       }
+      for (int k = max(0, i - kXBufs); k < i && ok; ++k) ok = store_z(k);
+      bulk_wait_group0();
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -158,54 +176,57 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ LayerNorm: thread = pixel row of the tile
-    const int r0 = threadIdx.x - 64;
-    const uint32_t sw = (uint32_t)(r0 & 7) << 4;
+  } else if (warp < kEpi0) {
+    // ------------------------------------------------------------------ LayerNorm: thread = half of a pixel row of the tile
+    const int r = (warp - 2) * 16 + (lane & 15), kb = lane >> 4;
+    const uint32_t sw = (uint32_t)(r & 7) << 4;
     const T* mask = reinterpret_cast<const T*>(g.mask);
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const int b = i % kXBufs;
       const bool landed = mbar_wait(&xfull[b], (i / kXBufs) & 1, g.err, 14);
       if (!__all_sync(0xffffffffu, landed)) break;
-      const int r = r0;
       uint8_t* rowp = sX + b * kXBytes + r * 128;
+      uint8_t* part = rowp + kb * kSub;
       // Statistics in one pass over the row, shifted by its first element K: sums of (x - K) and (x - K)^2.  K is one
       // of the 128 samples, so (mean - K)^2 <= 128 var and the subtraction below loses at most seven bits of fp32.
       // Packed fp32x2 arithmetic and two accumulators each: the pass is a chain of dependent additions.
       float2 s0 = make_float2(0.f, 0.f), s1 = s0, q0 = s0, q1 = s0;
       const float k0 = unpack2<T>(*reinterpret_cast<const uint32_t*>(rowp + sw)).x;
       const float2 nk = make_float2(-k0, -k0);
-#pragma unroll 4
-      for (int c = 0; c < 16; ++c) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
         float2 v[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(rowp + (c >> 3) * kSub + (((c & 7) << 4) ^ sw)), v);
+        unpack8p<T>(*reinterpret_cast<const uint4*>(part + ((c << 4) ^ sw)), v);
         const float2 d0 = __fadd2_rn(v[0], nk), d1 = __fadd2_rn(v[1], nk), d2 = __fadd2_rn(v[2], nk), d3 = __fadd2_rn(v[3], nk);
         s0 = __fadd2_rn(s0, d0); q0 = __ffma2_rn(d0, d0, q0);
         s1 = __fadd2_rn(s1, d1); q1 = __ffma2_rn(d1, d1, q1);
         s0 = __fadd2_rn(s0, d2); q0 = __ffma2_rn(d2, d2, q0);
         s1 = __fadd2_rn(s1, d3); q1 = __ffma2_rn(d3, d3, q1);
       }
-      const float ms = ((s0.x + s0.y) + (s1.x + s1.y)) * (1.0f / 128);          // mean - K
+      float sum = (s0.x + s0.y) + (s1.x + s1.y), sq = (q0.x + q0.y) + (q1.x + q1.y);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+      const float ms = sum * (1.0f / 128);          // mean - K
       const float mu = ms - nk.x;
-      const float var = fmaxf(((q0.x + q0.y) + (q1.x + q1.y)) * (1.0f / 128) - ms * ms, 0.f);
+      const float var = fmaxf(sq * (1.0f / 128) - ms * ms, 0.f);
       const long long m = (long long)tile * 128 + r;
       const float rs = pixel_rstd(var, g.eps, m, g.n, g.pitch);
       const float2 nmu = make_float2(-mu, -mu);
       const float2 rs2 = make_float2(rs, rs);
 #pragma unroll 4
-      for (int c = 0; c < 16; ++c) {
-        uint4* p = reinterpret_cast<uint4*>(rowp + (c >> 3) * kSub + (((c & 7) << 4) ^ sw));
+      for (int c = 0; c < 8; ++c) {
+        uint4* p = reinterpret_cast<uint4*>(part + ((c << 4) ^ sw));
         float2 v[4];
         unpack8p<T>(*p, v);
         float2 gm[4], bt[4], o[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(s_gamma + c * 8), gm);
-        unpack8p<T>(*reinterpret_cast<const uint4*>(s_beta + c * 8), bt);
+        unpack8p<T>(*reinterpret_cast<const uint4*>(s_gamma + kb * 64 + c * 8), gm);
+        unpack8p<T>(*reinterpret_cast<const uint4*>(s_beta + kb * 64 + c * 8), bt);
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = __ffma2_rn(__fadd2_rn(v[e], nmu), __fmul2_rn(rs2, gm[e]), bt[e]);
         *p = pack8p<T>(o);
       }
-      if (m < g.M) {
+      if (m < g.M && kb == 0) {
         g.mean[m] = mu; g.rstd[m] = rs;
         T* keep = s_mask + (i % kMaskRing) * 128 + r;
         if (g.own_pitch) {   // the mask in its own pitch too, zero at the pixels beyond n
@@ -218,46 +239,36 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       fence_proxy_async_smem();   // the tile is read next by tcgen05.mma and by the TMA store
       __syncwarp();
       if (lane == 0) mbar_arrive(&xnorm[b]);
-      if (r0 == 0) {
-        // every row is normalised once all four warps have arrived; then z leaves from shared memory
-        if (mbar_wait(&xnorm[b], (i / kXBufs) & 1, g.err, 15)) {
-          tma_store_3d(&tmZ, sX + b * kXBytes, 0, tile * 128, 0);
-          tma_store_3d(&tmZ, sX + b * kXBytes + kSub, 64, tile * 128, 0);
-          bulk_commit_group();
-          bulk_wait_group_read0();
-          mbar_arrive(&xempty[b]);
-        }
-      }
-      __syncwarp();
     }
-    if (r0 == 0) bulk_wait_group0();
   } else {
-    // ------------------------------------------------------------------ gate epilogue: thread = channel of the half
-    const int quarter = warp & 3, j = (warp - 6) >> 2;   // TMEM lane quarter; 32-pixel chunk of the tile
+    // ------------------------------------------------------------------ gate epilogue: thread = channel of the set's half
+    const int half = (warp - kEpi0) >> 3, j = (warp - kEpi0) >> 2 & 1, quarter = warp & 3;   // half; 32 pixels of 64; TMEM lane quarter
     const int row = quarter * 32 + lane;
     const bool masked = g.mask != nullptr || g.own_pitch, staged = g.staged != 0;
     const uint32_t plane = (uint32_t)g.plane, M = (uint32_t)g.M;
-    // staging: the 64-pixel chunk of warps j, j ^ 1 and its issuing thread
-    uint8_t* orow = sO + (j >> 1) * kSub + row * 128;
-    const bool issuer = (j & 1) == 0 && quarter == 0 && lane == 0;
+    // staging: a set's 64-pixel chunk and its issuing thread
+    uint8_t* orow = sO + half * kSub + row * 128;
+    const bool issuer = j == 0 && quarter == 0 && lane == 0;
+    float bp = 0.f, bg = 0.f;
+    if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
+    const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+    const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 256;
     int i = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const uint32_t n0 = (uint32_t)tile * 128, nb0 = n0 / plane, np0 = n0 - nb0 * plane;   // one division per tile
-      const uint4* mrow = reinterpret_cast<const uint4*>(s_mask + (i % kMaskRing) * 128 + j * 32);
-      for (int half = 0; half < 2; ++half) {
-        ok = mbar_wait(&tfull[half], i & 1, g.err, 16) && ok;
-        tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 256 + j * 32;
-        float bp = 0.f, bg = 0.f;
-        if (g.bias != nullptr) { bp = g.bias[half * 256 + row]; bg = g.bias[half * 256 + 128 + row]; }
-        const float2 bp2 = make_float2(bp, bp), nbg2 = make_float2(-1.4426950408889634f * bg, -1.4426950408889634f * bg);
+      ok = mbar_wait(&tfull[half], i & 1, g.err, 16) && ok;
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        const uint32_t off = c * 64 + j * 32;
+        const uint4* mrow = reinterpret_cast<const uint4*>(s_mask + (i % kMaskRing) * 128 + off);
         Raw8<T> o[4];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           float p[16], gt[16];
-          ld16x2_f(t_row + hf * 16, t_row + 128 + hf * 16, p, gt);
-          if (hf == 1) {
+          ld16x2_f(t_row + off + hf * 16, t_row + 128 + off + hf * 16, p, gt);
+          if (c == 1 && hf == 1) {
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[half]);
@@ -276,24 +287,24 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           }
         }
         if (staged) {
-          if (issuer) bulk_wait_group_read0();   // the previous half's store has left the chunk
-          named_barrier(1 + (j >> 1), 256);
+          if (issuer) bulk_wait_group_read0();   // the chunk before has left
+          named_barrier(1 + half, 256);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(orow + ((((j & 1) * 4 + u) ^ (row & 7)) << 4)) = o[u].w[0];
+          for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(orow + (((j * 4 + u) ^ (row & 7)) << 4)) = o[u].w[0];
           fence_proxy_async_smem();
-          named_barrier(3 + (j >> 1), 256);
-          const uint32_t px = n0 + (j >> 1) * 64;
+          named_barrier(3 + half, 256);
+          const uint32_t px = n0 + c * 64;
           if (issuer && px < M && ok) {          // a chunk of 64 pixels never straddles two batch entries here
-            tma_store_3d(half == 0 ? &tmA : &tmB, sO + (j >> 1) * kSub, px % plane, 0, px / plane);
+            tma_store_3d(half == 0 ? &tmA : &tmB, sO + half * kSub, px % plane, 0, px / plane);
             bulk_commit_group();
           }
         } else if (ok) {
-          T* base = reinterpret_cast<T*>(half == 0 ? g.a_cm : g.b_cm) + ((long long)nb0 * 128 + row) * g.plane + np0 + j * 32;
+          T* base = reinterpret_cast<T*>(half == 0 ? g.a_cm : g.b_cm) + ((long long)nb0 * 128 + row) * g.plane + np0 + off;
 #pragma unroll
           for (int u = 0; u < 4; ++u) {          // 8 pixels: same batch entry, all valid or none
             T* d8 = base + u * 8;
-            for (uint32_t pix = np0 + j * 32 + u * 8; pix >= plane; pix -= plane) d8 += 127 * g.plane;   // the next batch entry's plane of this channel
-            if (n0 + j * 32 + u * 8 < M) straw8<T>(d8, o[u]);
+            for (uint32_t pix = np0 + off + u * 8; pix >= plane; pix -= plane) d8 += 127 * g.plane;   // the next batch entry's plane of this channel
+            if (n0 + off + u * 8 < M) straw8<T>(d8, o[u]);
           }
         }
       }
@@ -353,12 +364,13 @@ int launch(cudaStream_t st, const LnGateIn& p) {
 // =================================================================================================================
 // ln_gate_out: LayerNorm over the channels of channel-major t, fused into the output projection and gate
 // =================================================================================================================
-// 704 threads as above.  A tile is 128 pixels.  Its t part arrives as the MN-major A operand of the product
+// 832 threads as above.  A tile is 128 pixels.  Its t part arrives as the MN-major A operand of the product
 // y = u Wo^T: per 64-channel half, two chunks of [64 channel rows x 128 bytes = 64 pixels] (128-byte swizzle), which
 // is how the contraction's output lies in memory -- nothing is transposed.  The LayerNorm role normalises every
-// pixel's 128 channels in place: a thread owns 8 pixels (one 16-byte piece of a row) and 16 of the 128 channels;
-// the eight partial (mean, M2) pairs of a pixel are combined through shared memory (Chan's formula), then each
+// pixel's 128 channels in place: a thread owns 8 pixels (one 16-byte piece of a row) and 8 of the 128 channels;
+// the sixteen partial (mean, M2) pairs of a pixel are combined through shared memory (Chan's formula), then each
 // thread rewrites its pieces and, for training, stores them to the channel-major u the backward pass reads.
+// With 128 threads of 16 channels the role took 6.8 k of the 7.1 k cycles of a tile (768 x 768 pixels: 142 us, 118 with 256).
 // The z part (K-major) feeds the gate product unchanged.  Output weights and gate weights stay in shared memory.
 constexpr uint32_t kOWBytes = 4 * kSub;     // (Wo, Wgo) x (k 0..63, k 64..127)
 constexpr uint32_t kOTile = 4 * kSub;       // t: 2 halves x [2 chunks x 8 KB]; z: 2 halves x 16 KB
@@ -389,9 +401,9 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
   uint8_t* sT = smem + kOWBytes;
-  float* s_pm = reinterpret_cast<float*>(sT + kOBufs * kOTile);   // [8][128] partial means
-  float* s_pq = s_pm + 8 * 128;                                   // [8][128] partial sums of squared deviations
-  float* s_mean = s_pq + 8 * 128;
+  float* s_pm = reinterpret_cast<float*>(sT + kOBufs * kOTile);   // [16][128] partial means
+  float* s_pq = s_pm + 16 * 128;                                  // [16][128] partial sums of squared deviations
+  float* s_mean = s_pq + 16 * 128;
   float* s_rstd = s_mean + 128;
   float* s_gamma = s_rstd + 128;
   float* s_beta = s_gamma + 128;
@@ -401,14 +413,15 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
   uint64_t* bempty = bnorm + kOBufs;      // [kOBufs] both products of the tile are done
   uint64_t* tfull = bempty + kOBufs;      // [2] accumulator complete
   uint64_t* tempty = tfull + 2;           // [2] accumulator read by all 16 epilogue warps
-  uint64_t* nsync = tempty + 2;           // [2] the two meeting points of the 128 LayerNorm threads
+  uint64_t* nsync = tempty + 2;           // [2] the two meeting points of the 256 LayerNorm threads
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(nsync + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(wfull, 1);
-    for (int b = 0; b < kOBufs; ++b) { mbar_init(&bfull[b], 1); mbar_init(&bnorm[b], 4); mbar_init(&bempty[b], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 16); mbar_init(&nsync[b], 128); }
+    for (int b = 0; b < kOBufs; ++b) { mbar_init(&bfull[b], 1); mbar_init(&bnorm[b], kLnWarps); mbar_init(&bempty[b], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 16); }
+    mbar_init(&nsync[0], 256); mbar_init(&nsync[1], 128);
     mbar_fence_init();
     tma_prefetch_desc(&tmT);
     tma_prefetch_desc(&tmZ);
@@ -486,20 +499,20 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
+  } else if (warp < kEpi0) {
     // ------------------------------------------------------------------ LayerNorm over channels
     const int tid = threadIdx.x - 64;
-    const int pg = tid & 15, kp = tid >> 4;       // 8-pixel group of the tile; 16-channel part
+    const int pg = tid & 15, kp = tid >> 4;       // 8-pixel group of the tile; 8-channel part
     const int gg = pg & 7;                        // 16-byte piece within the 128-byte row of its 64-pixel chunk
-    const uint32_t part_off = (kp >> 2) * kSub + (pg >> 3) * (kSub / 2) + (kp & 3) * 16 * 128;
+    const uint32_t part_off = (kp >> 3) * kSub + (pg >> 3) * (kSub / 2) + (kp & 7) * 8 * 128;
     T* u_cm = reinterpret_cast<T*>(g.u_cm);
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const int b = i % kOBufs;
       const bool landed = mbar_wait(&bfull[b], (i / kOBufs) & 1, g.err, 24);
       if (!__all_sync(0xffffffffu, landed)) break;
-      uint8_t* part = sT + b * kOTile + part_off;   // rows kp*16 .. kp*16+15 of this thread's chunk
-      // partial statistics of 8 pixels over 16 channels, shifted by the first channel's values
+      uint8_t* part = sT + b * kOTile + part_off;   // rows kp*8 .. kp*8+7 of this thread's chunk
+      // partial statistics of 8 pixels over 8 channels, shifted by the first channel's values
       float2 nk[4], s[4], q[4];
       {
         float2 v[4];
@@ -511,10 +524,10 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
           q[e] = s[e];
         }
       }
-#pragma unroll 4
-      for (int r = 0; r < 16; ++r) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
         float2 v[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(part + r * 128 + ((gg ^ (r & 7)) << 4)), v);
+        unpack8p<T>(*reinterpret_cast<const uint4*>(part + r * 128 + ((gg ^ r) << 4)), v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 d = __fadd2_rn(v[e], nk[e]);
@@ -526,8 +539,8 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
         float pm[8], pq[8];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float sx = s[e].x * (1.0f / 16), sy = s[e].y * (1.0f / 16);
-          pm[2 * e] = sx - nk[e].x;                       // mean of the 16 samples
+          const float sx = s[e].x * (1.0f / 8), sy = s[e].y * (1.0f / 8);
+          pm[2 * e] = sx - nk[e].x;                       // mean of the 8 samples
           pm[2 * e + 1] = sy - nk[e].y;
           pq[2 * e] = fmaxf(q[e].x - s[e].x * sx, 0.f);   // their sum of squared deviations
           pq[2 * e + 1] = fmaxf(q[e].y - s[e].y * sy, 0.f);
@@ -540,22 +553,22 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       mbar_arrive(&nsync[0]);
       const bool met0 = mbar_wait(&nsync[0], i & 1, g.err, 25);
       if (!__all_sync(0xffffffffu, met0)) break;
-      {
-        // thread = pixel: combine the eight partials (equal counts): M2 = sum M2_k + 16 sum (mean_k - mean)^2
-        float pm[8], m = 0.f, m2 = 0.f;
+      if (tid < 128) {
+        // thread = pixel: combine the sixteen partials (equal counts): M2 = sum M2_k + 8 sum (mean_k - mean)^2
+        float m = 0.f, m2 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) { pm[k] = s_pm[k * 128 + tid]; m += pm[k]; m2 += s_pq[k * 128 + tid]; }
-        m *= (1.0f / 8);
+        for (int k = 0; k < 16; ++k) { m += s_pm[k * 128 + tid]; m2 += s_pq[k * 128 + tid]; }
+        m *= (1.0f / 16);
         float dev = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dev = fmaf(pm[k] - m, pm[k] - m, dev);
+        for (int k = 0; k < 16; ++k) { const float d = s_pm[k * 128 + tid] - m; dev = fmaf(d, d, dev); }
         const long long px = (long long)tile * 128 + tid;
-        const float rs = pixel_rstd((m2 + 16.f * dev) * (1.0f / 128), g.eps, px, g.n, g.pitch);
+        const float rs = pixel_rstd((m2 + 8.f * dev) * (1.0f / 128), g.eps, px, g.n, g.pitch);
         s_mean[tid] = m;
         s_rstd[tid] = rs;
         if (px < g.M) { g.mean[px] = m; g.rstd[px] = rs; }
+        mbar_arrive(&nsync[1]);
       }
-      mbar_arrive(&nsync[1]);
       const bool met1 = mbar_wait(&nsync[1], i & 1, g.err, 26);
       if (!__all_sync(0xffffffffu, met1)) break;
       {
@@ -564,13 +577,13 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
         const float2 nm[4] = {make_float2(-m0.x, -m0.y), make_float2(-m0.z, -m0.w), make_float2(-m1.x, -m1.y), make_float2(-m1.z, -m1.w)};
         const float2 rr[4] = {make_float2(r0.x, r0.y), make_float2(r0.z, r0.w), make_float2(r1.x, r1.y), make_float2(r1.z, r1.w)};
         const long long px0 = (long long)tile * 128 + pg * 8;   // 8 pixels: all inside the tensor or none
-        T* udst = (u_cm != nullptr && px0 < g.M) ? u_cm + (long long)(kp * 16) * g.M + px0 : nullptr;
+        T* udst = (u_cm != nullptr && px0 < g.M) ? u_cm + (long long)(kp * 8) * g.M + px0 : nullptr;
 #pragma unroll 4
-        for (int r = 0; r < 16; ++r) {
-          uint4* p = reinterpret_cast<uint4*>(part + r * 128 + ((gg ^ (r & 7)) << 4));
+        for (int r = 0; r < 8; ++r) {
+          uint4* p = reinterpret_cast<uint4*>(part + r * 128 + ((gg ^ r) << 4));
           float2 v[4], o[4];
           unpack8p<T>(*p, v);
-          const float gm = s_gamma[kp * 16 + r], bt = s_beta[kp * 16 + r];
+          const float gm = s_gamma[kp * 8 + r], bt = s_beta[kp * 8 + r];
           const float2 gm2 = make_float2(gm, gm), bt2 = make_float2(bt, bt);
 #pragma unroll
           for (int e = 0; e < 4; ++e) o[e] = __ffma2_rn(__fadd2_rn(v[e], nm[e]), __fmul2_rn(rr[e], gm2), bt2);
@@ -585,7 +598,7 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
     }
   } else {
     // ------------------------------------------------------------------ gate epilogue: thread = pixel
-    const int quarter = warp & 3, j = (warp - 6) >> 2;   // TMEM lane quarter; 32-channel chunk of the output row
+    const int quarter = warp & 3, j = (warp - kEpi0) >> 2;   // TMEM lane quarter; 32-channel chunk of the output row
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       const int acc = i & 1;
@@ -667,7 +680,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   OutArgs a;
   a.M = p.M; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps; a.gamma = p.gamma; a.beta = p.beta;
   a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.n = p.n; a.pitch = p.pitch; a.own_pitch = p.own_pitch; a.err = p.err;
-  constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 8 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
+  constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 16 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_out_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
