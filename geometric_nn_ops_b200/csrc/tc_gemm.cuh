@@ -67,7 +67,7 @@ struct GemmArgs {
   int kblocks0, kblocks1;    // K blocks (of 128 bytes) in segment 0 / segment 1 (0 = no second segment)
   int seg1_col;              // accumulator column where segment 1 lands (0 = add to segment 0's columns)
   int seg1_n;                // N extent of segment 1's MMA (columns), segment 0 uses bn0
-  int bn0;                   // N extent of segment 0's MMA
+  int bn0;                   // N extent of segment 0's MMA: the columns from one tile to the next, up to the kernel's BN
   int batches, tiles_m, tiles_n;
   int split_k;               // batch index selects K range [batch*kblocks0, ...) instead of a batch entry
   int a_tile_batch;          // the M-tile index is A's batch coordinate (rows 0..127 of plane tile_m)
@@ -286,8 +286,15 @@ __device__ __forceinline__ void store_row32(TOUT* dst, const float (&v)[32], int
     for (int i = 0; i < 4; ++i) store8<TOUT>(dst + 8 * i, &v[8 * i]);
   } else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < valid) dst[i] = from_f32<TOUT>(v[i]);
+    for (int i = 0; i < 4; ++i) {
+      if (vec_ok && i * 8 + 8 <= valid) {
+        store8<TOUT>(dst + 8 * i, &v[8 * i]);
+      } else {
+#pragma unroll
+        for (int e = i * 8; e < i * 8 + 8; ++e)
+          if (e < valid) dst[e] = from_f32<TOUT>(v[e]);
+      }
+    }
   }
 }
 
@@ -649,7 +656,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
         int tm, tn, bz;
         decode(tile, tm, tn, bz);
-        const int n0 = tn * (g.seg1_col ? g.bn0 : BN);
+        const int n0 = tn * g.bn0;
         const int zc = g.split_k ? 0 : bz;
         const int koff = g.split_k ? bz * g.kblocks0 * BKE : 0;
         const int am = g.a_tile_batch ? 0 : tm * kBM, az = g.a_tile_batch ? tm : zc;
@@ -804,25 +811,23 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       if constexpr (EPI == EPI_STORE || EPI == EPI_GATE_MUL) {
-        const int m = tm * kBM + row, n0 = tn * BN;
+        const int m = tm * kBM + row, n0 = tn * g.bn0, n_end = min(g.N, n0 + g.bn0);
         TOUT* out = reinterpret_cast<TOUT*>(g.out0) + bz * g.batch_out + (long long)m * g.ld_out;
         const bool vec_ok = (g.ld_out * sizeof(TOUT)) % 16 == 0 && (g.batch_out * sizeof(TOUT)) % 16 == 0 && (reinterpret_cast<uintptr_t>(g.out0) & 15) == 0;
-        constexpr int CH = BN / 32 / NGRP;  // 32-column chunks per group
 #pragma unroll 1
-        for (int jj = 0; jj < CH; ++jj) {
-          const int j = grp * CH + jj;
+        for (int j = grp; j * 32 < g.bn0; j += NGRP) {   // 32-column chunks
           float v[32];
           ld32_f(t_row + j * 32, v);
           const int n = n0 + j * 32;
           if (g.bias0 != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) if (n + i < g.N) v[i] += g.bias0[n + i];
+            for (int i = 0; i < 32; ++i) if (n + i < n_end) v[i] += g.bias0[n + i];
           }
           if constexpr (EPI == EPI_GATE_MUL) {   // (N is a multiple of eight)
             const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const TIN*>(g.aux) + (long long)m * g.ld_out + n);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              if (m >= g.M || n + u * 8 >= g.N) continue;
+              if (m >= g.M || n + u * 8 >= n_end) continue;
               const uint4 x = src[u];
               const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -833,8 +838,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               }
             }
           }
-          if ((g.M & 3) == 0 && vec_ok && g.N - n >= 32) store_rows32<TOUT>(out + n, v, g.ld_out, m < g.M, lane);
-          else if (m < g.M && n < g.N) store_row32<TOUT>(out + n, v, g.N - n, vec_ok);
+          if ((g.M & 3) == 0 && vec_ok && n_end - n >= 32) store_rows32<TOUT>(out + n, v, g.ld_out, m < g.M, lane);
+          else if (m < g.M && n < n_end) store_row32<TOUT>(out + n, v, n_end - n, vec_ok);
         }
       } else if constexpr (EPI == EPI_GATE_IN || EPI == EPI_GATE_IN_BWD) {
         // row = channel of half tm; columns: P for pixels n0..n0+127, then G for the same pixels

@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 CASES = [  # batch, M, N, K
     (1, 128, 128, 64), (1, 128, 256, 128), (3, 256, 512, 192), (2, 200, 136, 72), (4, 768, 768, 768),
     (1, 64, 40, 24),
+    (2, 208, 208, 208), (2, 136, 264, 64), (1, 384, 384, 384), (1, 128, 520, 128),   # tiles narrower than 256 columns, pieces of 8 and 16
 ]
 
 
