@@ -1044,5 +1044,9 @@ struct GemmPlan {
 // dtype: TRI_F32 (tf32 MMA), TRI_BF16, TRI_F16.  out_f32: EPI_STORE writes fp32 instead of the input dtype.
 int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const GemmPlan& p, int* err);
 
+// The plain product on pairs of SMs (tc_gemm_pair.cu).  Does it suit, against tiles of 128 x `width`?  ta, tb: boxes of 128 rows.
+bool gemm_pair_fits(const GemmPlan& p, int width);
+int launch_gemm_pair(cudaStream_t st, int dtype, const CUtensorMap& ta, const CUtensorMap& tb, const GemmPlan& p, int* err);
+
 }  // namespace tc
 }  // namespace tri

@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 CASES = [  # batch, M, N, K
     (1, 128, 128, 64), (1, 128, 256, 128), (3, 256, 512, 192), (2, 200, 136, 72), (4, 768, 768, 768),
     (1, 64, 40, 24),
+    (40, 512, 512, 128), (80, 456, 504, 72), (40, 504, 488, 448),   # pairs of SMs: whole and ragged tiles, more stages than there are
     (2, 208, 208, 208), (2, 136, 264, 64), (1, 384, 384, 384), (1, 128, 520, 128),   # tiles narrower than 256 columns, pieces of 8 and 16
 ]
 
