@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(256) round_copies_kernel(const RoundArgs a) {
 // backward, in one launch: q, k, v and dO rounded, the row constants as factors and (for flagged rows) as prep = -m | -log l log2e |
 // -delta, the key-mask terms (0, -1e9, -inf beyond N; in a second plane times log2(e)), the bias transposed.  A block has a (batch, row,
 // head), a warp 32 queries at a time, eight lanes to a row of up to 32 channels; the first blocks transpose a tile of 32 x 32 each.  Bound by
-// the bytes: N = 256, 4 heads of 32, 56 us, 48 by the copy rate, as four kernels 35 + 26 + 3 + 4 and their gaps.
+// the bytes: N = 256, 4 heads of 32, 52 us, 48 by the copy rate (with three blocks an SM its
+// registers spill: 68), as four kernels 35 + 26 + 3 + 4 and their gaps.
 struct PrepareArgs {
   const float *q, *k, *v, *o, *d_o, *stats, *bias;
   float *q_r, *k_r, *v_r, *d_o_r;   // [B][S][N][H][D]
@@ -101,7 +102,7 @@ struct PrepareArgs {
   const uint8_t* mask;
   int npad, pitch, tiles, transposes;   // tiles of a side of the bias; blocks that transpose
 };
-__global__ void __launch_bounds__(256, 3) prepare_bwd_kernel(const TriAttnDesc d, const PrepareArgs a) {
+__global__ void __launch_bounds__(256, 2) prepare_bwd_kernel(const TriAttnDesc d, const PrepareArgs a) {
   __shared__ float tile[32][33];
   dependent_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = d.n_res;
@@ -129,8 +130,8 @@ __global__ void __launch_bounds__(256, 3) prepare_bwd_kernel(const TriAttnDesc d
       a.mask_terms[(planes + bs) * a.npad + k] = v * kLog2e;
     }
   }
-  const int ch = (lane & 7) * 4;
-  const bool on = ch < d.D;
+  const bool on = (lane & 7) * 4 < d.D;
+  const int ch = on ? (lane & 7) * 4 : 0;
   const float *qb = a.q + b * d.q_st[0] + s * d.q_st[1] + h * d.q_st[3] + ch, *kb = a.k + b * d.k_st[0] + s * d.k_st[1] + h * d.k_st[3] + ch,
               *vb = a.v + b * d.v_st[0] + s * d.v_st[1] + h * d.v_st[3] + ch, *ob = a.o + b * d.o_st[0] + s * d.o_st[1] + h * d.o_st[3] + ch,
               *gb = a.d_o + b * d.do_st[0] + s * d.do_st[1] + h * d.do_st[3] + ch;
@@ -145,20 +146,22 @@ __global__ void __launch_bounds__(256, 3) prepare_bwd_kernel(const TriAttnDesc d
     for (int e = 0; e < 8; e += 2) {
       float4 x[2][5];
       float part[2] = {0.f, 0.f};
+      bool live[2];
 #pragma unroll
       for (int f = 0; f < 2; ++f) {
         const int n = n0 + (e + f) * 4 + (lane >> 3);
-        if (!(on && n < N)) continue;
-        x[f][0] = *reinterpret_cast<const float4*>(ob + n * d.o_st[2]);
-        x[f][1] = *reinterpret_cast<const float4*>(gb + n * d.do_st[2]);
-        x[f][2] = *reinterpret_cast<const float4*>(qb + n * d.q_st[2]);
-        x[f][3] = *reinterpret_cast<const float4*>(kb + n * d.k_st[2]);
-        x[f][4] = *reinterpret_cast<const float4*>(vb + n * d.v_st[2]);
+        live[f] = on && n < N;
+        const int64_t r = live[f] ? n : 0;   // (a row that is there in place of one that is not: the loads need no branch)
+        x[f][0] = *reinterpret_cast<const float4*>(ob + r * d.o_st[2]);
+        x[f][1] = *reinterpret_cast<const float4*>(gb + r * d.do_st[2]);
+        x[f][2] = *reinterpret_cast<const float4*>(qb + r * d.q_st[2]);
+        x[f][3] = *reinterpret_cast<const float4*>(kb + r * d.k_st[2]);
+        x[f][4] = *reinterpret_cast<const float4*>(vb + r * d.v_st[2]);
       }
 #pragma unroll
       for (int f = 0; f < 2; ++f) {
         const int n = n0 + (e + f) * 4 + (lane >> 3);
-        if (!(on && n < N)) continue;
+        if (!live[f]) continue;
         part[f] = fmaf(x[f][0].x, x[f][1].x, fmaf(x[f][0].y, x[f][1].y, fmaf(x[f][0].z, x[f][1].z, x[f][0].w * x[f][1].w)));
         const long long to = (((long long)bs * N + n) * d.H + h) * d.D + ch;
         float* const dst[4] = {a.d_o_r, a.q_r, a.k_r, a.v_r};
