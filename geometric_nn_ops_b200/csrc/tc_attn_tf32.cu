@@ -839,7 +839,7 @@ int attn_tf32_backward(const TriAttnDesc* d, const void* q, const void* k, const
     p.tiles = cdiv(d->n_res, 32);
     p.transposes = bias != nullptr ? p.tiles * p.tiles * batches_of(d) * d->H : 0;
     const long long planes = (long long)d->B * d->n_seq;
-    KernelTimer kt("tc_attn_prepare", st, 0.0, 9.0 * tensor);
+    KernelTimer kt("tc_attn_delta", st, 0.0, 9.0 * tensor);
     prepare_bwd_kernel<<<(unsigned)(p.transposes + planes * d->H), 256, 0, st>>>(*d, p);
     TRI_LAUNCH_OK();
   }

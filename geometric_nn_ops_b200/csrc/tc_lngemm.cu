@@ -17,9 +17,10 @@
 // at first, 0.165 with a reciprocal instead of a quotient in the sigmoid, pairwise conversions, the mask read once per
 // tile and staged stores, and 0.145 with eight LayerNorm warps (four took 5.3 k cycles a tile, one of them 2 k more for the store of
 // z, where a tile takes 8.5 k in all) and the epilogue in two sets (as one, 4.8 k cycles of arithmetic, 1.4 of staging and 1.3 of
-// waiting followed one another); floor by bytes 0.092.  What bounds it is the path of shared memory and TMEM: MMA operands, accumulators,
-// the LayerNorm's passes and the tiles' ways in and out take about 6.6 k of the 7.4 k cycles of a tile at 128 bytes each.  (One reciprocal for
-// two sigmoids changes nothing; rows kept in registers between the passes spill at 72 a thread.)
+// waiting followed one another); floor by bytes 0.092.  What bounds it is likely the path of shared memory and TMEM: counted at 128 bytes a cycle,
+// MMA operands, accumulators, the LayerNorm's passes and the tiles' ways in and out take about 6.6 k of the 7.4 k cycles of a tile (an estimate;
+// ncu: load / store wavefronts 40 %, XU 54 %, tensor 26 %, DRAM 46 %).  (One reciprocal for two sigmoids changes nothing; rows kept in registers
+// between the passes spill at 72 a thread.)
 // Every mbarrier wait is bounded; a timeout lands in *err and all roles drain.
 #include "tc_lngemm.cuh"
 
