@@ -14,8 +14,8 @@
 // Row constants come with the products (TfFactors); the mathematics is that of tc_attn.cu.
 //
 // What bounds them: the chain of a step (no pipe is above 40 %), and the copies: 100 to 270 MB of rounded operands per direction.
-// One training step at N = 256, 4 heads of 32, 785 us on the CUDA cores' path: rounding 76, forward 70, delta 31, dK / dV 98,
-// dQ 85, dbias 64.  What took the passes there: sums that are stored beside the next item's first step (dK / dV 113 -> 98 us,
+// One training step at N = 256, 4 heads of 32, 785 us on the CUDA cores' path: rounding 34, forward 70, the backward's
+// preparation 52, dK / dV 93, dQ 87, dbias 60.  What took the passes there: sums that are stored beside the next item's first step (dK / dV 113 -> 98 us,
 // with the copies issued in the order in which their places become free).  Two sets of warps on alternate steps: no difference.
 #include <algorithm>
 #include <cstdlib>
