@@ -902,7 +902,7 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
           }
         }
       }
-      if (ok) umma_commit(sums);
+      umma_commit(sums);   // (after a wait that ran out too: the products issued before it)
       bulk_wait_group0();
     }
     __syncwarp();
@@ -1007,9 +1007,10 @@ gate_in_bwd_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
       __syncwarp();
       if (lane == 0) { mbar_arrive(&ofull[2 * i % kO]); mbar_arrive(&ofull[(2 * i + 1) % kO]); }
     }
+    // The products into the sums read shared memory and write TMEM until this commit, whether or not the sums are asked for.
+    if (items > 0) ok = mbar_wait(sums, 0, g.err, 71) && ok;
     // the sums: this thread's row of dP and of dG, a quarter of the 256 columns
     if (g.partial != nullptr && items > 0) {
-      ok = mbar_wait(sums, 0, g.err, 71) && ok;
       tc_fence_after_sync();
       float* dst = g.partial + ((long long)tile0 * 512 + half * 256 + (j >> 1) * 128 + row) * 128 + (j & 1) * 64;
 #pragma unroll 1

@@ -276,3 +276,19 @@ def test_input_weight_gradients_over_few_tiles(tmu, n, dtype, precision):
     _, g_ref = util.trimul_oracle(x, mask, w, "outgoing", d_out)
     for name in ("x", "p_in_weight", "g_in_weight"):
         util.check_close("grad_" + name, grads[name], g_ref[name], *_tol(dtype, precision))
+
+
+@pytest.mark.parametrize("frozen", [("p_in_weight", "g_in_weight"), ("p_in_weight",), ("g_in_weight",)], ids=lambda f: "+".join(n[0] for n in f))
+@pytest.mark.parametrize("n", [8, 72, 104])
+@pytest.mark.parametrize("dtype,precision", [m for m in MODES if m != (torch.float32, "ieee")], ids=lambda v: str(v).replace("torch.", ""))
+def test_frozen_input_weights(tmu, n, dtype, precision, frozen):
+    """The input gate's backward where no sums over the pixels are asked for, or those of one weight."""
+    x, mask, w, d_out = util.trimul_inputs(1, n, 128, 128, dtype, seed=n, biases=True)
+    leaves = {k: v.requires_grad_() for k, v in {"x": x, **w}.items() if k not in frozen}
+    with util.matmul_precision(precision):
+        out = tmu(x, "outgoing", mask, **w)
+        grads = dict(zip(leaves, torch.autograd.grad(out, list(leaves.values()), grad_outputs=d_out)))
+    _, g_ref = util.trimul_oracle(x, mask, w, "outgoing", d_out)
+    cos_min, fro = util.TRIMUL_TOL[dtype, precision]
+    for name, grad in grads.items():
+        util.check_close("grad_" + name, grad, g_ref[name], cos_min, 2 * fro)   # (small sums: twice the tables' bound)
