@@ -292,3 +292,19 @@ def test_frozen_input_weights(tmu, n, dtype, precision, frozen):
     cos_min, fro = util.TRIMUL_TOL[dtype, precision]
     for name, grad in grads.items():
         util.check_close("grad_" + name, grad, g_ref[name], cos_min, 2 * fro)   # (small sums: twice the tables' bound)
+
+
+def test_unasked_sums_are_not_formed(tmu):
+    """Without gradients of the input weights the input gate's backward has no products over the pixels."""
+    from geometric_nn_ops_b200 import _lib
+    x, mask, w, d_out = util.trimul_inputs(1, 64, 128, 128, torch.bfloat16)
+    flops = {}
+    for frozen in (False, True):
+        leaves = [v.requires_grad_(not (frozen and k in ("p_in_weight", "g_in_weight"))) for k, v in {"x": x, **w}.items()]
+        out = tmu(x, "outgoing", mask, **w)
+        _lib.profile_enable(True)
+        torch.autograd.grad(out, [v for v in leaves if v.requires_grad], grad_outputs=d_out)
+        torch.cuda.synchronize()
+        flops[frozen] = _lib.profile_summary()["tc_gate_in_bwd"][2]
+        _lib.profile_enable(False)
+    assert flops[False] > 0 and flops[True] == 0
