@@ -155,7 +155,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 9) {
     // ---------------------------------- TMA copies, mask terms -----------------------------------
-    // The warp runs together: a lane writes the terms of four keys of a tile, lane 0 issues the copies.
+    // The warp runs together, and gives up together: a lane writes the terms of four keys of a tile, lane 0 issues the copies.
     auto load_q = [&](int n) {
       if (lane != 0) return;
       const Item it = item_of(n);
@@ -211,7 +211,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     int jt = 0, n_cur = 0;   // key tile and item of stream position c
     for (int c = 0; c < total && ok; ++c) {
       if (c + 2 < total) fetch_mask(la, la_t);
-      ok = mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16) && ok;   // S(c) has been read: its K stage and mask terms are free
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16));   // S(c) has been read: its K stage and mask terms are free
       if (++jt == nt) {                                    // ... and it was the item's last use of Q
         jt = 0;
         if (++n_cur < my_items) load_q(n_cur);
@@ -219,7 +219,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (c + 2 < total) {
         load_k(c + 2, la, la_t);
         if (HB && TMEM_P) load_bias(c + 2, la, la_t);      // the bias tile has been read too and P does not replace it
-        ok = mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, a.err, 15) && ok;   // P V(c) done: its V stage and P buffer are free
+        ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, a.err, 15)) && ok;   // P V(c) done: its V stage and P buffer are free
         if (HB && !TMEM_P) load_bias(c + 2, la, la_t);
         load_v(c + 2, la, la_t);
         advance();

@@ -212,7 +212,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int n = 0; n < my_items && ok; ++n) {
         const Item after = item_of(n + 1 < my_items ? n + 1 : n);
         for (int j = 0; j < nk; ++j) {
-          ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51);
+          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51));   // (the warp gives up together)
           if (!ok) break;
           if (lane == 0) {
             mbar_expect_tx(&b_full[stg], HB ? M::TB : 0);
@@ -380,12 +380,11 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         a.stats[(long long)a.B * a.S * a.H * a.N + pstat] = (logf(pl) - factor(pm) * kLn2) - (top - pm);
       }
     };
-    for (int n = 0; g < R && n < my_items && ok; ++n) {
+    for (int n = 0; g < R && n < my_items && __all_sync(0xffffffffu, ok); ++n) {
       const Item it = item_of(n);
       if (it.s0 + g >= a.S) {   // no row for this group: let the bias tiles pass
         for (int j = 0; j < nk && ok; ++j) {
-          ok = mbar_wait_relaxed(&b_full[bstg], bph, a.err, 57);
-          __syncwarp();
+          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_full[bstg], bph, a.err, 57));
           if (lane == 0) mbar_arrive(&b_free[bstg]);
           if (++bstg == kBiasStages) { bstg = 0; bph ^= 1; }
         }

@@ -469,7 +469,7 @@ attn_bwd_tf32_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_cons
       }
     };
     int c = 0, flag = total > 0 ? flag_of(0) : 0;
-    for (int n = 0; n < my_items && ok; ++n) {
+    for (int n = 0; n < my_items && __all_sync(0xffffffffu, ok); ++n) {
       const bool folded = flag == 0;
       flag = flag_of(n + 1);
       for (int j = 0; j < nsteps; ++j, ++c) {

@@ -807,7 +807,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       decode(tile, tm, tn, bz);
       Raw8<TIN> dpre[CPG][4];
       if constexpr (kGradTile) fetch_grad(tile, dpre);
-      if (!mbar_wait(&tfull[acc], acc_phase, g.err, 4)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&tfull[acc], acc_phase, g.err, 4))) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       if constexpr (EPI == EPI_STORE || EPI == EPI_GATE_MUL) {
