@@ -5,8 +5,9 @@
 //                two 32 KB buffers; stores each tile as z once it is normalised
 //   warp 1       tcgen05.mma: per tile and half (a, b) the P and G products, M = the half's 128 channels, N = 128
 //                pixels, into the half's 256-column accumulator
-//   warps 2-9    LayerNorm: thread = half of a pixel row; normalises it in place (two passes over it in shared memory:
-//                statistics, result), writes the statistics and releases the tile to the MMA warp and to the store.
+//   warps 2-9    LayerNorm: two threads to a pixel row, which is normalised in place (two passes over it in shared memory: one
+//                chain of the statistics' sums each, half of the result each); they write the statistics and release the tile
+//                to the MMA warp and to the store.
 //   warps 10-25  gate epilogue, thread = channel holding consecutive pixels (the order of the channel-major a / b); a set of
 //                eight warps for each half, so that one set's waits and stores run beside the other's arithmetic
 //
@@ -178,7 +179,7 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     }
     __syncwarp();
   } else if (warp < kEpi0) {
-    // ------------------------------------------------------------------ LayerNorm: thread = half of a pixel row of the tile
+    // ------------------------------------------------------------------ LayerNorm: two threads to a pixel row of the tile
     const int r = (warp - 2) * 16 + (lane & 15), kb = lane >> 4;
     const uint32_t sw = (uint32_t)(r & 7) << 4;
     const T* mask = reinterpret_cast<const T*>(g.mask);
@@ -191,21 +192,22 @@ ln_gate_in_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       uint8_t* part = rowp + kb * kSub;
       // Statistics in one pass over the row, shifted by its first element K: sums of (x - K) and (x - K)^2.  K is one
       // of the 128 samples, so (mean - K)^2 <= 128 var and the subtraction below loses at most seven bits of fp32.
-      // Packed fp32x2 arithmetic and two accumulators each: the pass is a chain of dependent additions.
-      float2 s0 = make_float2(0.f, 0.f), s1 = s0, q0 = s0, q1 = s0;
+      // Packed fp32x2 arithmetic: a row's even pairs of channels are one chain of additions and its odd pairs the other, a
+      // thread has one of the two.  (So the sums do not depend on how many threads share a row; split by halves of the row they
+      // had other last bits, which in 16 bits a stack of blocks carries on.)
+      float2 s = make_float2(0.f, 0.f), q = s;
       const float k0 = unpack2<T>(*reinterpret_cast<const uint32_t*>(rowp + sw)).x;
       const float2 nk = make_float2(-k0, -k0);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float2 v[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(part + ((c << 4) ^ sw)), v);
-        const float2 d0 = __fadd2_rn(v[0], nk), d1 = __fadd2_rn(v[1], nk), d2 = __fadd2_rn(v[2], nk), d3 = __fadd2_rn(v[3], nk);
-        s0 = __fadd2_rn(s0, d0); q0 = __ffma2_rn(d0, d0, q0);
-        s1 = __fadd2_rn(s1, d1); q1 = __ffma2_rn(d1, d1, q1);
-        s0 = __fadd2_rn(s0, d2); q0 = __ffma2_rn(d2, d2, q0);
-        s1 = __fadd2_rn(s1, d3); q1 = __ffma2_rn(d3, d3, q1);
+      const uint8_t* chain = rowp + kb * 4;
+#pragma unroll 8
+      for (int c = 0; c < 16; ++c) {
+        const uint8_t* p = chain + (c >> 3) * kSub + (((c & 7) << 4) ^ sw);
+        const float2 d0 = __fadd2_rn(unpack2<T>(*reinterpret_cast<const uint32_t*>(p)), nk);
+        const float2 d1 = __fadd2_rn(unpack2<T>(*reinterpret_cast<const uint32_t*>(p + 8)), nk);
+        s = __fadd2_rn(s, d0); q = __ffma2_rn(d0, d0, q);
+        s = __fadd2_rn(s, d1); q = __ffma2_rn(d1, d1, q);
       }
-      float sum = (s0.x + s0.y) + (s1.x + s1.y), sq = (q0.x + q0.y) + (q1.x + q1.y);
+      float sum = s.x + s.y, sq = q.x + q.y;
       sum += __shfl_xor_sync(0xffffffffu, sum, 16);
       sq += __shfl_xor_sync(0xffffffffu, sq, 16);
       const float ms = sum * (1.0f / 128);          // mean - K
@@ -368,9 +370,9 @@ int launch(cudaStream_t st, const LnGateIn& p) {
 // 832 threads as above.  A tile is 128 pixels.  Its t part arrives as the MN-major A operand of the product
 // y = u Wo^T: per 64-channel half, two chunks of [64 channel rows x 128 bytes = 64 pixels] (128-byte swizzle), which
 // is how the contraction's output lies in memory -- nothing is transposed.  The LayerNorm role normalises every
-// pixel's 128 channels in place: a thread owns 8 pixels (one 16-byte piece of a row) and 8 of the 128 channels;
-// the sixteen partial (mean, M2) pairs of a pixel are combined through shared memory (Chan's formula), then each
-// thread rewrites its pieces and, for training, stores them to the channel-major u the backward pass reads.
+// pixel's 128 channels in place: a thread sums 4 pixels over 16 of the 128 channels, the eight partial (mean, M2) pairs of a
+// pixel are combined through shared memory (Chan's formula), then each thread rewrites 8 pixels (one 16-byte piece of a row) of
+// 8 channels and, for training, stores them to the channel-major u the backward pass reads.
 // With 128 threads of 16 channels the role took 6.8 k of the 7.1 k cycles of a tile (768 x 768 pixels: 142 us, 118 with 256).
 // The z part (K-major) feeds the gate product unchanged.  Output weights and gate weights stay in shared memory.
 constexpr uint32_t kOWBytes = 4 * kSub;     // (Wo, Wgo) x (k 0..63, k 64..127)
@@ -402,9 +404,9 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sW = smem;
   uint8_t* sT = smem + kOWBytes;
-  float* s_pm = reinterpret_cast<float*>(sT + kOBufs * kOTile);   // [16][128] partial means
-  float* s_pq = s_pm + 16 * 128;                                  // [16][128] partial sums of squared deviations
-  float* s_mean = s_pq + 16 * 128;
+  float* s_pm = reinterpret_cast<float*>(sT + kOBufs * kOTile);   // [8][128] partial means
+  float* s_pq = s_pm + 8 * 128;                                   // [8][128] partial sums of squared deviations
+  float* s_mean = s_pq + 8 * 128;
   float* s_rstd = s_mean + 128;
   float* s_gamma = s_rstd + 128;
   float* s_beta = s_gamma + 128;
@@ -506,6 +508,10 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
     const int pg = tid & 15, kp = tid >> 4;       // 8-pixel group of the tile; 8-channel part
     const int gg = pg & 7;                        // 16-byte piece within the 128-byte row of its 64-pixel chunk
     const uint32_t part_off = (kp >> 3) * kSub + (pg >> 3) * (kSub / 2) + (kp & 7) * 8 * 128;
+    // the statistics: 4-pixel group; 16-channel part (a warp's).  As in ln_gate_in, the sums are those that 128 threads formed.
+    const int p4 = tid & 31, k16 = tid >> 5;
+    const uint32_t stat_off = (k16 >> 2) * kSub + (p4 >> 4) * (kSub / 2) + (k16 & 3) * 16 * 128 + (p4 & 1) * 8;
+    const int g4 = p4 >> 1 & 7;
     T* u_cm = reinterpret_cast<T*>(g.u_cm);
     int i = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
@@ -513,58 +519,52 @@ ln_gate_out_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constan
       const bool landed = mbar_wait(&bfull[b], (i / kOBufs) & 1, g.err, 24);
       if (!__all_sync(0xffffffffu, landed)) break;
       uint8_t* part = sT + b * kOTile + part_off;   // rows kp*8 .. kp*8+7 of this thread's chunk
-      // partial statistics of 8 pixels over 8 channels, shifted by the first channel's values
-      float2 nk[4], s[4], q[4];
-      {
-        float2 v[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(part + (gg << 4)), v);
+      // partial statistics of 4 pixels over 16 channels, shifted by the first channel's values
+      const uint8_t* stat = sT + b * kOTile + stat_off;
+      float2 nk[2], s[2], q[2];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          nk[e] = make_float2(-v[e].x, -v[e].y);
-          s[e] = make_float2(0.f, 0.f);
-          q[e] = s[e];
-        }
-      }
+      for (int r = 0; r < 16; ++r) {
+        const uint2 w = *reinterpret_cast<const uint2*>(stat + r * 128 + ((g4 ^ (r & 7)) << 4));
+        const float2 v[2] = {unpack2<T>(w.x), unpack2<T>(w.y)};
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        float2 v[4];
-        unpack8p<T>(*reinterpret_cast<const uint4*>(part + r * 128 + ((gg ^ r) << 4)), v);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 2; ++e) {
+          if (r == 0) {
+            nk[e] = make_float2(-v[e].x, -v[e].y);
+            s[e] = make_float2(0.f, 0.f);
+            q[e] = s[e];
+          }
           const float2 d = __fadd2_rn(v[e], nk[e]);
           s[e] = __fadd2_rn(s[e], d);
           q[e] = __ffma2_rn(d, d, q[e]);
         }
       }
       {
-        float pm[8], pq[8];
+        float pm[4], pq[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float sx = s[e].x * (1.0f / 8), sy = s[e].y * (1.0f / 8);
-          pm[2 * e] = sx - nk[e].x;                       // mean of the 8 samples
+        for (int e = 0; e < 2; ++e) {
+          const float sx = s[e].x * (1.0f / 16), sy = s[e].y * (1.0f / 16);
+          pm[2 * e] = sx - nk[e].x;                       // mean of the 16 samples
           pm[2 * e + 1] = sy - nk[e].y;
           pq[2 * e] = fmaxf(q[e].x - s[e].x * sx, 0.f);   // their sum of squared deviations
           pq[2 * e + 1] = fmaxf(q[e].y - s[e].y * sy, 0.f);
         }
-        float4* dm = reinterpret_cast<float4*>(s_pm + kp * 128 + pg * 8);
-        float4* dq = reinterpret_cast<float4*>(s_pq + kp * 128 + pg * 8);
-        dm[0] = make_float4(pm[0], pm[1], pm[2], pm[3]); dm[1] = make_float4(pm[4], pm[5], pm[6], pm[7]);
-        dq[0] = make_float4(pq[0], pq[1], pq[2], pq[3]); dq[1] = make_float4(pq[4], pq[5], pq[6], pq[7]);
+        *reinterpret_cast<float4*>(s_pm + k16 * 128 + p4 * 4) = make_float4(pm[0], pm[1], pm[2], pm[3]);
+        *reinterpret_cast<float4*>(s_pq + k16 * 128 + p4 * 4) = make_float4(pq[0], pq[1], pq[2], pq[3]);
       }
       mbar_arrive(&nsync[0]);
       const bool met0 = mbar_wait(&nsync[0], i & 1, g.err, 25);
       if (!__all_sync(0xffffffffu, met0)) break;
       if (tid < 128) {
-        // thread = pixel: combine the sixteen partials (equal counts): M2 = sum M2_k + 8 sum (mean_k - mean)^2
-        float m = 0.f, m2 = 0.f;
+        // thread = pixel: combine the eight partials (equal counts): M2 = sum M2_k + 16 sum (mean_k - mean)^2
+        float pm[8], m = 0.f, m2 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) { m += s_pm[k * 128 + tid]; m2 += s_pq[k * 128 + tid]; }
-        m *= (1.0f / 16);
+        for (int k = 0; k < 8; ++k) { pm[k] = s_pm[k * 128 + tid]; m += pm[k]; m2 += s_pq[k * 128 + tid]; }
+        m *= (1.0f / 8);
         float dev = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) { const float d = s_pm[k * 128 + tid] - m; dev = fmaf(d, d, dev); }
+        for (int k = 0; k < 8; ++k) dev = fmaf(pm[k] - m, pm[k] - m, dev);
         const long long px = (long long)tile * 128 + tid;
-        const float rs = pixel_rstd((m2 + 8.f * dev) * (1.0f / 128), g.eps, px, g.n, g.pitch);
+        const float rs = pixel_rstd((m2 + 16.f * dev) * (1.0f / 128), g.eps, px, g.n, g.pitch);
         s_mean[tid] = m;
         s_rstd[tid] = rs;
         if (px < g.M) { g.mean[px] = m; g.rstd[px] = rs; }
@@ -681,7 +681,7 @@ int launch_out(cudaStream_t st, const LnGateOut& p) {
   OutArgs a;
   a.M = p.M; a.tiles = (int)((p.M + 127) / 128); a.eps = p.eps; a.gamma = p.gamma; a.beta = p.beta;
   a.bias = p.bias_out; a.u_cm = p.u_cm; a.mean = p.mean; a.rstd = p.rstd; a.out = p.out; a.residual = p.residual; a.n = p.n; a.pitch = p.pitch; a.own_pitch = p.own_pitch; a.err = p.err;
-  constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 16 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
+  constexpr size_t smem = 1024 + kOWBytes + kOBufs * kOTile + (2 * 8 * 128 + 4 * 128) * sizeof(float) + (1 + 3 * kOBufs + 6) * 8 + 16;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kern = ln_gate_out_kernel<T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -308,3 +308,40 @@ def test_unasked_sums_are_not_formed(tmu):
         flops[frozen] = _lib.profile_summary()["tc_gate_in_bwd"][2]
         _lib.profile_enable(False)
     assert flops[False] > 0 and flops[True] == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=str)
+@pytest.mark.parametrize("n", [8, 64, 72, 200])
+def test_layernorm_sums_keep_their_order(n, dtype):
+    """The means of both LayerNorms, bit for bit: a row's even and odd pairs of channels as two chains of additions; parts of 16 channels of
+    the contraction.  Another order flips last bits of z and u, which a stack in 16 bits carries on."""
+    import ctypes
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle._trimul import _DTYPES
+    lib, M = _lib.load(), n * n
+    x, mask, w, _ = util.trimul_inputs(1, n, 128, 128, dtype, seed=n)
+    d = _lib.TriMulDesc(1, n, 128, 128, _DTYPES[dtype], _lib.PREC_IEEE, _lib.OUTGOING, 1e-5)
+    wp = _lib.TriMulWeights(**{_lib.abi_field(k): t.data_ptr() for k, t in w.items()})
+    saved = torch.empty(lib.tri_mul_saved_bytes(ctypes.byref(d)), dtype=torch.uint8, device="cuda")
+    ws = torch.empty(lib.tri_mul_ws_bytes(ctypes.byref(d), 0), dtype=torch.uint8, device="cuda")
+    out, at = torch.empty_like(x), lambda t: ctypes.c_void_p(t.data_ptr())
+    _lib.check(lib.tri_mul_fwd(ctypes.byref(d), at(x), at(mask), ctypes.byref(wp), at(out), at(saved), at(ws), ws.numel(),
+                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "fwd")
+    saved = saved.cpu()
+    unit, room = -(-M * 256 // 256) * 256, -(-M * 4 // 256) * 256   # z, a, b, t, u; then mean, rstd of either LayerNorm
+    floats = lambda i: saved[5 * unit + i * room:][:M * 4].view(torch.float32)  # noqa: E731
+    rows = x.reshape(M, 64, 2).cpu().float()
+    k = rows[:, 0, 0]
+    chain = [torch.zeros(M, 2), torch.zeros(M, 2)]
+    for i in range(64):
+        chain[i & 1] = chain[i & 1] + (rows[:, i] - k[:, None])
+    s = [c[:, 0] + c[:, 1] for c in chain]
+    assert torch.equal(floats(0), (s[0] + s[1]) / 128 + k)
+    t = saved[3 * unit:][:M * 256].view(dtype).reshape(8, 16, M).float()
+    mean = torch.zeros(M)
+    for part in t:
+        s = torch.zeros(M)
+        for c in part:
+            s = s + (c - part[0])
+        mean = mean + (s / 16 + part[0])
+    assert torch.equal(floats(2), mean / 8)
