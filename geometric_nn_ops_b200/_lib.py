@@ -176,7 +176,7 @@ def check(code: int, what: str) -> None:
 
 
 def check_device_status(ws, stream) -> None:
-    """With TRI_B200_CHECK=1, read back the tensor-core kernels' status word (synchronises the stream)."""
+    """With TRI_B200_CHECK=1, read back the tensor-core kernels' status (synchronises the stream)."""
     if os.environ.get("TRI_B200_CHECK") == "1" and last_path() == "tcgen05":
         check(load().tri_ws_status(ctypes.c_void_p(ws.data_ptr()), stream), "device status")
 

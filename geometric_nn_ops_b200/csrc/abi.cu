@@ -551,9 +551,16 @@ int tri_peer_barrier(const TriPeerSignal* sig, int64_t limit_cycles, tri_stream_
 
 int tri_ws_status(const void* ws, tri_stream_t stream) {
   if (ws == nullptr) return fail(TRI_ERR_ARG, "ws is null");
-  int code = 0;
-  TRI_CUDA_OK(cudaMemcpyAsync(&code, ws, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  int head[2] = {0, 0};
+  TRI_CUDA_OK(cudaMemcpyAsync(head, ws, sizeof(head), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   TRI_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+  int code = head[0];
+  unsigned char own[tc::kStatusCtas];
+  if (code == 0 && head[1] > 0 && head[1] <= tc::kStatusCtas) {   // (see leave_status)
+    TRI_CUDA_OK(cudaMemcpyAsync(own, static_cast<const char*>(ws) + 8, head[1], cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    TRI_CUDA_OK(cudaStreamSynchronize((cudaStream_t)stream));
+    for (int i = 0; i < head[1] && code == 0; ++i) code = own[i];
+  }
   if (code != 0) return fail(TRI_ERR_DEVICE, "a tensor-core kernel gave up waiting (code %d)", code);
   return 0;
 }

@@ -42,7 +42,7 @@ struct AttnArgs {
   int64_t mask_st[2];
   int bias_b_mul;        // 0 when the bias is broadcast over the batch
   uint32_t idesc_s, idesc_pv;
-  int* err;
+  int* status;
 };
 
 template <int HD> struct Geo {
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) mask_terms_kernel(const uint8_t* __restri
                                                          float* __restrict__ out, int* err) {
   dependent_trigger();
   const long long idx = blockIdx.x * 256LL + threadIdx.x;
-  if (idx == 0) *err = 0;
+  if (idx == 0) err[0] = err[1] = 0;
   if (idx >= (long long)B * S * npad) return;
   const int k = (int)(idx % npad);
   const long long bs = idx / npad, b = bs / S, s = bs - b * S;
@@ -109,6 +109,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                                     // two tiles, so two tiles that share a barrier are never both pending)
   uint64_t* bar_p = bar_q + 14;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_q + 15);
+  int* const err = reinterpret_cast<int*>(tmem_slot + 1);   // this CTA's (see leave_status)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid & 127, hh = (tid >> 7) & 1;
   const int qblocks = (a.N + 127) / 128;
@@ -136,7 +137,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(bar_s, 1); mbar_init(bar_p, 8);
     for (int i = 0; i < 4; ++i) mbar_init(&bar_free[i], 8);
     mbar_fence_init();
-    *a.err = 0;   // (by every CTA: its waits read the word.  One that gives up does so two seconds after all have started)
+    *err = 0;
   }
   if (warp == 0) tmem_alloc(tmem_slot, 256);
   tc_fence_before_sync();
@@ -211,7 +212,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     int jt = 0, n_cur = 0;   // key tile and item of stream position c
     for (int c = 0; c < total && ok; ++c) {
       if (c + 2 < total) fetch_mask(la, la_t);
-      ok = __all_sync(0xffffffffu, mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16));   // S(c) has been read: its K stage and mask terms are free
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar_free[c & 3], (c >> 2) & 1, err, 16));   // S(c) has been read: its K stage and mask terms are free
       if (++jt == nt) {                                    // ... and it was the item's last use of Q
         jt = 0;
         if (++n_cur < my_items) load_q(n_cur);
@@ -219,7 +220,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (c + 2 < total) {
         load_k(c + 2, la, la_t);
         if (HB && TMEM_P) load_bias(c + 2, la, la_t);      // the bias tile has been read too and P does not replace it
-        ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, a.err, 15)) && ok;   // P V(c) done: its V stage and P buffer are free
+        ok = __all_sync(0xffffffffu, mbar_wait(&bar_pv[c & 1], (c >> 1) & 1, err, 15)) && ok;   // P V(c) done: its V stage and P buffer are free
         if (HB && !TMEM_P) load_bias(c + 2, la, la_t);
         load_v(c + 2, la, la_t);
         advance();
@@ -234,9 +235,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t p_lo = desc_lo(smem_u32(sP), 16), vmn_lo = desc_lo(smem_u32(sV), 128 * G::RB);   // V as [n = d, k = key]
       int s_t = 0, s_n = 0;   // key tile and item of the next S product
       auto issue_s = [&](int c) {
-        if (s_t == 0) ok = mbar_wait(bar_q, s_n & 1, a.err, 11) && ok;   // first tile of an item: its Q
+        if (s_t == 0) ok = mbar_wait(bar_q, s_n & 1, err, 11) && ok;   // first tile of an item: its Q
         if (++s_t == nt) { s_t = 0; ++s_n; }
-        ok = mbar_wait(&bar_k[c & 1], (c >> 1) & 1, a.err, 12) && ok;
+        ok = mbar_wait(&bar_k[c & 1], (c >> 1) & 1, err, 12) && ok;
         tc_fence_after_sync();
         const uint32_t so = (c & 1) * (G::TILE >> 4);
 #pragma unroll
@@ -248,10 +249,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       int j = 0;
       for (int c = 0; c < total && ok; ++c, j = (j + 1 == nt ? 0 : j + 1)) {
         const int stg = c & 1;
-        ok = mbar_wait(&bar_free[c & 3], (c >> 2) & 1, a.err, 16) && ok;   // logits of tile c are in registers
+        ok = mbar_wait(&bar_free[c & 3], (c >> 2) & 1, err, 16) && ok;   // logits of tile c are in registers
         if (c + 1 < total) issue_s(c + 1);
-        ok = mbar_wait(bar_p, c & 1, a.err, 17) && ok;
-        ok = mbar_wait(&bar_v[stg], (c >> 1) & 1, a.err, 18) && ok;
+        ok = mbar_wait(bar_p, c & 1, err, 17) && ok;
+        ok = mbar_wait(&bar_v[stg], (c >> 1) & 1, err, 18) && ok;
         tc_fence_after_sync();
         const uint32_t so = stg * (G::TILE >> 4), po = stg * (32768 >> 4);
 #pragma unroll
@@ -273,10 +274,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       float m_run = -INFINITY, l_run = 0.f;
       for (int j = 0; j < nt; ++j) {
         const int c = n * nt + j, stg = c & 1;
-        ok = mbar_wait(bar_s, c & 1, a.err, 13) && ok;
+        ok = mbar_wait(bar_s, c & 1, err, 13) && ok;
         tc_fence_after_sync();
-        ok = mbar_wait(&bar_k[stg], (c >> 1) & 1, a.err, 12) && ok;   // the tile's mask terms
-        if (HB) ok = mbar_wait(&bar_bias[stg], (c >> 1) & 1, a.err, 14) && ok;
+        ok = mbar_wait(&bar_k[stg], (c >> 1) & 1, err, 12) && ok;   // the tile's mask terms
+        if (HB) ok = mbar_wait(&bar_bias[stg], (c >> 1) & 1, err, 14) && ok;
         const uint32_t sPj = smem_u32(sP) + stg * 32768;   // holds the bias tile; with P in shared memory, P when this step is done
 
         // ---- logits of this thread's 64 keys into registers, their maximum ----------------------------
@@ -314,7 +315,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const bool grow = mx > m_run + kRescale;          // (always true on the first tile with a key in range)
         const float m_new = grow ? mx : m_run;
         if (j > 0 && __any_sync(0xffffffffu, grow)) {     // tcgen05.ld / st are warp-wide: rows that keep their maximum scale by 1
-          ok = mbar_wait(&bar_pv[(c - 1) & 1], ((c - 1) >> 1) & 1, a.err, 15) && ok;   // O is current
+          ok = mbar_wait(&bar_pv[(c - 1) & 1], ((c - 1) >> 1) & 1, err, 15) && ok;   // O is current
           tc_fence_after_sync();
           const float alpha = grow ? ex2_approx((m_run - m_new) * kLog2e) : 1.0f;   // m_run = -inf gives 0 (O_hh is 0 then)
           l_run *= alpha;
@@ -349,7 +350,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         l_run += (ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y);
         if constexpr (TMEM_P) {
-          if (c > 0) ok = mbar_wait(&bar_pv[(c - 1) & 1], ((c - 1) >> 1) & 1, a.err, 15) && ok;   // the previous P has been read
+          if (c > 0) ok = mbar_wait(&bar_pv[(c - 1) & 1], ((c - 1) >> 1) & 1, err, 15) && ok;   // the previous P has been read
           tc_fence_after_sync();
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {   // this thread's query row, its 64 keys as 32 packed columns
@@ -374,7 +375,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       // The next item's first P V, which overwrites O, is issued only after every warp has arrived on bar_p
       // for that tile, hence after this.
       const int cl = n * nt + nt - 1;
-      ok = mbar_wait(&bar_pv[cl & 1], (cl >> 1) & 1, a.err, 15) && ok;
+      ok = mbar_wait(&bar_pv[cl & 1], (cl >> 1) & 1, err, 15) && ok;
       tc_fence_after_sync();
       if (hh == 1) { sX[2 * r] = m_run; sX[2 * r + 1] = l_run; }
       named_barrier(1, 256);
@@ -421,6 +422,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 256);
   }
+  if (tid == 0) leave_status(a.status, err);
 }
 
 // =================================================================================================
@@ -1411,7 +1413,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 3) attn_prepare_kernel(const TriAttnDesc d, const T* o, const T* d_o, const PrepareArgs a) {
   __shared__ uint16_t tile[64][66];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = d.n_res;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.err[0] = a.err[1] = 0;
   if ((int)blockIdx.x < a.transposes) {
     unsigned z = blockIdx.x;
     const int k0 = (int)(z % (unsigned)a.tiles) * 64; z /= (unsigned)a.tiles;
@@ -1739,7 +1741,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   const int kind = d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   a.idesc_s = make_idesc(kind, 128, 128, false, false);
   a.idesc_pv = make_idesc(kind, 128, HD, false, true);
-  a.err = err;
+  a.status = err;
   const bool own = bias == nullptr || bias_fits_tma(d, bias);   // (else a copy with padded rows is the first kernel)
   if (!own) TRI_TRY(launch_pad_bias(d, bias, bias_c, st));
   if (bias != nullptr) TRI_TRY(bias_map(&tb, bias, own ? nullptr : bias_c, d, 128));
@@ -1760,7 +1762,7 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto kern = bias != nullptr ? attn_fwd_tc_kernel<T, HD, true> : attn_fwd_tc_kernel<T, HD, false>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<HD>::SMEM));
-  launch_dependent(own ? kLaunchPlainly : us_of_logits(pairs), kern, (unsigned)std::min<long long>(blocks, 2LL * sm_count()), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
+  launch_dependent(own ? kLaunchPlainly : us_of_logits(pairs), kern, (unsigned)std::min<long long>({blocks, 2LL * sm_count(), kStatusCtas}), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
   TRI_LAUNCH_OK();
   return 0;
 }
@@ -1835,8 +1837,8 @@ bool attn_bwd_supported(const TriAttnDesc* d) {
 
 // everything but the padded copy of the bias, which comes last
 static size_t attn_ws_base(const TriAttnDesc* d, int is_bwd) {
-  // (the status word, the key-mask terms)
-  if (!is_bwd) return 512 + (wants_mask_terms(d) ? align_up((size_t)d->B * d->n_seq * ((d->n_res + 127) / 128 * 128) * sizeof(float)) : 0);
+  // (the status, the key-mask terms)
+  if (!is_bwd) return 8 + kStatusCtas + (wants_mask_terms(d) ? align_up((size_t)d->B * d->n_seq * ((d->n_res + 127) / 128 * 128) * sizeof(float)) : 0);
   Arena a(nullptr, 0);
   BwdWs w;
   carve_bwd(a, d, &w);
@@ -1857,7 +1859,7 @@ int attn_forward(const TriAttnDesc* d, const void* q, const void* k, const void*
                  const uint8_t* mask, void* o, float* lse, void* ws, size_t ws_size, cudaStream_t st) {
   if (ws == nullptr || ws_size < attn_ws_bytes(d, 0)) return fail(TRI_ERR_WORKSPACE, "attention forward workspace too small");
   int* err = static_cast<int*>(ws);
-  float* mt = reinterpret_cast<float*>(static_cast<char*>(ws) + 512);
+  float* mt = reinterpret_cast<float*>(static_cast<char*>(ws) + 8 + kStatusCtas);
   void* bc = static_cast<char*>(ws) + attn_ws_base(d, 0);
   if (d->dtype == TRI_BF16) {
     if (d->D <= 32) return fwd_launch<__nv_bfloat16, 32>(d, q, k, v, bias, mask, o, lse, err, mt, bc, st);

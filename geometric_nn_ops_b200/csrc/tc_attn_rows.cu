@@ -57,6 +57,7 @@ template <typename T> struct RowsCfg {
   static constexpr int OFF_V = OFF_K + kGroups * 3 * TK;        // [group][3]
   static constexpr int OFF_M = OFF_V + kGroups * 3 * TK;        // [bias stage][group] x 64 mask terms
   static constexpr int OFF_BAR = OFF_M + kBiasStages * kGroups * 256;
+  static constexpr int OFF_ERR = OFF_BAR + 1020;          // this CTA's status
   static constexpr int SMEM = OFF_BAR + 1024 + 1024;
   static constexpr int PC = F32 ? 64 : 32;         // columns of P: a step's 64 keys
   static constexpr int KS = F32 ? 4 : 2;           // products of a step's S: 32 channels, 32 bytes each
@@ -79,7 +80,7 @@ struct RowsArgs {
   int bias_b_mul;
   int rows_per_item;         // groups in use (fewer where a triple per CTA would leave SMs idle)
   uint32_t idesc_s, idesc_pv;
-  int* err;
+  int* status;
   const uint8_t* mask;       // [B][S][N], or null
   int64_t mask_st[2];
 };
@@ -114,6 +115,9 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* b_full = reinterpret_cast<uint64_t*>(bars + kGroups);   // [kBiasStages]
   uint64_t* b_free = b_full + kBiasStages;                          // [kBiasStages]: the softmax warps of the groups in use
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(b_free + kBiasStages);
+  // Without TERMS no kernel has cleared the call's status: see leave_status.  (Formed where it is used: as a variable 41.1 us in place
+  // of 40.8 at N = 256.)
+  auto err = [&]() { return TERMS ? a.status : reinterpret_cast<int*>(smem + M::OFF_ERR); };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qblocks = (a.N + 127) / 128, nk = (a.N + 63) / 64;
@@ -139,6 +143,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], TERMS ? 1 : 2); mbar_init(&b_free[i], 4 * R); }
     mbar_fence_init();
+    if (!TERMS) *err() = 0;
   }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
@@ -169,7 +174,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int n = 0; n < my_items && ok; ++n) {
           const Item it = item_of(n);
           for (int j = 0; j < nk; ++j) {
-            ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51);
+            ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, err(), 51);
             if (!ok) break;
             const int rows = min(R, a.S - it.s0);
             mbar_expect_tx(&b_full[stg], (HB ? M::TB : 0) + rows * 256);
@@ -186,7 +191,6 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // their mask bytes are fetched a step ahead, as three aligned words of which the funnel shift takes the eight bytes.  The
       // softmax warps of the sub-partition miss the instructions: N = 768 took 761 us so and 729 with terms made before, launch
       // included; N = 256 42.3 and 42.9.
-      if (lane == 0) *a.err = 0;   // (by every CTA: its waits read the word.  One that gives up does so two seconds after all have started)
       dependent_wait();
       int stg = 0;
       uint32_t ph = 0, w[3] = {};
@@ -212,7 +216,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int n = 0; n < my_items && ok; ++n) {
         const Item after = item_of(n + 1 < my_items ? n + 1 : n);
         for (int j = 0; j < nk; ++j) {
-          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_free[stg], ph ^ 1, a.err, 51));   // (the warp gives up together)
+          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_free[stg], ph ^ 1, err(), 51));   // (the warp gives up together)
           if (!ok) break;
           if (lane == 0) {
             mbar_expect_tx(&b_full[stg], HB ? M::TB : 0);
@@ -299,7 +303,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int c = 0; c < 2 && c < total; ++c) load(&gb.first[c], true, false);
       if (total > 0) load(&gb.in[0], total > 2, true);
       for (int c = 0; c < 2 && c < total; ++c) {
-        ok = mbar_wait(&gb.first[c], 0, a.err, 52) && ok;
+        ok = mbar_wait(&gb.first[c], 0, err(), 52) && ok;
         tc_fence_after_sync();
         issue_s(t0 + c * 64);
         if (leader) umma_commit(&gb.mma[c]);
@@ -309,10 +313,10 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int c = 0; c < total && ok; ++c) {
         const bool more = c + 2 < total;
         const uint32_t v_at = v_lo + stg * (M::TK >> 4), tp = t0 + (c & 1) * 64, first = j > 0 ? 1u : 0u;
-        ok = mbar_wait_relaxed(&gb.in[stg], ph, a.err, 53) && ok;
+        ok = mbar_wait_relaxed(&gb.in[stg], ph, err(), 53) && ok;
         // every warp has stored P(c): it had waited for S(c), which followed P V(c - 2): the K stage of c and the V stage
         // of c - 2 are free
-        ok = mbar_wait_relaxed(&gb.p_ready[c & 1], (c >> 1) & 1, a.err, 55) && ok;
+        ok = mbar_wait_relaxed(&gb.p_ready[c & 1], (c >> 1) & 1, err(), 55) && ok;
         tc_fence_after_sync();
         if (leader) {
 #pragma unroll
@@ -350,7 +354,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     int po = -1, pstat = 0;   // O row in 16-byte pieces, -1 where the query is beyond N; row of the statistics
     // O and the statistics of the row, once P V of its last step `cl` is done; no later P V can have been issued yet
     auto finish = [&](int cl) {
-      if (!mbar_wait(&gb.mma[cl & 1], ((cl >> 1) + 1) & 1, a.err, 59)) ok = false;
+      if (!mbar_wait(&gb.mma[cl & 1], ((cl >> 1) + 1) & 1, err(), 59)) ok = false;
       tc_fence_after_sync();
       uint32_t o[2][16];
       tmem_ld_32x16(t_row + COL_O, o[0]);
@@ -384,7 +388,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const Item it = item_of(n);
       if (it.s0 + g >= a.S) {   // no row for this group: let the bias tiles pass
         for (int j = 0; j < nk && ok; ++j) {
-          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_full[bstg], bph, a.err, 57));
+          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_full[bstg], bph, err(), 57));
           if (lane == 0) mbar_arrive(&b_free[bstg]);
           if (++bstg == kBiasStages) { bstg = 0; bph ^= 1; }
         }
@@ -395,8 +399,8 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       float seen = 0.f;               // largest sum of a step against this reference
       bool by_diff = false;           // P from differences (the same for the whole warp)
       for (int j = 0; j < nk; ++j, ++c) {
-        if (!early_s && !mbar_wait(&gb.mma[c & 1], (c >> 1) & 1, a.err, 58)) ok = false;
-        if (!early_b && !mbar_wait(&b_full[bstg], bph, a.err, 57)) ok = false;
+        if (!early_s && !mbar_wait(&gb.mma[c & 1], (c >> 1) & 1, err(), 58)) ok = false;
+        if (!early_b && !mbar_wait(&b_full[bstg], bph, err(), 57)) ok = false;
         tc_fence_after_sync();
         const uint32_t mrow = mask_s + bstg * (kGroups * 256), brow = bias_row + bstg * M::TB, t_s = t_row + (c & 1) * 64;
         auto logits = [&](const uint32_t (&cur)[16], int q, float2 (&x)[8]) {
@@ -494,7 +498,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // (fp32: the rest of P has one buffer, and P V of the step before reads it; its commit is the next step's S)
         if (M::F32 && c > 0) {
           if (!early_s) {
-            early_s = mbar_wait(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1, a.err, 58);
+            early_s = mbar_wait(&gb.mma[(c + 1) & 1], ((c + 1) >> 1) & 1, err(), 58);
             ok = early_s && ok;
           }
           tc_fence_after_sync();
@@ -528,7 +532,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           m = top;
           l *= alpha;
           if (j > 0) {
-            ok = mbar_wait(&gb.mma[(c - 1) & 1], (((c - 1) >> 1) + 1) & 1, a.err, 59) && ok;
+            ok = mbar_wait(&gb.mma[(c - 1) & 1], (((c - 1) >> 1) + 1) & 1, err(), 59) && ok;
             tc_fence_after_sync();
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
@@ -582,6 +586,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
+  if (!TERMS && tid == 0) leave_status(a.status, err());
 }
 
 }  // namespace
@@ -602,7 +607,7 @@ int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap
   a.stats = stats; a.mask = mask; a.mask_st[0] = d->mask_st[0]; a.mask_st[1] = d->mask_st[1];
   a.mask_terms = mask_terms; a.npad = (d->n_res + 127) / 128 * 128;
   a.bias_b_mul = bias_batched ? 1 : 0;
-  a.err = err;
+  a.status = err;
   const int kind = d->dtype == TRI_F32 ? KIND_TF32 : d->dtype == TRI_BF16 ? KIND_BF16 : KIND_F16;
   a.idesc_s = make_idesc(kind, 128, 64, false, false);
   a.idesc_pv = make_idesc(kind, 128, 32, false, true);

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256, 2) prepare_bwd_kernel(const TriAttnDesc d
   __shared__ float tile[32][33];
   dependent_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = d.n_res;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.err[0] = a.err[1] = 0;
   if ((int)blockIdx.x < a.transposes) {
     unsigned z = blockIdx.x;
     const int k0 = (int)(z % (unsigned)a.tiles) * 32; z /= (unsigned)a.tiles;

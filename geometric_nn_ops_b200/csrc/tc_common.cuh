@@ -1,7 +1,7 @@
 // Blackwell (sm_100a) building blocks: mbarrier, TMA (cp.async.bulk.tensor), TMEM allocation,
 // tcgen05.mma / commit / ld, and the shared-memory and instruction descriptors they take.
 //
-// Every wait here is BOUNDED: after a limit (kWaitLimitCycles) the waiter records a code in a device error
+// Every wait here is BOUNDED: after a limit (kWaitLimitCycles) the waiter records a code in an error
 // word and returns, so a protocol bug shows up as TRI_ERR_DEVICE instead of a hung GPU.
 #pragma once
 
@@ -13,7 +13,23 @@ namespace tri {
 namespace tc {
 
 // ---------------------------------------------------------------------------------------------
-// device error word (one per launch, zeroed by the host before the launch)
+// status block, at the start of a workspace
+// ---------------------------------------------------------------------------------------------
+// Word 0: the code of the first wait of the call's kernels that ran out, or 0.  It is cleared in stream order before the first kernel
+// that may report there starts to wait: by a small kernel that comes first in any case, or by a memset.  Word 1: how many CTAs of the
+// call's first kernel have a byte of their own from byte 8 on.  A kernel that starts a call by itself reports so: its CTAs keep their
+// codes in shared memory and write their bytes as they end (`leave_status`), so that neither a CTA that starts late nor what the
+// workspace held before can be taken for a report, or hide one.
+constexpr int kStatusCtas = 504;   // at most: 512 bytes (148 CTAs: 256)
+
+// one thread, after the block's last barrier
+__device__ __forceinline__ void leave_status(int* status, const int* code) {
+  reinterpret_cast<uint8_t*>(status)[8 + blockIdx.x] = (uint8_t)*code;   // (codes are below 256)
+  if (blockIdx.x == 0) { status[0] = 0; status[1] = (int)gridDim.x; }
+}
+
+// ---------------------------------------------------------------------------------------------
+// bounded waits
 // ---------------------------------------------------------------------------------------------
 // A try_wait suspends the thread in hardware for a moment and is repeated in a loop of three instructions: with the loop
 // in C (a counter, the error word, a hint of a long suspension that put the warp to sleep past the arrival) the waiting

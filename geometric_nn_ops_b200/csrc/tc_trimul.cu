@@ -72,7 +72,7 @@ __global__ void prep_weights_kernel(const T* wp, const T* wg, const T* bp, const
                                     T* wcat, float* bias_cat, float* bias_out, int* err) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx == 0) {
-    *err = 0;   // the error word of the launches that follow
+    err[0] = err[1] = 0;   // the status of the launches that follow
     __threadfence();
   }
   dependent_trigger();

@@ -67,7 +67,7 @@ void bind(const std::string& path) {
 void ok(int code, const char* what) {
   TORCH_CHECK(code == 0, what, " failed with code ", code, ": ", api.last_error());
 }
-// with TRI_B200_CHECK=1, read back the tensor-core kernels' status word (synchronises the stream)
+// with TRI_B200_CHECK=1, read back the tensor-core kernels' status (synchronises the stream)
 void check_device(const Tensor& ws, cudaStream_t st) {
   const char* e = std::getenv("TRI_B200_CHECK");
   if (e != nullptr && std::strcmp(e, "1") == 0 && std::strcmp(api.last_path(), "tcgen05") == 0)

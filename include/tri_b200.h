@@ -151,7 +151,7 @@ int tri_attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w /
                      tri_stream_t stream);
 
 /* The same LayerNorm and the pair bias alone, for up to 16 heads (bf16 / fp16; d->D is not read).  `plane`: pixels of
- * one batch entry (it divides M); bias: [M / plane, H, plane].  ws: 256 bytes of device memory (the status word). */
+ * one batch entry (it divides M); bias: [M / plane, H, plane].  ws: 256 bytes of device memory (the status). */
 int tri_attn_project_bias(const TriAttnProjDesc* d, int64_t plane, const void* z, const void* ln_w /*nullable*/,
                           const void* ln_b /*nullable*/, const void* w_bias, void* bias, void* ws, tri_stream_t stream);
 
@@ -356,9 +356,10 @@ typedef struct TriPeerSignal {
 
 int tri_peer_barrier(const TriPeerSignal* sig, int64_t limit_cycles, tri_stream_t stream);
 
-/* The tensor-core kernels bound every wait; if one runs out, the kernel records a code in the first
- * word of the workspace it was given and drains instead of hanging.  This call copies that word back
- * (it synchronises the stream) and returns it: 0 = no failure. */
+/* The tensor-core kernels bound every wait; if one runs out, the kernel records a code at the start
+ * of the workspace it was given (its first word, or a byte per thread block in its first 512 bytes)
+ * and drains instead of hanging.  This call copies that back (it synchronises the stream): 0 = no
+ * failure, TRI_ERR_DEVICE with the first code in tri_last_error() otherwise. */
 int tri_ws_status(const void* ws, tri_stream_t stream);
 
 #ifdef __cplusplus
