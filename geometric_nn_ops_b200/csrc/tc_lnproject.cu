@@ -38,7 +38,7 @@ struct Args {
   const void* gamma;
   const void* beta;
   void* bias;
-  int* err;
+  int* status;
 };
 
 __device__ __forceinline__ void next_stage(int& b, uint32_t& phase, int stages) {
@@ -65,6 +65,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
   uint64_t* tfull = zempty + kMaxStages;    // [4] block complete (3: heads)
   uint64_t* tempty = tfull + 4;             // [4] block read (8 warps; heads: 4)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 4);
+  int* const err = reinterpret_cast<int*>(tmem_slot + 1);   // this CTA's (see leave_status)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -72,7 +73,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     for (int b = 0; b < g.stages; ++b) { mbar_init(&zfull[b], 1); mbar_init(&znorm[b], 8); mbar_init(&zempty[b], 1); }
     for (int b = 0; b < 4; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], b < 3 ? 8 : 4); }
     mbar_fence_init();
-    if (blockIdx.x == 0) *g.err = 0;        // a wait gives up seconds after this
+    *err = 0;
   }
   if (threadIdx.x < 128) {
     s_gamma[threadIdx.x] = g.gamma ? reinterpret_cast<const T*>(g.gamma)[threadIdx.x] : from_f32<T>(1.f);
@@ -95,7 +96,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
       int b = 0;
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, next_stage(b, ph, g.stages)) {
-        if (!mbar_wait(&zempty[b], ph ^ 1, g.err, 70)) break;
+        if (!mbar_wait(&zempty[b], ph ^ 1, err, 70)) break;
         mbar_expect_tx(&zfull[b], kTile);
         for (int kb = 0; kb < 2; ++kb) tma_load_3d(sZ + b * kTile + kb * kSub, &tmZ, &zfull[b], kb * 64, tile * 128, 0);
       }
@@ -106,14 +107,14 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     if (elect_one()) {
       const uint32_t idesc = make_idesc(KIND, 128, 128, false, false), idesc_h = make_idesc(KIND, 128, kHeads, false, false);
       const uint32_t z_base = smem_u32(sZ), w_base = smem_u32(sW), h_base = smem_u32(sH);
-      bool ok = mbar_wait(wfull, 0, g.err, 71);
+      bool ok = mbar_wait(wfull, 0, err, 71);
       int i = 0, b = 0;
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, ++i, next_stage(b, ph, g.stages)) {
-        if (!mbar_wait(&znorm[b], ph, g.err, 72)) break;
+        if (!mbar_wait(&znorm[b], ph, err, 72)) break;
         for (int n = 0; n <= g.blocks && ok; ++n) {
           const int blk = n < g.blocks ? n : 3;
-          if (!mbar_wait(&tempty[blk], (i & 1) ^ 1, g.err, 73)) { ok = false; break; }
+          if (!mbar_wait(&tempty[blk], (i & 1) ^ 1, err, 73)) { ok = false; break; }
           tc_fence_after_sync();
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
@@ -143,7 +144,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     int b = 0;
     uint32_t ph = 0;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, next_stage(b, ph, g.stages)) {
-      const bool landed = mbar_wait(&zfull[b], ph, g.err, 74);
+      const bool landed = mbar_wait(&zfull[b], ph, err, 74);
       if (!__all_sync(0xffffffffu, landed)) break;
       const uint32_t rowp = smem_u32(sZ + b * kTile + half * kSub + r * 128);
       auto unpack = [](const uint4& w, float2 (&v)[4]) {
@@ -205,7 +206,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     bool ok = true;
     for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++i) {
       for (int blk = 0; blk < g.blocks; ++blk) {
-        ok = mbar_wait(&tfull[blk], i & 1, g.err, 75) && ok;
+        ok = mbar_wait(&tfull[blk], i & 1, err, 75) && ok;
         tc_fence_after_sync();
         uint32_t w[32];
 #pragma unroll
@@ -232,7 +233,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         }
       }
       if (part == 0) {
-        ok = mbar_wait(&tfull[3], i & 1, g.err, 76) && ok;
+        ok = mbar_wait(&tfull[3], i & 1, err, 76) && ok;
         tc_fence_after_sync();
         uint32_t v[16];
         tmem_ld_32x16(t_row + kHCol, v);
@@ -258,6 +259,7 @@ ln_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
+  if (threadIdx.x == 0) leave_status(g.status, err);
 }
 
 template <typename T>
@@ -273,7 +275,7 @@ int launch(cudaStream_t st, const LnProject& p) {
   tw = to = tz;
   Args a;
   a.M = p.M; a.tiles = cdiv(p.M, 128); a.blocks = cdiv(p.n_out, 128); a.heads = p.heads; a.plane = p.plane; a.eps = p.eps;
-  a.gamma = p.gamma; a.beta = p.beta; a.bias = p.bias; a.err = p.err;
+  a.gamma = p.gamma; a.beta = p.beta; a.bias = p.bias; a.status = p.err;
   if (a.blocks > 0) {
     TRI_TRY(make_tmap_3d(&tw, p.w_qkv, 2, f16, wd, ws, box, false));
     TRI_TRY(make_tmap_3d(&to, p.qkv, 2, f16, od, os, box, false));

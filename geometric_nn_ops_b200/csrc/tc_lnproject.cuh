@@ -18,7 +18,7 @@ struct LnProject {
   const void* w_bias;        // [heads, 128]
   void* qkv;                 // [M, n_out]
   void* bias;                // [M / plane][heads][plane]
-  int* err;                  // device status word (cleared by the kernel)
+  int* err;                  // 256 bytes: the status (see leave_status)
 };
 
 bool ln_project_supported(int dtype, long long M, int n_out, int heads);

@@ -49,3 +49,19 @@ def test_attention_forward(S, n, H, dim, dtype, ctas):
                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "fwd")
     assert _lib.last_path() == "tcgen05" and torch.equal(o, want) and bool((ws[size:] == 0x5A).all())
     _reports(ws, ctas)
+
+
+@pytest.mark.parametrize("M,ctas", [(40 * 40, 13), (200 * 200, 148)])
+def test_pair_bias_projection(M, ctas):
+    """The first kernel of a call of attention_pair_bias, in the 256 bytes that it asks for."""
+    from geometric_nn_ops_b200 import _lib
+    g = torch.Generator().manual_seed(M)
+    z, w = torch.randn(M, 128, generator=g).bfloat16().cuda(), torch.randn(8, 128, generator=g).bfloat16().cuda()
+    bias = torch.empty(1, 8, M, dtype=torch.bfloat16, device="cuda")
+    d = _lib.TriAttnProjDesc(M, 128, 8, 32, _lib.BF16, _lib.PREC_IEEE, 1e-5)
+    ws = torch.full((512,), 0x5A, dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.load().tri_attn_project_bias(ctypes.byref(d), M, _p(z), None, None, _p(w), _p(bias), _p(ws),
+                                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "bias")
+    want = torch.nn.functional.layer_norm(z.double(), (128,)).bfloat16().double() @ w.double().T
+    assert float((bias[0].double().T - want).norm() / want.norm()) < 2.0 ** -8 and bool((ws[256:] == 0x5A).all())
+    _reports(ws, ctas)
