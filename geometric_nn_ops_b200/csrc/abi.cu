@@ -583,7 +583,7 @@ int tri_bgemm(const TriGemmDesc* d, const void* a, const void* b, void* c, void*
   p.M = d->M; p.N = d->N; p.K0 = d->K; p.batches = d->batch;
   p.out0 = c; p.ld_out = d->ldc; p.batch_out = d->batch_c;
   p.first = true;
-  p.name = "tc_bgemm";
+  p.name = "tc_bgemm"; p.pair_name = "tc_bgemm_pair";
   p.flops = 2.0 * d->batch * d->M * (double)d->N * d->K;
   const double es = d->dtype == TRI_F32 ? 4.0 : 2.0;
   p.bytes = d->batch * (es * ((double)d->M * d->K + (double)d->N * d->K) + (d->out_f32 ? 4.0 : es) * d->M * d->N);

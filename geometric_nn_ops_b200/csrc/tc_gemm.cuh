@@ -1038,6 +1038,7 @@ struct GemmPlan {
   int peer_world = 0, peer_rank = 0, peer_batches = 0;
   bool first = false;                // no kernel of this call came before: launched plainly
   const char* name = "tc_gemm";
+  const char* pair_name = nullptr;   // the timer's name for it on pairs of SMs (null: the same)
   double flops = 0, bytes = 0;
 };
 

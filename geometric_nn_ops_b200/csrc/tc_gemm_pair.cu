@@ -212,7 +212,7 @@ int start(cudaStream_t st, const CUtensorMap& ta, const CUtensorMap& tb, const P
   auto kern = tc_gemm_pair_kernel<T, T>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long total = (long long)a.batches * a.tiles_m * a.tiles_n;
-  KernelTimer kt(p.name, st, p.flops, p.bytes);
+  KernelTimer kt(p.pair_name != nullptr ? p.pair_name : p.name, st, p.flops, p.bytes);
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;

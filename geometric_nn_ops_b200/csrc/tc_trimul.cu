@@ -538,13 +538,14 @@ Operand plane_operand(const void* p, int n, int planes, bool mn) {
 
 // One N x N x N product per channel plane: out[p] = A[p] B[p]^T with the given operand majors.
 int contraction(cudaStream_t st, int dtype, int planes, int n, const void* a, bool a_mn, const void* b, bool b_mn,
-                void* out, int* err, const char* name) {
+                void* out, int* err, bool bwd) {
   GemmPlan p;
   p.a[0] = plane_operand(a, n, planes, a_mn);
   p.b[0] = plane_operand(b, n, planes, b_mn);
   p.M = n; p.N = n; p.K0 = n; p.batches = planes;
   p.out0 = out; p.ld_out = n; p.batch_out = (long long)n * n;
-  p.name = name;
+  p.name = bwd ? "tc_gemm_contract_bwd" : "tc_gemm_contract";
+  p.pair_name = bwd ? "tc_gemm_contract_bwd_pair" : "tc_gemm_contract_pair";
   p.flops = 2.0 * planes * n * (double)n * n;
   p.bytes = 3.0 * planes * (double)n * n * (dtype == TRI_F32 ? 4 : 2);
   return launch_gemm(st, dtype, EPI_STORE, n > 128 ? 256 : 128, false, p, err);
@@ -879,7 +880,7 @@ int forward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMul
   TRI_TRY(run_prep<T>(st, w, pr));
   TRI_TRY(phase_project<T>(st, gm, x, mask, w, pr, s.z, s.mean_in, s.rstd_in, s.a, s.b, nullptr, 0, 0, own_pitch));
   const bool incoming = d->direction == TRI_INCOMING;
-  TRI_TRY(contraction(st, d->dtype, d->B * CW, d->N, s.a, incoming, s.b, incoming, s.t, pr.err, "tc_gemm_contract"));
+  TRI_TRY(contraction(st, d->dtype, d->B * CW, d->N, s.a, incoming, s.b, incoming, s.t, pr.err, false));
   return phase_output<T>(st, gm, s.t, s.z, w, pr, s.u, s.mean_out, s.rstd_out, out, /*keep_u=*/saved != nullptr, residual, own_pitch);
 }
 
@@ -901,11 +902,11 @@ int backward_t(const TriMulDesc* d, const void* x, const void* mask, const TriMu
   // contraction backward: the same batched GEMM, only the operand majors change
   const int planes = d->B * CW, n = d->N, dt = d->dtype;
   if (d->direction == TRI_OUTGOING) {
-    TRI_TRY(contraction(st, dt, planes, n, b.dt, false, s.b, true, b.da, pr.err, "tc_gemm_contract_bwd"));  // da[i,k] = sum_j dt[i,j] b[j,k]
-    TRI_TRY(contraction(st, dt, planes, n, b.dt, true, s.a, true, b.db, pr.err, "tc_gemm_contract_bwd"));   // db[j,k] = sum_i dt[i,j] a[i,k]
+    TRI_TRY(contraction(st, dt, planes, n, b.dt, false, s.b, true, b.da, pr.err, true));  // da[i,k] = sum_j dt[i,j] b[j,k]
+    TRI_TRY(contraction(st, dt, planes, n, b.dt, true, s.a, true, b.db, pr.err, true));   // db[j,k] = sum_i dt[i,j] a[i,k]
   } else {
-    TRI_TRY(contraction(st, dt, planes, n, s.b, false, b.dt, false, b.da, pr.err, "tc_gemm_contract_bwd")); // da[k,i] = sum_j b[k,j] dt[i,j]
-    TRI_TRY(contraction(st, dt, planes, n, s.a, false, b.dt, true, b.db, pr.err, "tc_gemm_contract_bwd"));  // db[k,j] = sum_i a[k,i] dt[i,j]
+    TRI_TRY(contraction(st, dt, planes, n, s.b, false, b.dt, false, b.da, pr.err, true)); // da[k,i] = sum_j b[k,j] dt[i,j]
+    TRI_TRY(contraction(st, dt, planes, n, s.a, false, b.dt, true, b.db, pr.err, true));  // db[k,j] = sum_i a[k,i] dt[i,j]
   }
   return phase_project_bwd<T>(st, gm, x, mask, s.z, b.da, b.db, b.dgo, s.mean_in, s.rstd_in, w, pr, g, b.dpg, dx,
                               b.partial);

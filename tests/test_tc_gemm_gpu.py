@@ -31,3 +31,28 @@ def test_bgemm(case, dtype, a_mn, b_mn):
     got = bgemm(a_in, b_in, a_mn_major=a_mn, b_mn_major=b_mn, check=True)
     assert got.dtype == dtype
     assert torch.equal(got, got32.to(dtype))
+
+
+# whole tiles; an M that is no multiple of four, whose rows are stored one by one; rows of an odd length; one tile of 256 x 256 for 148 pairs
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=str)
+@pytest.mark.parametrize("case", [(40, 512, 512, 128), (40, 509, 512, 72), (40, 510, 511, 200), (148, 256, 256, 64)], ids=str)
+def test_pairs_of_sms(case, dtype, a_mn, b_mn):
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.gemm import bgemm
+    batch, M, N, K = case
+    if (a_mn and M % 8 != 0) or (b_mn and N % 8 != 0):
+        pytest.skip("rows of such operands start on 16-byte boundaries")
+    g = torch.Generator().manual_seed(M + N + K)
+    a = torch.randn(batch, M, K, generator=g).to(dtype).cuda()
+    b = torch.randn(batch, N, K, generator=g).to(dtype).cuda()
+    want = torch.matmul(a.double(), b.double().transpose(1, 2))
+    a, b = (t.transpose(1, 2).contiguous() if mn else t for t, mn in ((a, a_mn), (b, b_mn)))
+    _lib.profile_enable(True)
+    got = bgemm(a, b, a_mn_major=a_mn, b_mn_major=b_mn, check=True)
+    names = set(_lib.profile_summary())
+    _lib.profile_enable(False)
+    assert names == {"tc_bgemm_pair"}, names
+    rel = ((got.double() - want).norm() / want.norm()).item()
+    # tf32 drops 13 mantissa bits of either factor; the results' own rounding otherwise
+    assert rel < {torch.float32: 1e-3, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype], rel
