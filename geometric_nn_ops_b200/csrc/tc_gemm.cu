@@ -149,7 +149,7 @@ int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const
   const int es = dtype == TRI_F32 ? 4 : 2;
   const int bke = 128 / es;
   const bool two = p.K1 > 0;
-  if (epi == EPI_STORE && bn == 256 && (!out_f32 || es == 4) && gemm_pair_fits(p, tile_width(p, bn, es))) {
+  if (epi == EPI_STORE && bn == 256 && (!out_f32 || es == 4) && gemm_pair_fits(p, tile_width(p, bn, es), (p.K0 + bke - 1) / bke, es)) {
     CUtensorMap ta, tb;
     TRI_TRY(operand_map(&ta, p.a[0], dtype, kBM));
     TRI_TRY(operand_map(&tb, p.b[0], dtype, kBM));

@@ -2,8 +2,8 @@
 //
 //   warp 0      TMA producer: fills a ring of shared-memory stages (128-byte swizzle) with operand tiles
 //   warp 1      MMA issuer:   tcgen05.mma from the stages into one of two TMEM accumulators
-//   warps 2..9  epilogue:     two groups of four warps (each group covers the 128 TMEM lanes and takes half
-//                             of the accumulator columns): tcgen05.ld, fused epilogue, 16/32-byte stores
+//   warps 2..9  epilogue:     two groups of four warps (each group covers the 128 TMEM lanes and takes every
+//                             other 32 of the accumulator columns): tcgen05.ld, fused epilogue, 16/32-byte stores
 //
 // A tile is 128 (M) x BN (N); K advances 128 bytes per stage (64 bf16/fp16 or 32 fp32 elements).  Each
 // operand may be K-major (K contiguous in global memory) or MN-major (M or N contiguous); the second form
@@ -1045,8 +1045,8 @@ struct GemmPlan {
 // dtype: TRI_F32 (tf32 MMA), TRI_BF16, TRI_F16.  out_f32: EPI_STORE writes fp32 instead of the input dtype.
 int launch_gemm(cudaStream_t st, int dtype, int epi, int bn, bool out_f32, const GemmPlan& p, int* err);
 
-// The plain product on pairs of SMs (tc_gemm_pair.cu).  Does it suit, against tiles of 128 x `width`?  ta, tb: boxes of 128 rows.
-bool gemm_pair_fits(const GemmPlan& p, int width);
+// The plain product on pairs of SMs (tc_gemm_pair.cu).  Does it suit, against tiles of 128 x `width`, elements of `es` bytes?  ta, tb: boxes of 128 rows.
+bool gemm_pair_fits(const GemmPlan& p, int width, int kblocks, int es);
 int launch_gemm_pair(cudaStream_t st, int dtype, const CUtensorMap& ta, const CUtensorMap& tb, const GemmPlan& p, int* err);
 
 }  // namespace tc

@@ -229,8 +229,13 @@ int start(cudaStream_t st, const CUtensorMap& ta, const CUtensorMap& tb, const P
 
 }  // namespace
 
-bool gemm_pair_fits(const GemmPlan& p, int width) {
+bool gemm_pair_fits(const GemmPlan& p, int width, int kblocks, int es) {
   if (p.K1 > 0 || p.split_k || p.a_tiles > 0 || p.bias0 != nullptr) return false;
+  // A tile's products must outlast the stores of the one before, 256 KB of fp32 or half of that.  128 planes of 512 x 512, us on single
+  // SMs and on pairs: 16 bits K = 512 (8 blocks of 128 bytes) 41.3 and 42.9, 576 45.4 and 45.3, 640 49.3 and 47.2, 768 55.5 and 50.0;
+  // TF32 K = 256 (8) 50.1 and 55.4, 320 57.2 and 58.0, 384 63.5 and 60.9, 512 78.0 and 71.9.  64 planes of 768 x 768 and 32 of
+  // 1024 x 1024 cross there or one block earlier.
+  if (kblocks < (es == 4 ? 12 : 9)) return false;
   const auto up = [](long long v, long long u) { return (v + u - 1) / u * u; };
   // The products of a pair's tiles beyond the matrix must not outweigh what it saves (a side of 384, training: 380 us without, 395 with),
   // and there must be two tiles for a pair (256, one and three quarters: 203.5 us without, 206 with).

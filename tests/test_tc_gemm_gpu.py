@@ -36,7 +36,7 @@ def test_bgemm(case, dtype, a_mn, b_mn):
 # whole tiles; an M that is no multiple of four, whose rows are stored one by one; rows of an odd length; one tile of 256 x 256 for 148 pairs
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=str)
-@pytest.mark.parametrize("case", [(40, 512, 512, 128), (40, 509, 512, 72), (40, 510, 511, 200), (148, 256, 256, 64)], ids=str)
+@pytest.mark.parametrize("case", [(40, 512, 512, 576), (40, 509, 512, 584), (40, 510, 511, 600), (148, 256, 256, 640)], ids=str)
 def test_pairs_of_sms(case, dtype, a_mn, b_mn):
     from geometric_nn_ops_b200 import _lib
     from geometric_nn_ops_b200.gemm import bgemm
@@ -56,3 +56,18 @@ def test_pairs_of_sms(case, dtype, a_mn, b_mn):
     rel = ((got.double() - want).norm() / want.norm()).item()
     # tf32 drops 13 mantissa bits of either factor; the results' own rounding otherwise
     assert rel < {torch.float32: 1e-3, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype], rel
+
+
+@pytest.mark.parametrize("dtype,K,pair", [(torch.bfloat16, 512, False), (torch.bfloat16, 576, True), (torch.float16, 520, True), (torch.float32, 352, False),
+                                          (torch.float32, 384, True)], ids=str)
+def test_short_sums_stay_on_single_sms(dtype, K, pair):
+    """A pair's tile gains where its products outlast the stores of the tile before."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.gemm import bgemm
+    a, b = torch.ones(40, 512, K, dtype=dtype, device="cuda"), torch.ones(40, 512, K, dtype=dtype, device="cuda")
+    _lib.profile_enable(True)
+    got = bgemm(a, b)
+    names = set(_lib.profile_summary())
+    _lib.profile_enable(False)
+    assert names == {"tc_bgemm_pair" if pair else "tc_bgemm"}
+    assert bool((got == float(K)).all())
