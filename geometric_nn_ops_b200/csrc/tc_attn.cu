@@ -1762,12 +1762,18 @@ int fwd_launch(const TriAttnDesc* d, const void* q, const void* k, const void* v
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, 2.0 * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
   auto kern = bias != nullptr ? attn_fwd_tc_kernel<T, HD, true> : attn_fwd_tc_kernel<T, HD, false>;
   TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<HD>::SMEM));
+  sms_beside_attention() = (int)std::max(0LL, sm_count() - ((blocks - 1) % ((HD == 32 ? 2LL : 1LL) * sm_count()) + 1));   // (32: two CTAs per SM)
   launch_dependent(own ? kLaunchPlainly : us_of_logits(pairs), kern, (unsigned)std::min<long long>({blocks, 2LL * sm_count(), kStatusCtas}), 320, Geo<HD>::SMEM, st, tq, tk, tv, tb, a);
   TRI_LAUNCH_OK();
   return 0;
 }
 
 }  // namespace
+
+int& sms_beside_attention() {
+  static thread_local int sms = 0;
+  return sms;
+}
 
 bool wants_mask_terms(const TriAttnDesc* d) {
   return us_of_logits((double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res) >= kEarlyStartUs;

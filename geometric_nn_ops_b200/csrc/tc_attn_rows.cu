@@ -34,6 +34,7 @@
 
 #include "tc_attn_common.cuh"
 #include "tc_attn_rows.cuh"
+#include "tc_paths.cuh"
 
 namespace tri {
 namespace tc {
@@ -618,6 +619,7 @@ int attn_fwd_rows(const TriAttnDesc* d, const CUtensorMap& tq, const CUtensorMap
   const long long items = combos * cdiv(d->n_seq, rows);
   const double pairs = (double)d->B * d->n_seq * d->H * d->n_res * (double)d->n_res;
   KernelTimer kt("tc_attn_fwd", st, 4.0 * pairs * d->D, (double)dtype_size(d->dtype) * 4.0 * d->B * d->n_seq * (double)d->n_res * d->H * d->D);
+  sms_beside_attention() = (int)(sm_count() - ((items - 1) % sm_count() + 1));
   auto launch = [&](auto elem, auto kern, const CUtensorMap& tb) {
     using M = RowsCfg<decltype(elem)>;
     TRI_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::SMEM));

@@ -141,7 +141,13 @@ static int tile_width(const GemmPlan& p, int bn, int es) {
   int w = std::min(bn, ((p.N + tiles - 1) / tiles + unit - 1) / unit * unit);
   // The tiles of a small product are halved until there is one for every second SM (384 x 768 x 768, 18 of 128 columns: gated product
   // 9.4 -> 7.3 us in 72 of 32, plain one 7.6 -> 7.0; 1000 x 768 x 768, 48: a call of attention_pair_bias 124 -> 122.5).
-  while (w % (2 * unit) == 0 && !p.split_k && 2LL * p.batches * ((p.M + kBM - 1) / kBM) * ((p.N + w - 1) / w) <= sm_count()) w /= 2;
+  // Beside another kernel (the gated product and the attention before it) they are halved as long as they fit the SMs that it leaves,
+  // where they fit at all: attention_pair_bias with one row of 384, 512, 640, 768 tokens, 16 heads, by the rule above, in tiles of 128 and
+  // so: 36.0, 37.6, 36.0 us; 51.2, 49.6, 48.3; 64.7, 63.0, 61.6; 80.3, 78.4, 78.4; three rows of 200 and 512: 31.8, 30.0, 30.0; 65.6,
+  // 63.2, 63.2; where not even those of 128 fit (896, 1000): 97.2, 98.3; 113.7, 114.8.
+  auto count = [&](int width) { return (long long)p.batches * ((p.M + kBM - 1) / kBM) * ((p.N + width - 1) / width); };
+  const int sms = p.beside > 0 && count(w) <= p.beside ? p.beside : sm_count();
+  while (w % (2 * unit) == 0 && !p.split_k && 2 * count(w) <= sms) w /= 2;
   return w;
 }
 

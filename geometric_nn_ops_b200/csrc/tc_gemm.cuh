@@ -1037,6 +1037,7 @@ struct GemmPlan {
   void* const* peer_out = nullptr;   // GATE_IN: per-rank exchange buffers (see GemmArgs)
   int peer_world = 0, peer_rank = 0, peer_batches = 0;
   bool first = false;                // no kernel of this call came before: launched plainly
+  int beside = 0;                    // SMs that the kernel before leaves to this one, which starts beside it
   const char* name = "tc_gemm";
   const char* pair_name = nullptr;   // the timer's name for it on pairs of SMs (null: the same)
   double flops = 0, bytes = 0;

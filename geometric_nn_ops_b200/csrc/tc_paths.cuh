@@ -35,6 +35,8 @@ bool attn_project_supported(const TriAttnProjDesc* d);
 size_t attn_project_ws_bytes(const TriAttnProjDesc* d);
 int attn_project(const TriAttnProjDesc* d, const void* z, const void* ln_w, const void* ln_b, const void* w_qkv,
                  const void* w_bias, void* qkv, void* bias, void* ws, size_t ws_size, cudaStream_t st);
+// SMs without a CTA in the last round of the attention forward that this thread launched last
+int& sms_beside_attention();
 int gate_mul(int dtype, long long n, const void* a, const void* gate, void* out, cudaStream_t st);
 int gated_linear(int dtype, long long M, int K, int W, int N, const void* s, const void* w_gate, const void* o, const void* w_out, void* gated,
                  void* out, int* status, bool after, cudaStream_t st);

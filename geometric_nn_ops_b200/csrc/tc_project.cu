@@ -234,6 +234,7 @@ int gated_linear(int dtype, long long M, int K, int W, int N, const void* s, con
     p.a[0].ptr = a; p.a[0].mn_major = false; p.a[0].inner = k; p.a[0].outer = M; p.a[0].batch = 1; p.a[0].st_outer = k;
     p.b[0].ptr = w; p.b[0].mn_major = false; p.b[0].inner = k; p.b[0].outer = n; p.b[0].batch = 1; p.b[0].st_outer = k;
     p.M = (int)M; p.N = n; p.K0 = k; p.out0 = to; p.ld_out = n; p.aux = aux; p.first = epi == EPI_GATE_MUL && !after;
+    if (epi == EPI_GATE_MUL && after) p.beside = sms_beside_attention();
     p.name = name; p.flops = 2.0 * M * k * n; p.bytes = 2.0 * (M * (double)(k + n) + (double)k * n);
     return launch_gemm(st, dtype, epi, 128, false, p, status);
   };

@@ -108,3 +108,32 @@ def test_refusals():
     assert f(_lib.BF16, 1, 12, 8, 8, p, p, p, p, p, p, p, st) != 0
     assert f(_lib.BF16, 1, 8, 8, 8, off, p, p, p, p, p, p, st) != 0
     assert f(_lib.BF16, 0, 8, 8, 8, p, p, p, p, p, p, p, st) != 0
+
+
+@pytest.mark.parametrize("rows,n", [(1, 200), (1, 512), (1, 768), (1, 1000), (3, 200)])
+def test_beside_an_attention(rows, n):
+    """The gated product's tiles are as many as the attention before it leaves SMs, of 32, 64 or 128 columns: the result is the same."""
+    from geometric_nn_ops_b200 import _lib
+    from geometric_nn_ops_b200.triangle import triangle_attention
+    lib, H, D = _lib.load(), 16, 48
+    M, W = rows * n, H * D
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(1, rows, n, H, D, generator=g, device="cuda").bfloat16() for _ in range(3))
+    bias = torch.randn(1, 1, H, n, n, generator=g, device="cuda").bfloat16()
+    s, _, wg, wo = _operands(M, W)
+    status = torch.zeros(64, dtype=torch.int32, device="cuda")
+    gated, out, g1, want = (torch.full_like(s, float("nan")) for _ in range(4))
+    with torch.no_grad():
+        o = triangle_attention(q, k, v, bias)
+        torch.cuda.synchronize()
+        _call(lib.tri_gated_linear, M, W, s, wg, o, wo, g1, want, status)
+        torch.cuda.synchronize()
+        for _ in range(5):
+            out.fill_(float("nan"))
+            torch.cuda.synchronize()
+            o = triangle_attention(q, k, v, bias)
+            assert _lib.last_path() == "tcgen05"
+            _call(lib.tri_gated_linear_after, M, W, s, wg, o, wo, gated, out, status)
+            torch.cuda.synchronize()
+            assert torch.equal(gated, g1) and torch.equal(out, want)
+    assert int(status[0]) == 0
