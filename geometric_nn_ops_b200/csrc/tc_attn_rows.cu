@@ -142,7 +142,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int i = 0; i < 3; ++i) mbar_init(&bars[g].in[i], 1);
       mbar_init(&bars[g].mma[0], 1); mbar_init(&bars[g].mma[1], 1); mbar_init(&bars[g].p_ready[0], 4); mbar_init(&bars[g].p_ready[1], 4);
     }
-    for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], TERMS ? 1 : 2); mbar_init(&b_free[i], 4 * R); }
+    for (int i = 0; i < kBiasStages; ++i) { mbar_init(&b_full[i], TERMS ? 1 : 1 + 8 * kGroups); mbar_init(&b_free[i], 4 * R); }
     mbar_fence_init();
     if (!TERMS) *err() = 0;
   }
@@ -191,7 +191,9 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // The terms of short calls are made here, which saves a launch: eight lanes have the 64 keys of a row's step, eight keys each;
       // their mask bytes are fetched a step ahead, as three aligned words of which the funnel shift takes the eight bytes.  The
       // softmax warps of the sub-partition miss the instructions: N = 768 took 761 us so and 729 with terms made before, launch
-      // included; N = 256 42.3 and 42.9.
+      // included; N = 256 42.3 and 42.9.  Every lane that writes terms arrives for itself: the lanes then need not meet, and one whose
+      // wait runs out may leave alone (meeting at each step, with a vote on the waits: N = 256 40.1 us in place of 39.7, 301 79.1 and
+      // 76.0; lane 0 waiting for all 41.2 and 79.8).
       dependent_wait();
       int stg = 0;
       uint32_t ph = 0, w[3] = {};
@@ -217,7 +219,7 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int n = 0; n < my_items && ok; ++n) {
         const Item after = item_of(n + 1 < my_items ? n + 1 : n);
         for (int j = 0; j < nk; ++j) {
-          ok = __all_sync(0xffffffffu, mbar_wait_relaxed(&b_free[stg], ph ^ 1, err(), 51));   // (the warp gives up together)
+          ok = mbar_wait_relaxed(&b_free[stg], ph ^ 1, err(), 51);
           if (!ok) break;
           if (lane == 0) {
             mbar_expect_tx(&b_full[stg], HB ? M::TB : 0);
@@ -238,9 +240,8 @@ attn_fwd_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             float4* to = reinterpret_cast<float4*>(smem + M::OFF_M + (stg * kGroups + g) * 256 + k_lane * 4);
             to[0] = make_float4(term[0], term[1], term[2], term[3]);
             to[1] = make_float4(term[4], term[5], term[6], term[7]);
+            mbar_arrive(&b_full[stg]);
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&b_full[stg]);
           if (j + 1 == nk) row = row_of(after);
           fetch(j + 1 < nk ? j + 1 : 0);
           if (++stg == kBiasStages) { stg = 0; ph ^= 1; }
