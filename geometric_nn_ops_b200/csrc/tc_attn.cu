@@ -1395,9 +1395,9 @@ attn_bwd_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 //   The key-mask terms of a (batch, row), by its first head's block: 0 for a kept key, -1e9 for a masked one, -inf beyond N; and in a
 //   second plane times log2(e).
 //   The first blocks transpose the bias instead: out[b][h][k][q] = bias[b][h][q][k], a 64 x 64 tile each.
-// One launch in place of four.  At 301 x 301 residues, 4 heads of 32: 22 us against 18 + 3 + 9 and the gaps between them; at 768 x 768
-// 97 against 88 + 5 + 11, where the bytes are 60: what it waits for is the load, sum, exchange and store of an item, with 24 warps an SM
-// on it (three blocks; two 127).  Also clears the error word.
+// One launch in place of three.  At 301 x 301 residues, 4 heads of 32: 16 us under ncu against 20 + 3 + 9 and the gaps between them; at
+// 768 x 768 71 against 87 + 6 + 12 (85 to 97 in a long step at the power limit), where the bytes are 60: what it waits for is the load,
+// sum, exchange and store of an item, with 24 warps an SM on it (three blocks; with two 1.3 times as long).  Also clears the status.
 struct PrepareArgs {
   const float* stats;
   float *delta, *prep, *mask_terms;

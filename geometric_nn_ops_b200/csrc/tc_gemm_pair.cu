@@ -2,9 +2,10 @@
 //
 // A 128 x 256 tile on one SM reads 12 KB of operands from shared memory per 128 cycles of products (16 k of 16 bits) and gets as much
 // by TMA: 192 bytes a cycle where shared memory carries 128, which is what the kernel of tc_gemm.cuh runs at (768 x 768 x 768, 128
-// planes, bf16: 117 us, 1.0 PFLOP/s).  In a pair each SM has 128 rows of A and half of B: 8 KB and 8 KB for the same products, and two
-// thirds of the reads from L2.  The same product takes 93 us (1.25 PFLOP/s; 69 by the bytes or the measured GEMM rate), with TF32
-// 512 x 512 x 512 67 instead of 77 (62 by the bytes), 1024 x 1024 x 1024 in bf16 198 instead of 232.
+// planes, bf16: 116 us, 1.0 PFLOP/s).  In a pair each SM has 128 rows of A and half of B: 8 KB and 8 KB for the same products, and two
+// thirds of the reads from L2.  The same product takes 95 us alone and 99 to 107 in loops and steps (1.1 to 1.2 PFLOP/s; 69 by the bytes
+// or the measured GEMM rate), with TF32 512 x 512 x 512 72 instead of 78 (62 by the bytes), 32 planes of 1024 x 1024 x 1024 in bf16 51
+// instead of 61.
 //
 // A cluster of two CTAs, 320 threads each, persistent.  Warp 0 fetches this CTA's part of a stage; its bytes count on the stage's
 // barrier of the first CTA, whose warp 1 issues the products for both and commits to the barriers of both; warps 2-9 are the epilogue:
